@@ -116,6 +116,7 @@ __global__ void __launch_bounds__(256) rope_kernel(__nv_bfloat16* __restrict__ q
 // ------------------------------------------------------------------------------------------
 // plan: page table -> per-row attention / append metadata  (flashinfer_utils.py:86-124, 217-225)
 // ------------------------------------------------------------------------------------------
+constexpr int PLAN_SMEM_REQ = 1024;     // request tables up to this long are searched in shared memory, longer ones in place
 __global__ void __launch_bounds__(1024) plan_rows_kernel(const int32_t* __restrict__ qo_indptr,
                                                          const int32_t* __restrict__ kv_indptr,
                                                          const int32_t* __restrict__ kv_indices,
@@ -130,17 +131,43 @@ __global__ void __launch_bounds__(1024) plan_rows_kernel(const int32_t* __restri
   pdl_sync();
   __shared__ int32_t warp_tot[32];
   __shared__ int32_t carry;
+  __shared__ int32_t qo_sm[PLAN_SMEM_REQ + 1];
   const int tid = threadIdx.x;
-  // pass 1: per request, fill its rows
-  for (int r = tid; r < n_req; r += blockDim.x) {
-    const int row0 = qo_indptr ? qo_indptr[r] : r;
-    const int n_new = qo_indptr ? qo_indptr[r + 1] - row0 : 1;
-    const int p0 = kv_indptr[r];
-    const int kv_len = kv_len_in ? kv_len_in[r] : (kv_indptr[r + 1] - p0 - 1) * page_size + last_page_len[r];
-    for (int j = 0; j < n_new; ++j) {
-      const int row = row0 + j;
-      if (row >= n_rows_padded) break;
-      const int g = kv_len - n_new + j;
+  // pass 1: every row finds its request in qo_indptr (the last one that starts at or before it: requests without rows
+  // are stepped over).  One thread per row, not per request: a thread that walked its request's rows one after the other
+  // made the plan of a 1024-row prompt step 89 us (three prompts) to 120 us (two), most of it dependent page-table loads;
+  // this way it takes 5 us.
+  const int32_t* qo = qo_indptr;
+  if (qo_indptr && n_req <= PLAN_SMEM_REQ) {
+    for (int r = tid; r <= n_req; r += blockDim.x) qo_sm[r] = qo_indptr[r];
+    __syncthreads();
+    qo = qo_sm;
+  }
+  const int n_valid = qo ? qo[n_req] : n_req;
+  const int first = qo ? qo[0] : 0;
+  for (int row = tid; row < n_rows_padded; row += blockDim.x) {
+    if (row >= n_valid) {
+      row_req[row] = -1;
+      row_pagebase[row] = 0;
+      row_old[row] = 0;
+      row_kvlen[row] = 0;
+      row_page[row] = -1;
+      row_slot[row] = 0;
+    } else if (row >= first) {
+      int r = row, row0 = row, n_new = 1;
+      if (qo) {
+        int lo = 0, hi = n_req;          // qo[lo] <= row < qo[hi]
+        while (hi - lo > 1) {
+          const int mid = (lo + hi) >> 1;
+          if (qo[mid] <= row) lo = mid; else hi = mid;
+        }
+        r = lo;
+        row0 = qo[r];
+        n_new = qo[r + 1] - row0;
+      }
+      const int p0 = kv_indptr[r];
+      const int kv_len = kv_len_in ? kv_len_in[r] : (kv_indptr[r + 1] - p0 - 1) * page_size + last_page_len[r];
+      const int g = kv_len - n_new + (row - row0);
       row_req[row] = r;
       row_pagebase[row] = p0;
       row_old[row] = kv_len - n_new;
@@ -148,15 +175,6 @@ __global__ void __launch_bounds__(1024) plan_rows_kernel(const int32_t* __restri
       row_page[row] = kv_indices[p0 + g / page_size];
       row_slot[row] = g % page_size;
     }
-  }
-  const int n_valid = qo_indptr ? qo_indptr[n_req] : n_req;
-  for (int row = n_valid + tid; row < n_rows_padded; row += blockDim.x) {
-    row_req[row] = -1;
-    row_pagebase[row] = 0;
-    row_old[row] = 0;
-    row_kvlen[row] = 0;
-    row_page[row] = -1;
-    row_slot[row] = 0;
   }
   if (tid == 0) carry = 0;
   __syncthreads();

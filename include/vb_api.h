@@ -484,6 +484,18 @@ int vb_gemm_bf16_grouped_glu(void* d_y, const void* d_w_tiles, const void* x_map
                              int n_out, int t_tile, const int32_t* d_tile_group, long long group_bytes, float limit,
                              float slope, void* stream);
 
+/* The projections above for steps of many rows, on pairs of SMs (gemm_wide.cu): modes, packed weights, epilogues and rounding as
+ * vb_gemm_bf16 / _grouped / _glu (glu_limit > 0), tile_rows 32, 64, 96 or 128.  n_tok: token rows per tile, a multiple of 16 up to
+ * 256; x_map (row-major activations): a vb_tensor_map_2d_bf16 map whose box has n_tok / 2 rows; d_x_tiles: the XT(vb_gemm_t_tile(T))
+ * layout, whatever n_tok is (y_tiled output is written in the same layout).  With d_tile_group, tile i (rows i * n_tok ..) is
+ * multiplied by the weights of group d_tile_group[i].
+ * vb_gemm_wide_timeouts: how many waits of that kernel have run out in this process (0 unless something is wrong; synchronises). */
+int vb_gemm_bf16_wide(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
+                      int mode, int split_k, int tile_rows, int n_out, int y_tiled, const void* d_bias, int act, int n_tok,
+                      const int32_t* d_tile_group, long long group_bytes, int w_kb_stride, int group_kb, int kb_base,
+                      float glu_limit, float glu_slope, void* stream);
+int vb_gemm_wide_timeouts(void);
+
 /* ---- hybrid decoder stacks with an fp32 residual stream (norm_linear.cu, window_attn.cu, linear_attn.cu,
  * gated_recurrence.cu, moe.cu) ----
  * dtype arguments: 0 = bf16, 1 = fp32.  Norm weights, router weights, decays and recurrent states are always fp32.

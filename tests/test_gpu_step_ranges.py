@@ -41,3 +41,63 @@ def test_plan_rows_prefill(ops, new, old, pad):
     assert plan.row_pagebase[:T].tolist() == [ip[r] for r in req] and plan.row_old[:T].tolist() == [kv[r] - new[r] for r in req]
     chunks = [(g + chunk) // chunk for g in at] + [0] * pad
     assert plan.row_chunk_start[:T + pad + 1].tolist() == [0] + np.cumsum(chunks).tolist()
+
+
+def _tiled(ops, x):
+    """x in the tiled activation layout, written through its index formula"""
+    T, K = x.shape
+    t = ops.TiledAct(T, K, "cuda")
+    n, kb = t.t_tile, (K + 63) // 64
+    r, k = torch.arange(T, device="cuda")[:, None], torch.arange(K, device="cuda")[None]
+    at = (((r // n) * kb + (k >> 6)) * n + r % n) * 64 + ((((k >> 3) & 7) ^ (r % n & 7)) << 3) + (k & 7)
+    t.data[at.reshape(-1)] = x.reshape(-1)
+    return t
+
+
+def _close(got, ref, bound):
+    err = ((got.double() - ref).norm() / ref.norm()).item()
+    assert err < bound, err
+
+
+# rows: first one of the kernel for pairs of SMs, its 16-row remainders, one block of the tiled layout and one row more, three
+# blocks; weight rows: one tile, an odd number of tiles (the last pair half empty), tile heights with 1, 2 and 4 tiles per CTA;
+# k: a remainder of the 64-k blocks, odd numbers of blocks per 128-k stage, more than the ring holds
+@pytest.mark.parametrize("T,N,K,tile_rows", [(65, 128, 64, 128), (96, 384, 200, 128), (133, 640, 704, 64), (255, 96, 192, 32),
+                                             (256, 480, 320, 96), (257, 1280, 1096, 128), (529, 960, 512, 96), (777, 448, 576, 64)])
+def test_wide_projection(ops, T, N, K, tile_rows):
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, K, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    b = torch.randn(N, generator=g, device="cuda").bfloat16()
+    ref = x.double() @ w.double().T
+    pw = ops.pack_weight(w, tile_rows)
+    for xin in (x, _tiled(ops, x)):
+        for split in (1, min(3, (K + 63) // 64)):
+            p = ops.gemm(xin, pw, mode=1, split_k=split, tile_rows=tile_rows, out=torch.full((split, T, N), float("nan"), device="cuda"))
+            _close(p.sum(0), ref, 2e-6)                       # 32-bit sums: 2^-24 times the square root of the terms
+        y = ops.gemm(xin, pw, mode=0, tile_rows=tile_rows, bias=b, act="relu2", out=torch.full((T, N), float("nan"), device="cuda").bfloat16())
+        _close(y, torch.relu(ref + b.double()) ** 2, 2 ** -8)   # one rounding to bf16
+    if N % 64 == 0 and (N // 2) % (tile_rows // 2) == 0:
+        gate, up = w[:N // 2].contiguous(), w[N // 2:].contiguous()
+        gu = ops.pack_weight(ops.interleave_gate_up(gate, up, tile_rows // 2), tile_rows)
+        ref = torch.nn.functional.silu(x.double() @ gate.double().T) * (x.double() @ up.double().T)
+        xt, yt = _tiled(ops, x), ops.TiledAct(T, N // 2, "cuda")
+        _close(ops.gemm(x, gu, mode=2, tile_rows=tile_rows, n_out=N // 2), ref, 4 * 2 ** -8)      # gate, up, silu and product rounded
+        _close(ops.gemm(xt, gu, mode=2, tile_rows=tile_rows, n_out=N // 2, out=yt).to_rows(), ref, 4 * 2 ** -8)
+    from vox_serve_b200 import _lib
+
+    assert _lib.load().vb_gemm_wide_timeouts() == 0
+
+
+@pytest.mark.parametrize("groups,tt,N,K", [(1, 128, 256, 128), (3, 128, 320, 456), (5, 64, 128, 192)])
+def test_wide_grouped_projection(ops, groups, tt, N, K):
+    g = torch.Generator(device="cuda").manual_seed(groups)
+    tiles = groups + 2
+    x = torch.randn(tiles * tt, K, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(groups, N, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    pw = ops.pack_weight(w.view(groups * N, K), 64)
+    grp = [(7 * i) % groups for i in range(tiles)]
+    out = torch.full((tiles * tt, N), float("nan"), device="cuda")
+    ops.gemm_grouped(x, pw, out, 1, N, K, tt, _i32(grp), group_bytes=ops.weight_tiles_bytes(N, K, 64))
+    ref = torch.cat([x[i * tt:(i + 1) * tt].double() @ w[e].double().T for i, e in enumerate(grp)])
+    _close(out, ref, 2e-6)

@@ -189,10 +189,10 @@ class LlamaEngine:
         self.split_qkv = int(os.environ.get("VB_SPLIT_QKV", self.split_qkv))
         self.split_o = int(os.environ.get("VB_SPLIT_O", self.split_o))
         self.split_down = int(os.environ.get("VB_SPLIT_DOWN", self.split_down))
-        self._split_cache: Dict[Tuple[int, int], Tuple[int, int, int]] = {}
+        self._split_cache: Dict[int, Tuple[int, int, int]] = {}
         # split-K partials: the largest (split x rows) any step size up to R needs (prefill-sized steps split as well, see
         # _splits: 24-40 weight tiles x one or two token tiles do not fill 148 SMs)
-        need = max(max(self._splits(t)) * t for t in sorted({min(R, t) for t in (64, 256, 512, 768, 1024, R)}))
+        need = max(max(self._splits(min(R, 64))) * min(R, 64), ops.WIDE_SPLIT_ROWS if R >= ops.WIDE_MIN_ROWS else 0)
         self.hidden = torch.zeros(R, H, dtype=BF16, device=dev)
         self.normed = torch.zeros(R, H, dtype=BF16, device=dev)
         self.partials = torch.zeros(max(need, R) * max(self.qkv_w, H), dtype=torch.float32, device=dev)
@@ -236,14 +236,13 @@ class LlamaEngine:
 
     def _splits(self, rows: int) -> Tuple[int, int, int]:
         """split-K of the QKV / O / down projections of a step with ``rows`` token rows.  Decode-sized steps use the tuned
-        values; larger steps re-apply the same rule to (weight tiles x 256-row token tiles): a 133-row prefill is ONE token
-        tile, i.e. 24-40 CTAs per projection without split-K (measured: the 133-token Orpheus prefill took ~7 ms of a 63 ms
-        TTFA that way)."""
+        values; larger steps weigh the last wave against the planes a split leaves (ops.wide_plan): a 133-row prompt is ONE token
+        tile, i.e. 12-20 units per projection on 74 pairs of SMs without a split, a 1024-row step needs none."""
         if rows <= self.FUSED_MAX_ROWS:
             return self.split_qkv, self.split_o, self.split_down
         if os.environ.get("VB_PREFILL_SPLIT", "1") == "0":           # (A/B switch: round-1 behaviour)
             return 1, 1, 1
-        key = (rows + 255) // 256
+        key = rows
         if key not in self._split_cache:
             d = self.dims
             H, I, hqD = d.hidden_size, d.intermediate_size, d.num_attention_heads * d.head_dim

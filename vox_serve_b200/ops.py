@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes
 import math
 import os
+from functools import lru_cache
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -368,9 +369,55 @@ def gemm_t_tile(T: int) -> int:
     return _lib.load().vb_gemm_t_tile(int(T))
 
 
+# Steps of more rows than this run their projections on the kernel for pairs of SMs (gemm_wide.cu): from 80 rows on it is
+# as fast or faster on every projection measured (80 rows: QKV 11.1 against 12.3 us, gate/up 25.1 against 27.4, down 13.0
+# against 14.5; 1024 rows: 33 / 63, 86 / 171, 41 / 79); up to 64 rows the one-SM kernel's layouts and fused tails apply.
+WIDE_MIN_ROWS = 65
+WIDE_TILE_ROWS = (32, 64, 96, 128)
+WIDE_SPLIT_ROWS = 1664       # most (split x rows) of fp32 planes a projection is split into
+
+
+@lru_cache(maxsize=8192)
+def wide_plan(T: int, N: int, K: int, tile_rows: int, pairs: int, splittable: bool = False) -> Tuple[int, int]:
+    """(token rows per tile, split of k) of a projection on ``pairs`` pairs of SMs.  A pair works through whole units of 256
+    weight rows x one token tile x one k range, so the last wave decides: 1024 rows in 256-token tiles leave the 5120-row QKV
+    projection 80 units on 74 pairs (38.7 us), in 176-token tiles 120 (35.7 us).  The model behind the choice, in us, fitted
+    to measured launches: a 128-k stage takes 0.52 up to 128 tokens and 0.0008 more per further token, a unit 2.5 beside its
+    stages (its epilogue where nothing overlaps it), a plane beyond the first its reading by the consumer."""
+    kb, tiles = (K + 63) // 64, (N + tile_rows - 1) // tile_rows
+    per_pair = 2 * (128 // tile_rows)
+    n_pairs = (tiles + per_pair - 1) // per_pair
+    best = None
+    b0 = (T + 255) // 256
+    for blocks in range(b0, b0 + 4):
+        n = min(256, ((T + blocks - 1) // blocks + 15) // 16 * 16)
+        t_blocks = (T + n - 1) // n
+        stage = 0.52 + 0.0008 * max(0, n - 128)
+        for split in range(1, max(1, min(16, kb // 8)) + 1 if splittable else 2):
+            if split > 1 and split * T > WIDE_SPLIT_ROWS:
+                break
+            waves = (n_pairs * t_blocks * split + pairs - 1) // pairs
+            cost = waves * (stage * ((kb + split - 1) // split + 1) / 2 + 2.5) + (split - 1) * T * N * 8e-7
+            if best is None or cost < best[0] - 1e-9:
+                best = (cost, n, split)
+    return best[1], best[2]
+
+
+def _use_wide(T: int, tile_rows: int) -> bool:
+    return T >= WIDE_MIN_ROWS and tile_rows in WIDE_TILE_ROWS
+
+
+def _wide_tokens(T: int, N: int, K: int, tile_rows: int, split: int) -> int:
+    """token rows per tile for a given split: the choice for ``split`` times as many weight tiles on a k range as long"""
+    return wide_plan(T, N * split, max(64, K // split), tile_rows, device_info()[0] // 2)[0]
+
+
 def choose_split_k(N: int, K: int, T: int, sms: Optional[int] = None) -> int:
-    """Spread a skinny (weight-streaming) projection over all SMs: CTAs = ceil(N/128) * split_k."""
+    """Spread a projection over all SMs.  Up to 64 rows: skinny (weight streaming), CTAs = ceil(N/128) * split_k; beyond:
+    ``wide_plan``."""
     sms = device_info()[0] if sms is None else sms
+    if T >= WIDE_MIN_ROWS:
+        return wide_plan(T, N, K, 128, sms // 2, True)[1]
     tiles = (N + 127) // 128 * ((T + 255) // 256)
     num_kb = (K + 63) // 64
     if tiles >= sms:
@@ -451,21 +498,32 @@ def gemm(x, w, mode: int = 0, split_k: int = 1, out=None, tile_rows: int = 128, 
     (with act: act(gate)*up in fp32, rounded once) with w rows packed per tile_rows-row tile (see interleave_gate_up; n_out
     defaults to N/2)."""
     pw = _packed(w, tile_rows)
-    if isinstance(x, TiledAct):
-        T, K = x.T, x.K
+    tiled_x = isinstance(x, TiledAct)
+    if tiled_x:
+        T, K, dev = x.T, x.K, x.data.device
         assert K == pw.K and x.t_tile == gemm_t_tile(T)
-        x_map_ptr, x_tiles_ptr, dev = None, x.data.data_ptr(), x.data.device
     else:
         _need_cuda(x)
         assert x.dtype == BF16 and x.dim() == 2 and x.shape[1] == pw.K
-        T, K = x.shape
-        x_map_ptr, x_tiles_ptr, dev = tensor_map_2d(x, gemm_t_tile(T)).ptr, None, x.device
+        (T, K), dev = x.shape, x.device
     N = pw.N
+    wide = _use_wide(T, tile_rows) and (tiled_x or not isinstance(out, TiledAct))
+    n_tok = _wide_tokens(T, N, K, tile_rows, split_k) if wide else 0
+    x_map_ptr = None if tiled_x else tensor_map_2d(x, n_tok // 2 if wide else gemm_t_tile(T)).ptr
+    x_tiles_ptr = x.data.data_ptr() if tiled_x else None
     n_out = (N // 2 if mode == 2 else N) if n_out is None else n_out
+
+    def launch(y, y_tiled, b, a):
+        if wide:
+            call("vb_gemm_bf16_wide", y.data_ptr(), pw.data.data_ptr(), x_map_ptr, x_tiles_ptr, T, N, K, n_out, mode, split_k, tile_rows,
+                 n_out, y_tiled, _p(b), a, n_tok, None, 0, 0, 0, 0, 0.0, 0.0, _stream())
+        else:
+            call("vb_gemm_bf16", y.data_ptr(), pw.data.data_ptr(), x_map_ptr, x_tiles_ptr, T, N, K, n_out, mode, split_k, tile_rows,
+                 n_out, y_tiled, _p(b), a, _stream())
+
     if isinstance(out, TiledAct):
         assert mode == 2 and out.T == T and out.K == n_out
-        call("vb_gemm_bf16", out.data.data_ptr(), pw.data.data_ptr(), x_map_ptr, x_tiles_ptr, T, N, K, n_out, mode, split_k,
-             tile_rows, n_out, 1, None, 0, _stream())
+        launch(out.data, 1, None, 0)
         return out
     if out is None:
         if mode == 1:
@@ -476,8 +534,7 @@ def gemm(x, w, mode: int = 0, split_k: int = 1, out=None, tile_rows: int = 128, 
         _need_cuda(bias)
         assert mode == 0 and bias.dtype == BF16 and bias.numel() == N and bias.is_contiguous()
     assert act is None or mode in (0, 2)
-    call("vb_gemm_bf16", out.data_ptr(), pw.data.data_ptr(), x_map_ptr, x_tiles_ptr, T, N, K, n_out, mode, split_k,
-         tile_rows, n_out, 0, _p(bias), GEMM_ACTS[act], _stream())
+    launch(out, 0, bias, GEMM_ACTS[act])
     return out
 
 
@@ -487,6 +544,11 @@ def gemm_glu(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, limit: float
     _need_cuda(x, out)
     assert x.dtype == BF16 and x.dim() == 2 and x.shape[1] == w.K and out.dtype == BF16 and out.is_contiguous()
     T = x.shape[0]
+    if _use_wide(T, w.tile_rows):
+        n_tok = _wide_tokens(T, w.N, w.K, w.tile_rows, 1)
+        call("vb_gemm_bf16_wide", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, n_tok // 2).ptr, None, T, w.N, w.K, out.shape[1], 2, 1,
+             w.tile_rows, out.shape[1], 0, None, 0, n_tok, None, 0, 0, 0, 0, float(limit), float(slope), _stream())
+        return out
     call("vb_gemm_bf16_glu", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, gemm_t_tile(T)).ptr, T, w.N, w.K, out.shape[1],
          w.tile_rows, out.shape[1], float(limit), float(slope), _stream())
     return out
@@ -1476,6 +1538,12 @@ def gemm_grouped(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, mode: in
     assert x.dtype == BF16 and x.dim() == 2 and x.shape[1] == K and out.is_contiguous()
     assert tile_group is None or x.shape[0] % t_tile == 0
     n_out = (N // 2 if mode == 2 else N) if n_out is None else n_out
+    if _use_wide(x.shape[0], w.tile_rows):       # (row tiles of groups keep their size: a tile belongs to one group)
+        n_tok = t_tile if tile_group is not None else _wide_tokens(x.shape[0], N, K, w.tile_rows, 1)
+        call("vb_gemm_bf16_wide", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, n_tok // 2).ptr, None, x.shape[0], N, K, n_out, mode, 1,
+             w.tile_rows, n_out, 0, None, GEMM_ACTS[act], n_tok, _p(tile_group), int(group_bytes), int(w_kb_stride), int(group_kb),
+             int(kb_base), 0.0, 0.0, _stream())
+        return out
     call("vb_gemm_bf16_grouped", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, t_tile).ptr, x.shape[0], N, K, n_out,
          mode, w.tile_rows, n_out, t_tile, _p(tile_group), int(group_bytes), int(w_kb_stride), int(group_kb), int(kb_base),
          GEMM_ACTS[act], _stream())
@@ -1728,6 +1796,10 @@ def gemm_grouped_glu(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, N: i
     (N = 2 * ff rows per group), out bf16 [rows, N / 2]."""
     _need_cuda(x, out)
     assert x.dtype == BF16 and x.dim() == 2 and x.shape[1] == K and out.is_contiguous() and x.shape[0] % t_tile == 0
+    if _use_wide(x.shape[0], w.tile_rows):
+        call("vb_gemm_bf16_wide", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, t_tile // 2).ptr, None, x.shape[0], N, K, N // 2, 2, 1,
+             w.tile_rows, N // 2, 0, None, 0, t_tile, _p(tile_group), int(group_bytes), 0, 0, 0, float(limit), float(slope), _stream())
+        return out
     call("vb_gemm_bf16_grouped_glu", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, t_tile).ptr, x.shape[0], N, K, N // 2,
          w.tile_rows, N // 2, t_tile, _p(tile_group), int(group_bytes), float(limit), float(slope), _stream())
     return out

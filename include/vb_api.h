@@ -492,8 +492,11 @@ int vb_gemm_bf16_grouped_glu(void* d_y, const void* d_w_tiles, const void* x_map
  * vb_gemm_wide_timeouts: how many waits of that kernel have run out in this process (0 unless something is wrong; synchronises). */
 int vb_gemm_bf16_wide(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
                       int mode, int split_k, int tile_rows, int n_out, int y_tiled, const void* d_bias, int act, int n_tok,
-                      const int32_t* d_tile_group, long long group_bytes, int w_kb_stride, int group_kb, int kb_base,
-                      float glu_limit, float glu_slope, void* stream);
+                      void* stream);
+int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
+                              int mode, int split_k, int tile_rows, int n_out, int y_tiled, const void* d_bias, int act, int n_tok,
+                              const int32_t* d_tile_group, long long group_bytes, int w_kb_stride, int group_kb, int kb_base,
+                              float glu_limit, float glu_slope, void* stream);
 int vb_gemm_wide_timeouts(void);
 
 /* ---- hybrid decoder stacks with an fp32 residual stream (norm_linear.cu, window_attn.cu, linear_attn.cu,

@@ -53,8 +53,9 @@ SIGNATURES = {
     "vb_weight_tiles_bytes": (c_size_t, [c_int, c_int, c_int]),
     "vb_pack_weight_tiles": (c_int, [P, P, c_int, c_int, c_int64, c_int, P]),
     "vb_gemm_bf16": (c_int, [P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, c_int, P]),
-    "vb_gemm_bf16_wide": (c_int, [P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, c_int, c_int, P, C.c_longlong,
-                                  c_int, c_int, c_int, c_float, c_float, P]),
+    "vb_gemm_bf16_wide": (c_int, [P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, c_int, c_int, P]),
+    "vb_gemm_bf16_wide_grouped": (c_int, [P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, c_int, c_int, P,
+                                          C.c_longlong, c_int, c_int, c_int, c_float, c_float, P]),
     "vb_gemm_wide_timeouts": (c_int, []),
     "vb_proj_residual": (c_int, [P, P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P]),
     "vb_proj_norm_gateup_silu": (c_int, [P, P, P, P, P, c_int, P, c_float, c_int, c_int, c_int, c_int, c_int, c_int, P]),
@@ -258,5 +259,7 @@ launch_counter = [0]
 
 def call(name: str, *args):
     """Invoke an int-returning entry point and raise on error."""
-    check(getattr(load(), name)(*args), name)
+    rc = getattr(_lib or load(), name)(*args)
+    if rc != 0:
+        check(rc, name)
     launch_counter[0] += LAUNCHES.get(name, 1)

@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace vb {
 
 // ---------------------------------------------------------------------------------------------
@@ -32,6 +34,24 @@ void set_error(const char* fmt, ...);
 // of the launch at hand): a per-launch value would be baked into nothing -- CUDA-graph kernel nodes replay
 // against whatever the function attribute was set to last, so a later, smaller launch would break them.
 constexpr int VB_MAX_DYN_SMEM = 227 * 1024;
+// ... once per kernel and device (one flag per instantiation: call it with the kernel itself, not with a pointer that may
+// name several; two threads that arrive together both set the same value)
+template <typename Kernel>
+inline cudaError_t max_dyn_smem_once(Kernel kernel) {
+  static std::atomic<unsigned long long> done{0ull};
+  static std::atomic<const void*> whose{nullptr};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const void* fn = reinterpret_cast<const void*>(kernel);
+  const bool mine = whose.load(std::memory_order_acquire) == fn;
+  if (mine && dev < 64 && (done.load(std::memory_order_acquire) >> dev & 1ull)) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VB_MAX_DYN_SMEM);
+  if (e != cudaSuccess || dev >= 64) return e;
+  const void* none = nullptr;
+  if (mine || whose.compare_exchange_strong(none, fn) || none == fn) done.fetch_or(1ull << dev, std::memory_order_release);
+  return cudaSuccess;
+}
 
 // ---------------------------------------------------------------------------------------------
 // programmatic dependent launch (PDL)

@@ -667,7 +667,7 @@ static int launch_gemm(GemmParams& p, const void* w_tiles, const void* x_map, cu
   const int smem = stages * stage_bytes + p.pad + extra;
   VB_CHECK_ARG(stages <= 20 && smem <= VB_MAX_DYN_SMEM, "gemm: tile too large for shared memory (%d bytes)", smem);
   p.stages = stages;
-  VB_CHECK_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VB_MAX_DYN_SMEM));
+  VB_CHECK_CUDA(max_dyn_smem_once(gemm_bf16_kernel));
   dim3 grid((p.N + p.tile_rows - 1) / p.tile_rows, p.split_k, (p.T + p.t_tile - 1) / p.t_tile);
   // the fused modes reduce split-K through distributed shared memory: cluster = the split_k CTAs of a tile
   const dim3 cluster(1, reducing ? p.split_k : 1, 1);

@@ -455,7 +455,7 @@ int vb_gemm_wide_timeouts(void) {
   return static_cast<int>(n);
 }
 
-int vb_gemm_bf16_wide(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
+int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
                       int mode, int split_k, int tile_rows, int n_out, int y_tiled, const void* d_bias, int act, int n_tok,
                       const int32_t* d_tile_group, long long group_bytes, int w_kb_stride, int group_kb, int kb_base,
                       float glu_limit, float glu_slope, void* stream) {
@@ -491,11 +491,18 @@ int vb_gemm_bf16_wide(void* d_y, const void* d_w_tiles, const void* x_map, const
   const int tail = 1024 /*barriers*/ + 1024 /*alignment*/;
   p.stages = min(GW_MAX_STAGES, (VB_MAX_DYN_SMEM - tail) / stage_bytes);
   const int smem = p.stages * stage_bytes + tail;
-  VB_CHECK_CUDA(cudaFuncSetAttribute(gemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VB_MAX_DYN_SMEM));
+  VB_CHECK_CUDA(max_dyn_smem_once(gemm_wide_kernel));
   const int pairs = min(p.units, gw_pairs());
   VB_CHECK_CUDA(launch_kernel(gemm_wide_kernel, dim3(2 * pairs), dim3(GW_THREADS), smem, static_cast<cudaStream_t>(stream), true, p,
                               x_map ? *static_cast<const CUtensorMap*>(x_map) : dummy_map));
   return 0;
+}
+
+int vb_gemm_bf16_wide(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
+                      int mode, int split_k, int tile_rows, int n_out, int y_tiled, const void* d_bias, int act, int n_tok,
+                      void* stream) {
+  return vb_gemm_bf16_wide_grouped(d_y, d_w_tiles, x_map, d_x_tiles, T, N, K, ldy, mode, split_k, tile_rows, n_out, y_tiled, d_bias, act,
+                                   n_tok, nullptr, 0, 0, 0, 0, 0.f, 0.f, stream);
 }
 
 }  // extern "C"

@@ -20,8 +20,12 @@ from ._lib import VoxB200Error, call
 BF16 = torch.bfloat16
 
 
+# (the raw handle of the current stream, without a torch.cuda.Stream object around it: every launch asks for it)
+_device_index, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_device_index())
 
 
 def _p(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -365,6 +369,7 @@ def paged_attn(q: torch.Tensor, kv_cache, slab_base: int, plan: RowPlan, n_rows:
 # ----------------------------------------------------------------------------------------------
 # projections
 # ----------------------------------------------------------------------------------------------
+@lru_cache(maxsize=8192)
 def gemm_t_tile(T: int) -> int:
     return _lib.load().vb_gemm_t_tile(int(T))
 
@@ -407,6 +412,7 @@ def _use_wide(T: int, tile_rows: int) -> bool:
     return T >= WIDE_MIN_ROWS and tile_rows in WIDE_TILE_ROWS
 
 
+@lru_cache(maxsize=8192)
 def _wide_tokens(T: int, N: int, K: int, tile_rows: int, split: int) -> int:
     """token rows per tile for a given split: the choice for ``split`` times as many weight tiles on a k range as long"""
     return wide_plan(T, N * split, max(64, K // split), tile_rows, device_info()[0] // 2)[0]
@@ -513,17 +519,14 @@ def gemm(x, w, mode: int = 0, split_k: int = 1, out=None, tile_rows: int = 128, 
     x_tiles_ptr = x.data.data_ptr() if tiled_x else None
     n_out = (N // 2 if mode == 2 else N) if n_out is None else n_out
 
-    def launch(y, y_tiled, b, a):
-        if wide:
-            call("vb_gemm_bf16_wide", y.data_ptr(), pw.data.data_ptr(), x_map_ptr, x_tiles_ptr, T, N, K, n_out, mode, split_k, tile_rows,
-                 n_out, y_tiled, _p(b), a, n_tok, None, 0, 0, 0, 0, 0.0, 0.0, _stream())
-        else:
-            call("vb_gemm_bf16", y.data_ptr(), pw.data.data_ptr(), x_map_ptr, x_tiles_ptr, T, N, K, n_out, mode, split_k, tile_rows,
-                 n_out, y_tiled, _p(b), a, _stream())
-
     if isinstance(out, TiledAct):
         assert mode == 2 and out.T == T and out.K == n_out
-        launch(out.data, 1, None, 0)
+        if wide:
+            call("vb_gemm_bf16_wide", out.data.data_ptr(), pw.data.data_ptr(), x_map_ptr, x_tiles_ptr, T, N, K, n_out, mode, split_k,
+                 tile_rows, n_out, 1, None, 0, n_tok, _stream())
+        else:
+            call("vb_gemm_bf16", out.data.data_ptr(), pw.data.data_ptr(), x_map_ptr, x_tiles_ptr, T, N, K, n_out, mode, split_k,
+                 tile_rows, n_out, 1, None, 0, _stream())
         return out
     if out is None:
         if mode == 1:
@@ -534,7 +537,12 @@ def gemm(x, w, mode: int = 0, split_k: int = 1, out=None, tile_rows: int = 128, 
         _need_cuda(bias)
         assert mode == 0 and bias.dtype == BF16 and bias.numel() == N and bias.is_contiguous()
     assert act is None or mode in (0, 2)
-    launch(out, 0, bias, GEMM_ACTS[act])
+    if wide:
+        call("vb_gemm_bf16_wide", out.data_ptr(), pw.data.data_ptr(), x_map_ptr, x_tiles_ptr, T, N, K, n_out, mode, split_k, tile_rows,
+             n_out, 0, _p(bias), GEMM_ACTS[act], n_tok, _stream())
+    else:
+        call("vb_gemm_bf16", out.data_ptr(), pw.data.data_ptr(), x_map_ptr, x_tiles_ptr, T, N, K, n_out, mode, split_k,
+             tile_rows, n_out, 0, _p(bias), GEMM_ACTS[act], _stream())
     return out
 
 
@@ -546,7 +554,7 @@ def gemm_glu(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, limit: float
     T = x.shape[0]
     if _use_wide(T, w.tile_rows):
         n_tok = _wide_tokens(T, w.N, w.K, w.tile_rows, 1)
-        call("vb_gemm_bf16_wide", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, n_tok // 2).ptr, None, T, w.N, w.K, out.shape[1], 2, 1,
+        call("vb_gemm_bf16_wide_grouped", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, n_tok // 2).ptr, None, T, w.N, w.K, out.shape[1], 2, 1,
              w.tile_rows, out.shape[1], 0, None, 0, n_tok, None, 0, 0, 0, 0, float(limit), float(slope), _stream())
         return out
     call("vb_gemm_bf16_glu", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, gemm_t_tile(T)).ptr, T, w.N, w.K, out.shape[1],
@@ -1540,7 +1548,7 @@ def gemm_grouped(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, mode: in
     n_out = (N // 2 if mode == 2 else N) if n_out is None else n_out
     if _use_wide(x.shape[0], w.tile_rows):       # (row tiles of groups keep their size: a tile belongs to one group)
         n_tok = t_tile if tile_group is not None else _wide_tokens(x.shape[0], N, K, w.tile_rows, 1)
-        call("vb_gemm_bf16_wide", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, n_tok // 2).ptr, None, x.shape[0], N, K, n_out, mode, 1,
+        call("vb_gemm_bf16_wide_grouped", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, n_tok // 2).ptr, None, x.shape[0], N, K, n_out, mode, 1,
              w.tile_rows, n_out, 0, None, GEMM_ACTS[act], n_tok, _p(tile_group), int(group_bytes), int(w_kb_stride), int(group_kb),
              int(kb_base), 0.0, 0.0, _stream())
         return out
@@ -1797,7 +1805,7 @@ def gemm_grouped_glu(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, N: i
     _need_cuda(x, out)
     assert x.dtype == BF16 and x.dim() == 2 and x.shape[1] == K and out.is_contiguous() and x.shape[0] % t_tile == 0
     if _use_wide(x.shape[0], w.tile_rows):
-        call("vb_gemm_bf16_wide", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, t_tile // 2).ptr, None, x.shape[0], N, K, N // 2, 2, 1,
+        call("vb_gemm_bf16_wide_grouped", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, t_tile // 2).ptr, None, x.shape[0], N, K, N // 2, 2, 1,
              w.tile_rows, N // 2, 0, None, 0, t_tile, _p(tile_group), int(group_bytes), 0, 0, 0, float(limit), float(slope), _stream())
         return out
     call("vb_gemm_bf16_grouped_glu", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, t_tile).ptr, x.shape[0], N, K, N // 2,

@@ -499,6 +499,39 @@ int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_ma
                               float glu_limit, float glu_slope, void* stream);
 int vb_gemm_wide_timeouts(void);
 
+/* ---- vocoder stages over channels-last fp32 activations [B][T][C] (cl_conv.cu) ----
+ * vb_cl_pack: fp32 weights [N][K] (K = taps x channels, tap-major, the tap furthest back first) -> vb_cl_pack_bytes(N, K) bytes for
+ *   vb_cl_conv; N and K multiples of 32.
+ * vb_cl_conv: y[b][t][n] = sum over taps j < ksize and channels c of x[b][t - (ksize - 1 - j) dil][c] w[n][j][c] for rows
+ *   n_lo <= t < n_hi (positions of x outside [0, Tx) are zero); v += bias[n % cmod]; epilogue 1: v += resid, 2: v = resid + scale[n] v,
+ *   3: v = resid + noise[b * noise_ld + t] v; act 1: Snake with alpha[n % cmod] (alpha tables: [C] values, then [C]
+ *   1 / (alpha + 1e-9)), 2: ELU, 3: gelu (erf).  x_bstride / y_bstride /
+ *   r_bstride: floats from one batch entry to the next (rows are dense: Cin, N and N floats); y, y2 and resid rows on 16-byte
+ *   boundaries.  d_y2 (optional): the activated values, d_y then holds the plain ones.  A transposed convolution of stride s (2 s
+ *   taps): ksize 2, N = s * Cout with n = phase * Cout + co, rows 0 .. T; its output flattened to positions starts `padding` positions in.
+ * vb_cl_dwconv7 / vb_cl_last_conv: depthwise 7 taps ("same") with Snake on both sides; one output channel, `left` positions of
+ *   context, optional tanh -> y [B][t1 - t0].
+ * vb_cl_from_codes, vb_cl_codes_sum, vb_cl_upsample (w [C][2 s]), vb_cl_layernorm, vb_cl_chunk_attention (qkv [B][T][3 C], T <= 64).
+ * vb_cl_timeouts: as vb_gemm_wide_timeouts. */
+int vb_cl_timeouts(void);
+long long vb_cl_pack_bytes(int N, int K);
+int vb_cl_pack(void* d_dst, const float* d_w, int N, int K, void* stream);
+int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, int Tx, const void* d_w, const float* d_bias,
+               const float* d_resid, long long r_bstride, const float* d_scale, const float* d_noise, int noise_ld,
+               const float* d_alpha, int epilogue, int act, int B, int Cin, int N, int cmod, int ksize, int dil, int n_lo, int n_hi,
+               long long y_bstride, void* stream);
+int vb_cl_dwconv7(float* d_y, const float* d_x, long long x_bstride, const float* d_w, const float* d_bias, const float* d_alpha_in,
+                  const float* d_alpha_out, int B, int C, int T, int dilation, int t_lo, int t_hi, void* stream);
+int vb_cl_last_conv(float* d_y, const float* d_x, long long x_bstride, const float* d_w, const float* d_bias, int B, int C, int T,
+                    int ksize, int left, int t0, int t1, int use_tanh, void* stream);
+int vb_cl_from_codes(float* d_z, const int32_t* d_codes0, const int32_t* d_codes1, const int32_t* d_codes2, const float* d_codebooks,
+                     const float* d_proj_w, const float* d_proj_b, int B, int C, int T, int cb_size, int cb_dim, int stride0, int stride1,
+                     int stride2, void* stream);
+int vb_cl_codes_sum(float* d_z0, float* d_z1, const int64_t* d_codes, const float* d_emb, int B, int K, int bins, int D, int T, void* stream);
+int vb_cl_upsample(float* d_y, const float* d_x, const float* d_w, int B, int C, int T, int stride, void* stream);
+int vb_cl_layernorm(float* d_y, const float* d_x, const float* d_w, const float* d_b, int rows, int C, float eps, void* stream);
+int vb_cl_chunk_attention(float* d_out, const float* d_qkv, int B, int C, int H, int T, float max_period, void* stream);
+
 /* ---- hybrid decoder stacks with an fp32 residual stream (norm_linear.cu, window_attn.cu, linear_attn.cu,
  * gated_recurrence.cu, moe.cu) ----
  * dtype arguments: 0 = bf16, 1 = fp32.  Norm weights, router weights, decays and recurrent states are always fp32.

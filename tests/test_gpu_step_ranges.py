@@ -101,3 +101,68 @@ def test_wide_grouped_projection(ops, groups, tt, N, K):
     ops.gemm_grouped(x, pw, out, 1, N, K, tt, _i32(grp), group_bytes=ops.weight_tiles_bytes(N, K, 64))
     ref = torch.cat([x[i * tt:(i + 1) * tt].double() @ w[e].double().T for i, e in enumerate(grp)])
     _close(out, ref, 2e-6)
+
+
+# channels-last vocoder convolutions: one row and several batch entries in a box, box sizes around 128 rows, a range inside the
+# sequence, column tiles with a remainder, dilated taps reaching in front of the start; every epilogue and activation
+@pytest.mark.parametrize("B,T,C,N,ksize,dil,lo,hi,epi,act", [
+    (1, 1, 32, 32, 1, 1, 0, 1, "plain", None), (7, 16, 64, 96, 1, 1, 0, 16, "resid", "snake"), (2, 128, 32, 128, 3, 1, 0, 128, "plain", "elu"),
+    (3, 129, 96, 160, 1, 1, 5, 129, "noise", None), (1, 300, 64, 64, 7, 9, 130, 299, "scale_resid", "gelu"), (40, 3, 128, 512, 2, 1, 0, 3, "resid", None)])
+def test_channels_last_conv(B, T, C, N, ksize, dil, lo, hi, epi, act):
+    from vox_serve_b200 import _lib
+    from vox_serve_b200.tokenizer import _cl
+
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")                 # noqa: E731
+    x, w, b, r = rnd(B, T, C), rnd(N, C, ksize) * (C * ksize) ** -0.5, rnd(N), rnd(B, T, N)
+    sc, nz, al = rnd(N), rnd(B, T), torch.rand(N, generator=g, device="cuda") + 0.5
+    wrap = lambda t: _cl.Act(t.reshape(-1).clone(), B, T, t.shape[-1])           # noqa: E731
+    kw = dict(ksize=ksize, dil=dil, epi=epi, resid=None if epi == "plain" else wrap(r), scale=sc, noise=nz, act=act,
+              alpha=torch.cat((al, 1 / (al + 1e-9))), lo=lo, hi=hi)
+    v = torch.nn.functional.conv1d(torch.nn.functional.pad(x.double().transpose(1, 2), ((ksize - 1) * dil, 0)), w.double(), b.double(),
+                                   dilation=dil).transpose(1, 2)
+    v = {"plain": v, "resid": r + v, "scale_resid": r + sc * v, "noise": r + nz[..., None] * v}[epi].double()
+    z = {None: v, "snake": v + torch.sin(al * v) ** 2 / (al.double() + 1e-9), "elu": torch.nn.functional.elu(v),
+         "gelu": torch.nn.functional.gelu(v)}[act]
+    _close(_cl.conv(wrap(x), _cl.pack_conv(w.reshape(N, -1), C, ksize), N, b, **kw).tensor()[:, lo:hi], z[:, lo:hi], 5e-6)
+    plain, both = _cl.conv(wrap(x), _cl.pack_conv(w.reshape(N, -1), C, ksize), N, b, both=True, **kw)
+    _close(plain.tensor()[:, lo:hi], v[:, lo:hi], 5e-6)                          # 32-bit sums of products exact to 2^-22
+    _close(both.tensor()[:, lo:hi], z[:, lo:hi], 5e-6)
+    assert _lib.load().vb_cl_timeouts() == 0
+
+
+@pytest.mark.parametrize("B,T,C,cout,s,pad", [(1, 1, 32, 32, 2, 1), (5, 17, 64, 64, 8, 4), (2, 130, 128, 32, 5, 0), (1, 200, 64, 96, 3, 2)])
+def test_channels_last_transposed_conv(B, T, C, cout, s, pad):
+    from vox_serve_b200.tokenizer import _cl
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x, w = torch.randn(B, T, C, generator=g, device="cuda"), torch.randn(C, cout, 2 * s, generator=g, device="cuda") * (2 * C) ** -0.5
+    b = torch.randn(cout, generator=g, device="cuda")
+    wp = w.view(C, cout, 2, s).permute(3, 1, 2, 0).reshape(s, cout, 2 * C)
+    y = _cl.conv_transposed(_cl.Act(x.reshape(-1).clone(), B, T, C), _cl.pack_convtr(wp), cout, s, b, pad)
+    ref = torch.nn.functional.conv_transpose1d(x.double().transpose(1, 2), w.double(), b.double(), stride=s)[..., pad:pad + T * s]
+    _close(y.tensor(), ref.transpose(1, 2), 5e-6)
+
+
+@pytest.mark.parametrize("B,T,C,dil,lo,hi,big", [(1, 1, 64, 1, 0, 1, 1.0), (3, 65, 128, 3, 0, 65, 1.0), (2, 200, 64, 9, 7, 199, 1.0), (1, 70, 64, 1, 0, 70, 3e5)])
+def test_channels_last_depthwise_and_last(B, T, C, dil, lo, hi, big):
+    """``big``: arguments of the sine past the range of its reduction (they take the library's)."""
+    from vox_serve_b200.tokenizer import _cl
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x, w = torch.randn(B, T, C, generator=g, device="cuda") * big, torch.randn(C, 7, generator=g, device="cuda")
+    b, a1, a2 = (torch.rand(C, generator=g, device="cuda") + 0.5 for _ in range(3))
+    table = lambda a: torch.cat((a, 1 / (a + 1e-9)))                             # noqa: E731
+
+    def snake(v, a):                       # (the sine of the 32-bit product: at large arguments its rounding is the result)
+        y = (v.float() * a[:, None]).double()
+        return v.double() + torch.sin(y) ** 2 / (a.double()[:, None] + 1e-9)
+
+    xs = _cl.Act(x.reshape(-1).clone(), B, T, C)
+    y = _cl.depthwise7(xs, w, b, table(a1), table(a2) if big == 1.0 else None, dil, lo, hi).tensor()
+    v = torch.nn.functional.conv1d(snake(x.transpose(1, 2), a1), w.double()[:, None], b.double(), dilation=dil, padding=3 * dil, groups=C)
+    v = snake(v.float(), a2) if big == 1.0 else v
+    _close(y[:, lo:hi], v.transpose(1, 2)[:, lo:hi], 5e-6)
+    last = _cl.last_conv(xs, w, b[:1], 7, 3, lo, hi, tanh=False)
+    ref = torch.nn.functional.conv1d(x.double().transpose(1, 2), w.double()[None], b[:1].double(), padding=3)[..., lo:hi]
+    _close(last, ref, 5e-6)

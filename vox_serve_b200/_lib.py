@@ -57,6 +57,18 @@ SIGNATURES = {
     "vb_gemm_bf16_wide_grouped": (c_int, [P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, c_int, c_int, P,
                                           C.c_longlong, c_int, c_int, c_int, c_float, c_float, P]),
     "vb_gemm_wide_timeouts": (c_int, []),
+    "vb_cl_timeouts": (c_int, []),
+    "vb_cl_pack_bytes": (C.c_longlong, [c_int, c_int]),
+    "vb_cl_pack": (c_int, [P, P, c_int, c_int, P]),
+    "vb_cl_conv": (c_int, [P, P, P, C.c_longlong, c_int, P, P, P, C.c_longlong, P, P, c_int, P, c_int, c_int, c_int, c_int, c_int, c_int,
+                           c_int, c_int, c_int, c_int, C.c_longlong, P]),
+    "vb_cl_dwconv7": (c_int, [P, P, C.c_longlong, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P]),
+    "vb_cl_last_conv": (c_int, [P, P, C.c_longlong, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P]),
+    "vb_cl_from_codes": (c_int, [P, P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P]),
+    "vb_cl_codes_sum": (c_int, [P, P, P, P, c_int, c_int, c_int, c_int, c_int, P]),
+    "vb_cl_upsample": (c_int, [P, P, P, c_int, c_int, c_int, c_int, P]),
+    "vb_cl_layernorm": (c_int, [P, P, P, P, c_int, c_int, c_float, P]),
+    "vb_cl_chunk_attention": (c_int, [P, P, c_int, c_int, c_int, c_int, c_float, P]),
     "vb_proj_residual": (c_int, [P, P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P]),
     "vb_proj_norm_gateup_silu": (c_int, [P, P, P, P, P, c_int, P, c_float, c_int, c_int, c_int, c_int, c_int, c_int, P]),
     "vb_proj_norm_qkv_rope_append": (c_int, [P, P, P, P, P, P, c_int, P, c_float, P, P, P, c_int, c_int, c_int, c_int,
@@ -249,7 +261,7 @@ def check(rc: int, what: str = ""):
 
 # kernels (+ memset nodes) each entry point enqueues; everything not listed launches exactly one
 LAUNCHES = {"vb_set_pdl": 0, "vb_set_trace": 0, "vb_weight_tiles_bytes": 0, "vb_tensor_map_kv": 0,
-            "vb_tensor_map_2d_bf16": 0, "vb_gemm_wide_timeouts": 0, "vb_device_info": 0, "vb_sample": 1, "vb_update_repetition_cache": 1,
+            "vb_tensor_map_2d_bf16": 0, "vb_gemm_wide_timeouts": 0, "vb_cl_timeouts": 0, "vb_cl_pack_bytes": 0, "vb_device_info": 0, "vb_sample": 1, "vb_update_repetition_cache": 1,
             "vb_set_gemm_smem_kb": 0, "vb_window_attn_tile_rows": 0, "vb_decay_attn_tile_rows": 0, "vb_decay_attn_tiled": 3, "vb_window_attn": 2, "vb_mingru_tiled": 3, "vb_mingru_scratch_floats": 0,
             "vb_short_conv": 2, "vb_selective_scan_tiled": 3, "vb_selective_scan_piece_rows": 0,
             "vb_selective_scan_scratch_floats": 0, "vb_sigmoid_attn": 1, "vb_ssd_tiled": 3, "vb_ssd_tile_rows": 0,

@@ -30,7 +30,7 @@ bool pdl_enabled(int family) {
 
 // cuTensorMapEncodeTiled comes from the driver; resolve it at run time so the library links without
 // libcuda (the authoring container has no driver).
-static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
+PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   if (fn) return fn;
   void* p = nullptr;

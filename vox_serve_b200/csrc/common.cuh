@@ -294,6 +294,30 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
   __trap();
 }
 
+// A wait that gives up: after 2 s it notes the fact in its translation unit's counter and every later wait of the thread
+// returns at once, so that the block can stop issuing, let its copies land and leave with the context usable.
+static __device__ unsigned int g_wait_timeouts = 0;
+struct BoundedWait {
+  bool dead = false;
+  __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity) {
+    if (dead) return;
+    unsigned long long t0 = 0ull;
+#pragma unroll 1
+    for (uint32_t spin = 1;; ++spin) {
+      if (mbar_try_wait(bar, parity)) return;
+      if ((spin & 255u) == 0u) {
+        const unsigned long long now = gtimer();
+        if (t0 == 0ull) t0 = now;
+        else if (now - t0 > 2000000000ull) {
+          dead = true;
+          atomicAdd(&g_wait_timeouts, 1u);
+          return;
+        }
+      }
+    }
+  }
+};
+
 // ---------------------------------------------------------------------------------------------
 // TMA
 // ---------------------------------------------------------------------------------------------

@@ -47,38 +47,6 @@ struct GemmWideParams {
   float glu_limit, glu_slope;
 };
 
-__device__ unsigned int g_gemm_wide_timeouts = 0;
-
-struct BoundedWait {
-  bool dead = false;
-  __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity) {
-    if (dead) return;
-    const uint32_t a = smem_u32(bar);
-    unsigned long long t0 = 0ull;
-#pragma unroll 1
-    for (uint32_t spin = 1;; ++spin) {
-      uint32_t ok;
-      asm volatile(
-          "{\n\t.reg .pred P;\n\t"
-          "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-          "selp.u32 %0, 1, 0, P;\n\t}\n"
-          : "=r"(ok)
-          : "r"(a), "r"(parity)
-          : "memory");
-      if (ok) return;
-      if ((spin & 255u) == 0u) {
-        const unsigned long long now = gtimer();
-        if (t0 == 0ull) t0 = now;
-        else if (now - t0 > 2000000000ull) {
-          dead = true;
-          atomicAdd(&g_gemm_wide_timeouts, 1u);
-          return;
-        }
-      }
-    }
-  }
-};
-
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
@@ -451,7 +419,7 @@ extern "C" {
 
 int vb_gemm_wide_timeouts(void) {
   unsigned int n = 0;
-  if (cudaMemcpyFromSymbol(&n, g_gemm_wide_timeouts, sizeof(n)) != cudaSuccess) return -1;
+  if (cudaMemcpyFromSymbol(&n, g_wait_timeouts, sizeof(n)) != cudaSuccess) return -1;
   return static_cast<int>(n);
 }
 

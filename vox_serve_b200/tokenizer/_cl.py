@@ -1,0 +1,101 @@
+"""Vocoder convolutions over channels-last activations [B, T, C] (csrc/cl_conv.cu), shared by the SNAC and Mimi decoders: layers
+whose widths are multiples of 32 channels run as one product per tap on tcgen05 (tf32 halves, fp32 accumulation)."""
+from __future__ import annotations
+
+from typing import Optional
+
+import torch
+
+from .. import _lib, ops
+from .._lib import call
+
+EPI = {"plain": 0, "resid": 1, "scale_resid": 2, "noise": 3}
+ACT = {None: 0, "snake": 1, "elu": 2, "gelu": 3}
+
+
+def pack(w: torch.Tensor) -> torch.Tensor:
+    """w fp32 [N, K] on the device (K tap-major, the tap furthest back first) -> packed tiles"""
+    N, K = w.shape
+    dst = torch.empty(_lib.load().vb_cl_pack_bytes(N, K), dtype=torch.uint8, device=w.device)
+    call("vb_cl_pack", dst.data_ptr(), w.contiguous().data_ptr(), N, K, ops._stream())
+    return dst
+
+
+def pack_conv(w: torch.Tensor, cin: int, ksize: int) -> torch.Tensor:
+    """w [Cout, Cin * ksize], channel-major and tap-minor (a flattened Conv1d weight)"""
+    cout = w.shape[0]
+    return pack(w.view(cout, cin, ksize).permute(0, 2, 1).reshape(cout, ksize * cin))
+
+
+def pack_convtr(wp: torch.Tensor) -> torch.Tensor:
+    """wp [stride, Cout, 2 Cin]: per output phase the tap on the input position itself, then the one on its predecessor"""
+    s, cout, k = wp.shape
+    return pack(torch.cat((wp[..., k // 2:], wp[..., :k // 2]), -1).reshape(s * cout, k))
+
+
+class Act:
+    """An activation [B, T, C] inside a buffer: entry b starts at offset + b * bstride floats."""
+    __slots__ = ("buf", "B", "T", "C", "offset", "bstride")
+
+    def __init__(self, buf: torch.Tensor, B: int, T: int, C: int, offset: int = 0, bstride: Optional[int] = None):
+        self.buf, self.B, self.T, self.C, self.offset = buf, B, T, C, offset
+        self.bstride = T * C if bstride is None else bstride
+
+    @classmethod
+    def empty(cls, B: int, T: int, C: int, device) -> "Act":
+        return cls(torch.empty(B * T * C, dtype=torch.float32, device=device), B, T, C)
+
+    @property
+    def ptr(self) -> int:
+        return self.buf.data_ptr() + 4 * self.offset
+
+    def tensor(self) -> torch.Tensor:
+        """[B, T, C] view"""
+        return self.buf.as_strided((self.B, self.T, self.C), (self.bstride, self.C, 1), self.offset)
+
+
+def _ptr(t) -> Optional[int]:
+    return None if t is None else (t.ptr if isinstance(t, Act) else t.data_ptr())
+
+
+def conv(x: Act, w: torch.Tensor, N: int, bias=None, ksize: int = 1, dil: int = 1, epi: str = "plain", resid: Optional[Act] = None,
+         scale=None, noise=None, act: Optional[str] = None, alpha=None, lo: int = 0, hi: Optional[int] = None,
+         both: bool = False):
+    """Causal convolution (zeros before the start) of rows [lo, hi) -> Act [B, T, N]; ``both``: (plain, activated)."""
+    hi = x.T if hi is None else hi
+    y = Act.empty(x.B, x.T, N, x.buf.device)
+    y2 = Act.empty(x.B, x.T, N, x.buf.device) if both else None
+    call("vb_cl_conv", y.ptr, _ptr(y2), x.ptr, x.bstride, x.T, w.data_ptr(), _ptr(bias), _ptr(resid), resid.bstride if resid else 0,
+         _ptr(scale), _ptr(noise), noise.shape[-1] if noise is not None else 0, _ptr(alpha), EPI[epi], ACT[act], x.B, x.C, N, N, ksize, dil,
+         lo, hi, y.bstride, ops._stream())
+    return (y, y2) if both else y
+
+
+def conv_transposed(x: Act, w: torch.Tensor, cout: int, stride: int, bias, pad: int = 0, o_lo: int = 0, o_hi: Optional[int] = None,
+                    act: Optional[str] = None, both: bool = False):
+    """Transposed convolution with 2 * stride taps -> Act [B, T * stride, cout]; ``pad`` positions are dropped in front.  Output
+    positions [o_lo, o_hi) are computed."""
+    T_out = x.T * stride
+    o_hi = T_out if o_hi is None else o_hi
+    n_lo, n_hi = (o_lo + pad) // stride, (o_hi - 1 + pad) // stride + 1
+    N = stride * cout
+    rows = x.T + (1 if pad else 0)
+    out = [Act(torch.empty(x.B * rows * N, dtype=torch.float32, device=x.buf.device), x.B, T_out, cout, pad * cout, rows * N)
+           for _ in range(2 if both else 1)]
+    call("vb_cl_conv", out[0].buf.data_ptr(), out[1].buf.data_ptr() if both else None, x.ptr, x.bstride, x.T, w.data_ptr(), _ptr(bias), None, 0,
+         None, None, 0, None, EPI["plain"], ACT[act], x.B, x.C, N, cout, 2, 1, n_lo, n_hi, rows * N, ops._stream())
+    return tuple(out) if both else out[0]
+
+
+def depthwise7(x: Act, w: torch.Tensor, bias, alpha_in, alpha_out, dil: int, lo: int, hi: int) -> Act:
+    y = Act.empty(x.B, x.T, x.C, x.buf.device)
+    call("vb_cl_dwconv7", y.ptr, x.ptr, x.bstride, w.data_ptr(), _ptr(bias), _ptr(alpha_in), _ptr(alpha_out), x.B, x.C, x.T, dil, lo, hi,
+         ops._stream())
+    return y
+
+
+def last_conv(x: Act, w: torch.Tensor, bias, ksize: int, left: int, t0: int, t1: int, tanh: bool) -> torch.Tensor:
+    """one output channel -> [B, 1, t1 - t0]; w [C, ksize]"""
+    y = torch.empty(x.B, 1, t1 - t0, dtype=torch.float32, device=x.buf.device)
+    call("vb_cl_last_conv", y.data_ptr(), x.ptr, x.bstride, w.data_ptr(), _ptr(bias), x.B, x.C, x.T, ksize, left, t0, t1, int(tanh), ops._stream())
+    return y

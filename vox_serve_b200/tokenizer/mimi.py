@@ -22,7 +22,7 @@ import torch
 
 from .. import ops
 from .._lib import VoxB200Error, call
-from . import _tc
+from . import _cl, _tc
 
 F32 = torch.float32
 
@@ -175,6 +175,10 @@ class MimiDecoder:
         # tensor-core copies (tf32 hi/lo tiles, csrc/snac_mma.cu) of the wide convolutions: key -> packed tiles
         self.tc: Dict[str, torch.Tensor] = {}
         kinds = {idx: kd for kd, idx in self.layout}
+        self.channels_last = self._pack_channels_last(kinds)
+        if self.channels_last:
+            self.loaded = True
+            return self
         for k, v in self.w.items():
             t = None
             if k in ("rvq_first.proj", "rvq_rest.proj") or (k[0] == "t" and k.split(".")[-1] in ("in", "out", "l1", "l2")):
@@ -191,6 +195,78 @@ class MimiDecoder:
                 self.tc[k] = t
         self.loaded = True
         return self
+
+    def _pack_channels_last(self, kinds) -> bool:
+        """Every width a multiple of 32 channels (the deployed configuration): the decoder runs channels-last (_cl.py)."""
+        cfg = self.cfg
+        last = cfg.n_filters
+        widths = [cfg.dimension, cfg.codebook_dim, cfg.dim_feedforward, last] + [
+            last * 2 ** i // cfg.compress for i in range(len(cfg.ratios))]
+        if not (_tc.tc_enabled() and self.device.type == "cuda" and all(n % 32 == 0 and n > 0 for n in widths) and cfg.dimension <= 1024 and
+                last <= 256 and cfg.n_q <= 64 and cfg.dimension % cfg.num_heads == 0 and (cfg.dimension // cfg.num_heads) % 4 == 0 and
+                (cfg.dimension // cfg.num_heads) <= 256):
+            return False
+        for k, v in self.w.items():
+            if k in ("rvq_first.proj", "rvq_rest.proj") or (k[0] == "t" and k.split(".")[-1] in ("in", "out", "l1", "l2")):
+                self.tc[k] = _cl.pack(v)
+            elif k[0] == "d" and k.endswith((".w", ".w1", ".w3")):
+                kind = kinds[int(k[1:].split(".")[0])]
+                if kind == "convtr":
+                    self.tc[k] = _cl.pack_convtr(v)
+                elif kind != "conv_out":
+                    ks = cfg.kernel_size if kind == "conv_in" else (cfg.residual_kernel_size if k.endswith(".w1") else 1)
+                    self.tc[k] = _cl.pack_conv(v, v.shape[1] // ks, ks)
+        return True
+
+    def _decode_channels_last(self, c: torch.Tensor, taps: Optional[dict]) -> torch.Tensor:
+        """The decoder over [B, T, C] activations: the stages of the channel-first form below, every ELU applied where its
+        input is produced."""
+        cfg, w, tc, st = self.cfg, self.w, self.tc, ops._stream()
+        (B, K, T), C, D, s = c.shape, cfg.dimension, cfg.codebook_dim, cfg.upsample_stride
+        if T * s > 64:
+            raise VoxB200Error(f"chunks of {T} frames exceed the attention kernel's 64 positions: decode in shorter chunks")
+        new = lambda t, ch: _cl.Act.empty(B, t, ch, self.device)                 # noqa: E731
+        z0, z1 = new(T, D), new(T, D)
+        call("vb_cl_codes_sum", z0.ptr, z1.ptr, c.data_ptr(), w["codebooks"].data_ptr(), B, K, cfg.bins, D, T, st)
+        x = _cl.conv(z0, tc["rvq_first.proj"], C)
+        if K > 1:
+            x = _cl.conv(z1, tc["rvq_rest.proj"], C, epi="resid", resid=x)
+        u, T = new(T * s, C), T * s
+        call("vb_cl_upsample", u.ptr, x.ptr, w["upsample"].data_ptr(), B, C, T // s, s, st)
+        x = u
+        if taps is not None:
+            taps["latent"] = x.tensor().transpose(1, 2).contiguous()
+
+        def norm(v, name):
+            y = new(T, C)
+            call("vb_cl_layernorm", y.ptr, v.ptr, w[name + "w"].data_ptr(), w[name + "b"].data_ptr(), B * T, C, 1e-5, st)
+            return y
+
+        for i in range(cfg.num_layers):
+            p = f"t{i}."
+            qkv, a = _cl.conv(norm(x, p + "n1"), tc[p + "in"], 3 * C), new(T, C)
+            call("vb_cl_chunk_attention", a.ptr, qkv.ptr, B, C, cfg.num_heads, T, float(cfg.max_period), st)
+            x = _cl.conv(a, tc[p + "out"], C, epi="scale_resid", resid=x, scale=w[p + "s1"])
+            m = _cl.conv(norm(x, p + "n2"), tc[p + "l1"], cfg.dim_feedforward, act="gelu")
+            x = _cl.conv(m, tc[p + "l2"], C, epi="scale_resid", resid=x, scale=w[p + "s2"])
+        if taps is not None:
+            taps["transformer_out"] = x.tensor().transpose(1, 2).contiguous()
+        ch, ratios = cfg.n_filters * 2 ** len(cfg.ratios), list(cfg.ratios)
+        plain = None
+        for kind, idx in self.layout:
+            d = f"d{idx}."
+            if kind == "conv_in":
+                x = _cl.conv(x, tc[d + "w"], ch, w[d + "b"], ksize=cfg.kernel_size, act="elu")
+            elif kind == "convtr":
+                ch //= 2
+                plain, x = _cl.conv_transposed(x, tc[d + "w"], ch, ratios.pop(0), w[d + "b"], act="elu", both=True)
+            elif kind == "res":
+                h = _cl.conv(x, tc[d + "w1"], ch // cfg.compress, w[d + "b1"], ksize=cfg.residual_kernel_size, act="elu")
+                x = _cl.conv(h, tc[d + "w3"], ch, w[d + "b3"], epi="resid", resid=plain, act="elu")
+            else:
+                k = cfg.last_kernel_size
+                return _cl.last_conv(x, w[d + "w"], w[d + "b"], k, k - 1, 0, x.T, tanh=False)
+        raise VoxB200Error("a decoder without its last convolution")
 
     # ---- kernels ------------------------------------------------------------------------------------------
     def _conv(self, y, x, key, bias, B, cin, cout, T, ksize=1, dil=1, epi=0, resid=None, scale=None, elu_in=False):
@@ -223,6 +299,8 @@ class MimiDecoder:
         B, K, T = c.shape
         if K > cfg.n_q:
             raise VoxB200Error(f"{K} codebooks given, the quantizer has {cfg.n_q}")
+        if self.channels_last:
+            return self._decode_channels_last(c, taps)
         C, D = cfg.dimension, cfg.codebook_dim
         e = dict(dtype=F32, device=dev)
         # ---- split RVQ decode: rvq_first(codebook 0) + rvq_rest(codebooks 1..) ----

@@ -19,6 +19,7 @@ import torch
 
 from .. import ops
 from .. import _lib
+from . import _cl
 from .._lib import VoxB200Error, call
 
 
@@ -130,7 +131,19 @@ class SNAC:
         tcgen05 tf32 hi/lo kernel (vb_snac_pack_tf32x3); narrower layers (test-sized configs) stay on the SIMT
         kernels.  VB_SNAC_FP32=1 keeps everything on the SIMT kernels."""
         self.tc: Dict[str, torch.Tensor] = {}
+        self.channels_last = False
         if self.device.type != "cuda" or os.environ.get("VB_SNAC_FP32", "0") == "1":
+            return
+        # every width a multiple of 64 channels (the deployed configuration): the whole decoder runs channels-last (_cl.py)
+        if self.latent_dim % 64 == 0 and self.decoder_dim % (64 << len(self.decoder_rates)) == 0:
+            self.channels_last = True
+            for k, v in self.w.items():
+                if k.endswith(("pw_w", "noise_w")):
+                    self.tc[k] = _cl.pack(v)
+                elif k.endswith("ct_w"):
+                    self.tc[k] = _cl.pack_convtr(v)
+                elif "alpha" in k:
+                    self.tc[k] = torch.cat((v, 1.0 / (v + 1e-9)))
             return
         st = ops._stream()
         for k, v in self.w.items():
@@ -228,6 +241,44 @@ class SNAC:
             hi = min(lens[b], (cur[1] - 1 + pad) // s + 1)
         return blocks, (lo, hi)
 
+    def _noises(self, noises, B: int, T: int):
+        if noises is not None:
+            return noises
+        shapes = self.noise_shapes(B, T)
+        if self.noise_source is not None:
+            return self.noise_source(shapes)
+        # one launch for the four NoiseBlock inputs (the reference draws torch.randn per block, snac.py:208); the
+        # device-side offset advances per call, so a captured vocoder graph draws fresh noise every replay
+        sizes = [math.prod(s) for s in shapes]
+        flat = ops.randn(torch.empty(sum(sizes), dtype=torch.float32, device=self.device), rng_state=self.ensure_noise_state())
+        return [t.view(s) for t, s in zip(torch.split(flat, sizes), shapes)]
+
+    def _decode_channels_last(self, c, B: int, T: int, blocks, in_range, out_range, noises) -> torch.Tensor:
+        """The decoder over [B, T, C] activations: same stages, ranges and fused Snakes as the channel-first form below."""
+        w, dev, C = self.w, self.device, self.latent_dim
+        z = _cl.Act.empty(B, T, C, dev)
+        call("vb_cl_from_codes", z.ptr, c[0].data_ptr(), c[1].data_ptr(), c[2].data_ptr(), w["codebooks"].data_ptr(),
+             w["proj_w"].data_ptr(), w["proj_b"].data_ptr(), B, C, T, self.codebook_size, self.codebook_dim, *self.vq_strides, ops._stream())
+        x = _cl.depthwise7(z, w["in_dw_w"], w["in_dw_b"], None, None, 1, *in_range)
+        ch = self.decoder_dim
+        x = _cl.conv(x, self.tc["in_pw_w"], ch, w["in_pw_b"], act="snake", alpha=self.tc["b0.alpha"], lo=in_range[0], hi=in_range[1])
+        noises, nb = self._noises(noises, B, T), len(self.decoder_rates)
+        for bi, s in enumerate(self.decoder_rates):
+            (c_lo, c_hi), units = blocks[bi]
+            ch //= 2
+            u = _cl.conv_transposed(x, self.tc[f"b{bi}.ct_w"], ch, s, w[f"b{bi}.ct_b"], (s + 1) // 2, c_lo, c_hi)
+            nz = noises[bi].to(device=dev, dtype=torch.float32).contiguous()
+            assert nz.numel() == B * u.T, "noise tensor shape mismatch"
+            x = _cl.conv(u, self.tc[f"b{bi}.noise_w"], ch, epi="noise", resid=u, noise=nz.view(B, u.T), lo=c_lo, hi=c_hi)
+            for j, dil in enumerate((1, 3, 9)):
+                q, (u_lo, u_hi) = f"b{bi}.r{j}.", units[j]
+                h = _cl.depthwise7(x, w[q + "dw_w"], w[q + "dw_b"], self.tc[q + "alpha1"], self.tc[q + "alpha2"], dil, u_lo, u_hi)
+                # the last unit's output only feeds the next stage's Snake: fused into this epilogue
+                nxt = None if j < 2 else self.tc[f"b{bi + 1}.alpha" if bi + 1 < nb else "out.alpha"]
+                x = _cl.conv(h, self.tc[q + "pw_w"], ch, w[q + "pw_b"], epi="resid", resid=x, act=None if nxt is None else "snake",
+                             alpha=nxt, lo=u_lo, hi=u_hi)
+        return _cl.last_conv(x, w["out.w"], w["out.b"], 7, 3, *out_range, tanh=True)
+
     @torch.no_grad()
     def decode(self, codes: List[torch.Tensor], noises: Optional[Sequence[torch.Tensor]] = None,
                out_range: Optional[Sequence[int]] = None) -> torch.Tensor:
@@ -245,6 +296,8 @@ class SNAC:
         T_out = T * math.prod(self.decoder_rates)
         t0, t1 = (0, T_out) if out_range is None else (int(out_range[0]), int(out_range[1]))
         blocks, (in_lo, in_hi) = self._stage_ranges(T, (t0, t1))
+        if self.channels_last:
+            return self._decode_channels_last(c, B, T, blocks, (in_lo, in_hi), (t0, t1), noises)
         f32 = dict(dtype=torch.float32, device=dev)
         z = torch.empty(B, C, T, **f32)
         call("vb_snac_from_codes", z.data_ptr(), c[0].data_ptr(), c[1].data_ptr(), c[2].data_ptr(),
@@ -259,16 +312,7 @@ class SNAC:
         self._pwconv("in_pw_w", y, x, w["in_pw_b"], None, None, w["b0.alpha"], 0, B, C, ch, T, in_lo, in_hi, st)
         x = y
         nb = len(self.decoder_rates)
-        if noises is None:
-            shapes = self.noise_shapes(B, T)
-            if self.noise_source is not None:
-                noises = self.noise_source(shapes)
-            else:
-                # one launch for the four NoiseBlock inputs (the reference draws torch.randn per block, snac.py:208);
-                # the device-side offset advances per call, so a captured vocoder graph draws fresh noise every replay
-                sizes = [math.prod(s) for s in shapes]
-                flat = ops.randn(torch.empty(sum(sizes), **f32), rng_state=self.ensure_noise_state())
-                noises = [t.view(s) for t, s in zip(torch.split(flat, sizes), shapes)]
+        noises = self._noises(noises, B, T)
         for bi, s in enumerate(self.decoder_rates):
             (c_lo, c_hi), units = blocks[bi]
             cin, cout = ch, ch // 2

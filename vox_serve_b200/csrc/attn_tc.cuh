@@ -1,0 +1,328 @@
+// The tcgen05 attention core of prompt rows, of prefill_attn_tc.cu (paged cache of the speech LMs): one accumulator row of 128 per softmax thread, scores and probabilities in TMEM, K and V
+// tiles of 64 keys through two-stage rings.  A kernel brings an object `rows` that says what its thread's row sees:
+//   n_tiles, tile(it)        the key tiles to walk, in order (tile i holds keys 64 i ..)
+//   scale_log2               what a score is multiplied by, times log2(e)
+//   full(tok0), visible(kj)  whether all 64 keys from tok0 / key kj are visible to this thread's row
+//   q_row()                  this thread's query row, or nullptr (a padding row: zeros)
+//   finish(m_ref, l)         factor for the accumulated row, given the exponents' reference and the denominator against it
+//   store(c0, o, f)          32 output values from column c0, times the factor
+// See prefill_attn_tc.cu for the schedule and what bounds it.
+#pragma once
+#include "common.cuh"
+#include <cudaTypedefs.h>
+
+namespace vb {
+
+__device__ __forceinline__ void ptc_cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void ptc_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void ptc_cp_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ float ptc_ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+constexpr int PTC_THREADS = 224;       // 4 softmax warps, 1 MMA warp, 2 loader warps
+constexpr int PTC_KT = 64;             // tokens per K / V tile
+constexpr int PTC_STAGES = 2;          // K and V tiles in flight, each with barriers of their own
+constexpr float PTC_RESCALE = 8.f;     // growth of a row's maximum (base 2) that moves the exponents' reference
+
+template <int D>
+struct PtcLayout {
+  static constexpr int TILE = PTC_KT * D * 2;               // [D / 64][64 tokens][64 dims] bf16
+  static constexpr int Q = 0;                               // [D / 64][128][64]
+  static constexpr int K = Q + 128 * D * 2;
+  static constexpr int V = K + PTC_STAGES * TILE;
+  static constexpr int BAR = V + PTC_STAGES * TILE;
+  static constexpr int TOTAL = BAR + 256 + 1024;            // PtcShared, alignment slack
+};
+
+// B operand stored [k][n] with the n's contiguous (128-byte swizzled rows of 64 n, 8-row groups of k 1024 bytes apart, blocks of
+// 64 n `block_bytes` apart)
+__device__ __forceinline__ uint64_t umma_desc_sw128_mnmajor(uint32_t smem_addr, uint32_t block_bytes) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((smem_addr & 0x3ffffu) >> 4);
+  d |= static_cast<uint64_t>(block_bytes >> 4) << 16;      // LBO
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;             // SBO
+  d |= static_cast<uint64_t>(1) << 46;
+  d |= static_cast<uint64_t>(2) << 61;
+  return d;
+}
+__device__ __forceinline__ void ptc_tma_5d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2, int c3, int c4) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+      : "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem]; A: two bf16 per 32-bit column
+__device__ __forceinline__ void umma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void ptc_tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]),
+        "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]),
+        "r"(v[30]), "r"(v[31])
+      : "memory");
+}
+__device__ __forceinline__ void ptc_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// barriers and scalars behind the operand tiles
+struct PtcShared {
+  uint64_t q_full, k_full[PTC_STAGES], k_empty[PTC_STAGES], v_full[PTC_STAGES], v_empty[PTC_STAGES];
+  uint64_t s_full[2];       // scores complete
+  uint64_t p_full[2];       // probabilities written, O ready to be added to
+  uint64_t o_done;          // P V of a tile complete
+  uint64_t o_last;          // ... of the last tile
+  uint64_t v_tail;          // the last V tile has landed (its rows past the last key are cleared next)
+  uint32_t tmem;
+  int tile[3];
+  int warp_tot[PTC_THREADS / 32];
+};
+
+__device__ __forceinline__ void ptc_init(PtcShared* sh, int loader_arrivals) {
+  mbar_init(&sh->q_full, 128);
+  for (int i = 0; i < PTC_STAGES; ++i) {
+    mbar_init(&sh->k_full[i], loader_arrivals);
+    mbar_init(&sh->k_empty[i], 1);
+    mbar_init(&sh->v_full[i], loader_arrivals);
+    mbar_init(&sh->v_empty[i], 1);
+  }
+  for (int i = 0; i < 2; ++i) {
+    mbar_init(&sh->s_full[i], 1);
+    mbar_init(&sh->p_full[i], 128);
+  }
+  mbar_init(&sh->o_done, 1);
+  mbar_init(&sh->o_last, 1);
+  mbar_init(&sh->v_tail, 1);
+  fence_barrier_init();
+  sh->tile[0] = -1;
+}
+
+// ================= warps 0..3: softmax =================
+template <int D, class Rows>
+__device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const Rows& rows, BoundedWait& bw) {
+  using L = PtcLayout<D>;
+  constexpr int KBD = D / 64, CPR = D * 2 / 16;
+  const int tid = threadIdx.x, warp = tid >> 5, n_tiles = rows.n_tiles;
+  {
+    const __nv_bfloat16* src = rows.q_row();
+    __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem + L::Q);
+#pragma unroll
+    for (int c = 0; c < CPR; ++c) {
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (src) v = *reinterpret_cast<const uint4*>(src + c * 8);
+      *reinterpret_cast<uint4*>(sQ + xt_index(tid, c * 8, 128, KBD)) = v;
+    }
+    fence_proxy_async();
+    mbar_arrive(&sh->q_full);
+  }
+  const uint32_t t_lane = sh->tmem + (static_cast<uint32_t>(warp * 32) << 16);   // this warp's TMEM lane quarter
+  const float scale = rows.scale_log2 > 0.f ? rows.scale_log2 : 1.f;
+  float m_ref = -INFINITY, l_run = 0.f;            // the exponents' reference and the denominator against it
+  for (int j = 0; j < n_tiles && !bw.dead; ++j) {
+    const uint32_t sc = t_lane + (j & 1) * 64;
+    bw.wait(&sh->s_full[j & 1], (j >> 1) & 1);
+    if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+    tc_fence_after();
+    uint32_t v[64];
+    {
+      uint32_t a[32], c[32];
+      tmem_ld_32x32(sc, a);
+      tmem_ld_32x32(sc + 32, c);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 32; ++i) { v[i] = a[i]; v[32 + i] = c[i]; }
+    }
+    const int tok0 = rows.tile(j) * PTC_KT;
+    if (!(rows.scale_log2 > 0.f)) {                            // (a scale that is not positive goes in before the maximum)
+#pragma unroll
+      for (int i = 0; i < 64; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * rows.scale_log2);
+    }
+    if (!__all_sync(0xffffffffu, rows.full(tok0))) {           // some row of the warp does not see all of the tile
+#pragma unroll
+      for (int i = 0; i < 64; ++i)
+        if (!rows.visible(tok0 + i)) v[i] = 0xff800000u;       // -inf
+    }
+    float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < 64; i += 4) {
+      m0 = fmaxf(m0, __uint_as_float(v[i]));
+      m1 = fmaxf(m1, __uint_as_float(v[i + 1]));
+      m2 = fmaxf(m2, __uint_as_float(v[i + 2]));
+      m3 = fmaxf(m3, __uint_as_float(v[i + 3]));
+    }
+    const float mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) * scale;
+    const bool move = mx > m_ref + PTC_RESCALE || (m_ref == -INFINITY && mx > -INFINITY);
+    if (__any_sync(0xffffffffu, move)) {
+      const float alpha = move ? ptc_ex2(m_ref - mx) : 1.f;                  // ex2(-inf) = 0
+      if (move) m_ref = mx;
+      l_run *= alpha;
+      if (j > 0) {
+        bw.wait(&sh->o_done, (j - 1) & 1);                                   // tile j - 1 has been added
+        if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+        tc_fence_after();
+#pragma unroll 1
+        for (int c0 = 0; c0 < D; c0 += 32) {
+          uint32_t o[32];
+          tmem_ld_32x32(t_lane + 128 + c0, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          ptc_tmem_st32(t_lane + 128 + c0, o);
+        }
+      }
+    }
+    const float u = m_ref == -INFINITY ? 0.f : m_ref;          // every key masked so far
+    float l0 = 0.f, l1 = 0.f;
+    uint32_t pk[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      pk[i] = pack_bf16(ptc_ex2(fmaf(__uint_as_float(v[2 * i]), scale, -u)), ptc_ex2(fmaf(__uint_as_float(v[2 * i + 1]), scale, -u)));
+      l0 += bf16_lo(pk[i]);                                    // denominator from the rounded probabilities
+      l1 += bf16_hi(pk[i]);
+    }
+    l_run += l0 + l1;
+    ptc_tmem_st32(sc, pk);
+    ptc_tmem_st_wait();
+    tc_fence_before();
+    mbar_arrive(&sh->p_full[j & 1]);
+  }
+  // ---- normalise and store this thread's row ----
+  if (n_tiles > 0 && !bw.dead) {
+    bw.wait(&sh->o_last, 0);
+    if (!__all_sync(0xffffffffu, !bw.dead)) bw.dead = true;
+  }
+  if (bw.dead) return;
+  tc_fence_after();
+  const float f = rows.finish(m_ref, l_run);
+#pragma unroll 1
+  for (int c0 = 0; c0 < D; c0 += 32) {
+    uint32_t o[32];
+    if (n_tiles > 0) {
+      tmem_ld_32x32(t_lane + 128 + c0, o);
+      tmem_ld_wait();
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) o[i] = 0u;
+    }
+    rows.store(c0, o, f);
+  }
+}
+
+// ================= warp 4, one lane: MMA issuer =================
+template <int D>
+__device__ __forceinline__ void ptc_issue(uint8_t* smem, PtcShared* sh, int n_tiles, BoundedWait& bw) {
+  using L = PtcLayout<D>;
+  constexpr int KBD = D / 64;
+  const uint32_t tmem = sh->tmem;
+  const uint32_t idesc_s = umma_idesc(128, PTC_KT, 1u), idesc_o = umma_idesc(128, D, 1u) | (1u << 16);   // (B of P V: MN-major)
+  const uint64_t q_desc = umma_desc_sw128_kmajor(smem_u32(smem + L::Q));
+  auto scores = [&](int j) {
+    bw.wait(&sh->k_full[j & 1], (j >> 1) & 1);
+    if (bw.dead) return;
+    tc_fence_after();
+    const uint64_t k_desc = umma_desc_sw128_kmajor(smem_u32(smem + L::K + (j & 1) * L::TILE));
+#pragma unroll
+    for (int kb = 0; kb < KBD; ++kb)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        umma_bf16(tmem + (j & 1) * 64, q_desc + kb * (128 * 128 >> 4) + 2 * k, k_desc + kb * (PTC_KT * 128 >> 4) + 2 * k, idesc_s,
+                  (kb > 0 || k > 0) ? 1u : 0u);
+    umma_commit(&sh->k_empty[j & 1]);
+    umma_commit(&sh->s_full[j & 1]);
+  };
+  if (n_tiles > 0) {
+    bw.wait(&sh->q_full, 0);
+    if (!bw.dead) scores(0);
+  }
+  for (int j = 0; j < n_tiles && !bw.dead; ++j) {
+    if (j + 1 < n_tiles) {
+      // the other score buffer holds the probabilities of tile j - 1 until they have been multiplied
+      if (j > 0) bw.wait(&sh->o_done, (j - 1) & 1);
+      if (!bw.dead) scores(j + 1);
+    }
+    bw.wait(&sh->p_full[j & 1], (j >> 1) & 1);
+    bw.wait(&sh->v_full[j & 1], (j >> 1) & 1);
+    if (bw.dead) break;
+    tc_fence_after();
+    const uint64_t v_desc = umma_desc_sw128_mnmajor(smem_u32(smem + L::V + (j & 1) * L::TILE), PTC_KT * 128);
+#pragma unroll
+    for (int k = 0; k < PTC_KT / 16; ++k)          // 16 tokens: 8 columns of probabilities, two 8-row groups of V
+      umma_bf16_ta(tmem + 128, tmem + (j & 1) * 64 + 8 * k, v_desc + k * (2048 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+    umma_commit(&sh->v_empty[j & 1]);
+    umma_commit(&sh->o_done);
+    if (j + 1 == n_tiles) umma_commit(&sh->o_last);
+  }
+}
+
+// ================= warp 5, one lane: boxes of `bt` keys x 64 dims of one head; fetch(tok, is_v, box destination, dim, barrier) =================
+template <int D, class Rows, class Fetch>
+__device__ __forceinline__ void ptc_load(uint8_t* smem, PtcShared* sh, const Rows& rows, int kmax, int bt, BoundedWait& bw, Fetch fetch_box) {
+  using L = PtcLayout<D>;
+  constexpr int KBD = D / 64;
+  const int n_tiles = rows.n_tiles, boxes = PTC_KT / bt;
+  auto fetch = [&](int j, int is_v, uint64_t* bar) {
+    const uint32_t dst = smem_u32(smem + (is_v ? L::V : L::K) + (j & 1) * L::TILE), mb = smem_u32(bar);
+    const int tok0 = rows.tile(j) * PTC_KT;
+    mbar_arrive_expect_tx(bar, min(boxes, (kmax - tok0 + bt - 1) / bt) * bt * D * 2);
+    for (int i = 0; i < boxes; ++i) {
+      const int tok = tok0 + i * bt;
+      if (tok >= kmax) break;                     // (pages past the last key are not the request's)
+#pragma unroll
+      for (int kb = 0; kb < KBD; ++kb) fetch_box(tok, is_v, dst + kb * (PTC_KT * 128) + i * bt * 128, kb * 64, mb);
+    }
+  };
+  for (int j = 0; j < n_tiles; ++j) {
+    bw.wait(&sh->k_empty[j & 1], ((j >> 1) & 1) ^ 1);
+    if (bw.dead) break;
+    fetch(j, 0, &sh->k_full[j & 1]);
+    bw.wait(&sh->v_empty[j & 1], ((j >> 1) & 1) ^ 1);
+    if (bw.dead) break;
+    fetch(j, 1, j + 1 < n_tiles ? &sh->v_full[j & 1] : &sh->v_tail);
+  }
+  if (bw.dead) {                                  // let the copies in flight land before the block may leave
+    const unsigned long long t0 = gtimer();
+    while (gtimer() - t0 < 2000000ull) __nanosleep(1000);
+  }
+}
+
+// ================= warp 6: rows of the last V tile past the last key =================
+// They are multiplied by probability 0: whatever the cache holds there, they must be finite.  (The last tile of the walk is the one
+// that holds key kmax - 1; tiles before it hold written keys only.)
+template <int D>
+__device__ __forceinline__ void ptc_clear_tail(uint8_t* smem, PtcShared* sh, int n_tiles, int kmax, BoundedWait& bw) {
+  using L = PtcLayout<D>;
+  constexpr int KBD = D / 64;
+  const int lane = threadIdx.x & 31, j = n_tiles - 1;
+  bw.wait(&sh->v_tail, 0);
+  if (!__all_sync(0xffffffffu, !bw.dead)) return;
+  uint8_t* tile = smem + L::V + (j & 1) * L::TILE;
+  const int r0 = kmax - (kmax - 1) / PTC_KT * PTC_KT, chunks = (PTC_KT - r0) * 8;
+  for (int i = lane; i < KBD * chunks; i += 32) {
+    const int kb = i / chunks, c = i - kb * chunks;
+    *reinterpret_cast<uint4*>(tile + kb * (PTC_KT * 128) + r0 * 128 + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  fence_proxy_async();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(&sh->v_full[j & 1]);
+}
+
+inline int ptc_box_tokens(int page_size) { return page_size % 64 == 0 ? 64 : (page_size % 32 == 0 ? 32 : (page_size % 16 == 0 ? 16 : 8)); }
+PFN_cuTensorMapEncodeTiled_v12000 encode_fn();      // api.cu
+
+}  // namespace vb

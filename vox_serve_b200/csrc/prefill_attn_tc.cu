@@ -1,24 +1,31 @@
 // Tiled paged prefill attention on the 5th-generation tensor cores (tcgen05 + TMEM): the FlashAttention schedule of
-// prefill_attn.cu with both contractions issued as tcgen05.mma from shared-memory operand tiles and their accumulators
-// in tensor memory.  Same inputs, same result contract (FlashInferPrefillWrapper.run, flashinfer_utils.py:68-80, 132).
+// prefill_attn.cu with both contractions issued as tcgen05.mma and their accumulators in tensor memory.  Same inputs, same
+// result contract (FlashInferPrefillWrapper.run, flashinfer_utils.py:68-80, 132).
 //
 //  * a CTA owns (Q tile, kv head).  The Q tile is M = 128 accumulator rows = TQ = 128 / G consecutive prompt rows of ONE
 //    request x the G grouped query heads of the kv head (row r = token r / G, head r % G): the GQA group rides in the MMA's
 //    M dimension, so a K/V tile is fetched once for all of them;
-//  * operand tiles are the 128-byte-swizzled K-major images the projection kernel uses (xt_index): Q [128 rows][D],
-//    K [128 tokens][D] (B operand of S = Q K^T), P [128 rows][128 tokens] bf16 (A operand of O = P V) and V TRANSPOSED
-//    [D dims][128 tokens] (B operand, K-major = tokens contiguous).  K arrives with cp.async straight into its swizzled
-//    place; V arrives row-major in a staging buffer (cp.async) and is transposed shared -> shared;
-//  * S (128 x 128 fp32) and the per-tile product P V (128 x D fp32) live in TMEM (256 columns); thread r of the CTA's 128
-//    threads owns accumulator row r = TMEM lane r: it reads its S row with tcgen05.ld, keeps the online-softmax state
-//    and the running output row in registers (no shuffles: a row is one thread), writes its P row as the next MMA's
-//    operand; exp2 via ex2.approx, P rounded to bf16, denominator from the rounded P (as the other attention kernels);
-//  * one elected thread issues the MMAs; completion comes back through mbarriers (tcgen05.commit); the K tile of the next
-//    step is requested as soon as S is complete and its V rows as soon as the transpose has read the staging buffer, so
-//    the loads run under the softmax and the second MMA.
+//  * warps 0..3 are the softmax: thread r owns accumulator row r = TMEM lane r.  It reads its 64 scores at once, keeps the
+//    running maximum and denominator in registers (no shuffles: a row is one thread) and writes its probabilities (bf16) over
+//    the scores in TMEM, where they are the A operand of O += P V;
+//  * O stays in TMEM for the whole sequence.  The maximum that the exponents are taken against is only moved when a row's
+//    maximum has grown by more than 8 (base 2), and only then is O rescaled: probabilities stay below 2^8, in bf16 and fp32 as
+//    exact as below 1, and the final division uses the same denominator;
+//  * warp 4 issues the MMAs: the scores of tile j + 1 are multiplied while the softmax works on tile j (two score buffers);
+//  * warps 5 and 6 bring K and V tiles as boxes of a tensor map over the paged cache (pages of a multiple of 8 tokens; cp.async
+//    per token row otherwise), the 128-byte-swizzled images that the MMAs read.  V is
+//    the B operand of P V as it lies in memory, [token][dim] (MN-major): nothing is transposed.
+// 98 KB of shared memory and 256 TMEM columns per CTA: two CTAs share an SM and fill each other's waits.
+// The form before this one had one warp group for everything -- loads, an element-wise transpose of every V tile, softmax, both
+// waits on the tensor cores -- one after the other (2.5 us per 64-token tile), and the kernel for smaller prompts ran on
+// mma.sync.  Measured per launch (mma.sync / this kernel, us): one 133-row prompt 12.0 / 9.2, eight of them 29 / 13, four portions
+// of 997 rows on up to 1063 cached tokens 92 / 35, three prompts of 1024 rows 46 / 19, four of 600 rows with 64-wide heads 75 / 33.
+// What bounds it: the serial chain of a tile (scores -> maximum -> exponentials -> P V, about 1.3 us), and where few tiles see
+// a long context the longest of them.
+// Every wait is bounded (BoundedWait): a block whose wait runs out notes it, stops issuing and leaves.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 1
-#include "common.cuh"
+#include "attn_tc.cuh"
 
 namespace vb {
 
@@ -33,78 +40,59 @@ struct PrefillTcParams {
   int slab_base;
   int n_req, n_rows, n_q, n_kv, G, TQ, page_size;
   int out_xt_tile;
+  int box_tokens;
   float scale_log2;
 };
 
-constexpr int PTC_THREADS = 128;
-
-__device__ __forceinline__ void ptc_cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void ptc_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void ptc_cp_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ float ptc_ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// KT = tokens per K/V tile: 128 at head_dim 64, 64 at head_dim 128 -- either way a CTA stays below half an SM's shared
-// memory (98 KB) and half its tensor memory (256 columns), so TWO CTAs share an SM and one's loads / softmax run under
-// the other's MMAs (the phases inside a CTA are serial).
-template <int D, int KT>
-struct PtcLayout {
-  static constexpr int Q = 0;                               // [D/64][128][64] bf16
-  static constexpr int K = Q + 128 * D * 2;                 // [D/64][KT][64]
-  static constexpr int VT = K + KT * D * 2;                 // [KT/64][D][64]
-  static constexpr int P = VT + KT * D * 2;                 // [KT/64][128][64]
-  static constexpr int VRAW = P + 128 * KT * 2;             // [KT][D * 2 + 16 bytes]
-  static constexpr int VRS = D * 2 + 16;
-  static constexpr int BAR = VRAW + KT * VRS;               // bar_s, bar_o, tmem slot
-  static constexpr int TOTAL = BAR + 64 + 1024;             // + alignment slack
+// what this thread's row sees: the first kl keys of its request
+struct PagedRows {
+  const PrefillTcParams& p;
+  int n_tiles, kl, row, head, D;
+  bool ok;
+  float scale_log2;
+  __device__ __forceinline__ int tile(int it) const { return it; }
+  __device__ __forceinline__ bool full(int tok0) const { return tok0 + PTC_KT <= kl; }
+  __device__ __forceinline__ bool visible(int kj) const { return kj < kl; }
+  __device__ __forceinline__ const __nv_bfloat16* q_row() const {
+    return ok ? p.q + (static_cast<size_t>(row) * p.n_q + head) * D : nullptr;
+  }
+  __device__ __forceinline__ float finish(float, float l) const { return l > 0.f ? 1.f / l : 0.f; }
+  __device__ __forceinline__ void store(int c0, const uint32_t (&o)[32], float f) const {
+    if (!ok) return;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = pack_bf16(__uint_as_float(o[c * 8 + 2 * i]) * f, __uint_as_float(o[c * 8 + 2 * i + 1]) * f);
+      const int e = head * D + c0 + c * 8;
+      const size_t at = p.out_xt_tile ? xt_index(row, e, p.out_xt_tile, (p.n_q * D + 63) >> 6) : static_cast<size_t>(row) * p.n_q * D + e;
+      *reinterpret_cast<uint4*>(p.out + at) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
 };
 
-template <int D, int KT>
-__global__ void __launch_bounds__(PTC_THREADS, 1) paged_prefill_attn_tc_kernel(const PrefillTcParams p) {
-  using L = PtcLayout<D, KT>;
-  constexpr int PTC_KT = KT;
-  constexpr int KBD = D / 64;          // 64-element k-blocks of the head dim
-  constexpr int KBT = PTC_KT / 64;     // ... of a token tile
+template <int D, bool TMA>
+__global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(const PrefillTcParams p,
+                                                                               const __grid_constant__ CUtensorMap kv_map) {
+  using L = PtcLayout<D>;
   constexpr int CPR = D * 2 / 16;      // 16-byte chunks per K / V row
-  constexpr int TPT = PTC_THREADS / PTC_KT;      // threads that share one token's K / V row (1 or 2)
-  constexpr int CPT = CPR / TPT;                 // 16-byte chunks of the row per thread
   extern __shared__ uint8_t ptc_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ptc_smem_raw) + 1023) & ~uintptr_t(1023));
-  __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem + L::Q);
-  __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem + L::K);
-  __nv_bfloat16* sVT = reinterpret_cast<__nv_bfloat16*>(smem + L::VT);
-  __nv_bfloat16* sP = reinterpret_cast<__nv_bfloat16*>(smem + L::P);
-  uint8_t* sVraw = smem + L::VRAW;
-  uint64_t* bar_s = reinterpret_cast<uint64_t*>(smem + L::BAR);
-  uint64_t* bar_o = bar_s + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_s + 2);
-  __shared__ int s_warp[PTC_THREADS / 32];
-  __shared__ int s_tile[3];
-
+  PtcShared* sh = reinterpret_cast<PtcShared*>(smem + L::BAR);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  BoundedWait bw;
   if (tid == 0) {
-    mbar_init(bar_s, 1);
-    mbar_init(bar_o, 1);
-    fence_barrier_init();
-    s_tile[0] = -1;
+    ptc_init(sh, TMA ? 1 : 64);
+    if (TMA) prefetch_tmap(&kv_map);
   }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, 256);
+  if (warp == 4) {
+    tmem_alloc(&sh->tmem, 256);                   // scores at 0 and 64, O at 128
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
+  const uint32_t tmem_base = sh->tmem;
   pdl_sync();
 
   // rows beyond the last request (CUDA-graph padding) produce zeros
@@ -119,8 +107,9 @@ __global__ void __launch_bounds__(PTC_THREADS, 1) paged_prefill_attn_tc_kernel(c
       }
   }
 
-  // ---- which (request, rows) is tile blockIdx.x?  prefix sum of ceil(n_new / TQ) over the requests ----
-  const int TQ = p.TQ;
+  // ---- which (request, rows) is this block's tile?  prefix sum of ceil(n_new / TQ) over the requests.  Blocks take the tiles
+  // from the last one back: late rows see the most keys, and the longest tiles should not start last ----
+  const int TQ = p.TQ, b = static_cast<int>(gridDim.x - 1 - blockIdx.x);
   int base = 0;
   for (int r0 = 0; r0 < p.n_req; r0 += PTC_THREADS) {
     __syncthreads();
@@ -137,240 +126,124 @@ __global__ void __launch_bounds__(PTC_THREADS, 1) paged_prefill_attn_tc_kernel(c
       const int n = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += n;
     }
-    if (lane == 31) s_warp[warp] = incl;
+    if (lane == 31) sh->warp_tot[warp] = incl;
     __syncthreads();
     int woff = 0, tot = 0;
     for (int w = 0; w < PTC_THREADS / 32; ++w) {
-      const int v = s_warp[w];
+      const int v = sh->warp_tot[w];
       if (w < warp) woff += v;
       tot += v;
     }
     const int excl = base + woff + incl - nt;
-    const int b = static_cast<int>(blockIdx.x);
     if (nt > 0 && b >= excl && b < excl + nt) {
-      s_tile[0] = r;
-      s_tile[1] = row0 + (b - excl) * TQ;
-      s_tile[2] = min(TQ, nnew - (b - excl) * TQ);
+      sh->tile[0] = r;
+      sh->tile[1] = row0 + (b - excl) * TQ;
+      sh->tile[2] = min(TQ, nnew - (b - excl) * TQ);
     }
     base += tot;
   }
   __syncthreads();
-  const int req = s_tile[0];
+  const int req = sh->tile[0];
   if (req >= 0) {
-    const int row0 = s_tile[1], nrows = s_tile[2];
-    const int hk = blockIdx.y;
-    const int pbase = p.kv_indptr[req];
-    // this thread's accumulator row: prompt row t of the tile, grouped head g
-    const int t = tid / p.G, g = tid - t * p.G;
-    const bool row_ok = t < nrows;
-    const int kl = row_ok ? p.row_kvlen[row0 + t] : 0;
+    const int row0 = sh->tile[1], nrows = sh->tile[2], hk = blockIdx.y;
     // the tile's largest bound (the bounds do not decrease inside a request: the last row's)
     const int kmax = p.row_kvlen[row0 + nrows - 1];
     const int n_tiles = (kmax + PTC_KT - 1) / PTC_KT;
-    const size_t page_elems = static_cast<size_t>(p.page_size) * p.n_kv * D;
-
-    // ---- Q tile: row r = tid -> swizzled K-major image ----
-    {
-      const __nv_bfloat16* src = p.q + (static_cast<size_t>(row0 + (row_ok ? t : 0)) * p.n_q + hk * p.G + g) * D;
-#pragma unroll
-      for (int c = 0; c < CPR; ++c) {
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (row_ok) v = *reinterpret_cast<const uint4*>(src + c * 8);
-        *reinterpret_cast<uint4*>(sQ + xt_index(tid, c * 8, 128, KBD)) = v;
+    const int t = tid / p.G;                      // (softmax) this thread's accumulator row: prompt row t of the tile, head tid % G
+    const bool ok = warp < 4 && t < nrows;
+    const PagedRows rows{p, n_tiles, ok ? p.row_kvlen[row0 + t] : 0, row0 + t, hk * p.G + tid - t * p.G, D, ok, p.scale_log2};
+    if (warp < 4) {
+      ptc_softmax<D>(smem, sh, rows, bw);
+    } else if (warp == 4) {
+      if (lane == 0) ptc_issue<D>(smem, sh, n_tiles, bw);
+      __syncwarp();
+    } else if (TMA) {
+      if (warp == 5 && lane == 0) {
+        const int pbase = p.kv_indptr[req];
+        ptc_load<D>(smem, sh, rows, kmax, p.box_tokens, bw, [&](int tok, int is_v, uint32_t dst, int dim, uint32_t bar) {
+          const int page = __ldg(&p.kv_indices[pbase + tok / p.page_size]);
+          ptc_tma_5d(dst, &kv_map, bar, dim, hk, tok % p.page_size, is_v, p.slab_base + page);
+        });
+      } else if (warp == 6 && n_tiles > 0) {
+        ptc_clear_tail<D>(smem, sh, n_tiles, kmax, bw);
       }
-    }
-    // ---- K / V loads: thread j fetches token tok0 + j of the CTA's kv head ----
-    auto token_src = [&](int tok) -> const __nv_bfloat16* {
-      const int page = __ldg(&p.kv_indices[pbase + tok / p.page_size]);
-      return p.kv + static_cast<size_t>(p.slab_base + page) * 2 * page_elems +
-             (static_cast<size_t>(tok % p.page_size) * p.n_kv + hk) * D;
-    };
-    const int ltok = tid / TPT, lc0 = (tid % TPT) * CPT;      // this thread's token of a tile and its first chunk
-    auto load_k = [&](int tile) {
-      const int tok = tile * PTC_KT + ltok;
-      if (tok < kmax) {
-        const __nv_bfloat16* src = token_src(tok);
+      __syncwarp();
+    } else {
+      // ================= loaders for pages that do not divide into 8-token groups: one token's K / V row per thread =================
+      const int ltok = tid - 160, pbase = p.kv_indptr[req];
+      const size_t page_elems = static_cast<size_t>(p.page_size) * p.n_kv * D;
+      auto fetch = [&](int j, int is_v) {
+        const int tok = j * PTC_KT + ltok;
+        const uint32_t dst = smem_u32(smem + (is_v ? L::V : L::K) + (j & 1) * L::TILE) + ltok * 128;
+        if (tok < kmax) {
+          const int page = __ldg(&p.kv_indices[pbase + tok / p.page_size]);
+          const __nv_bfloat16* src = p.kv + (static_cast<size_t>(p.slab_base + page) * 2 + is_v) * page_elems +
+                                     (static_cast<size_t>(tok % p.page_size) * p.n_kv + hk) * D;
 #pragma unroll
-        for (int c = lc0; c < lc0 + CPT; ++c) ptc_cp_async16(smem_u32(sK + xt_index(ltok, c * 8, PTC_KT, KBD)), src + c * 8);
-      } else {
+          for (int ch = 0; ch < CPR; ++ch) {
+            ptc_cp_async16(dst + (ch >> 3) * (PTC_KT * 128) + (((ch & 7) ^ (ltok & 7)) << 4), src + ch * 8);
+          }
+        } else {                       // rows past the last key are multiplied by probability 0: they must be finite
 #pragma unroll
-        for (int c = lc0; c < lc0 + CPT; ++c)
-          *reinterpret_cast<uint4*>(sK + xt_index(ltok, c * 8, PTC_KT, KBD)) = make_uint4(0u, 0u, 0u, 0u);
-      }
-      ptc_cp_commit();
-    };
-    auto load_v = [&](int tile) {
-      const int tok = tile * PTC_KT + ltok;
-      uint8_t* dst = sVraw + ltok * L::VRS;
-      if (tok < kmax) {
-        const __nv_bfloat16* src = token_src(tok) + page_elems;
-#pragma unroll
-        for (int c = lc0; c < lc0 + CPT; ++c) ptc_cp_async16(smem_u32(dst + c * 16), src + c * 8);
-      } else {
-#pragma unroll
-        for (int c = lc0; c < lc0 + CPT; ++c) *reinterpret_cast<uint4*>(dst + c * 16) = make_uint4(0u, 0u, 0u, 0u);
-      }
-      ptc_cp_commit();
-    };
-
-    float O[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) O[i] = 0.f;
-    float m_run = -INFINITY, l_run = 0.f;
-    const uint32_t idesc_s = umma_idesc(128, PTC_KT, 1u);
-    const uint32_t idesc_o = umma_idesc(128, D, 1u);
-    const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);   // this warp's TMEM lane quarter
-
-    if (n_tiles > 0) {
-      load_k(0);
-      load_v(0);
-    }
-    uint32_t ph = 0;
-    for (int tile = 0; tile < n_tiles; ++tile) {
-      const int tok0 = tile * PTC_KT;
-      // ---- K (and, for tile 0, Q) in place -> S = Q K^T ----
-      // tile 0: groups were committed K then V -- the K group is enough here; later tiles: V (requested first) and K
-      if (tile == 0) ptc_cp_wait<1>(); else ptc_cp_wait<0>();
-      fence_proxy_async();
-      __syncthreads();
-      if (tid == 0) {
-        tc_fence_after();
-#pragma unroll
-        for (int kb = 0; kb < KBD; ++kb) {
-          const uint64_t a_desc = umma_desc_sw128_kmajor(smem_u32(sQ) + kb * (128 * 128));
-          const uint64_t b_desc = umma_desc_sw128_kmajor(smem_u32(sK) + kb * (PTC_KT * 128));
-#pragma unroll
-          for (int k = 0; k < 4; ++k) umma_bf16(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc_s, (kb > 0 || k > 0) ? 1u : 0u);
+          for (int ch = 0; ch < CPR; ++ch) {
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst + (ch >> 3) * (PTC_KT * 128) + (((ch & 7) ^ (ltok & 7)) << 4)),
+                         "r"(0) : "memory");
+          }
         }
-        umma_commit(bar_s);
+        ptc_cp_commit();
+      };
+      // K(j) and V(j) are requested one after the other; a tile is announced once a later group is in flight behind it
+      for (int j = 0; j < n_tiles && !bw.dead; ++j) {
+        bw.wait(&sh->k_empty[j & 1], ((j >> 1) & 1) ^ 1);
+        if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+        fetch(j, 0);
+        if (j > 0) {                   // V(j - 1)
+          ptc_cp_wait<1>();
+          fence_proxy_async();
+          mbar_arrive(&sh->v_full[(j - 1) & 1]);
+        }
+        bw.wait(&sh->v_empty[j & 1], ((j >> 1) & 1) ^ 1);
+        if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+        fetch(j, 1);
+        ptc_cp_wait<1>();              // K(j)
+        fence_proxy_async();
+        mbar_arrive(&sh->k_full[j & 1]);
       }
-      // ---- meanwhile: V rows -> transposed, swizzled operand tile ----
       ptc_cp_wait<0>();
-      __syncthreads();               // every thread's V row has landed in the staging buffer
-      {
-        // this thread's token of the tile: its (part of the) row, 8 dims at a time, scattered to rows d of the [D][KT] tile
-        const uint8_t* srow = sVraw + ltok * L::VRS;
-#pragma unroll 4
-        for (int c = lc0; c < lc0 + CPT; ++c) {
-          const uint4 v = *reinterpret_cast<const uint4*>(srow + c * 16);
-          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const uint16_t h = static_cast<uint16_t>((e & 1) ? (w[e >> 1] >> 16) : (w[e >> 1] & 0xffffu));
-            *reinterpret_cast<uint16_t*>(sVT + xt_index(c * 8 + e, ltok, D, KBT)) = h;
-          }
-        }
-      }
-      __syncthreads();               // the staging buffer has been read by everybody
-      if (tile + 1 < n_tiles) load_v(tile + 1);
-      // ---- S complete: this thread's row ----
-      mbar_wait(bar_s, ph);
-      tc_fence_after();
-      if (tile + 1 < n_tiles) load_k(tile + 1);      // the first MMA has read K: fetch the next tile under the softmax
-      float mx = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < PTC_KT / 16; ++c) {
-        uint32_t v[16];
-        tmem_ld_32x16(t_lane + c * 16, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (tok0 + c * 16 + i < kl) mx = fmaxf(mx, __uint_as_float(v[i]) * p.scale_log2);
-      }
-      const float m_new = fmaxf(m_run, mx);
-      const float u = (m_new == -INFINITY) ? 0.f : m_new;       // every key masked so far
-      const float alpha = ptc_ex2(m_run - u);                    // ex2(-inf) = 0
-      m_run = m_new;
-      float lsum = 0.f;
-#pragma unroll
-      for (int c = 0; c < PTC_KT / 16; ++c) {
-        uint32_t v[16];
-        tmem_ld_32x16(t_lane + c * 16, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i8 = 0; i8 < 2; ++i8) {
-          uint32_t pk[4];
-#pragma unroll
-          for (int i2 = 0; i2 < 4; ++i2) {
-            const int i = i8 * 8 + i2 * 2, j = tok0 + c * 16 + i;
-            const float p0 = (j < kl) ? round_bf16(ptc_ex2(__uint_as_float(v[i]) * p.scale_log2 - u)) : 0.f;
-            const float p1 = (j + 1 < kl) ? round_bf16(ptc_ex2(__uint_as_float(v[i + 1]) * p.scale_log2 - u)) : 0.f;
-            lsum += p0 + p1;
-            pk[i2] = pack_bf16(p0, p1);
-          }
-          *reinterpret_cast<uint4*>(sP + xt_index(tid, c * 16 + i8 * 8, 128, KBT)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        }
-      }
-      l_run = l_run * alpha + lsum;
-      // ---- O_tile = P V ----
-      fence_proxy_async();           // P and V^T were written with ordinary stores
-      tc_fence_before();
-      __syncthreads();
-      if (tid == 0) {
-        tc_fence_after();
-#pragma unroll
-        for (int kb = 0; kb < KBT; ++kb) {
-          const uint64_t a_desc = umma_desc_sw128_kmajor(smem_u32(sP) + kb * (128 * 128));
-          const uint64_t b_desc = umma_desc_sw128_kmajor(smem_u32(sVT) + kb * (D * 128));
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_bf16(tmem_base + 128, a_desc + 2 * k, b_desc + 2 * k, idesc_o, (kb > 0 || k > 0) ? 1u : 0u);
-        }
-        umma_commit(bar_o);
-      }
-      mbar_wait(bar_o, ph);
-      tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < D / 16; ++c) {
-        uint32_t v[16];
-        tmem_ld_32x16(t_lane + 128 + c * 16, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) O[c * 16 + i] = O[c * 16 + i] * alpha + __uint_as_float(v[i]);
-      }
-      tc_fence_before();             // TMEM reads done before the next tile's MMAs overwrite S / O_tile
-      ph ^= 1;
-    }
-
-    // ---- normalise and store this thread's row ----
-    if (row_ok) {
-      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-      const int hq = hk * p.G + g;
-#pragma unroll
-      for (int c = 0; c < D / 8; ++c) {
-        uint32_t pk[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) pk[i] = pack_bf16(O[c * 8 + 2 * i] * inv, O[c * 8 + 2 * i + 1] * inv);
-        const size_t o = p.out_xt_tile ? xt_index(row0 + t, hq * D + c * 8, p.out_xt_tile, (p.n_q * D + 63) >> 6)
-                                       : (static_cast<size_t>(row0 + t) * p.n_q + hq) * D + c * 8;
-        *reinterpret_cast<uint4*>(p.out + o) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+      if (n_tiles > 0 && !bw.dead) {
+        fence_proxy_async();
+        mbar_arrive(&sh->v_full[(n_tiles - 1) & 1]);
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 4) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 256);
   }
 }
 
-template <int D, int KT>
-static int launch_prefill_tc(const PrefillTcParams& p, dim3 grid, cudaStream_t stream) {
-  auto kern = paged_prefill_attn_tc_kernel<D, KT>;
-  // (a fixed size per instantiation -- safe under CUDA-graph replay -- and below the limit together with the few
-  // bytes of static shared memory)
-  constexpr int smem_bytes = PtcLayout<D, KT>::TOTAL;
+template <int D, bool TMA>
+static int launch_prefill_tc(const PrefillTcParams& p, const CUtensorMap& map, dim3 grid, cudaStream_t stream) {
+  auto kern = paged_prefill_attn_tc_kernel<D, TMA>;
+  // (a fixed size per instantiation -- safe under CUDA-graph replay)
+  constexpr int smem_bytes = PtcLayout<D>::TOTAL;
   VB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-  VB_LAUNCH_PDL(kern, grid, PTC_THREADS, smem_bytes, stream, p);
+  VB_LAUNCH_PDL(kern, grid, PTC_THREADS, smem_bytes, stream, p, map);
   return 0;
 }
-
 }  // namespace vb
 
 using namespace vb;
 
 extern "C" {
+
+int vb_prefill_attn_tc_timeouts(void) {
+  unsigned int n = 0;
+  if (cudaMemcpyFromSymbol(&n, g_wait_timeouts, sizeof(n)) != cudaSuccess) return -1;
+  return static_cast<int>(n);
+}
 
 int vb_prefill_attn_tc_tile_rows(int n_q, int n_kv) {
   if (n_kv < 1 || n_q < n_kv || n_q % n_kv != 0 || n_q / n_kv > 128) return -1;
@@ -403,7 +276,23 @@ int vb_paged_prefill_attn_tc(void* d_out, const void* d_q, const void* d_kv, int
   p.scale_log2 = sm_scale * 1.4426950408889634f;
   const dim3 grid((n_rows + p.TQ - 1) / p.TQ + n_req, n_kv, 1);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  return head_dim == 128 ? launch_prefill_tc<128, 64>(p, grid, st) : launch_prefill_tc<64, 128>(p, grid, st);
+  p.box_tokens = ptc_box_tokens(page_size);
+  CUtensorMap map = {};
+  if (page_size % 8 == 0) {
+    auto fn = encode_fn();
+    VB_CHECK_ARG(fn, "cuTensorMapEncodeTiled not available (no CUDA driver?)");
+    // (dim, head, token, K | V, page); how many pages there are is the caller's: every box starts at a page of the table
+    const cuuint64_t H = n_kv, P = page_size, Dd = head_dim;
+    cuuint64_t dims[5] = {Dd, H, P, 2, 1ull << 30};
+    cuuint64_t strides[4] = {Dd * 2, H * Dd * 2, P * H * Dd * 2, 2 * P * H * Dd * 2};
+    cuuint32_t box[5] = {64, 1, static_cast<cuuint32_t>(p.box_tokens), 1, 1}, estr[5] = {1, 1, 1, 1, 1};
+    const CUresult r = fn(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(d_kv), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    VB_CHECK_ARG(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(paged K/V) failed: CUresult %d", static_cast<int>(r));
+    return head_dim == 128 ? launch_prefill_tc<128, true>(p, map, grid, st) : launch_prefill_tc<64, true>(p, map, grid, st);
+  }
+  return head_dim == 128 ? launch_prefill_tc<128, false>(p, map, grid, st) : launch_prefill_tc<64, false>(p, map, grid, st);
 }
 
 }  // extern "C"

@@ -157,6 +157,7 @@ int vb_paged_prefill_attn(void* d_out, const void* d_q, const void* d_kv, int64_
  * tile = 128 / group prompt rows of one request), K/V tiles of 128 tokens (any page size).  Arguments as
  * vb_paged_prefill_attn. */
 int vb_prefill_attn_tc_timeouts(void);      /* as vb_gemm_wide_timeouts */
+int vb_window_attn_tc_timeouts(void);
 int vb_prefill_attn_tc_tile_rows(int n_q, int n_kv);
 int vb_paged_prefill_attn_tc(void* d_out, const void* d_q, const void* d_kv, int64_t slab_base,
                              const int32_t* d_qo_indptr, const int32_t* d_kv_indptr, const int32_t* d_kv_indices,

@@ -166,3 +166,57 @@ def test_channels_last_depthwise_and_last(B, T, C, dil, lo, hi, big):
     last = _cl.last_conv(xs, w, b[:1], 7, 3, lo, hi, tanh=False)
     ref = torch.nn.functional.conv1d(x.double().transpose(1, 2), w.double()[None], b[:1].double(), padding=3)[..., lo:hi]
     _close(last, ref, 5e-6)
+
+
+# prompt rows of window attention on tcgen05: head sizes, heads per key head (rows per tile), page sizes down to one 8-token group, row
+# tiles of one row and of 64, windows and chunks that start inside key tiles, kept tokens near and far, sinks, both gates, fp32 output
+@pytest.mark.parametrize("D,H,G,page,new,old,window,chunk,keep,sink,gate,share,f32", [
+    (128, 4, 1, 64, [1, 64, 65], [0, 0, 0], 0, 0, 0, False, None, 1, False), (64, 6, 2, 8, [130], [0], 0, 0, 0, True, "head", 1, False),
+    (128, 3, 3, 16, [70, 3], [200, 61], 50, 0, 0, False, "value", 1, True), (64, 16, 1, 32, [100], [300], 64, 0, 5, True, None, 1, False),
+    (128, 8, 2, 64, [129], [500], 130, 0, 70, True, "head", 1, False), (64, 4, 4, 64, [200], [10], 0, 96, 0, False, None, 2, False),
+    (128, 130, 10, 64, [33], [31], 0, 0, 0, False, None, 1, False), (64, 200, 2, 24, [5], [64], 3, 0, 2, False, None, 1, False)])
+def test_window_attention_prompt_rows(ops, D, H, G, page, new, old, window, chunk, keep, sink, gate, share, f32):
+    from vox_serve_b200 import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(H * D + page)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")                 # noqa: E731
+    n, T, Gv = [a + b for a, b in zip(new, old)], sum(new), G // share
+    pages = [(x + page - 1) // page for x in n]
+    ip = np.concatenate([[0], np.cumsum(pages)]).tolist()
+    idx = np.random.RandomState(T).permutation(ip[-1]).tolist()
+    # what no position of a request has written is not a number: nothing of it may reach a result
+    kc, vc = (torch.full((ip[-1], page, h, D), float("nan"), device="cuda").bfloat16() for h in (G, Gv))
+    q, snk = rnd(T, H, D).bfloat16(), rnd(H) if sink else None
+    gt = rnd(T, H if gate == "head" else H * D) if gate else None
+    ref, at, treq, trow, pos = [], 0, [], [], []
+    for b, L in enumerate(n):
+        k, v = rnd(L, G, D).bfloat16(), rnd(L, Gv, D).bfloat16()
+        tok = torch.arange(L, device="cuda")
+        pg = torch.tensor(idx[ip[b]:ip[b + 1]], device="cuda")[tok // page]
+        kc[pg, tok % page], vc[pg, tok % page] = k, v
+        i, j = torch.arange(old[b], L, device="cuda")[:, None], tok[None]
+        lo = torch.zeros_like(i) if not window else (i - window + 1).clamp(min=0)
+        lo = torch.maximum(lo, i - i % chunk) if chunk else lo
+        seen = (j <= i) & ((j >= lo) | (j < keep))
+        for h in range(H):
+            kg = h // (H // G)
+            s = (q[at:at + new[b], h].double() @ k[:, kg].double().T * D ** -0.5).masked_fill(~seen, -float("inf"))
+            if sink:
+                s = torch.cat((s, snk[h].double().expand(new[b], 1)), 1)
+            ref.append((torch.softmax(s, -1)[:, :L] @ v[:, kg // share].double(), at, h))
+        for r in range(0, new[b], 64):
+            treq.append(b)
+            trow.append(at + r)
+        pos += list(range(old[b], L))
+        at += new[b]
+    want = torch.empty(T, H, D, dtype=torch.float64, device="cuda")
+    for o, t0, h in ref:
+        want[t0:t0 + o.shape[0], h] = o
+    if gate:
+        want = want * torch.sigmoid(gt.double().view(T, H, -1))
+    out = torch.full((T, H * D), float("nan"), device="cuda", dtype=torch.float32 if f32 else torch.bfloat16)
+    ops.window_attn(q.view(T, H * D), kc, vc, out, gt, None, _i32(pos), _i32(ip), _i32(idx), T, H, G, D, D, window, D ** -0.5,
+                    tiles=(_i32([0] + np.cumsum(new).tolist()), _i32(treq), _i32(trow), len(treq)), chunk=chunk, v_share=share, sink=snk,
+                    keep_first=keep, head_gate=gate == "head")
+    _close(out.view(T, H, D), want, 2 ** -8)         # probabilities and the output rounded to bf16
+    assert _lib.load().vb_window_attn_tc_timeouts() == 0

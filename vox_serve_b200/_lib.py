@@ -45,6 +45,7 @@ SIGNATURES = {
     "vb_paged_prefill_attn": (c_int, [P, P, P, c_int64, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                                       c_int, P]),
     "vb_prefill_attn_tc_timeouts": (c_int, []),
+    "vb_window_attn_tc_timeouts": (c_int, []),
     "vb_prefill_attn_tc_tile_rows": (c_int, [c_int, c_int]),
     "vb_paged_prefill_attn_tc": (c_int, [P, P, P, c_int64, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                                          c_int, P]),
@@ -262,7 +263,7 @@ def check(rc: int, what: str = ""):
 
 # kernels (+ memset nodes) each entry point enqueues; everything not listed launches exactly one
 LAUNCHES = {"vb_set_pdl": 0, "vb_set_trace": 0, "vb_weight_tiles_bytes": 0, "vb_tensor_map_kv": 0,
-            "vb_tensor_map_2d_bf16": 0, "vb_gemm_wide_timeouts": 0, "vb_cl_timeouts": 0, "vb_prefill_attn_tc_timeouts": 0, "vb_cl_pack_bytes": 0, "vb_device_info": 0, "vb_sample": 1, "vb_update_repetition_cache": 1,
+            "vb_tensor_map_2d_bf16": 0, "vb_gemm_wide_timeouts": 0, "vb_cl_timeouts": 0, "vb_prefill_attn_tc_timeouts": 0, "vb_window_attn_tc_timeouts": 0, "vb_cl_pack_bytes": 0, "vb_device_info": 0, "vb_sample": 1, "vb_update_repetition_cache": 1,
             "vb_set_gemm_smem_kb": 0, "vb_window_attn_tile_rows": 0, "vb_decay_attn_tile_rows": 0, "vb_decay_attn_tiled": 3, "vb_window_attn": 2, "vb_mingru_tiled": 3, "vb_mingru_scratch_floats": 0,
             "vb_short_conv": 2, "vb_selective_scan_tiled": 3, "vb_selective_scan_piece_rows": 0,
             "vb_selective_scan_scratch_floats": 0, "vb_sigmoid_attn": 1, "vb_ssd_tiled": 3, "vb_ssd_tile_rows": 0,

@@ -1,4 +1,5 @@
-// The tcgen05 attention core of prompt rows, of prefill_attn_tc.cu (paged cache of the speech LMs): one accumulator row of 128 per softmax thread, scores and probabilities in TMEM, K and V
+// The tcgen05 attention core of prompt rows, shared by prefill_attn_tc.cu (paged cache of the speech LMs) and window_attn_tc.cu
+// (sliding windows of the text LMs): one accumulator row of 128 per softmax thread, scores and probabilities in TMEM, K and V
 // tiles of 64 keys through two-stage rings.  A kernel brings an object `rows` that says what its thread's row sees:
 //   n_tiles, tile(it)        the key tiles to walk, in order (tile i holds keys 64 i ..)
 //   scale_log2               what a score is multiplied by, times log2(e)

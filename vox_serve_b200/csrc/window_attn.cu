@@ -1051,6 +1051,14 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(WindowAttnParams p
   }
 }
 
+// window_attn_tc.cu
+bool window_attn_tc_takes(int H, int G, int dim, int vdim, int page_size, int k_ld, int v_ld, const void* q, const void* k, const void* v,
+                          const void* out);
+int window_attn_tc(void* out, const void* q, const void* k_cache, const void* v_cache, const float* gate, int ld_gate, const int32_t* pos,
+                   const int32_t* page_indptr, const int32_t* page_indices, const int32_t* qo_indptr, const int32_t* tile_req,
+                   const int32_t* tile_row0, int n_tiles, int H, int G, int dim, int page_size, int window, float scale, int chunk, int k_ld,
+                   int v_ld, int v_share, int out_f32, const float* sink, int keep_first, int head_gate, cudaStream_t stream);
+
 }  // namespace vb
 
 using namespace vb;
@@ -1274,6 +1282,11 @@ int vb_window_attn_tiled(void* d_out, const void* d_q, const void* d_k_cache, co
   WindowAttnParams p{d_q, d_k_cache, d_v_cache, d_out, d_gate, ld_gate, nullptr, d_pos, d_page_indptr, d_page_indices,
                      d_qo_indptr, d_tile_req, d_tile_row0, T, H, G, dim, vdim, page_size, window, chunk, k_ld, v_ld, v_share,
                      out_f32, scale, nullptr, 0, 1, nullptr, d_sink, max(keep_first, 0), head_gate};
+  // keys and values of one size (64 or 128) run on tcgen05 with a key head's query heads in one row tile (window_attn_tc.cu)
+  if (dtype == 0 && window_attn_tc_takes(H, G, dim, vdim, page_size, k_ld, v_ld, d_q, d_k_cache, d_v_cache, d_out))
+    return window_attn_tc(d_out, d_q, d_k_cache, d_v_cache, d_gate, ld_gate, d_pos, d_page_indptr, d_page_indices, d_qo_indptr, d_tile_req,
+                          d_tile_row0, n_tiles, H, G, dim, page_size, window, scale, chunk, k_ld, v_ld, v_share, out_f32, d_sink,
+                          max(keep_first, 0), head_gate, static_cast<cudaStream_t>(stream));
   dim3 grid(n_tiles, H);
   if (dtype == 0 && dim % 16 == 0 && vdim % 16 == 0 && dim <= 16 * F_KB && vdim <= 8 * F_NT && k_ld % 8 == 0 && v_ld % 8 == 0) {
     const size_t msmem = 2 * static_cast<size_t>(FN) * (dim + 8 + vdim + 8) * sizeof(__nv_bfloat16);      // two stages

@@ -225,7 +225,7 @@ __device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const 
   }
 }
 
-// ================= warp 4, one lane: MMA issuer =================
+// ================= warp 4: MMA issuer (the whole warp walks the loop, one elected lane issues: operands stay in uniform registers) =================
 template <int D>
 __device__ __forceinline__ void ptc_issue(uint8_t* smem, PtcShared* sh, int n_tiles, BoundedWait& bw) {
   using L = PtcLayout<D>;
@@ -233,41 +233,51 @@ __device__ __forceinline__ void ptc_issue(uint8_t* smem, PtcShared* sh, int n_ti
   const uint32_t tmem = sh->tmem;
   const uint32_t idesc_s = umma_idesc(128, PTC_KT, 1u), idesc_o = umma_idesc(128, D, 1u) | (1u << 16);   // (B of P V: MN-major)
   const uint64_t q_desc = umma_desc_sw128_kmajor(smem_u32(smem + L::Q));
+  auto alive = [&]() {
+    if (!__all_sync(0xffffffffu, !bw.dead)) bw.dead = true;
+    return !bw.dead;
+  };
   auto scores = [&](int j) {
     bw.wait(&sh->k_full[j & 1], (j >> 1) & 1);
-    if (bw.dead) return;
+    if (!alive()) return;
     tc_fence_after();
     const uint64_t k_desc = umma_desc_sw128_kmajor(smem_u32(smem + L::K + (j & 1) * L::TILE));
+    if (elect_one()) {
 #pragma unroll
-    for (int kb = 0; kb < KBD; ++kb)
+      for (int kb = 0; kb < KBD; ++kb)
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        umma_bf16(tmem + (j & 1) * 64, q_desc + kb * (128 * 128 >> 4) + 2 * k, k_desc + kb * (PTC_KT * 128 >> 4) + 2 * k, idesc_s,
-                  (kb > 0 || k > 0) ? 1u : 0u);
-    umma_commit(&sh->k_empty[j & 1]);
-    umma_commit(&sh->s_full[j & 1]);
+        for (int k = 0; k < 4; ++k)
+          umma_bf16(tmem + (j & 1) * 64, q_desc + kb * (128 * 128 >> 4) + 2 * k, k_desc + kb * (PTC_KT * 128 >> 4) + 2 * k, idesc_s,
+                    (kb > 0 || k > 0) ? 1u : 0u);
+      umma_commit(&sh->k_empty[j & 1]);
+      umma_commit(&sh->s_full[j & 1]);
+    }
+    __syncwarp();
   };
   if (n_tiles > 0) {
     bw.wait(&sh->q_full, 0);
-    if (!bw.dead) scores(0);
+    if (alive()) scores(0);
   }
   for (int j = 0; j < n_tiles && !bw.dead; ++j) {
     if (j + 1 < n_tiles) {
       // the other score buffer holds the probabilities of tile j - 1 until they have been multiplied
       if (j > 0) bw.wait(&sh->o_done, (j - 1) & 1);
-      if (!bw.dead) scores(j + 1);
+      if (alive()) scores(j + 1);
     }
     bw.wait(&sh->p_full[j & 1], (j >> 1) & 1);
     bw.wait(&sh->v_full[j & 1], (j >> 1) & 1);
-    if (bw.dead) break;
+    if (!alive()) break;
     tc_fence_after();
     const uint64_t v_desc = umma_desc_sw128_mnmajor(smem_u32(smem + L::V + (j & 1) * L::TILE), PTC_KT * 128);
+    if (elect_one()) {
 #pragma unroll
-    for (int k = 0; k < PTC_KT / 16; ++k)          // 16 tokens: 8 columns of probabilities, two 8-row groups of V
-      umma_bf16_ta(tmem + 128, tmem + (j & 1) * 64 + 8 * k, v_desc + k * (2048 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-    umma_commit(&sh->v_empty[j & 1]);
-    umma_commit(&sh->o_done);
-    if (j + 1 == n_tiles) umma_commit(&sh->o_last);
+      for (int k = 0; k < PTC_KT / 16; ++k)          // 16 tokens: 8 columns of probabilities, two 8-row groups of V
+        umma_bf16_ta(tmem + 128, tmem + (j & 1) * 64 + 8 * k, v_desc + k * (2048 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+      umma_commit(&sh->v_empty[j & 1]);
+      umma_commit(&sh->o_done);
+      if (j + 1 == n_tiles) umma_commit(&sh->o_last);
+    }
+    __syncwarp();
   }
 }
 

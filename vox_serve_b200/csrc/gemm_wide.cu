@@ -251,49 +251,51 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GW_THREADS, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 0;
-      int it = 0;
-      if (rank == 0) {
-        // ================= MMA issuer =================
-        const uint64_t desc0 = umma_desc_sw128_kmajor(smem_u32(smem));
-        for (int u = first; u < p.units && !bw.dead; u += step, ++it) {
-          const GwUnit g = gw_unit(p, u);
-          const int acc = it & 1;
-          bw.wait(&acc_empty[acc], ((it >> 1) & 1) ^ 1);
-          if (bw.dead) break;
+    int s = 0, it = 0;
+    uint32_t ph = 0;
+    if (rank == 0) {
+      // ================= MMA issuer =================
+      // (the whole warp walks the loop and one elected lane issues: the operands stay in uniform registers; with a loop under
+      // `if (lane == 0)` moving them there cost 70 cycles per MMA)
+      const uint64_t desc0 = umma_desc_sw128_kmajor(smem_u32(smem));
+      for (int u = first; u < p.units && !bw.dead; u += step, ++it) {
+        const GwUnit g = gw_unit(p, u);
+        const int acc = it & 1;
+        bw.wait(&acc_empty[acc], ((it >> 1) & 1) ^ 1);
+        if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+        tc_fence_after();
+        const uint32_t d = tmem_base + acc * GW_ACC_COLS, idesc = umma_idesc(256, g.n_cur, 1u);
+        for (int kb = g.kb0; kb < g.kb1; kb += GW_KPS) {
+          bw.wait(&full[s], ph);
+          bw.wait(&peer[s], ph);
+          if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
           tc_fence_after();
-          const uint32_t d = tmem_base + acc * GW_ACC_COLS;
-          const uint32_t idesc = umma_idesc(256, g.n_cur, 1u);
-          for (int kb = g.kb0; kb < g.kb1; kb += GW_KPS) {
-            bw.wait(&full[s], ph);
-            bw.wait(&peer[s], ph);
-            if (bw.dead) break;
-            tc_fence_after();
-            uint64_t a_desc = desc0 + static_cast<uint64_t>(s) * (stage_bytes >> 4), b_desc = a_desc + (b_off >> 4);
-            const int nk = min(GW_KPS, g.kb1 - kb);
-            for (int j = 0; j < nk; ++j, a_desc += GW_A_BYTES >> 4, b_desc += b_bytes >> 4) {
+          const uint64_t a0 = desc0 + static_cast<uint64_t>(s) * (stage_bytes >> 4), b0 = a0 + (b_off >> 4);
+          const int nk = min(GW_KPS, g.kb1 - kb);
+          if (elect_one()) {
+            for (int j = 0; j < nk; ++j) {
+              const uint64_t a_desc = a0 + j * (GW_A_BYTES >> 4), b_desc = b0 + j * (b_bytes >> 4);
 #pragma unroll
               for (int k = 0; k < GW_BLOCK_K / 16; ++k)
                 umma2_bf16(d, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > g.kb0 || j > 0 || k > 0) ? 1u : 0u);
             }
             umma2_commit(&empty[s]);
-            if (++s == p.stages) { s = 0; ph ^= 1u; }
+            if (kb + GW_KPS >= g.kb1) umma2_commit(&acc_full[acc]);
           }
-          if (!bw.dead) umma2_commit(&acc_full[acc]);
+          __syncwarp();
+          if (++s == p.stages) { s = 0; ph ^= 1u; }
         }
-      } else {
-        // ================= relay: this CTA's half of a stage has landed =================
-        const uint32_t peer0 = cluster_addr(peer, 0);
-        for (int u = first; u < p.units && !bw.dead; u += step) {
-          const GwUnit g = gw_unit(p, u);
-          for (int kb = g.kb0; kb < g.kb1; kb += GW_KPS) {
-            bw.wait(&full[s], ph);
-            if (bw.dead) break;
-            mbar_arrive_cluster(peer0 + 8 * s);
-            if (++s == p.stages) { s = 0; ph ^= 1u; }
-          }
+      }
+    } else if (lane == 0) {
+      // ================= relay: this CTA's half of a stage has landed =================
+      const uint32_t peer0 = cluster_addr(peer, 0);
+      for (int u = first; u < p.units && !bw.dead; u += step) {
+        const GwUnit g = gw_unit(p, u);
+        for (int kb = g.kb0; kb < g.kb1; kb += GW_KPS) {
+          bw.wait(&full[s], ph);
+          if (bw.dead) break;
+          mbar_arrive_cluster(peer0 + 8 * s);
+          if (++s == p.stages) { s = 0; ph ^= 1u; }
         }
       }
     }

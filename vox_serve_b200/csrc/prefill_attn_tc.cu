@@ -155,8 +155,7 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
     if (warp < 4) {
       ptc_softmax<D>(smem, sh, rows, bw);
     } else if (warp == 4) {
-      if (lane == 0) ptc_issue<D>(smem, sh, n_tiles, bw);
-      __syncwarp();
+      ptc_issue<D>(smem, sh, n_tiles, bw);
     } else if (TMA) {
       if (warp == 5 && lane == 0) {
         const int pbase = p.kv_indptr[req];

@@ -511,7 +511,7 @@ int vb_gemm_wide_timeouts(void);
  *   r_bstride: floats from one batch entry to the next (rows are dense: Cin, N and N floats); y, y2 and resid rows on 16-byte
  *   boundaries.  d_y2 (optional): the activated values, d_y then holds the plain ones.  A transposed convolution of stride s (2 s
  *   taps): ksize 2, N = s * Cout with n = phase * Cout + co, rows 0 .. T; its output flattened to positions starts `padding` positions in.
- * vb_cl_dwconv7 / vb_cl_last_conv: depthwise 7 taps ("same") with Snake on both sides; one output channel, `left` positions of
+ * vb_cl_dwconv7 / vb_cl_last_conv: depthwise 7 taps (w [7][C], "same") with Snake on both sides; one output channel, `left` positions of
  *   context, optional tanh -> y [B][t1 - t0].
  * vb_cl_from_codes, vb_cl_codes_sum, vb_cl_upsample (w [C][2 s]), vb_cl_layernorm, vb_cl_chunk_attention (qkv [B][T][3 C], T <= 64).
  * vb_cl_timeouts: as vb_gemm_wide_timeouts. */

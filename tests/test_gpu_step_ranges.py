@@ -159,7 +159,7 @@ def test_channels_last_depthwise_and_last(B, T, C, dil, lo, hi, big):
         return v.double() + torch.sin(y) ** 2 / (a.double()[:, None] + 1e-9)
 
     xs = _cl.Act(x.reshape(-1).clone(), B, T, C)
-    y = _cl.depthwise7(xs, w, b, table(a1), table(a2) if big == 1.0 else None, dil, lo, hi).tensor()
+    y = _cl.depthwise7(xs, w.t().contiguous(), b, table(a1), table(a2) if big == 1.0 else None, dil, lo, hi).tensor()
     v = torch.nn.functional.conv1d(snake(x.transpose(1, 2), a1), w.double()[:, None], b.double(), dilation=dil, padding=3 * dil, groups=C)
     v = snake(v.float(), a2) if big == 1.0 else v
     _close(y[:, lo:hi], v.transpose(1, 2)[:, lo:hi], 5e-6)

@@ -19,7 +19,10 @@
 // 6..13 are the epilogue.  Persistent CTAs, two accumulators, 4 to 7 stages (TMEM and shared memory both bound them).
 // The width of a column tile (32, 64 or 128) is chosen per launch from the number of tiles: a transformer layer of 640 rows
 // has 5 x 4 tiles of 128.
-// Measured (device time, one pass): see the table at vb_cl_conv.
+// What bounds it: wide layers of few positions are one chain of 32-deep k-blocks (0.41 us each, the split into halves), narrow
+// layers of many positions the rows that the epilogue reads and writes (1x1 with residual, 64 channels: 1.0 GB in 235 us).
+// Measured (one pass): SNAC 32 windows 1454 us channel-first, 733 here; 1 window 711 and 313; Mimi 32 chunks 6721 and 2407.
+// The residual's rows asked for before the accumulator is waited for, and row offsets taken once per CTA: Mimi 2499 -> 2407.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 32
 #include "common.cuh"
@@ -100,16 +103,6 @@ __device__ __forceinline__ float cl_sin_sq(float x) {
   const float sn = fmaf(r * u, q, r);
   return sn * sn;
 }
-__device__ __forceinline__ float cl_snake(float x, float a, float inv) {
-  const float y = a * x;
-  float s2 = cl_sin_sq(y);
-  if (!(fabsf(y) <= CL_SIN_MAX)) {
-    const float sn = sinf(y);
-    s2 = sn * sn;
-  }
-  return x + inv * s2;
-}
-
 struct ClUnit {
   int n0, n_cur, t0, b0;
 };
@@ -290,42 +283,58 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
     float* st = epi_sm + (warp - 6) * 1024;
     float4* my_row = reinterpret_cast<float4*>(st + lane * 32);
     const int cq = lane & 7, rq = lane >> 3, sw = lane & 7;      // transposed side: 16-byte chunk cq of rows rq, rq + 4, ...
+    // rows rq, rq + 4, ... of the quarter -> (batch entry, position) inside a tile, and where they lie from the tile's first row on
+    // (the same for every tile; 32-bit offsets, the host keeps a launch below 2^31 elements)
+    int bt[8], yrel[8], rrel[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = quarter * 32 + i * 4 + rq, bb = r / p.nr, tt = r - bb * p.nr;
+      bt[i] = bb < p.nb ? (bb << 16) | tt : -1;
+      yrel[i] = bb * static_cast<int>(p.y_bstride) + tt * p.ldy + cq * 4;
+      rrel[i] = bb * static_cast<int>(p.r_bstride) + tt * p.ldr + cq * 4;
+    }
     int it = 0;
     for (int u = blockIdx.x; u < p.units && !bw.dead; u += gridDim.x, ++it) {
       const ClUnit g = cl_unit(p, u);
       const int acc = it & 1;
-      // rows of the tile -> (batch, position)
       uint32_t live = 0;
-      int rb[8], rt[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int r = quarter * 32 + i * 4 + rq, bb = r / p.nr;
-        rb[i] = g.b0 + bb;
-        rt[i] = g.t0 + r - bb * p.nr;
-        live |= ((bb < p.nb && rb[i] < p.B && rt[i] < p.n_hi) ? 1u : 0u) << i;
-      }
-      bw.wait(&acc_full[acc], (it >> 1) & 1);
-      if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
-      tc_fence_after();
-      // (everything below follows the accumulator, i.e. copies issued after the previous kernel had finished)
+      for (int i = 0; i < 8; ++i)
+        live |= ((bt[i] >= 0 && g.b0 + (bt[i] >> 16) < p.B && g.t0 + (bt[i] & 0xffff) < p.n_hi) ? 1u : 0u) << i;
+      const int y0 = g.b0 * static_cast<int>(p.y_bstride) + g.t0 * p.ldy + g.n0;
+      const int r0 = g.b0 * static_cast<int>(p.r_bstride) + g.t0 * p.ldr + g.n0;
+      bool first = true;
       float nz = 0.f;
-      if (p.epi == CE_NOISE) {
-        const int r = quarter * 32 + lane, bb = r / p.nr, b = g.b0 + bb, t = g.t0 + r - bb * p.nr;
-        if (bb < p.nb && b < p.B && t < p.n_hi) nz = __ldcg(&p.noise[static_cast<long long>(b) * p.noise_ld + t]);
-      }
-      const uint32_t taddr = tmem_base + acc * p.nt + (static_cast<uint32_t>(quarter * 32) << 16);
 #pragma unroll 1
-      for (int c0 = 0; c0 < g.n_cur; c0 += 32) {
-        if ((((c0 >> 5) + it) & 1) != half) continue;            // (by unit as well: a 32-column tile has one chunk)
+      for (int c0 = (((it & 1) ^ half) << 5); c0 < g.n_cur; c0 += 64) {      // (by unit as well: a 32-column tile has one chunk)
         const int n0 = g.n0 + c0, nm = n0 % p.cmod;              // 32 columns from a multiple of 32 lie in one group of channels
+        // the residual's rows are requested before the accumulator is waited for.  (Its producer is the kernel in front of this
+        // one or an earlier one: the first unit waits for it by name, later units follow accumulators that did.)
+        float4 rs[8];
+        if (p.epi != CE_PLAIN) {
+          if (it == 0 && first) pdl_wait();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            rs[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live >> i & 1u) rs[i] = __ldcg(reinterpret_cast<const float4*>(p.resid + (r0 + c0 + rrel[i])));
+          }
+          if (p.epi == CE_NOISE) {
+            const int r = quarter * 32 + lane, bb = r / p.nr, nb = g.b0 + bb, t = g.t0 + r - bb * p.nr;
+            if (bb < p.nb && nb < p.B && t < p.n_hi) nz = __ldcg(&p.noise[static_cast<long long>(nb) * p.noise_ld + t]);
+          }
+        }
+        if (first) {
+          bw.wait(&acc_full[acc], (it >> 1) & 1);
+          if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+          tc_fence_after();
+          first = false;
+        }
+        const uint32_t taddr = tmem_base + acc * p.nt + (static_cast<uint32_t>(quarter * 32) << 16);
         if (p.epi != CE_PLAIN) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live >> i & 1u)
-              q = __ldcg(reinterpret_cast<const float4*>(p.resid + rb[i] * p.r_bstride + static_cast<long long>(rt[i]) * p.ldr + n0 + cq * 4));
             const int r = i * 4 + rq;
-            *reinterpret_cast<float4*>(st + r * 32 + ((cq ^ (r & 7)) << 2)) = q;
+            *reinterpret_cast<float4*>(st + r * 32 + ((cq ^ (r & 7)) << 2)) = rs[i];
           }
         }
         uint32_t tv[32];
@@ -369,7 +378,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
             const int r = i * 4 + rq;
             const float4 q = *reinterpret_cast<const float4*>(st + r * 32 + ((cq ^ (r & 7)) << 2));
             if (live >> i & 1u)
-              *reinterpret_cast<float4*>(y + rb[i] * p.y_bstride + static_cast<long long>(rt[i]) * p.ldy + n0 + cq * 4) = q;
+              *reinterpret_cast<float4*>(y + (y0 + c0 + yrel[i])) = q;
           }
           __syncwarp();
         };
@@ -411,6 +420,11 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
         }
         store(p.y2 ? p.y2 : p.y);
       }
+      if (bw.dead) break;
+      if (first) {                    // (a warp without a chunk of this unit keeps in step with the accumulators all the same)
+        bw.wait(&acc_full[acc], (it >> 1) & 1);
+        if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
@@ -449,8 +463,20 @@ __global__ void __launch_bounds__(256) cl_pack_kernel(float4* __restrict__ dst, 
 // depthwise convolution, 7 taps, dilation d, "same" padding; Snake on the input and on the output (optional both)
 // ------------------------------------------------------------------------------------------
 // A block owns 64 channels x DW_T positions: the (activated) input rows with their halo are staged once in shared memory, so
-// every element is read and put through its sine once, in 256-byte rows; a thread finishes four channels of several rows.
-constexpr int DW_T = 64;
+// every element is read and put through its sine once, in 256-byte rows; a thread finishes four channels of DW_T / 16 rows, whose
+// chains interleave (the activation branches once per four values, to the library's sine when an argument is out of range).
+// DW_T 128 and four-wide activations against 64 and one by one: 12 to 30 us a layer -> 4 to 14, SNAC 32 windows 858 -> 733 us.
+constexpr int DW_T = 128;
+__device__ __forceinline__ float4 cl_snake4(float4 v, const float4& a, const float4& inv) {
+  const float4 y = make_float4(a.x * v.x, a.y * v.y, a.z * v.z, a.w * v.w);
+  const float big = fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w)));
+  float4 s = make_float4(cl_sin_sq(y.x), cl_sin_sq(y.y), cl_sin_sq(y.z), cl_sin_sq(y.w));
+  if (!(big <= CL_SIN_MAX)) {
+    const float4 t = make_float4(sinf(y.x), sinf(y.y), sinf(y.z), sinf(y.w));
+    s = make_float4(t.x * t.x, t.y * t.y, t.z * t.z, t.w * t.w);
+  }
+  return make_float4(fmaf(inv.x, s.x, v.x), fmaf(inv.y, s.y, v.y), fmaf(inv.z, s.z, v.z), fmaf(inv.w, s.w, v.w));
+}
 __global__ void __launch_bounds__(256) cl_dwconv7_kernel(float* __restrict__ y, const float* __restrict__ x, long long x_bstride,
                                                          const float* __restrict__ w, const float* __restrict__ bias,
                                                          const float* __restrict__ alpha_in, const float* __restrict__ alpha_out,
@@ -459,52 +485,43 @@ __global__ void __launch_bounds__(256) cl_dwconv7_kernel(float* __restrict__ y, 
   const int c4 = threadIdx.x & 15, r0 = threadIdx.x >> 4;
   const int c = blockIdx.y * 64 + c4 * 4, b = blockIdx.z, t0 = t_lo + blockIdx.x * DW_T;
   const int halo = 3 * dil, n_out = min(DW_T, t_hi - t0), rows = n_out + 2 * halo;
-  float wk[7][4];
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto ld4 = [&](const float* p) { return p ? __ldg(reinterpret_cast<const float4*>(p + c)) : zero; };
+  const float4 ai = ld4(alpha_in), ii = ld4(alpha_in ? alpha_in + C : nullptr), ao = ld4(alpha_out),
+               io = ld4(alpha_out ? alpha_out + C : nullptr), bv = ld4(bias);
+  float4 wk[7];
 #pragma unroll
-  for (int k = 0; k < 7; ++k)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) wk[k][e] = __ldg(&w[(c + e) * 7 + k]);
-  float ai[4] = {0.f, 0.f, 0.f, 0.f}, ii[4], ao[4] = {0.f, 0.f, 0.f, 0.f}, io[4], bv[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    ii[e] = io[e] = 0.f;
-    if (alpha_in) { ai[e] = __ldg(&alpha_in[c + e]); ii[e] = __ldg(&alpha_in[C + c + e]); }
-    if (alpha_out) { ao[e] = __ldg(&alpha_out[c + e]); io[e] = __ldg(&alpha_out[C + c + e]); }
-    if (bias) bv[e] = __ldg(&bias[c + e]);
-  }
+  for (int k = 0; k < 7; ++k) wk[k] = ld4(w + k * C);
   pdl_sync();
   const float* xb = x + static_cast<size_t>(b) * x_bstride + c;
-  for (int r = r0; r < rows; r += 16) {
-    const int t = t0 - halo + r;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (t >= 0 && t < T) {
-      v = __ldcg(reinterpret_cast<const float4*>(xb + static_cast<size_t>(t) * C));
-      if (alpha_in) {
-        v.x = cl_snake(v.x, ai[0], ii[0]);
-        v.y = cl_snake(v.y, ai[1], ii[1]);
-        v.z = cl_snake(v.z, ai[2], ii[2]);
-        v.w = cl_snake(v.w, ai[3], ii[3]);
-      }
+  for (int rb = r0; rb < rows; rb += 64) {
+    float4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = rb + 16 * i, t = t0 - halo + r;
+      v[i] = (r < rows && t >= 0 && t < T) ? __ldcg(reinterpret_cast<const float4*>(xb + static_cast<size_t>(t) * C)) : zero;
     }
-    tile[r * 16 + c4] = v;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (alpha_in) v[i] = cl_snake4(v[i], ai, ii);              // (the activation of zero is zero)
+      if (rb + 16 * i < rows) tile[(rb + 16 * i) * 16 + c4] = v[i];
+    }
   }
   __syncthreads();
   float* yb = y + static_cast<size_t>(b) * T * C + c;
+#pragma unroll 2
   for (int r = r0; r < n_out; r += 16) {
-    float o[4] = {bv[0], bv[1], bv[2], bv[3]};
+    float4 o = bv;
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
       const float4 v = tile[(r + k * dil) * 16 + c4];
-      o[0] += wk[k][0] * v.x;
-      o[1] += wk[k][1] * v.y;
-      o[2] += wk[k][2] * v.z;
-      o[3] += wk[k][3] * v.w;
+      o.x = fmaf(wk[k].x, v.x, o.x);
+      o.y = fmaf(wk[k].y, v.y, o.y);
+      o.z = fmaf(wk[k].z, v.z, o.z);
+      o.w = fmaf(wk[k].w, v.w, o.w);
     }
-    if (alpha_out) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) o[e] = cl_snake(o[e], ao[e], io[e]);
-    }
-    *reinterpret_cast<float4*>(yb + static_cast<size_t>(t0 + r) * C) = make_float4(o[0], o[1], o[2], o[3]);
+    if (alpha_out) o = cl_snake4(o, ao, io);
+    *reinterpret_cast<float4*>(yb + static_cast<size_t>(t0 + r) * C) = o;
   }
 }
 
@@ -780,6 +797,20 @@ int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, i
                    (!d_y2 || reinterpret_cast<uintptr_t>(d_y2) % 16 == 0),
                "vb_cl_conv: rows must start on 16-byte boundaries");
   if (B <= 0 || n_lo >= n_hi) return 0;
+  // the epilogue addresses rows with 32-bit offsets: batches beyond that run in several launches
+  const long long per_entry = max(max(y_bstride, r_bstride), static_cast<long long>(n_hi) * N);
+  VB_CHECK_ARG(per_entry < (1LL << 30) && N <= (1 << 20), "vb_cl_conv: a batch entry of %lld elements is too large", per_entry);
+  const int max_b = static_cast<int>(((1LL << 31) - 1) / per_entry) - 1;
+  if (B > max_b) {
+    for (int b0 = 0; b0 < B; b0 += max_b) {
+      const int rc = vb_cl_conv(d_y + b0 * y_bstride, d_y2 ? d_y2 + b0 * y_bstride : nullptr, d_x + b0 * x_bstride, x_bstride, Tx, d_w, d_bias,
+                                d_resid ? d_resid + b0 * r_bstride : nullptr, r_bstride, d_scale,
+                                d_noise ? d_noise + static_cast<long long>(b0) * noise_ld : nullptr, noise_ld, d_alpha, epilogue, act,
+                                min(max_b, B - b0), Cin, N, cmod, ksize, dil, n_lo, n_hi, y_bstride, stream);
+      if (rc != 0) return rc;
+    }
+    return 0;
+  }
   auto fn = encode_fn();
   VB_CHECK_ARG(fn, "cuTensorMapEncodeTiled not available (no CUDA driver?)");
   ClConvParams p = {};

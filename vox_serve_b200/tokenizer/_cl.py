@@ -88,6 +88,7 @@ def conv_transposed(x: Act, w: torch.Tensor, cout: int, stride: int, bias, pad: 
 
 
 def depthwise7(x: Act, w: torch.Tensor, bias, alpha_in, alpha_out, dil: int, lo: int, hi: int) -> Act:
+    """w [7, C]; alpha tables [2, C]: values, then 1 / (alpha + 1e-9)"""
     y = Act.empty(x.B, x.T, x.C, x.buf.device)
     call("vb_cl_dwconv7", y.ptr, x.ptr, x.bstride, w.data_ptr(), _ptr(bias), _ptr(alpha_in), _ptr(alpha_out), x.B, x.C, x.T, dil, lo, hi,
          ops._stream())

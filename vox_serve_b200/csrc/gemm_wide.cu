@@ -10,8 +10,8 @@
 //   * the ring holds 3 or 4 stages of 128 k;
 //   * the token tile is a launch parameter (a multiple of 16, at most 256): the host picks the one that fills the last wave.
 //     With 148 SMs and 1024 rows, 256-token tiles leave the QKV projection of 5120 rows in 80 units on 74 pairs.
-// Measured per launch (one-SM kernel -> this one, us): 1024 rows, QKV 5120 x 3072: 63 -> 33, O 3072 x 3072: 40 -> 21, gate/up
-// 16384 x 3072: 171 -> 87 (1.2 PFLOP/s), down 3072 x 8192: 79 -> 41; 133 rows: 16 -> 11.4, 13.6 -> 10.4, 32 -> 28.5, 17.5 ->
+// Measured per launch (one-SM kernel -> this one, us): 1024 rows, QKV 5120 x 3072: 63 -> 32, O 3072 x 3072: 40 -> 19, gate/up
+// 16384 x 3072: 171 -> 77 (1.34 PFLOP/s), down 3072 x 8192: 79 -> 38; 133 rows: 16 -> 11.4, 13.6 -> 10.4, 32 -> 28.5, 17.5 ->
 // 13.7.  What bounds it now: operands out of L2 (with the products left out the copies alone run at 15.5 TB/s over all SMs,
 // 0.31 us per 64-k block of a 256-token tile, where the tensor cores need 0.27) and the last wave.
 // Operands: weights as vb_pack_weight_tiles lays them out (linear bulk copies); activations in the tiled XT layout (linear
@@ -108,7 +108,8 @@ __device__ __forceinline__ GwUnit gw_unit(const GemmWideParams& p, int u) {
   return r;
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GW_THREADS, 1)
+// (bounded to 128 registers: what is left of the file holds the first blocks of the kernel behind this one, which start early)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
     gemm_wide_kernel(const GemmWideParams p, const __grid_constant__ CUtensorMap x_map) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -331,29 +332,48 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GW_THREADS, 1)
           __nv_bfloat16* yc = p.y_tiled ? y + ((static_cast<size_t>(tb) * nkb_y + (n_out >> 6)) * p.x_tile + tt) * 64 + (n_out & 7)
                                         : y + static_cast<size_t>(tc) * p.ldy + n_out;
           tmem_ld_wait();
+          // this lane finishes tokens c0 + 2 i + hi: gate from the low half-warp, up from the high one.  The eight values are
+          // taken through each step together (no branch inside: uniform choices stand outside the loops), or a warp waits out
+          // every exponential and division on its own: 18 us per 256-token unit, more than its products take (gate/up of 1024
+          // rows: 86 -> 77 us)
+          float gt[8], up[8], o[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            // this lane finishes token c0 + 2 i + hi: gate from the low half-warp, up from the high one
-            const float mine = __uint_as_float(v[2 * i + (hi ? 1 : 0)]);
-            const float send = __uint_as_float(v[2 * i + (hi ? 0 : 1)]);
+            const float mine = __uint_as_float(hi ? v[2 * i + 1] : v[2 * i]);
+            const float send = __uint_as_float(hi ? v[2 * i] : v[2 * i + 1]);
             const float other = __shfl_xor_sync(0xffffffffu, send, 16);
-            float o;
-            if (p.glu_limit > 0.f) {
-              const float gt = fminf(hi ? other : mine, p.glu_limit);
-              const float up = fminf(fmaxf(hi ? mine : other, -p.glu_limit), p.glu_limit);
-              o = gt / (1.0f + expf(-p.glu_slope * gt)) * (up + 1.0f);
-            } else if (p.act != 0) {
-              o = gw_act(hi ? other : mine, p.act) * (hi ? mine : other);
-            } else {
-              const float gt = round_bf16(hi ? other : mine);
-              const float up = round_bf16(hi ? mine : other);
-              o = round_bf16(gt / (1.0f + expf(-gt))) * up;
+            gt[i] = hi ? other : mine;
+            up[i] = hi ? mine : other;
+          }
+          if (p.glu_limit > 0.f) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              gt[i] = fminf(gt[i], p.glu_limit);
+              up[i] = fminf(fmaxf(up[i], -p.glu_limit), p.glu_limit);
+              o[i] = __fdividef(gt[i], 1.0f + expf(-p.glu_slope * gt[i])) * (up[i] + 1.0f);
             }
+          } else if (p.act == 1) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = gw_act(gt[i], 1) * up[i];
+          } else if (p.act == 2) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = gw_act(gt[i], 2) * up[i];
+          } else if (p.act == 3) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = gw_act(gt[i], 3) * up[i];
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              gt[i] = round_bf16(gt[i]);
+              o[i] = round_bf16(__fdividef(gt[i], 1.0f + expf(-gt[i]))) * round_bf16(up[i]);
+            }
+          }
+          const int lim = live ? p.T - tc : 0;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
             const int j = 2 * i + (hi ? 1 : 0);
-            if (live && tc + j < p.T) {
-              const size_t yi = p.y_tiled ? static_cast<size_t>(j) * 64 + ((yk ^ (j & 7)) << 3) : static_cast<size_t>(j) * p.ldy;
-              yc[yi] = __float2bfloat16_rn(o);
-            }
+            const size_t yi = p.y_tiled ? static_cast<size_t>(j * 64 + ((yk ^ (j & 7)) << 3)) : static_cast<size_t>(j) * p.ldy;
+            if (j < lim) yc[yi] = __float2bfloat16_rn(o[i]);
           }
         }
       } else {
@@ -379,11 +399,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GW_THREADS, 1)
             uint32_t v[16];
             tmem_ld_32x16(taddr + c0, v);
             tmem_ld_wait();
+            float a[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) a[j] = __uint_as_float(v[j]) + bv;
+            if (p.act == 1) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) a[j] = gw_act(a[j], 1);
+            } else if (p.act == 2) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) a[j] = gw_act(a[j], 2);
+            } else if (p.act == 3) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) a[j] = gw_act(a[j], 3);
+            }
             if (live) {
               const int t = g.t0 + c0, m = min(16, p.T - t);
 #pragma unroll
               for (int j = 0; j < 16; ++j)
-                if (j < m) y[static_cast<size_t>(t + j) * p.ldy] = __float2bfloat16_rn(gw_act(__uint_as_float(v[j]) + bv, p.act));
+                if (j < m) y[static_cast<size_t>(t + j) * p.ldy] = __float2bfloat16_rn(a[j]);
             }
           }
         }

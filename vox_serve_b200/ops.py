@@ -383,7 +383,7 @@ def gemm_t_tile(T: int) -> int:
 
 # Steps of more rows than this run their projections on the kernel for pairs of SMs (gemm_wide.cu): from 80 rows on it is
 # as fast or faster on every projection measured (80 rows: QKV 11.1 against 12.3 us, gate/up 25.1 against 27.4, down 13.0
-# against 14.5; 1024 rows: 33 / 63, 86 / 171, 41 / 79); up to 64 rows the one-SM kernel's layouts and fused tails apply.
+# against 14.5; 1024 rows: 32 / 63, 77 / 171, 38 / 79); up to 64 rows the one-SM kernel's layouts and fused tails apply.
 WIDE_MIN_ROWS = 65
 WIDE_TILE_ROWS = (32, 64, 96, 128)
 WIDE_SPLIT_ROWS = 1664       # most (split x rows) of fp32 planes a projection is split into

@@ -220,3 +220,54 @@ def test_window_attention_prompt_rows(ops, D, H, G, page, new, old, window, chun
                     keep_first=keep, head_gate=gate == "head")
     _close(out.view(T, H, D), want, 2 ** -8)         # probabilities and the output rounded to bf16
     assert _lib.load().vb_window_attn_tc_timeouts() == 0
+
+
+@pytest.mark.parametrize("T,N,S,resid,tiled,hidden", [
+    (513, 8, 1, True, False, True), (514, 2048, 3, True, True, True), (600, 3072, 1, False, True, False), (515, 4096, 2, True, False, True),
+    (516, 1032, 9, True, False, True), (1024, 264, 1, True, False, False),
+])
+def test_reduce_residual_rmsnorm_many_rows(ops, T, N, S, resid, tiled, hidden):
+    """A step of more than 512 rows against the same rows in steps of 200, which take the other kernel."""
+    g = torch.Generator("cuda").manual_seed(T)
+    parts = torch.randn(S, T, N, generator=g, device="cuda")
+    res = torch.randn(T, N, generator=g, device="cuda").to(torch.bfloat16) if resid else None
+    w = torch.randn(N, generator=g, device="cuda").to(torch.bfloat16)
+    out = ops.TiledAct(T, N, torch.device("cuda")) if tiled else None
+    h, y = ops.reduce_residual_rmsnorm(parts, res, w, 1e-6, normed_out=out, want_hidden=hidden)
+    y = y.to_rows() if tiled else y
+    cut = [slice(a, min(a + 200, T)) for a in range(0, T, 200)]
+    want = [ops.reduce_residual_rmsnorm(parts[:, c].contiguous(), None if res is None else res[c].contiguous(), w, 1e-6) for c in cut]
+    if hidden:
+        assert torch.equal(h, torch.cat([a for a, _ in want]))
+    ref = torch.cat([b for _, b in want])
+    # the sum of squares is taken in another order: the scale moves by a few 2^-24, a result by one bf16 step at most
+    assert ((y.float() - ref.float()).abs() <= ref.float().abs() * 2.0 ** -7).all()
+
+
+@pytest.mark.parametrize("T,n_q,n_kv,D,S,bias", [(257, 1, 1, 16, 1, False), (300, 24, 8, 128, 1, False), (258, 5, 1, 80, 3, True), (600, 2, 2, 256, 2, False)])
+def test_qkv_rope_append_many_rows(ops, T, n_q, n_kv, D, S, bias):
+    """A step of more than 256 rows against the same rows in steps of at most 256; rows without a page keep the cache as it is."""
+    g = torch.Generator("cuda").manual_seed(T)
+    W, page = (n_q + 2 * n_kv) * D, 16
+    parts = torch.randn(S, T, W, generator=g, device="cuda")
+    b = torch.randn(W, generator=g, device="cuda").to(torch.bfloat16) if bias else None
+    freq = (1.0 / 10000 ** (torch.arange(D, device="cuda") % (D // 2) / (D // 2))).float()
+    pos = torch.randint(0, 4096, (T,), generator=g, device="cuda", dtype=torch.int32)
+    n_pages = (T + page - 1) // page
+    plan = ops.RowPlan(T, "cuda")
+    at = torch.randperm(n_pages * page, generator=g, device="cuda")[:T].int()
+    plan.row_page[:T] = at // page
+    plan.row_slot[:T] = at % page
+    plan.row_page[T // 2] = -1
+    kv = [torch.full((n_pages, 2, page, n_kv, D), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    q = ops.qkv_rope_append(parts, kv[0], pos, freq, plan, n_q, n_kv, D, qkv_bias=b)
+    want = []
+    for a in range(0, T, 200):
+        n = min(200, T - a)
+        sub = ops.RowPlan(n, "cuda")
+        sub.row_page[:n] = plan.row_page[a:a + n]
+        sub.row_slot[:n] = plan.row_slot[a:a + n]
+        want.append(ops.qkv_rope_append(parts[:, a:a + n].contiguous(), kv[1], pos[a:a + n].contiguous(), freq, sub, n_q, n_kv, D, qkv_bias=b))
+    # the same products and one sum, which the compiler may fuse on either side: one bf16 step of the larger term at most
+    for got, ref in ((q, torch.cat(want)), (kv[0], kv[1])):
+        assert ((got.float() - ref.float()).abs() <= ref.float().abs() * 2.0 ** -7 + 2.0 ** -20 * 8).all()

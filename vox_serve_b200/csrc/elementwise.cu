@@ -320,6 +320,93 @@ __global__ void __launch_bounds__(RR_THREADS) reduce_residual_rmsnorm_kernel(
   trace_end(tr);
 }
 
+// The same for steps of many rows: one WARP per row, no shared memory and no barrier.  A lane takes 8 columns of every 256, all
+// planes of four such groups in flight together, keeps the new row as packed bf16 and writes 16 bytes at a time.  With a CTA per row
+// a 1024-row step of 3072 columns took 23.5 us for 31 MB (three loads in flight per thread, then two barriers), now 16.7.
+constexpr int RW_GROUPS = 16;       // N <= 256 * RW_GROUPS
+__global__ void __launch_bounds__(128) reduce_residual_rmsnorm_rows_kernel(
+    __nv_bfloat16* __restrict__ hidden_out, __nv_bfloat16* __restrict__ normed_out, const float* __restrict__ partials, int split_k,
+    const __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ norm_w, int T, int N, float eps, int xt_tile) {
+  const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const size_t plane = static_cast<size_t>(T) * N, row = static_cast<size_t>(t) * N;
+  pdl_sync();
+  if (t >= T) return;
+  uint4 h[RW_GROUPS];
+  float ss = 0.f;
+#pragma unroll
+  for (int g0 = 0; g0 < RW_GROUPS; g0 += 4) {
+    if (g0 * 256 < N) {
+      float4 a[4][2];
+      uint4 r[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int n = (g0 + i) * 256 + lane * 8;
+        a[i][0] = a[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        r[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (n < N) {
+          const float4* src = reinterpret_cast<const float4*>(partials + row + n);
+          a[i][0] = __ldcg(src);
+          a[i][1] = __ldcg(src + 1);
+          if (residual) r[i] = __ldcg(reinterpret_cast<const uint4*>(residual + row + n));
+        }
+      }
+      for (int s = 1; s < split_k; ++s) {
+        float4 b[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int n = (g0 + i) * 256 + lane * 8;
+          b[i][0] = b[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (n < N) {
+            const float4* src = reinterpret_cast<const float4*>(partials + s * plane + row + n);
+            b[i][0] = __ldcg(src);
+            b[i][1] = __ldcg(src + 1);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            a[i][k].x += b[i][k].x; a[i][k].y += b[i][k].y; a[i][k].z += b[i][k].z; a[i][k].w += b[i][k].w;
+          }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int n = (g0 + i) * 256 + lane * 8;
+        const float x[8] = {a[i][0].x, a[i][0].y, a[i][0].z, a[i][0].w, a[i][1].x, a[i][1].y, a[i][1].z, a[i][1].w};
+        const uint32_t rr[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float u = round_bf16(x[2 * j]), v = round_bf16(x[2 * j + 1]);
+          if (residual) {
+            u = round_bf16(bf16_lo(rr[j]) + u);
+            v = round_bf16(bf16_hi(rr[j]) + v);
+          }
+          o[j] = pack_bf16(u, v);
+          ss += u * u + v * v;
+        }
+        h[g0 + i] = make_uint4(o[0], o[1], o[2], o[3]);
+        if (hidden_out && n < N) *reinterpret_cast<uint4*>(hidden_out + row + n) = h[g0 + i];
+      }
+    }
+  }
+  if (!normed_out) return;
+  const float rcp = rsqrtf(warp_sum(ss) / static_cast<float>(N) + eps);
+#pragma unroll
+  for (int g = 0; g < RW_GROUPS; ++g) {
+    const int n = g * 256 + lane * 8;
+    if (n < N) {
+      const uint4 w4 = __ldg(reinterpret_cast<const uint4*>(norm_w + n));
+      const uint32_t hv[4] = {h[g].x, h[g].y, h[g].z, h[g].w}, wv[4] = {w4.x, w4.y, w4.z, w4.w};
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[j] = pack_bf16(bf16_lo(hv[j]) * rcp * bf16_lo(wv[j]), bf16_hi(hv[j]) * rcp * bf16_hi(wv[j]));
+      const size_t oi = xt_tile ? xt_index(t, n, xt_tile, (N + 63) >> 6) : row + n;
+      *reinterpret_cast<uint4*>(normed_out + oi) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------
 // fused QKV tail: reduce partials -> bf16, RoPE(q, k), q out, K/V scatter into the layer cache.
 // Heads are independent, so a row is split over gridDim.x CTAs by groups of heads (blockIdx.x).
@@ -414,6 +501,73 @@ __global__ void __launch_bounds__(256) qkv_rope_append_kernel(
     }
   }
   trace_end(tr);
+}
+
+// The tail for whole heads rotated in halves without norms, steps of many rows: a thread finishes 8 columns of a head and the 8 that
+// turn with them, straight from the planes (no shared-memory row, one barrier for the row's cos / sin), in 16-byte pieces.  1024 rows of 40 heads of 128: 21.5 -> 15.4 us.
+__global__ void __launch_bounds__(256) qkv_rope_rows_kernel(__nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ kv,
+                                                            const float* __restrict__ partials, int split_k, const int32_t* __restrict__ pos,
+                                                            const float* __restrict__ freq, const int32_t* __restrict__ row_page,
+                                                            const int32_t* __restrict__ row_slot, int T, int n_q, int n_kv, int D,
+                                                            int page_size, const __nv_bfloat16* __restrict__ qkv_bias) {
+  extern __shared__ float sm[];      // [D] cos, [D] sin
+  const size_t t = blockIdx.x;
+  const int n_heads = n_q + 2 * n_kv, half = D >> 1, per_head = half >> 3, W = n_heads * D;
+  const size_t plane = static_cast<size_t>(T) * W;
+  pdl_sync();
+  if (threadIdx.x < D) {
+    float s, c;
+    sincosf(static_cast<float>(pos[t]) * freq[threadIdx.x], &s, &c);
+    sm[threadIdx.x] = c;
+    sm[D + threadIdx.x] = s;
+  }
+  const int page = row_page[t];
+  const size_t row_elems = static_cast<size_t>(n_kv) * D, slab = static_cast<size_t>(page_size) * row_elems;
+  __nv_bfloat16* kd = page >= 0 ? kv + static_cast<size_t>(page) * 2 * slab + static_cast<size_t>(row_slot[t]) * row_elems : nullptr;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n_heads * per_head; i += 256) {
+    const int h = i / per_head, e = (i - h * per_head) * 8, n = h * D + e;
+    float x[2][8];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float4* src = reinterpret_cast<const float4*>(partials + t * W + n + k * half);
+      const float4 a = __ldcg(src), b = __ldcg(src + 1);
+      x[k][0] = a.x; x[k][1] = a.y; x[k][2] = a.z; x[k][3] = a.w; x[k][4] = b.x; x[k][5] = b.y; x[k][6] = b.z; x[k][7] = b.w;
+    }
+    for (int s = 1; s < split_k; ++s)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float4* src = reinterpret_cast<const float4*>(partials + s * plane + t * W + n + k * half);
+        const float4 a = __ldcg(src), b = __ldcg(src + 1);
+        x[k][0] += a.x; x[k][1] += a.y; x[k][2] += a.z; x[k][3] += a.w; x[k][4] += b.x; x[k][5] += b.y; x[k][6] += b.z; x[k][7] += b.w;
+      }
+    uint32_t o[2][4];
+    float y[2][8];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (qkv_bias) x[k][j] += __bfloat162float(qkv_bias[n + k * half + j]);
+        x[k][j] = round_bf16(x[k][j]);
+      }
+    const bool rot = h < n_q + n_kv;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      y[0][j] = rot ? x[0][j] * sm[e + j] + -x[1][j] * sm[D + e + j] : x[0][j];
+      y[1][j] = rot ? x[1][j] * sm[e + half + j] + x[0][j] * sm[D + e + half + j] : x[1][j];
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[k][j] = pack_bf16(y[k][2 * j], y[k][2 * j + 1]);
+    __nv_bfloat16* dst = nullptr;
+    if (h < n_q) dst = q_out + (t * n_q + h) * D + e;
+    else if (kd) dst = kd + (h < n_q + n_kv ? (h - n_q) * D : slab + (h - n_q - n_kv) * D) + e;
+    if (dst) {
+      *reinterpret_cast<uint4*>(dst) = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]);
+      *reinterpret_cast<uint4*>(dst + half) = make_uint4(o[1][0], o[1][1], o[1][2], o[1][3]);
+    }
+  }
 }
 
 __global__ void embedding_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ table,
@@ -531,9 +685,19 @@ int vb_reduce_residual_rmsnorm(void* d_hidden_out, void* d_normed_out, const flo
   VB_CHECK_ARG(N % 4 == 0, "vb_reduce_residual_rmsnorm: N %d must be a multiple of 4", N);
   VB_CHECK_ARG(!d_normed_out || d_norm_weight, "vb_reduce_residual_rmsnorm: norm output needs a weight");
   if (T <= 0) return 0;
+  auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
+  // (512 rows of 3072: 14.3 us with a CTA per row, 15.1 with a warp; 1024 rows: 23.5 and 16.7)
+  if (T > 512 && N % 8 == 0 && N <= 256 * RW_GROUPS && aligned(d_partials) && aligned(d_hidden_out) && aligned(d_normed_out) &&
+      aligned(d_residual) && aligned(d_norm_weight)) {
+    VB_LAUNCH_PDL(reduce_residual_rmsnorm_rows_kernel, (T + 3) / 4, 128, 0, stream, static_cast<__nv_bfloat16*>(d_hidden_out),
+                  static_cast<__nv_bfloat16*>(d_normed_out), d_partials, split_k, static_cast<const __nv_bfloat16*>(d_residual),
+                  static_cast<const __nv_bfloat16*>(d_norm_weight), T, N, eps, normed_xt_tile);
+    return 0;
+  }
   // widest cluster (<= 8, the portable limit) that divides the row into float4-aligned parts; few rows -> more parts
   int parts = 1;
-  const int want = T <= 64 ? 8 : (T <= 256 ? 4 : 1);
+  // (past some 512 CTAs a split row costs more than it gives: 256 rows of 3072, 15.4 us in four parts, 11 whole)
+  const int want = T <= 64 ? 8 : (T <= 128 ? 4 : (T <= 192 ? 2 : 1));
   for (int c = want; c >= 1; c >>= 1)
     if (N % (4 * c) == 0) { parts = c; break; }
   while (N / parts > RR_THREADS * 4 * RR_MAX_ITER) {
@@ -557,6 +721,15 @@ int vb_qkv_rope_append(void* d_q_out, void* d_layer_kv, const float* d_partials,
   VB_CHECK_ARG(head_dim % 4 == 0 && rotary_dim % 2 == 0 && rotary_dim <= head_dim, "vb_qkv_rope_append: bad dims");
   if (T <= 0) return 0;
   const int n_heads = n_q + 2 * n_kv;
+  auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
+  // (257 rows of 40 heads of 128: 11.3 us by the kernel below, 9.2 here; it spreads a row's heads over CTAs up to 256 rows)
+  if (T > 256 && !interleave && rotary_dim == head_dim && head_dim % 16 == 0 && head_dim <= 256 && !d_q_norm && aligned(d_q_out) &&
+      aligned(d_layer_kv) && aligned(d_partials)) {
+    VB_LAUNCH_PDL(qkv_rope_rows_kernel, T, 256, 2 * head_dim * sizeof(float), stream, static_cast<__nv_bfloat16*>(d_q_out),
+                  static_cast<__nv_bfloat16*>(d_layer_kv), d_partials, split_k, d_pos, d_freq, d_row_page, d_row_slot, T, n_q, n_kv, head_dim,
+                  page_size, static_cast<const __nv_bfloat16*>(d_qkv_bias));
+    return 0;
+  }
   // few rows (decode): spread a row's heads over several CTAs; many rows (prefill): one CTA per row is enough
   int heads_per_cta = T <= 64 ? 4 : (T <= 256 ? 8 : n_heads);
   while (static_cast<size_t>(2 * rotary_dim + heads_per_cta * head_dim) * sizeof(float) > 96 * 1024 && heads_per_cta > 1)

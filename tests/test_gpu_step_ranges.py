@@ -271,3 +271,18 @@ def test_qkv_rope_append_many_rows(ops, T, n_q, n_kv, D, S, bias):
     # the same products and one sum, which the compiler may fuse on either side: one bf16 step of the larger term at most
     for got, ref in ((q, torch.cat(want)), (kv[0], kv[1])):
         assert ((got.float() - ref.float()).abs() <= ref.float().abs() * 2.0 ** -7 + 2.0 ** -20 * 8).all()
+
+
+@pytest.mark.parametrize("penalty", [1.3, 0.7, 3.0, 1.0 + 2.0 ** -23, 2.0 - 2.0 ** -23, 1e-3, 2.0 ** 39, 2.0 ** 41])
+def test_sampler_quotients(ops, penalty):
+    """The sampler's quotient of every positive bf16 against the division of the stand-alone penalty kernel: a penalised token ties
+    with a token that already holds the divided value (the smaller index wins a tie) whichever of the two comes first."""
+    code = torch.arange(1, 0x7f80, device="cuda").to(torch.int16).view(torch.bfloat16)
+    n = code.numel()
+    seen = torch.ones(n, 1, 1, 1, dtype=torch.bool, device="cuda")
+    div = ops.apply_repetition_penalty(code.view(n, 1, 1), seen, penalty).view(n)
+    for first in (0, 1):
+        pair = torch.stack([code, div] if first == 0 else [div, code], 1).contiguous()
+        mark = torch.zeros(n, 1, 1, 2, dtype=torch.bool, device="cuda")
+        mark[..., first] = True
+        assert (ops.sample(pair, "greedy", rep_cache=mark, penalty=penalty) == 0).all()

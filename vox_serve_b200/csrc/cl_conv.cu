@@ -13,16 +13,17 @@
 // Products: x = hi + lo and w = hi + lo, both halves rounded to tf32 (to nearest), lo_w hi_x + hi_w lo_x + hi_w hi_x with
 // fp32 accumulation; what is dropped is below 2^-22 of a product (the channel-first kernel truncates: 2^-20).
 //
-// Roles of a CTA's fourteen warps: 0 copies (activation box and two weight tiles per stage), 1 issues the MMAs, 2..5 split a
+// Roles of a CTA's eighteen warps: 0 copies (activation box and two weight tiles per stage), 1 issues the MMAs, 2..5 split a
 // stage's raw activations into the two halves and put them into TMEM as the MMA's A operand (128 x 32 columns each; through
 // shared memory the operand would cost 12 KB of its bandwidth per 8-deep product, and the two tiles another 32 KB of stores),
-// 6..13 are the epilogue.  Persistent CTAs, two accumulators, 4 to 7 stages (TMEM and shared memory both bound them).
+// 6..17 are the epilogue.  Persistent CTAs, two accumulators, 4 to 7 stages (TMEM and shared memory both bound them).
 // The width of a column tile (32, 64 or 128) is chosen per launch from the number of tiles: a transformer layer of 640 rows
 // has 5 x 4 tiles of 128.
 // What bounds it: wide layers of few positions are one chain of 32-deep k-blocks (0.41 us each, the split into halves), narrow
-// layers of many positions the rows that the epilogue reads and writes (1x1 with residual, 64 channels: 1.0 GB in 235 us).
-// Measured (one pass): SNAC 32 windows 1454 us channel-first, 733 here; 1 window 711 and 313; Mimi 32 chunks 6721 and 2407.
-// The residual's rows asked for before the accumulator is waited for, and row offsets taken once per CTA: Mimi 2499 -> 2407.
+// layers of many positions the epilogue (1x1 with residual, 614400 positions of 64 channels: 393 MB in 126 us).
+// Measured (one pass): SNAC 32 windows 1454 us channel-first, 647 here; 1 window 711 and 266; Mimi 32 chunks 6721 and 1933.
+// Of that, the residual's rows asked for before the accumulator is waited for: Mimi 2499 -> 2407; 16 columns at a time on twelve warps
+// without a spilled register, where 32 on eight spilled 53: Mimi 2403 -> 1933, SNAC 746 -> 647 and 313 -> 266.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 32
 #include "common.cuh"
@@ -31,11 +32,11 @@
 namespace vb {
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn();      // api.cu
 
-constexpr int CL_THREADS = 448;
+constexpr int CL_THREADS = 576;
 constexpr int CL_A_BYTES = 128 * 128;       // 128 positions x 32 channels
 constexpr int CL_MAX_STAGES = 7;
-constexpr int CL_EPI_WARPS = 8;
-constexpr int CL_EPI_BYTES = CL_EPI_WARPS * 4096;      // a 32 x 32 transpose per epilogue warp
+constexpr int CL_EPI_WARPS = 12;
+constexpr int CL_EPI_BYTES = CL_EPI_WARPS * 2048;      // a transpose of 32 rows x 16 columns per epilogue warp
 
 struct ClConvParams {
   const uint8_t* w;          // [tap * kb][hi | lo][n_pad][32], rows swizzled
@@ -76,15 +77,11 @@ __device__ __forceinline__ void umma_tf32_ta(uint32_t d_tmem, uint32_t a_tmem, u
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const float (&v)[32]) {
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const float (&v)[16]) {
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
       ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
-        "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]), "f"(v[16]), "f"(v[17]), "f"(v[18]), "f"(v[19]),
-        "f"(v[20]), "f"(v[21]), "f"(v[22]), "f"(v[23]), "f"(v[24]), "f"(v[25]), "f"(v[26]), "f"(v[27]), "f"(v[28]), "f"(v[29]),
-        "f"(v[30]), "f"(v[31])
+        "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
       : "memory");
 }
 
@@ -103,6 +100,20 @@ __device__ __forceinline__ float cl_sin_sq(float x) {
   const float sn = fmaf(r * u, q, r);
   return sn * sn;
 }
+// ELU without a branch: e^x - 1 = 2^n (e^r - 1) + (2^n - 1) with x = n ln 2 + r, |r| <= ln 2 / 2, and e^r - 1 = r + r^2 Q(r) with a
+// fitted polynomial of degree 4.  Largest relative error against 64 bits 8.7e-8 over [-90, 0].
+__device__ __forceinline__ float cl_elu(float v) {
+  const float x = fmaxf(v, -80.f);
+  const float t = fmaf(x, 1.44269504f, 12582912.f), n = t - 12582912.f;        // n in the low bits of t as well
+  float r = fmaf(n, -0.693359375f, x);
+  r = fmaf(n, 2.12194440e-4f, r);
+  float q = fmaf(r, 0.0013882514f, 0.0083665475f);
+  q = fmaf(q, r, 0.0416672f);
+  q = fmaf(q, r, 0.16666543f);
+  q = fmaf(q, r, 0.49999997f);
+  const float e = fmaf(r * r, q, r), s = __uint_as_float((__float_as_uint(t) << 23) + 0x3f800000u);
+  return v <= 0.f ? fmaf(s, e, s - 1.f) : v;
+}
 struct ClUnit {
   int n0, n_cur, t0, b0;
 };
@@ -117,7 +128,8 @@ __device__ __forceinline__ ClUnit cl_unit(const ClConvParams& p, int u) {
   return r;
 }
 
-__global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvParams p, const __grid_constant__ CUtensorMap x_map) {
+// (96 registers a thread: what the epilogue needs.  Spilled registers go to a first-level cache that the stages leave 28 KB)
+__global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, const __grid_constant__ CUtensorMap x_map) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int stage_bytes = CL_A_BYTES + p.nt * 256;
@@ -128,6 +140,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
   uint64_t* acc_full = empty + CL_MAX_STAGES;    // [2]
   uint64_t* acc_empty = acc_full + 2;            // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  int4* row_tab = reinterpret_cast<int4*>(smem + p.stages * stage_bytes + CL_EPI_BYTES + 512);     // [128]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   BoundedWait bw;
 
@@ -147,6 +160,13 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
   if (warp == 1) {
     tmem_alloc(tmem_slot, p.tmem_cols);
     tmem_relinquish();
+  }
+  // tile row -> (batch entry << 16 | position) inside a tile, and where it lies from the tile's first row on in the output and in the
+  // residual: the same for every tile (32-bit offsets, the host keeps a launch below 2^31 elements)
+  if (warp >= 6 && warp < 10) {
+    const int r = (warp - 6) * 32 + lane, bb = r / p.nr, tt = r - bb * p.nr;
+    row_tab[r] = make_int4(bb < p.nb ? (bb << 16) | tt : -1, bb * static_cast<int>(p.y_bstride) + tt * p.ldy,
+                           bb * static_cast<int>(p.r_bstride) + tt * p.ldr, 0);
   }
   tc_fence_before();
   __syncthreads();
@@ -253,20 +273,23 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
         bw.wait(&full[s], ph);
         if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
         const uint8_t* src = smem + s * stage_bytes + row * 128;
-        float hi[32], lo[32];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const float4 v = *reinterpret_cast<const float4*>(src + ((c ^ (row & 7)) << 4));
-          const float x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            hi[4 * c + e] = tf32_rna(x[e]);
-            lo[4 * c + e] = tf32_rna(x[e] - hi[4 * c + e]);
-          }
-        }
         const uint32_t t = a_col0 + s * 64 + (static_cast<uint32_t>(quarter * 32) << 16);
-        tmem_st_32x32(t, hi);
-        tmem_st_32x32(t + 32, lo);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          float hi[16], lo[16];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const float4 v = *reinterpret_cast<const float4*>(src + (((half * 4 + c) ^ (row & 7)) << 4));
+            const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              hi[4 * c + e] = tf32_rna(x[e]);
+              lo[4 * c + e] = tf32_rna(x[e] - hi[4 * c + e]);
+            }
+          }
+          tmem_st_32x16(t + 16 * half, hi);
+          tmem_st_32x16(t + 32 + 16 * half, lo);
+        }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
         __syncwarp();
@@ -276,47 +299,41 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
     }
   } else {
     // ================= epilogue =================
-    // Two warps per TMEM quarter take alternate 32-column chunks.  A lane holds 32 columns of one row, so bias, activation and
-    // residual are 32 independent chains; with four columns at a time and one warp per scheduler the activations alone took
-    // 46 us per 128 x 128 tile.  Rows leave (and residuals come) through a 32 x 32 transpose: 128-byte runs per row.
-    const int quarter = warp & 3, half = (warp - 6) >> 2;
-    float* st = epi_sm + (warp - 6) * 1024;
-    float4* my_row = reinterpret_cast<float4*>(st + lane * 32);
-    const int cq = lane & 7, rq = lane >> 3, sw = lane & 7;      // transposed side: 16-byte chunk cq of rows rq, rq + 4, ...
-    // rows rq, rq + 4, ... of the quarter -> (batch entry, position) inside a tile, and where they lie from the tile's first row on
-    // (the same for every tile; 32-bit offsets, the host keeps a launch below 2^31 elements)
-    int bt[8], yrel[8], rrel[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = quarter * 32 + i * 4 + rq, bb = r / p.nr, tt = r - bb * p.nr;
-      bt[i] = bb < p.nb ? (bb << 16) | tt : -1;
-      yrel[i] = bb * static_cast<int>(p.y_bstride) + tt * p.ldy + cq * 4;
-      rrel[i] = bb * static_cast<int>(p.r_bstride) + tt * p.ldr + cq * 4;
-    }
-    int it = 0;
+    // Three warps per TMEM quarter take 16-column chunks in turn.  A lane holds 16 columns of one row, so bias, activation and
+    // residual are 16 independent chains, and three warps per scheduler hide each other's loads and transposes.  Rows leave (and
+    // residuals come) through a 32 x 16 transpose: 64-byte runs per row.
+    const int quarter = warp & 3, group = (warp - 6) >> 2;
+    float* st = epi_sm + (warp - 6) * 512;
+    float4* my_row = reinterpret_cast<float4*>(st + lane * 16);
+    const int cq = lane & 3, rq = lane >> 2, sw = (lane >> 1) & 3;      // transposed side: 16-byte chunk cq of rows rq, rq + 8, ...
+    const int tq = ((cq ^ (rq >> 1)) << 2) + rq * 16;                   // (rq + 8 i swizzles as rq does)
+    const int4* tab = row_tab + quarter * 32 + rq;               // rows rq, rq + 8, ... of the quarter: tab[0], tab[8], ...
+    int it = 0, turn = group;                                    // first chunk of the unit that is this warp's
     for (int u = blockIdx.x; u < p.units && !bw.dead; u += gridDim.x, ++it) {
       const ClUnit g = cl_unit(p, u);
       const int acc = it & 1;
       uint32_t live = 0;
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        live |= ((bt[i] >= 0 && g.b0 + (bt[i] >> 16) < p.B && g.t0 + (bt[i] & 0xffff) < p.n_hi) ? 1u : 0u) << i;
-      const int y0 = g.b0 * static_cast<int>(p.y_bstride) + g.t0 * p.ldy + g.n0;
-      const int r0 = g.b0 * static_cast<int>(p.r_bstride) + g.t0 * p.ldr + g.n0;
+      for (int i = 0; i < 4; ++i) {
+        const int bt = tab[8 * i].x;
+        live |= ((bt >= 0 && g.b0 + (bt >> 16) < p.B && g.t0 + (bt & 0xffff) < p.n_hi) ? 1u : 0u) << i;
+      }
+      const int y0 = g.b0 * static_cast<int>(p.y_bstride) + g.t0 * p.ldy + g.n0 + cq * 4;
+      const int r0 = g.b0 * static_cast<int>(p.r_bstride) + g.t0 * p.ldr + g.n0 + cq * 4;
       bool first = true;
       float nz = 0.f;
 #pragma unroll 1
-      for (int c0 = (((it & 1) ^ half) << 5); c0 < g.n_cur; c0 += 64) {      // (by unit as well: a 32-column tile has one chunk)
-        const int n0 = g.n0 + c0, nm = n0 % p.cmod;              // 32 columns from a multiple of 32 lie in one group of channels
+      for (int c0 = turn << 4; c0 < g.n_cur; c0 += 48) {
+        const int n0 = g.n0 + c0, nm = n0 % p.cmod;              // 16 columns from a multiple of 16 lie in one group of channels
         // the residual's rows are requested before the accumulator is waited for.  (Its producer is the kernel in front of this
         // one or an earlier one: the first unit waits for it by name, later units follow accumulators that did.)
-        float4 rs[8];
+        float4 rs[4];
         if (p.epi != CE_PLAIN) {
           if (it == 0 && first) pdl_wait();
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
+          for (int i = 0; i < 4; ++i) {
             rs[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live >> i & 1u) rs[i] = __ldcg(reinterpret_cast<const float4*>(p.resid + (r0 + c0 + rrel[i])));
+            if (live >> i & 1u) rs[i] = __ldcg(reinterpret_cast<const float4*>(p.resid + (r0 + c0 + tab[8 * i].z)));
           }
           if (p.epi == CE_NOISE) {
             const int r = quarter * 32 + lane, bb = r / p.nr, nb = g.b0 + bb, t = g.t0 + r - bb * p.nr;
@@ -332,20 +349,17 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
         const uint32_t taddr = tmem_base + acc * p.nt + (static_cast<uint32_t>(quarter * 32) << 16);
         if (p.epi != CE_PLAIN) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int r = i * 4 + rq;
-            *reinterpret_cast<float4*>(st + r * 32 + ((cq ^ (r & 7)) << 2)) = rs[i];
-          }
+          for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(st + i * 128 + tq) = rs[i];
         }
-        uint32_t tv[32];
-        tmem_ld_32x32(taddr + c0, tv);
+        uint32_t tv[16];
+        tmem_ld_32x16(taddr + c0, tv);
         tmem_ld_wait();
-        float v[32];
+        float v[16];
 #pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = __uint_as_float(tv[c]);
+        for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(tv[c]);
         if (p.bias) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
+          for (int c = 0; c < 4; ++c) {
             const float4 q = __ldg(reinterpret_cast<const float4*>(p.bias + nm) + c);
             v[4 * c] += q.x; v[4 * c + 1] += q.y; v[4 * c + 2] += q.z; v[4 * c + 3] += q.w;
           }
@@ -354,16 +368,16 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
           __syncwarp();
           if (p.epi == CE_SCALE_RESID) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
+            for (int c = 0; c < 4; ++c) {
               const float4 q = __ldg(reinterpret_cast<const float4*>(p.scale + n0) + c);
               v[4 * c] *= q.x; v[4 * c + 1] *= q.y; v[4 * c + 2] *= q.z; v[4 * c + 3] *= q.w;
             }
           } else if (p.epi == CE_NOISE) {
 #pragma unroll
-            for (int c = 0; c < 32; ++c) v[c] *= nz;
+            for (int c = 0; c < 16; ++c) v[c] *= nz;
           }
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
+          for (int c = 0; c < 4; ++c) {
             const float4 q = my_row[c ^ sw];
             v[4 * c] += q.x; v[4 * c + 1] += q.y; v[4 * c + 2] += q.z; v[4 * c + 3] += q.w;
           }
@@ -371,14 +385,13 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
         }
         auto store = [&](float* y) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c) my_row[c ^ sw] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+          for (int c = 0; c < 4; ++c) my_row[c ^ sw] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
           __syncwarp();
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int r = i * 4 + rq;
-            const float4 q = *reinterpret_cast<const float4*>(st + r * 32 + ((cq ^ (r & 7)) << 2));
+          for (int i = 0; i < 4; ++i) {
+            const float4 q = *reinterpret_cast<const float4*>(st + i * 128 + tq);
             if (live >> i & 1u)
-              *reinterpret_cast<float4*>(y + (y0 + c0 + yrel[i])) = q;
+              *reinterpret_cast<float4*>(y + (y0 + c0 + tab[8 * i].y)) = q;
           }
           __syncwarp();
         };
@@ -388,13 +401,13 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
           const float4* ia = reinterpret_cast<const float4*>(p.alpha + p.cmod + nm);
           float big = 0.f;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
+          for (int c = 0; c < 4; ++c) {
             const float4 q = __ldg(al + c);
             big = fmaxf(fmaxf(big, fmaxf(fabsf(v[4 * c] * q.x), fabsf(v[4 * c + 1] * q.y))), fmaxf(fabsf(v[4 * c + 2] * q.z), fabsf(v[4 * c + 3] * q.w)));
           }
           if (big <= CL_SIN_MAX) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
+            for (int c = 0; c < 4; ++c) {
               const float4 q = __ldg(al + c), w = __ldg(ia + c);
               v[4 * c] = fmaf(w.x, cl_sin_sq(q.x * v[4 * c]), v[4 * c]);
               v[4 * c + 1] = fmaf(w.y, cl_sin_sq(q.y * v[4 * c + 1]), v[4 * c + 1]);
@@ -403,20 +416,17 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
             }
           } else {
 #pragma unroll
-            for (int c = 0; c < 32; ++c) {
+            for (int c = 0; c < 16; ++c) {
               const float a = __ldg(p.alpha + nm + c), sn = sinf(a * v[c]);
               v[c] = fmaf(__ldg(p.alpha + p.cmod + nm + c), sn * sn, v[c]);
             }
           }
         } else if (p.act == CA_ELU) {
 #pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            const float e = expm1f(v[c]);
-            v[c] = v[c] > 0.f ? v[c] : e;
-          }
+          for (int c = 0; c < 16; ++c) v[c] = cl_elu(v[c]);
         } else if (p.act == CA_GELU) {
 #pragma unroll
-          for (int c = 0; c < 32; ++c) v[c] = 0.5f * v[c] * (1.f + erff(v[c] * 0.70710678118654752f));
+          for (int c = 0; c < 16; ++c) v[c] = 0.5f * v[c] * (1.f + erff(v[c] * 0.70710678118654752f));
         }
         store(p.y2 ? p.y2 : p.y);
       }
@@ -425,6 +435,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) cl_conv_kernel(const ClConvPara
         bw.wait(&acc_full[acc], (it >> 1) & 1);
         if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
       }
+      turn = (turn + 24 - (g.n_cur >> 4)) % 3;                   // the turns go on over the units (a 32-column tile has two chunks)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
@@ -465,7 +476,7 @@ __global__ void __launch_bounds__(256) cl_pack_kernel(float4* __restrict__ dst, 
 // A block owns 64 channels x DW_T positions: the (activated) input rows with their halo are staged once in shared memory, so
 // every element is read and put through its sine once, in 256-byte rows; a thread finishes four channels of DW_T / 16 rows, whose
 // chains interleave (the activation branches once per four values, to the library's sine when an argument is out of range).
-// DW_T 128 and four-wide activations against 64 and one by one: 12 to 30 us a layer -> 4 to 14, SNAC 32 windows 858 -> 733 us.
+// DW_T 128 and four-wide activations against 64 and one by one: 12 to 30 us a layer -> 4 to 14 (SNAC, 32 windows).
 constexpr int DW_T = 128;
 __device__ __forceinline__ float4 cl_snake4(float4 v, const float4& a, const float4& inv) {
   const float4 y = make_float4(a.x * v.x, a.y * v.y, a.z * v.z, a.w * v.w);
@@ -838,7 +849,7 @@ int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, i
   p.y = d_y; p.y2 = d_y2; p.bias = d_bias; p.resid = d_resid; p.scale = d_scale; p.noise = d_noise; p.alpha = d_alpha;
   p.y_bstride = y_bstride; p.r_bstride = r_bstride; p.ldy = N; p.ldr = N; p.noise_ld = noise_ld; p.cmod = cmod;
   p.epi = epilogue; p.act = act; p.B = B; p.n_lo = n_lo; p.n_hi = n_hi; p.ksize = ksize; p.dil = dil; p.N = N; p.n_pad = N;
-  const int stage_bytes = CL_A_BYTES + p.nt * 256, tail = CL_EPI_BYTES + 1024 /*barriers*/ + 1024 /*alignment*/;
+  const int stage_bytes = CL_A_BYTES + p.nt * 256, tail = CL_EPI_BYTES + 512 /*barriers*/ + 2048 /*row table*/ + 1024 /*alignment*/;
   p.stages = min(min(CL_MAX_STAGES, (512 - 2 * p.nt) / 64), (VB_MAX_DYN_SMEM - tail) / stage_bytes);
   p.tmem_cols = 512;
   CUtensorMap map;

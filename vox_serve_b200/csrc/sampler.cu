@@ -76,25 +76,26 @@ __device__ __forceinline__ double philox_uniform(uint64_t seed, uint64_t offset,
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// One thread-block CLUSTER per row.  The row's tokens are spread over S CTAs x 1024 slots x (2 * PAIRS) tokens;
-// after one pass over the logits (+ repetition cache) every token lives on chip -- its 16-bit value key in a
-// register, its fixed-point probability mass in shared memory -- and everything else is on-chip reductions:
+// One thread-block CLUSTER per row.  The row's tokens are spread over S CTAs x 1024 threads x (2 * PAIRS) tokens;
+// after one pass over the logits (+ repetition cache) every token lives on chip -- its 16-bit value key
+// and its bf16 probability in one word of shared memory -- and everything else is on-chip reductions:
 // block tree -> one DSMEM store per peer CTA -> one cluster barrier.  No histogram, no atomics, no second
 // pass over HBM/L2.
 //   max key -> [top-k: 16-step bisection on counts] -> softmax denominator (fp32, fixed summation tree) ->
-//   mass q_i = floor(bf16(p_i) * 2^32) -> [min-p: direct filter] -> draw by inverse CDF in (cta, slot, pair)
+//   mass q_i = floor(bf16(p_i) * 2^32) -> [min-p: direct filter] -> draw by inverse CDF in (cta, thread, pair)
 //   order; top-p by REJECTION: the drawn token j is in the nucleus iff mass{p > p_j} < top_p, otherwise
 //   everything with p <= p_j is discarded and the draw repeats on what is left (acceptance >= top_p per round;
 //   conditional on acceptance the draw is the renormalised nucleus -- the scheme of FlashInfer's sorting-free
 //   sampler, with exact integer masses instead of float partial sums, hence scheduling-independent).
 // ---------------------------------------------------------------------------------------------------------
-// A thread stands for SMP_V of the 1024: 64 registers per thread did not hold 20 key pairs and the loops over them (190 local
-// memory accesses per thread, whose 139 KB did not fit beside the masses in an SM's first-level cache either).
-// 32 rows of 156,940 tokens, top-p: 71 -> 53 us.
-constexpr int SMP_SLOTS = 1024;          // (cta, slot, pair) order of the tokens
-constexpr int SMP_V = 2;
-constexpr int SMP_THREADS = SMP_SLOTS / SMP_V;
-constexpr int SMP_PAIRS = 20;            // 40 tokens per slot: 40960 tokens per CTA, 327680 per 8-CTA cluster
+// A token's word in shared memory holds its key above and, once the softmax is known, its probability (bf16) below; a mass is taken
+// from the probability where it is needed.  Every pass is then a short loop over the thread's pairs: with the keys in registers the
+// passes had to be unrolled forty tokens deep, and reading that code once took longer than running it (top-p, cold: 32 rows of 2,051
+// tokens 61 us against 18 here; 32 rows of 156,940 tokens in a row of calls 53 against 39, and 67 with 1024 threads that spilled).
+// Above that row's 2.3 us of traffic it now spends 16 us on launch, load latency and the largest key, 15 on the two exponentials a
+// token, and 10 on the draws.
+constexpr int SMP_THREADS = 1024;        // (cta, thread, pair) order of the tokens
+constexpr int SMP_PAIRS = 20;            // 40 tokens per thread: 40960 tokens per CTA, 327680 per 8-CTA cluster
 constexpr int SMP_MAX_CLUSTER = 8;
 
 __device__ __forceinline__ void st_dsmem_u64(unsigned long long* local_ptr, uint32_t cta_rank, unsigned long long v) {
@@ -133,9 +134,9 @@ __device__ __forceinline__ unsigned long long smp_reduce(unsigned long long v, S
   if (lane == 0) c.sh[warp] = v;
   __syncthreads();
   if (warp == 0) {
-    unsigned long long x = c.sh[lane & (SMP_THREADS / 32 - 1)];
+    unsigned long long x = c.sh[lane];
 #pragma unroll
-    for (int o = SMP_THREADS / 64; o > 0; o >>= 1) x = smp_op<OP>(x, __shfl_xor_sync(0xffffffffu, x, o));
+    for (int o = 16; o > 0; o >>= 1) x = smp_op<OP>(x, __shfl_xor_sync(0xffffffffu, x, o));
     c.publish(x);
   }
   c.sync();
@@ -144,15 +145,12 @@ __device__ __forceinline__ unsigned long long smp_reduce(unsigned long long v, S
   c.buf ^= 1;
   return r;
 }
-// fp32 sum with a fixed tree over the 1024 slots (xor butterfly inside 32 slots and across them, CTA partials in rank order)
-__device__ __forceinline__ float smp_sum_f32(const float (&v)[SMP_V], SmpCtx& c) {
+// fp32 sum with a fixed tree (xor butterfly inside the warp and across warps, CTA partials in rank order)
+__device__ __forceinline__ float smp_sum_f32(float v, SmpCtx& c) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v = warp_sum(v);
   float* shf = reinterpret_cast<float*>(c.sh);
-#pragma unroll
-  for (int k = 0; k < SMP_V; ++k) {
-    const float x = warp_sum(v[k]);
-    if (lane == 0) shf[warp + k * (SMP_THREADS / 32)] = x;
-  }
+  if (lane == 0) shf[warp] = v;
   __syncthreads();
   if (warp == 0) {
     const float x = warp_sum(shf[lane]);
@@ -174,21 +172,16 @@ __device__ __forceinline__ float smp_ex2(float x) {
   return y;
 }
 
-// Exclusive scan of one u64 per slot, slot order; returns the prefixes, *total = sum.
-__device__ __forceinline__ void smp_excl_scan(const unsigned long long (&v)[SMP_V], unsigned long long (&excl)[SMP_V], unsigned long long* sh,
-                                              unsigned long long* total) {
+// Block-wide exclusive scan of one u64 per thread, thread order; returns exclusive prefix, *total = sum.
+__device__ __forceinline__ unsigned long long block_excl_scan(unsigned long long v, unsigned long long* sh, unsigned long long* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long incl[SMP_V];
+  unsigned long long incl = v;
 #pragma unroll
-  for (int k = 0; k < SMP_V; ++k) {
-    incl[k] = v[k];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long n = __shfl_up_sync(0xffffffffu, incl[k], o);
-      if (lane >= o) incl[k] += n;
-    }
-    if (lane == 31) sh[warp + k * (SMP_THREADS / 32)] = incl[k];
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long n = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += n;
   }
+  if (lane == 31) sh[warp] = incl;
   __syncthreads();
   if (warp == 0) {
     const unsigned long long w = sh[lane];
@@ -202,10 +195,10 @@ __device__ __forceinline__ void smp_excl_scan(const unsigned long long (&v)[SMP_
     if (lane == 31) sh[32] = wi;
   }
   __syncthreads();
-#pragma unroll
-  for (int k = 0; k < SMP_V; ++k) excl[k] = sh[warp + k * (SMP_THREADS / 32)] + incl[k] - v[k];
+  const unsigned long long res = sh[warp] + incl - v;
   *total = sh[32];
   __syncthreads();
+  return res;
 }
 
 // a / b to the nearest, for one divisor of many dividends: quotient by the correctly rounded reciprocal and two corrections by the
@@ -224,27 +217,19 @@ struct SmpDiv {
     return q;
   }
 };
-// a pair of keys as a loop reads it: opaque, or what one loop unpacks of all forty pairs is kept in (then spilled) registers for the next
-__device__ __forceinline__ uint32_t key_load(uint32_t kk) {
-  asm volatile("" : "+r"(kk));
-  return kk;
-}
 // the two keys of a pair of bf16 codes, and back (bf16_key / key_value on both halves at once)
 __device__ __forceinline__ uint32_t key_pair(uint32_t bits) {
   const uint32_t neg = (bits >> 15) & 0x00010001u;
   return bits ^ (0x80008000u | neg * 0x7fffu);
 }
-__device__ __forceinline__ uint32_t key_pair_bits(uint32_t keys) {
-  const uint32_t pos = (keys >> 15) & 0x00010001u;
-  return keys ^ (0xffffffffu - pos * 0x7fffu);
-}
+// a probability (bf16 in the low half of a token's word) as a mass: floor(p 2^32), saturating at 2^32 - 1
+__device__ __forceinline__ uint32_t smp_mass(uint32_t word) { return __float2uint_rz(bf16_lo(word) * 4294967296.f); }
 
 __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SampleParams p, const int npairs) {
-  extern __shared__ uint32_t q_sm[];                 // [2 * npairs][1024] masses (Q32)
+  extern __shared__ uint2 tok_sm[];                  // [npairs][1024] token pairs: (key << 16 | probability) each
   __shared__ unsigned long long xch[2][SMP_MAX_CLUSTER];
-  __shared__ unsigned long long pick[2][2];
+  __shared__ unsigned long long pick[2];
   __shared__ unsigned long long sh[34];
-  static_assert(SMP_V == 2, "the shares of a thread's slots are added in pairs");
   SmpCtx c;
   c.S = gridDim.x; c.rank = blockIdx.x; c.buf = 0; c.xch = xch; c.sh = sh;
   const int S = c.S, rank = c.rank, row = blockIdx.y, tid = threadIdx.x;
@@ -253,11 +238,10 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
   pdl_sync();
 
   // ---- one pass over the row: keys (0 = no token / NaN) ----
-  // Load latency first: ten token pairs of both slots at a time -- one 32-bit load for the two logits, one 16-bit load for their
-  // repetition flags, forty requests in flight together -- and only then finished (penalty, mask, temperature: same operations and
-  // rounding points as token_value()).  Rows whose layout does not allow the paired loads (odd leading dimension / vocabulary,
-  // unaligned base) take the scalar path.
-  uint32_t kk[SMP_V][SMP_PAIRS];
+  // Load latency first: ten token pairs at a time -- one 32-bit load for the two logits, one 16-bit load for their repetition flags,
+  // all in flight together -- and only then finished (penalty, mask, temperature: same operations and rounding points as
+  // token_value()).  Rows whose layout does not allow the paired loads (odd leading dimension / vocabulary, unaligned base) take the
+  // scalar path.  A thread reads back only what it wrote itself.
   const __nv_bfloat16* lrow = p.logits + static_cast<size_t>(row) * p.ld;
   const uint8_t* rep0 = nullptr;
   size_t rep_wstride = 0;
@@ -272,59 +256,54 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
                       ((reinterpret_cast<uintptr_t>(rep0) | rep_wstride) & 1) == 0;
   const int n_seen = rep0 ? p.W : 0;
   const SmpDiv by_penalty(p.penalty), by_temperature(scaled ? p.temperature : 1.f);
-  auto tok_index = [&](int k, int j, int half) { return 2 * ((j * S + rank) * SMP_SLOTS + k * SMP_THREADS + tid) + half; };
-  constexpr int SMP_BATCH = 5;
-#pragma unroll
-  for (int j0 = 0; j0 < SMP_PAIRS; j0 += SMP_BATCH) {
-    uint32_t lw[SMP_V][SMP_BATCH], sb[SMP_V][SMP_BATCH];
+  auto tok_index = [&](int j, int half) { return 2 * ((j * S + rank) * SMP_THREADS + tid) + half; };
+  constexpr int SMP_BATCH = 10;
+  uint32_t kloc = 0u;
+#pragma unroll 1
+  for (int j0 = 0; j0 < npairs; j0 += SMP_BATCH) {
+    uint32_t lw[SMP_BATCH], sb[SMP_BATCH];
     if (paired) {
 #pragma unroll
-      for (int jj = 0; jj < SMP_BATCH; ++jj)
-#pragma unroll
-        for (int k = 0; k < SMP_V; ++k) {
-          const int i0 = tok_index(k, j0 + jj, 0);
-          const bool in = j0 + jj < npairs && i0 < p.vocab;
-          lw[k][jj] = in ? __ldg(reinterpret_cast<const uint32_t*>(lrow + i0)) : 0u;
-          sb[k][jj] = in && n_seen ? __ldg(reinterpret_cast<const unsigned short*>(rep0 + i0)) : 0u;
-        }
+      for (int jj = 0; jj < SMP_BATCH; ++jj) {
+        const int i0 = tok_index(j0 + jj, 0);
+        const bool in = j0 + jj < npairs && i0 < p.vocab;
+        lw[jj] = in ? __ldg(reinterpret_cast<const uint32_t*>(lrow + i0)) : 0u;
+        sb[jj] = in && n_seen ? __ldg(reinterpret_cast<const unsigned short*>(rep0 + i0)) : 0u;
+      }
+#pragma unroll 1
       for (int w = 1; w < n_seen; ++w) {
         const uint8_t* rw = rep0 + w * rep_wstride;
 #pragma unroll
-        for (int jj = 0; jj < SMP_BATCH; ++jj)
-#pragma unroll
-          for (int k = 0; k < SMP_V; ++k) {
-            const int i0 = tok_index(k, j0 + jj, 0);
-            if (j0 + jj < npairs && i0 < p.vocab) sb[k][jj] |= __ldg(reinterpret_cast<const unsigned short*>(rw + i0));
-          }
+        for (int jj = 0; jj < SMP_BATCH; ++jj) {
+          const int i0 = tok_index(j0 + jj, 0);
+          if (j0 + jj < npairs && i0 < p.vocab) sb[jj] |= __ldg(reinterpret_cast<const unsigned short*>(rw + i0));
+        }
       }
     } else {
 #pragma unroll
-      for (int jj = 0; jj < SMP_BATCH; ++jj)
-#pragma unroll
-        for (int k = 0; k < SMP_V; ++k) {
-          const int i0 = tok_index(k, j0 + jj, 0);
-          lw[k][jj] = sb[k][jj] = 0u;
-          if (j0 + jj < npairs && i0 < p.vocab) {
-            const bool two = i0 + 1 < p.vocab;
-            lw[k][jj] = __ldg(reinterpret_cast<const unsigned short*>(lrow + i0));
-            if (two) lw[k][jj] |= static_cast<uint32_t>(__ldg(reinterpret_cast<const unsigned short*>(lrow + i0 + 1))) << 16;
-            for (int w = 0; w < n_seen; ++w) {
-              sb[k][jj] |= __ldg(rep0 + w * rep_wstride + i0);
-              if (two) sb[k][jj] |= static_cast<uint32_t>(__ldg(rep0 + w * rep_wstride + i0 + 1)) << 8;
-            }
+      for (int jj = 0; jj < SMP_BATCH; ++jj) {
+        const int i0 = tok_index(j0 + jj, 0);
+        lw[jj] = sb[jj] = 0u;
+        if (j0 + jj < npairs && i0 < p.vocab) {
+          const bool two = i0 + 1 < p.vocab;
+          lw[jj] = __ldg(reinterpret_cast<const unsigned short*>(lrow + i0));
+          if (two) lw[jj] |= static_cast<uint32_t>(__ldg(reinterpret_cast<const unsigned short*>(lrow + i0 + 1))) << 16;
+          for (int w = 0; w < n_seen; ++w) {
+            sb[jj] |= __ldg(rep0 + w * rep_wstride + i0);
+            if (two) sb[jj] |= static_cast<uint32_t>(__ldg(rep0 + w * rep_wstride + i0 + 1)) << 8;
           }
         }
+      }
     }
 #pragma unroll
-    for (int jj = 0; jj < SMP_BATCH; ++jj)
-#pragma unroll
-      for (int k = 0; k < SMP_V; ++k) {
-        const int i0 = tok_index(k, j0 + jj, 0);
-        float l[2] = {bf16_lo(lw[k][jj]), bf16_hi(lw[k][jj])};
-        if (sb[k][jj]) {
+    for (int jj = 0; jj < SMP_BATCH; ++jj) {
+      if (j0 + jj < npairs) {
+        const int i0 = tok_index(j0 + jj, 0);
+        float l[2] = {bf16_lo(lw[jj]), bf16_hi(lw[jj])};
+        if (sb[jj]) {
 #pragma unroll
           for (int h = 0; h < 2; ++h)
-            if (sb[k][jj] >> (8 * h) & 0xffu) l[h] = round_bf16(l[h] > 0.f ? by_penalty(l[h]) : l[h] * p.penalty);   // sampling.py:143-144
+            if (sb[jj] >> (8 * h) & 0xffu) l[h] = round_bf16(l[h] > 0.f ? by_penalty(l[h]) : l[h] * p.penalty);   // sampling.py:143-144
         }
         if ((i0 ^ p.mask_token) >> 1 == 0) {
           if (p.mask_token & 1) l[1] = -INFINITY; else l[0] = -INFINITY;
@@ -334,35 +313,28 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
           l[1] = by_temperature(l[1]);
         }
         uint32_t keep = 0u;
-        if (j0 + jj < npairs && i0 < p.vocab) {
+        if (i0 < p.vocab) {
           if (l[0] == l[0]) keep = 0xffffu;
           if (i0 + 1 < p.vocab && l[1] == l[1]) keep |= 0xffff0000u;
         }
-        kk[k][j0 + jj] = key_pair(pack_bf16(l[0], l[1])) & keep;
+        const uint32_t keys = key_pair(pack_bf16(l[0], l[1])) & keep;
+        tok_sm[(j0 + jj) * SMP_THREADS + tid] = make_uint2(keys << 16, keys & 0xffff0000u);
+        kloc = max(kloc, max(keys & 0xffffu, keys >> 16));
       }
+    }
   }
 
   // ---- max key ----
-  uint32_t kloc = 0u;
-#pragma unroll
-  for (int k = 0; k < SMP_V; ++k)
-#pragma unroll
-    for (int j = 0; j < SMP_PAIRS; ++j) {
-      const uint32_t v = key_load(kk[k][j]);
-      kloc = max(kloc, max(v & 0xffffu, v >> 16));
-    }
   const uint32_t kmax = static_cast<uint32_t>(smp_reduce<SMP_MAX>(kloc, c));
   // smallest index holding the max key: the greedy answer and the fallback of degenerate rows
   auto first_max_index = [&]() -> unsigned long long {
     unsigned long long best = 0xffffffffull;
-#pragma unroll
-    for (int j = SMP_PAIRS - 1; j >= 0; --j)
-#pragma unroll
-      for (int k = SMP_V - 1; k >= 0; --k) {
-        const uint32_t v = key_load(kk[k][j]);
-        if ((v >> 16) == kmax) best = static_cast<unsigned long long>(tok_index(k, j, 1));
-        if ((v & 0xffffu) == kmax) best = static_cast<unsigned long long>(tok_index(k, j, 0));
-      }
+#pragma unroll 4
+    for (int j = npairs - 1; j >= 0; --j) {
+      const uint2 t = tok_sm[j * SMP_THREADS + tid];
+      if ((t.y >> 16) == kmax) best = static_cast<unsigned long long>(tok_index(j, 1));
+      if ((t.x >> 16) == kmax) best = static_cast<unsigned long long>(tok_index(j, 0));
+    }
     const unsigned long long r = smp_reduce<SMP_MIN>(kmax ? best : 0xffffffffull, c);
     return r == 0xffffffffull ? 0ull : r;
   };
@@ -377,16 +349,15 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
   if (p.strategy == 1 || p.strategy == 3) {
     uint32_t lo = 0u, hi = 65535u;          // invariant: count(> hi) < top_k; count(> lo - 1) >= top_k or lo == 0
     // bisection over [0, 65535] for the smallest k with count(> k) < top_k
+#pragma unroll 1
     while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
+      const uint32_t mid = (lo + hi) >> 1, lim = mid << 16 | 0xffffu;      // (no probabilities yet: the low halves are zero)
       uint32_t cnt = 0u;
-#pragma unroll
-      for (int k = 0; k < SMP_V; ++k)
-#pragma unroll
-        for (int j = 0; j < SMP_PAIRS; ++j) {
-          const uint32_t v = key_load(kk[k][j]);
-          cnt += ((v & 0xffffu) > mid ? 1u : 0u) + ((v >> 16) > mid ? 1u : 0u);
-        }
+#pragma unroll 4
+      for (int j = 0; j < npairs; ++j) {
+        const uint2 t = tok_sm[j * SMP_THREADS + tid];
+        cnt += (t.x > lim ? 1u : 0u) + (t.y > lim ? 1u : 0u);
+      }
       const unsigned long long tot = smp_reduce<SMP_SUM>(cnt, c);
       if (tot < static_cast<unsigned long long>(p.top_k)) hi = mid; else lo = mid + 1;
     }
@@ -396,47 +367,36 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
 
   // ---- softmax denominator (fp32) ----
   const float xmax = key_value(kmax);
-  float zpart[SMP_V];
-#pragma unroll
-  for (int k = 0; k < SMP_V; ++k) {
-    zpart[k] = 0.f;
-#pragma unroll
-    for (int j = 0; j < SMP_PAIRS; ++j) {
-      const uint32_t v = key_load(kk[k][j]), a = v & 0xffffu, b = v >> 16, bits = key_pair_bits(v);
-      if (a != 0u && a >= z_floor) zpart[k] += smp_ex2((bf16_lo(bits) - xmax) * kLog2e);
-      if (b != 0u && b >= z_floor) zpart[k] += smp_ex2((bf16_hi(bits) - xmax) * kLog2e);
-    }
+  float zpart = 0.f;
+#pragma unroll 4
+  for (int j = 0; j < npairs; ++j) {
+    const uint2 t = tok_sm[j * SMP_THREADS + tid];
+    const uint32_t a = t.x >> 16, b = t.y >> 16;
+    if (a != 0u && a >= z_floor) zpart += smp_ex2((key_value(a) - xmax) * kLog2e);
+    if (b != 0u && b >= z_floor) zpart += smp_ex2((key_value(b) - xmax) * kLog2e);
   }
   const float Z = smp_sum_f32(zpart, c);
   const float log2Z = log2f(Z);
 
-  // ---- masses: bf16-rounded softmax output as Q32 fixed point; filtered tokens get 0 ----
+  // ---- probabilities: bf16-rounded softmax output; filtered tokens get 0 ----
   const uint32_t keep_floor = (p.strategy == 1 || p.strategy == 3) ? k_floor : 0u;
   const float minp_thr = (p.strategy == 4) ? p.min_p * round_bf16(smp_ex2(-log2Z)) : 0.f;
-  unsigned long long mine[SMP_V];           // this slot's share of the candidates
-#pragma unroll
-  for (int k = 0; k < SMP_V; ++k) {
-    mine[k] = 0ull;
-#pragma unroll
-    for (int j = 0; j < SMP_PAIRS; ++j) {
-      if (j < npairs) {
-        const uint32_t v = key_load(kk[k][j]), bits = key_pair_bits(v);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const uint32_t key = h ? (v >> 16) : (v & 0xffffu);
-          uint32_t q = 0u;
-          if (key != 0u && key >= z_floor && key >= keep_floor) {
-            // softmax output e^(x - max) / Z as ONE exponential: 2^((x - max) log2 e - log2 Z)
-            const float pr = round_bf16(smp_ex2(((h ? bf16_hi(bits) : bf16_lo(bits)) - xmax) * kLog2e - log2Z));
-            if (pr >= minp_thr) q = __float2uint_rz(pr * 4294967296.f);   // saturates at 2^32 - 1
-          }
-          q_sm[(2 * j + h) * SMP_SLOTS + k * SMP_THREADS + tid] = q;
-          mine[k] += q;
-        }
-      }
-    }
+  auto probability = [&](uint32_t k) -> uint32_t {
+    // softmax output e^(x - max) / Z as ONE exponential: 2^((x - max) log2 e - log2 Z)
+    const float pr = round_bf16(smp_ex2((key_value(k) - xmax) * kLog2e - log2Z));
+    return k != 0u && k >= z_floor && k >= keep_floor && pr >= minp_thr ? __float_as_uint(pr) >> 16 : 0u;
+  };
+  unsigned long long mine = 0ull;           // this thread's share of the candidates' mass
+#pragma unroll 4
+  for (int j = 0; j < npairs; ++j) {
+    uint2 t = tok_sm[j * SMP_THREADS + tid];
+    t.x |= probability(t.x >> 16);
+    t.y |= probability(t.y >> 16);
+    tok_sm[j * SMP_THREADS + tid] = t;
+    mine += smp_mass(t.x);
+    mine += smp_mass(t.y);
   }
-  unsigned long long Mc = smp_reduce<SMP_SUM>(mine[0] + mine[1], c);   // mass of the current candidate set
+  unsigned long long Mc = smp_reduce<SMP_SUM>(mine, c);   // mass of the current candidate set
   const uint64_t seed = p.rng_state ? p.rng_state[0] : p.seed;
   const uint64_t offset = p.rng_state ? p.rng_state[1] : p.offset;
   if (Mc == 0ull || !(Z > 0.f)) {
@@ -450,10 +410,11 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
     uint32_t pivot = 0u;                     // candidates: key > pivot
     int pb = 0;
     unsigned long long result = 0ull;
+#pragma unroll 1
     for (uint32_t round = 0; round < 64u; ++round) {
-      // inverse CDF over the candidates in (cta, thread, slot) order
-      unsigned long long cta_total, excl[SMP_V];
-      smp_excl_scan(mine, excl, sh, &cta_total);
+      // inverse CDF over the candidates in (cta, thread, pair) order
+      unsigned long long cta_total;
+      const unsigned long long excl = block_excl_scan(mine, sh, &cta_total);
       if (tid < 32) c.publish(cta_total);
       c.sync();
       unsigned long long base = 0ull;
@@ -462,53 +423,41 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
       const double u = philox_uniform(seed, offset, static_cast<uint32_t>(row), round);
       unsigned long long target = static_cast<unsigned long long>(u * static_cast<double>(Mc));
       if (target >= Mc) target = Mc - 1;
-#pragma unroll
-      for (int k = 0; k < SMP_V; ++k) {
-        const unsigned long long lo = base + excl[k];
-        if (mine[k] != 0ull && lo <= target && target < lo + mine[k]) {
-          unsigned long long run = lo;
-          unsigned long long found = 0ull;
-          bool done = false;
-#pragma unroll
-          for (int j = 0; j < SMP_PAIRS; ++j) {
-            if (j < npairs) {
-              const uint32_t v = key_load(kk[k][j]);
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const uint32_t key = h ? (v >> 16) : (v & 0xffffu);
-                if (!done && key > pivot) {
-                  const unsigned long long q = q_sm[(2 * j + h) * SMP_SLOTS + k * SMP_THREADS + tid];
-                  if (target < run + q) {
-                    found = (static_cast<unsigned long long>(key) << 32) | static_cast<uint32_t>(tok_index(k, j, h));
-                    done = true;
-                  }
-                  run += q;
-                }
-              }
-            }
+      const unsigned long long lo = base + excl;
+      if (mine != 0ull && lo <= target && target < lo + mine) {
+        unsigned long long run = lo;
+        unsigned long long found = 0ull;
+#pragma unroll 1
+        for (int j = 0; j < npairs; ++j) {
+          const uint2 t = tok_sm[j * SMP_THREADS + tid];
+          const uint32_t qx = (t.x >> 16) > pivot ? smp_mass(t.x) : 0u, qy = (t.y >> 16) > pivot ? smp_mass(t.y) : 0u;
+          if (target < run + qx) {
+            found = (static_cast<unsigned long long>(t.x >> 16) << 32) | static_cast<uint32_t>(tok_index(j, 0));
+            break;
           }
-          if (S == 1) pick[pb][0] = found;
-          else for (int r = 0; r < S; ++r) st_dsmem_u64(&pick[pb][0], r, found);
+          run += qx;
+          if (target < run + qy) {
+            found = (static_cast<unsigned long long>(t.y >> 16) << 32) | static_cast<uint32_t>(tok_index(j, 1));
+            break;
+          }
+          run += qy;
         }
+        if (S == 1) pick[pb] = found;
+        else for (int r = 0; r < S; ++r) st_dsmem_u64(&pick[pb], r, found);
       }
       c.sync();
-      result = pick[pb][0];
+      result = pick[pb];
       pb ^= 1;
       if (!nucleus) break;
       const uint32_t kj = static_cast<uint32_t>(result >> 32);
-#pragma unroll
-      for (int k = 0; k < SMP_V; ++k) {
-        mine[k] = 0ull;                      // what lies above j: the slot's share of the next round, should there be one
-#pragma unroll
-        for (int j = 0; j < SMP_PAIRS; ++j) {
-          if (j < npairs) {
-            const uint32_t v = key_load(kk[k][j]);
-            if ((v & 0xffffu) > kj) mine[k] += q_sm[(2 * j) * SMP_SLOTS + k * SMP_THREADS + tid];
-            if ((v >> 16) > kj) mine[k] += q_sm[(2 * j + 1) * SMP_SLOTS + k * SMP_THREADS + tid];
-          }
-        }
+      mine = 0ull;                           // what lies above j: this thread's share of the next round, should there be one
+#pragma unroll 4
+      for (int j = 0; j < npairs; ++j) {
+        const uint2 t = tok_sm[j * SMP_THREADS + tid];
+        if ((t.x >> 16) > kj) mine += smp_mass(t.x);
+        if ((t.y >> 16) > kj) mine += smp_mass(t.y);
       }
-      const unsigned long long above = smp_reduce<SMP_SUM>(mine[0] + mine[1], c);
+      const unsigned long long above = smp_reduce<SMP_SUM>(mine, c);
       if (above < P) break;                  // j is inside the nucleus: accept
       pivot = kj;                            // nothing with p <= p_j is: drop it and redraw
       Mc = above;
@@ -666,16 +615,16 @@ int vb_sample(int64_t* d_out_ids, const void* d_logits, int rows, int vocab, int
               d_workspace, d_rng_state, d_cache_rows);
   // smallest cluster (1, 2, 4 or 8 CTAs) whose threads can hold the row on chip
   int S = 1;
-  while (S < SMP_MAX_CLUSTER && static_cast<long long>(S) * SMP_SLOTS * 2 * SMP_PAIRS < vocab) S <<= 1;
-  VB_CHECK_ARG(static_cast<long long>(S) * SMP_SLOTS * 2 * SMP_PAIRS >= vocab,
+  while (S < SMP_MAX_CLUSTER && static_cast<long long>(S) * SMP_THREADS * 2 * SMP_PAIRS < vocab) S <<= 1;
+  VB_CHECK_ARG(static_cast<long long>(S) * SMP_THREADS * 2 * SMP_PAIRS >= vocab,
                "vb_sample: vocab %d exceeds the %d tokens one cluster holds on chip", vocab,
-               SMP_MAX_CLUSTER * SMP_SLOTS * 2 * SMP_PAIRS);
+               SMP_MAX_CLUSTER * SMP_THREADS * 2 * SMP_PAIRS);
   VB_CHECK_ARG(rows <= 65535, "vb_sample: %d rows exceed the grid limit (65535)", rows);
-  const int npairs = (vocab + S * SMP_SLOTS * 2 - 1) / (S * SMP_SLOTS * 2);
-  const size_t smem = static_cast<size_t>(2 * npairs) * SMP_SLOTS * sizeof(uint32_t);
+  const int npairs = (vocab + S * SMP_THREADS * 2 - 1) / (S * SMP_THREADS * 2);
+  const size_t smem = static_cast<size_t>(2 * npairs) * SMP_THREADS * sizeof(uint32_t);
   // (static shared memory counts against the same 227 KiB: leave room for it)
   VB_CHECK_CUDA(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     2 * SMP_PAIRS * SMP_SLOTS * static_cast<int>(sizeof(uint32_t))));
+                                     2 * SMP_PAIRS * SMP_THREADS * static_cast<int>(sizeof(uint32_t))));
   VB_LAUNCH_PDL_CLUSTER(sample_kernel, dim3(S, rows), SMP_THREADS, smem, st, S, p, npairs);
   return 0;
 }

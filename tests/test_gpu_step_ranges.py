@@ -286,3 +286,14 @@ def test_sampler_quotients(ops, penalty):
         mark = torch.zeros(n, 1, 1, 2, dtype=torch.bool, device="cuda")
         mark[..., first] = True
         assert (ops.sample(pair, "greedy", rep_cache=mark, penalty=penalty) == 0).all()
+
+
+@pytest.mark.parametrize("rows,dim,tiled", [(1, 8, False), (3, 2040, False), (33, 2056, True), (1, 3072, True), (2, 8192, False), (2, 8200, False)])
+def test_rmsnorm_rows(ops, rows, dim, tiled):
+    """Rows on 16-byte boundaries against the same rows with weights that are not, which take the general kernel."""
+    g = torch.Generator("cuda").manual_seed(dim)
+    x = torch.randn(rows, dim, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(dim + 1, generator=g, device="cuda").to(torch.bfloat16)
+    out = ops.TiledAct(rows, dim, torch.device("cuda")) if tiled else None
+    got = ops.rmsnorm(x, w[1:].clone(), 1e-5, out=out)
+    assert torch.equal(got.to_rows() if tiled else got, ops.rmsnorm(x, w[1:], 1e-5))

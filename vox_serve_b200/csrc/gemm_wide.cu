@@ -90,6 +90,28 @@ __device__ __forceinline__ float gw_act(float v, int act) {
   return v;
 }
 
+// a / d to the nearest, eight at a time and d >= 1: reciprocal, one Newton step, quotient, one correction by the exact remainder (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34, 1990).  No branch between the eight; where
+// a divisor is near overflow all of them take the division itself.
+__device__ __forceinline__ void gw_div8(float (&a)[8], const float (&d)[8]) {
+  float far = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) far = fmaxf(far, d[i]);
+  if (far < 0x1p120f) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float y;
+      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d[i]));
+      y = fmaf(fmaf(-d[i], y, 1.f), y, y);
+      const float q = a[i] * y, m = fabsf(a[i]);
+      a[i] = m > 0x1p-90f && m < 0x1p120f ? fmaf(fmaf(-q, d[i], a[i]), y, q) : q;      // (zeros and infinities are right as they are)
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = a[i] / d[i];
+  }
+}
+
 struct GwUnit {
   int split, pair, tblk, kb0, kb1, t0, n_cur;    // n_cur: token rows of the tile rounded up to 16
 };
@@ -350,8 +372,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
             for (int i = 0; i < 8; ++i) {
               gt[i] = fminf(gt[i], p.glu_limit);
               up[i] = fminf(fmaxf(up[i], -p.glu_limit), p.glu_limit);
-              o[i] = __fdividef(gt[i], 1.0f + expf(-p.glu_slope * gt[i])) * (up[i] + 1.0f);
+              o[i] = 1.0f + expf(-p.glu_slope * gt[i]);
             }
+            gw_div8(gt, o);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = gt[i] * (up[i] + 1.0f);
           } else if (p.act == 1) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) o[i] = gw_act(gt[i], 1) * up[i];
@@ -365,8 +390,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               gt[i] = round_bf16(gt[i]);
-              o[i] = round_bf16(__fdividef(gt[i], 1.0f + expf(-gt[i]))) * round_bf16(up[i]);
+              o[i] = 1.0f + expf(-gt[i]);
             }
+            gw_div8(gt, o);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = round_bf16(gt[i]) * round_bf16(up[i]);
           }
           const int lim = live ? p.T - tc : 0;
 #pragma unroll

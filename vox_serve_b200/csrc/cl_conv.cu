@@ -21,7 +21,7 @@
 // has 5 x 4 tiles of 128.
 // What bounds it: wide layers of few positions are one chain of 32-deep k-blocks (0.41 us each, the split into halves), narrow
 // layers of many positions the epilogue (1x1 with residual, 614400 positions of 64 channels: 393 MB in 126 us).
-// Measured (one pass): SNAC 32 windows 1454 us channel-first, 647 here; 1 window 711 and 266; Mimi 32 chunks 6721 and 1933.
+// Measured (one pass): SNAC 32 windows 1454 us channel-first, 623 here; 1 window 711 and 262; Mimi 32 chunks 6721 and 1881.
 // Of that, the residual's rows asked for before the accumulator is waited for: Mimi 2499 -> 2407; 16 columns at a time on twelve warps
 // without a spilled register, where 32 on eight spilled 53: Mimi 2403 -> 1933, SNAC 746 -> 647 and 313 -> 266.
 #include "../../include/vb_api.h"
@@ -51,6 +51,7 @@ struct ClConvParams {
   int ldy, ldr, noise_ld, cmod, epi, act;
   int B, n_lo, n_hi, ksize, dil, N, n_pad, kb_per_tap, ksteps;
   int nt, n_tiles, nr, nb, t_tiles, units, stages, tmem_cols;
+  int acc_cols;              // TMEM columns of an accumulator: nt, or 2 nt where the two halves of the weights have their own
 };
 enum ClEpi { CE_PLAIN = 0, CE_RESID = 1, CE_SCALE_RESID = 2, CE_NOISE = 3 };
 enum ClAct { CA_NONE = 0, CA_SNAKE = 1, CA_ELU = 2, CA_GELU = 3 };
@@ -114,6 +115,16 @@ __device__ __forceinline__ float cl_elu(float v) {
   const float e = fmaf(r * r, q, r), s = __uint_as_float((__float_as_uint(t) << 23) + 0x3f800000u);
   return v <= 0.f ? fmaf(s, e, s - 1.f) : v;
 }
+__device__ __forceinline__ float4 cl_snake4(float4 v, const float4& a, const float4& inv) {
+  const float4 y = make_float4(a.x * v.x, a.y * v.y, a.z * v.z, a.w * v.w);
+  const float big = fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w)));
+  float4 s = make_float4(cl_sin_sq(y.x), cl_sin_sq(y.y), cl_sin_sq(y.z), cl_sin_sq(y.w));
+  if (!(big <= CL_SIN_MAX)) {
+    const float4 t = make_float4(sinf(y.x), sinf(y.y), sinf(y.z), sinf(y.w));
+    s = make_float4(t.x * t.x, t.y * t.y, t.z * t.z, t.w * t.w);
+  }
+  return make_float4(fmaf(inv.x, s.x, v.x), fmaf(inv.y, s.y, v.y), fmaf(inv.z, s.z, v.z), fmaf(inv.w, s.w, v.w));
+}
 struct ClUnit {
   int n0, n_cur, t0, b0;
 };
@@ -172,7 +183,7 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t a_col0 = tmem_base + 2 * p.nt;    // stage s: hi at + 64 s, lo at + 64 s + 32
+  const uint32_t a_col0 = tmem_base + 2 * p.acc_cols;    // stage s: hi at + 64 s, lo at + 64 s + 32
 
   if (warp == 0) {
     // ================= copies =================
@@ -241,7 +252,7 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
       bw.wait(&acc_empty[acc], ((it >> 1) & 1) ^ 1);
       if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
       tc_fence_after();
-      const uint32_t d = tmem_base + acc * p.nt, idesc = umma_idesc(128, g.n_cur, 2u);
+      const uint32_t d = tmem_base + acc * p.acc_cols, idesc = umma_idesc(128, g.n_cur, 2u), idesc2 = umma_idesc(128, 2 * g.n_cur, 2u);
       for (int i = 0; i < p.ksteps; ++i) {
         bw.wait(&full[s], ph);
         bw.wait(&ready[s], ph);
@@ -250,6 +261,16 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
         const uint64_t b_hi = desc0 + static_cast<uint64_t>(s) * (stage_bytes >> 4), b_lo = b_hi + ((g.n_cur * 128) >> 4);
         const uint32_t a_hi = a_col0 + s * 64, a_lo = a_hi + 32;
         if (elect_one()) {
+          if (p.acc_cols != p.nt) {
+            // narrow tiles, where an instruction costs more than its columns: hi_x times both halves of the weights (they lie one
+            // behind the other) in one instruction, hi_w hi_x and lo_w hi_x in accumulators of their own: Mimi 1929 -> 1881 us, SNAC 32
+            // windows 638 -> 623, and a third off the error against 64 bits (tiles of 128 leave no TMEM for it)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              umma_tf32_ta(d, a_hi + 8 * k, b_hi + 2 * k, idesc2, (i > 0 || k > 0) ? 1u : 0u);
+              umma_tf32_ta(d, a_lo + 8 * k, b_hi + 2 * k, idesc, 1u);
+            }
+          } else
 #pragma unroll
           for (int k = 0; k < 4; ++k) {                      // small terms first
             umma_tf32_ta(d, a_lo + 8 * k, b_hi + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
@@ -318,8 +339,8 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
         const int bt = tab[8 * i].x;
         live |= ((bt >= 0 && g.b0 + (bt >> 16) < p.B && g.t0 + (bt & 0xffff) < p.n_hi) ? 1u : 0u) << i;
       }
-      const int y0 = g.b0 * static_cast<int>(p.y_bstride) + g.t0 * p.ldy + g.n0 + cq * 4;
-      const int r0 = g.b0 * static_cast<int>(p.r_bstride) + g.t0 * p.ldr + g.n0 + cq * 4;
+      const int y0 = g.b0 * static_cast<int>(p.y_bstride) + (g.t0 - p.n_lo) * p.ldy + g.n0 + cq * 4;
+      const int r0 = g.b0 * static_cast<int>(p.r_bstride) + (g.t0 - p.n_lo) * p.ldr + g.n0 + cq * 4;
       bool first = true;
       float nz = 0.f;
 #pragma unroll 1
@@ -346,7 +367,7 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
           tc_fence_after();
           first = false;
         }
-        const uint32_t taddr = tmem_base + acc * p.nt + (static_cast<uint32_t>(quarter * 32) << 16);
+        const uint32_t taddr = tmem_base + acc * p.acc_cols + (static_cast<uint32_t>(quarter * 32) << 16);
         if (p.epi != CE_PLAIN) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(st + i * 128 + tq) = rs[i];
@@ -357,6 +378,12 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
         float v[16];
 #pragma unroll
         for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(tv[c]);
+        if (p.acc_cols != p.nt) {
+          tmem_ld_32x16(taddr + g.n_cur + c0, tv);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < 16; ++c) v[c] += __uint_as_float(tv[c]);
+        }
         if (p.bias) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
@@ -399,27 +426,10 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
         if (p.act == CA_SNAKE) {
           const float4* al = reinterpret_cast<const float4*>(p.alpha + nm);
           const float4* ia = reinterpret_cast<const float4*>(p.alpha + p.cmod + nm);
-          float big = 0.f;
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const float4 q = __ldg(al + c);
-            big = fmaxf(fmaxf(big, fmaxf(fabsf(v[4 * c] * q.x), fabsf(v[4 * c + 1] * q.y))), fmaxf(fabsf(v[4 * c + 2] * q.z), fabsf(v[4 * c + 3] * q.w)));
-          }
-          if (big <= CL_SIN_MAX) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const float4 q = __ldg(al + c), w = __ldg(ia + c);
-              v[4 * c] = fmaf(w.x, cl_sin_sq(q.x * v[4 * c]), v[4 * c]);
-              v[4 * c + 1] = fmaf(w.y, cl_sin_sq(q.y * v[4 * c + 1]), v[4 * c + 1]);
-              v[4 * c + 2] = fmaf(w.z, cl_sin_sq(q.z * v[4 * c + 2]), v[4 * c + 2]);
-              v[4 * c + 3] = fmaf(w.w, cl_sin_sq(q.w * v[4 * c + 3]), v[4 * c + 3]);
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-              const float a = __ldg(p.alpha + nm + c), sn = sinf(a * v[c]);
-              v[c] = fmaf(__ldg(p.alpha + p.cmod + nm + c), sn * sn, v[c]);
-            }
+            const float4 o = cl_snake4(make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]), __ldg(al + c), __ldg(ia + c));
+            v[4 * c] = o.x; v[4 * c + 1] = o.y; v[4 * c + 2] = o.z; v[4 * c + 3] = o.w;
           }
         } else if (p.act == CA_ELU) {
 #pragma unroll
@@ -478,16 +488,6 @@ __global__ void __launch_bounds__(256) cl_pack_kernel(float4* __restrict__ dst, 
 // chains interleave (the activation branches once per four values, to the library's sine when an argument is out of range).
 // DW_T 128 and four-wide activations against 64 and one by one: 12 to 30 us a layer -> 4 to 14 (SNAC, 32 windows).
 constexpr int DW_T = 128;
-__device__ __forceinline__ float4 cl_snake4(float4 v, const float4& a, const float4& inv) {
-  const float4 y = make_float4(a.x * v.x, a.y * v.y, a.z * v.z, a.w * v.w);
-  const float big = fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w)));
-  float4 s = make_float4(cl_sin_sq(y.x), cl_sin_sq(y.y), cl_sin_sq(y.z), cl_sin_sq(y.w));
-  if (!(big <= CL_SIN_MAX)) {
-    const float4 t = make_float4(sinf(y.x), sinf(y.y), sinf(y.z), sinf(y.w));
-    s = make_float4(t.x * t.x, t.y * t.y, t.z * t.z, t.w * t.w);
-  }
-  return make_float4(fmaf(inv.x, s.x, v.x), fmaf(inv.y, s.y, v.y), fmaf(inv.z, s.z, v.z), fmaf(inv.w, s.w, v.w));
-}
 __global__ void __launch_bounds__(256) cl_dwconv7_kernel(float* __restrict__ y, const float* __restrict__ x, long long x_bstride,
                                                          const float* __restrict__ w, const float* __restrict__ bias,
                                                          const float* __restrict__ alpha_in, const float* __restrict__ alpha_out,
@@ -808,10 +808,9 @@ int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, i
                    (!d_y2 || reinterpret_cast<uintptr_t>(d_y2) % 16 == 0),
                "vb_cl_conv: rows must start on 16-byte boundaries");
   if (B <= 0 || n_lo >= n_hi) return 0;
-  // the epilogue addresses rows with 32-bit offsets: batches beyond that run in several launches
-  const long long per_entry = max(max(y_bstride, r_bstride), static_cast<long long>(n_hi) * N);
-  VB_CHECK_ARG(per_entry < (1LL << 30) && N <= (1 << 20), "vb_cl_conv: a batch entry of %lld elements is too large", per_entry);
-  const int max_b = static_cast<int>(((1LL << 31) - 1) / per_entry) - 1;
+  // the epilogue addresses rows with 32-bit offsets from the first one: what is beyond that runs in several launches
+  const long long per_entry = max(y_bstride, r_bstride);
+  const int max_b = per_entry >= (1LL << 30) ? 1 : static_cast<int>(((1LL << 31) - 1) / max(per_entry, 1LL)) - 1;
   if (B > max_b) {
     for (int b0 = 0; b0 < B; b0 += max_b) {
       const int rc = vb_cl_conv(d_y + b0 * y_bstride, d_y2 ? d_y2 + b0 * y_bstride : nullptr, d_x + b0 * x_bstride, x_bstride, Tx, d_w, d_bias,
@@ -822,6 +821,17 @@ int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, i
     }
     return 0;
   }
+  const long long max_rows = max((1LL << 30) / N / 128 * 128, 128LL);
+  if (n_hi - n_lo > max_rows) {
+    for (long long t = n_lo; t < n_hi; t += max_rows) {
+      const int rc = vb_cl_conv(d_y, d_y2, d_x, x_bstride, Tx, d_w, d_bias, d_resid, r_bstride, d_scale, d_noise, noise_ld, d_alpha, epilogue, act,
+                                B, Cin, N, cmod, ksize, dil, static_cast<int>(t), static_cast<int>(min(t + max_rows, static_cast<long long>(n_hi))),
+                                y_bstride, stream);
+      if (rc != 0) return rc;
+    }
+    return 0;
+  }
+  VB_CHECK_ARG(N <= (1 << 22), "vb_cl_conv: %d columns", N);
   auto fn = encode_fn();
   VB_CHECK_ARG(fn, "cuTensorMapEncodeTiled not available (no CUDA driver?)");
   ClConvParams p = {};
@@ -846,11 +856,13 @@ int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, i
   VB_CHECK_ARG(m_tiles * ((N + p.nt - 1) / p.nt) < 0x7fffffffLL, "vb_cl_conv: too many tiles");
   p.n_tiles = (N + p.nt - 1) / p.nt;
   p.w = static_cast<const uint8_t*>(d_w);
-  p.y = d_y; p.y2 = d_y2; p.bias = d_bias; p.resid = d_resid; p.scale = d_scale; p.noise = d_noise; p.alpha = d_alpha;
+  const long long first = static_cast<long long>(n_lo) * N;
+  p.y = d_y + first; p.y2 = d_y2 ? d_y2 + first : nullptr; p.bias = d_bias; p.resid = d_resid ? d_resid + first : nullptr; p.scale = d_scale; p.noise = d_noise; p.alpha = d_alpha;
   p.y_bstride = y_bstride; p.r_bstride = r_bstride; p.ldy = N; p.ldr = N; p.noise_ld = noise_ld; p.cmod = cmod;
   p.epi = epilogue; p.act = act; p.B = B; p.n_lo = n_lo; p.n_hi = n_hi; p.ksize = ksize; p.dil = dil; p.N = N; p.n_pad = N;
   const int stage_bytes = CL_A_BYTES + p.nt * 256, tail = CL_EPI_BYTES + 512 /*barriers*/ + 2048 /*row table*/ + 1024 /*alignment*/;
-  p.stages = min(min(CL_MAX_STAGES, (512 - 2 * p.nt) / 64), (VB_MAX_DYN_SMEM - tail) / stage_bytes);
+  p.acc_cols = p.nt <= 64 ? 2 * p.nt : p.nt;
+  p.stages = min(min(CL_MAX_STAGES, (512 - 2 * p.acc_cols) / 64), (VB_MAX_DYN_SMEM - tail) / stage_bytes);
   p.tmem_cols = 512;
   CUtensorMap map;
   {

@@ -131,6 +131,22 @@ def test_channels_last_conv(B, T, C, N, ksize, dil, lo, hi, epi, act):
     assert _lib.load().vb_cl_timeouts() == 0
 
 
+@pytest.mark.parametrize("B,T,C,N,ksize", [(1, 128, 1024, 128, 7), (3, 40, 256, 32, 3), (160, 128, 64, 64, 3)])
+def test_channels_last_conv_reuses_stages(B, T, C, N, ksize):
+    """A stage's tensor-memory columns are written again while products of earlier k-blocks may still be running: many turns of the
+    ring (long k, and several units per CTA), every run equal to the first bit for bit and to 64 bits."""
+    from vox_serve_b200.tokenizer import _cl
+
+    g = torch.Generator(device="cuda").manual_seed(C)
+    x, w = torch.randn(B, T, C, generator=g, device="cuda"), torch.randn(N, C, ksize, generator=g, device="cuda") * (C * ksize) ** -0.5
+    xa, wp = _cl.Act(x.reshape(-1), B, T, C), _cl.pack_conv(w.reshape(N, -1), C, ksize)
+    y = _cl.conv(xa, wp, N, ksize=ksize).tensor()
+    ref = torch.nn.functional.conv1d(torch.nn.functional.pad(x.double().transpose(1, 2), (ksize - 1, 0)), w.double()).transpose(1, 2)
+    _close(y, ref, 3 * C * ksize / 8 * 2 ** -24)      # each of the 3 K / 8 accumulations cuts off up to 2^-23, half of it on average
+    for _ in range(20):
+        assert torch.equal(_cl.conv(xa, wp, N, ksize=ksize).tensor(), y)
+
+
 @pytest.mark.parametrize("B,T,C,cout,s,pad", [(1, 1, 32, 32, 2, 1), (5, 17, 64, 64, 8, 4), (2, 130, 128, 32, 5, 0), (1, 200, 64, 96, 3, 2)])
 def test_channels_last_transposed_conv(B, T, C, cout, s, pad):
     from vox_serve_b200.tokenizer import _cl

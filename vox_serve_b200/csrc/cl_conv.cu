@@ -293,6 +293,7 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
       for (int i = 0; i < p.ksteps; ++i) {
         bw.wait(&full[s], ph);
         if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+        tc_fence_after();            // the products that read this stage's columns before are behind the copy that was waited for
         const uint8_t* src = smem + s * stage_bytes + row * 128;
         const uint32_t t = a_col0 + s * 64 + (static_cast<uint32_t>(quarter * 32) << 16);
 #pragma unroll

@@ -147,6 +147,75 @@ def test_channels_last_conv_reuses_stages(B, T, C, N, ksize):
         assert torch.equal(_cl.conv(xa, wp, N, ksize=ksize).tensor(), y)
 
 
+def _bits(*codes):
+    return torch.tensor([c - (1 << 32) if c >> 31 else c for c in codes], dtype=torch.int32, device="cuda").view(torch.float32)
+
+
+# NaN as arithmetic writes it, quiet, negative, with a payload in the bits that tf32 drops; both infinities; the largest finite values
+@pytest.mark.parametrize("code,finite", [(0x7fffffff, False), (0x7fc00000, False), (0xffffffff, False), (0x7f800001, False), (0xff801000, False),
+                                         (0x7f800000, False), (0xff800000, False), (0x7f7fffff, True), (0xff7ff000, True), (0x7f7fefff, True)])
+@pytest.mark.parametrize("where", ["x", "w"])
+def test_channels_last_conv_special_values(code, finite, where):
+    from vox_serve_b200.tokenizer import _cl
+
+    B, T, C, N, ks = 2, 70, 64, 96, 3
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x, w = torch.randn(B, T, C, generator=g, device="cuda"), torch.randn(N, C, ks, generator=g, device="cuda") * 2.0 ** -10
+    if where == "x":
+        x[1, 33, 37] = _bits(code)
+        bad = torch.zeros(B, T, N, dtype=torch.bool, device="cuda")
+        bad[1, 33:33 + ks] = True
+    else:
+        x *= 2.0 ** -10
+        w[50, 21, 1] = _bits(code)
+        bad = torch.zeros(B, T, N, dtype=torch.bool, device="cuda")
+        bad[:, :, 50] = True                             # (the first position too: its tap reads the zero in front)
+    y = _cl.conv(_cl.Act(x.reshape(-1).clone(), B, T, C), _cl.pack_conv(w.reshape(N, -1), C, ks), N, ksize=ks).tensor()
+    if not finite:
+        assert torch.equal(~torch.isfinite(y), bad)
+        if code & 0x7fffffff != 0x7f800000:
+            assert torch.isnan(y[bad]).all()
+    else:
+        ref = torch.nn.functional.conv1d(torch.nn.functional.pad(x.double().transpose(1, 2), (ks - 1, 0)), w.double()).transpose(1, 2)
+        assert torch.isfinite(y).all()
+        _close(y[bad], ref[bad], 5e-6)
+        _close(y[~bad], ref[~bad], 5e-6)
+
+
+def test_vocoders_keep_nan(monkeypatch):
+    """What is not a number comes out as such, at the positions of the decoders on CUDA cores."""
+    from vox_serve_b200.tokenizer.mimi import MimiConfig, MimiDecoder, synthetic_state_dict
+    from vox_serve_b200.tokenizer.snac import SNAC
+
+    nan = _bits(0x7fffffff)[0]
+    out = []
+    for plain in ("0", "1"):
+        monkeypatch.setenv("VB_SNAC_FP32", plain)
+        m = SNAC(device="cuda")
+        sd = m.synthetic_state_dict(3)
+        m.load_state_dict(sd)
+        assert m.channels_last == (plain == "0")
+        m.w["codebooks"][1, 7] = nan
+        codes = [torch.zeros(1, n, dtype=torch.int64, device="cuda") for n in (16, 32, 64)]
+        codes[1][0, 12] = 7
+        noises = [torch.zeros(*s, device="cuda") for s in m.noise_shapes(1, 64)]
+        out.append(torch.isnan(m.decode(codes, noises=noises)))
+    assert out[0].any() and not out[0].all() and torch.equal(out[0], out[1])
+
+    cfg = MimiConfig(num_layers=2)
+    sd = synthetic_state_dict(cfg, 4)
+    codes = torch.zeros(2, cfg.n_q, 8, dtype=torch.int64, device="cuda")
+    codes[1, 3, 5] = 9
+    out = []
+    for plain in ("0", "1"):
+        monkeypatch.setenv("VB_CODEC_FP32", plain)
+        m = MimiDecoder(mimi_config=cfg, state_dict=sd)
+        assert m.channels_last == (plain == "0")
+        m.w["codebooks"][3, 9] = nan
+        out.append(torch.isnan(m.decode(codes)))
+    assert not out[0][0].any() and out[0][1].any() and not out[0][1].all() and torch.equal(out[0], out[1])
+
+
 @pytest.mark.parametrize("B,T,C,cout,s,pad", [(1, 1, 32, 32, 2, 1), (5, 17, 64, 64, 8, 4), (2, 130, 128, 32, 5, 0), (1, 200, 64, 96, 3, 2)])
 def test_channels_last_transposed_conv(B, T, C, cout, s, pad):
     from vox_serve_b200.tokenizer import _cl

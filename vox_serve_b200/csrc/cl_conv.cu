@@ -57,8 +57,14 @@ enum ClEpi { CE_PLAIN = 0, CE_RESID = 1, CE_SCALE_RESID = 2, CE_NOISE = 3 };
 enum ClAct { CA_NONE = 0, CA_SNAKE = 1, CA_ELU = 2, CA_GELU = 3 };
 
 // round to the 10 mantissa bits of tf32, halves away from zero (integer arithmetic: the conversion instruction runs at a
-// quarter of the rate and made the split the longest step of a stage)
-__device__ __forceinline__ float tf32_rna(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
+// quarter of the rate and made the split the longest step of a stage).  Only below CL_ROUND_MAX: from there on up the sum would leave
+// the exponent -- the largest finite values would become infinite, and NaN as arithmetic writes it, 0x7fffffff, a zero -- and the
+// low bits are cut off instead, so that a NaN or an infinity stays one.
+constexpr float CL_ROUND_MAX = 0x1.ffep127f;
+__device__ __forceinline__ float tf32_rna_below(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
+__device__ __forceinline__ float tf32_rna(float x) {
+  return __uint_as_float((__float_as_uint(x) + (fabsf(x) < CL_ROUND_MAX ? 0x1000u : 0u)) & 0xffffe000u);
+}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
@@ -84,6 +90,26 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const float (&v)[1
       ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
         "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
       : "memory");
+}
+
+// a stage's row split once more, value by value (out of line: hardly any stage needs it, and its registers are the whole kernel's)
+__device__ __noinline__ void cl_split_again(const uint8_t* src, uint32_t t, int row) {
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    float hi[16], lo[16];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float4 v = *reinterpret_cast<const float4*>(src + (((half * 4 + c) ^ (row & 7)) << 4));
+      const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        hi[4 * c + e] = tf32_rna(x[e]);
+        lo[4 * c + e] = tf32_rna(x[e] - hi[4 * c + e]);
+      }
+    }
+    tmem_st_32x16(t + 16 * half, hi);
+    tmem_st_32x16(t + 32 + 16 * half, lo);
+  }
 }
 
 // sin(x)^2: the square needs x only modulo pi, so one rounding step k = x / pi and two fused steps x - k pi leave
@@ -286,38 +312,63 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
     }
   } else if (warp < 6) {
     // ================= split: raw activations -> two halves in TMEM =================
+    // A stage is split as if all its values were ordinary ones, with the sum of four times the values kept beside it: that leaves the
+    // finite range for a NaN, an infinity and anything from CL_ROUND_MAX on.  Whether it did is asked once the next stage has landed and
+    // its values are on the way, when the stores have had their time as well, and only then is the stage handed to the products; one
+    // with such a value is split again first.  (The check costs 32 multiply-adds and a vote a stage.  Asked at the end of its own stage: SNAC
+    // one window 263 -> 279 us, 32 windows 628 -> 671, Mimi 1904 -> 2047; this way, the second half's low bits left to the product, which
+    // reads the upper 19 of a tf32 operand, and the second split out of line: 262, 651, 1929.)
     const int quarter = warp & 3, row = quarter * 32 + lane;
-    int s = 0;
+    const uint32_t t0 = a_col0 + (static_cast<uint32_t>(quarter * 32) << 16);
+    int s = 0, last = -1;                          // last: the stage that has been split and not handed over
     uint32_t ph = 0;
+    float sum = 0.f;
+    auto hand_over = [&]() {
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ready[last]);
+    };
     for (int u = blockIdx.x; u < p.units && !bw.dead; u += gridDim.x) {
       for (int i = 0; i < p.ksteps; ++i) {
         bw.wait(&full[s], ph);
-        if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
-        tc_fence_after();            // the products that read this stage's columns before are behind the copy that was waited for
+        if (!__all_sync(0xffffffffu, !bw.dead && fabsf(sum) < INFINITY)) {
+          if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+          cl_split_again(smem + last * stage_bytes + row * 128, t0 + last * 64, row);
+        }
         const uint8_t* src = smem + s * stage_bytes + row * 128;
-        const uint32_t t = a_col0 + s * 64 + (static_cast<uint32_t>(quarter * 32) << 16);
+        const uint32_t t = t0 + s * 64;
+        float4 in[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) in[c] = *reinterpret_cast<const float4*>(src + ((c ^ (row & 7)) << 4));
+        if (last >= 0) hand_over();
+        tc_fence_after();            // the products that read this stage's columns before are behind the copy that was waited for
+        float odd[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           float hi[16], lo[16];
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const float4 v = *reinterpret_cast<const float4*>(src + (((half * 4 + c) ^ (row & 7)) << 4));
+            const float4 v = in[half * 4 + c];
             const float x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              hi[4 * c + e] = tf32_rna(x[e]);
-              lo[4 * c + e] = tf32_rna(x[e] - hi[4 * c + e]);
+              hi[4 * c + e] = tf32_rna_below(x[e]);
+              lo[4 * c + e] = __uint_as_float(__float_as_uint(x[e] - hi[4 * c + e]) + 0x1000u);
+              odd[e] = fmaf(x[e], 4.f, odd[e]);
             }
           }
           tmem_st_32x16(t + 16 * half, hi);
           tmem_st_32x16(t + 32 + 16 * half, lo);
         }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ready[s]);
+        sum = (odd[0] + odd[1]) + (odd[2] + odd[3]);
+        last = s;
         if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
+    }
+    if (last >= 0 && !bw.dead) {
+      if (!__all_sync(0xffffffffu, fabsf(sum) < INFINITY)) cl_split_again(smem + last * stage_bytes + row * 128, t0 + last * 64, row);
+      hand_over();
     }
   } else {
     // ================= epilogue =================

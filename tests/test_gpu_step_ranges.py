@@ -307,6 +307,38 @@ def test_window_attention_prompt_rows(ops, D, H, G, page, new, old, window, chun
     assert _lib.load().vb_window_attn_tc_timeouts() == 0
 
 
+# keys between the kept tokens and the first one that a row tile sees: inside a key tile, over several, inside the tile of the kept tokens,
+# from a chunk's start, none at all; pages larger and smaller than what they cover
+@pytest.mark.parametrize("D,H,G,page,new,old,window,chunk,keep", [
+    (128, 4, 2, 64, 20, 500, 100, 0, 0), (64, 4, 4, 8, 60, 300, 50, 0, 5), (128, 8, 2, 16, 32, 200, 30, 0, 70), (64, 2, 1, 32, 10, 100, 0, 96, 0),
+    (128, 2, 2, 16, 40, 80, 45, 0, 20), (128, 2, 2, 16, 40, 60, 45, 0, 20), (64, 4, 1, 24, 3, 1000, 1, 0, 65)])
+def test_window_attention_unseen_keys(ops, D, H, G, page, new, old, window, chunk, keep):
+    """Nothing of the keys that no row sees reaches a result, and their pages need not be the request's."""
+    g = torch.Generator(device="cuda").manual_seed(old)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()      # noqa: E731
+    L = old + new
+    first = lambda i: max(i - window + 1 if window else 0, i - i % chunk if chunk else 0, 0)     # noqa: E731
+    hole = range(min(keep, first(old)), first(old))
+    n = (L + page - 1) // page
+    idx = np.random.RandomState(L).permutation(n).tolist()
+    kc, vc = (torch.full((n + 1, page, G, D), float("nan"), device="cuda").bfloat16() for _ in range(2))
+    q, k, v = rnd(new, H, D), rnd(L, G, D), rnd(L, G, D)
+    for j in range(L):
+        if j not in hole:
+            kc[idx[j // page], j % page], vc[idx[j // page], j % page] = k[j], v[j]
+    table = [n if set(range(i * page, (i + 1) * page)) <= set(hole) else idx[i] for i in range(n)]
+    i, j = torch.arange(old, L, device="cuda")[:, None], torch.arange(L, device="cuda")[None]
+    lo = torch.tensor([first(a) for a in range(old, L)], device="cuda")[:, None]
+    seen = (j <= i) & ((j >= lo) | (j < keep))
+    kk, vv = (x.double().repeat_interleave(H // G, 1) for x in (k, v))
+    s = torch.einsum("qhd,khd->hqk", q.double(), kk) * D ** -0.5
+    want = torch.einsum("hqk,khd->qhd", torch.softmax(s.masked_fill(~seen, -float("inf")), -1), vv)
+    out = torch.full((new, H * D), float("nan"), device="cuda").bfloat16()
+    ops.window_attn(q.view(new, H * D), kc, vc, out, None, None, _i32(list(range(old, L))), _i32([0, n]), _i32(table), new, H, G, D, D, window,
+                    D ** -0.5, tiles=(_i32([0, new]), _i32([0]), _i32([0]), 1), chunk=chunk, keep_first=keep)
+    _close(out.view(new, H, D), want, 2 ** -8)
+
+
 @pytest.mark.parametrize("T,N,S,resid,tiled,hidden", [
     (513, 8, 1, True, False, True), (514, 2048, 3, True, True, True), (600, 3072, 1, False, True, False), (515, 4096, 2, True, False, True),
     (516, 1032, 9, True, False, True), (1024, 264, 1, True, False, False),

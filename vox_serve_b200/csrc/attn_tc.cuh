@@ -7,6 +7,7 @@
 //   q_row()                  this thread's query row, or nullptr (a padding row: zeros)
 //   finish(m_ref, l)         factor for the accumulated row, given the exponents' reference and the denominator against it
 //   store(c0, o, f)          32 output values from column c0, times the factor
+//   HOLE, hole0, hole1       keys [hole0, hole1) are seen by no row of the block: they are neither fetched nor multiplied
 // See prefill_attn_tc.cu for the schedule and what bounds it.
 #pragma once
 #include "common.cuh"
@@ -89,7 +90,7 @@ struct PtcShared {
   uint64_t p_full[2];       // probabilities written, O ready to be added to
   uint64_t o_done;          // P V of a tile complete
   uint64_t o_last;          // ... of the last tile
-  uint64_t v_tail;          // the last V tile has landed (its rows past the last key are cleared next)
+  uint64_t v_part[PTC_STAGES];      // a V tile with rows that no row may see has landed (they are cleared next)
   uint32_t tmem;
   int tile[3];
   int warp_tot[PTC_THREADS / 32];
@@ -102,6 +103,7 @@ __device__ __forceinline__ void ptc_init(PtcShared* sh, int loader_arrivals) {
     mbar_init(&sh->k_empty[i], 1);
     mbar_init(&sh->v_full[i], loader_arrivals);
     mbar_init(&sh->v_empty[i], 1);
+    mbar_init(&sh->v_part[i], 1);
   }
   for (int i = 0; i < 2; ++i) {
     mbar_init(&sh->s_full[i], 1);
@@ -109,7 +111,6 @@ __device__ __forceinline__ void ptc_init(PtcShared* sh, int loader_arrivals) {
   }
   mbar_init(&sh->o_done, 1);
   mbar_init(&sh->o_last, 1);
-  mbar_init(&sh->v_tail, 1);
   fence_barrier_init();
   sh->tile[0] = -1;
 }
@@ -281,19 +282,34 @@ __device__ __forceinline__ void ptc_issue(uint8_t* smem, PtcShared* sh, int n_ti
   }
 }
 
+// whether V tile j holds rows to clear: past the last key, or in the hole
+template <class Rows>
+__device__ __forceinline__ bool ptc_partial(const Rows& rows, int j, int kmax) {
+  const int tok0 = rows.tile(j) * PTC_KT;
+  return j + 1 == rows.n_tiles || (Rows::HOLE && max(tok0, rows.hole0) < min(tok0 + PTC_KT, rows.hole1));
+}
+
 // ================= warp 5, one lane: boxes of `bt` keys x 64 dims of one head; fetch(tok, is_v, box destination, dim, barrier) =================
 template <int D, class Rows, class Fetch>
 __device__ __forceinline__ void ptc_load(uint8_t* smem, PtcShared* sh, const Rows& rows, int kmax, int bt, BoundedWait& bw, Fetch fetch_box) {
   using L = PtcLayout<D>;
   constexpr int KBD = D / 64;
   const int n_tiles = rows.n_tiles, boxes = PTC_KT / bt;
+  // (pages past the last key and pages inside the hole are not the request's)
+  auto wanted = [&](int tok) { return tok < kmax && !(Rows::HOLE && tok >= rows.hole0 && tok + bt <= rows.hole1); };
   auto fetch = [&](int j, int is_v, uint64_t* bar) {
     const uint32_t dst = smem_u32(smem + (is_v ? L::V : L::K) + (j & 1) * L::TILE), mb = smem_u32(bar);
     const int tok0 = rows.tile(j) * PTC_KT;
-    mbar_arrive_expect_tx(bar, min(boxes, (kmax - tok0 + bt - 1) / bt) * bt * D * 2);
+    int n = 0;
+    if (Rows::HOLE) {
+      for (int i = 0; i < boxes; ++i) n += wanted(tok0 + i * bt) ? 1 : 0;
+    } else {
+      n = min(boxes, (kmax - tok0 + bt - 1) / bt);
+    }
+    mbar_arrive_expect_tx(bar, n * bt * D * 2);
     for (int i = 0; i < boxes; ++i) {
       const int tok = tok0 + i * bt;
-      if (tok >= kmax) break;                     // (pages past the last key are not the request's)
+      if (!wanted(tok)) continue;
 #pragma unroll
       for (int kb = 0; kb < KBD; ++kb) fetch_box(tok, is_v, dst + kb * (PTC_KT * 128) + i * bt * 128, kb * 64, mb);
     }
@@ -304,7 +320,7 @@ __device__ __forceinline__ void ptc_load(uint8_t* smem, PtcShared* sh, const Row
     fetch(j, 0, &sh->k_full[j & 1]);
     bw.wait(&sh->v_empty[j & 1], ((j >> 1) & 1) ^ 1);
     if (bw.dead) break;
-    fetch(j, 1, j + 1 < n_tiles ? &sh->v_full[j & 1] : &sh->v_tail);
+    fetch(j, 1, ptc_partial(rows, j, kmax) ? &sh->v_part[j & 1] : &sh->v_full[j & 1]);
   }
   if (bw.dead) {                                  // let the copies in flight land before the block may leave
     const unsigned long long t0 = gtimer();
@@ -312,25 +328,36 @@ __device__ __forceinline__ void ptc_load(uint8_t* smem, PtcShared* sh, const Row
   }
 }
 
-// ================= warp 6: rows of the last V tile past the last key =================
-// They are multiplied by probability 0: whatever the cache holds there, they must be finite.  (The last tile of the walk is the one
-// that holds key kmax - 1; tiles before it hold written keys only.)
-template <int D>
-__device__ __forceinline__ void ptc_clear_tail(uint8_t* smem, PtcShared* sh, int n_tiles, int kmax, BoundedWait& bw) {
+// ================= warp 6: rows of V tiles that no row may see =================
+// They are multiplied by probability 0: whatever the cache holds there, they must be finite.  The last tile of the walk holds key
+// kmax - 1 and rows past it; tiles at the edges of the hole hold rows inside it.
+template <int D, class Rows>
+__device__ __forceinline__ void ptc_clear_unseen(uint8_t* smem, PtcShared* sh, const Rows& rows, int kmax, BoundedWait& bw) {
   using L = PtcLayout<D>;
   constexpr int KBD = D / 64;
-  const int lane = threadIdx.x & 31, j = n_tiles - 1;
-  bw.wait(&sh->v_tail, 0);
-  if (!__all_sync(0xffffffffu, !bw.dead)) return;
-  uint8_t* tile = smem + L::V + (j & 1) * L::TILE;
-  const int r0 = kmax - (kmax - 1) / PTC_KT * PTC_KT, chunks = (PTC_KT - r0) * 8;
-  for (int i = lane; i < KBD * chunks; i += 32) {
-    const int kb = i / chunks, c = i - kb * chunks;
-    *reinterpret_cast<uint4*>(tile + kb * (PTC_KT * 128) + r0 * 128 + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+  const int lane = threadIdx.x & 31;
+  uint32_t turn = 0;                              // bit s: parity of stage s's next partial tile
+  for (int j = 0; j < rows.n_tiles; ++j) {
+    if (!ptc_partial(rows, j, kmax)) continue;
+    const int s = j & 1, tok0 = rows.tile(j) * PTC_KT;
+    bw.wait(&sh->v_part[s], turn >> s & 1u);
+    if (!__all_sync(0xffffffffu, !bw.dead)) return;
+    turn ^= 1u << s;
+    uint8_t* tile = smem + L::V + s * L::TILE;
+    auto clear = [&](int r0, int r1) {            // rows [r0, r1) of the tile
+      const int chunks = (r1 - r0) * 8;
+      for (int i = lane; i < KBD * chunks; i += 32) {
+        const int kb = i / chunks, c = i - kb * chunks;
+        *reinterpret_cast<uint4*>(tile + kb * (PTC_KT * 128) + r0 * 128 + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+      }
+    };
+    if (kmax - tok0 < PTC_KT) clear(kmax - tok0, PTC_KT);
+    if (Rows::HOLE && max(tok0, rows.hole0) < min(tok0 + PTC_KT, rows.hole1))
+      clear(max(rows.hole0 - tok0, 0), min(rows.hole1 - tok0, PTC_KT));
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh->v_full[s]);
   }
-  fence_proxy_async();
-  __syncwarp();
-  if (lane == 0) mbar_arrive(&sh->v_full[j & 1]);
 }
 
 inline int ptc_box_tokens(int page_size) { return page_size % 64 == 0 ? 64 : (page_size % 32 == 0 ? 32 : (page_size % 16 == 0 ? 16 : 8)); }

@@ -46,6 +46,8 @@ struct PrefillTcParams {
 
 // what this thread's row sees: the first kl keys of its request
 struct PagedRows {
+  static constexpr bool HOLE = false;
+  static constexpr int hole0 = 0, hole1 = 0;
   const PrefillTcParams& p;
   int n_tiles, kl, row, head, D;
   bool ok;
@@ -164,7 +166,7 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
           ptc_tma_5d(dst, &kv_map, bar, dim, hk, tok % p.page_size, is_v, p.slab_base + page);
         });
       } else if (warp == 6 && n_tiles > 0) {
-        ptc_clear_tail<D>(smem, sh, n_tiles, kmax, bw);
+        ptc_clear_unseen<D>(smem, sh, rows, kmax, bw);
       }
       __syncwarp();
     } else {

@@ -4,7 +4,8 @@
 // A CTA owns TQ = min(64, 128 / R) rows of one request x the R query heads of ONE key head (accumulator row r: prompt row r / R,
 // head r % R), so a group's K / V tiles are fetched once for all its heads; the mma.sync tiles of window_attn.cu take one query
 // head each.  A row tile of 64 is dealt to ceil(64 / TQ) CTAs.  Keys are walked in tiles of 64 positions: first those with kept
-// tokens, then from the tile of the first key that the CTA's first row sees; within a tile the mask is per key.
+// tokens, then from the tile of the first key that the CTA's first row sees; within a tile the mask is per key.  What lies between the two is
+// nobody's to read (a page table may name other requests' pages there, or unwritten ones): its boxes are skipped, its V rows cleared.
 // Measured (16 query heads on 4 key heads of 128, two prompts of 1001 rows in all): 102 us per launch with mma.sync, about 20 here; the
 // three-layer prompt step around it 1058 -> 884 us.
 #include "../../include/vb_api.h"
@@ -37,8 +38,10 @@ __device__ __forceinline__ void wtc_tma_4d(uint32_t dst, const CUtensorMap* m, u
 }
 
 struct WindowRows {
+  static constexpr bool HOLE = true;
   const WindowTcParams& p;
   int n_tiles, n0, t1;           // tiles 0 .. n0 - 1 hold kept tokens, the rest start at t1
+  int hole0, hole1;              // between the kept tokens and the first key that the block's first row sees
   int pos, lo, row, head, D;
   bool ok;
   float scale_log2;
@@ -123,7 +126,7 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) window_attn_tc_kernel(const Wi
     const int n0 = (min(p.keep, lo0) + PTC_KT - 1) / PTC_KT, t1 = max(lo0 / PTC_KT, n0), n_tiles = n0 + (kmax + PTC_KT - 1) / PTC_KT - t1;
     const int t = tid / p.R;
     const bool ok = warp < 4 && t < nrows;
-    const WindowRows rows{p, n_tiles, n0, t1, pos0 + t, first_key(pos0 + t), row0 + t, g * p.R + tid - t * p.R, D, ok, p.scale_log2};
+    const WindowRows rows{p, n_tiles, n0, t1, min(p.keep, lo0), lo0, pos0 + t, first_key(pos0 + t), row0 + t, g * p.R + tid - t * p.R, D, ok, p.scale_log2};
     if (warp < 4) {
       ptc_softmax<D>(smem, sh, rows, bw);
     } else if (warp == 4) {
@@ -136,7 +139,7 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) window_attn_tc_kernel(const Wi
           wtc_tma_4d(dst, is_v ? &v_map : &k_map, bar, dim, is_v ? gv : g, tok % p.page_size, page);
         });
       } else if (warp == 6) {
-        ptc_clear_tail<D>(smem, sh, n_tiles, kmax, bw);
+        ptc_clear_unseen<D>(smem, sh, rows, kmax, bw);
       }
       __syncwarp();
     }

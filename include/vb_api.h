@@ -491,7 +491,13 @@ int vb_gemm_bf16_grouped_glu(void* d_y, const void* d_w_tiles, const void* x_map
  * 256; x_map (row-major activations): a vb_tensor_map_2d_bf16 map whose box has n_tok / 2 rows; d_x_tiles: the XT(vb_gemm_t_tile(T))
  * layout, whatever n_tok is (y_tiled output is written in the same layout).  With d_tile_group, tile i (rows i * n_tok ..) is
  * multiplied by the weights of group d_tile_group[i].
- * vb_gemm_wide_timeouts: how many waits of that kernel have run out in this process (0 unless something is wrong; synchronises). */
+ * vb_gemm_wide_timeouts: whether a wait of that kernel has run out since its flag was last cleared (0 unless something is wrong;
+ * synchronises the device).
+ * vb_wait_flags: eight bytes of host memory, one flag per kind of kernel whose waits give up after two seconds -- 0 prompt projections, 1
+ * vocoder convolutions, 2 prompt attention, 3 window attention of prompts, 4 vb_wait_check.  A kernel whose wait ran out sets its
+ * flag and leaves its output incomplete: look at them after synchronising, before results are used, and clear them (NULL: no device).
+ * vb_wait_check: one kernel that waits on a barrier at most limit_us from the moment a second warp opens it, pause_us after the start;
+ * that warp then completes the barrier, or with complete = 0 does not (flag 4). */
 int vb_gemm_bf16_wide(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
                       int mode, int split_k, int tile_rows, int n_out, int y_tiled, const void* d_bias, int act, int n_tok,
                       void* stream);
@@ -500,6 +506,8 @@ int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_ma
                               const int32_t* d_tile_group, long long group_bytes, int w_kb_stride, int group_kb, int kb_base,
                               float glu_limit, float glu_slope, void* stream);
 int vb_gemm_wide_timeouts(void);
+void* vb_wait_flags(void);
+int vb_wait_check(int limit_us, int pause_us, int complete, void* stream);
 
 /* ---- vocoder stages over channels-last fp32 activations [B][T][C] (cl_conv.cu) ----
  * vb_cl_pack: fp32 weights [N][K] (K = taps x channels, tap-major, the tap furthest back first) -> vb_cl_pack_bytes(N, K) bytes for

@@ -414,3 +414,24 @@ def test_rmsnorm_rows(ops, rows, dim, tiled):
     out = ops.TiledAct(rows, dim, torch.device("cuda")) if tiled else None
     got = ops.rmsnorm(x, w[1:].clone(), 1e-5, out=out)
     assert torch.equal(got.to_rows() if tiled else got, ops.rmsnorm(x, w[1:], 1e-5))
+
+
+def test_a_wait_that_runs_out_is_reported(ops):
+    """The limit counts from the moment the block's gate opens; the flag reaches the host and the next call."""
+    from vox_serve_b200 import _lib
+
+    for pause in (0, 20000):                             # a wait of twenty times the limit in front of the gate is not late
+        _lib.call("vb_wait_check", 1000, pause, 1, ops._stream())
+    torch.cuda.synchronize()
+    ops.check_waits()
+    _lib.call("vb_wait_check", 1000, 0, 0, ops._stream())
+    torch.cuda.synchronize()
+    with pytest.raises(_lib.VoxB200Error, match="vb_wait_check"):
+        ops.check_waits()
+    ops.check_waits()
+    _lib.call("vb_wait_check", 1000, 0, 0, ops._stream())
+    torch.cuda.synchronize()
+    with pytest.raises(_lib.VoxB200Error, match="ran out"):
+        _lib.call("vb_wait_check", 1000, 0, 1, ops._stream())
+    with pytest.raises(_lib.VoxB200Error, match="outside"):
+        _lib.call("vb_wait_check", -1, 0, 1, ops._stream())

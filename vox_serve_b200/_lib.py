@@ -59,6 +59,8 @@ SIGNATURES = {
     "vb_gemm_bf16_wide_grouped": (c_int, [P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, c_int, c_int, P,
                                           C.c_longlong, c_int, c_int, c_int, c_float, c_float, P]),
     "vb_gemm_wide_timeouts": (c_int, []),
+    "vb_wait_flags": (P, []),
+    "vb_wait_check": (c_int, [c_int, c_int, c_int, P]),
     "vb_cl_timeouts": (c_int, []),
     "vb_cl_pack_bytes": (C.c_longlong, [c_int, c_int]),
     "vb_cl_pack": (c_int, [P, P, c_int, c_int, P]),
@@ -207,6 +209,9 @@ SIGNATURES = {
 
 _lock = threading.Lock()
 _lib = None
+# flags in mapped host memory, one byte per kind of kernel whose waits give up (csrc/common.cuh, BoundedWait)
+_wait_flags = None
+WAIT_KINDS = ("a projection of a prompt step", "a vocoder convolution", "prompt attention", "window attention of a prompt", "vb_wait_check")
 
 
 class VoxB200Error(RuntimeError):
@@ -261,9 +266,26 @@ def check(rc: int, what: str = ""):
         raise VoxB200Error(f"{what} failed (rc={rc}): {msg.decode() if msg else ''}")
 
 
+def check_waits():
+    """Raise if a wait inside a kernel ran out: that kernel left its output incomplete, and what was computed from it since is
+    wrong.  Workers look here once they have waited for a step's ids, logits or audio; every further ``call`` looks too.  A program
+    that reads results by other means calls this after it has synchronised."""
+    global _wait_flags
+    if _wait_flags is None:
+        at = load().vb_wait_flags()
+        if not at:                       # no device
+            return
+        _wait_flags = C.c_uint64.from_address(at)
+    bits = _wait_flags.value
+    if bits:
+        _wait_flags.value = 0
+        kinds = [name for i, name in enumerate(WAIT_KINDS) if bits >> (8 * i) & 0xff] or ["a kernel"]
+        raise VoxB200Error(f"a wait inside {' and '.join(kinds)} ran out: results since then are incomplete")
+
+
 # kernels (+ memset nodes) each entry point enqueues; everything not listed launches exactly one
 LAUNCHES = {"vb_set_pdl": 0, "vb_set_trace": 0, "vb_weight_tiles_bytes": 0, "vb_tensor_map_kv": 0,
-            "vb_tensor_map_2d_bf16": 0, "vb_gemm_wide_timeouts": 0, "vb_cl_timeouts": 0, "vb_prefill_attn_tc_timeouts": 0, "vb_window_attn_tc_timeouts": 0, "vb_cl_pack_bytes": 0, "vb_device_info": 0, "vb_sample": 1, "vb_update_repetition_cache": 1,
+            "vb_tensor_map_2d_bf16": 0, "vb_gemm_wide_timeouts": 0, "vb_wait_flags": 0, "vb_cl_timeouts": 0, "vb_prefill_attn_tc_timeouts": 0, "vb_window_attn_tc_timeouts": 0, "vb_cl_pack_bytes": 0, "vb_device_info": 0, "vb_sample": 1, "vb_update_repetition_cache": 1,
             "vb_set_gemm_smem_kb": 0, "vb_window_attn_tile_rows": 0, "vb_decay_attn_tile_rows": 0, "vb_decay_attn_tiled": 3, "vb_window_attn": 2, "vb_mingru_tiled": 3, "vb_mingru_scratch_floats": 0,
             "vb_short_conv": 2, "vb_selective_scan_tiled": 3, "vb_selective_scan_piece_rows": 0,
             "vb_selective_scan_scratch_floats": 0, "vb_sigmoid_attn": 1, "vb_ssd_tiled": 3, "vb_ssd_tile_rows": 0,
@@ -273,6 +295,8 @@ launch_counter = [0]
 
 def call(name: str, *args):
     """Invoke an int-returning entry point and raise on error."""
+    if _wait_flags is None or _wait_flags.value:
+        check_waits()
     rc = getattr(_lib or load(), name)(*args)
     if rc != 0:
         check(rc, name)

@@ -3,6 +3,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 
 #include <cudaTypedefs.h>
 
@@ -41,6 +42,54 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
   return fn;
 }
+// One flag (a byte) per kind of kernel in host memory that every device maps: set by a wait that ran out, read and cleared by the
+// host.  Allocated once and kept: captured graphs hold its address.
+static unsigned char *g_wait_host = nullptr, *g_wait_dev = nullptr;
+static std::mutex g_wait_lock;
+unsigned char* wait_flag(WaitKind kind) {
+  std::lock_guard<std::mutex> hold(g_wait_lock);
+  if (!g_wait_dev) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;        // (the first launch may be a captured one)
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void *h = nullptr, *d = nullptr;
+    if (cudaHostAlloc(&h, WK_KINDS, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+      memset(h, 0, WK_KINDS);
+      if (cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess) {
+        g_wait_host = static_cast<unsigned char*>(h);
+        g_wait_dev = static_cast<unsigned char*>(d);
+      } else {
+        cudaFreeHost(h);
+      }
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+  return g_wait_dev ? g_wait_dev + kind : nullptr;
+}
+int wait_ran_out(WaitKind kind) {
+  if (!wait_flag(kind) || cudaDeviceSynchronize() != cudaSuccess) return -1;
+  return *(volatile unsigned char*)(g_wait_host + kind);
+}
+
+// A barrier that one warp waits for and another completes (or not) after a pause: what the flags and the gate are tested with
+__global__ void wait_check_kernel(unsigned char* flag, unsigned long long limit, unsigned long long pause, int complete) {
+  __shared__ uint64_t bar;
+  __shared__ uint32_t gate;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    fence_barrier_init();
+    gate = 0u;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    BoundedWait bw{flag, smem_u32(&gate), limit};
+    bw.wait(&bar, 0);
+  } else if (threadIdx.x == 32) {
+    const unsigned long long t0 = gtimer();
+    while (gtimer() - t0 < pause) __nanosleep(1000);
+    wait_gate_open(smem_u32(&gate));
+    if (complete) mbar_arrive(&bar);
+  }
+}
 // weak: a library built from a subset of the sources (vox_serve_b200/build.py profiles) lacks some of these
 __attribute__((weak)) cudaError_t trace_set_elementwise(unsigned long long*);
 __attribute__((weak)) cudaError_t trace_set_attn(unsigned long long*);
@@ -67,6 +116,16 @@ int vb_set_pdl(int enabled) {
   const int old = vb::pdl_enabled(0) ? 1 : 0;
   vb::g_pdl = enabled ? 1 : 0;
   return old;
+}
+
+void* vb_wait_flags(void) { return vb::wait_flag(vb::WK_GEMM_WIDE) ? vb::g_wait_host : nullptr; }
+int vb_wait_check(int limit_us, int pause_us, int complete, void* stream) {
+  VB_CHECK_ARG(limit_us >= 0 && limit_us <= 1000000 && pause_us >= 0 && pause_us <= 1000000, "vb_wait_check: %d us, %d us outside [0, 1000000]", limit_us, pause_us);
+  unsigned char* flag = vb::wait_flag(vb::WK_CHECK);
+  VB_CHECK_ARG(flag, "vb_wait_check: no mapped host memory");
+  vb::wait_check_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(flag, limit_us * 1000ull, pause_us * 1000ull, complete);
+  VB_CHECK_LAUNCH();
+  return 0;
 }
 
 int vb_device_info(int* sm_count, int* max_smem_optin) {

@@ -51,6 +51,7 @@ struct ClConvParams {
   int ldy, ldr, noise_ld, cmod, epi, act;
   int B, n_lo, n_hi, ksize, dil, N, n_pad, kb_per_tap, ksteps;
   int nt, n_tiles, nr, nb, t_tiles, units, stages, tmem_cols;
+  unsigned char* wait_flag;
   int acc_cols;              // TMEM columns of an accumulator: nt, or 2 nt where the two halves of the weights have their own
 };
 enum ClEpi { CE_PLAIN = 0, CE_RESID = 1, CE_SCALE_RESID = 2, CE_NOISE = 3 };
@@ -177,11 +178,13 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
   uint64_t* acc_full = empty + CL_MAX_STAGES;    // [2]
   uint64_t* acc_empty = acc_full + 2;            // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  const uint32_t gate = smem_u32(tmem_slot + 1);  // set once the kernels in front have completed
   int4* row_tab = reinterpret_cast<int4*>(smem + p.stages * stage_bytes + CL_EPI_BYTES + 512);     // [128]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  BoundedWait bw;
+  BoundedWait bw{p.wait_flag, gate};
 
   if (warp == 0 && lane == 0) {
+    tmem_slot[1] = 0u;
     prefetch_tmap(&x_map);
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(&full[s], 1);
@@ -242,6 +245,7 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
             load_w(j);
           }
           pdl_wait();
+          wait_gate_open(gate);
           pdl_trigger();
           for (int j = 0; j < npre; ++j) load_x(j);
           waited = true;
@@ -824,9 +828,7 @@ using namespace vb;
 extern "C" {
 
 int vb_cl_timeouts(void) {
-  unsigned int n = 0;
-  if (cudaMemcpyFromSymbol(&n, g_wait_timeouts, sizeof(n)) != cudaSuccess) return -1;
-  return static_cast<int>(n);
+  return wait_ran_out(WK_CL_CONV);
 }
 
 long long vb_cl_pack_bytes(int N, int K) {
@@ -887,6 +889,7 @@ int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, i
   auto fn = encode_fn();
   VB_CHECK_ARG(fn, "cuTensorMapEncodeTiled not available (no CUDA driver?)");
   ClConvParams p = {};
+  VB_CHECK_ARG(p.wait_flag = wait_flag(WK_CL_CONV), "vb_cl_conv: no mapped host memory");
   const int range = n_hi - n_lo;
   p.nr = min(range, 128);
   p.nb = min(B, 128 / p.nr);

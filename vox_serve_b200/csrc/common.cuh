@@ -294,10 +294,17 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
   __trap();
 }
 
-// A wait that gives up: after 2 s it notes the fact in its translation unit's counter and every later wait of the thread
-// returns at once, so that the block can stop issuing, let its copies land and leave with the context usable.
-static __device__ unsigned int g_wait_timeouts = 0;
+// A wait that gives up.  After 2 s it sets its kind's flag in host memory (vb_wait_flags: whoever collects results looks there) and
+// every later wait of the thread returns at once, so that the block can stop issuing, let its copies land and leave with the
+// context usable.  `gate`: shared-memory word that the block sets once the kernels in front have completed (0: they have); the
+// clock starts there, or a predecessor's running time would count as the wait's own.
+enum WaitKind { WK_GEMM_WIDE = 0, WK_CL_CONV = 1, WK_PREFILL_ATTN = 2, WK_WINDOW_ATTN = 3, WK_CHECK = 4, WK_KINDS = 8 };
+unsigned char* wait_flag(WaitKind kind);      // api.cu: its address on the device, nullptr if the flags could not be allocated
+int wait_ran_out(WaitKind kind);              // api.cu: after all work on the device
 struct BoundedWait {
+  unsigned char* flag;
+  uint32_t gate = 0u;
+  unsigned long long limit = 2000000000ull;
   bool dead = false;
   __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity) {
     if (dead) return;
@@ -306,17 +313,23 @@ struct BoundedWait {
     for (uint32_t spin = 1;; ++spin) {
       if (mbar_try_wait(bar, parity)) return;
       if ((spin & 255u) == 0u) {
+        uint32_t open = 1u;
+        if (gate) asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(open) : "r"(gate) : "memory");
         const unsigned long long now = gtimer();
-        if (t0 == 0ull) t0 = now;
-        else if (now - t0 > 2000000000ull) {
+        if (t0 == 0ull || !open) t0 = now;
+        else if (now - t0 > limit) {
           dead = true;
-          atomicAdd(&g_wait_timeouts, 1u);
+          *reinterpret_cast<volatile unsigned char*>(flag) = 1;
+          __threadfence_system();
           return;
         }
       }
     }
   }
 };
+__device__ __forceinline__ void wait_gate_open(uint32_t gate) {
+  asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(gate), "r"(1u) : "memory");
+}
 
 // ---------------------------------------------------------------------------------------------
 // TMA

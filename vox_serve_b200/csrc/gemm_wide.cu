@@ -20,7 +20,7 @@
 //
 // Warp roles per CTA: warp 0 producer, warp 1 MMA issuer (leader CTA) or relay (the other CTA: tells the leader that its
 // half of a stage has landed), warps 2..9 epilogue (two per TMEM quarter, alternating 16-column chunks).
-// Every wait is bounded (2 s of %globaltimer): a CTA whose wait runs out records it, stops issuing and leaves.
+// Every wait is bounded (BoundedWait): a CTA whose wait runs out sets its flag, stops issuing and leaves.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 2
 #include "common.cuh"
@@ -45,6 +45,7 @@ struct GemmWideParams {
   int n_tok;                   // token rows per tile (multiple of 16, <= 256)
   int stages, num_kb, n_tiles, n_pairs, t_blocks, units, w_kb_stride, group_kb, kb_base;
   float glu_limit, glu_slope;
+  unsigned char* wait_flag;
 };
 
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
@@ -144,13 +145,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
   uint64_t* acc_full = empty + GW_MAX_STAGES;                                     // [2]
   uint64_t* acc_empty = acc_full + 2;                                             // (leader) [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  const uint32_t gate = smem_u32(tmem_slot + 1);                                  // set once the kernels in front have completed
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
-  BoundedWait bw;
+  BoundedWait bw{p.wait_flag, gate};
 
   if (warp == 0 && lane == 0) {
+    tmem_slot[1] = 0u;
     if (!p.x_tiles) prefetch_tmap(&x_map);
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(&full[s], 1);
@@ -237,6 +240,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
           };
           if (!p.tile_group) pre_a();
           pdl_wait();
+          wait_gate_open(gate);
           pdl_trigger();
           if (p.tile_group) {
             const size_t grp = p.tile_group[g.tblk];
@@ -267,7 +271,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
         }
         if (bw.dead) break;
       }
-      if (!waited) { pdl_wait(); pdl_trigger(); }       // (a pair without units)
+      if (!waited) { pdl_wait(); pdl_trigger(); }       // (a pair without units: nobody waits)
       if (bw.dead) {                                    // let the copies in flight land before the block may leave
         const unsigned long long t0 = gtimer();
         while (gtimer() - t0 < 2000000ull) __nanosleep(1000);
@@ -481,9 +485,7 @@ using namespace vb;
 extern "C" {
 
 int vb_gemm_wide_timeouts(void) {
-  unsigned int n = 0;
-  if (cudaMemcpyFromSymbol(&n, g_wait_timeouts, sizeof(n)) != cudaSuccess) return -1;
-  return static_cast<int>(n);
+  return wait_ran_out(WK_GEMM_WIDE);
 }
 
 int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
@@ -504,6 +506,7 @@ int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_ma
   VB_CHECK_ARG(!d_tile_group || x_map, "vb_gemm_bf16_wide: groups need row-major activations");
   static const CUtensorMap dummy_map = {};
   GemmWideParams p = {};
+  VB_CHECK_ARG(p.wait_flag = wait_flag(WK_GEMM_WIDE), "vb_gemm_bf16_wide: no mapped host memory");
   p.num_kb = (K + GW_BLOCK_K - 1) / GW_BLOCK_K;
   VB_CHECK_ARG(split_k >= 1 && split_k <= p.num_kb, "vb_gemm_bf16_wide: split_k %d outside [1, %d]", split_k, p.num_kb);
   p.y = d_y; p.w_tiles = static_cast<const uint8_t*>(d_w_tiles); p.x_tiles = static_cast<const uint8_t*>(d_x_tiles);

@@ -22,7 +22,7 @@
 // of 997 rows on up to 1063 cached tokens 92 / 35, three prompts of 1024 rows 46 / 19, four of 600 rows with 64-wide heads 75 / 33.
 // What bounds it: the serial chain of a tile (scores -> maximum -> exponentials -> P V, about 1.3 us), and where few tiles see
 // a long context the longest of them.
-// Every wait is bounded (BoundedWait): a block whose wait runs out notes it, stops issuing and leaves.
+// Every wait is bounded (BoundedWait): a block whose wait runs out sets its flag, stops issuing and leaves.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 1
 #include "attn_tc.cuh"
@@ -42,6 +42,7 @@ struct PrefillTcParams {
   int out_xt_tile;
   int box_tokens;
   float scale_log2;
+  unsigned char* wait_flag;
 };
 
 // what this thread's row sees: the first kl keys of its request
@@ -82,7 +83,7 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ptc_smem_raw) + 1023) & ~uintptr_t(1023));
   PtcShared* sh = reinterpret_cast<PtcShared*>(smem + L::BAR);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  BoundedWait bw;
+  BoundedWait bw{p.wait_flag};
   if (tid == 0) {
     ptc_init(sh, TMA ? 1 : 64);
     if (TMA) prefetch_tmap(&kv_map);
@@ -241,9 +242,7 @@ using namespace vb;
 extern "C" {
 
 int vb_prefill_attn_tc_timeouts(void) {
-  unsigned int n = 0;
-  if (cudaMemcpyFromSymbol(&n, g_wait_timeouts, sizeof(n)) != cudaSuccess) return -1;
-  return static_cast<int>(n);
+  return wait_ran_out(WK_PREFILL_ATTN);
 }
 
 int vb_prefill_attn_tc_tile_rows(int n_q, int n_kv) {
@@ -263,6 +262,7 @@ int vb_paged_prefill_attn_tc(void* d_out, const void* d_q, const void* d_kv, int
   VB_CHECK_ARG(page_size >= 1, "vb_paged_prefill_attn_tc: page_size %d", page_size);
   if (n_rows <= 0 || n_req <= 0) return 0;
   PrefillTcParams p;
+  VB_CHECK_ARG(p.wait_flag = wait_flag(WK_PREFILL_ATTN), "vb_paged_prefill_attn_tc: no mapped host memory");
   p.out = static_cast<__nv_bfloat16*>(d_out);
   p.q = static_cast<const __nv_bfloat16*>(d_q);
   p.kv = static_cast<const __nv_bfloat16*>(d_kv);

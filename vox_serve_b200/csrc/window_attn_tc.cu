@@ -27,6 +27,7 @@ struct WindowTcParams {
   const float* sink;             // [H] or nullptr
   int ld_gate, H, G, R, TQ, subs, page_size, window, chunk, keep, v_share, out_f32, head_gate, box_tokens;
   float scale_log2;
+  unsigned char* wait_flag;
 };
 
 __device__ __forceinline__ void wtc_tma_4d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2, int c3) {
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) window_attn_tc_kernel(const Wi
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wtc_smem_raw) + 1023) & ~uintptr_t(1023));
   PtcShared* sh = reinterpret_cast<PtcShared*>(smem + L::BAR);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  BoundedWait bw;
+  BoundedWait bw{p.wait_flag};
   if (tid == 0) {
     ptc_init(sh, 1);
     prefetch_tmap(&k_map);
@@ -165,6 +166,7 @@ int window_attn_tc(void* out, const void* q, const void* k_cache, const void* v_
                    const int32_t* tile_row0, int n_tiles, int H, int G, int dim, int page_size, int window, float scale, int chunk, int k_ld,
                    int v_ld, int v_share, int out_f32, const float* sink, int keep_first, int head_gate, cudaStream_t stream) {
   WindowTcParams p{};
+  VB_CHECK_ARG(p.wait_flag = wait_flag(WK_WINDOW_ATTN), "vb_window_attn_tiled: no mapped host memory");
   p.q = static_cast<const __nv_bfloat16*>(q); p.out = out; p.gate = gate; p.pos = pos; p.page_indptr = page_indptr;
   p.page_indices = page_indices; p.qo_indptr = qo_indptr; p.tile_req = tile_req; p.tile_row0 = tile_row0; p.sink = sink;
   p.ld_gate = ld_gate; p.H = H; p.G = G; p.R = H / G; p.TQ = min(64, 128 / p.R); p.subs = (64 + p.TQ - 1) / p.TQ;
@@ -195,7 +197,5 @@ int window_attn_tc(void* out, const void* q, const void* k_cache, const void* v_
 }  // namespace vb
 
 extern "C" int vb_window_attn_tc_timeouts(void) {
-  unsigned int n = 0;
-  if (cudaMemcpyFromSymbol(&n, vb::g_wait_timeouts, sizeof(n)) != cudaSuccess) return -1;
-  return static_cast<int>(n);
+  return vb::wait_ran_out(vb::WK_WINDOW_ATTN);
 }

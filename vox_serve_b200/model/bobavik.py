@@ -24,7 +24,7 @@ import numpy as np
 import torch
 
 from .. import ops
-from .._lib import VoxB200Error
+from .._lib import VoxB200Error, check_waits
 from ..hybrid_engine import HybridCache, HybridConfig, HybridEngine, HybridWeights, StepInputs
 from ..requests import Request
 from ..sampling import Sampler, SamplingConfig
@@ -240,6 +240,7 @@ class BobavikModel(BaseLM):
             else:
                 host = output_ids.to("cpu")
             col0 = host[:, 0].tolist()
+            check_waits()
             for i, req in enumerate(requests):
                 if not takes[i]:
                     continue

@@ -21,7 +21,7 @@ from typing import Any, Dict, List, Optional, Tuple
 import torch
 
 from .. import ops
-from .._lib import VoxB200Error
+from .._lib import VoxB200Error, check_waits
 from ..depth_engine import BB, DD, CsmDims, CsmEngine, CsmWeights
 from ..engine import hf_layer_names
 from ..requests import Request
@@ -245,6 +245,7 @@ class CSMModel(BaseLMWithDepth):
         ops.multi_embed_sum(c0, ids[:, 0:1].contiguous(), self.weights.embed_audio, col_offset=self.vocab_size, col0=0)
         hidden_for_depth = torch.stack((hidden_states, c0), dim=1)
         host = ids.cpu()
+        check_waits()
         for i, req in enumerate(requests):
             req.input_tokens = torch.zeros(1, self.n_codebooks, dtype=torch.long)
             req.input_tokens[0, 0] = host[i, 0]
@@ -280,6 +281,7 @@ class CSMModel(BaseLMWithDepth):
         emb = torch.empty(ids.shape[0], self.hidden_size, dtype=BF16, device=ids.device)
         ops.multi_embed_sum(emb, ids.view(-1, 1), self.weights.embed_audio, col_offset=self.vocab_size, col0=i_iteration)
         host = ids.cpu().tolist()
+        check_waits()
         for i, req in enumerate(requests):
             req.input_tokens[0, i_iteration] = host[i]
             req.lm_output_tokens[-1][0, i_iteration] = host[i]

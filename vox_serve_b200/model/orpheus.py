@@ -23,7 +23,7 @@ from typing import Any, Dict, List, Optional
 import torch
 
 from .. import ops
-from .._lib import VoxB200Error
+from .._lib import VoxB200Error, check_waits
 from ..engine import LlamaDims, LlamaEngine, LlamaWeights, hf_layer_names
 from ..requests import Request
 from ..sampling import Sampler, SamplingConfig
@@ -279,6 +279,7 @@ class OrpheusModel(BaseLM):
             else:
                 host = output_ids.to("cpu")
             col0 = host[:, 0].tolist()
+            check_waits()
             for i, req in enumerate(requests):
                 tok = host[i:i + 1]
                 req.lm_output_tokens.append(tok)

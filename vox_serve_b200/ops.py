@@ -15,7 +15,7 @@ from typing import Dict, Optional, Tuple
 import torch
 
 from . import _lib
-from ._lib import VoxB200Error, call
+from ._lib import VoxB200Error, call, check_waits  # noqa: F401  (check_waits: for programs that read results by other means than a worker)
 
 BF16 = torch.bfloat16
 

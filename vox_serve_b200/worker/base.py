@@ -29,7 +29,7 @@ import numpy as np
 import torch
 
 from .. import _lib, ops
-from .._lib import VoxB200Error
+from .._lib import VoxB200Error, check_waits
 from ..flashinfer_utils import FlashInferDecodeWrapper, FlashInferPrefillWrapper
 from ..model import load_model
 from ..requests import LMInputs, Request
@@ -540,6 +540,7 @@ class ModelWorker:
                     self._vocoder_body(n)
                 self.pcm_host[:n].copy_(self.voc_pcm[:n], non_blocking=True)
             ds.synchronize()
+            check_waits()
             self.nvtx_range_pop()
             pcm_np = self.pcm_host.numpy()
             for i, (ri, ci, n_valid) in enumerate(mapping):
@@ -674,6 +675,7 @@ class ModelWorker:
             timing["lm_nodes"], timing["detok_nodes"] = n_lm, n_win + n_voc
         # ---- bring the host-side request state up to date ----
         torch.cuda.synchronize()
+        check_waits()
         hist = self.history.cpu()
         n_now = self.n_out.cpu()
         for i, req in enumerate(requests):

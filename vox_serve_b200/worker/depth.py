@@ -22,7 +22,7 @@ from typing import Coroutine, List, Optional
 import torch
 
 from .. import ops
-from .._lib import VoxB200Error
+from .._lib import VoxB200Error, check_waits
 from ..requests import Request
 from .base import CudaGraphWorker, I32
 
@@ -155,6 +155,7 @@ class DepthModelWorker(CudaGraphWorker):
             ready.synchronize()
             host = ids_host[:len(requests)].clone()
             cb0 = host[:, 0].tolist()
+            check_waits()
             for i, req in enumerate(requests):
                 row = host[i:i + 1]
                 req.input_tokens = row.clone()

@@ -24,7 +24,7 @@ import numpy as np
 import torch
 
 from .. import ops
-from .._lib import VoxB200Error
+from .._lib import VoxB200Error, check_waits
 from ..hybrid_engine import StepInputs
 from ..requests import LMInputs, Request
 from .base import CudaGraphWorker, I32, _Staging
@@ -228,7 +228,9 @@ class TextModelWorker(CudaGraphWorker):
         if any(not 0 <= i < buf.shape[0] for i in idx):
             raise VoxB200Error("logit row outside the engine's buffer")
         sel = torch.as_tensor(idx, dtype=torch.int64, device=buf.device)
-        return buf.index_select(0, sel).cpu()
+        rows = buf.index_select(0, sel).cpu()
+        check_waits()
+        return rows
 
     # ---- tokens out ---------------------------------------------------------------------------------------------
     def run_detokenize(self, requests: List[Request]):

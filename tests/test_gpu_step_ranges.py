@@ -339,6 +339,27 @@ def test_window_attention_unseen_keys(ops, D, H, G, page, new, old, window, chun
     _close(out.view(new, H, D), want, 2 ** -8)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("width", [1.0, 3.0])
+def test_prompt_attention_probabilities(ops, D, width):
+    """The attention core of prompt rows with fp32 output: probabilities are two bf16 terms (2^-17 together), their sum and the products
+    32-bit, whatever the reference of the exponents (one bf16 term against the exact maximum: 2^-10 or so)."""
+    H, new, L, page = 4, 256, 1000, 64
+    g = torch.Generator(device="cuda").manual_seed(D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")                 # noqa: E731
+    n = (L + page - 1) // page
+    q, k, v = (rnd(new, H, D) * width).bfloat16(), rnd(n * page, H, D).bfloat16(), rnd(n * page, H, D).bfloat16()
+    out = torch.full((new, H * D), float("nan"), device="cuda")
+    ops.window_attn(q.view(new, H * D), k.view(n, page, H, D), v.view(n, page, H, D), out, None, None, _i32(list(range(L - new, L))), _i32([0, n]),
+                    _i32(list(range(n))), new, H, H, D, D, 0, D ** -0.5, tiles=(_i32([0, new]), _i32(list([0] * 4)), _i32([0, 64, 128, 192]), 4))
+    s = torch.einsum("qhd,khd->hqk", q.double(), k[:L].double()) * D ** -0.5
+    s = s.masked_fill(torch.arange(L, device="cuda")[None] > torch.arange(L - new, L, device="cuda")[:, None], -float("inf"))
+    vd = v[:L].double().transpose(0, 1)
+    want = torch.softmax(s, -1) @ vd
+    err = ((out.view(new, H, D).transpose(0, 1).double() - want).norm() / want.norm()).item()
+    assert err <= 2.0 ** -15, err
+
+
 @pytest.mark.parametrize("T,N,S,resid,tiled,hidden", [
     (513, 8, 1, True, False, True), (514, 2048, 3, True, True, True), (600, 3072, 1, False, True, False), (515, 4096, 2, True, False, True),
     (516, 1032, 9, True, False, True), (1024, 264, 1, True, False, False),

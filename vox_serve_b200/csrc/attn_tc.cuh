@@ -190,16 +190,21 @@ __device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const 
       }
     }
     const float u = m_ref == -INFINITY ? 0.f : m_ref;          // every key masked so far
+    // a probability goes in as two bf16 terms, its rounding and what that left (relative 2^-17): the reference may lag, and the largest
+    // of a row, 1 and exact against the maximum itself, need not be a power of two
     float l0 = 0.f, l1 = 0.f;
-    uint32_t pk[32];
+    uint32_t ph[32], pl[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-      pk[i] = pack_bf16(ptc_ex2(fmaf(__uint_as_float(v[2 * i]), scale, -u)), ptc_ex2(fmaf(__uint_as_float(v[2 * i + 1]), scale, -u)));
-      l0 += bf16_lo(pk[i]);                                    // denominator from the rounded probabilities
-      l1 += bf16_hi(pk[i]);
+      const float p0 = ptc_ex2(fmaf(__uint_as_float(v[2 * i]), scale, -u)), p1 = ptc_ex2(fmaf(__uint_as_float(v[2 * i + 1]), scale, -u));
+      l0 += p0;
+      l1 += p1;
+      ph[i] = pack_bf16(p0, p1);
+      pl[i] = pack_bf16(p0 - bf16_lo(ph[i]), p1 - bf16_hi(ph[i]));
     }
     l_run += l0 + l1;
-    ptc_tmem_st32(sc, pk);
+    ptc_tmem_st32(sc, ph);
+    ptc_tmem_st32(sc + 32, pl);
     ptc_tmem_st_wait();
     tc_fence_before();
     mbar_arrive(&sh->p_full[j & 1]);
@@ -272,8 +277,10 @@ __device__ __forceinline__ void ptc_issue(uint8_t* smem, PtcShared* sh, int n_ti
     const uint64_t v_desc = umma_desc_sw128_mnmajor(smem_u32(smem + L::V + (j & 1) * L::TILE), PTC_KT * 128);
     if (elect_one()) {
 #pragma unroll
-      for (int k = 0; k < PTC_KT / 16; ++k)          // 16 tokens: 8 columns of probabilities, two 8-row groups of V
-        umma_bf16_ta(tmem + 128, tmem + (j & 1) * 64 + 8 * k, v_desc + k * (2048 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+      for (int k = 0; k < PTC_KT / 16; ++k) {        // 16 tokens: 8 columns of either term of the probabilities, two 8-row groups of V
+        umma_bf16_ta(tmem + 128, tmem + (j & 1) * 64 + 32 + 8 * k, v_desc + k * (2048 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+        umma_bf16_ta(tmem + 128, tmem + (j & 1) * 64 + 8 * k, v_desc + k * (2048 >> 4), idesc_o, 1u);
+      }
       umma_commit(&sh->v_empty[j & 1]);
       umma_commit(&sh->o_done);
       if (j + 1 == n_tiles) umma_commit(&sh->o_last);

@@ -9,8 +9,11 @@
 //    running maximum and denominator in registers (no shuffles: a row is one thread) and writes its probabilities (bf16) over
 //    the scores in TMEM, where they are the A operand of O += P V;
 //  * O stays in TMEM for the whole sequence.  The maximum that the exponents are taken against is only moved when a row's
-//    maximum has grown by more than 8 (base 2), and only then is O rescaled: probabilities stay below 2^8, in bf16 and fp32 as
-//    exact as below 1, and the final division uses the same denominator;
+//    maximum has grown by more than 8 (base 2), and only then is O rescaled.  Probabilities stay below 2^8 but a row's largest is no
+//    longer 1, which bf16 holds exactly (error before the output's own rounding 6.0e-4 -> 1.03e-3 for scores of standard deviation 3), so
+//    they are multiplied as two bf16 terms, rounding and remainder, side by side where the scores were.  997 rows on cached tokens, error
+//    after the output's rounding / a plan of two layers: 1.94e-3 / 89 us with one term and the lag, 1.92e-3 / 101 us with one term and
+//    the exact maximum (most tiles rescale), 1.59e-3 / 102 us with two terms and the lag;
 //  * warp 4 issues the MMAs: the scores of tile j + 1 are multiplied while the softmax works on tile j (two score buffers);
 //  * warps 5 and 6 bring K and V tiles as boxes of a tensor map over the paged cache (pages of a multiple of 8 tokens; cp.async
 //    per token row otherwise), the 128-byte-swizzled images that the MMAs read.  V is

@@ -89,6 +89,30 @@ def test_wide_projection(ops, T, N, K, tile_rows):
     assert _lib.load().vb_gemm_wide_timeouts() == 0
 
 
+@pytest.mark.parametrize("kind,scale,slope", [("silu", 1.0, 0), ("silu", 40.0, 0), ("silu", 2.0 ** -120, 0), ("glu", 1.0, 1.702), ("glu", 30.0, 1.702),
+                                              ("glu", 2.0 ** -92, 2.0 ** 92), ("glu", 2.0 ** -101, 2.0 ** 103)])
+def test_wide_gate_quotients(ops, kind, scale, slope):
+    """The gate/up epilogue against the same operations one by one, on two million gates: one value of the quotient that is not
+    the division's shows as soon as it lies next to where the output's rounding turns."""
+    T, N, K = 1024, 2048, 64
+    g = torch.Generator(device="cuda").manual_seed(int(scale * 7) + len(kind))
+    x = torch.randn(T, K, generator=g, device="cuda").bfloat16()
+    gate, up = ((torch.randn(N, K, generator=g, device="cuda") * K ** -0.5 * s).bfloat16() for s in (scale, 1.0))
+    gate[:8] = 0.0
+    pw = ops.pack_weight(ops.interleave_gate_up(gate, up, 64), 128)
+    gt, ut = (ops.gemm(x, ops.pack_weight(w, 128), mode=1)[0] for w in (gate, up))        # fp32 sums in the same order
+    if kind == "silu":
+        got = ops.gemm(x, pw, mode=2, tile_rows=128, n_out=N)
+        gr = gt.bfloat16().float()
+        want = ((gr / (1.0 + torch.exp(-gr))).bfloat16().float() * ut.bfloat16().float()).bfloat16()
+    else:
+        limit = 7.0
+        got = ops.gemm_glu(x, pw, torch.empty(T, N, dtype=torch.bfloat16, device="cuda"), limit, slope)
+        gr, ur = gt.clamp(max=limit), ut.clamp(-limit, limit)
+        want = ((gr / (1.0 + torch.exp(-slope * gr))) * (ur + 1.0)).bfloat16()
+    assert torch.equal(got, want), (got != want).sum().item()
+
+
 @pytest.mark.parametrize("groups,tt,N,K", [(1, 128, 256, 128), (3, 128, 320, 456), (5, 64, 128, 192)])
 def test_wide_grouped_projection(ops, groups, tt, N, K):
     g = torch.Generator(device="cuda").manual_seed(groups)

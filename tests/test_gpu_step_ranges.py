@@ -480,3 +480,17 @@ def test_a_wait_that_runs_out_is_reported(ops):
         _lib.call("vb_wait_check", 1000, 0, 1, ops._stream())
     with pytest.raises(_lib.VoxB200Error, match="outside"):
         _lib.call("vb_wait_check", -1, 0, 1, ops._stream())
+
+
+def test_snac_decoder_that_ends_wide(monkeypatch):
+    """A decoder whose last convolution has more channels than the channels-last one takes decodes channel-first."""
+    from vox_serve_b200.tokenizer.snac import SNAC
+
+    out = []
+    for plain in ("0", "1"):
+        monkeypatch.setenv("VB_SNAC_FP32", plain)
+        m = SNAC(decoder_dim=1024, decoder_rates=(4,), device="cuda")
+        m.load_state_dict(m.synthetic_state_dict(5))
+        codes = [torch.arange(n, device="cuda")[None] for n in (2, 4, 8)]
+        out.append(m.decode(codes, noises=[torch.zeros(*s, device="cuda") for s in m.noise_shapes(1, 8)]))
+    _close(out[0], out[1].double(), 1e-4)                # (tf32 halves cut off at 2^-20 beside plain 32-bit products)

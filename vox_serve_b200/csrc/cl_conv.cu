@@ -812,6 +812,8 @@ __global__ void __launch_bounds__(256) cl_chunk_attention_kernel(float* __restri
   }
 }
 
+static bool on16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }      // (a null pointer is)
+
 static int cl_sms() {
   static int sms = 0;
   if (!sms) {
@@ -838,6 +840,7 @@ long long vb_cl_pack_bytes(int N, int K) {
 
 int vb_cl_pack(void* d_dst, const float* d_w, int N, int K, void* stream) {
   VB_CHECK_ARG(d_dst && d_w, "vb_cl_pack: null pointer");
+  VB_CHECK_ARG(on16(d_dst) && on16(d_w), "vb_cl_pack: pointers must lie on 16-byte boundaries");
   VB_CHECK_ARG(vb_cl_pack_bytes(N, K) > 0, "vb_cl_pack: N = %d and K = %d must be positive multiples of 32", N, K);
   cl_pack_kernel<<<dim3(K / 32, (N * 8 + 2047) / 2048), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<float4*>(d_dst), d_w, N, K, N);
   VB_CHECK_LAUNCH();
@@ -857,10 +860,9 @@ int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, i
   VB_CHECK_ARG(epilogue != CE_SCALE_RESID || d_scale, "vb_cl_conv: the scaled residual needs d_scale");
   VB_CHECK_ARG(epilogue != CE_NOISE || d_noise, "vb_cl_conv: the noise epilogue needs d_noise");
   VB_CHECK_ARG(act != CA_SNAKE || d_alpha, "vb_cl_conv: Snake needs d_alpha");
-  VB_CHECK_ARG(reinterpret_cast<uintptr_t>(d_x) % 16 == 0 && x_bstride % 4 == 0 && reinterpret_cast<uintptr_t>(d_y) % 16 == 0 &&
-                   y_bstride % 4 == 0 && (!d_resid || (reinterpret_cast<uintptr_t>(d_resid) % 16 == 0 && r_bstride % 4 == 0)) &&
-                   (!d_y2 || reinterpret_cast<uintptr_t>(d_y2) % 16 == 0),
+  VB_CHECK_ARG(on16(d_x) && x_bstride % 4 == 0 && on16(d_y) && on16(d_y2) && y_bstride % 4 == 0 && on16(d_resid) && (!d_resid || r_bstride % 4 == 0),
                "vb_cl_conv: rows must start on 16-byte boundaries");
+  VB_CHECK_ARG(on16(d_w) && on16(d_bias) && on16(d_scale) && on16(d_alpha), "vb_cl_conv: weights, bias, scale and alpha must lie on 16-byte boundaries");
   if (B <= 0 || n_lo >= n_hi) return 0;
   // the epilogue addresses rows with 32-bit offsets from the first one: what is beyond that runs in several launches
   const long long per_entry = max(y_bstride, r_bstride);
@@ -939,6 +941,7 @@ int vb_cl_dwconv7(float* d_y, const float* d_x, long long x_bstride, const float
                   const float* d_alpha_out, int B, int C, int T, int dilation, int t_lo, int t_hi, void* stream) {
   VB_CHECK_ARG(d_y && d_x && d_w, "vb_cl_dwconv7: null pointer");
   VB_CHECK_ARG(C % 64 == 0 && dilation >= 1 && dilation <= 64 && x_bstride % 4 == 0, "vb_cl_dwconv7: C = %d (a multiple of 64), dilation %d", C, dilation);
+  VB_CHECK_ARG(on16(d_y) && on16(d_x) && on16(d_w) && on16(d_bias) && on16(d_alpha_in) && on16(d_alpha_out), "vb_cl_dwconv7: pointers must lie on 16-byte boundaries");
   VB_CHECK_ARG(0 <= t_lo && t_lo <= t_hi && t_hi <= T, "vb_cl_dwconv7: range [%d, %d) outside [0, %d)", t_lo, t_hi, T);
   if (B <= 0 || t_lo == t_hi) return 0;
   VB_CHECK_CUDA(max_dyn_smem_once(cl_dwconv7_kernel));
@@ -951,6 +954,7 @@ int vb_cl_last_conv(float* d_y, const float* d_x, long long x_bstride, const flo
                     int ksize, int left, int t0, int t1, int use_tanh, void* stream) {
   VB_CHECK_ARG(d_y && d_x && d_w && d_bias, "vb_cl_last_conv: null pointer");
   VB_CHECK_ARG(C % 4 == 0 && C <= 256 && ksize >= 1 && ksize <= 16 && x_bstride % 4 == 0, "vb_cl_last_conv: C = %d, ksize %d", C, ksize);
+  VB_CHECK_ARG(on16(d_x), "vb_cl_last_conv: rows must start on 16-byte boundaries");
   VB_CHECK_ARG(0 <= t0 && t0 < t1 && t1 <= T, "vb_cl_last_conv: bad output range [%d, %d) of %d", t0, t1, T);
   if (B <= 0) return 0;
   VB_CHECK_CUDA(max_dyn_smem_once(cl_last_conv_kernel));
@@ -988,6 +992,7 @@ int vb_cl_upsample(float* d_y, const float* d_x, const float* d_w, int B, int C,
 
 int vb_cl_layernorm(float* d_y, const float* d_x, const float* d_w, const float* d_b, int rows, int C, float eps, void* stream) {
   VB_CHECK_ARG(d_y && d_x && d_w && d_b, "vb_cl_layernorm: null pointer");
+  VB_CHECK_ARG(on16(d_y) && on16(d_x) && on16(d_w) && on16(d_b), "vb_cl_layernorm: pointers must lie on 16-byte boundaries");
   VB_CHECK_ARG(C > 0 && C % 4 == 0 && C <= 1024, "vb_cl_layernorm: C = %d (a multiple of 4, <= 1024)", C);
   if (rows <= 0) return 0;
   VB_LAUNCH_PDL(cl_layernorm_kernel, (rows + 3) / 4, 128, 0, stream, d_y, d_x, d_w, d_b, rows, C, eps);
@@ -996,6 +1001,7 @@ int vb_cl_layernorm(float* d_y, const float* d_x, const float* d_w, const float*
 
 int vb_cl_chunk_attention(float* d_out, const float* d_qkv, int B, int C, int H, int T, float max_period, void* stream) {
   VB_CHECK_ARG(d_out && d_qkv, "vb_cl_chunk_attention: null pointer");
+  VB_CHECK_ARG(reinterpret_cast<uintptr_t>(d_qkv) % 8 == 0, "vb_cl_chunk_attention: rows must start on 8-byte boundaries");
   VB_CHECK_ARG(H >= 1 && C % H == 0 && (C / H) % 4 == 0 && C / H <= 256 && T >= 1 && T <= 64, "vb_cl_chunk_attention: C %d, H %d, T %d (<= 64)", C, H, T);
   if (B <= 0) return 0;
   const size_t smem = (static_cast<size_t>(3) * T * (C / H + 4) + static_cast<size_t>(T) * (T + 1) + C / H / 2) * sizeof(float);

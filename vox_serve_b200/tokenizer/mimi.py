@@ -53,6 +53,15 @@ class MimiConfig:
         return self.upsample_stride * math.prod(self.ratios)
 
 
+def fits_channels_last(cfg: MimiConfig) -> bool:
+    """Every width a multiple of 32 channels (the deployed configuration), and what the channels-last kernels hold in registers and
+    shared memory: the decoder runs channels-last (_cl.py).  Heads of more than 128 dims run in neither form."""
+    last, head = cfg.n_filters, cfg.dimension // cfg.num_heads
+    widths = [cfg.dimension, cfg.codebook_dim, cfg.dim_feedforward, last] + [last * 2 ** i // cfg.compress for i in range(len(cfg.ratios))]
+    return (all(n % 32 == 0 and n > 0 for n in widths) and cfg.dimension <= 1024 and last <= 256 and cfg.last_kernel_size <= 16 and
+            cfg.n_q <= 64 and cfg.dimension % cfg.num_heads == 0 and head % 4 == 0 and head <= 128)
+
+
 def seanet_layout(cfg: MimiConfig) -> List[Tuple[str, int]]:
     """[(kind, index in decoder.model)] in execution order (SEANetDecoder.__init__, mimi.py:2625-2693)."""
     out, i = [("conv_in", 0)], 1
@@ -197,14 +206,8 @@ class MimiDecoder:
         return self
 
     def _pack_channels_last(self, kinds) -> bool:
-        """Every width a multiple of 32 channels (the deployed configuration): the decoder runs channels-last (_cl.py)."""
         cfg = self.cfg
-        last = cfg.n_filters
-        widths = [cfg.dimension, cfg.codebook_dim, cfg.dim_feedforward, last] + [
-            last * 2 ** i // cfg.compress for i in range(len(cfg.ratios))]
-        if not (_tc.tc_enabled() and self.device.type == "cuda" and all(n % 32 == 0 and n > 0 for n in widths) and cfg.dimension <= 1024 and
-                last <= 256 and cfg.n_q <= 64 and cfg.dimension % cfg.num_heads == 0 and (cfg.dimension // cfg.num_heads) % 4 == 0 and
-                (cfg.dimension // cfg.num_heads) <= 256):
+        if not (_tc.tc_enabled() and self.device.type == "cuda" and fits_channels_last(cfg)):
             return False
         for k, v in self.w.items():
             if k in ("rvq_first.proj", "rvq_rest.proj") or (k[0] == "t" and k.split(".")[-1] in ("in", "out", "l1", "l2")):

@@ -126,6 +126,12 @@ class SNAC:
             self.noise_state = torch.tensor([seed ^ 0x534E4143, 0, 0], dtype=torch.int64, device=dev)
         return self.noise_state
 
+    def _fits_channels_last(self) -> bool:
+        """Every width a multiple of 64 channels (the deployed configuration): the whole decoder runs channels-last (_cl.py).  Its last
+        convolution keeps a row of at most 256 channels in shared memory; a decoder that ends wider stays channel-first."""
+        n = len(self.decoder_rates)
+        return self.latent_dim % 64 == 0 and self.decoder_dim % (64 << n) == 0 and self.decoder_dim >> n <= 256
+
     def _pack_tensor_core_weights(self):
         """The 1x1 and transposed-conv weights whose input width is a multiple of 32 channels are re-tiled for the
         tcgen05 tf32 hi/lo kernel (vb_snac_pack_tf32x3); narrower layers (test-sized configs) stay on the SIMT
@@ -134,8 +140,7 @@ class SNAC:
         self.channels_last = False
         if self.device.type != "cuda" or os.environ.get("VB_SNAC_FP32", "0") == "1":
             return
-        # every width a multiple of 64 channels (the deployed configuration): the whole decoder runs channels-last (_cl.py)
-        if self.latent_dim % 64 == 0 and self.decoder_dim % (64 << len(self.decoder_rates)) == 0:
+        if self._fits_channels_last():
             self.channels_last = True
             for k, v in self.w.items():
                 if k.endswith(("pw_w", "noise_w")):

@@ -363,6 +363,39 @@ def test_window_attention_unseen_keys(ops, D, H, G, page, new, old, window, chun
     _close(out.view(new, H, D), want, 2 ** -8)
 
 
+# boxes of 8, 16, 32 and 64 tokens and pages that no box divides (copied row by row); requests that end on a key tile, one before and one
+# behind it; rows that see one tile, two, several; heads per key head from one to a whole row tile
+@pytest.mark.parametrize("page", [8, 24, 16, 32, 96, 64, 192, 1, 5, 20, 66])
+@pytest.mark.parametrize("D,H,G,kv,new", [(128, 6, 2, [63, 64, 65], [63, 1, 65]), (64, 4, 4, [127, 129, 300], [127, 70, 40]), (128, 64, 1, [1, 130], [1, 3])])
+def test_paged_prompt_attention_pages(ops, page, D, H, G, kv, new):
+    from vox_serve_b200 import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(page)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()      # noqa: E731
+    pages = [(x + page - 1) // page for x in kv]
+    ip = np.concatenate([[0], np.cumsum(pages)]).tolist()
+    idx = (np.random.RandomState(page).permutation(ip[-1]) + 1).tolist()
+    T, pad, base = sum(new), 3, 2
+    cache = torch.full((base + ip[-1] + 1, 2, page, G, D), float("nan"), device="cuda").bfloat16()       # what no request has written
+    q, want, at = rnd(T + pad, H, D), [], 0
+    for b, L in enumerate(kv):
+        k, v, tok = rnd(L, G, D), rnd(L, G, D), torch.arange(L, device="cuda")
+        pg = torch.tensor(idx[ip[b]:ip[b + 1]], device="cuda")[tok // page] + base
+        cache[pg, 0, tok % page], cache[pg, 1, tok % page] = k, v
+        s = torch.einsum("qhd,khd->hqk", q[at:at + new[b]].double(), k.double().repeat_interleave(H // G, 1)) * D ** -0.5
+        s = s.masked_fill(tok[None] > torch.arange(L - new[b], L, device="cuda")[:, None], -float("inf"))
+        want.append(torch.einsum("hqk,khd->qhd", torch.softmax(s, -1), v.double().repeat_interleave(H // G, 1)))
+        at += new[b]
+    plan = ops.RowPlan(T + pad, "cuda")
+    chunk = page
+    ops.plan_rows(plan, _i32([0] + np.cumsum(new).tolist()), _i32(ip), _i32(idx), _i32([(x - 1) % page + 1 for x in kv]), len(kv), T + pad, page, chunk)
+    out = torch.full((T + pad, H, D), 7.0, device="cuda").bfloat16()
+    ops.paged_attn(q, cache, base, plan, T + pad, G, page, chunk, None, out=out, prefill_tiles="tc")
+    _close(out[:T], torch.cat(want), 2 ** -8)        # probabilities and the output rounded to bf16
+    assert (out[T:] == 0).all()
+    assert _lib.load().vb_prefill_attn_tc_timeouts() == 0
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("width", [1.0, 3.0])
 def test_prompt_attention_probabilities(ops, D, width):

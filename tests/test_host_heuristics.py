@@ -95,9 +95,9 @@ def test_tf32_hi_lo_split_is_fp32_grade():
     assert err1.max() > 50 * err3.max()
 
 
-def test_prefill_kernel_selection_rules():
-    """Which attention kernel a plan runs on is a host-side decision on shapes only (ops.use_prefill_tiles /
-    use_prefill_tc): stable under CUDA-graph capture, no device read."""
+def test_prefill_kernel_selection_rules(monkeypatch):
+    """Which attention kernel a plan runs on is a host-side decision on shapes only (ops.use_prefill_tiles): stable under
+    CUDA-graph capture, no device read.  Prefill-shaped plans run on the tcgen05 kernel unless VB_PREFILL_TC is 0."""
     from types import SimpleNamespace
 
     def plan(n_req, prefill=True):
@@ -109,10 +109,9 @@ def test_prefill_kernel_selection_rules():
     assert not ops.use_prefill_tiles(plan(64), 128, 128, 32)                      # 2-row depth-decoder prefill, batch 64
     assert not ops.use_prefill_tiles(plan(16), 32, 128, 32)
     assert not ops.use_prefill_tiles(plan(1), 133, 96, 128)                       # head_dim the tiled kernels do not take
-    assert not ops.use_prefill_tc(plan(1), 435) and not ops.use_prefill_tc(plan(16), 800)
-    assert not ops.use_prefill_tc(plan(32), 956)                                   # 7 prompts among 25 decode rows
-    assert ops.use_prefill_tc(plan(4), 2400) and ops.use_prefill_tc(plan(1), 600)  # long prompts: the tcgen05 tiles
-    assert ops.use_prefill_tc(plan(8), 1064)                                       # ... and big batches of prompts
+    for env, entry in (("auto", "vb_paged_prefill_attn_tc"), ("1", "vb_paged_prefill_attn_tc"), ("0", "vb_paged_prefill_attn")):
+        monkeypatch.setattr(ops, "_PREFILL_TC", env)
+        assert ops._prefill_entry() == entry
 
 
 def test_speech_tokenizer_config_and_mask_bounds():

@@ -300,24 +300,15 @@ def prefill_attn_tile_rows(n_q: int, n_kv: int) -> int:
 
 
 _PREFILL_TILES = os.environ.get("VB_PREFILL_TILES", "auto")      # "0": never, "1": every prefill plan, "auto": by shape
-# which tiled prefill kernel: "auto" / "1" = tcgen05, "0" = mma.sync
+# which tiled prefill kernel: "0" = mma.sync, anything else tcgen05
 _PREFILL_TC = os.environ.get("VB_PREFILL_TC", "auto")
 
 
-def use_prefill_tc(plan: "RowPlan", n_rows: int) -> bool:
-    """Long prompts and big batches of prompts, by shape: where the tcgen05 kernel's row tiles are well filled."""
-    if _PREFILL_TC in ("0", "1"):
-        return _PREFILL_TC == "1"
-    n_req = max(1, plan.n_req)
-    return n_rows >= 512 * n_req or (n_rows >= 1024 and n_rows >= 128 * n_req)
-
-
-def _prefill_entry(plan: "RowPlan", n_rows: int) -> str:
-    """The kernel of a prefill-shaped plan.  Measured per launch, mma.sync / tcgen05 (us): 4 x 600 rows 75 / 33, 8 x 133 rows 29 / 13;
-    of the plans ``use_prefill_tc`` does not name, one 133-row prompt 12.0 / 9.2, 31 decode rows beside a 133-row prompt 53 / 22,
-    one of 435 rows 28 / 14, 16 x 50 rows 10.1 / 10.0, 16 x 24 rows 8.8 / 9.1 (the one where most of a 128-row tile is padding) -- so
-    only VB_PREFILL_TC=0 still picks mma.sync."""
-    return "vb_paged_prefill_attn_tc" if use_prefill_tc(plan, n_rows) or _PREFILL_TC == "auto" else "vb_paged_prefill_attn"
+def _prefill_entry() -> str:
+    """The kernel of a prefill-shaped plan.  Measured per launch, mma.sync / tcgen05 (us): 4 x 600 rows 75 / 33, 8 x 133 rows 29 / 13,
+    one 133-row prompt 12.0 / 9.2, 31 decode rows beside a 133-row prompt 53 / 22, one of 435 rows 28 / 14, 16 x 50 rows 10.1 / 10.0,
+    16 x 24 rows 8.8 / 9.1 (the one where most of a 128-row tile is padding)."""
+    return "vb_paged_prefill_attn" if _PREFILL_TC == "0" else "vb_paged_prefill_attn_tc"
 
 
 def use_prefill_tiles(plan: RowPlan, n_rows: int, head_dim: int, page_size: int) -> bool:
@@ -359,7 +350,7 @@ def paged_attn(q: torch.Tensor, kv_cache, slab_base: int, plan: RowPlan, n_rows:
     if tiles:
         assert plan.qo_indptr is not None, "the tiled prefill kernel needs a prefill plan (qo_indptr)"
         fn = "vb_paged_prefill_attn_tc" if prefill_tiles == "tc" else (
-            _prefill_entry(plan, n_rows) if prefill_tiles is None else "vb_paged_prefill_attn")
+            _prefill_entry() if prefill_tiles is None else "vb_paged_prefill_attn")
         call(fn, out_ptr, q.data_ptr(), kv_cache.data_ptr(), int(slab_base),
              plan.qo_indptr.data_ptr(), plan.kv_indptr.data_ptr(), plan.kv_indices.data_ptr(),
              plan.row_kvlen.data_ptr(), plan.n_req, n_rows, n_q, n_kv, d, page_size, sc, xt, _stream())

@@ -171,6 +171,60 @@ def test_channels_last_conv_reuses_stages(B, T, C, N, ksize):
         assert torch.equal(_cl.conv(xa, wp, N, ksize=ksize).tensor(), y)
 
 
+def _activated(values, act, alpha=None):
+    """The epilogue's activation of given fp32 values: a convolution of zeros with the values as its residual"""
+    from vox_serve_b200.tokenizer import _cl
+
+    n = values.numel() // 32
+    zero = _cl.Act(torch.zeros(n * 32, device="cuda"), 1, n, 32)
+    w = _cl.pack(torch.zeros(32, 32, device="cuda"))
+    return _cl.conv(zero, w, 32, epi="resid", resid=_cl.Act(values, 1, n, 32), act=act, alpha=alpha).tensor().reshape(-1).double()
+
+
+def test_vocoder_activations_over_their_range():
+    """The polynomials against 64 bits: ELU down to where it is -1, the squared sine to the end of its reduction and past it."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    u = torch.rand(1 << 20, generator=g, device="cuda")
+    neg = torch.cat((-90 * u, -2.0 ** (-140 * u), torch.tensor([0.0, -0.0, -80.0, -1e4, 1.5, 3e38] + [0.0] * 26, device="cuda")))
+    v = neg.double()
+    want = torch.where(v > 0, v, torch.expm1(v))
+    got = _activated(neg, "elu")
+    assert ((got - want).abs() <= 1e-7 * want.abs() + 2.0 ** -149).all()
+    # value + scale sin^2: the scale brings the square to the top of the sum.  Three roundings of a remainder of up to pi / 2
+    scale = 2.0 ** 24
+    table = torch.cat((torch.ones(32, device="cuda"), torch.full((32,), scale, device="cuda")))
+    for top, bound in ((4.0, 5e-7), (65536.0, 5e-7), (1e6, 5e-7)):
+        x = (2 * u - 1) * top
+        got = (_activated(x, "snake", table) - x.double()) / scale
+        assert ((got - torch.sin(x.double()) ** 2).abs() <= bound + x.double().abs() * 2.0 ** -24 / scale).all(), top
+    x = 2.0 ** (-20 * u)                                  # small arguments keep their relative accuracy
+    got = (_activated(x, "snake", table) - x.double()) / scale
+    assert ((got - torch.sin(x.double()) ** 2).abs() <= 5e-7 * torch.sin(x.double()) ** 2 + x.double() * 2.0 ** -23 / scale).all()
+
+
+@pytest.mark.parametrize("entries,rows,N,far", [(3, 40, 32, (1 << 30) + 64), (1, (1 << 20) + 300, 1024, 0), (2, 150, 64, (1 << 30) - 64)])
+def test_channels_last_conv_past_32_bit_offsets(entries, rows, N, far):
+    """Batch entries 2^30 floats apart and results of more than 2^30 floats run in several launches."""
+    from vox_serve_b200.tokenizer import _cl
+
+    C, B, T = 32, entries, rows
+    g = torch.Generator(device="cuda").manual_seed(N)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")                 # noqa: E731
+    x, w, b = rnd(B, T, C), rnd(N, C) * C ** -0.5, rnd(N)
+    r, nz = (rnd(B, T, N), rnd(B, T)) if far else (None, None)
+    y = torch.empty((B - 1) * far + T * N, device="cuda")
+    from vox_serve_b200 import ops
+    from vox_serve_b200._lib import call
+
+    call("vb_cl_conv", y.data_ptr(), None, x.data_ptr(), T * C, T, _cl.pack(w).data_ptr(), b.data_ptr(), None if r is None else r.data_ptr(), T * N, None,
+         None if nz is None else nz.data_ptr(), T, None, 3 if far else 0, 0, B, C, N, N, 1, 1, 0, T, far if far else T * N, ops._stream())
+    for i in range(B):
+        got = y[i * far:i * far + T * N].view(T, N)
+        for c in (slice(0, 200), slice(T - 400 if T > 400 else 0, T)):
+            ref = x[i, c].double() @ w.double().T + b.double()
+            _close(got[c], ref if r is None else r[i, c] + nz[i, c, None] * ref, 5e-6)
+
+
 def _bits(*codes):
     return torch.tensor([c - (1 << 32) if c >> 31 else c for c in codes], dtype=torch.int32, device="cuda").view(torch.float32)
 

@@ -153,9 +153,9 @@ int vb_paged_prefill_attn(void* d_out, const void* d_q, const void* d_kv, int64_
                           int page_size, float sm_scale, int out_xt_tile, void* stream);
 
 /* The same operator on the 5th-generation tensor cores: both contractions as tcgen05.mma from swizzled shared-memory
- * operand tiles, S and the per-tile P V product in TMEM, the GQA group folded into the MMA's 128 accumulator rows (a Q
- * tile = 128 / group prompt rows of one request), K/V tiles of 128 tokens (any page size).  Arguments as
- * vb_paged_prefill_attn. */
+ * operand tiles, scores, probabilities and the whole output row in TMEM, the GQA group folded into the MMA's 128 accumulator rows (a Q
+ * tile = 128 / group prompt rows of one request), K/V tiles of 64 tokens -- boxes of a tensor map where the page size is a multiple of
+ * 8, row by row for any other.  Arguments as vb_paged_prefill_attn. */
 int vb_prefill_attn_tc_timeouts(void);      /* as vb_gemm_wide_timeouts */
 int vb_window_attn_tc_timeouts(void);
 int vb_prefill_attn_tc_tile_rows(int n_q, int n_kv);

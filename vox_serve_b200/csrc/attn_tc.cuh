@@ -8,7 +8,10 @@
 //   finish(m_ref, l)         factor for the accumulated row, given the exponents' reference and the denominator against it
 //   store(c0, o, f)          32 output values from column c0, times the factor
 //   HOLE, hole0, hole1       keys [hole0, hole1) are seen by no row of the block: they are neither fetched nor multiplied
-// See prefill_attn_tc.cu for the schedule and what bounds it.
+// The running maximum, its rescale and the division at the end are the online softmax of M. Milakov and N. Gimelshein ("Online normalizer
+// calculation for softmax", 2018) as FlashAttention walks it over key tiles (T. Dao et al., 2022); the roles of the warps and scores
+// multiplied one tile ahead follow the published schedule of FlashAttention-3 (J. Shah et al., 2024).
+// See prefill_attn_tc.cu for the schedule here and what bounds it.
 #pragma once
 #include "common.cuh"
 #include <cudaTypedefs.h>

@@ -16,7 +16,7 @@
 // Roles of a CTA's eighteen warps: 0 copies (activation box and two weight tiles per stage), 1 issues the MMAs, 2..5 split a
 // stage's raw activations into the two halves and put them into TMEM as the MMA's A operand (128 x 32 columns each; through
 // shared memory the operand would cost 12 KB of its bandwidth per 8-deep product, and the two tiles another 32 KB of stores),
-// 6..17 are the epilogue.  Persistent CTAs, two accumulators, 4 to 7 stages (TMEM and shared memory both bound them).
+// 6..17 are the epilogue.  Persistent CTAs, two accumulators, 4 stages (6 where column tiles are 32 wide): TMEM bounds them.
 // The width of a column tile (32, 64 or 128) is chosen per launch from the number of tiles: a transformer layer of 640 rows
 // has 5 x 4 tiles of 128.
 // What bounds it: wide layers of few positions are one chain of 32-deep k-blocks (0.41 us each, the split into halves), narrow
@@ -34,7 +34,7 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn();      // api.cu
 
 constexpr int CL_THREADS = 576;
 constexpr int CL_A_BYTES = 128 * 128;       // 128 positions x 32 channels
-constexpr int CL_MAX_STAGES = 7;
+constexpr int CL_MAX_STAGES = 6;            // 512 TMEM columns less two accumulators, 64 a stage
 constexpr int CL_EPI_WARPS = 12;
 constexpr int CL_EPI_BYTES = CL_EPI_WARPS * 2048;      // a transpose of 32 rows x 16 columns per epilogue warp
 

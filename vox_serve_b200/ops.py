@@ -372,9 +372,11 @@ def gemm_t_tile(T: int) -> int:
     return _lib.load().vb_gemm_t_tile(int(T))
 
 
-# Steps of more rows than this run their projections on the kernel for pairs of SMs (gemm_wide.cu): from 80 rows on it is
-# as fast or faster on every projection measured (80 rows: QKV 11.1 against 12.3 us, gate/up 25.1 against 27.4, down 13.0
-# against 14.5; 1024 rows: 32 / 63, 77 / 171, 38 / 79); up to 64 rows the one-SM kernel's layouts and fused tails apply.
+# Steps of this many rows or more run their projections on the kernel for pairs of SMs (gemm_wide.cu); up to 64 rows the one-SM
+# kernel's layouts and fused tails apply.  Per launch, one-SM kernel / this one (us, graph of launches, weights cold): 65 rows, QKV
+# 5120 x 3072 11.0 / 9.0, O 3072 x 3072 9.9 / 7.4, gate/up 16384 x 3072 24.6 / 20.1, down 3072 x 8192 13.1 / 11.7; narrower, 3072 x 2048
+# 10.4 / 6.3, 2048 x 8192 12.0 / 9.4, 1536 x 1024 10.2 / 4.9, 6144 x 1024 14.2 / 8.1, 1024 x 3072 8.9 / 5.0; 79 rows the same to 0.5 us;
+# 1024 rows: 63 / 32, 171 / 77, 79 / 38 (QKV, gate/up, down).
 WIDE_MIN_ROWS = 65
 WIDE_TILE_ROWS = (32, 64, 96, 128)
 WIDE_SPLIT_ROWS = 1664       # most (split x rows) of fp32 planes a projection is split into

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Headline benchmark: Orpheus-3B streaming TTS, batch 32 per GPU, SNAC codec path (BASELINE.json configs[1]).
+"""Headline benchmark: Orpheus-3B streaming TTS, batch 32 per GPU, SNAC codec path.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
@@ -21,7 +21,7 @@ Two figures per run, same state, same K steps:
 TTFA (time to first audio chunk, benchmark/goodput.py:250-262) is reported for a lone request, for a request joining
 31 running streams, and for a burst of 32 -- the burst with the reference's one-prefill-per-step policy and, separately,
 with prompts batched into shared prefill steps.
-N > 1: one replica per GPU (request-parallel, no data-path collective; SURVEY.md §8e), barrier + max over ranks.
+N > 1: one replica per GPU (request-parallel, no data-path collective), barrier + max over ranks.
 --impl reference: the CPU oracle port of the reference's path (oracle/), all host threads, bounded sample.
 """
 from __future__ import annotations
@@ -428,7 +428,7 @@ def run_gpu(args):
     ttfa_single.sort()
 
     # ------------------------------------------------ steady-state TTFA: one request joins 31 running streams ------
-    # ("define TTFA as steady-state (one request joining 31 running streams)"; goodput.py:250-262: first
+    # (steady state: one request joins 31 running streams; goodput.py:250-262: first
     # audio chunk arrival - request start.)  The joining prefill rides in the same step as the 31 decodes.
     ttfa_join = []
     if joins > 0:
@@ -512,7 +512,7 @@ def kernel_rooflines(worker, model, reqs, torch, ops):
     """Times, with CUDA events on the launching stream, (a) all projection GEMM launches of one decode step and
     (b) the 28 paged-attention launches of one step, each as a CUDA graph replayed back to back on the live
     buffers (weights of 28 different layers: 6.6 GB per replay, far beyond L2).  Average launch duration =
-    replay time / launches; achieved = algorithmic bytes / time (DESIGN.md §roofline)."""
+    replay time / launches; achieved = algorithmic bytes / time."""
     eng = model.engine_for(worker.kv_cache, worker.page_size)
     d, B = eng.dims, len(reqs)
     H, I, V = d.hidden_size, d.intermediate_size, d.vocab_size

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Open-loop streaming benchmark (the shape of BASELINE.json configs[2]: continuous batching under Poisson arrivals
+"""Open-loop streaming benchmark (continuous batching under Poisson arrivals
 on 1/2/4/8 replicas), with the metric definitions of the reference's own client (benchmark/goodput.py):
 
   * arrivals: inter-arrival ~ Gamma(k = burstiness = 1, theta = 1/rate), seed 42          (goodput.py:354-363)

@@ -1,6 +1,5 @@
 /*
- * vb_api.h -- C ABI of libvoxb200.so: the B200 (sm_100a) kernels behind VoxServe's operator boundary
- * (level b4).
+ * vb_api.h -- C ABI of libvoxb200.so: the B200 (sm_100a) kernels behind VoxServe's operator boundary.
  *
  * Conventions
  *   - every pointer named d_* / *_dev is a DEVICE pointer; tensors are dense row-major unless a stride
@@ -76,7 +75,7 @@ int vb_rope(void* d_q_out, void* d_k_out, const void* d_q, const void* d_k, cons
  * qo_indptr == NULL means decode (one row per request).  d_kv_len (optional, [B]) gives each request's kv
  * length explicitly -- then the page table may hold pre-allocated pages beyond it and last_page_len is
  * ignored (device-resident decode loop; the reference derives the length from the table, :96-97).  Rows >= n_rows_valid up to n_rows_padded get
- * page = -1 (their K/V append is skipped; the reference scatters them into page -1, see DESIGN.md).
+ * page = -1 (their K/V append is skipped; the reference scatters them into page -1).
  * Outputs (device int32): row_req[R], row_kvlen[R], row_page[R], row_slot[R], row_chunk_start[R+1] (exclusive
  * prefix of ceil(kvlen / chunk_tokens): the attention kernel's work list), row_pagebase[R] (= kv_indptr of the
  * row's request, so the attention kernel resolves a tile's page with one load) and row_old[R] (tokens of the
@@ -113,7 +112,7 @@ int vb_avgpool_rows(void* d_out, const void* d_in, int T, int D, int k, void* st
 int vb_vq_argmin(int64_t* d_ids, const float* d_acc, const void* d_x, const void* d_c2, int T, int N, int D,
                  void* stream);
 
-/* ---- whole-page gather / scatter (prefill-KV hand-off between replicas, SURVEY.md section 8e; the reference pins a
+/* ---- whole-page gather / scatter (prefill-KV hand-off between replicas; the reference pins a
  * request to one replica, launch.py:471-474, and has no such transfer).  d_cache: the whole cache
  * [n_layers][pages_per_layer][page_bytes]; d_staging: [n_layers][n_pages][page_bytes] contiguous (what goes on the
  * wire); d_page_ids [n_pages] int32 (device).  to_cache = 0: staging <- cache (sender), 1: cache <- staging (receiver). */

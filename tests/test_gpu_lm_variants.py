@@ -1,6 +1,5 @@
-"""The CosyVoice2 and GLM-4-Voice decoder stacks on the sm_100a engine (BASELINE.json
-configs[0] and configs[4]'s LM): q / k / v bias, biased output head, embeddings-in prefill, rotation of half of every head in
-(even, odd) pairs, fused gate | up weights.  Checked against the golden files produced by the reference's own
+"""The CosyVoice2 and GLM-4-Voice decoder stacks on the sm_100a engine (q / k / v bias, biased output head, embeddings-in prefill, rotation of half of every head in
+(even, odd) pairs, fused gate | up weights).  Checked against the golden files produced by the reference's own
 ``CosyVoice2ForCausalLM`` / ``GLMVoiceForCausalLM`` on CPU (tests/golden/cosyvoice2_tiny_lm.npz, glm_voice_tiny_lm.npz):
 prefill + greedy decode steps across two page boundaries, teacher-forced with the golden ids, every step's logits within
 2 % of the row scale and the argmax equal unless the golden's own top-2 margin is a near-tie."""

@@ -25,7 +25,7 @@
 //    online-softmax state across tiles.  Tokens are the MMA M dimension: S^T = K Q^T (mma.sync m16n8k16, the G
 //    grouped query heads are the N columns), P^T is transposed in registers with movmatrix, O^T += V^T P^T;
 //    exp2 via ex2.approx, P rounded to bf16 and the denominator summed from the rounded P (FlashInfer FA2
-//    numerics, SURVEY.md section 7).  No block-wide synchronisation per tile -- only at the end of a segment;
+//    numerics).  No block-wide synchronisation per tile -- only at the end of a segment;
 //  * a row that spans several CTAs leaves one partial per CTA; the last CTA to arrive (one atomic per segment)
 //    merges them in CTA order (deterministic) and restores the arrival counter to 0.
 #include "../../include/vb_api.h"

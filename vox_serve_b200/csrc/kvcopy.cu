@@ -1,7 +1,7 @@
 // Whole-page gather / scatter between the paged KV cache and a contiguous staging buffer: the device half of the
-// prefill-KV hand-off between replicas ("[L, n_pages, 2, page, Hkv, D] slices over NVLink").
-// The reference has no such path (one replica serves a request for its lifetime, vox_serve/launch.py:471-474);
-// north_star names it as the one optional NCCL transfer.  Pure HBM copy: 16-byte vectors, four independent loads in
+// prefill-KV hand-off between replicas ([L, n_pages, 2, page, Hkv, D] slices over NVLink).
+// The reference has no such path (one replica serves a request for its lifetime, vox_serve/launch.py:471-474).
+// Pure HBM copy: 16-byte vectors, four independent loads in
 // flight per thread, a grid of a few CTAs per SM.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 4

@@ -1,4 +1,4 @@
-"""Backbone + depth-transformer frame step on the sm_100a kernels (SURVEY.md §8 rows a24 / f1).
+"""Backbone + depth-transformer frame step on the sm_100a kernels.
 
 The reference runs one audio frame of a multi-codebook model as 1 backbone graph replay + (N - 1) depth graph replays,
 each with a FlashInfer plan, two device synchronisations and a ``.item()`` per request between them

@@ -1,6 +1,6 @@
 """GLM-4-Voice speech tokenizer on the B200 kernels: the Whisper-style VQ encoder that turns the log-mel features of
-a spoken prompt into ``<|audio_N|>`` ids (``vox_serve/encoder/glm.py:84-369``; the STS prompt side, SURVEY.md §8f
-row 3).  Same class names, constructor arguments and call signatures as the reference module:
+a spoken prompt into ``<|audio_N|>`` ids (``vox_serve/encoder/glm.py:84-369``; the prompt side of
+speech to speech).  Same class names, constructor arguments and call signatures as the reference module:
 ``GLMWhisperVQEncoder(config)(input_features, attention_mask) -> ids`` and ``GLMVoiceEncoder(...).encode(audio)``.
 
 How it maps to the kernels (everything bf16, token-major ``[T][C]``, rounded where the reference's bf16 modules round):

@@ -2,7 +2,7 @@
 (vox_serve/model/orpheus.py:125-221) as a fixed sequence of C-ABI launches over preallocated buffers, so
 the whole step is CUDA-graph capturable (no host sync, no allocation).
 
-Decode-sized steps (<= 64 rows), 5 launches per layer (the reference issues ~18-20, SURVEY.md §8 a10):
+Decode-sized steps (<= 64 rows), 5 launches per layer (the reference issues ~18-20):
     [RMSNorm -> QKV projection -> RoPE -> KV append]  ->  paged attention
     -> [O projection -> + residual (+ sums of squares for the next norm)]
     -> [RMSNorm -> gate/up projection -> SiLU * up]  ->  [down projection -> + residual (+ sums of squares)]
@@ -240,7 +240,7 @@ class LlamaEngine:
         tile, i.e. 12-20 units per projection on 74 pairs of SMs without a split, a 1024-row step needs none."""
         if rows <= self.FUSED_MAX_ROWS:
             return self.split_qkv, self.split_o, self.split_down
-        if os.environ.get("VB_PREFILL_SPLIT", "1") == "0":           # (A/B switch: round-1 behaviour)
+        if os.environ.get("VB_PREFILL_SPLIT", "1") == "0":           # (A/B switch: no split of prompt steps)
             return 1, 1, 1
         key = rows
         if key not in self._split_cache:
@@ -297,7 +297,7 @@ class LlamaEngine:
     # kernels 2.61 ms per forward, the norm-/residual-fused projections 2.95 ms (VB_DECODE_MODE=fused; value 130 vs 142.7
     # audio-s/s, batch-1 TTFA 68 vs 62 ms): their cluster-reduced epilogues cost more than the launches they save
     # (profiles/r02_decode_modes.txt).  A third variant -- one persistent kernel per layer -- measured 3.2 ms and was
-    # removed in round 2.  The fused projections stay as parity-tested C-ABI operators.
+    # removed.  The fused projections stay as parity-tested C-ABI operators.
     force_unfused = os.environ.get("VB_DECODE_MODE", "unfused") == "unfused"
 
     def _layers_fused(self, position_ids: torch.Tensor, R: int, plan: ops.RowPlan) -> None:

@@ -1,5 +1,5 @@
 """Prefill-KV hand-off between replicas: a request that was prefilled (or partly decoded) on one GPU continues on
-another (north_star: "NCCL over NVLink only for the optional STS prefill-KV broadcast"; SURVEY.md §8e: point-to-point
+another, over NCCL (point-to-point
 send / recv -- or a broadcast when one prompt's KV fans out to several replicas -- of ``[L, n_pages, 2, page, Hkv, D]``
 slices).  The reference has no counterpart: it pins a request to one replica for its lifetime
 (``vox_serve/launch.py:471-474``) and its disaggregation mode moves only token ids between an LM and a detokenizer

@@ -1,7 +1,7 @@
 """The decoder stacks of the reference's other adapters on ``LlamaEngine``: the same packed-weight projections, paged
 attention, fused reduce / norm / RoPE kernels as Orpheus, configured through ``LlamaDims``:
 
-* **CosyVoice2 speech LM** (BASELINE.json configs[0]; ``vox_serve/model/cosyvoice2.py:26-38, 122-315``): Qwen2-0.5B-shaped
+* **CosyVoice2 speech LM** (``vox_serve/model/cosyvoice2.py:26-38, 122-315``): Qwen2-0.5B-shaped
   stack with q / k / v bias, plain rotate-half RoPE at theta 1e6, driven with ``inputs_embeds`` (text-token, task and
   speech-token embeddings), output head ``llm_decoder`` with bias over 6561 + 3 speech ids;
 * **GLM-4-Voice decoder** (configs[4]; ``vox_serve/model/glm_voice.py:22-304``): fused biased ``query_key_value``,

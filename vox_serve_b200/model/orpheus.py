@@ -10,7 +10,7 @@ What differs from the reference adapter is only *where the arithmetic runs*:
 
 Weights: a local HF directory (``config.json`` + ``*.safetensors``), an explicit ``state_dict=``, or
 ``model_name="orpheus-synthetic[:seed]"`` (seeded N(0, 0.02) weights at the true Orpheus shapes -- the image
-has no network, so this is what bench.py and the parity tests use; SURVEY.md §8d).
+has no network, so this is what bench.py and the parity tests use).
 """
 from __future__ import annotations
 
@@ -129,7 +129,7 @@ class OrpheusModel(BaseLM):
         self.stop_token_id = self.STOP_TOKEN_ID if stop_token_id is None else stop_token_id
         self.audio_id_base = self.AUDIO_ID_BASE if audio_id_base is None else audio_id_base
         self._max_tokens = max_tokens
-        # benchmark hook ("fixed 700 decode steps/request (stop id masked out)")
+        # benchmark hook (a fixed number of decode steps per request, the stop id masked out)
         self.mask_stop_token = mask_stop_token
         self.default_sampling_config = SamplingConfig(top_k=None, top_p=0.8, min_p=None, temperature=0.6,
                                                       repetition_penalty=1.3, repetition_window=-1, cfg_scale=None)

@@ -1,4 +1,4 @@
-"""Request-parallel sharding across the GPUs of one box (SURVEY.md §8e): every request is pinned to one replica (one
+"""Request-parallel sharding across the GPUs of one box: every request is pinned to one replica (one
 process + one GPU with its own weights, KV cache and worker) for its lifetime; there is no data-path collective.
 
 * ``ReplicaRouter``: the assignment rule.  ``round_robin`` is the reference's (``vox_serve/launch.py:471-474``:

@@ -2,8 +2,8 @@
 its ZMQ transport replaced by Python queues -- request intake, detokenize / LM selection policies
 (``:234-333``), the fixed call order into the five worker methods, response collection and page release
 (``:335-363``).  It exists so the hot path can be driven, timed (bench.py) and parity-tested end to end without
-the HTTP / ZMQ control plane, which is out of scope (SURVEY.md §2.1 rows 7, 9); the reference's own schedulers
-drive the same worker methods unchanged (INTEGRATION.md).
+the HTTP / ZMQ control plane, which is out of scope; the reference's own schedulers
+drive the same worker methods unchanged.
 """
 from __future__ import annotations
 

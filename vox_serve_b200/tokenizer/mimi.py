@@ -2,7 +2,7 @@
 ``MimiDecoder(...).decode(codes [B, K, T]) -> [B, 1, T * 1920]``, mimi.py:3024-3090 / ``MimiModel.decode`` :2993-3018).
 
 CSM's vocoder (``vox_serve/model/csm.py:771-785``): the reference decodes every 10-frame chunk independently with zero
-left context (``StreamingConv1d.forward`` builds a fresh zero state per call, mimi.py:2116-2148; SURVEY Appendix C), so
+left context (``StreamingConv1d.forward`` builds a fresh zero state per call, mimi.py:2116-2148), so
 the decoder here is stateless as well.  Only the decode side exists (split RVQ codebooks + output projections, the learnt
 x2 upsampling, the decoder transformer, the SEANet decoder); the encoder is prompt-side and not on the serving path.
 

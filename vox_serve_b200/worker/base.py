@@ -3,8 +3,8 @@
 (``prepare_lm_inputs``, ``run_lm_prefill``, ``run_lm_decode``, ``run_detokenize``, ``free_kv_cache``), the same
 properties / attributes, and the same side effects on ``Request`` objects.
 
-What is re-done underneath (SURVEY.md §3.2 "per step the host issues >= 4 device-wide synchronisations, one
-FlashInfer plan, ~6 small H2D copies"):
+What is re-done underneath (per step the reference's host issues four device-wide synchronisations or more, one FlashInfer
+plan and some six small H2D copies):
   * every request owns a *batch slot*; its repetition cache row, last sampled id, token history ring and token
     counter live on the device for the request's lifetime (the reference re-stacks 5 MB of caches and
     concatenates 32 one-element tensors every step, worker/base.py:329-345);
@@ -106,7 +106,7 @@ class ModelWorker:
         if not torch.cuda.is_available():
             raise VoxB200Error("ModelWorker needs a CUDA device: there is no CPU path")
         if detokenizer_device not in (None, "cuda", "cuda:0", f"cuda:{torch.cuda.current_device()}"):
-            raise VoxB200Error("LM/detokenizer disaggregation across GPUs is out of scope (SURVEY.md §8): replicas "
+            raise VoxB200Error("LM/detokenizer disaggregation across GPUs is out of scope: replicas "
                                "are request-parallel, one full pipeline per GPU")
         self.device = f"cuda:{torch.cuda.current_device()}"
         self.detokenizer_device = self.device

@@ -743,7 +743,9 @@ int vb_reduce_residual_rmsnorm(void* d_hidden_out, void* d_normed_out, const flo
   VB_CHECK_ARG(!d_normed_out || d_norm_weight, "vb_reduce_residual_rmsnorm: norm output needs a weight");
   if (T <= 0) return 0;
   auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
-  // (512 rows of 3072: 14.3 us with a CTA per row, 15.1 with a warp; 1024 rows: 23.5 and 16.7)
+  // (512 rows of 3072, operands cold: 14.3 us with a CTA per row, 15.1 with a warp; 1024 rows: 23.5 and 16.7.  Launches back to back,
+  // CTA / warp: 512 rows of 1024 columns 4.9 / 4.1 us, 2048 7.4 / 7.4, 3072 9.9 / 10.2, 4096 11.9 / 13.1; 640 rows 6.5 / 4.5, 10.1 / 7.9,
+  // 13.4 / 10.7, 17.0 / 13.7: the line holds for every width)
   if (T > 512 && N % 8 == 0 && N <= 256 * RW_GROUPS && aligned(d_partials) && aligned(d_hidden_out) && aligned(d_normed_out) &&
       aligned(d_residual) && aligned(d_norm_weight)) {
     VB_LAUNCH_PDL(reduce_residual_rmsnorm_rows_kernel, (T + 3) / 4, 128, 0, stream, static_cast<__nv_bfloat16*>(d_hidden_out),
@@ -753,7 +755,9 @@ int vb_reduce_residual_rmsnorm(void* d_hidden_out, void* d_normed_out, const flo
   }
   // widest cluster (<= 8, the portable limit) that divides the row into float4-aligned parts; few rows -> more parts
   int parts = 1;
-  // (past some 512 CTAs a split row costs more than it gives: 256 rows of 3072, 15.4 us in four parts, 11 whole)
+  // (past some 512 CTAs a split row costs more than it gives: 256 rows of 3072, operands cold, 15.4 us in four parts, 11 whole.  Launches
+  // back to back, where a neighbour covers a row's latency, want whole rows earlier, in 4 / 2 / 1 parts: 128 rows of 1024 columns
+  // 4.6 / 2.5 / 1.8 us, 3072 5.7 / 4.4 / 4.3, 4096 6.1 / 4.8 / 5.8; 192 rows 6.6 / 4.4 / 2.0, 8.8 / 8.2 / 5.3, 9.2 / 8.5 / 6.4)
   const int want = T <= 64 ? 8 : (T <= 128 ? 4 : (T <= 192 ? 2 : 1));
   for (int c = want; c >= 1; c >>= 1)
     if (N % (4 * c) == 0) { parts = c; break; }
@@ -779,7 +783,9 @@ int vb_qkv_rope_append(void* d_q_out, void* d_layer_kv, const float* d_partials,
   if (T <= 0) return 0;
   const int n_heads = n_q + 2 * n_kv;
   auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
-  // (257 rows of 40 heads of 128: 11.3 us by the kernel below, 9.2 here; it spreads a row's heads over CTAs up to 256 rows)
+  // (257 rows of 40 heads of 128, operands cold: 11.3 us by the kernel below, 9.2 here; it spreads a row's heads over CTAs up to 256 rows.
+  // Launches back to back, below / here: 257 rows of 24 + 8 + 8 heads of 128 7.5 / 4.9 us, 32 + 8 + 8 of 64 5.3 / 3.3, 14 + 2 + 2 of 64
+  // 3.2 / 2.3, 16 + 8 + 8 of 128 6.6 / 3.7; down to some 100 rows this kernel is ahead there too, 4.0 / 3.6, 3.1 / 2.2, 2.5 / 2.1, 3.1 / 2.5)
   if (T > 256 && !interleave && rotary_dim == head_dim && head_dim % 16 == 0 && head_dim <= 256 && !d_q_norm && aligned(d_q_out) &&
       aligned(d_layer_kv) && aligned(d_partials)) {
     VB_LAUNCH_PDL(qkv_rope_rows_kernel, T, 256, 2 * head_dim * sizeof(float), stream, static_cast<__nv_bfloat16*>(d_q_out),

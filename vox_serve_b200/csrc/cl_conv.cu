@@ -21,7 +21,7 @@
 // has 5 x 4 tiles of 128.
 // What bounds it: wide layers of few positions are one chain of 32-deep k-blocks (0.41 us each, the split into halves), narrow
 // layers of many positions the epilogue (1x1 with residual, 614400 positions of 64 channels: 393 MB in 126 us).
-// Measured (one pass): SNAC 32 windows 1454 us channel-first, 623 here; 1 window 711 and 262; Mimi 32 chunks 6721 and 1881.
+// Measured (one pass): SNAC 32 windows 1454 us channel-first, 651 here; 1 window 711 and 262; Mimi 32 chunks 6721 and 1930.
 // Of that, the residual's rows asked for before the accumulator is waited for: Mimi 2499 -> 2407; 16 columns at a time on twelve warps
 // without a spilled register, where 32 on eight spilled 53: Mimi 2403 -> 1933, SNAC 746 -> 647 and 313 -> 266.
 #include "../../include/vb_api.h"

@@ -21,8 +21,9 @@
 // 98 KB of shared memory and 256 TMEM columns per CTA: two CTAs share an SM and fill each other's waits.
 // The form before this one had one warp group for everything -- loads, an element-wise transpose of every V tile, softmax, both
 // waits on the tensor cores -- one after the other (2.5 us per 64-token tile), and the kernel for smaller prompts ran on
-// mma.sync.  Measured per launch (mma.sync / this kernel, us): one 133-row prompt 12.0 / 9.2, eight of them 29 / 13, four portions
-// of 997 rows on up to 1063 cached tokens 92 / 35, three prompts of 1024 rows 46 / 19, four of 600 rows with 64-wide heads 75 / 33.
+// mma.sync.  Measured per launch (mma.sync / this kernel, us, back to back): one 133-row prompt 11.6 / 10.1, eight of them 29 / 14,
+// four portions of 997 rows on up to 1063 cached tokens 112 / 40, three prompts of 1024 rows each 187 / 61, four of 600 with 64-wide heads
+// 74 / 32.
 // What bounds it: the serial chain of a tile (scores -> maximum -> exponentials -> P V, about 1.3 us), and where few tiles see
 // a long context the longest of them.
 // Every wait is bounded (BoundedWait): a block whose wait runs out sets its flag, stops issuing and leaves.

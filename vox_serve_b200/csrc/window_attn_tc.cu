@@ -6,8 +6,8 @@
 // head each.  A row tile of 64 is dealt to ceil(64 / TQ) CTAs.  Keys are walked in tiles of 64 positions: first those with kept
 // tokens, then from the tile of the first key that the CTA's first row sees; within a tile the mask is per key.  What lies between the two is
 // nobody's to read (a page table may name other requests' pages there, or unwritten ones): its boxes are skipped, its V rows cleared.
-// Measured (16 query heads on 4 key heads of 128, two prompts of 1001 rows in all): 102 us per launch with mma.sync, about 20 here; the
-// three-layer prompt step around it 1058 -> 884 us.
+// Measured (16 query heads on 4 key heads of 128, two prompts of 1001 rows in all): the three-layer prompt step around it 1058 us with
+// mma.sync, 884 here.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 1
 #include "attn_tc.cuh"

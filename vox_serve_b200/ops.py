@@ -305,9 +305,9 @@ _PREFILL_TC = os.environ.get("VB_PREFILL_TC", "auto")
 
 
 def _prefill_entry() -> str:
-    """The kernel of a prefill-shaped plan.  Measured per launch, mma.sync / tcgen05 (us): 4 x 600 rows 75 / 33, 8 x 133 rows 29 / 13,
-    one 133-row prompt 12.0 / 9.2, 31 decode rows beside a 133-row prompt 53 / 22, one of 435 rows 28 / 14, 16 x 50 rows 10.1 / 10.0,
-    16 x 24 rows 8.8 / 9.1 (the one where most of a 128-row tile is padding)."""
+    """The kernel of a prefill-shaped plan.  Measured per launch, mma.sync / tcgen05 (us): 4 x 600 rows 74 / 32, 8 x 133 rows 29 / 14,
+    one 133-row prompt 11.6 / 10.1, 31 decode rows beside a 133-row prompt 54 / 26, one of 435 rows 28 / 15, 16 x 50 rows 16.9 / 12.6,
+    16 x 24 rows 8.8 / 9.6 (the one where most of a 128-row tile is padding)."""
     return "vb_paged_prefill_attn" if _PREFILL_TC == "0" else "vb_paged_prefill_attn_tc"
 
 

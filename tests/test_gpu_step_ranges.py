@@ -113,6 +113,27 @@ def test_wide_gate_quotients(ops, kind, scale, slope):
     assert torch.equal(got, want), (got != want).sum().item()
 
 
+@pytest.mark.parametrize("T", [64, 128])
+def test_projections_refuse_alike(ops, T):
+    """What the one-SM entries refuse is refused for steps of many rows too: a clamp that is not positive, an activation on a grouped
+    gated product."""
+    from vox_serve_b200._lib import VoxB200Error
+
+    x = torch.randn(T, 64, device="cuda").bfloat16()
+    pw = ops.pack_weight(torch.randn(256, 64, device="cuda").bfloat16(), 64)
+    out, grp = torch.empty(T, 128, device="cuda").bfloat16(), _i32([0] * (T // 64))
+    for limit in (0.0, -1.0, float("nan")):
+        with pytest.raises(VoxB200Error):
+            ops.gemm_glu(x, pw, out, limit, 1.0)
+        with pytest.raises(VoxB200Error):
+            ops.gemm_grouped_glu(x, pw, out, 256, 64, 64, grp, 0, limit, 1.0)
+    for tiles in (grp, None):
+        with pytest.raises(VoxB200Error):
+            ops.gemm_grouped(x, pw, out, 2, 256, 64, 64, tiles, act="gelu")
+    ops.gemm_glu(x, pw, out, 7.0, 1.0)
+    ops.gemm_grouped(x, pw, out, 2, 256, 64, 64, grp)
+
+
 @pytest.mark.parametrize("groups,tt,N,K", [(1, 128, 256, 128), (3, 128, 320, 456), (5, 64, 128, 192)])
 def test_wide_grouped_projection(ops, groups, tt, N, K):
     g = torch.Generator(device="cuda").manual_seed(groups)

@@ -511,6 +511,7 @@ int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_ma
   VB_CHECK_ARG(n_tok >= 16 && n_tok <= 256 && n_tok % 16 == 0, "vb_gemm_bf16_wide: n_tok %d outside [16, 256] or not a multiple of 16", n_tok);
   VB_CHECK_ARG(group_bytes >= 0 && w_kb_stride >= 0 && group_kb >= 0 && kb_base >= 0, "vb_gemm_bf16_wide: offsets");
   VB_CHECK_ARG(!d_tile_group || x_map, "vb_gemm_bf16_wide: groups need row-major activations");
+  VB_CHECK_ARG(glu_limit >= 0.f && (glu_limit == 0.f || (mode == 2 && act == 0)), "vb_gemm_bf16_wide: a positive limit belongs to mode 2 without an activation");
   static const CUtensorMap dummy_map = {};
   GemmWideParams p = {};
   VB_CHECK_ARG(p.wait_flag = wait_flag(WK_GEMM_WIDE), "vb_gemm_bf16_wide: no mapped host memory");

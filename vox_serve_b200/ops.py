@@ -412,6 +412,12 @@ def _use_wide(T: int, tile_rows: int) -> bool:
     return T >= WIDE_MIN_ROWS and tile_rows in WIDE_TILE_ROWS
 
 
+def _positive_limit(limit: float) -> None:
+    """(vb_gemm_bf16_wide_grouped takes a limit of 0 for the plain gate; the one-SM entries refuse it themselves)"""
+    if not limit > 0.0:
+        raise VoxB200Error(f"the clamped gate needs a positive limit, not {limit}")
+
+
 @lru_cache(maxsize=8192)
 def _wide_tokens(T: int, N: int, K: int, tile_rows: int, split: int) -> int:
     """token rows per tile for a given split: the choice for ``split`` times as many weight tiles on a k range as long"""
@@ -553,6 +559,7 @@ def gemm_glu(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, limit: float
     assert x.dtype == BF16 and x.dim() == 2 and x.shape[1] == w.K and out.dtype == BF16 and out.is_contiguous()
     T = x.shape[0]
     if _use_wide(T, w.tile_rows):
+        _positive_limit(limit)
         n_tok = _wide_tokens(T, w.N, w.K, w.tile_rows, 1)
         call("vb_gemm_bf16_wide_grouped", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, n_tok // 2).ptr, None, T, w.N, w.K, out.shape[1], 2, 1,
              w.tile_rows, out.shape[1], 0, None, 0, n_tok, None, 0, 0, 0, 0, float(limit), float(slope), _stream())
@@ -1547,6 +1554,8 @@ def gemm_grouped(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, mode: in
     assert tile_group is None or x.shape[0] % t_tile == 0
     n_out = (N // 2 if mode == 2 else N) if n_out is None else n_out
     if _use_wide(x.shape[0], w.tile_rows):       # (row tiles of groups keep their size: a tile belongs to one group)
+        if act is not None and mode != 0:
+            raise VoxB200Error(f"gemm_grouped: activation {act!r} is a mode 0 option")
         n_tok = t_tile if tile_group is not None else _wide_tokens(x.shape[0], N, K, w.tile_rows, 1)
         call("vb_gemm_bf16_wide_grouped", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, n_tok // 2).ptr, None, x.shape[0], N, K, n_out, mode, 1,
              w.tile_rows, n_out, 0, None, GEMM_ACTS[act], n_tok, _p(tile_group), int(group_bytes), int(w_kb_stride), int(group_kb),
@@ -1805,6 +1814,7 @@ def gemm_grouped_glu(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, N: i
     _need_cuda(x, out)
     assert x.dtype == BF16 and x.dim() == 2 and x.shape[1] == K and out.is_contiguous() and x.shape[0] % t_tile == 0
     if _use_wide(x.shape[0], w.tile_rows):
+        _positive_limit(limit)
         call("vb_gemm_bf16_wide_grouped", out.data_ptr(), w.data.data_ptr(), tensor_map_2d(x, t_tile // 2).ptr, None, x.shape[0], N, K, N // 2, 2, 1,
              w.tile_rows, N // 2, 0, None, 0, t_tile, _p(tile_group), int(group_bytes), 0, 0, 0, float(limit), float(slope), _stream())
         return out

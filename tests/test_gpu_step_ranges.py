@@ -471,6 +471,21 @@ def test_paged_prompt_attention_pages(ops, page, D, H, G, kv, new):
     assert _lib.load().vb_prefill_attn_tc_timeouts() == 0
 
 
+@pytest.mark.parametrize("H", [128, 129, 200])
+def test_paged_prompt_attention_many_heads_per_key_head(ops, H):
+    """More query heads on one key head than a tcgen05 row tile has rows: an automatic plan runs all the same."""
+    D, page, L = 64, 16, 40
+    g = torch.Generator(device="cuda").manual_seed(H)
+    q, cache = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((L, H, D), (3, 2, page, 1, D)))
+    plan = ops.RowPlan(L, "cuda")
+    ops.plan_rows(plan, _i32([0, L]), _i32([0, 3]), _i32([0, 1, 2]), _i32([8]), 1, L, page, page)
+    out = ops.paged_attn(q, cache, 0, plan, L, 1, page, page, None)
+    k, v = (cache[:, i, :, 0].reshape(-1, D)[:L].double() for i in (0, 1))
+    s = torch.einsum("qhd,kd->hqk", q.double(), k) * D ** -0.5
+    s = s.masked_fill(torch.ones(L, L, device="cuda").triu(1).bool(), -float("inf"))
+    _close(out, torch.einsum("hqk,kd->qhd", torch.softmax(s, -1), v), 2 ** -8)
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("width", [1.0, 3.0])
 def test_prompt_attention_probabilities(ops, D, width):

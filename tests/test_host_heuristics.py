@@ -111,7 +111,8 @@ def test_prefill_kernel_selection_rules(monkeypatch):
     assert not ops.use_prefill_tiles(plan(1), 133, 96, 128)                       # head_dim the tiled kernels do not take
     for env, entry in (("auto", "vb_paged_prefill_attn_tc"), ("1", "vb_paged_prefill_attn_tc"), ("0", "vb_paged_prefill_attn")):
         monkeypatch.setattr(ops, "_PREFILL_TC", env)
-        assert ops._prefill_entry() == entry
+        assert [ops._prefill_entry(g) for g in (1, 3, 128)] == [entry] * 3
+        assert ops._prefill_entry(129) == "vb_paged_prefill_attn"          # more heads than a tcgen05 row tile has rows
 
 
 def test_speech_tokenizer_config_and_mask_bounds():

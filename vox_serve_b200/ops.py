@@ -304,11 +304,12 @@ _PREFILL_TILES = os.environ.get("VB_PREFILL_TILES", "auto")      # "0": never, "
 _PREFILL_TC = os.environ.get("VB_PREFILL_TC", "auto")
 
 
-def _prefill_entry() -> str:
-    """The kernel of a prefill-shaped plan.  Measured per launch, mma.sync / tcgen05 (us): 4 x 600 rows 74 / 32, 8 x 133 rows 29 / 14,
+def _prefill_entry(group: int) -> str:
+    """The kernel of a prefill-shaped plan with ``group`` query heads per key head (more than a row tile of the tcgen05 kernel holds run on
+    mma.sync).  Measured per launch, mma.sync / tcgen05 (us): 4 x 600 rows 74 / 32, 8 x 133 rows 29 / 14,
     one 133-row prompt 11.6 / 10.1, 31 decode rows beside a 133-row prompt 54 / 26, one of 435 rows 28 / 15, 16 x 50 rows 16.9 / 12.6,
     16 x 24 rows 8.8 / 9.6 (the one where most of a 128-row tile is padding)."""
-    return "vb_paged_prefill_attn" if _PREFILL_TC == "0" else "vb_paged_prefill_attn_tc"
+    return "vb_paged_prefill_attn" if _PREFILL_TC == "0" or group > 128 else "vb_paged_prefill_attn_tc"
 
 
 def use_prefill_tiles(plan: RowPlan, n_rows: int, head_dim: int, page_size: int) -> bool:
@@ -350,7 +351,7 @@ def paged_attn(q: torch.Tensor, kv_cache, slab_base: int, plan: RowPlan, n_rows:
     if tiles:
         assert plan.qo_indptr is not None, "the tiled prefill kernel needs a prefill plan (qo_indptr)"
         fn = "vb_paged_prefill_attn_tc" if prefill_tiles == "tc" else (
-            _prefill_entry() if prefill_tiles is None else "vb_paged_prefill_attn")
+            _prefill_entry(n_q // n_kv) if prefill_tiles is None else "vb_paged_prefill_attn")
         call(fn, out_ptr, q.data_ptr(), kv_cache.data_ptr(), int(slab_base),
              plan.qo_indptr.data_ptr(), plan.kv_indptr.data_ptr(), plan.kv_indices.data_ptr(),
              plan.row_kvlen.data_ptr(), plan.n_req, n_rows, n_q, n_kv, d, page_size, sc, xt, _stream())

@@ -166,7 +166,7 @@ def _nccl_rank_body(rank, port, out):
 
 def test_request_migrates_between_gpus_nccl():
     if torch.cuda.device_count() < 2:
-        pytest.skip("needs two GPUs (gpurun --gpus 2)")
+        pytest.skip("needs two GPUs")
     import queue as pyqueue
     import time
 

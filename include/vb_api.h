@@ -521,8 +521,24 @@ int vb_wait_check(int limit_us, int pause_us, int complete, void* stream);
  * vb_cl_dwconv7 / vb_cl_last_conv: depthwise 7 taps (w [7][C], "same") with Snake on both sides; one output channel, `left` positions of
  *   context, optional tanh -> y [B][t1 - t0].
  * vb_cl_from_codes, vb_cl_codes_sum, vb_cl_upsample (w [C][2 s]), vb_cl_layernorm, vb_cl_chunk_attention (qkv [B][T][3 C], T <= 64).
+ * Parts: an activation whose only readers are these convolutions can be kept as what they multiply -- in the place of 32 fp32 channels
+ *   [32 high | 32 low] fp16, v = (high + low / 2048) / 16, with one code byte per 32 channels (1 ordinary, 2 all below 2^-16, 0 all zero, 4 the
+ *   32 fp32 values themselves, one of them being out of range or not a number).  The codes of element e lie at e / 32.  vb_cl_conv_parts takes x as
+ *   parts (d_x_code) or as fp32 (NULL), and gives the activated values as parts in d_yp / d_yp_code (d_y: the plain ones, or NULL; not with
+ *   d_y2); entries of parts lie multiples of 32 floats apart.  vb_cl_{dwconv7, codes_sum, layernorm, chunk_attention}_parts: the result as
+ *   parts where the codes are not NULL (D, C and the head size then multiples of 32).
  * vb_cl_timeouts: as vb_gemm_wide_timeouts. */
 int vb_cl_timeouts(void);
+int vb_cl_conv_parts(float* d_y, float* d_y2, void* d_yp, void* d_yp_code, const void* d_x, const void* d_x_code, long long x_bstride, int Tx,
+                     const void* d_w, const float* d_bias, const float* d_resid, long long r_bstride, const float* d_scale, const float* d_noise,
+                     int noise_ld, const float* d_alpha, int epilogue, int act, int B, int Cin, int N, int cmod, int ksize, int dil, int n_lo,
+                     int n_hi, long long y_bstride, void* stream);
+int vb_cl_dwconv7_parts(float* d_y, void* d_code, const float* d_x, long long x_bstride, const float* d_w, const float* d_bias,
+                        const float* d_alpha_in, const float* d_alpha_out, int B, int C, int T, int dilation, int t_lo, int t_hi, void* stream);
+int vb_cl_codes_sum_parts(float* d_z0, float* d_z1, void* d_code0, void* d_code1, const int64_t* d_codes, const float* d_emb, int B, int K, int bins,
+                          int D, int T, void* stream);
+int vb_cl_layernorm_parts(float* d_y, void* d_code, const float* d_x, const float* d_w, const float* d_b, int rows, int C, float eps, void* stream);
+int vb_cl_chunk_attention_parts(float* d_out, void* d_code, const float* d_qkv, int B, int C, int H, int T, float max_period, void* stream);
 long long vb_cl_pack_bytes(int N, int K);
 int vb_cl_pack(void* d_dst, const float* d_w, int N, int K, void* stream);
 int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, int Tx, const void* d_w, const float* d_bias,

@@ -192,6 +192,67 @@ def test_channels_last_conv_reuses_stages(B, T, C, N, ksize):
         assert torch.equal(_cl.conv(xa, wp, N, ksize=ksize).tensor(), y)
 
 
+# activations kept as parts: several entries and their halos in a tile, runs with a remainder, taps further apart than a tile's halo holds, K
+# divided over a cluster, boxes of results and none, two results; values of ordinary size, larger than fp16 and all below its normal range
+@pytest.mark.parametrize("B,T,C,N,ksize,dil,lo,hi,epi,act,both,size", [
+    (1, 1, 32, 32, 1, 1, 0, 1, "plain", None, False, 1.0), (7, 16, 64, 96, 3, 1, 0, 16, "resid", "snake", False, 1.0), (2, 128, 32, 128, 3, 1, 0, 128, "plain", "elu", True, 1.0),
+    (3, 129, 96, 160, 2, 1, 5, 129, "noise", None, False, 1.0), (1, 300, 64, 64, 7, 9, 130, 299, "scale_resid", "gelu", False, 1.0),
+    (40, 3, 128, 512, 2, 1, 0, 3, "resid", None, True, 1.0), (1, 40, 64, 32, 5, 30, 0, 40, "plain", None, False, 1.0), (1, 17, 1024, 256, 2, 1, 0, 17, "plain", "elu", True, 1.0),
+    (3, 700, 64, 128, 1, 1, 0, 700, "resid", "elu", False, 1.0), (2, 900, 128, 256, 2, 1, 3, 899, "plain", "elu", True, 1.0), (2, 50, 64, 64, 3, 1, 0, 50, "resid", "elu", True, 3e5),
+    (2, 50, 64, 64, 3, 1, 0, 50, "plain", None, False, 1e-6)])
+def test_channels_last_parts(B, T, C, N, ksize, dil, lo, hi, epi, act, both, size):
+    from vox_serve_b200 import _lib
+    from vox_serve_b200.tokenizer import _cl
+
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")                 # noqa: E731
+    x, w, b, r = rnd(B, T, C) * size, rnd(N, C, ksize) * (C * ksize) ** -0.5, rnd(N) * size, rnd(B, T, N) * size
+    sc, nz, al = rnd(N), rnd(B, T), torch.rand(N, generator=g, device="cuda") + 0.5
+    wrap = lambda t: _cl.Act(t.reshape(-1).clone(), B, T, t.shape[-1])           # noqa: E731
+    eye = _cl.pack(torch.eye(C, device="cuda"))
+    xp = _cl.conv(wrap(x), eye, C, out="parts")                                  # the values, to the 2^-22 that parts hold
+    kw = dict(ksize=ksize, dil=dil, epi=epi, resid=None if epi == "plain" else wrap(r), scale=sc, noise=nz, act=act,
+              alpha=torch.cat((al, 1 / (al + 1e-9))), lo=lo, hi=hi)
+    v = torch.nn.functional.conv1d(torch.nn.functional.pad(x.double().transpose(1, 2), ((ksize - 1) * dil, 0)), w.double(), b.double(),
+                                   dilation=dil).transpose(1, 2)
+    v = {"plain": v, "resid": r + v, "scale_resid": r + sc * v, "noise": r + nz[..., None] * v}[epi].double()
+    z = {None: v, "snake": v + torch.sin(al * v) ** 2 / (al.double() + 1e-9), "elu": torch.nn.functional.elu(v),
+         "gelu": torch.nn.functional.gelu(v)}[act]
+    wp = _cl.pack_conv(w.reshape(N, -1), C, ksize)
+    _close(_cl.conv(xp, wp, N, b, **kw).tensor()[:, lo:hi], z[:, lo:hi], 5e-6)
+    out = _cl.conv(xp, wp, N, b, both=both, out="parts", **kw)                   # what the next convolution reads, through an identity
+    plain, out = out if both else (None, out)
+    if both:
+        _close(plain.tensor()[:, lo:hi], v[:, lo:hi], 5e-6)
+    back = _cl.conv(out, _cl.pack(torch.eye(N, device="cuda")), N, lo=lo, hi=hi)
+    _close(back.tensor()[:, lo:hi], z[:, lo:hi], 5e-6)
+    assert _lib.load().vb_cl_timeouts() == 0
+
+
+@pytest.mark.parametrize("code", [0x7fffffff, 0x7f800000, 0x7f7fffff])
+@pytest.mark.parametrize("C,ksize", [(64, 3), (64, 1)])
+def test_channels_last_parts_special_values(code, C, ksize):
+    """What parts cannot hold is kept as it is, and reaches the positions and channels that it reaches in fp32, no others."""
+    from vox_serve_b200.tokenizer import _cl
+
+    B, T, N = 2, 300, 96
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x, w = torch.randn(B, T, C, generator=g, device="cuda"), torch.randn(N, C, ksize, generator=g, device="cuda") * 2.0 ** -10
+    zero = _cl.Act(torch.zeros(B * T * C, device="cuda"), B, T, C)
+    x[1, 133, 37] = _bits(code)
+    xp = _cl.conv(zero, _cl.pack(torch.eye(C, device="cuda")), C, epi="resid", resid=_cl.Act(x.reshape(-1).clone(), B, T, C), out="parts")
+    y = _cl.conv(xp, _cl.pack_conv(w.reshape(N, -1), C, ksize), N, ksize=ksize).tensor()
+    bad = torch.zeros(B, T, N, dtype=torch.bool, device="cuda")
+    bad[1, 133:133 + ksize] = True
+    if code == 0x7f7fffff:
+        ref = torch.nn.functional.conv1d(torch.nn.functional.pad(x.double().transpose(1, 2), (ksize - 1, 0)), w.double()).transpose(1, 2)
+        assert torch.isfinite(y).all()
+        _close(y[bad], ref[bad], 5e-6)
+        _close(y[~bad], ref[~bad], 5e-6)
+    else:
+        assert torch.equal(~torch.isfinite(y), bad)
+
+
 def _activated(values, act, alpha=None):
     """The epilogue's activation of given fp32 values: a convolution of zeros with the values as its residual"""
     from vox_serve_b200.tokenizer import _cl

@@ -66,6 +66,12 @@ SIGNATURES = {
     "vb_cl_pack": (c_int, [P, P, c_int, c_int, P]),
     "vb_cl_conv": (c_int, [P, P, P, C.c_longlong, c_int, P, P, P, C.c_longlong, P, P, c_int, P, c_int, c_int, c_int, c_int, c_int, c_int,
                            c_int, c_int, c_int, c_int, C.c_longlong, P]),
+    "vb_cl_conv_parts": (c_int, [P, P, P, P, P, P, C.c_longlong, c_int, P, P, P, C.c_longlong, P, P, c_int, P, c_int, c_int, c_int, c_int, c_int,
+                                 c_int, c_int, c_int, c_int, c_int, C.c_longlong, P]),
+    "vb_cl_dwconv7_parts": (c_int, [P, P, P, C.c_longlong, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P]),
+    "vb_cl_codes_sum_parts": (c_int, [P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P]),
+    "vb_cl_layernorm_parts": (c_int, [P, P, P, P, P, c_int, c_int, c_float, P]),
+    "vb_cl_chunk_attention_parts": (c_int, [P, P, P, c_int, c_int, c_int, c_int, c_float, P]),
     "vb_cl_dwconv7": (c_int, [P, P, C.c_longlong, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P]),
     "vb_cl_last_conv": (c_int, [P, P, C.c_longlong, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P]),
     "vb_cl_from_codes": (c_int, [P, P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P]),

@@ -1,70 +1,87 @@
 // Vocoder convolutions over channels-last activations [B][T][C] (fp32), on tcgen05 with fp32-grade products.
 //
-// The channel-first kernel (snac_mma.cu) gathers its activation operand with one strided load per element, splits it in
-// registers and stores both halves to shared memory: 1.5 - 2 us per 32-deep k-block however small the problem, no overlap of
-// the epilogue, a 128-row weight tile even for layers of 32 channels, and layers narrower than 128 channels left to CUDA
-// cores.  With the channels innermost the convolution is a plain matrix product per tap:
-//   D[position][n] += sum_c X[position - shift(tap)][c] * W[tap][n][c]
-// whose activation tile (128 positions x 32 channels) is one box of a tensor map -- positions before the start and past the
-// end are the map's zero fill, short sequences put several batch entries into one box -- and whose output rows are contiguous.
-// A transposed convolution of stride s is the same product with two taps and n = (phase, channel): row n of the result holds
-// the s output positions of input position n.
+// With the channels innermost a convolution is a plain matrix product per tap:
+//   D[n][position] += sum_c W[tap][n][c] * X[position - shift(tap)][c]
+// The weights are the MMA's first operand (128 output channels = the lanes of the accumulator), the positions its columns: a lane
+// of the epilogue owns one channel -- bias, scale and alpha are scalars of the thread -- and 32 lanes store 32 neighbouring channels,
+// so rows leave and residuals come without a transpose.  A transposed convolution of stride s is the same product with two taps and
+// n = (phase, channel): row n of the result holds the s output positions of input position n.
 //
-// Products: x = hi + lo and w = hi + lo, both halves rounded to tf32 (to nearest), lo_w hi_x + hi_w lo_x + hi_w hi_x with
-// fp32 accumulation; what is dropped is below 2^-22 of a product (the channel-first kernel truncates: 2^-20).
+// Products: both operands as two fp16 parts, v = hi + lo / 2048 (the low part scaled into the normal range: 22 bits and a sign), hi_w hi_x in
+// one accumulator, hi_w lo_x + lo_w hi_x in a second one; what is dropped is below 2^-22 of a product.  Half the MMA time and half the
+// weight bytes of the two tf32 parts that stood here, at the same width; error against 64 bits of a decode 4.7e-6 (Mimi, was 2.8e-5).  Weights are
+// scaled per output channel by a power of two when they are packed.  Activations by 16: their parts hold 22 bits where a tile's largest
+// value lies in [2^-16, 4092) (smaller values in such a tile to 2^-40 absolute).  A tile that is outside -- NaN, infinity, huge values, or a
+// whole tile of nothing but tiny ones -- is multiplied again in fp32 on CUDA cores (cl_exact_chunk), eight positions at a time.
+// What only these convolutions read is written as parts by the kernel that produces it, in the bytes its fp32 values would have taken, and
+// fetched by TMA: nothing is converted here, and a tap is the same tile in shared memory read from a later row on.  Activations that come
+// as fp32 are split on the way by eight warps, once per tile and 64 channels for all taps.
 //
-// Roles of a CTA's eighteen warps: 0 copies (activation box and two weight tiles per stage), 1 issues the MMAs, 2..5 split a
-// stage's raw activations into the two halves and put them into TMEM as the MMA's A operand (128 x 32 columns each; through
-// shared memory the operand would cost 12 KB of its bandwidth per 8-deep product, and the two tiles another 32 KB of stores),
-// 6..17 are the epilogue.  Persistent CTAs, two accumulators, 4 stages (6 where column tiles are 32 wide): TMEM bounds them.
-// The width of a column tile (32, 64 or 128) is chosen per launch from the number of tiles: a transformer layer of 640 rows
-// has 5 x 4 tiles of 128.
-// What bounds it: wide layers of few positions are one chain of 32-deep k-blocks (0.41 us each, the split into halves), narrow
-// layers of many positions the epilogue (1x1 with residual, 614400 positions of 64 channels: 393 MB in 126 us).
-// Measured (one pass): SNAC 32 windows 1454 us channel-first, 651 here; 1 window 711 and 262; Mimi 32 chunks 6721 and 1930.
-// Of that, the residual's rows asked for before the accumulator is waited for: Mimi 2499 -> 2407; 16 columns at a time on twelve warps
-// without a spilled register, where 32 on eight spilled 53: Mimi 2403 -> 1933, SNAC 746 -> 647 and 313 -> 266.
+// Warps: 0 copies weights (one bulk copy a stage), 1 issues the MMAs, 2 copies activations, 3 looks at the codes of a tile's rows (with fp32
+// activations 2..9 split), the rest is the epilogue.  Persistent CTAs, two accumulator pairs where they fit, weights that stay in shared
+// memory where a CTA's units share them.  Long sums of narrow layers are divided over a cluster (cl_splits) and added through
+// distributed shared memory in rank order, by the layer alone: an entry's values do not depend on its batch.
+// What bounds it (640 rows of 512 x 2048, split in four: 12.8 us, was 28.4; 5120 x 1536 x 1024: 60 us, was 161): the wide layers the bytes
+// through L2 and shared memory, 0.6 us for 64 channels and one tap of 128 x 128; the layers of many positions the epilogue's instructions,
+// some 30 per value (153600 x 128 with residual 61 us, was 71, 30 of DRAM time).
+// Measured (one pass): SNAC 32 windows 652 -> 543 us, 1 window 262 -> 246, Mimi 32 chunks 1926 -> 1333.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 32
 #include "common.cuh"
+#include <cuda_fp16.h>
 #include <cudaTypedefs.h>
 
 namespace vb {
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn();      // api.cu
 
-constexpr int CL_THREADS = 576;
-constexpr int CL_A_BYTES = 128 * 128;       // 128 positions x 32 channels
-constexpr int CL_MAX_STAGES = 6;            // 512 TMEM columns less two accumulators, 64 a stage
-constexpr int CL_EPI_WARPS = 12;
-constexpr int CL_EPI_BYTES = CL_EPI_WARPS * 2048;      // a transpose of 32 rows x 16 columns per epilogue warp
+constexpr int CL_SPLIT_WARPS = 8;
+constexpr int CL_X_STAGES = 4, CL_W_STAGES = 8, CL_TOPS = 8;
+constexpr int CL_ROWS = 256;                // rows of a stage of activations: columns of the tile and the halo
+constexpr int CL_W_BLOCK = 128 * 128;       // 128 output channels x 32 input channels, high and low parts
+constexpr int CL_TAIL = 8192;               // barriers, tables, alignment
+constexpr float CL_X_SCALE = 16.f, CL_LO_SCALE = 2048.f;      // of activations; of low parts against high ones
+// what the two parts of an activation hold to 2^-22: a tile whose largest value is not between these (or zero) is multiplied on CUDA cores
+constexpr float CL_X_TOP = 65472.f / CL_X_SCALE, CL_X_LOW = 0x1p-12f / CL_X_SCALE;
+enum ClCode { CB_NORMAL = 1, CB_QUIET = 2, CB_RAW = 4 };      // of a block of 32 activations kept as parts (all zero: 0)
 
 struct ClConvParams {
-  const uint8_t* w;          // [tap * kb][hi | lo][n_pad][32], rows swizzled
-  float* y;                  // [b * y_bstride + t * ldy + n]
-  float* y2;                 // optional: the activated values; y then holds the plain ones
+  const uint8_t* w;          // [128 channels][32 of K][128][32 hi | 32 lo], rows of 128 bytes swizzled
+  const float* w_inv;        // [n_pad] 1 / (scale of the channel's weights * CL_X_SCALE)
+  const float* x;            // fp32, or parts
+  const uint8_t* x_code;     // of the parts
+  float* y;                  // [b * y_bstride + t * N + n]; the plain values where another output is given
+  float* y2;                 // optional: the activated values
+  uint32_t* yp;              // optional: the activated values as parts
+  uint8_t* yp_code;
   const float* bias;         // [cmod], column n takes entry n % cmod
   const float* resid;
   const float* scale;        // [N]
   const float* noise;        // [b * noise_ld + t]
   const float* alpha;        // [cmod] alpha, then [cmod] 1 / (alpha + 1e-9)
-  long long y_bstride, r_bstride;
-  int ldy, ldr, noise_ld, cmod, epi, act;
-  int B, n_lo, n_hi, ksize, dil, N, n_pad, kb_per_tap, ksteps;
-  int nt, n_tiles, nr, nb, t_tiles, units, stages, tmem_cols;
+  long long x_bstride, y_bstride, r_bstride;
+  int noise_ld, cmod, epi, act;
+  int B, Tx, Cin, N, n_lo, n_hi, ksize, dil;
+  int group;                 // 32-channel blocks a stage
+  int kb;                    // stages of channels
+  int taps;                  // taps that one stage of activations serves: all of them, or one
+  int halo;                  // rows of an entry in front of its first position (taps == ksize), else 0
+  int nr, nb, pitch, cols, rows_pad;      // a tile: nb entries of nr positions, `pitch` rows apart; columns in all
+  int m_tiles, t_tiles, units, grid;
+  int splits;                // parts of K, each on a CTA of a cluster
+  uint32_t m_tiles_inv, t_tiles_inv;      // for cl_div
+  int x_stages, w_stages, acc_cols, acc_bufs;
+  int resident;              // the weights of a CTA's units are the same and stay in shared memory
+  int staged;                // results and residuals pass through boxes of 8 positions x 32 channels in shared memory, four per warp
+  int passes;                // rows of a stage that a thread of the split takes: 1, 2, 4, 8 or 16
   unsigned char* wait_flag;
-  int acc_cols;              // TMEM columns of an accumulator: nt, or 2 nt where the two halves of the weights have their own
 };
 enum ClEpi { CE_PLAIN = 0, CE_RESID = 1, CE_SCALE_RESID = 2, CE_NOISE = 3 };
 enum ClAct { CA_NONE = 0, CA_SNAKE = 1, CA_ELU = 2, CA_GELU = 3 };
 
-// round to the 10 mantissa bits of tf32, halves away from zero (integer arithmetic: the conversion instruction runs at a
-// quarter of the rate and made the split the longest step of a stage).  Only below CL_ROUND_MAX: from there on up the sum would leave
-// the exponent -- the largest finite values would become infinite, and NaN as arithmetic writes it, 0x7fffffff, a zero -- and the
-// low bits are cut off instead, so that a NaN or an infinity stays one.
-constexpr float CL_ROUND_MAX = 0x1.ffep127f;
-__device__ __forceinline__ float tf32_rna_below(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
-__device__ __forceinline__ float tf32_rna(float x) {
-  return __uint_as_float((__float_as_uint(x) + (fabsf(x) < CL_ROUND_MAX ? 0x1000u : 0u)) & 0xffffe000u);
+__device__ __forceinline__ void cl_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
+               : "memory");
 }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2) {
   asm volatile(
@@ -72,196 +89,736 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, 
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
-__device__ __forceinline__ void cl_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, uint32_t src, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(src), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem], tf32
-__device__ __forceinline__ void umma_tf32_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}\n"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const float (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
 }
-__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const float (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
-        "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
-      : "memory");
+__device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ float2 unpack_f16(uint32_t v) {
+  return __half22float2(*reinterpret_cast<const __half2*>(&v));
+}
+// the larger magnitude of three, NaN if one is
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
-// a stage's row split once more, value by value (out of line: hardly any stage needs it, and its registers are the whole kernel's)
-__device__ __noinline__ void cl_split_again(const uint8_t* src, uint32_t t, int row) {
-#pragma unroll 1
-  for (int half = 0; half < 2; ++half) {
-    float hi[16], lo[16];
+// two fp32 values in one register pair: an instruction for both
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ float2 f2_get(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+// parts of two values, v * scale = hi + lo / 2048
+__device__ __forceinline__ void cl_parts(F2 a, float scale, uint32_t& hi, uint32_t& lo) {
+  const float2 x = f2_get(f2_mul(a, f2(scale))), y = f2_get(f2_mul(a, f2(scale * CL_LO_SCALE)));
+  hi = pack_f16(x.x, x.y);
+  float l0, l1;          // 2048 (x - hi), both steps exact
+  asm("{\n\t.reg .b16 h0, h1, m;\n\tmov.b32 {h0, h1}, %2;\n\tmov.b16 m, 0xE800;\n\tfma.rn.f32.f16 %0, h0, m, %3;\n\tfma.rn.f32.f16 %1, h1, m, %4;\n\t}\n"
+      : "=f"(l0), "=f"(l1)
+      : "r"(hi), "f"(y.x), "f"(y.y));
+  lo = pack_f16(l0, l1);
+}
+// Two rows of a block whose channels lie in the lanes: neighbouring lanes exchange, even ones keep two high parts, odd ones two low parts of each
+// row -> word (lane & 1 ? 16 : 0) + (lane >> 1) of either row
+__device__ __forceinline__ void cl_exchange(uint32_t hi, uint32_t lo, uint32_t& w0, uint32_t& w1) {
+  const bool odd = threadIdx.x & 1;
+  const uint32_t own = odd ? lo : hi, got = __shfl_xor_sync(0xffffffffu, odd ? hi : lo, 1);
+  w0 = __byte_perm(own, got, odd ? 0x1054u : 0x5410u);
+  w1 = __byte_perm(own, got, odd ? 0x3276u : 0x7632u);
+}
+// what a block of 32 activations with the largest magnitude m is kept as
+__device__ __forceinline__ uint32_t cl_code(float m) { return !(m < CL_X_TOP) ? CB_RAW : m == 0.f ? 0u : m < CL_X_LOW ? CB_QUIET : CB_NORMAL; }
+// Activations kept as parts: 128 bytes per 32 channels as in fp32, [32 high | 32 low] fp16 -- or, where one of the 32 is out of range, the fp32
+// values themselves, with CB_RAW in the block's code byte.  Here for eight neighbouring lanes that hold a block's channels, four each.
+__device__ __forceinline__ void cl_put4(uint32_t* yp, uint8_t* code, size_t at, const float4& v) {
+  float m = max3_abs(max3_abs(v.x, v.y, v.z), v.w, v.w);
+  const uint32_t eight = 0xffu << (threadIdx.x & 24);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const float4 v = *reinterpret_cast<const float4*>(src + (((half * 4 + c) ^ (row & 7)) << 4));
-      const float x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        hi[4 * c + e] = tf32_rna(x[e]);
-        lo[4 * c + e] = tf32_rna(x[e] - hi[4 * c + e]);
-      }
-    }
-    tmem_st_32x16(t + 16 * half, hi);
-    tmem_st_32x16(t + 32 + 16 * half, lo);
+  for (int o = 1; o < 8; o <<= 1) {
+    const float other = __shfl_xor_sync(eight, m, o);
+    m = max3_abs(m, other, other);
   }
+  const uint32_t c = cl_code(m), in = static_cast<uint32_t>(at) & 31u;
+  uint32_t* blk = yp + (at - in);
+  if (c == CB_RAW) {
+    *reinterpret_cast<float4*>(blk + in) = v;
+  } else {
+    uint2 hi, lo;
+    cl_parts(f2(v.x, v.y), CL_X_SCALE, hi.x, lo.x);
+    cl_parts(f2(v.z, v.w), CL_X_SCALE, hi.y, lo.y);
+    *reinterpret_cast<uint2*>(blk + (in >> 1)) = hi;
+    *reinterpret_cast<uint2*>(blk + 16 + (in >> 1)) = lo;
+  }
+  if (in == 0) code[at >> 5] = static_cast<uint8_t>(c);
+}
+// ... and for a warp that holds a block, a channel a lane
+__device__ __forceinline__ void cl_put1(uint32_t* yp, uint8_t* code, size_t block, float v) {
+  const int lane = threadIdx.x & 31;
+  float m = v;
+  asm volatile("redux.sync.max.NaN.abs.f32 %0, %0, 0xffffffff;" : "+f"(m));
+  const uint32_t c = cl_code(m);
+  uint32_t hi, lo, word, unused;
+  cl_parts(f2(v, 0.f), CL_X_SCALE, hi, lo);
+  cl_exchange(hi, lo, word, unused);
+  if (c == CB_RAW) yp[block * 32 + lane] = __float_as_uint(v);
+  else yp[block * 32 + (lane & 1 ? 16 : 0) + (lane >> 1)] = word;
+  if (lane == 0) code[block] = static_cast<uint8_t>(c);
 }
 
-// sin(x)^2: the square needs x only modulo pi, so one rounding step k = x / pi and two fused steps x - k pi leave
-// |r| <= pi / 2, where sin r = r + r^3 P(r^2) with a fitted polynomial of degree 3 (largest relative error 6e-9).  Valid up to
-// |x| = 2^16 (k pi exact to 2^-33 there); larger arguments take sinf.  No branch per element: a row of 32 is interleaved.
+// sin(x)^2: the square needs x only modulo pi, so one rounding step k = x / pi (in the low bits of a sum with 1.5 2^23) and two fused steps
+// x - k pi leave |r| <= pi / 2, where sin r = r + r^3 P(r^2) with a fitted polynomial of degree 3 (largest relative error 6e-9).  Valid up
+// to |x| = 2^16 (k pi exact to 2^-33 there); larger arguments take sinf.  Two values an instruction and no branch per element.
 constexpr float CL_SIN_MAX = 65536.f;
-__device__ __forceinline__ float cl_sin_sq(float x) {
-  const float k = rintf(x * 0.318309886f);
-  float r = fmaf(k, -3.14159274101f, x);
-  r = fmaf(k, 8.742278012619e-08f, r);
-  const float u = r * r;
-  float q = fmaf(u, 2.605780761e-06f, -1.980960296e-04f);
-  q = fmaf(u, q, 8.333066247e-03f);
-  q = fmaf(u, q, -1.666665955e-01f);
-  const float sn = fmaf(r * u, q, r);
-  return sn * sn;
+__device__ __forceinline__ F2 cl_sin_sq(F2 x) {
+  const F2 k = f2_add(f2_fma(x, f2(0.318309886f), f2(12582912.f)), f2(-12582912.f));
+  const F2 r = f2_fma(k, f2(8.742278012619e-08f), f2_fma(k, f2(-3.14159274101f), x));
+  const F2 u = f2_mul(r, r);
+  F2 q = f2_fma(u, f2(2.605780761e-06f), f2(-1.980960296e-04f));
+  q = f2_fma(u, q, f2(8.333066247e-03f));
+  q = f2_fma(u, q, f2(-1.666665955e-01f));
+  const F2 sn = f2_fma(f2_mul(r, u), q, r);
+  return f2_mul(sn, sn);
 }
 // ELU without a branch: e^x - 1 = 2^n (e^r - 1) + (2^n - 1) with x = n ln 2 + r, |r| <= ln 2 / 2, and e^r - 1 = r + r^2 Q(r) with a
 // fitted polynomial of degree 4.  Largest relative error against 64 bits 8.7e-8 over [-90, 0].
-__device__ __forceinline__ float cl_elu(float v) {
-  const float x = fmaxf(v, -80.f);
-  const float t = fmaf(x, 1.44269504f, 12582912.f), n = t - 12582912.f;        // n in the low bits of t as well
-  float r = fmaf(n, -0.693359375f, x);
-  r = fmaf(n, 2.12194440e-4f, r);
-  float q = fmaf(r, 0.0013882514f, 0.0083665475f);
-  q = fmaf(q, r, 0.0416672f);
-  q = fmaf(q, r, 0.16666543f);
-  q = fmaf(q, r, 0.49999997f);
-  const float e = fmaf(r * r, q, r), s = __uint_as_float((__float_as_uint(t) << 23) + 0x3f800000u);
-  return v <= 0.f ? fmaf(s, e, s - 1.f) : v;
+__device__ __forceinline__ F2 cl_elu(F2 v) {
+  const float2 w = f2_get(v);
+  const F2 x = f2(fmaxf(w.x, -80.f), fmaxf(w.y, -80.f));
+  const F2 t = f2_fma(x, f2(1.44269504f), f2(12582912.f)), n = f2_add(t, f2(-12582912.f));        // n in the low bits of t as well
+  F2 r = f2_fma(n, f2(-0.693359375f), x);
+  r = f2_fma(n, f2(2.12194440e-4f), r);
+  F2 q = f2_fma(r, f2(0.0013882514f), f2(0.0083665475f));
+  q = f2_fma(q, r, f2(0.0416672f));
+  q = f2_fma(q, r, f2(0.16666543f));
+  q = f2_fma(q, r, f2(0.49999997f));
+  const F2 e = f2_fma(f2_mul(r, r), q, r);
+  const float2 tb = f2_get(t);
+  const F2 s = f2(__uint_as_float((__float_as_uint(tb.x) << 23) + 0x3f800000u), __uint_as_float((__float_as_uint(tb.y) << 23) + 0x3f800000u));
+  const float2 o = f2_get(f2_fma(s, e, f2_add(s, f2(-1.f))));
+  return f2(w.x <= 0.f ? o.x : w.x, w.y <= 0.f ? o.y : w.y);
 }
-__device__ __forceinline__ float4 cl_snake4(float4 v, const float4& a, const float4& inv) {
-  const float4 y = make_float4(a.x * v.x, a.y * v.y, a.z * v.z, a.w * v.w);
-  const float big = fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w)));
-  float4 s = make_float4(cl_sin_sq(y.x), cl_sin_sq(y.y), cl_sin_sq(y.z), cl_sin_sq(y.w));
-  if (!(big <= CL_SIN_MAX)) {
-    const float4 t = make_float4(sinf(y.x), sinf(y.y), sinf(y.z), sinf(y.w));
-    s = make_float4(t.x * t.x, t.y * t.y, t.z * t.z, t.w * t.w);
+// v + inv sin(a v)^2 of four values, two channels a pair
+__device__ __forceinline__ void cl_snake4(F2& v0, F2& v1, F2 a0, F2 a1, F2 i0, F2 i1) {
+  const F2 y0 = f2_mul(a0, v0), y1 = f2_mul(a1, v1);
+  const float2 p = f2_get(y0), q = f2_get(y1);
+  F2 s0 = cl_sin_sq(y0), s1 = cl_sin_sq(y1);
+  if (!(max3_abs(max3_abs(p.x, p.y, q.x), q.y, q.y) <= CL_SIN_MAX)) {      // (each value by itself: its result does not depend on the others)
+    const float2 a = f2_get(s0), b = f2_get(s1);
+    auto one = [](float y, float s) {
+      if (fabsf(y) <= CL_SIN_MAX) return s;
+      const float sn = sinf(y);
+      return sn * sn;
+    };
+    s0 = f2(one(p.x, a.x), one(p.y, a.y));
+    s1 = f2(one(q.x, b.x), one(q.y, b.y));
   }
-  return make_float4(fmaf(inv.x, s.x, v.x), fmaf(inv.y, s.y, v.y), fmaf(inv.z, s.z, v.z), fmaf(inv.w, s.w, v.w));
+  v0 = f2_fma(i0, s0, v0);
+  v1 = f2_fma(i1, s1, v1);
+}
+__device__ __forceinline__ float4 cl_snake4(const float4& v, const float4& a, const float4& inv) {
+  F2 v0 = f2(v.x, v.y), v1 = f2(v.z, v.w);
+  cl_snake4(v0, v1, f2(a.x, a.y), f2(a.z, a.w), f2(inv.x, inv.y), f2(inv.z, inv.w));
+  const float2 p = f2_get(v0), q = f2_get(v1);
+  return make_float4(p.x, p.y, q.x, q.y);
+}
+// a / b for 0 <= a < 2^31 with inv = ceil(2^32 / b), 0 for b == 1: the quotient or one more, as a product
+__device__ __forceinline__ int cl_div(int a, int b, uint32_t inv) {
+  if (inv == 0u) return a;
+  const int q = static_cast<int>(__umulhi(static_cast<uint32_t>(a), inv));
+  return q * static_cast<long long>(b) > a ? q - 1 : q;
 }
 struct ClUnit {
-  int n0, n_cur, t0, b0;
+  int m0, t0, b0;
 };
 __device__ __forceinline__ ClUnit cl_unit(const ClConvParams& p, int u) {
   ClUnit r;
-  const int m = u / p.n_tiles;                 // column tiles fastest: they share the activation boxes in L2
-  r.n0 = (u - m * p.n_tiles) * p.nt;
-  r.n_cur = min(p.nt, p.N - r.n0);
-  const int bt = m / p.t_tiles;
+  const int m = cl_div(u, p.m_tiles, p.m_tiles_inv);                 // channel tiles fastest: they share the activations in L2
+  r.m0 = (u - m * p.m_tiles) * 128;
+  const int bt = cl_div(m, p.t_tiles, p.t_tiles_inv);
   r.t0 = p.n_lo + (m - bt * p.t_tiles) * p.nr;
   r.b0 = bt * p.nb;
   return r;
 }
 
-// (96 registers a thread: what the epilogue needs.  Spilled registers go to a first-level cache that the stages leave 28 KB)
-__global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, const __grid_constant__ CUtensorMap x_map) {
+// Eight columns of a tile outside the split's range, in fp32: this warp's 32 channels, blocks [blk_lo, blk_hi) of K.  The weights come from their
+// packed parts.  Writes the accumulators, so that the epilogue goes on as if the products had.
+__device__ __noinline__ void cl_exact_chunk(const ClConvParams& p, const int4* col_tab, int m0, int t0, int b0, int c0, int lane_row,
+                                            int blk_lo, int blk_hi, uint32_t t_hi, uint32_t t_lo) {
+  float out[8];
+  const int blocks_per_tap = p.Cin >> 5;
+  const uint8_t* wt = p.w + static_cast<size_t>(m0 >> 7) * (blocks_per_tap * p.ksize) * CL_W_BLOCK + lane_row * 128;
+  const float w_scale = p.w_inv[m0 + lane_row] * CL_X_SCALE;
+#pragma unroll 1
+  for (int c = 0; c < 8; ++c) {
+    const int e = col_tab[c0 + c].x;
+    float acc = 0.f;
+    if (e >= 0) {
+      const int b = b0 + (e >> 16), t = t0 + (e & 0xffff);
+#pragma unroll 1
+      for (int tap = 0; tap < p.ksize; ++tap) {
+        const int ts = t - (p.ksize - 1 - tap) * p.dil;
+        const bool in = b < p.B && ts >= 0 && ts < p.Tx;
+        const long long row = in ? b * p.x_bstride + static_cast<long long>(ts) * p.Cin : 0ll;
+#pragma unroll 1
+        for (int k = blk_lo * 32; k < blk_hi * 32; ++k) {
+          const uint8_t* blk = wt + static_cast<size_t>(tap * blocks_per_tap + (k >> 5)) * CL_W_BLOCK + (k & 7) * 2;
+          const int chunk = (k >> 3) & 3, sw = lane_row & 7;
+          const float hi = __half2float(*reinterpret_cast<const __half*>(blk + ((chunk ^ sw) << 4))),
+                      lo = __half2float(*reinterpret_cast<const __half*>(blk + (((chunk + 4) ^ sw) << 4)));
+          float xv = 0.f;
+          if (in) {
+            if (!p.x_code || (__ldcg(p.x_code + ((row + k) >> 5)) & CB_RAW)) {
+              xv = __ldcg(p.x + row + k);
+            } else {
+              const __half* xb = reinterpret_cast<const __half*>(p.x + ((row + k) & ~31ll));
+              xv = fmaf(__half2float(__ldcg(xb + 32 + (k & 31))), 1.f / CL_LO_SCALE, __half2float(__ldcg(xb + (k & 31)))) * (1.f / CL_X_SCALE);
+            }
+          }
+          acc = fmaf(xv, fmaf(lo, 1.f / CL_LO_SCALE, hi) * w_scale, acc);
+        }
+      }
+    }
+    out[c] = acc;
+  }
+  tmem_st_32x8(t_hi, out);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) out[c] = 0.f;
+  tmem_st_32x8(t_lo, out);
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// copies of a channel tile of `width` channels in the 128 rows of its weights: the epilogue's warps share their columns
+__host__ __device__ __forceinline__ int cl_copies(int width) { return width == 32 ? 4 : width == 64 ? 2 : 1; }
+
+struct ClEpiState {          // of a thread of the epilogue, for one unit: its channel and where that lies at the unit's first position
+  int n;
+  float bias, scale, alpha, ialpha;
+  float *y, *y2;
+  uint32_t* yp;                // the block of 32 channels that the warp holds
+  uint8_t* code;
+  const float *resid, *noise;
+};
+// What the epilogue's loops read of the launch's parameters, in registers: behind every asm statement that clobbers memory the compiler reads
+// the parameters themselves again, and a dozen such reads were most of a chunk's time (Mimi's 1x1 layer of 153600 x 128: 62 us).
+struct ClHot {
+  int cols, N, epi, act;
+  bool two, res, parts;
+};
+// The epilogue works on eight columns at a time, in a loop that is short enough for the instruction caches: sixteen columns in straight-line
+// code took twice as long (Mimi's 1x1 layer of 153600 x 128 85 us).
+constexpr int CL_EC = 8;
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr));
+}
+// where column c0 + (lane & 7) lies: its entry in the table, or x = -1 where there is no such position
+__device__ __forceinline__ int4 cl_column(const ClConvParams& p, const ClUnit& g, const int4* col_tab, int c0) {
+  int4 tb = col_tab[c0 + (threadIdx.x & (CL_EC - 1))];
+  if (!(tb.x >= 0 && g.b0 + (tb.x >> 16) < p.B && g.t0 + (tb.x & 0xffff) < p.n_hi)) tb.x = -1;
+  return tb;
+}
+__device__ __forceinline__ void cl_residual(const ClConvParams& p, const ClHot& h, const ClEpiState& e, const ClUnit& g, const int4* col_tab, int c0, int inside,
+                                            float (&rs)[CL_EC]) {
+  if (c0 + CL_EC <= inside) {
+    const float* r = e.resid + static_cast<long long>(c0) * h.N;
+#pragma unroll
+    for (int c = 0; c < CL_EC; ++c) rs[c] = __ldcg(r + c * h.N);
+    return;
+  }
+  const int4 tb = cl_column(p, g, col_tab, c0);
+#pragma unroll
+  for (int c = 0; c < CL_EC; ++c) {
+    const bool ok = __shfl_sync(0xffffffffu, tb.x, c) >= 0;
+    const int o = __shfl_sync(0xffffffffu, tb.z, c);
+    rs[c] = ok ? __ldcg(e.resid + o) : 0.f;
+  }
+}
+__device__ __forceinline__ void cl_load_acc(uint32_t taddr, int cols, float inv, F2 (&v)[CL_EC / 2]) {
+  uint32_t hi[CL_EC], lo[CL_EC];
+  tmem_ld_32x8(taddr, hi);
+  tmem_ld_32x8(taddr + cols, lo);
+  tmem_ld_wait();
+#pragma unroll
+  for (int c = 0; c < CL_EC / 2; ++c)
+    v[c] = f2_mul(f2_fma(f2(__uint_as_float(lo[2 * c]), __uint_as_float(lo[2 * c + 1])), f2(1.f / CL_LO_SCALE),
+                         f2(__uint_as_float(hi[2 * c]), __uint_as_float(hi[2 * c + 1]))),
+                  f2(inv));
+}
+__device__ __forceinline__ void cl_linear(const ClConvParams& p, const ClHot& h, const ClEpiState& e, const ClUnit& g, const int4* col_tab, int c0, F2 (&v)[CL_EC / 2],
+                                          const float (&rs)[CL_EC]) {
+#pragma unroll
+  for (int c = 0; c < CL_EC / 2; ++c) v[c] = f2_add(v[c], f2(e.bias));
+  if (h.epi == CE_SCALE_RESID) {
+#pragma unroll
+    for (int c = 0; c < CL_EC / 2; ++c) v[c] = f2_fma(v[c], f2(e.scale), f2(rs[2 * c], rs[2 * c + 1]));
+  } else if (h.epi == CE_NOISE) {
+    const int4 tb = cl_column(p, g, col_tab, c0);
+    const float nz = tb.x >= 0 ? __ldcg(e.noise + tb.w) : 0.f;
+#pragma unroll
+    for (int c = 0; c < CL_EC / 2; ++c)
+      v[c] = f2_fma(v[c], f2(__shfl_sync(0xffffffffu, nz, 2 * c), __shfl_sync(0xffffffffu, nz, 2 * c + 1)), f2(rs[2 * c], rs[2 * c + 1]));
+  } else if (h.epi == CE_RESID) {
+#pragma unroll
+    for (int c = 0; c < CL_EC / 2; ++c) v[c] = f2_add(v[c], f2(rs[2 * c], rs[2 * c + 1]));
+  }
+}
+// act(v), in place
+template <int ACT>
+__device__ __forceinline__ void cl_act(const ClEpiState& e, F2 (&v)[CL_EC / 2]) {
+  if (ACT == CA_SNAKE) {
+#pragma unroll
+    for (int c = 0; c < CL_EC / 2; c += 2) cl_snake4(v[c], v[c + 1], f2(e.alpha), f2(e.alpha), f2(e.ialpha), f2(e.ialpha));
+  } else if (ACT == CA_ELU) {
+#pragma unroll
+    for (int c = 0; c < CL_EC / 2; ++c) v[c] = cl_elu(v[c]);
+  } else if (ACT == CA_GELU) {
+#pragma unroll
+    for (int c = 0; c < CL_EC / 2; ++c) {
+      const float2 x = f2_get(v[c]);
+      v[c] = f2(0.5f * x.x * (1.f + erff(x.x * 0.70710678118654752f)), 0.5f * x.y * (1.f + erff(x.y * 0.70710678118654752f)));
+    }
+  }
+}
+// eight words of a thread, one a row
+__device__ __forceinline__ void cl_store(const ClConvParams& p, const ClHot& h, const ClUnit& g, const int4* col_tab, int c0, int inside, uint32_t* y,
+                                         const uint32_t (&w)[CL_EC]) {
+  if (c0 + CL_EC <= inside) {
+    y += static_cast<long long>(c0) * h.N;
+#pragma unroll
+    for (int c = 0; c < CL_EC; ++c) y[c * h.N] = w[c];
+    return;
+  }
+  const int4 tb = cl_column(p, g, col_tab, c0);
+#pragma unroll
+  for (int c = 0; c < CL_EC; ++c) {
+    const bool ok = __shfl_sync(0xffffffffu, tb.x, c) >= 0;
+    const int o = __shfl_sync(0xffffffffu, tb.y, c);
+    if (ok) y[o] = w[c];
+  }
+}
+__device__ __forceinline__ void cl_store(const ClConvParams& p, const ClHot& h, const ClUnit& g, const int4* col_tab, int c0, int inside, float* y,
+                                         const F2 (&v)[CL_EC / 2]) {
+  uint32_t w[CL_EC];
+#pragma unroll
+  for (int c = 0; c < CL_EC / 2; ++c) {
+    const float2 x = f2_get(v[c]);
+    w[2 * c] = __float_as_uint(x.x);
+    w[2 * c + 1] = __float_as_uint(x.y);
+  }
+  cl_store(p, h, g, col_tab, c0, inside, reinterpret_cast<uint32_t*>(y), w);
+}
+// eight rows of a block as parts.  One code for all of them: what is out of range somewhere in a chunk is kept as it is in all of it
+__device__ __forceinline__ void cl_store_parts(const ClConvParams& p, const ClHot& h, const ClEpiState& e, const ClUnit& g, const int4* col_tab, int c0, int inside,
+                                               const F2 (&v)[CL_EC / 2]) {
+  const int lane = threadIdx.x & 31;
+  const int4 tb = cl_column(p, g, col_tab, c0);
+  float m = 0.f;
+#pragma unroll
+  for (int c = 0; c < CL_EC / 2; ++c) {
+    float2 x = f2_get(v[c]);
+    if (c0 + CL_EC > inside) {
+      x.x = __shfl_sync(0xffffffffu, tb.x, 2 * c) >= 0 ? x.x : 0.f;
+      x.y = __shfl_sync(0xffffffffu, tb.x, 2 * c + 1) >= 0 ? x.y : 0.f;
+    }
+    m = max3_abs(m, x.x, x.y);
+  }
+  asm volatile("redux.sync.max.NaN.abs.f32 %0, %0, 0xffffffff;" : "+f"(m));
+  const uint32_t code = cl_code(m);
+  if (lane < CL_EC && tb.x >= 0) e.code[tb.y >> 5] = static_cast<uint8_t>(code);
+  if (code == CB_RAW) {
+    cl_store(p, h, g, col_tab, c0, inside, reinterpret_cast<float*>(e.yp + lane), v);
+    return;
+  }
+  uint32_t w[CL_EC];
+#pragma unroll
+  for (int c = 0; c < CL_EC / 2; ++c) {
+    uint32_t hi, lo;
+    cl_parts(v[c], CL_X_SCALE, hi, lo);
+    cl_exchange(hi, lo, w[2 * c], w[2 * c + 1]);
+  }
+  cl_store(p, h, g, col_tab, c0, inside, e.yp + (lane & 1 ? 16 : 0) + (lane >> 1), w);
+}
+__device__ __forceinline__ void cl_finish(const ClConvParams& p, const ClHot& h, const ClEpiState& e, const ClUnit& g, const int4* col_tab, int c0, int inside,
+                                          F2 (&v)[CL_EC / 2]) {
+  if (h.two) cl_store(p, h, g, col_tab, c0, inside, e.y, v);
+  if (h.act == CA_SNAKE) cl_act<CA_SNAKE>(e, v);
+  else if (h.act == CA_ELU) cl_act<CA_ELU>(e, v);
+  else if (h.act == CA_GELU) cl_act<CA_GELU>(e, v);
+  if (h.parts) cl_store_parts(p, h, e, g, col_tab, c0, inside, v);
+  else cl_store(p, h, g, col_tab, c0, inside, e.y2 ? e.y2 : e.y, v);
+}
+
+struct ClMaps {
+  CUtensorMap x, y, last, r;         // activations; boxes of plain values beside others, of the last values (fp32 or parts), of residuals
+};
+struct ClBoxes {               // a warp's boxes of 8 x 32 words
+  uint32_t at;                 // four of them
+  uint64_t* res_full;          // the box of residuals has landed
+  uint32_t res_ph, flip;
+};
+// The chunks of a unit whose tile is one run of positions: results leave and residuals come as boxes.  A thread's words lie 128 bytes apart in
+// them, so a word costs one instruction with a constant offset (its address in global memory costs two or three more).
+template <int ACT>
+__device__ __forceinline__ void cl_boxed_chunks(const ClHot& h, const ClMaps& maps, const ClEpiState& e, int n_box, int t0, int b0, int inside,
+                                                uint32_t taddr, float inv, int c_first, int c_step, ClBoxes& bx, BoundedWait& bw) {
+  const int lane = threadIdx.x & 31, cols = h.cols;
+  const bool two = h.two, res = h.res, parts = h.parts;
+#pragma unroll 1
+  for (int c0 = c_first; c0 < cols; c0 += c_step) {
+    const uint32_t in = bx.at + (bx.flip ? 1024u : 0u) + lane * 4;                       // residuals, or plain values
+    const uint32_t out = bx.at + (res ? 2048u : two ? (bx.flip ? 3072u : 1024u) : 2048u) + (res || !two ? (bx.flip ? 1024u : 0u) : 0u);
+    const uint32_t plain = bx.at + (bx.flip ? 2048u : 0u);
+    if (res) {
+      bw.wait(bx.res_full, bx.res_ph);
+      if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; return; }
+      bx.res_ph ^= 1u;
+      if (lane == 0 && c0 + c_step < cols) {           // (the other box has been read: every lane has passed the chunk in front)
+        mbar_arrive_expect_tx(bx.res_full, 1024u);
+        tma_load_3d(bx.at + (bx.flip ? 0u : 1024u), &maps.r, smem_u32(bx.res_full), n_box, t0 + c0 + c_step, b0);
+      }
+    }
+    F2 v[CL_EC / 2];
+    cl_load_acc(taddr + c0, cols, inv, v);
+#pragma unroll
+    for (int c = 0; c < CL_EC / 2; ++c) v[c] = f2_add(v[c], f2(e.bias));
+    if (res) {
+      float rs[CL_EC];
+#pragma unroll
+      for (int c = 0; c < CL_EC; ++c) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(rs[c]) : "r"(in + c * 128) : "memory");
+      if (h.epi == CE_RESID) {
+#pragma unroll
+        for (int c = 0; c < CL_EC / 2; ++c) v[c] = f2_add(v[c], f2(rs[2 * c], rs[2 * c + 1]));
+      } else if (h.epi == CE_SCALE_RESID) {
+#pragma unroll
+        for (int c = 0; c < CL_EC / 2; ++c) v[c] = f2_fma(v[c], f2(e.scale), f2(rs[2 * c], rs[2 * c + 1]));
+      } else {
+        const float nz = (lane & 7) + c0 < inside ? __ldcg(e.noise + c0 + (lane & 7)) : 0.f;
+#pragma unroll
+        for (int c = 0; c < CL_EC / 2; ++c)
+          v[c] = f2_fma(v[c], f2(__shfl_sync(0xffffffffu, nz, 2 * c), __shfl_sync(0xffffffffu, nz, 2 * c + 1)), f2(rs[2 * c], rs[2 * c + 1]));
+      }
+    }
+    // the boxes stored two chunks ago have been read
+    if (lane == 0) bulk_wait_read<1>();
+    __syncwarp();
+    auto put = [&](uint32_t a) {
+#pragma unroll
+      for (int c = 0; c < CL_EC / 2; ++c) {
+        const float2 x = f2_get(v[c]);
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(a + 2 * c * 128), "f"(x.x) : "memory");
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(a + (2 * c + 1) * 128), "f"(x.y) : "memory");
+      }
+    };
+    if (two) put(plain + lane * 4);
+    cl_act<ACT>(e, v);
+    if (parts) {
+      float m = 0.f;
+      if (c0 + CL_EC <= inside) {
+#pragma unroll
+        for (int c = 0; c < CL_EC / 2; ++c) {
+          const float2 x = f2_get(v[c]);
+          m = max3_abs(m, x.x, x.y);
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < CL_EC / 2; ++c) {
+          const float2 x = f2_get(v[c]);
+          m = max3_abs(m, c0 + 2 * c < inside ? x.x : 0.f, c0 + 2 * c + 1 < inside ? x.y : 0.f);
+        }
+      }
+      asm volatile("redux.sync.max.NaN.abs.f32 %0, %0, 0xffffffff;" : "+f"(m));
+      const uint32_t code = cl_code(m);
+      if (lane < CL_EC && c0 + lane < inside) e.code[(c0 + lane) * (h.N >> 5)] = static_cast<uint8_t>(code);
+      if (code == CB_RAW) {
+        put(out + lane * 4);
+      } else {
+        const uint32_t a = out + (lane & 1 ? 64u : 0u) + (lane >> 1) * 4;
+#pragma unroll
+        for (int c = 0; c < CL_EC / 2; ++c) {
+          uint32_t hi, lo, w0, w1;
+          cl_parts(v[c], CL_X_SCALE, hi, lo);
+          cl_exchange(hi, lo, w0, w1);
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(a + 2 * c * 128), "r"(w0) : "memory");
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(a + (2 * c + 1) * 128), "r"(w1) : "memory");
+        }
+      }
+    } else {
+      put(out + lane * 4);
+    }
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) {             // (what a box has past the last position is not written)
+      if (two) tma_store_3d(&maps.y, plain, n_box, t0 + c0, b0);
+      tma_store_3d(&maps.last, out, n_box, t0 + c0, b0);
+      bulk_commit();
+    }
+    bx.flip ^= 1u;
+  }
+}
+
+struct ClSplit {
+  uint32_t smem0;
+  int x_bytes, u_first, u_step, kb_lo, x_steps;
+  uint64_t *x_ready, *x_empty, *top_full, *top_empty;
+  float* tops;
+  const int2* row_tab;
+};
+// The split's loop.  A thread takes one 16-byte chunk of every 16th row (32nd where a stage is 32 channels wide): NP rows of a stage, in batches
+// of eight loads -- half a stage or several stages.  As soon as a row is converted the row of the next batch that takes its registers is asked
+// for, so eight loads a thread are on the way all the time, across stages and units.
+template <int NP>
+__device__ __forceinline__ void cl_split(const ClConvParams& p, const ClSplit& sp, BoundedWait& bw) {
+  constexpr int NJ = 8, PB = NP < NJ ? NP : NJ, SB = NJ / PB, HALVES = NP / PB;      // rows and stages of a batch, batches of a stage
+  constexpr int NONE = static_cast<int>(0x80000000u);
+  const int wsp = (threadIdx.x >> 5) - 2, lane = threadIdx.x & 31;
+  const int lanes = 8 * p.group, ch = lane & (lanes - 1), rows_pass = 256 / lanes, row0 = wsp * (32 / lanes) + lane / lanes;
+  const int rows = p.cols + p.halo;
+  // (rows_pass is a multiple of 16, so the swizzle of a thread's rows is one)
+  const uint32_t dst0 = sp.smem0 + (ch >> 3) * p.rows_pad * 128 + (ch & 1) * 8 + row0 * 128 + ((((ch >> 1) & 3) ^ (row0 & 7)) << 4);
+  int off[NP];
+  const float* xu = p.x;             // first position of the unit's first entry, this thread's channels
+  int u = sp.u_first, st = 0, half = 0;                    // the batch in registers
+  // rows of unit `v` (for stage `stage` where every tap has its own)
+  auto rows_of = [&](int v, int stage) {
+    const ClUnit g = cl_unit(p, v);
+    const int shift = p.taps > 1 ? p.halo : (p.ksize > 1 ? (p.ksize - 1 - stage % p.ksize) * p.dil : 0);
+    xu = p.x + g.b0 * p.x_bstride + static_cast<long long>(g.t0 - shift) * p.Cin + ch * 4;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int r = i * rows_pass + row0;
+      const int2 tab = r < rows ? sp.row_tab[r] : make_int2(-1, 0);
+      const int t = g.t0 - shift + (tab.x & 0xffff);
+      off[i] = tab.x >= 0 && g.b0 + (tab.x >> 16) < p.B && t >= 0 && t < min(p.Tx, p.n_hi) ? tab.y : NONE;
+    }
+  };
+  const bool by_tap = p.taps == 1 && p.ksize > 1;          // (only with one stage a batch)
+  auto channels = [&](int stage) { return xu + (sp.kb_lo + (by_tap ? stage / p.ksize : stage)) * p.group * 32; };
+  auto load = [&](const float* xk, int o) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (o != NONE) v = __ldcg(reinterpret_cast<const float4*>(xk + o));
+    return v;
+  };
+  float4 v[NJ];
+  if (u < p.units) {
+    rows_of(u, 0);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (j / PB < sp.x_steps) v[j] = load(channels(j / PB), off[j % PB]);
+    }
+  }
+  int s = 0, it = 0;
+  uint32_t ph = 0;
+  float top = 0.f;
+#pragma unroll 1
+  while (u < p.units) {
+    int nu = u, ns = st, nh = half + 1;
+    if (nh == HALVES) {
+      nh = 0;
+      ns += SB;
+      if (ns >= sp.x_steps) {
+        ns = 0;
+        nu += sp.u_step;
+      }
+    }
+    const bool more = nu < p.units;
+    if (more && (nu != u || (by_tap && ns != st))) rows_of(nu, ns);
+    const float* xk = channels(ns);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const bool on = SB == 1 || st + j / PB < sp.x_steps;
+      if (on) {
+        if (j % PB == 0 && (HALVES == 1 || half == 0)) {
+          bw.wait(&sp.x_empty[s], ph ^ 1u);
+          if (!__all_sync(0xffffffffu, !bw.dead)) {
+            bw.dead = true;
+            return;
+          }
+        }
+        const int pass = HALVES == 1 ? j % PB : half * PB + j;
+        if (pass * rows_pass < rows) {
+          uint32_t h0, h1, l0, l1;
+          cl_parts(f2(v[j].x, v[j].y), CL_X_SCALE, h0, l0);
+          cl_parts(f2(v[j].z, v[j].w), CL_X_SCALE, h1, l1);
+          top = max3_abs(max3_abs(top, v[j].x, v[j].y), v[j].z, v[j].w);
+          const uint32_t a = dst0 + s * sp.x_bytes + pass * rows_pass * 128;
+          asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(h0), "r"(h1) : "memory");
+          asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a ^ 64u), "r"(l0), "r"(l1) : "memory");
+        }
+      }
+      if (more) {
+        if (HALVES == 1) {
+          if (SB == 1 || ns + j / PB < sp.x_steps) v[j] = load(SB == 1 ? xk : xk + (j / PB) * p.group * 32, off[j % PB]);
+        } else {
+          v[j] = load(xk, nh == 0 ? off[j] : off[(PB + j) % NP]);
+        }
+      }
+      if (on && j % PB == PB - 1 && (HALVES == 1 || half == HALVES - 1)) {        // the warp's rows of the stage are there
+        const bool last = st + j / PB + 1 == sp.x_steps;
+        if (last) {
+          asm volatile("redux.sync.max.NaN.abs.f32 %0, %0, 0xffffffff;" : "+f"(top));
+          bw.wait(&sp.top_empty[it & 7], ((it >> 3) & 1) ^ 1);
+          if (lane == 0) sp.tops[(it & 7) * CL_SPLIT_WARPS + wsp] = top;
+          top = 0.f;
+        }
+        __syncwarp();
+        if (lane == 0) {
+          if (last) mbar_arrive(&sp.top_full[it & 7]);
+          mbar_arrive(&sp.x_ready[s]);
+        }
+        if (last) ++it;
+        if (++s == p.x_stages) { s = 0; ph ^= 1u; }
+      }
+    }
+    u = nu;
+    st = ns;
+    half = nh;
+  }
+}
+
+// PARTS: the activations come as parts, fetched by a tensor map; otherwise as fp32, split on the way
+template <bool PARTS>
+struct ClRoles {
+  static constexpr int FIRST_EPI = PARTS ? 4 : 2 + CL_SPLIT_WARPS, EPI_WARPS = PARTS ? 12 : 8, THREADS = 32 * (FIRST_EPI + EPI_WARPS);
+};
+template <bool PARTS>
+__global__ void __launch_bounds__(ClRoles<PARTS>::THREADS, 1) cl_conv_kernel(const __grid_constant__ ClConvParams p, const __grid_constant__ ClMaps maps) {
+  constexpr int FIRST_EPI = ClRoles<PARTS>::FIRST_EPI, EPI_WARPS = ClRoles<PARTS>::EPI_WARPS, THREADS = ClRoles<PARTS>::THREADS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int stage_bytes = CL_A_BYTES + p.nt * 256;
-  float* epi_sm = reinterpret_cast<float*>(smem + p.stages * stage_bytes);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes + CL_EPI_BYTES);   // copies have landed
-  uint64_t* ready = full + CL_MAX_STAGES;        // the halves are in TMEM
-  uint64_t* empty = ready + CL_MAX_STAGES;       // the MMAs have read the stage
-  uint64_t* acc_full = empty + CL_MAX_STAGES;    // [2]
-  uint64_t* acc_empty = acc_full + 2;            // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-  const uint32_t gate = smem_u32(tmem_slot + 1);  // set once the kernels in front have completed
-  int4* row_tab = reinterpret_cast<int4*>(smem + p.stages * stage_bytes + CL_EPI_BYTES + 512);     // [128]
+  const int x_sub = p.rows_pad * 128, x_bytes = p.group * x_sub, w_bytes = p.group * CL_W_BLOCK;
+  uint8_t* w_smem = smem + p.x_stages * x_bytes;
+  uint8_t* boxes = w_smem + p.w_stages * w_bytes;               // four boxes per epilogue warp
+  uint8_t* tail = boxes + (p.staged ? EPI_WARPS * 4096 : 0);
+  uint64_t* x_ready = reinterpret_cast<uint64_t*>(tail);        // a stage's parts are in shared memory
+  uint64_t* x_empty = x_ready + CL_X_STAGES;                    // the MMAs have read them
+  uint64_t* w_full = x_empty + CL_X_STAGES;
+  uint64_t* w_empty = w_full + CL_W_STAGES;
+  uint64_t* acc_full = w_empty + CL_W_STAGES;                   // [2]
+  uint64_t* acc_empty = acc_full + 2;                           // [2]
+  uint64_t* top_full = acc_empty + 2;                           // [CL_TOPS] a unit's range of values is known (units taken in turn)
+  uint64_t* top_empty = top_full + CL_TOPS;
+  uint64_t* res_full = top_empty + CL_TOPS;                     // [EPI_WARPS]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(res_full + 12);
+  const uint32_t gate = smem_u32(tmem_slot + 1);                // set once the kernels in front have completed
+  float* tops = reinterpret_cast<float*>(tail + 640);           // [CL_TOPS][CL_SPLIT_WARPS] largest magnitudes; with PARTS one word of codes
+  int2* row_tab = reinterpret_cast<int2*>(tail + 1024);         // [CL_ROWS] (entry << 16 | row of the entry) or -1, offset in x
+  int4* col_tab = reinterpret_cast<int4*>(tail + 1024 + CL_ROWS * 8);      // [CL_ROWS] the same or -1, offsets in y, resid, noise
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   BoundedWait bw{p.wait_flag, gate};
 
   if (warp == 0 && lane == 0) {
     tmem_slot[1] = 0u;
-    prefetch_tmap(&x_map);
-    for (int s = 0; s < p.stages; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&ready[s], 4);
-      mbar_init(&empty[s], 1);
+    if (PARTS) prefetch_tmap(&maps.x);
+    for (int s = 0; s < CL_X_STAGES; ++s) {
+      mbar_init(&x_ready[s], PARTS ? 1 : CL_SPLIT_WARPS);
+      mbar_init(&x_empty[s], 1);
+    }
+    for (int s = 0; s < CL_W_STAGES; ++s) {
+      mbar_init(&w_full[s], 1);
+      mbar_init(&w_empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&acc_full[i], 1);
-      mbar_init(&acc_empty[i], CL_EPI_WARPS);
+      mbar_init(&acc_empty[i], EPI_WARPS);
     }
+    for (int i = 0; i < CL_TOPS; ++i) {
+      mbar_init(&top_full[i], PARTS ? 1 : CL_SPLIT_WARPS);
+      mbar_init(&top_empty[i], EPI_WARPS);
+    }
+    for (int i = 0; i < EPI_WARPS; ++i) mbar_init(&res_full[i], 1);
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, p.tmem_cols);
+    tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  // tile row -> (batch entry << 16 | position) inside a tile, and where it lies from the tile's first row on in the output and in the
-  // residual: the same for every tile (32-bit offsets, the host keeps a launch below 2^31 elements)
-  if (warp >= 6 && warp < 10) {
-    const int r = (warp - 6) * 32 + lane, bb = r / p.nr, tt = r - bb * p.nr;
-    row_tab[r] = make_int4(bb < p.nb ? (bb << 16) | tt : -1, bb * static_cast<int>(p.y_bstride) + tt * p.ldy,
-                           bb * static_cast<int>(p.r_bstride) + tt * p.ldr, 0);
+  for (int r = threadIdx.x; r < CL_ROWS; r += THREADS) {      // the same for every tile
+    const int e = r / p.pitch, q = r - e * p.pitch;
+    row_tab[r] = make_int2(e < p.nb ? (e << 16) | q : -1, static_cast<int>(e * p.x_bstride) + q * p.Cin);
+    col_tab[r] = make_int4(e < p.nb && q < p.nr ? (e << 16) | q : -1, static_cast<int>(e * p.y_bstride) + q * p.N,
+                           static_cast<int>(e * p.r_bstride) + q * p.N, e * p.noise_ld + q);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t a_col0 = tmem_base + 2 * p.acc_cols;    // stage s: hi at + 64 s, lo at + 64 s + 32
+  // this CTA's units, and its share of a unit's channels
+  const int rank = p.splits > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int u_first = p.splits > 1 ? blockIdx.x / p.splits : blockIdx.x, u_step = p.splits > 1 ? p.units : gridDim.x;
+  const int kb_lo = rank * p.kb / p.splits, kb_n = (rank + 1) * p.kb / p.splits - kb_lo;
+  const int tap_steps = p.ksize / p.taps, x_steps = kb_n * tap_steps;        // stages of activations a unit takes
 
   if (warp == 0) {
-    // ================= copies =================
+    // ================= weights =================
     if (lane == 0) {
-      const uint32_t box_bytes = static_cast<uint32_t>(p.nr * p.nb) * 128u, smem_a = smem_u32(smem), bar0 = smem_u32(full);
-      const size_t half_bytes = static_cast<size_t>(p.n_pad) * 128;
-      int s = 0;
+      const int blocks_per_tap = p.Cin >> 5;
+      const size_t tile_bytes = static_cast<size_t>(blocks_per_tap) * p.ksize * CL_W_BLOCK;
+      const uint32_t dst0 = smem_u32(w_smem), bar0 = smem_u32(w_full);
+      int s = 0, pre = p.w_stages;         // stages filled before the kernels in front have completed: weights do not depend on them
       uint32_t ph = 0;
-      bool waited = false;
-      for (int u = blockIdx.x; u < p.units && !bw.dead; u += gridDim.x) {
-        const ClUnit g = cl_unit(p, u);
-        const uint32_t w_bytes = static_cast<uint32_t>(g.n_cur) * 128u;
-        const uint8_t* wsrc = p.w + static_cast<size_t>(g.n0) * 128;
-        auto load_w = [&](int stage) {
-          const uint32_t dst = smem_a + stage * stage_bytes + CL_A_BYTES, bar = bar0 + 8 * stage;
-          cl_bulk(dst, wsrc, w_bytes, bar);
-          cl_bulk(dst + w_bytes, wsrc + half_bytes, w_bytes, bar);
-          wsrc += 2 * half_bytes;
-        };
-        int tap = 0, kb = 0;
-        auto load_x = [&](int stage) {
-          tma_load_3d(smem_a + stage * stage_bytes, &x_map, bar0 + 8 * stage, kb * 32, g.t0 - (p.ksize - 1 - tap) * p.dil, g.b0);
-          if (++kb == p.kb_per_tap) { kb = 0; ++tap; }
-        };
-        int i = 0;
-        if (!waited) {          // weights do not depend on the previous kernel
-          const int npre = min(p.stages, p.ksteps);
-          for (int j = 0; j < npre; ++j) {
-            mbar_arrive_expect_tx(&full[j], box_bytes + 2 * w_bytes);
-            load_w(j);
+      auto after_wait = [&]() {
+        pdl_wait();
+        wait_gate_open(gate);
+        pdl_trigger();
+      };
+      for (int u = u_first; u < p.units && !bw.dead; u += u_step) {
+        const uint8_t* src = p.w + static_cast<size_t>(cl_unit(p, u).m0 >> 7) * tile_bytes;
+        for (int i = kb_lo; i < kb_lo + kb_n && !bw.dead; ++i) {
+          for (int tap = 0; tap < p.ksize; ++tap) {
+            if (pre == 0) after_wait();
+            --pre;
+            if (!p.resident) bw.wait(&w_empty[s], ph ^ 1u);
+            if (bw.dead) break;
+            mbar_arrive_expect_tx(&w_full[s], w_bytes);
+            cl_bulk(dst0 + s * w_bytes, src + static_cast<size_t>(tap * blocks_per_tap + i * p.group) * CL_W_BLOCK, w_bytes, bar0 + 8 * s);
+            if (++s == p.w_stages) { s = 0; ph ^= 1u; }
           }
-          pdl_wait();
-          wait_gate_open(gate);
-          pdl_trigger();
-          for (int j = 0; j < npre; ++j) load_x(j);
-          waited = true;
-          i = npre;
-          s = npre == p.stages ? 0 : npre;
-          ph = npre == p.stages ? 1u : 0u;
         }
-        for (; i < p.ksteps; ++i) {
-          bw.wait(&empty[s], ph ^ 1u);
-          if (bw.dead) break;
-          mbar_arrive_expect_tx(&full[s], box_bytes + 2 * w_bytes);
-          load_x(s);
-          load_w(s);
-          if (++s == p.stages) { s = 0; ph ^= 1u; }
-        }
+        if (p.resident) break;
       }
+      if (pre >= 0) after_wait();
       if (bw.dead) {            // let the copies in flight land before the block may leave
         const unsigned long long t0 = gtimer();
         while (gtimer() - t0 < 2000000ull) __nanosleep(1000);
@@ -270,269 +827,338 @@ __global__ void __launch_bounds__(640, 1) cl_conv_kernel(const ClConvParams p, c
     __syncwarp();
   } else if (warp == 1) {
     // ================= MMA issuer =================
-    // The whole warp walks the loop and one elected lane issues: descriptors and TMEM addresses then stay in uniform registers.
-    // Under `if (lane == 0)` every operand of every MMA was moved there first, 70 cycles per instruction whatever its width
-    // (64 k-blocks of a 640-row layer: 50 -> 33 us).
-    const uint64_t desc0 = umma_desc_sw128_kmajor(smem_u32(smem) + CL_A_BYTES);
-    int s = 0, it = 0;
-    uint32_t ph = 0;
-    for (int u = blockIdx.x; u < p.units && !bw.dead; u += gridDim.x, ++it) {
-      const ClUnit g = cl_unit(p, u);
-      const int acc = it & 1;
-      bw.wait(&acc_empty[acc], ((it >> 1) & 1) ^ 1);
+    // The whole warp walks the loop and one elected lane issues: descriptors and TMEM addresses stay in uniform registers.
+    const uint64_t w_desc0 = umma_desc_sw128_kmajor(smem_u32(w_smem)), x_desc0 = umma_desc_sw128_kmajor(smem_u32(smem));
+    const uint32_t idesc = umma_idesc(128, p.cols, 0u);
+    int xs = 0, ws = 0, it = 0;
+    uint32_t xph = 0, wph = 0;
+    for (int u = u_first; u < p.units && !bw.dead; u += u_step, ++it) {
+      const int acc = p.acc_bufs > 1 ? it & 1 : 0;
+      bw.wait(&acc_empty[acc], ((p.acc_bufs > 1 ? it >> 1 : it) & 1) ^ 1);
       if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
       tc_fence_after();
-      const uint32_t d = tmem_base + acc * p.acc_cols, idesc = umma_idesc(128, g.n_cur, 2u), idesc2 = umma_idesc(128, 2 * g.n_cur, 2u);
-      for (int i = 0; i < p.ksteps; ++i) {
-        bw.wait(&full[s], ph);
-        bw.wait(&ready[s], ph);
-        if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
-        tc_fence_after();
-        const uint64_t b_hi = desc0 + static_cast<uint64_t>(s) * (stage_bytes >> 4), b_lo = b_hi + ((g.n_cur * 128) >> 4);
-        const uint32_t a_hi = a_col0 + s * 64, a_lo = a_hi + 32;
-        if (elect_one()) {
-          if (p.acc_cols != p.nt) {
-            // narrow tiles, where an instruction costs more than its columns: hi_x times both halves of the weights (they lie one
-            // behind the other) in one instruction, hi_w hi_x and lo_w hi_x in accumulators of their own: Mimi 1929 -> 1881 us, SNAC 32
-            // windows 638 -> 623, and a third off the error against 64 bits (tiles of 128 leave no TMEM for it)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              umma_tf32_ta(d, a_hi + 8 * k, b_hi + 2 * k, idesc2, (i > 0 || k > 0) ? 1u : 0u);
-              umma_tf32_ta(d, a_lo + 8 * k, b_hi + 2 * k, idesc, 1u);
-            }
-          } else
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {                      // small terms first
-            umma_tf32_ta(d, a_lo + 8 * k, b_hi + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-            umma_tf32_ta(d, a_hi + 8 * k, b_lo + 2 * k, idesc, 1u);
-            umma_tf32_ta(d, a_hi + 8 * k, b_hi + 2 * k, idesc, 1u);
-          }
-          umma_commit(&empty[s]);
-          if (i + 1 == p.ksteps) umma_commit(&acc_full[acc]);
-        }
-        __syncwarp();
-        if (++s == p.stages) { s = 0; ph ^= 1u; }
-      }
-    }
-  } else if (warp < 6) {
-    // ================= split: raw activations -> two halves in TMEM =================
-    // A stage is split as if all its values were ordinary ones, with the sum of four times the values kept beside it: that leaves the
-    // finite range for a NaN, an infinity and anything from CL_ROUND_MAX on.  Whether it did is asked once the next stage has landed and
-    // its values are on the way, when the stores have had their time as well, and only then is the stage handed to the products; one
-    // with such a value is split again first.  (The check costs 32 multiply-adds and a vote a stage.  Asked at the end of its own stage: SNAC
-    // one window 263 -> 279 us, 32 windows 628 -> 671, Mimi 1904 -> 2047; this way, the second half's low bits left to the product, which
-    // reads the upper 19 of a tf32 operand, and the second split out of line: 262, 651, 1929.)
-    const int quarter = warp & 3, row = quarter * 32 + lane;
-    const uint32_t t0 = a_col0 + (static_cast<uint32_t>(quarter * 32) << 16);
-    int s = 0, last = -1;                          // last: the stage that has been split and not handed over
-    uint32_t ph = 0;
-    float sum = 0.f;
-    auto hand_over = [&]() {
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&ready[last]);
-    };
-    for (int u = blockIdx.x; u < p.units && !bw.dead; u += gridDim.x) {
-      for (int i = 0; i < p.ksteps; ++i) {
-        bw.wait(&full[s], ph);
-        if (!__all_sync(0xffffffffu, !bw.dead && fabsf(sum) < INFINITY)) {
+      const uint32_t d = tmem_base + acc * p.acc_cols, d2 = d + p.cols;
+      for (int i = 0; i < x_steps && !bw.dead; ++i) {
+        bw.wait(&x_ready[xs], xph);
+        // parts written by threads, to be read by the tensor core.  (The fence stands here and not with the writers: there it would wait
+        // for the loads that they have on the way.)
+        if (!PARTS) fence_proxy_async();
+        for (int tap = 0; tap < p.taps; ++tap) {
+          if (!p.resident || it == 0) bw.wait(&w_full[ws], wph);
           if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
-          cl_split_again(smem + last * stage_bytes + row * 128, t0 + last * 64, row);
-        }
-        const uint8_t* src = smem + s * stage_bytes + row * 128;
-        const uint32_t t = t0 + s * 64;
-        float4 in[8];
+          tc_fence_after();
+          if (elect_one()) {
+            uint64_t w_hi = w_desc0 + static_cast<uint64_t>(ws) * (w_bytes >> 4);
+            uint64_t x_hi = x_desc0 + static_cast<uint64_t>(xs) * (x_bytes >> 4) + tap * p.dil * 8;      // a tap: the tile from a later row on
+            for (int g = 0; g < p.group; ++g) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) in[c] = *reinterpret_cast<const float4*>(src + ((c ^ (row & 7)) << 4));
-        if (last >= 0) hand_over();
-        tc_fence_after();            // the products that read this stage's columns before are behind the copy that was waited for
-        float odd[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          float hi[16], lo[16];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float4 v = in[half * 4 + c];
-            const float x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              hi[4 * c + e] = tf32_rna_below(x[e]);
-              lo[4 * c + e] = __uint_as_float(__float_as_uint(x[e] - hi[4 * c + e]) + 0x1000u);
-              odd[e] = fmaf(x[e], 4.f, odd[e]);
+              for (int k = 0; k < 2; ++k) {            // (the low parts lie 64 bytes behind the high ones)
+                const uint32_t go = (i | tap | g | k) ? 1u : 0u;
+                umma_bf16(d, w_hi + 2 * k, x_hi + 2 * k, idesc, go);
+                umma_bf16(d2, w_hi + 2 * k, x_hi + 4 + 2 * k, idesc, go);
+                umma_bf16(d2, w_hi + 4 + 2 * k, x_hi + 2 * k, idesc, 1u);
+              }
+              w_hi += CL_W_BLOCK >> 4;
+              x_hi += x_sub >> 4;
+            }
+            if (!p.resident) umma_commit(&w_empty[ws]);
+            if (tap + 1 == p.taps) {
+              umma_commit(&x_empty[xs]);
+              if (i + 1 == x_steps) umma_commit(&acc_full[acc]);
             }
           }
-          tmem_st_32x16(t + 16 * half, hi);
-          tmem_st_32x16(t + 32 + 16 * half, lo);
+          __syncwarp();
+          if (++ws == p.w_stages) { ws = 0; wph ^= 1u; }
         }
-        sum = (odd[0] + odd[1]) + (odd[2] + odd[3]);
-        last = s;
-        if (++s == p.stages) { s = 0; ph ^= 1u; }
+        if (++xs == p.x_stages) { xs = 0; xph ^= 1u; }
       }
     }
-    if (last >= 0 && !bw.dead) {
-      if (!__all_sync(0xffffffffu, fabsf(sum) < INFINITY)) cl_split_again(smem + last * stage_bytes + row * 128, t0 + last * 64, row);
-      hand_over();
+  } else if (PARTS && warp == 2) {
+    // ================= activations =================
+    if (lane == 0) {
+      const uint32_t box = static_cast<uint32_t>(p.nb * p.pitch) * 128u, dst0 = smem_u32(smem), bar0 = smem_u32(x_ready);
+      int s = 0;
+      uint32_t ph = 0;
+      pdl_wait();
+      for (int u = u_first; u < p.units && !bw.dead; u += u_step) {
+        const ClUnit g = cl_unit(p, u);
+        for (int i = kb_lo; i < kb_lo + kb_n && !bw.dead; ++i) {
+          for (int tap = 0; tap < tap_steps; ++tap) {
+            bw.wait(&x_empty[s], ph ^ 1u);
+            if (bw.dead) break;
+            const int t = g.t0 - (p.taps > 1 ? p.halo : (p.ksize - 1 - tap) * p.dil);
+            mbar_arrive_expect_tx(&x_ready[s], p.group * box);
+            for (int b = 0; b < p.group; ++b)
+              tma_load_3d(dst0 + s * x_bytes + b * x_sub, &maps.x, bar0 + 8 * s, (i * p.group + b) * 64, t, g.b0);
+            if (++s == p.x_stages) { s = 0; ph ^= 1u; }
+          }
+        }
+      }
+      if (bw.dead) {            // let the copies in flight land before the block may leave
+        const unsigned long long t0 = gtimer();
+        while (gtimer() - t0 < 2000000ull) __nanosleep(1000);
+      }
+    }
+    __syncwarp();
+  } else if (PARTS && warp == 3) {
+    // ================= codes of the rows that a unit's outputs are made of =================
+    const int cb = p.Cin >> 5, back = (p.ksize - 1) * p.dil;
+    pdl_wait();
+    int it = 0;
+    for (int u = u_first; u < p.units && !bw.dead; u += u_step, ++it) {
+      const ClUnit g = cl_unit(p, u);
+      uint32_t code = 0u;
+      const int ta = max(g.t0 - back, 0), tb = min(min(g.t0 + p.nr, p.n_hi), p.Tx);
+      for (int e = 0; e < p.nb && g.b0 + e < p.B && ta < tb; ++e) {
+        const uint8_t* base = p.x_code + ((g.b0 + e) * p.x_bstride >> 5);
+        const long long lo = static_cast<long long>(ta) * cb, hi = static_cast<long long>(tb) * cb;
+        const uintptr_t a = reinterpret_cast<uintptr_t>(base + lo), b = reinterpret_cast<uintptr_t>(base + hi), a4 = min((a + 3) & ~uintptr_t(3), b),
+                        b4 = max(b & ~uintptr_t(3), a4);
+        for (uintptr_t q = a4 + 4 * lane; q < b4; q += 128) code |= __ldcg(reinterpret_cast<const uint32_t*>(q));
+        if (a + lane < a4) code |= __ldcg(reinterpret_cast<const uint8_t*>(a + lane));
+        if (b4 + lane < b) code |= __ldcg(reinterpret_cast<const uint8_t*>(b4 + lane));
+      }
+      code = __reduce_or_sync(0xffffffffu, code);
+      code |= code >> 16;
+      code = (code | code >> 8) & 0xffu;
+      bw.wait(&top_empty[it & (CL_TOPS - 1)], ((it / CL_TOPS) & 1) ^ 1);
+      if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+      if (lane == 0) {
+        tops[(it & (CL_TOPS - 1)) * CL_SPLIT_WARPS] = __uint_as_float(code);
+        mbar_arrive(&top_full[it & (CL_TOPS - 1)]);
+      }
+      __syncwarp();
+    }
+  } else if (!PARTS && warp < 2 + CL_SPLIT_WARPS) {
+    // ================= split: global memory -> registers -> two fp16 parts in shared memory =================
+    const ClSplit sp{smem_u32(smem), x_bytes, u_first, u_step, kb_lo, x_steps, x_ready, x_empty, top_full, top_empty, tops, row_tab};
+    pdl_wait();
+    switch (p.passes) {
+      case 1: cl_split<1>(p, sp, bw); break;
+      case 2: cl_split<2>(p, sp, bw); break;
+      case 4: cl_split<4>(p, sp, bw); break;
+      case 8: cl_split<8>(p, sp, bw); break;
+      default: cl_split<16>(p, sp, bw); break;
     }
   } else {
     // ================= epilogue =================
-    // Three warps per TMEM quarter take 16-column chunks in turn.  A lane holds 16 columns of one row, so bias, activation and
-    // residual are 16 independent chains, and three warps per scheduler hide each other's loads and transposes.  Rows leave (and
-    // residuals come) through a 32 x 16 transpose: 64-byte runs per row.
-    const int quarter = warp & 3, group = (warp - 6) >> 2;
-    float* st = epi_sm + (warp - 6) * 512;
-    float4* my_row = reinterpret_cast<float4*>(st + lane * 16);
-    const int cq = lane & 3, rq = lane >> 2, sw = (lane >> 1) & 3;      // transposed side: 16-byte chunk cq of rows rq, rq + 8, ...
-    const int tq = ((cq ^ (rq >> 1)) << 2) + rq * 16;                   // (rq + 8 i swizzles as rq does)
-    const int4* tab = row_tab + quarter * 32 + rq;               // rows rq, rq + 8, ... of the quarter: tab[0], tab[8], ...
-    int it = 0, turn = group;                                    // first chunk of the unit that is this warp's
-    for (int u = blockIdx.x; u < p.units && !bw.dead; u += gridDim.x, ++it) {
+    // A lane holds one channel at eight positions, and every store and residual load of a warp is one run of 128
+    // bytes.  The four quarters of TMEM hold 128 channels, or copies of 64 or 32 that share the columns; two or three warps a
+    // quarter.
+    const int quarter = warp & 3, lane_row = quarter * 32 + lane;
+    const ClHot h{p.cols, p.N, p.epi, p.act, p.y && (p.y2 || p.yp), p.epi != CE_PLAIN, p.yp != nullptr};
+    ClBoxes bx{smem_u32(boxes) + (warp - FIRST_EPI) * 4096, &res_full[warp - FIRST_EPI], 0u, 0u};
+    int it = 0;
+    for (int u = u_first; u < p.units && !bw.dead; u += u_step, ++it) {
       const ClUnit g = cl_unit(p, u);
-      const int acc = it & 1;
-      uint32_t live = 0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int bt = tab[8 * i].x;
-        live |= ((bt >= 0 && g.b0 + (bt >> 16) < p.B && g.t0 + (bt & 0xffff) < p.n_hi) ? 1u : 0u) << i;
-      }
-      const int y0 = g.b0 * static_cast<int>(p.y_bstride) + (g.t0 - p.n_lo) * p.ldy + g.n0 + cq * 4;
-      const int r0 = g.b0 * static_cast<int>(p.r_bstride) + (g.t0 - p.n_lo) * p.ldr + g.n0 + cq * 4;
-      bool first = true;
-      float nz = 0.f;
-#pragma unroll 1
-      for (int c0 = turn << 4; c0 < g.n_cur; c0 += 48) {
-        const int n0 = g.n0 + c0, nm = n0 % p.cmod;              // 16 columns from a multiple of 16 lie in one group of channels
-        // the residual's rows are requested before the accumulator is waited for.  (Its producer is the kernel in front of this
-        // one or an earlier one: the first unit waits for it by name, later units follow accumulators that did.)
-        float4 rs[4];
-        if (p.epi != CE_PLAIN) {
-          if (it == 0 && first) pdl_wait();
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            rs[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live >> i & 1u) rs[i] = __ldcg(reinterpret_cast<const float4*>(p.resid + (r0 + c0 + tab[8 * i].z)));
-          }
-          if (p.epi == CE_NOISE) {
-            const int r = quarter * 32 + lane, bb = r / p.nr, nb = g.b0 + bb, t = g.t0 + r - bb * p.nr;
-            if (bb < p.nb && nb < p.B && t < p.n_hi) nz = __ldcg(&p.noise[static_cast<long long>(nb) * p.noise_ld + t]);
-          }
-        }
-        if (first) {
-          bw.wait(&acc_full[acc], (it >> 1) & 1);
-          if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
-          tc_fence_after();
-          first = false;
-        }
-        const uint32_t taddr = tmem_base + acc * p.acc_cols + (static_cast<uint32_t>(quarter * 32) << 16);
-        if (p.epi != CE_PLAIN) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(st + i * 128 + tq) = rs[i];
-        }
-        uint32_t tv[16];
-        tmem_ld_32x16(taddr + c0, tv);
-        tmem_ld_wait();
-        float v[16];
-#pragma unroll
-        for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(tv[c]);
-        if (p.acc_cols != p.nt) {
-          tmem_ld_32x16(taddr + g.n_cur + c0, tv);
-          tmem_ld_wait();
-#pragma unroll
-          for (int c = 0; c < 16; ++c) v[c] += __uint_as_float(tv[c]);
-        }
-        if (p.bias) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float4 q = __ldg(reinterpret_cast<const float4*>(p.bias + nm) + c);
-            v[4 * c] += q.x; v[4 * c + 1] += q.y; v[4 * c + 2] += q.z; v[4 * c + 3] += q.w;
-          }
-        }
-        if (p.epi != CE_PLAIN) {
-          __syncwarp();
-          if (p.epi == CE_SCALE_RESID) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const float4 q = __ldg(reinterpret_cast<const float4*>(p.scale + n0) + c);
-              v[4 * c] *= q.x; v[4 * c + 1] *= q.y; v[4 * c + 2] *= q.z; v[4 * c + 3] *= q.w;
-            }
-          } else if (p.epi == CE_NOISE) {
-#pragma unroll
-            for (int c = 0; c < 16; ++c) v[c] *= nz;
-          }
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float4 q = my_row[c ^ sw];
-            v[4 * c] += q.x; v[4 * c + 1] += q.y; v[4 * c + 2] += q.z; v[4 * c + 3] += q.w;
-          }
-          __syncwarp();
-        }
-        auto store = [&](float* y) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) my_row[c ^ sw] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float4 q = *reinterpret_cast<const float4*>(st + i * 128 + tq);
-            if (live >> i & 1u)
-              *reinterpret_cast<float4*>(y + (y0 + c0 + tab[8 * i].y)) = q;
-          }
-          __syncwarp();
-        };
-        if (p.y2) store(p.y);
+      const int acc = p.acc_bufs > 1 ? it & 1 : 0;
+      const uint32_t acc_ph = (p.acc_bufs > 1 ? it >> 1 : it) & 1;
+      const uint32_t taddr = tmem_base + acc * p.acc_cols + (static_cast<uint32_t>(quarter * 32) << 16);
+      const int width = min(128, p.N - g.m0), copies = cl_copies(width);        // (N is a multiple of 32)
+      const int row = copies == 1 ? lane_row : lane_row & (width - 1);
+      const bool mine = row < width;
+      // this warp's chunks of eight columns: every `turns`-th one
+      const int turn = ((warp - FIRST_EPI) >> 2) * copies + (copies == 4 ? quarter : copies == 2 ? quarter >> 1 : 0), turns = EPI_WARPS / 4 * copies;
+      ClEpiState e;
+      e.n = g.m0 + row;
+      const int nm = p.cmod == h.N ? e.n : e.n % p.cmod;
+      float inv = 0.f;
+      e.bias = e.alpha = e.ialpha = 0.f;
+      e.scale = 1.f;
+      if (mine) {
+        inv = __ldg(p.w_inv + g.m0 + lane_row);
+        if (p.bias) e.bias = __ldg(p.bias + nm);
+        if (p.epi == CE_SCALE_RESID) e.scale = __ldg(p.scale + e.n);
         if (p.act == CA_SNAKE) {
-          const float4* al = reinterpret_cast<const float4*>(p.alpha + nm);
-          const float4* ia = reinterpret_cast<const float4*>(p.alpha + p.cmod + nm);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float4 o = cl_snake4(make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]), __ldg(al + c), __ldg(ia + c));
-            v[4 * c] = o.x; v[4 * c + 1] = o.y; v[4 * c + 2] = o.z; v[4 * c + 3] = o.w;
-          }
-        } else if (p.act == CA_ELU) {
-#pragma unroll
-          for (int c = 0; c < 16; ++c) v[c] = cl_elu(v[c]);
-        } else if (p.act == CA_GELU) {
-#pragma unroll
-          for (int c = 0; c < 16; ++c) v[c] = 0.5f * v[c] * (1.f + erff(v[c] * 0.70710678118654752f));
+          e.alpha = __ldg(p.alpha + nm);
+          e.ialpha = __ldg(p.alpha + p.cmod + nm);
         }
-        store(p.y2 ? p.y2 : p.y);
       }
-      if (bw.dead) break;
-      if (first) {                    // (a warp without a chunk of this unit keeps in step with the accumulators all the same)
-        bw.wait(&acc_full[acc], (it >> 1) & 1);
-        if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+      const long long at = static_cast<long long>(g.t0 - p.n_lo) * p.N + e.n;
+      e.y = p.y ? p.y + (g.b0 * p.y_bstride + at) : nullptr;
+      e.y2 = p.y2 ? p.y2 + (g.b0 * p.y_bstride + at) : nullptr;
+      const long long block = g.b0 * p.y_bstride + (at - (e.n & 31));
+      e.yp = p.yp ? p.yp + block : nullptr;
+      e.code = p.yp_code + (block >> 5);
+      e.resid = p.resid + (g.b0 * p.r_bstride + at);
+      e.noise = p.noise + (static_cast<long long>(g.b0) * p.noise_ld + g.t0);
+      const int inside = p.nb == 1 ? min(p.nr, p.n_hi - g.t0) : 0;       // columns in front of this one are one run of rows
+      if (p.epi != CE_PLAIN && it == 0) pdl_wait();
+      bool first = true;
+      auto wait_acc = [&]() {
+        bw.wait(&top_full[it & (CL_TOPS - 1)], (it / CL_TOPS) & 1);
+        bw.wait(&acc_full[acc], acc_ph);
+        if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; return; }
+        tc_fence_after();
+        first = false;
+        bool exact;
+        if (PARTS) {
+          const uint32_t code = __float_as_uint(tops[(it & (CL_TOPS - 1)) * CL_SPLIT_WARPS]);
+          exact = (code & CB_RAW) || code == CB_QUIET;
+        } else {                                                        // (a NaN has the largest bits)
+          const float top = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(tops[(it & (CL_TOPS - 1)) * CL_SPLIT_WARPS + (lane & 7)])));
+          exact = !(top < CL_X_TOP) || (top < CL_X_LOW && top > 0.f);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&top_empty[it & (CL_TOPS - 1)]);
+        if (exact) {
+          if (mine) {
+#pragma unroll 1
+            for (int c0 = turn * CL_EC; c0 < p.cols; c0 += turns * CL_EC)
+              cl_exact_chunk(p, col_tab, g.m0, g.t0, g.b0, c0, lane_row, kb_lo * p.group, (kb_lo + kb_n) * p.group, taddr + c0,
+                             taddr + p.cols + c0);
+          }
+          inv = 1.f;
+        }
+      };
+      if (p.staged) {
+        const int c_first = turn * CL_EC, c_step = turns * CL_EC, n_box = g.m0 + (row & ~31);
+        const bool some = mine && c_first < h.cols;
+        if (some && h.res && lane == 0) {          // the first residuals, asked for before the accumulator is waited for
+          mbar_arrive_expect_tx(bx.res_full, 1024u);
+          tma_load_3d(bx.at + (bx.flip ? 1024u : 0u), &maps.r, smem_u32(bx.res_full), n_box, g.t0 - p.n_lo + c_first, g.b0);
+        }
+        wait_acc();
+        if (!bw.dead && some) {
+          switch (h.act) {
+            case CA_SNAKE: cl_boxed_chunks<CA_SNAKE>(h, maps, e, n_box, g.t0 - p.n_lo, g.b0, inside, taddr, inv, c_first, c_step, bx, bw); break;
+            case CA_ELU: cl_boxed_chunks<CA_ELU>(h, maps, e, n_box, g.t0 - p.n_lo, g.b0, inside, taddr, inv, c_first, c_step, bx, bw); break;
+            case CA_GELU: cl_boxed_chunks<CA_GELU>(h, maps, e, n_box, g.t0 - p.n_lo, g.b0, inside, taddr, inv, c_first, c_step, bx, bw); break;
+            default: cl_boxed_chunks<CA_NONE>(h, maps, e, n_box, g.t0 - p.n_lo, g.b0, inside, taddr, inv, c_first, c_step, bx, bw); break;
+          }
+        }
+        if (bw.dead) break;
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[acc]);
+      } else if (p.splits == 1) {
+        if (mine) {
+          float rs[CL_EC];
+          int c0 = turn * CL_EC;
+          if (h.res && c0 < h.cols) cl_residual(p, h, e, g, col_tab, c0, inside, rs);      // asked for before the accumulator is waited for
+#pragma unroll 1
+          for (; c0 < h.cols; c0 += turns * CL_EC) {
+            if (first) {
+              wait_acc();
+              if (bw.dead) break;
+            }
+            F2 v[CL_EC / 2];
+            cl_load_acc(taddr + c0, h.cols, inv, v);
+            cl_linear(p, h, e, g, col_tab, c0, v, rs);
+            if (h.res && c0 + turns * CL_EC < h.cols) cl_residual(p, h, e, g, col_tab, c0 + turns * CL_EC, inside, rs);
+            cl_finish(p, h, e, g, col_tab, c0, inside, v);
+          }
+          if (bw.dead) break;
+        }
+        if (first) wait_acc();          // (a warp without a chunk of this unit keeps in step with the accumulators all the same)
+        if (bw.dead) break;
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[acc]);
+      } else {
+        // this CTA's part of K into its own shared memory (its stages have been read), then every `splits`-th chunk of all parts
+        float* sums = reinterpret_cast<float*>(smem);        // [column][128]
+        wait_acc();
+        if (!bw.dead) {
+#pragma unroll 1
+          for (int c0 = turn * CL_EC; c0 < h.cols; c0 += turns * CL_EC) {
+            F2 v[CL_EC / 2];
+            cl_load_acc(taddr + c0, h.cols, inv, v);
+#pragma unroll
+            for (int c = 0; c < CL_EC / 2; ++c) {
+              const float2 x = f2_get(v[c]);
+              sums[(c0 + 2 * c) * 128 + row] = x.x;
+              sums[(c0 + 2 * c + 1) * 128 + row] = x.y;
+            }
+          }
+        }
+        cluster_sync_all();
+        if (!bw.dead && mine) {
+#pragma unroll 1
+          for (int c0 = (rank + turn * p.splits) * CL_EC; c0 < h.cols; c0 += p.splits * turns * CL_EC) {
+            float rs[CL_EC];
+            F2 v[CL_EC / 2];
+            if (h.res) cl_residual(p, h, e, g, col_tab, c0, inside, rs);
+#pragma unroll
+            for (int c = 0; c < CL_EC / 2; ++c) v[c] = f2(0.f);
+#pragma unroll 1
+            for (int k = 0; k < p.splits; ++k) {
+#pragma unroll
+              for (int c = 0; c < CL_EC / 2; ++c)
+                v[c] = f2_add(v[c], f2(ld_dsmem_f32(sums + (c0 + 2 * c) * 128 + row, k), ld_dsmem_f32(sums + (c0 + 2 * c + 1) * 128 + row, k)));
+            }
+            cl_linear(p, h, e, g, col_tab, c0, v, rs);
+            cl_finish(p, h, e, g, col_tab, c0, inside, v);
+          }
+        }
+        cluster_sync_all();
+        break;
       }
-      turn = (turn + 24 - (g.n_cur >> 4)) % 3;                   // the turns go on over the units (a 32-column tile has two chunks)
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[acc]);
     }
+    if (p.staged && lane == 0) {
+      bulk_wait_read<0>();
+      if (bw.dead) {            // a box of residuals may be on its way
+        const unsigned long long t0 = gtimer();
+        while (gtimer() - t0 < 2000000ull) __nanosleep(1000);
+      }
+    }
+    __syncwarp();
+  }
+  if (p.splits > 1 && warp < FIRST_EPI) {        // (the epilogue's two meetings of the cluster are every warp's)
+    __syncwarp();
+    cluster_sync_all();
+    cluster_sync_all();
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, p.tmem_cols);
+    tmem_dealloc(tmem_base, 512);
   }
 }
 
-// fp32 weights [N][K] (K = taps x channels, tap-major) -> [K / 32][hi | lo][n_pad][32], 128-byte rows swizzled; rows past N zero
-__global__ void __launch_bounds__(256) cl_pack_kernel(float4* __restrict__ dst, const float* __restrict__ w, int N, int K, int n_pad) {
-  const int kb = blockIdx.x;
-  for (int i = threadIdx.x + blockIdx.y * blockDim.x; i < n_pad * 8; i += blockDim.x * gridDim.y) {
-    const int r = i >> 3, c = i & 7;
-    float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
-    if (r < N) {
-      const float4 v = *reinterpret_cast<const float4*>(w + static_cast<size_t>(r) * K + kb * 32 + c * 4);
-      const float a[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        hi[e] = tf32_rna(a[e]);
-        lo[e] = tf32_rna(a[e] - hi[e]);
-      }
+// channel of a packed row: a last tile of 32 or 64 channels is repeated over its 128 rows
+__device__ __forceinline__ int cl_packed_row(int r, int N) {
+  const int m0 = r & ~127, width = min(128, N - m0);
+  return cl_copies(width) > 1 ? m0 + (r & (width - 1)) : r;
+}
+// scale of every output channel's weights: the power of two that brings the largest finite one into [2^13, 2^14)
+__global__ void __launch_bounds__(256) cl_scale_kernel(float* __restrict__ inv, const float* __restrict__ w, int N, int K) {
+  const int n = cl_packed_row(blockIdx.x, N);
+  __shared__ float sm[8];
+  float m = 0.f;
+  if (n < N) {
+    for (int k = threadIdx.x; k < K; k += 256) {
+      const float a = fabsf(w[static_cast<size_t>(n) * K + k]);
+      if (a < INFINITY) m = fmaxf(m, a);
     }
-    const size_t base = static_cast<size_t>(kb) * 2 * n_pad * 8 + static_cast<size_t>(r) * 8 + (c ^ (r & 7));
-    dst[base] = make_float4(hi[0], hi[1], hi[2], hi[3]);
-    dst[base + static_cast<size_t>(n_pad) * 8] = make_float4(lo[0], lo[1], lo[2], lo[3]);
+  }
+  m = warp_max(m);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; ++i) m = fmaxf(m, sm[i]);
+    const int e = m > 0.f ? max(ilogbf(m), -100) : 13;
+    inv[blockIdx.x] = ldexpf(1.f / CL_X_SCALE, e - 13);
+  }
+}
+
+// fp32 weights [N][K] (K = taps x channels, tap-major) -> [128 channels][K / 32][128][32 hi | 32 lo] fp16, 128-byte rows swizzled; channels past N
+// zero or (cl_packed_row) repeated
+__global__ void __launch_bounds__(256) cl_pack_kernel(uint4* __restrict__ dst, const float* __restrict__ inv, const float* __restrict__ w, int N, int K) {
+  const int blk = blockIdx.x, m = blockIdx.y, blocks = gridDim.x;
+  uint4* out = dst + (static_cast<size_t>(m) * blocks + blk) * (CL_W_BLOCK / 16);
+  for (int i = threadIdx.x; i < 128 * 4; i += 256) {
+    const int r = i >> 2, c = i & 3, n = cl_packed_row(m * 128 + r, N);
+    uint32_t hi[4] = {0u, 0u, 0u, 0u}, lo[4] = {0u, 0u, 0u, 0u};
+    if (n < N) {
+      const float s = 1.f / (inv[m * 128 + r] * CL_X_SCALE);
+      const float* src = w + static_cast<size_t>(n) * K + blk * 32 + c * 8;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) cl_parts(f2(src[2 * e], src[2 * e + 1]), s, hi[e], lo[e]);
+    }
+    out[r * 8 + (c ^ (r & 7))] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    out[r * 8 + ((c + 4) ^ (r & 7))] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
 }
 
@@ -544,7 +1170,7 @@ __global__ void __launch_bounds__(256) cl_pack_kernel(float4* __restrict__ dst, 
 // chains interleave (the activation branches once per four values, to the library's sine when an argument is out of range).
 // DW_T 128 and four-wide activations against 64 and one by one: 12 to 30 us a layer -> 4 to 14 (SNAC, 32 windows).
 constexpr int DW_T = 128;
-__global__ void __launch_bounds__(256) cl_dwconv7_kernel(float* __restrict__ y, const float* __restrict__ x, long long x_bstride,
+__global__ void __launch_bounds__(256) cl_dwconv7_kernel(float* __restrict__ y, uint8_t* __restrict__ code, const float* __restrict__ x, long long x_bstride,
                                                          const float* __restrict__ w, const float* __restrict__ bias,
                                                          const float* __restrict__ alpha_in, const float* __restrict__ alpha_out,
                                                          int C, int T, int dil, int t_lo, int t_hi) {
@@ -575,9 +1201,10 @@ __global__ void __launch_bounds__(256) cl_dwconv7_kernel(float* __restrict__ y, 
     }
   }
   __syncthreads();
-  float* yb = y + static_cast<size_t>(b) * T * C + c;
+  const size_t y0 = static_cast<size_t>(b) * T * C + c;
 #pragma unroll 2
-  for (int r = r0; r < n_out; r += 16) {
+  for (int r = r0; r < DW_T; r += 16) {
+    if (r >= n_out) break;           // (alike for the sixteen lanes of a row)
     float4 o = bv;
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
@@ -588,7 +1215,9 @@ __global__ void __launch_bounds__(256) cl_dwconv7_kernel(float* __restrict__ y, 
       o.w = fmaf(wk[k].w, v.w, o.w);
     }
     if (alpha_out) o = cl_snake4(o, ao, io);
-    *reinterpret_cast<float4*>(yb + static_cast<size_t>(t0 + r) * C) = o;
+    const size_t at = y0 + static_cast<size_t>(t0 + r) * C;
+    if (code) cl_put4(reinterpret_cast<uint32_t*>(y), code, at, o);
+    else *reinterpret_cast<float4*>(y + at) = o;
   }
 }
 
@@ -664,7 +1293,7 @@ __global__ void __launch_bounds__(256) cl_from_codes_kernel(float* __restrict__ 
 }
 
 // z0 [B][T][D] = entry of codebook 0, z1 = sum of the entries of codebooks 1 .. K - 1
-__global__ void __launch_bounds__(256) cl_codes_sum_kernel(float* __restrict__ z0, float* __restrict__ z1, const long long* __restrict__ codes,
+__global__ void __launch_bounds__(256) cl_codes_sum_kernel(float* __restrict__ z0, float* __restrict__ z1, uint8_t* __restrict__ code0, uint8_t* __restrict__ code1, const long long* __restrict__ codes,
                                                            const float* __restrict__ emb, int K, int bins, int D, int T) {
   const int t = blockIdx.x, b = blockIdx.y;
   __shared__ int row[64];
@@ -676,11 +1305,17 @@ __global__ void __launch_bounds__(256) cl_codes_sum_kernel(float* __restrict__ z
   __syncthreads();
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     const size_t o = (static_cast<size_t>(b) * T + t) * D + d;
-    z0[o] = emb[static_cast<size_t>(row[0]) * D + d];
+    const float first = emb[static_cast<size_t>(row[0]) * D + d];
     float acc = 0.f;
 #pragma unroll 8
     for (int k = 1; k < K; ++k) acc += emb[static_cast<size_t>(row[k]) * D + d];
-    z1[o] = acc;
+    if (code0) {                     // (D is a multiple of 32)
+      cl_put1(reinterpret_cast<uint32_t*>(z0), code0, o >> 5, first);
+      cl_put1(reinterpret_cast<uint32_t*>(z1), code1, o >> 5, acc);
+    } else {
+      z0[o] = first;
+      z1[o] = acc;
+    }
   }
 }
 
@@ -699,7 +1334,7 @@ __global__ void __launch_bounds__(256) cl_upsample_kernel(float* __restrict__ y,
 }
 
 // one warp per row, row kept in registers (C <= 1024, a multiple of 4)
-__global__ void __launch_bounds__(128) cl_layernorm_kernel(float* __restrict__ y, const float* __restrict__ x, const float* __restrict__ w,
+__global__ void __launch_bounds__(128) cl_layernorm_kernel(float* __restrict__ y, uint8_t* __restrict__ code, const float* __restrict__ x, const float* __restrict__ w,
                                                            const float* __restrict__ bias, int rows, int C, float eps) {
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, n4 = C >> 2;
   pdl_sync();
@@ -723,21 +1358,23 @@ __global__ void __launch_bounds__(128) cl_layernorm_kernel(float* __restrict__ y
     }
   }
   const float rstd = 1.f / sqrtf(warp_sum(sq) / static_cast<float>(C) + eps);
-  float4* yr = reinterpret_cast<float4*>(y + static_cast<size_t>(row) * C);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int c = lane + 32 * i;
-    if (c < n4) {
+    if (c < n4) {                    // (with codes: C is a multiple of 32, alike for the eight lanes of a block)
       const float4 ww = __ldg(reinterpret_cast<const float4*>(w) + c), bb = __ldg(reinterpret_cast<const float4*>(bias) + c);
-      yr[c] = make_float4((v[i].x - mean) * rstd * ww.x + bb.x, (v[i].y - mean) * rstd * ww.y + bb.y,
-                          (v[i].z - mean) * rstd * ww.z + bb.z, (v[i].w - mean) * rstd * ww.w + bb.w);
+      const float4 o = make_float4((v[i].x - mean) * rstd * ww.x + bb.x, (v[i].y - mean) * rstd * ww.y + bb.y,
+                                   (v[i].z - mean) * rstd * ww.z + bb.z, (v[i].w - mean) * rstd * ww.w + bb.w);
+      const size_t at = static_cast<size_t>(row) * C + 4 * c;
+      if (code) cl_put4(reinterpret_cast<uint32_t*>(y), code, at, o);
+      else *reinterpret_cast<float4*>(y + at) = o;
     }
   }
 }
 
 // causal attention inside one chunk of T <= 64 positions, rotary pairs (2j, 2j + 1); qkv [B][T][3 C] -> out [B][T][C].
 // One block per (head, batch entry): a chunk is a few dozen positions, so scores and weights stay in shared memory.
-__global__ void __launch_bounds__(256) cl_chunk_attention_kernel(float* __restrict__ out, const float* __restrict__ qkv, int C, int H,
+__global__ void __launch_bounds__(256) cl_chunk_attention_kernel(float* __restrict__ out, uint8_t* __restrict__ code, const float* __restrict__ qkv, int C, int H,
                                                                  int T, float max_period) {
   extern __shared__ float asm_[];      // q, k, v [T][D + 4], p [T][T + 1], frequencies
   const int h = blockIdx.x, b = blockIdx.y, D = C / H, ld = D + 4, half = D >> 1;
@@ -806,7 +1443,9 @@ __global__ void __launch_bounds__(256) cl_chunk_attention_kernel(float* __restri
     for (int d = lane; d < D; d += 32) {
       float a = 0.f;
       for (int tk = 0; tk <= tq; ++tk) a += p[tq * (T + 1) + tk] * v[tk * ld + d];
-      out[(static_cast<size_t>(b) * T + tq) * C + h * D + d] = a * inv;
+      const size_t at = (static_cast<size_t>(b) * T + tq) * C + h * D + d;
+      if (code) cl_put1(reinterpret_cast<uint32_t*>(out), code, at >> 5, a * inv);         // (D is a multiple of 32)
+      else out[at] = a * inv;
     }
     __syncwarp();
   }
@@ -835,23 +1474,194 @@ int vb_cl_timeouts(void) {
 
 long long vb_cl_pack_bytes(int N, int K) {
   if (N <= 0 || K <= 0 || N % 32 || K % 32) return -1;
-  return static_cast<long long>(N) * K * 8;
+  const long long n_pad = (static_cast<long long>(N) + 127) / 128 * 128;
+  return n_pad * K * 4 + n_pad * 4;
 }
 
 int vb_cl_pack(void* d_dst, const float* d_w, int N, int K, void* stream) {
   VB_CHECK_ARG(d_dst && d_w, "vb_cl_pack: null pointer");
   VB_CHECK_ARG(on16(d_dst) && on16(d_w), "vb_cl_pack: pointers must lie on 16-byte boundaries");
   VB_CHECK_ARG(vb_cl_pack_bytes(N, K) > 0, "vb_cl_pack: N = %d and K = %d must be positive multiples of 32", N, K);
-  cl_pack_kernel<<<dim3(K / 32, (N * 8 + 2047) / 2048), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<float4*>(d_dst), d_w, N, K, N);
+  const int m_tiles = (N + 127) / 128;
+  VB_CHECK_ARG(m_tiles <= 65535, "vb_cl_pack: N = %d", N);
+  float* inv = reinterpret_cast<float*>(static_cast<uint8_t*>(d_dst) + static_cast<long long>(m_tiles) * 128 * K * 4);
+  cl_scale_kernel<<<m_tiles * 128, 256, 0, static_cast<cudaStream_t>(stream)>>>(inv, d_w, N, K);
+  VB_CHECK_LAUNCH();
+  cl_pack_kernel<<<dim3(K / 32, m_tiles), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<uint4*>(d_dst), inv, d_w, N, K);
   VB_CHECK_LAUNCH();
   return 0;
 }
 
-int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, int Tx, const void* d_w, const float* d_bias,
-               const float* d_resid, long long r_bstride, const float* d_scale, const float* d_noise, int noise_ld,
-               const float* d_alpha, int epilogue, int act, int B, int Cin, int N, int cmod, int ksize, int dil, int n_lo, int n_hi,
-               long long y_bstride, void* stream) {
-  VB_CHECK_ARG(d_y && d_x && d_w, "vb_cl_conv: null pointer");
+}  // extern "C"
+
+namespace vb {
+// Long sums of narrow layers are one chain of products on few CTAs: 640 rows of 512 x 2048 23.3 us in one part, 15.7 in two, 12.9 in four; 1024 x 3584
+// 33.9, 26.0, 23.6.  Shorter sums and wider layers lose (5120 rows of 256 x 1536 20.6 -> 27.9, 640 of 4096 x 2048 38.8 -> 60.6).
+static int cl_splits(int blocks, int m_tiles, int kb) {
+  return blocks >= 64 && m_tiles <= 8 ? min(4, kb) : 1;
+}
+// How a launch is divided: columns of a tile, whether a stage of activations serves all taps, boxes for the results.  The fields of p that describe
+// the problem are set.  Costs in cycles, per 64 channels and tap: the MMAs' 6 a column; the bytes through L2, some 45 a cycle and SM (32 KB of
+// weights, 256 bytes a row of activations, once per stage); the bytes through shared memory, 128 a cycle (the MMAs read 12 times 4 KB of
+// weights and 32 bytes a column); a turn of the ring of weights.
+template <bool PARTS>
+static void cl_plan(ClConvParams& p, int sms) {
+  static const int kCols[] = {240, 224, 208, 192, 176, 160, 144, 128, 112, 96, 80, 64, 48, 32, 16};
+  const int range = p.n_hi - p.n_lo, blocks = p.Cin / 32;
+  p.m_tiles = (p.N + 127) / 128;
+  p.group = blocks % 2 ? 1 : 2;
+  p.kb = blocks / p.group;
+  // Parts of K: by the layer alone, not by the number of positions, so that a result's sum has one order whatever its batch.
+  p.splits = cl_splits(p.kb * p.ksize * p.group, p.m_tiles, p.kb);
+  const bool two = p.y && (p.y2 || p.yp);
+  double best = -1.0;
+  for (int per_tap = 0; per_tap < 2; ++per_tap) {
+    const long long back = static_cast<long long>(p.ksize - 1) * p.dil;
+    if (per_tap == 0 && (p.ksize == 1 || back > 64)) continue;
+    const int halo = per_tap ? 0 : static_cast<int>(back), taps = per_tap ? 1 : p.ksize;
+    for (int cand : kCols) {
+      int nr, nb;
+      if (range >= cand) {
+        nr = cand; nb = 1;
+      } else {
+        nr = range;
+        nb = max(min((cand + halo) / (nr + halo), p.B), 1);
+      }
+      const int pitch = nr + halo, cols = (nb * pitch - halo + 15) / 16 * 16, rows = cols + halo;
+      if (cols > 240 || rows > CL_ROWS) continue;
+      const int t_tiles = (range + nr - 1) / nr;
+      const long long units = static_cast<long long>(p.m_tiles) * t_tiles * ((p.B + nb - 1) / nb);
+      if (units > 0x7fffffffLL) continue;
+      const int pass = PARTS ? 8 : 32 / p.group, rows_pad = (rows + pass - 1) / pass * pass, x_bytes = p.group * rows_pad * 128,
+                w_bytes = p.group * CL_W_BLOCK, area = VB_MAX_DYN_SMEM - CL_TAIL;
+      for (int staged = 0; staged < 2; ++staged) {
+        if (staged && (nb != 1 || p.splits > 1 || (two && p.epi != CE_PLAIN))) continue;
+        const int s = p.splits, steps = (p.kb + s - 1) / s * p.ksize, room = area - (staged ? ClRoles<PARTS>::EPI_WARPS * 4096 : 0);
+        const bool resident = s == 1 && units > sms && p.m_tiles <= sms && steps <= CL_W_STAGES && steps * w_bytes + 2 * x_bytes <= room;
+        int xs = 2, ws = steps;
+        if (!resident) {
+          if (taps == 1 && 3 * x_bytes + 3 * w_bytes <= room) xs = 3;
+          ws = min(CL_W_STAGES, (room - xs * x_bytes) / w_bytes);
+          if (ws < 2) continue;
+        }
+        while (xs < CL_X_STAGES && (xs + 1) * x_bytes + ws * w_bytes <= room) ++xs;
+        if (s > 1 && (units * s > 0x7fffffffLL || xs * x_bytes + ws * w_bytes < cols * 512)) continue;
+        const long long grid = s > 1 ? units * s : resident ? sms / p.m_tiles * p.m_tiles : min(units, static_cast<long long>(sms));
+        const double share = p.group / 2.0, wl = resident ? 0.0 : 32768.0, xl = 256.0 * rows / taps;
+        const double stage = fmax(fmax(fmax(6.0 * cols, (wl + xl) / 45), (12 * (4096 + 32.0 * cols) + wl + xl) / 128) * share, resident ? 100.0 : 2400.0 / ws);
+        const double epi = 1000 + (staged ? 16.0 : 24.0) * cols * (two ? 1.4 : 1.0) * (p.epi != CE_PLAIN ? 1.2 : 1.0), main = stage * steps + 300;
+        double cost;
+        if (s > 1) cost = static_cast<double>((units * s + sms - 1) / sms) * (main + epi + 5000);
+        else cost = static_cast<double>((units + grid - 1) / grid) * (4 * cols <= 512 ? fmax(main, epi) : main + epi) + epi;
+        if (best < 0.0 || cost < best) {
+          best = cost;
+          p.taps = taps; p.halo = halo; p.nr = nr; p.nb = nb; p.pitch = pitch; p.cols = cols; p.rows_pad = rows_pad; p.resident = resident;
+          p.t_tiles = t_tiles; p.units = static_cast<int>(units); p.x_stages = xs; p.w_stages = ws; p.grid = static_cast<int>(grid); p.staged = staged;
+        }
+      }
+    }
+  }
+  const int rows_pass = 32 / p.group, passes = (p.cols + p.halo + rows_pass - 1) / rows_pass;
+  p.passes = passes > 8 ? 16 : passes > 4 || (p.taps == 1 && p.ksize > 1) ? 8 : passes > 2 ? 4 : passes;
+  p.m_tiles_inv = p.m_tiles > 1 ? static_cast<uint32_t>(((1ULL << 32) + p.m_tiles - 1) / p.m_tiles) : 0u;
+  p.t_tiles_inv = p.t_tiles > 1 ? static_cast<uint32_t>(((1ULL << 32) + p.t_tiles - 1) / p.t_tiles) : 0u;
+  p.acc_cols = 2 * p.cols;
+  p.acc_bufs = 2 * p.acc_cols <= 512 ? 2 : 1;
+}
+
+// boxes of 8 x 32 words of an fp32 (or parts) tensor [B][rows][N]
+static bool cl_box_map(CUtensorMap* map, const void* base, int N, int rows, int B, long long bstride) {
+  cuuint64_t dims[3] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(B)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(N) * 4, static_cast<cuuint64_t>(bstride) * 4};
+  cuuint32_t box[3] = {32, CL_EC, 1}, estr[3] = {1, 1, 1};
+  return encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <bool PARTS>
+static int cl_launch(ClConvParams p, cudaStream_t stream) {
+  cl_plan<PARTS>(p, cl_sms());
+  VB_CHECK_ARG(p.units > 0, "vb_cl_conv: too many tiles");
+  ClMaps maps = {};
+  VB_CHECK_ARG((!PARTS && !p.staged) || encode_fn(), "cuTensorMapEncodeTiled not available (no CUDA driver?)");
+  if (PARTS) {
+    cuuint64_t dims[3] = {static_cast<cuuint64_t>(p.Cin) * 2, static_cast<cuuint64_t>(p.Tx), static_cast<cuuint64_t>(p.B)};
+    cuuint64_t strides[2] = {static_cast<cuuint64_t>(p.Cin) * 4, static_cast<cuuint64_t>(p.x_bstride) * 4};
+    cuuint32_t box[3] = {64, static_cast<cuuint32_t>(p.pitch), static_cast<cuuint32_t>(p.nb)}, estr[3] = {1, 1, 1};
+    const CUresult r = encode_fn()(&maps.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<float*>(p.x), dims, strides, box, estr,
+                                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    VB_CHECK_ARG(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(channels last) failed: CUresult %d", static_cast<int>(r));
+  }
+  if (p.staged) {          // (rows of the results count from n_lo; what a box has past the last one is not written)
+    const int rows = p.n_hi - p.n_lo;
+    VB_CHECK_ARG((!p.y || cl_box_map(&maps.y, p.y, p.N, rows, p.B, p.y_bstride)) &&
+                     cl_box_map(&maps.last, p.y2 ? static_cast<void*>(p.y2) : p.yp ? static_cast<void*>(p.yp) : p.y, p.N, rows, p.B, p.y_bstride) &&
+                     (!p.resid || cl_box_map(&maps.r, p.resid, p.N, rows, p.B, p.r_bstride)),
+                 "cuTensorMapEncodeTiled(channels last, results) failed");
+  }
+  const int smem = p.x_stages * p.group * p.rows_pad * 128 + p.w_stages * p.group * CL_W_BLOCK + (p.staged ? ClRoles<PARTS>::EPI_WARPS * 4096 : 0) + CL_TAIL;
+  VB_CHECK_CUDA(max_dyn_smem_once(cl_conv_kernel<PARTS>));
+  VB_CHECK_CUDA(launch_kernel_cluster(cl_conv_kernel<PARTS>, dim3(p.grid), dim3(ClRoles<PARTS>::THREADS), smem, stream, true, p.splits, p, maps));
+  return 0;
+}
+
+// rows [n_lo, n_hi) of p's outputs, which point to the first of them
+static int cl_run(const ClConvParams& q, cudaStream_t stream) {
+  ClConvParams p = q;
+  // the epilogue addresses rows with 32-bit offsets from the first one: what is beyond that runs in several launches
+  const long long per_entry = max(max(p.y_bstride, p.r_bstride), p.x_bstride);
+  const int max_b = per_entry >= (1LL << 30) ? 1 : static_cast<int>(((1LL << 31) - 1) / max(per_entry, 1LL)) - 1;
+  const long long max_rows = max((1LL << 30) / p.N / 128 * 128, 128LL);
+  auto part = [&](int b0, int b, long long t, long long t1) {
+    ClConvParams r = p;
+    r.x += b0 * p.x_bstride;
+    if (p.x_code) r.x_code += b0 * p.x_bstride >> 5;
+    const long long at = b0 * p.y_bstride + (t - p.n_lo) * p.N;
+    if (p.y) r.y += at;
+    if (p.y2) r.y2 += at;
+    if (p.yp) r.yp += at, r.yp_code += at >> 5;
+    if (p.resid) r.resid += b0 * p.r_bstride + (t - p.n_lo) * p.N;
+    if (p.noise) r.noise += static_cast<long long>(b0) * p.noise_ld;
+    r.B = b;
+    r.n_lo = static_cast<int>(t);
+    r.n_hi = static_cast<int>(t1);
+    return cl_run(r, stream);
+  };
+  if (p.B > max_b) {
+    for (int b0 = 0; b0 < p.B; b0 += max_b) {
+      const int rc = part(b0, min(max_b, p.B - b0), p.n_lo, p.n_hi);
+      if (rc != 0) return rc;
+    }
+    return 0;
+  }
+  if (p.n_hi - p.n_lo > max_rows) {
+    for (long long t = p.n_lo; t < p.n_hi; t += max_rows) {
+      const int rc = part(0, p.B, t, min(t + max_rows, static_cast<long long>(p.n_hi)));
+      if (rc != 0) return rc;
+    }
+    return 0;
+  }
+  // dense rows without taps are one sequence, whatever entry they belong to
+  if (p.ksize == 1 && p.B > 1 && p.n_lo == 0 && p.n_hi == p.Tx && p.x_bstride == static_cast<long long>(p.Tx) * p.Cin &&
+      p.y_bstride == static_cast<long long>(p.Tx) * p.N && (!p.resid || p.r_bstride == p.y_bstride) && (!p.noise || p.noise_ld == p.Tx) &&
+      static_cast<long long>(p.B) * p.Tx * max(p.N, p.Cin) < (1LL << 30)) {
+    p.n_hi = p.Tx = p.B * p.Tx;
+    p.B = 1;
+  }
+  return p.x_code ? cl_launch<true>(p, stream) : cl_launch<false>(p, stream);
+}
+}  // namespace vb
+
+extern "C" {
+
+int vb_cl_conv_parts(float* d_y, float* d_y2, void* d_yp, void* d_yp_code, const void* d_x, const void* d_x_code, long long x_bstride, int Tx,
+                     const void* d_w, const float* d_bias, const float* d_resid, long long r_bstride, const float* d_scale, const float* d_noise,
+                     int noise_ld, const float* d_alpha, int epilogue, int act, int B, int Cin, int N, int cmod, int ksize, int dil, int n_lo,
+                     int n_hi, long long y_bstride, void* stream) {
+  VB_CHECK_ARG((d_y || d_yp) && d_x && d_w, "vb_cl_conv: null pointer");
+  VB_CHECK_ARG(!d_y2 || (d_y && !d_yp), "vb_cl_conv: activated values as fp32 or as parts");
+  VB_CHECK_ARG(!d_yp == !d_yp_code, "vb_cl_conv: parts come with their codes");
   VB_CHECK_ARG(Cin > 0 && Cin % 32 == 0 && N > 0 && N % 32 == 0, "vb_cl_conv: Cin = %d and N = %d must be positive multiples of 32", Cin, N);
   VB_CHECK_ARG(cmod > 0 && cmod % 32 == 0 && N % cmod == 0, "vb_cl_conv: %d columns do not divide into groups of %d channels", N, cmod);
   VB_CHECK_ARG(ksize >= 1 && dil >= 1 && Tx > 0 && n_lo >= 0, "vb_cl_conv: ksize %d, dilation %d, %d positions, rows from %d", ksize, dil, Tx, n_lo);
@@ -860,85 +1670,38 @@ int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, i
   VB_CHECK_ARG(epilogue != CE_SCALE_RESID || d_scale, "vb_cl_conv: the scaled residual needs d_scale");
   VB_CHECK_ARG(epilogue != CE_NOISE || d_noise, "vb_cl_conv: the noise epilogue needs d_noise");
   VB_CHECK_ARG(act != CA_SNAKE || d_alpha, "vb_cl_conv: Snake needs d_alpha");
-  VB_CHECK_ARG(on16(d_x) && x_bstride % 4 == 0 && on16(d_y) && on16(d_y2) && y_bstride % 4 == 0 && on16(d_resid) && (!d_resid || r_bstride % 4 == 0),
+  VB_CHECK_ARG(on16(d_x) && x_bstride % 4 == 0 && on16(d_y) && on16(d_y2) && on16(d_yp) && y_bstride % 4 == 0 && on16(d_resid) &&
+                   (!d_resid || r_bstride % 4 == 0),
                "vb_cl_conv: rows must start on 16-byte boundaries");
   VB_CHECK_ARG(on16(d_w) && on16(d_bias) && on16(d_scale) && on16(d_alpha), "vb_cl_conv: weights, bias, scale and alpha must lie on 16-byte boundaries");
-  if (B <= 0 || n_lo >= n_hi) return 0;
-  // the epilogue addresses rows with 32-bit offsets from the first one: what is beyond that runs in several launches
-  const long long per_entry = max(y_bstride, r_bstride);
-  const int max_b = per_entry >= (1LL << 30) ? 1 : static_cast<int>(((1LL << 31) - 1) / max(per_entry, 1LL)) - 1;
-  if (B > max_b) {
-    for (int b0 = 0; b0 < B; b0 += max_b) {
-      const int rc = vb_cl_conv(d_y + b0 * y_bstride, d_y2 ? d_y2 + b0 * y_bstride : nullptr, d_x + b0 * x_bstride, x_bstride, Tx, d_w, d_bias,
-                                d_resid ? d_resid + b0 * r_bstride : nullptr, r_bstride, d_scale,
-                                d_noise ? d_noise + static_cast<long long>(b0) * noise_ld : nullptr, noise_ld, d_alpha, epilogue, act,
-                                min(max_b, B - b0), Cin, N, cmod, ksize, dil, n_lo, n_hi, y_bstride, stream);
-      if (rc != 0) return rc;
-    }
-    return 0;
-  }
-  const long long max_rows = max((1LL << 30) / N / 128 * 128, 128LL);
-  if (n_hi - n_lo > max_rows) {
-    for (long long t = n_lo; t < n_hi; t += max_rows) {
-      const int rc = vb_cl_conv(d_y, d_y2, d_x, x_bstride, Tx, d_w, d_bias, d_resid, r_bstride, d_scale, d_noise, noise_ld, d_alpha, epilogue, act,
-                                B, Cin, N, cmod, ksize, dil, static_cast<int>(t), static_cast<int>(min(t + max_rows, static_cast<long long>(n_hi))),
-                                y_bstride, stream);
-      if (rc != 0) return rc;
-    }
-    return 0;
-  }
+  VB_CHECK_ARG((!d_x_code || x_bstride % 32 == 0) && (!d_yp || y_bstride % 32 == 0), "vb_cl_conv: entries of parts must lie multiples of 32 apart");
   VB_CHECK_ARG(N <= (1 << 22), "vb_cl_conv: %d columns", N);
-  auto fn = encode_fn();
-  VB_CHECK_ARG(fn, "cuTensorMapEncodeTiled not available (no CUDA driver?)");
+  if (B <= 0 || n_lo >= n_hi) return 0;
   ClConvParams p = {};
   VB_CHECK_ARG(p.wait_flag = wait_flag(WK_CL_CONV), "vb_cl_conv: no mapped host memory");
-  const int range = n_hi - n_lo;
-  p.nr = min(range, 128);
-  p.nb = min(B, 128 / p.nr);
-  p.t_tiles = (range + p.nr - 1) / p.nr;
-  const long long m_tiles = static_cast<long long>(p.t_tiles) * ((B + p.nb - 1) / p.nb);
-  p.kb_per_tap = Cin / 32;
-  p.ksteps = p.kb_per_tap * ksize;
-  // width of a column tile: rounds of units times what a unit costs -- a stage takes the products' 6 cycles a column or the
-  // split's 320, whichever is longer, the epilogue about 1000 plus 24 a column where nothing overlaps it
-  const int sms = cl_sms();
-  long long best = -1;
-  for (int nt = 128; nt >= 32; nt >>= 1) {
-    if (nt > N && nt > 32) continue;
-    const long long units = m_tiles * ((N + nt - 1) / nt), rounds = (units + sms - 1) / sms;
-    const long long stage = max(6 * nt, 320), unit = max(stage * p.ksteps, 500LL + 24 * nt);
-    const long long cost = rounds * unit + 1000 + 24 * nt;
-    if (best < 0 || cost < best) { best = cost; p.nt = nt; p.units = static_cast<int>(units); }
-  }
-  VB_CHECK_ARG(m_tiles * ((N + p.nt - 1) / p.nt) < 0x7fffffffLL, "vb_cl_conv: too many tiles");
-  p.n_tiles = (N + p.nt - 1) / p.nt;
+  const long long first = static_cast<long long>(n_lo) * N, n_pad = (N + 127LL) / 128 * 128;
   p.w = static_cast<const uint8_t*>(d_w);
-  const long long first = static_cast<long long>(n_lo) * N;
-  p.y = d_y + first; p.y2 = d_y2 ? d_y2 + first : nullptr; p.bias = d_bias; p.resid = d_resid ? d_resid + first : nullptr; p.scale = d_scale; p.noise = d_noise; p.alpha = d_alpha;
-  p.y_bstride = y_bstride; p.r_bstride = r_bstride; p.ldy = N; p.ldr = N; p.noise_ld = noise_ld; p.cmod = cmod;
-  p.epi = epilogue; p.act = act; p.B = B; p.n_lo = n_lo; p.n_hi = n_hi; p.ksize = ksize; p.dil = dil; p.N = N; p.n_pad = N;
-  const int stage_bytes = CL_A_BYTES + p.nt * 256, tail = CL_EPI_BYTES + 512 /*barriers*/ + 2048 /*row table*/ + 1024 /*alignment*/;
-  p.acc_cols = p.nt <= 64 ? 2 * p.nt : p.nt;
-  p.stages = min(min(CL_MAX_STAGES, (512 - 2 * p.acc_cols) / 64), (VB_MAX_DYN_SMEM - tail) / stage_bytes);
-  p.tmem_cols = 512;
-  CUtensorMap map;
-  {
-    cuuint64_t dims[3] = {static_cast<cuuint64_t>(Cin), static_cast<cuuint64_t>(Tx), static_cast<cuuint64_t>(B)};
-    cuuint64_t strides[2] = {static_cast<cuuint64_t>(Cin) * 4, static_cast<cuuint64_t>(x_bstride) * 4};
-    cuuint32_t box[3] = {32, static_cast<cuuint32_t>(p.nr), static_cast<cuuint32_t>(p.nb)}, estr[3] = {1, 1, 1};
-    const CUresult r = fn(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(d_x), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    VB_CHECK_ARG(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(channels last) failed: CUresult %d", static_cast<int>(r));
-  }
-  VB_CHECK_CUDA(max_dyn_smem_once(cl_conv_kernel));
-  const int smem = p.stages * stage_bytes + tail;
-  VB_CHECK_CUDA(launch_kernel(cl_conv_kernel, dim3(min(p.units, sms)), dim3(CL_THREADS), smem, static_cast<cudaStream_t>(stream), true, p, map));
-  return 0;
+  p.w_inv = reinterpret_cast<const float*>(p.w + n_pad * Cin * ksize * 4);
+  p.x = static_cast<const float*>(d_x); p.x_code = static_cast<const uint8_t*>(d_x_code);
+  p.y = d_y ? d_y + first : nullptr; p.y2 = d_y2 ? d_y2 + first : nullptr;
+  p.yp = d_yp ? static_cast<uint32_t*>(d_yp) + first : nullptr; p.yp_code = d_yp ? static_cast<uint8_t*>(d_yp_code) + (first >> 5) : nullptr;
+  p.bias = d_bias; p.resid = epilogue != CE_PLAIN ? d_resid + first : nullptr; p.scale = d_scale; p.noise = epilogue == CE_NOISE ? d_noise : nullptr;
+  p.alpha = d_alpha; p.x_bstride = x_bstride; p.y_bstride = y_bstride; p.r_bstride = p.resid ? r_bstride : 0; p.noise_ld = noise_ld;
+  p.cmod = cmod; p.epi = epilogue; p.act = act; p.B = B; p.Tx = Tx; p.Cin = Cin; p.N = N; p.n_lo = n_lo; p.n_hi = n_hi; p.ksize = ksize; p.dil = dil;
+  return cl_run(p, static_cast<cudaStream_t>(stream));
 }
 
-int vb_cl_dwconv7(float* d_y, const float* d_x, long long x_bstride, const float* d_w, const float* d_bias, const float* d_alpha_in,
-                  const float* d_alpha_out, int B, int C, int T, int dilation, int t_lo, int t_hi, void* stream) {
+int vb_cl_conv(float* d_y, float* d_y2, const float* d_x, long long x_bstride, int Tx, const void* d_w, const float* d_bias,
+               const float* d_resid, long long r_bstride, const float* d_scale, const float* d_noise, int noise_ld,
+               const float* d_alpha, int epilogue, int act, int B, int Cin, int N, int cmod, int ksize, int dil, int n_lo, int n_hi,
+               long long y_bstride, void* stream) {
+  VB_CHECK_ARG(d_y, "vb_cl_conv: null pointer");
+  return vb_cl_conv_parts(d_y, d_y2, nullptr, nullptr, d_x, nullptr, x_bstride, Tx, d_w, d_bias, d_resid, r_bstride, d_scale, d_noise, noise_ld,
+                          d_alpha, epilogue, act, B, Cin, N, cmod, ksize, dil, n_lo, n_hi, y_bstride, stream);
+}
+
+int vb_cl_dwconv7_parts(float* d_y, void* d_code, const float* d_x, long long x_bstride, const float* d_w, const float* d_bias,
+                        const float* d_alpha_in, const float* d_alpha_out, int B, int C, int T, int dilation, int t_lo, int t_hi, void* stream) {
   VB_CHECK_ARG(d_y && d_x && d_w, "vb_cl_dwconv7: null pointer");
   VB_CHECK_ARG(C % 64 == 0 && dilation >= 1 && dilation <= 64 && x_bstride % 4 == 0, "vb_cl_dwconv7: C = %d (a multiple of 64), dilation %d", C, dilation);
   VB_CHECK_ARG(on16(d_y) && on16(d_x) && on16(d_w) && on16(d_bias) && on16(d_alpha_in) && on16(d_alpha_out), "vb_cl_dwconv7: pointers must lie on 16-byte boundaries");
@@ -946,8 +1709,12 @@ int vb_cl_dwconv7(float* d_y, const float* d_x, long long x_bstride, const float
   if (B <= 0 || t_lo == t_hi) return 0;
   VB_CHECK_CUDA(max_dyn_smem_once(cl_dwconv7_kernel));
   VB_LAUNCH_PDL(cl_dwconv7_kernel, dim3((t_hi - t_lo + DW_T - 1) / DW_T, C / 64, B), 256, static_cast<size_t>(DW_T + 6 * dilation) * 256, stream,
-                d_y, d_x, x_bstride, d_w, d_bias, d_alpha_in, d_alpha_out, C, T, dilation, t_lo, t_hi);
+                d_y, static_cast<uint8_t*>(d_code), d_x, x_bstride, d_w, d_bias, d_alpha_in, d_alpha_out, C, T, dilation, t_lo, t_hi);
   return 0;
+}
+int vb_cl_dwconv7(float* d_y, const float* d_x, long long x_bstride, const float* d_w, const float* d_bias, const float* d_alpha_in,
+                  const float* d_alpha_out, int B, int C, int T, int dilation, int t_lo, int t_hi, void* stream) {
+  return vb_cl_dwconv7_parts(d_y, nullptr, d_x, x_bstride, d_w, d_bias, d_alpha_in, d_alpha_out, B, C, T, dilation, t_lo, t_hi, stream);
 }
 
 int vb_cl_last_conv(float* d_y, const float* d_x, long long x_bstride, const float* d_w, const float* d_bias, int B, int C, int T,
@@ -975,12 +1742,18 @@ int vb_cl_from_codes(float* d_z, const int32_t* d_codes0, const int32_t* d_codes
   return 0;
 }
 
-int vb_cl_codes_sum(float* d_z0, float* d_z1, const int64_t* d_codes, const float* d_emb, int B, int K, int bins, int D, int T, void* stream) {
+int vb_cl_codes_sum_parts(float* d_z0, float* d_z1, void* d_code0, void* d_code1, const int64_t* d_codes, const float* d_emb, int B, int K, int bins,
+                          int D, int T, void* stream) {
   VB_CHECK_ARG(d_z0 && d_z1 && d_codes && d_emb, "vb_cl_codes_sum: null pointer");
   VB_CHECK_ARG(K >= 1 && K <= 64, "vb_cl_codes_sum: %d codebooks", K);
+  VB_CHECK_ARG(!d_code0 == !d_code1 && (!d_code0 || D % 32 == 0), "vb_cl_codes_sum: parts need both codes and D = %d a multiple of 32", D);
   if (B <= 0 || T <= 0) return 0;
-  VB_LAUNCH_PDL(cl_codes_sum_kernel, dim3(T, B), 256, 0, stream, d_z0, d_z1, reinterpret_cast<const long long*>(d_codes), d_emb, K, bins, D, T);
+  VB_LAUNCH_PDL(cl_codes_sum_kernel, dim3(T, B), 256, 0, stream, d_z0, d_z1, static_cast<uint8_t*>(d_code0), static_cast<uint8_t*>(d_code1),
+                reinterpret_cast<const long long*>(d_codes), d_emb, K, bins, D, T);
   return 0;
+}
+int vb_cl_codes_sum(float* d_z0, float* d_z1, const int64_t* d_codes, const float* d_emb, int B, int K, int bins, int D, int T, void* stream) {
+  return vb_cl_codes_sum_parts(d_z0, d_z1, nullptr, nullptr, d_codes, d_emb, B, K, bins, D, T, stream);
 }
 
 int vb_cl_upsample(float* d_y, const float* d_x, const float* d_w, int B, int C, int T, int stride, void* stream) {
@@ -990,25 +1763,33 @@ int vb_cl_upsample(float* d_y, const float* d_x, const float* d_w, int B, int C,
   return 0;
 }
 
-int vb_cl_layernorm(float* d_y, const float* d_x, const float* d_w, const float* d_b, int rows, int C, float eps, void* stream) {
+int vb_cl_layernorm_parts(float* d_y, void* d_code, const float* d_x, const float* d_w, const float* d_b, int rows, int C, float eps, void* stream) {
   VB_CHECK_ARG(d_y && d_x && d_w && d_b, "vb_cl_layernorm: null pointer");
   VB_CHECK_ARG(on16(d_y) && on16(d_x) && on16(d_w) && on16(d_b), "vb_cl_layernorm: pointers must lie on 16-byte boundaries");
   VB_CHECK_ARG(C > 0 && C % 4 == 0 && C <= 1024, "vb_cl_layernorm: C = %d (a multiple of 4, <= 1024)", C);
+  VB_CHECK_ARG(!d_code || C % 32 == 0, "vb_cl_layernorm: parts need C = %d to be a multiple of 32", C);
   if (rows <= 0) return 0;
-  VB_LAUNCH_PDL(cl_layernorm_kernel, (rows + 3) / 4, 128, 0, stream, d_y, d_x, d_w, d_b, rows, C, eps);
+  VB_LAUNCH_PDL(cl_layernorm_kernel, (rows + 3) / 4, 128, 0, stream, d_y, static_cast<uint8_t*>(d_code), d_x, d_w, d_b, rows, C, eps);
   return 0;
 }
+int vb_cl_layernorm(float* d_y, const float* d_x, const float* d_w, const float* d_b, int rows, int C, float eps, void* stream) {
+  return vb_cl_layernorm_parts(d_y, nullptr, d_x, d_w, d_b, rows, C, eps, stream);
+}
 
-int vb_cl_chunk_attention(float* d_out, const float* d_qkv, int B, int C, int H, int T, float max_period, void* stream) {
+int vb_cl_chunk_attention_parts(float* d_out, void* d_code, const float* d_qkv, int B, int C, int H, int T, float max_period, void* stream) {
   VB_CHECK_ARG(d_out && d_qkv, "vb_cl_chunk_attention: null pointer");
   VB_CHECK_ARG(reinterpret_cast<uintptr_t>(d_qkv) % 8 == 0, "vb_cl_chunk_attention: rows must start on 8-byte boundaries");
   VB_CHECK_ARG(H >= 1 && C % H == 0 && (C / H) % 4 == 0 && C / H <= 256 && T >= 1 && T <= 64, "vb_cl_chunk_attention: C %d, H %d, T %d (<= 64)", C, H, T);
+  VB_CHECK_ARG(!d_code || (C / H) % 32 == 0, "vb_cl_chunk_attention: parts need heads of a multiple of 32, not %d", C / H);
   if (B <= 0) return 0;
   const size_t smem = (static_cast<size_t>(3) * T * (C / H + 4) + static_cast<size_t>(T) * (T + 1) + C / H / 2) * sizeof(float);
   VB_CHECK_ARG(smem <= VB_MAX_DYN_SMEM, "vb_cl_chunk_attention: head size %d too large", C / H);
   VB_CHECK_CUDA(max_dyn_smem_once(cl_chunk_attention_kernel));
-  VB_LAUNCH_PDL(cl_chunk_attention_kernel, dim3(H, B), 256, smem, stream, d_out, d_qkv, C, H, T, max_period);
+  VB_LAUNCH_PDL(cl_chunk_attention_kernel, dim3(H, B), 256, smem, stream, d_out, static_cast<uint8_t*>(d_code), d_qkv, C, H, T, max_period);
   return 0;
+}
+int vb_cl_chunk_attention(float* d_out, const float* d_qkv, int B, int C, int H, int T, float max_period, void* stream) {
+  return vb_cl_chunk_attention_parts(d_out, nullptr, d_qkv, B, C, H, T, max_period, stream);
 }
 
 }  // extern "C"

@@ -1,5 +1,5 @@
 """Vocoder convolutions over channels-last activations [B, T, C] (csrc/cl_conv.cu), shared by the SNAC and Mimi decoders: layers
-whose widths are multiples of 32 channels run as one product per tap on tcgen05 (tf32 halves, fp32 accumulation)."""
+whose widths are multiples of 32 channels run as one product per tap on tcgen05 (two fp16 parts a value, fp32 accumulation)."""
 from __future__ import annotations
 
 from typing import Optional
@@ -7,7 +7,7 @@ from typing import Optional
 import torch
 
 from .. import _lib, ops
-from .._lib import call
+from .._lib import VoxB200Error, call
 
 EPI = {"plain": 0, "resid": 1, "scale_resid": 2, "noise": 3}
 ACT = {None: 0, "snake": 1, "elu": 2, "gelu": 3}
@@ -34,23 +34,32 @@ def pack_convtr(wp: torch.Tensor) -> torch.Tensor:
 
 
 class Act:
-    """An activation [B, T, C] inside a buffer: entry b starts at offset + b * bstride floats."""
-    __slots__ = ("buf", "B", "T", "C", "offset", "bstride")
+    """An activation [B, T, C] inside a buffer: entry b starts at offset + b * bstride floats.  ``parts``: kept as what the convolutions
+    multiply, two fp16 parts a value in the place of a float, with a code byte per 32 channels behind them (written by the kernels
+    that produce them, read by ``conv`` and ``conv_transposed`` only)."""
+    __slots__ = ("buf", "B", "T", "C", "offset", "bstride", "parts")
 
-    def __init__(self, buf: torch.Tensor, B: int, T: int, C: int, offset: int = 0, bstride: Optional[int] = None):
-        self.buf, self.B, self.T, self.C, self.offset = buf, B, T, C, offset
+    def __init__(self, buf: torch.Tensor, B: int, T: int, C: int, offset: int = 0, bstride: Optional[int] = None, parts: bool = False):
+        self.buf, self.B, self.T, self.C, self.offset, self.parts = buf, B, T, C, offset, parts
         self.bstride = T * C if bstride is None else bstride
 
     @classmethod
-    def empty(cls, B: int, T: int, C: int, device) -> "Act":
-        return cls(torch.empty(B * T * C, dtype=torch.float32, device=device), B, T, C)
+    def empty(cls, B: int, T: int, C: int, device, parts: bool = False, offset: int = 0, bstride: Optional[int] = None) -> "Act":
+        n = B * (T * C if bstride is None else bstride)
+        return cls(torch.empty(n + n // 128 + 1 if parts else n, dtype=torch.float32, device=device), B, T, C, offset, bstride, parts)
 
     @property
     def ptr(self) -> int:
         return self.buf.data_ptr() + 4 * self.offset
 
+    @property
+    def codes(self) -> Optional[int]:
+        return self.buf.data_ptr() + 4 * self.B * self.bstride + self.offset // 32 if self.parts else None
+
     def tensor(self) -> torch.Tensor:
         """[B, T, C] view"""
+        if self.parts:
+            raise VoxB200Error("an activation kept as parts has no view as floats")
         return self.buf.as_strided((self.B, self.T, self.C), (self.bstride, self.C, 1), self.offset)
 
 
@@ -58,21 +67,32 @@ def _ptr(t) -> Optional[int]:
     return None if t is None else (t.ptr if isinstance(t, Act) else t.data_ptr())
 
 
+def _outputs(both: bool, out: str, new):
+    """(plain fp32, activated fp32, activated parts) of a convolution, and what it returns"""
+    if out not in ("f32", "parts"):
+        raise VoxB200Error(f"unknown form {out!r} of a convolution's result")
+    last = new(out == "parts")
+    plain = new(False) if both else None
+    if out == "parts":
+        return (plain, None, last), ((plain, last) if both else last)
+    return ((plain, last, None), (plain, last)) if both else ((last, None, None), last)
+
+
 def conv(x: Act, w: torch.Tensor, N: int, bias=None, ksize: int = 1, dil: int = 1, epi: str = "plain", resid: Optional[Act] = None,
          scale=None, noise=None, act: Optional[str] = None, alpha=None, lo: int = 0, hi: Optional[int] = None,
-         both: bool = False):
-    """Causal convolution (zeros before the start) of rows [lo, hi) -> Act [B, T, N]; ``both``: (plain, activated)."""
+         both: bool = False, out: str = "f32"):
+    """Causal convolution (zeros before the start) of rows [lo, hi) -> Act [B, T, N]; ``both``: (plain, activated).  ``out``: the
+    activated values as floats or as parts for the next convolution."""
     hi = x.T if hi is None else hi
-    y = Act.empty(x.B, x.T, N, x.buf.device)
-    y2 = Act.empty(x.B, x.T, N, x.buf.device) if both else None
-    call("vb_cl_conv", y.ptr, _ptr(y2), x.ptr, x.bstride, x.T, w.data_ptr(), _ptr(bias), _ptr(resid), resid.bstride if resid else 0,
-         _ptr(scale), _ptr(noise), noise.shape[-1] if noise is not None else 0, _ptr(alpha), EPI[epi], ACT[act], x.B, x.C, N, N, ksize, dil,
-         lo, hi, y.bstride, ops._stream())
-    return (y, y2) if both else y
+    (y, y2, yp), ret = _outputs(both, out, lambda parts: Act.empty(x.B, x.T, N, x.buf.device, parts))
+    call("vb_cl_conv_parts", _ptr(y), _ptr(y2), _ptr(yp), yp.codes if yp else None, x.ptr, x.codes, x.bstride, x.T, w.data_ptr(), _ptr(bias),
+         _ptr(resid), resid.bstride if resid else 0, _ptr(scale), _ptr(noise), noise.shape[-1] if noise is not None else 0, _ptr(alpha), EPI[epi],
+         ACT[act], x.B, x.C, N, N, ksize, dil, lo, hi, x.T * N, ops._stream())
+    return ret
 
 
 def conv_transposed(x: Act, w: torch.Tensor, cout: int, stride: int, bias, pad: int = 0, o_lo: int = 0, o_hi: Optional[int] = None,
-                    act: Optional[str] = None, both: bool = False):
+                    act: Optional[str] = None, both: bool = False, out: str = "f32"):
     """Transposed convolution with 2 * stride taps -> Act [B, T * stride, cout]; ``pad`` positions are dropped in front.  Output
     positions [o_lo, o_hi) are computed."""
     T_out = x.T * stride
@@ -80,17 +100,17 @@ def conv_transposed(x: Act, w: torch.Tensor, cout: int, stride: int, bias, pad: 
     n_lo, n_hi = (o_lo + pad) // stride, (o_hi - 1 + pad) // stride + 1
     N = stride * cout
     rows = x.T + (1 if pad else 0)
-    out = [Act(torch.empty(x.B * rows * N, dtype=torch.float32, device=x.buf.device), x.B, T_out, cout, pad * cout, rows * N)
-           for _ in range(2 if both else 1)]
-    call("vb_cl_conv", out[0].buf.data_ptr(), out[1].buf.data_ptr() if both else None, x.ptr, x.bstride, x.T, w.data_ptr(), _ptr(bias), None, 0,
-         None, None, 0, None, EPI["plain"], ACT[act], x.B, x.C, N, cout, 2, 1, n_lo, n_hi, rows * N, ops._stream())
-    return tuple(out) if both else out[0]
+    (y, y2, yp), ret = _outputs(both, out, lambda parts: Act.empty(x.B, T_out, cout, x.buf.device, parts, pad * cout, rows * N))
+    base = lambda a: None if a is None else a.buf.data_ptr()                 # noqa: E731  (the kernel's rows start before the padding)
+    call("vb_cl_conv_parts", base(y), base(y2), base(yp), yp.codes - yp.offset // 32 if yp else None, x.ptr, x.codes, x.bstride, x.T, w.data_ptr(),
+         _ptr(bias), None, 0, None, None, 0, None, EPI["plain"], ACT[act], x.B, x.C, N, cout, 2, 1, n_lo, n_hi, rows * N, ops._stream())
+    return ret
 
 
-def depthwise7(x: Act, w: torch.Tensor, bias, alpha_in, alpha_out, dil: int, lo: int, hi: int) -> Act:
+def depthwise7(x: Act, w: torch.Tensor, bias, alpha_in, alpha_out, dil: int, lo: int, hi: int, parts: bool = False) -> Act:
     """w [7, C]; alpha tables [2, C]: values, then 1 / (alpha + 1e-9)"""
-    y = Act.empty(x.B, x.T, x.C, x.buf.device)
-    call("vb_cl_dwconv7", y.ptr, x.ptr, x.bstride, w.data_ptr(), _ptr(bias), _ptr(alpha_in), _ptr(alpha_out), x.B, x.C, x.T, dil, lo, hi,
+    y = Act.empty(x.B, x.T, x.C, x.buf.device, parts)
+    call("vb_cl_dwconv7_parts", y.ptr, y.codes, x.ptr, x.bstride, w.data_ptr(), _ptr(bias), _ptr(alpha_in), _ptr(alpha_out), x.B, x.C, x.T, dil, lo, hi,
          ops._stream())
     return y
 

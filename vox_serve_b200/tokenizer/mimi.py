@@ -228,9 +228,9 @@ class MimiDecoder:
         (B, K, T), C, D, s = c.shape, cfg.dimension, cfg.codebook_dim, cfg.upsample_stride
         if T * s > 64:
             raise VoxB200Error(f"chunks of {T} frames exceed the attention kernel's 64 positions: decode in shorter chunks")
-        new = lambda t, ch: _cl.Act.empty(B, t, ch, self.device)                 # noqa: E731
-        z0, z1 = new(T, D), new(T, D)
-        call("vb_cl_codes_sum", z0.ptr, z1.ptr, c.data_ptr(), w["codebooks"].data_ptr(), B, K, cfg.bins, D, T, st)
+        new = lambda t, ch, parts=False: _cl.Act.empty(B, t, ch, self.device, parts)     # noqa: E731
+        z0, z1 = new(T, D, True), new(T, D, True)                                # (what only convolutions read is kept as parts)
+        call("vb_cl_codes_sum_parts", z0.ptr, z1.ptr, z0.codes, z1.codes, c.data_ptr(), w["codebooks"].data_ptr(), B, K, cfg.bins, D, T, st)
         x = _cl.conv(z0, tc["rvq_first.proj"], C)
         if K > 1:
             x = _cl.conv(z1, tc["rvq_rest.proj"], C, epi="resid", resid=x)
@@ -241,31 +241,33 @@ class MimiDecoder:
             taps["latent"] = x.tensor().transpose(1, 2).contiguous()
 
         def norm(v, name):
-            y = new(T, C)
-            call("vb_cl_layernorm", y.ptr, v.ptr, w[name + "w"].data_ptr(), w[name + "b"].data_ptr(), B * T, C, 1e-5, st)
+            y = new(T, C, True)
+            call("vb_cl_layernorm_parts", y.ptr, y.codes, v.ptr, w[name + "w"].data_ptr(), w[name + "b"].data_ptr(), B * T, C, 1e-5, st)
             return y
 
         for i in range(cfg.num_layers):
             p = f"t{i}."
-            qkv, a = _cl.conv(norm(x, p + "n1"), tc[p + "in"], 3 * C), new(T, C)
-            call("vb_cl_chunk_attention", a.ptr, qkv.ptr, B, C, cfg.num_heads, T, float(cfg.max_period), st)
+            qkv, a = _cl.conv(norm(x, p + "n1"), tc[p + "in"], 3 * C), new(T, C, C // cfg.num_heads % 32 == 0)
+            call("vb_cl_chunk_attention_parts", a.ptr, a.codes, qkv.ptr, B, C, cfg.num_heads, T, float(cfg.max_period), st)
             x = _cl.conv(a, tc[p + "out"], C, epi="scale_resid", resid=x, scale=w[p + "s1"])
-            m = _cl.conv(norm(x, p + "n2"), tc[p + "l1"], cfg.dim_feedforward, act="gelu")
-            x = _cl.conv(m, tc[p + "l2"], C, epi="scale_resid", resid=x, scale=w[p + "s2"])
-        if taps is not None:
-            taps["transformer_out"] = x.tensor().transpose(1, 2).contiguous()
+            m = _cl.conv(norm(x, p + "n2"), tc[p + "l1"], cfg.dim_feedforward, act="gelu", out="parts")
+            last = i + 1 == cfg.num_layers                 # the stream itself is not read behind the last layer
+            x = _cl.conv(m, tc[p + "l2"], C, epi="scale_resid", resid=x, scale=w[p + "s2"], both=last and taps is not None,
+                         out="parts" if last else "f32")
+            if last and taps is not None:
+                taps["transformer_out"], x = x[0].tensor().transpose(1, 2).contiguous(), x[1]
         ch, ratios = cfg.n_filters * 2 ** len(cfg.ratios), list(cfg.ratios)
         plain = None
         for kind, idx in self.layout:
             d = f"d{idx}."
             if kind == "conv_in":
-                x = _cl.conv(x, tc[d + "w"], ch, w[d + "b"], ksize=cfg.kernel_size, act="elu")
+                x = _cl.conv(x, tc[d + "w"], ch, w[d + "b"], ksize=cfg.kernel_size, act="elu", out="parts")
             elif kind == "convtr":
                 ch //= 2
-                plain, x = _cl.conv_transposed(x, tc[d + "w"], ch, ratios.pop(0), w[d + "b"], act="elu", both=True)
+                plain, x = _cl.conv_transposed(x, tc[d + "w"], ch, ratios.pop(0), w[d + "b"], act="elu", both=True, out="parts")
             elif kind == "res":
-                h = _cl.conv(x, tc[d + "w1"], ch // cfg.compress, w[d + "b1"], ksize=cfg.residual_kernel_size, act="elu")
-                x = _cl.conv(h, tc[d + "w3"], ch, w[d + "b3"], epi="resid", resid=plain, act="elu")
+                h = _cl.conv(x, tc[d + "w1"], ch // cfg.compress, w[d + "b1"], ksize=cfg.residual_kernel_size, act="elu", out="parts")
+                x = _cl.conv(h, tc[d + "w3"], ch, w[d + "b3"], epi="resid", resid=plain, act="elu", out="parts" if ratios else "f32")
             else:
                 k = cfg.last_kernel_size
                 return _cl.last_conv(x, w[d + "w"], w[d + "b"], k, k - 1, 0, x.T, tanh=False)

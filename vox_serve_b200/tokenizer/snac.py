@@ -266,24 +266,25 @@ class SNAC:
         z = _cl.Act.empty(B, T, C, dev)
         call("vb_cl_from_codes", z.ptr, c[0].data_ptr(), c[1].data_ptr(), c[2].data_ptr(), w["codebooks"].data_ptr(),
              w["proj_w"].data_ptr(), w["proj_b"].data_ptr(), B, C, T, self.codebook_size, self.codebook_dim, *self.vq_strides, ops._stream())
-        x = _cl.depthwise7(z, self.tc["in_dw_w"], w["in_dw_b"], None, None, 1, *in_range)
+        x = _cl.depthwise7(z, self.tc["in_dw_w"], w["in_dw_b"], None, None, 1, *in_range, parts=True)
         ch = self.decoder_dim
-        x = _cl.conv(x, self.tc["in_pw_w"], ch, w["in_pw_b"], act="snake", alpha=self.tc["b0.alpha"], lo=in_range[0], hi=in_range[1])
+        x = _cl.conv(x, self.tc["in_pw_w"], ch, w["in_pw_b"], act="snake", alpha=self.tc["b0.alpha"], lo=in_range[0], hi=in_range[1],
+                     out="parts")
         noises, nb = self._noises(noises, B, T), len(self.decoder_rates)
         for bi, s in enumerate(self.decoder_rates):
             (c_lo, c_hi), units = blocks[bi]
             ch //= 2
-            u = _cl.conv_transposed(x, self.tc[f"b{bi}.ct_w"], ch, s, w[f"b{bi}.ct_b"], (s + 1) // 2, c_lo, c_hi)
+            u, up = _cl.conv_transposed(x, self.tc[f"b{bi}.ct_w"], ch, s, w[f"b{bi}.ct_b"], (s + 1) // 2, c_lo, c_hi, both=True, out="parts")
             nz = noises[bi].to(device=dev, dtype=torch.float32).contiguous()
             assert nz.numel() == B * u.T, "noise tensor shape mismatch"
-            x = _cl.conv(u, self.tc[f"b{bi}.noise_w"], ch, epi="noise", resid=u, noise=nz.view(B, u.T), lo=c_lo, hi=c_hi)
+            x = _cl.conv(up, self.tc[f"b{bi}.noise_w"], ch, epi="noise", resid=u, noise=nz.view(B, u.T), lo=c_lo, hi=c_hi)
             for j, dil in enumerate((1, 3, 9)):
                 q, (u_lo, u_hi) = f"b{bi}.r{j}.", units[j]
-                h = _cl.depthwise7(x, self.tc[q + "dw_w"], w[q + "dw_b"], self.tc[q + "alpha1"], self.tc[q + "alpha2"], dil, u_lo, u_hi)
+                h = _cl.depthwise7(x, self.tc[q + "dw_w"], w[q + "dw_b"], self.tc[q + "alpha1"], self.tc[q + "alpha2"], dil, u_lo, u_hi, parts=True)
                 # the last unit's output only feeds the next stage's Snake: fused into this epilogue
                 nxt = None if j < 2 else self.tc[f"b{bi + 1}.alpha" if bi + 1 < nb else "out.alpha"]
                 x = _cl.conv(h, self.tc[q + "pw_w"], ch, w[q + "pw_b"], epi="resid", resid=x, act=None if nxt is None else "snake",
-                             alpha=nxt, lo=u_lo, hi=u_hi)
+                             alpha=nxt, lo=u_lo, hi=u_hi, out="parts" if j == 2 and bi + 1 < nb else "f32")
         return _cl.last_conv(x, w["out.w"], w["out.b"], 7, 3, *out_range, tanh=True)
 
     @torch.no_grad()

@@ -532,6 +532,37 @@ def test_paged_prompt_attention_pages(ops, page, D, H, G, kv, new):
     assert _lib.load().vb_prefill_attn_tc_timeouts() == 0
 
 
+# row tiles whose keys two blocks share: the fewest key tiles that are shared, a key before and behind; a second half that ends in a key tile of
+# one key, with rows of the tile that see nothing of it; boxes and rows of cp.async; both layouts of the result
+@pytest.mark.parametrize("page,tiled", [(64, True), (16, False), (20, False)])
+@pytest.mark.parametrize("D,H,G,kv,new", [(128, 6, 2, [320, 321, 384, 385], [1, 64, 100, 43]), (64, 4, 4, [449, 1000, 64], [449, 3, 2])])
+def test_paged_prompt_attention_shared_tiles(ops, page, tiled, D, H, G, kv, new):
+    from vox_serve_b200 import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(page + D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()      # noqa: E731
+    pages = [(x + page - 1) // page for x in kv]
+    ip = np.concatenate([[0], np.cumsum(pages)]).tolist()
+    T, q = sum(new), rnd(sum(new), H, D)
+    cache = torch.full((ip[-1], 2, page, G, D), float("nan"), device="cuda").bfloat16()
+    want, at = [], 0
+    for b, L in enumerate(kv):
+        k, v, tok = rnd(L, G, D), rnd(L, G, D), torch.arange(L, device="cuda")
+        cache[ip[b] + tok // page, 0, tok % page], cache[ip[b] + tok // page, 1, tok % page] = k, v
+        s = torch.einsum("qhd,khd->hqk", q[at:at + new[b]].double(), k.double().repeat_interleave(H // G, 1)) * D ** -0.5
+        s = s.masked_fill(tok[None] > torch.arange(L - new[b], L, device="cuda")[:, None], -float("inf"))
+        want.append(torch.einsum("hqk,khd->qhd", torch.softmax(s, -1), v.double().repeat_interleave(H // G, 1)))
+        at += new[b]
+    plan = ops.RowPlan(T, "cuda")
+    ops.plan_rows(plan, _i32([0] + np.cumsum(new).tolist()), _i32(ip), _i32(list(range(ip[-1]))), _i32([(x - 1) % page + 1 for x in kv]), len(kv), T,
+                  page, page, keys=ip[-1] * page)
+    out = ops.TiledAct(T, H * D, "cuda") if tiled else None
+    out = ops.paged_attn(q, cache, 0, plan, T, G, page, page, None, out=out, prefill_tiles="tc")
+    got = out.to_rows().view(T, H, D) if tiled else out
+    _close(got, torch.cat(want), 2 ** -8)            # probabilities and the output rounded to bf16
+    assert _lib.load().vb_prefill_attn_tc_timeouts() == 0
+
+
 @pytest.mark.parametrize("H", [128, 129, 200])
 def test_paged_prompt_attention_many_heads_per_key_head(ops, H):
     """More query heads on one key head than a tcgen05 row tile has rows: an automatic plan runs all the same."""

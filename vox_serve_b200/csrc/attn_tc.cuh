@@ -1,12 +1,15 @@
 // The tcgen05 attention core of prompt rows, shared by prefill_attn_tc.cu (paged cache of the speech LMs) and window_attn_tc.cu
 // (sliding windows of the text LMs): one accumulator row of 128 per softmax thread, scores and probabilities in TMEM, K and V
 // tiles of 64 keys through two-stage rings.  A kernel brings an object `rows` that says what its thread's row sees:
-//   n_tiles, tile(it)        the key tiles to walk, in order (tile i holds keys 64 i ..)
+//   n_tiles, tile(it)        the key tiles that the block walks, in order (tile i holds keys 64 i ..)
 //   scale_log2               what a score is multiplied by, times log2(e)
 //   full(tok0), visible(kj)  whether all 64 keys from tok0 / key kj are visible to this thread's row
-//   q_row()                  this thread's query row, or nullptr (a padding row: zeros)
+//   group, q_row(t, g)       accumulator row r is row t = r / group of the tile, head g = r % group of the group: its query row, or nullptr
+//                            (a padding row: zeros)
 //   finish(m_ref, l)         factor for the accumulated row, given the exponents' reference and the denominator against it
-//   store(c0, o, f)          32 output values from column c0, times the factor
+//   store(c0, o, f)          32 output values of this thread's row from column c0, times the factor: either out to memory, or
+//   STAGED                   as bf16 through shared memory; out_at(t, g, c) is then where 16-byte chunk c of a row goes (nullptr: a padding
+//                            row)
 //   HOLE, hole0, hole1       keys [hole0, hole1) are seen by no row of the block: they are neither fetched nor multiplied
 // The running maximum, its rescale and the division at the end are the online softmax of M. Milakov and N. Gimelshein ("Online normalizer
 // calculation for softmax", 2018) as FlashAttention walks it over key tiles (T. Dao et al., 2022); the roles of the warps and scores
@@ -32,9 +35,41 @@ __device__ __forceinline__ float ptc_ex2(float x) {
   return y;
 }
 
+// two fp32 values in a register pair: one instruction for both
+__device__ __forceinline__ uint64_t ptc_pair(uint32_t a, uint32_t b) { return static_cast<uint64_t>(b) << 32 | a; }
+__device__ __forceinline__ uint64_t ptc_pair(float a, float b) { return ptc_pair(__float_as_uint(a), __float_as_uint(b)); }
+__device__ __forceinline__ float ptc_lo(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v)); }
+__device__ __forceinline__ float ptc_hi(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v >> 32)); }
+__device__ __forceinline__ uint64_t ptc_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t ptc_add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float ptc_max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// what two bf16 roundings left of their values, as bf16 (the differences are exact)
+__device__ __forceinline__ uint32_t ptc_left(float p0, float p1, uint32_t h) {
+  float d0, d1;
+  asm("{\n\t.reg .b16 h0, h1, m;\n\tmov.b32 {h0, h1}, %2;\n\tmov.b16 m, 0xBF80;\n\tfma.rn.f32.bf16 %0, h0, m, %3;\n\tfma.rn.f32.bf16 %1, h1, m, %4;\n\t}\n"
+      : "=f"(d0), "=f"(d1)
+      : "r"(h), "f"(p0), "f"(p1));
+  return pack_bf16(d0, d1);
+}
+
 constexpr int PTC_THREADS = 224;       // 4 softmax warps, 1 MMA warp, 2 loader warps
 constexpr int PTC_KT = 64;             // tokens per K / V tile
 constexpr int PTC_STAGES = 2;          // K and V tiles in flight, each with barriers of their own
+// Where a launch has clusters of two blocks, row tiles that walk at least this many key tiles share them between the two (PtcHalf).  They meet at
+// the end, some 3 us, 1.3 us being a key tile's: nothing to gain below.
+constexpr int PTC_SPLIT_TILES = 6;
 constexpr float PTC_RESCALE = 8.f;     // growth of a row's maximum (base 2) that moves the exponents' reference
 
 template <int D>
@@ -118,21 +153,135 @@ __device__ __forceinline__ void ptc_init(PtcShared* sh, int loader_arrivals) {
   sh->tile[0] = -1;
 }
 
+// Accumulator rows r0, r0 + STEP, ... as (row of the tile, head of the group): one division for all of them
+template <int STEP>
+struct PtcWalk {
+  int t, g, dt, dg, group;
+  __device__ __forceinline__ PtcWalk(int r0, int group_) : t(r0 / group_), dt(STEP / group_), group(group_) {
+    g = r0 - t * group;
+    dg = STEP - dt * group;
+  }
+  __device__ __forceinline__ void next() {
+    t += dt;
+    g += dg;
+    if (g >= group) {
+      g -= group;
+      ++t;
+    }
+  }
+};
+// Results as bf16 on their way out: a thread's row goes to the place of the query rows (the last scores have been multiplied), 16-byte chunk c
+// of row r at chunk c ^ (r & 7) of its eight, and leaves in whole rows
+template <int D>
+__device__ __forceinline__ uint4* ptc_staged(uint8_t* smem, int r, int c) {
+  return reinterpret_cast<uint4*>(smem + PtcLayout<D>::Q + r * D * 2) + ((c & ~7) | ((c ^ r) & 7));
+}
+template <int D>
+__device__ __forceinline__ void ptc_put32(uint8_t* smem, int c0, const uint32_t (&o)[32], float f) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = pack_bf16(__uint_as_float(o[c * 8 + 2 * i]) * f, __uint_as_float(o[c * 8 + 2 * i + 1]) * f);
+    *ptc_staged<D>(smem, threadIdx.x, (c0 >> 3) + c) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+// columns [c_lo, c_lo + C) of all rows, once the four softmax warps have put theirs
+template <int D, int C, class Rows>
+__device__ __forceinline__ void ptc_send(uint8_t* smem, const Rows& rows, int c_lo) {
+  constexpr int CPR = C / 8;
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  constexpr int STEP = 128 / CPR;
+  const int c = (c_lo >> 3) + threadIdx.x % CPR, r0 = threadIdx.x / CPR;
+  PtcWalk<STEP> w(r0, rows.group);
+#pragma unroll 4
+  for (int i = 0; i < CPR; ++i, w.next()) {
+    uint4* dst = rows.out_at(w.t, w.g, c);
+    if (dst) *dst = *ptc_staged<D>(smem, r0 + i * STEP, c);
+  }
+}
+
+// The key tiles of a block: all of the row tile's, or its half of them where the cluster's two blocks share a row tile.
+struct PtcHalf {
+  int first, n, rank;
+  bool split;
+  __device__ __forceinline__ PtcHalf(int n_tiles, bool shared, int rank_) : rank(rank_) {
+    split = shared && n_tiles >= PTC_SPLIT_TILES;
+    const int half = (n_tiles + 1) >> 1;
+    first = split && rank ? half : 0;
+    n = split ? (rank ? n_tiles - half : half) : (rank ? 0 : n_tiles);
+  }
+};
+// What a thread of a shared row tile leaves for the other block, in its own block's K and V stages (their last tile has been multiplied): the
+// accumulated row's columns of the other block's half, [column][128 rows], the exponents' reference and the denominator.
+template <int D>
+__device__ __forceinline__ void ptc_give(uint8_t* smem, uint32_t t_lane, int rank, float m, float l) {
+  float* buf = reinterpret_cast<float*>(smem + PtcLayout<D>::K) + threadIdx.x;
+  const int c_other = (1 - rank) * (D / 2);
+#pragma unroll
+  for (int c0 = 0; c0 < D / 2; c0 += 32) {
+    uint32_t o[32];
+    tmem_ld_32x32(t_lane + 128 + c_other + c0, o);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) buf[(c0 + i) * 128] = __uint_as_float(o[i]);
+  }
+  buf[(D / 2) * 128] = m;
+  buf[(D / 2 + 1) * 128] = l;
+}
+// ... and the merge of this block's half of the columns, once both have met
+template <int D, class Rows>
+__device__ __forceinline__ void ptc_merge(uint8_t* smem, uint32_t tmem, const Rows& rows, int rank, float m, float l) {
+  const uint32_t t_lane = tmem + ((threadIdx.x >> 5) * 32u << 16);
+  uint32_t far;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(smem_u32(smem + PtcLayout<D>::K) + threadIdx.x * 4), "r"(1 - rank));
+  auto get = [&](int c) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(far + c * 512) : "memory");
+    return v;
+  };
+  const float m1 = get(D / 2), l1 = get(D / 2 + 1), M = fmaxf(m, m1);
+  const float a0 = m == -INFINITY ? 0.f : ptc_ex2(m - M), a1 = m1 == -INFINITY ? 0.f : ptc_ex2(m1 - M);
+  const float f = rows.finish(M, l * a0 + l1 * a1);
+#pragma unroll 1
+  for (int c0 = 0; c0 < D / 2; c0 += 32) {
+    uint32_t o[32];
+    float r[32];
+    tmem_ld_32x32(t_lane + 128 + rank * (D / 2) + c0, o);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) r[i] = get(c0 + i);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * a0 + r[i] * a1);
+    if (rows.STAGED) ptc_put32<D>(smem, rank * (D / 2) + c0, o, f);
+    else rows.store(rank * (D / 2) + c0, o, f);
+  }
+  if (rows.STAGED) ptc_send<D, D / 2>(smem, rows, rank * (D / 2));
+}
+
 // ================= warps 0..3: softmax =================
 template <int D, class Rows>
-__device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const Rows& rows, BoundedWait& bw) {
+__device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const Rows& rows, const PtcHalf& half, float& m_out, float& l_out,
+                                            BoundedWait& bw) {
   using L = PtcLayout<D>;
   constexpr int KBD = D / 64, CPR = D * 2 / 16;
   const int tid = threadIdx.x, warp = tid >> 5, n_tiles = rows.n_tiles;
   {
-    const __nv_bfloat16* src = rows.q_row();
+    // CPR neighbouring threads take a row: a warp reads whole rows, four or two at a time.  (A row per thread, 16 bytes of 32 rows an
+    // instruction: the rows were there after 6 us instead of 2.)
     __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem + L::Q);
+    constexpr int STEP = 128 / CPR;
+    const int c = tid % CPR, r0 = tid / CPR;
+    uint4 v[CPR];
+    PtcWalk<STEP> w(r0, rows.group);
 #pragma unroll
-    for (int c = 0; c < CPR; ++c) {
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (src) v = *reinterpret_cast<const uint4*>(src + c * 8);
-      *reinterpret_cast<uint4*>(sQ + xt_index(tid, c * 8, 128, KBD)) = v;
+    for (int i = 0; i < CPR; ++i, w.next()) {
+      const __nv_bfloat16* src = rows.q_row(w.t, w.g);
+      v[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (src) v[i] = *reinterpret_cast<const uint4*>(src + c * 8);
     }
+#pragma unroll
+    for (int i = 0; i < CPR; ++i) *reinterpret_cast<uint4*>(sQ + xt_index(r0 + i * STEP, c * 8, 128, KBD)) = v[i];
     fence_proxy_async();
     mbar_arrive(&sh->q_full);
   }
@@ -165,11 +314,11 @@ __device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const 
     }
     float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
-    for (int i = 0; i < 64; i += 4) {
-      m0 = fmaxf(m0, __uint_as_float(v[i]));
-      m1 = fmaxf(m1, __uint_as_float(v[i + 1]));
-      m2 = fmaxf(m2, __uint_as_float(v[i + 2]));
-      m3 = fmaxf(m3, __uint_as_float(v[i + 3]));
+    for (int i = 0; i < 64; i += 8) {
+      m0 = ptc_max3(m0, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+      m1 = ptc_max3(m1, __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
+      m2 = ptc_max3(m2, __uint_as_float(v[i + 4]), __uint_as_float(v[i + 5]));
+      m3 = ptc_max3(m3, __uint_as_float(v[i + 6]), __uint_as_float(v[i + 7]));
     }
     const float mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) * scale;
     const bool move = mx > m_ref + PTC_RESCALE || (m_ref == -INFINITY && mx > -INFINITY);
@@ -195,17 +344,18 @@ __device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const 
     const float u = m_ref == -INFINITY ? 0.f : m_ref;          // every key masked so far
     // a probability goes in as two bf16 terms, its rounding and what that left (relative 2^-17): the reference may lag, and the largest
     // of a row, 1 and exact against the maximum itself, need not be a power of two
-    float l0 = 0.f, l1 = 0.f;
+    uint64_t l2 = ptc_pair(0.f, 0.f);
+    const uint64_t scale2 = ptc_pair(scale, scale), u2 = ptc_pair(-u, -u);
     uint32_t ph[32], pl[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-      const float p0 = ptc_ex2(fmaf(__uint_as_float(v[2 * i]), scale, -u)), p1 = ptc_ex2(fmaf(__uint_as_float(v[2 * i + 1]), scale, -u));
-      l0 += p0;
-      l1 += p1;
+      const uint64_t x = ptc_fma2(ptc_pair(v[2 * i], v[2 * i + 1]), scale2, u2);
+      const float p0 = ptc_ex2(ptc_lo(x)), p1 = ptc_ex2(ptc_hi(x));
+      l2 = ptc_add2(l2, ptc_pair(p0, p1));
       ph[i] = pack_bf16(p0, p1);
-      pl[i] = pack_bf16(p0 - bf16_lo(ph[i]), p1 - bf16_hi(ph[i]));
+      pl[i] = ptc_left(p0, p1, ph[i]);
     }
-    l_run += l0 + l1;
+    l_run += ptc_lo(l2) + ptc_hi(l2);
     ptc_tmem_st32(sc, ph);
     ptc_tmem_st32(sc + 32, pl);
     ptc_tmem_st_wait();
@@ -219,6 +369,12 @@ __device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const 
   }
   if (bw.dead) return;
   tc_fence_after();
+  if (half.split) {
+    ptc_give<D>(smem, t_lane, half.rank, m_ref, l_run);
+    m_out = m_ref;
+    l_out = l_run;
+    return;
+  }
   const float f = rows.finish(m_ref, l_run);
 #pragma unroll 1
   for (int c0 = 0; c0 < D; c0 += 32) {
@@ -230,8 +386,10 @@ __device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const 
 #pragma unroll
       for (int i = 0; i < 32; ++i) o[i] = 0u;
     }
-    rows.store(c0, o, f);
+    if (rows.STAGED) ptc_put32<D>(smem, c0, o, f);
+    else rows.store(c0, o, f);
   }
+  if (rows.STAGED) ptc_send<D, D>(smem, rows, 0);
 }
 
 // ================= warp 4: MMA issuer (the whole warp walks the loop, one elected lane issues: operands stay in uniform registers) =================

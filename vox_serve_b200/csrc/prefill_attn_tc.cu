@@ -24,8 +24,10 @@
 // mma.sync.  Measured per launch (mma.sync / this kernel, us, back to back): one 133-row prompt 11.6 / 10.1, eight of them 29 / 14,
 // four portions of 997 rows on up to 1063 cached tokens 112 / 40, three prompts of 1024 rows each 187 / 61, four of 600 with 64-wide heads
 // 74 / 32.
-// What bounds it: the serial chain of a tile (scores -> maximum -> exponentials -> P V, about 1.3 us), and where few tiles see
-// a long context the longest of them.
+// Query rows come and results leave in whole rows, a few neighbouring threads each (a row per thread took 6 us until the rows were there and 3 us
+// at the end of a launch of cold data, 2 and 2 now); where portions continue long contexts two blocks of a cluster share a row tile's keys
+// and merge through distributed shared memory.  The 997 rows above: 45 us a layer of cold data, 36 with whole rows, 26 shared as well.
+// What bounds it: the serial chain of a tile (scores -> maximum -> exponentials -> P V, about 1.3 us), some 5 us around it.
 // Every wait is bounded (BoundedWait): a block whose wait runs out sets its flag, stops issuing and leaves.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 1
@@ -45,36 +47,31 @@ struct PrefillTcParams {
   int n_req, n_rows, n_q, n_kv, G, TQ, page_size;
   int out_xt_tile;
   int box_tokens;
+  int shared;
   float scale_log2;
   unsigned char* wait_flag;
 };
 
 // what this thread's row sees: the first kl keys of its request
 struct PagedRows {
-  static constexpr bool HOLE = false;
+  static constexpr bool HOLE = false, STAGED = true;
   static constexpr int hole0 = 0, hole1 = 0;
   const PrefillTcParams& p;
-  int n_tiles, kl, row, head, D;
-  bool ok;
+  int n_tiles, first, kl, row0, nrows, head0, group, D;
   float scale_log2;
-  __device__ __forceinline__ int tile(int it) const { return it; }
+  __device__ __forceinline__ int tile(int it) const { return first + it; }
   __device__ __forceinline__ bool full(int tok0) const { return tok0 + PTC_KT <= kl; }
   __device__ __forceinline__ bool visible(int kj) const { return kj < kl; }
-  __device__ __forceinline__ const __nv_bfloat16* q_row() const {
-    return ok ? p.q + (static_cast<size_t>(row) * p.n_q + head) * D : nullptr;
+  __device__ __forceinline__ const __nv_bfloat16* q_row(int t, int g) const {
+    return t < nrows ? p.q + (static_cast<size_t>(row0 + t) * p.n_q + head0 + g) * D : nullptr;
   }
   __device__ __forceinline__ float finish(float, float l) const { return l > 0.f ? 1.f / l : 0.f; }
-  __device__ __forceinline__ void store(int c0, const uint32_t (&o)[32], float f) const {
-    if (!ok) return;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      uint32_t w[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) w[i] = pack_bf16(__uint_as_float(o[c * 8 + 2 * i]) * f, __uint_as_float(o[c * 8 + 2 * i + 1]) * f);
-      const int e = head * D + c0 + c * 8;
-      const size_t at = p.out_xt_tile ? xt_index(row, e, p.out_xt_tile, (p.n_q * D + 63) >> 6) : static_cast<size_t>(row) * p.n_q * D + e;
-      *reinterpret_cast<uint4*>(p.out + at) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+  __device__ __forceinline__ void store(int, const uint32_t (&)[32], float) const {}
+  __device__ __forceinline__ uint4* out_at(int t, int g, int c) const {
+    if (t >= nrows) return nullptr;
+    const int row = row0 + t, e = (head0 + g) * D + c * 8;
+    const size_t at = p.out_xt_tile ? xt_index(row, e, p.out_xt_tile, (p.n_q * D + 63) >> 6) : static_cast<size_t>(row) * p.n_q * D + e;
+    return reinterpret_cast<uint4*>(p.out + at);
   }
 };
 
@@ -103,9 +100,11 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
   pdl_sync();
 
   // rows beyond the last request (CUDA-graph padding) produce zeros
-  if (blockIdx.y == 0) {
+  // key heads fastest; where row tiles may be shared a cluster is two blocks of one of them
+  const int rank = p.shared ? blockIdx.x & 1 : 0, hk = p.shared ? blockIdx.x >> 1 : blockIdx.x;
+  if (blockIdx.x == 0) {
     const int n_valid = p.qo_indptr[p.n_req];
-    for (int row = n_valid + blockIdx.x; row < p.n_rows; row += gridDim.x)
+    for (int row = n_valid + blockIdx.y; row < p.n_rows && blockIdx.z == 0; row += gridDim.y)
       for (int i = tid; i < p.n_q * D / 8; i += PTC_THREADS) {
         const int e = i * 8;
         const size_t o = p.out_xt_tile ? xt_index(row, e, p.out_xt_tile, (p.n_q * D + 63) >> 6)
@@ -116,7 +115,7 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
 
   // ---- which (request, rows) is this block's tile?  prefix sum of ceil(n_new / TQ) over the requests.  Blocks take the tiles
   // from the last one back: late rows see the most keys, and the longest tiles should not start last ----
-  const int TQ = p.TQ, b = static_cast<int>(gridDim.x - 1 - blockIdx.x);
+  const int TQ = p.TQ, b = static_cast<int>(gridDim.y * gridDim.z - 1 - (blockIdx.z * gridDim.y + blockIdx.y));
   int base = 0;
   for (int r0 = 0; r0 < p.n_req; r0 += PTC_THREADS) {
     __syncthreads();
@@ -151,16 +150,22 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
   }
   __syncthreads();
   const int req = sh->tile[0];
+  bool split = false;                             // alike in both blocks
   if (req >= 0) {
-    const int row0 = sh->tile[1], nrows = sh->tile[2], hk = blockIdx.y;
+    const int row0 = sh->tile[1], nrows = sh->tile[2];
     // the tile's largest bound (the bounds do not decrease inside a request: the last row's)
     const int kmax = p.row_kvlen[row0 + nrows - 1];
-    const int n_tiles = (kmax + PTC_KT - 1) / PTC_KT;
+    const PtcHalf half((kmax + PTC_KT - 1) / PTC_KT, p.shared != 0, rank);
+    const int n_tiles = half.n, first = half.first;
+    split = half.split;
     const int t = tid / p.G;                      // (softmax) this thread's accumulator row: prompt row t of the tile, head tid % G
     const bool ok = warp < 4 && t < nrows;
-    const PagedRows rows{p, n_tiles, ok ? p.row_kvlen[row0 + t] : 0, row0 + t, hk * p.G + tid - t * p.G, D, ok, p.scale_log2};
-    if (warp < 4) {
-      ptc_softmax<D>(smem, sh, rows, bw);
+    const PagedRows rows{p, n_tiles, first, ok ? p.row_kvlen[row0 + t] : 0, row0, nrows, hk * p.G, p.G, D, p.scale_log2};
+    float m = 0.f, l = 0.f;
+    if (rank == 1 && !split) {
+      // (the other block's row tile alone)
+    } else if (warp < 4) {
+      ptc_softmax<D>(smem, sh, rows, half, m, l, bw);
     } else if (warp == 4) {
       ptc_issue<D>(smem, sh, n_tiles, bw);
     } else if (TMA) {
@@ -179,7 +184,7 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
       const int ltok = tid - 160, pbase = p.kv_indptr[req];
       const size_t page_elems = static_cast<size_t>(p.page_size) * p.n_kv * D;
       auto fetch = [&](int j, int is_v) {
-        const int tok = j * PTC_KT + ltok;
+        const int tok = (first + j) * PTC_KT + ltok;
         const uint32_t dst = smem_u32(smem + (is_v ? L::V : L::K) + (j & 1) * L::TILE) + ltok * 128;
         if (tok < kmax) {
           const int page = __ldg(&p.kv_indices[pbase + tok / p.page_size]);
@@ -221,6 +226,13 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
         mbar_arrive(&sh->v_full[(n_tiles - 1) & 1]);
       }
     }
+    if (split) {
+      __syncwarp();
+      cluster_sync_all();
+      if (warp < 4 && !bw.dead) ptc_merge<D>(smem, tmem_base, rows, rank, m, l);
+      __syncwarp();
+      cluster_sync_all();                         // (the other block has read what this one gave)
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -236,7 +248,7 @@ static int launch_prefill_tc(const PrefillTcParams& p, const CUtensorMap& map, d
   // (a fixed size per instantiation -- safe under CUDA-graph replay)
   constexpr int smem_bytes = PtcLayout<D>::TOTAL;
   VB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-  VB_LAUNCH_PDL(kern, grid, PTC_THREADS, smem_bytes, stream, p, map);
+  VB_LAUNCH_PDL_CLUSTER(kern, grid, PTC_THREADS, smem_bytes, stream, p.shared ? 2 : 1, p, map);
   return 0;
 }
 }  // namespace vb
@@ -258,6 +270,14 @@ int vb_paged_prefill_attn_tc(void* d_out, const void* d_q, const void* d_kv, int
                              const int32_t* d_qo_indptr, const int32_t* d_kv_indptr, const int32_t* d_kv_indices,
                              const int32_t* d_row_kvlen, int n_req, int n_rows, int n_q, int n_kv, int head_dim,
                              int page_size, float sm_scale, int out_xt_tile, void* stream) {
+  return vb_paged_prefill_attn_tc_keys(d_out, d_q, d_kv, slab_base, d_qo_indptr, d_kv_indptr, d_kv_indices, d_row_kvlen, n_req, n_rows, n_q, n_kv,
+                                       head_dim, page_size, sm_scale, out_xt_tile, 0, stream);
+}
+
+int vb_paged_prefill_attn_tc_keys(void* d_out, const void* d_q, const void* d_kv, int64_t slab_base,
+                                  const int32_t* d_qo_indptr, const int32_t* d_kv_indptr, const int32_t* d_kv_indices,
+                                  const int32_t* d_row_kvlen, int n_req, int n_rows, int n_q, int n_kv, int head_dim,
+                                  int page_size, float sm_scale, int out_xt_tile, long long keys, void* stream) {
   VB_CHECK_ARG(d_out && d_q && d_kv && d_qo_indptr && d_kv_indptr && d_kv_indices && d_row_kvlen,
                "vb_paged_prefill_attn_tc: null pointer");
   VB_CHECK_ARG(n_kv > 0 && n_q % n_kv == 0 && n_q / n_kv <= 128, "vb_paged_prefill_attn_tc: %d query heads / %d kv heads",
@@ -279,7 +299,13 @@ int vb_paged_prefill_attn_tc(void* d_out, const void* d_q, const void* d_kv, int
   p.TQ = 128 / p.G;
   p.out_xt_tile = out_xt_tile;
   p.scale_log2 = sm_scale * 1.4426950408889634f;
-  const dim3 grid((n_rows + p.TQ - 1) / p.TQ + n_req, n_kv, 1);
+  const unsigned tiles = static_cast<unsigned>((n_rows + p.TQ - 1) / p.TQ) + static_cast<unsigned>(n_req), slices = (tiles + 65534) / 65535;
+  // Row tiles shared by two blocks: where portions continue long contexts -- the cached keys, pages counted whole, are more than twice the rows
+  // -- and the longest of them would run on alone (four portions of 997 rows on up to 1063 cached tokens: 36 us a layer, 26 shared), and where
+  // even twice the blocks find an SM of their own.  Elsewhere the clusters only start later (1024 rows of three fresh prompts, 20 launches
+  // around: 549 us, 565 shared).
+  p.shared = keys > 2LL * n_rows + static_cast<long long>(n_req) * page_size || static_cast<long long>(tiles) * n_kv * 2 <= 148;
+  const dim3 grid((p.shared ? 2 : 1) * n_kv, (tiles + slices - 1) / slices, slices);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   p.box_tokens = ptc_box_tokens(page_size);
   CUtensorMap map = {};

@@ -35,10 +35,13 @@ class _PagedWrapper:
         self.max_req = batch_size or 64
         self.max_pages = max_pages
         dev = self.device
-        self.d_qo = torch.zeros(self.max_req + 1, dtype=torch.int32, device=dev)
-        self.d_indptr = torch.zeros(self.max_req + 1, dtype=torch.int32, device=dev)
-        self.d_indices = torch.zeros(max_pages, dtype=torch.int32, device=dev)
-        self.d_last = torch.zeros(self.max_req, dtype=torch.int32, device=dev)
+        # the page tables of a plan lie in one buffer, so that tables built on the host go up in one copy; the long one last
+        sizes = (self.max_req + 1, self.max_req + 1, self.max_req, max_pages)
+        ends = [sum(sizes[:i + 1]) for i in range(4)]
+        self._at = [e - n for e, n in zip(ends, sizes)]
+        self._dev = torch.zeros(ends[-1], dtype=torch.int32, device=dev)
+        self._host = torch.zeros(ends[-1], dtype=torch.int32)
+        self.d_qo, self.d_indptr, self.d_last, self.d_indices = (self._dev[a:e] for a, e in zip(self._at, ends))
         self.plan_rows = ops.RowPlan(self.max_rows, dev)
         self.workspace = None
         self.n_rows = 0
@@ -62,6 +65,28 @@ class _PagedWrapper:
         dst[:n].copy_(t.to(torch.int32), non_blocking=True)
         return dst[:n]
 
+    def _upload_tables(self, qo, indptr, last, indices):
+        """The tables of a plan -> their places on the device (``qo`` None: a decode plan).  int32 tensors on the host go up in one copy
+        from a staging tensor (pageable: it may be written again once the call returns)."""
+        tables = (qo, indptr, last, indices)
+        if all(t is None or (isinstance(t, torch.Tensor) and t.device.type == "cpu" and t.dtype == torch.int32 and t.dim() == 1) for t in tables):
+            out, host, lo = [], self._host, None
+            for t, a, d in zip(tables, self._at, (self.d_qo, self.d_indptr, self.d_last, self.d_indices)):
+                if t is None:
+                    out.append(None)
+                    continue
+                n = t.numel()
+                if n > d.numel():
+                    raise VoxB200Error("page table larger than the wrapper's static buffers")
+                host[a:a + n].copy_(t)
+                lo = a if lo is None else lo
+                out.append(d[:n])
+            end = a + n
+            self._dev[lo:end].copy_(host[lo:end], non_blocking=True)
+            return out
+        qo = None if qo is None else self._upload(self.d_qo, qo)
+        return qo, self._upload(self.d_indptr, indptr), self._upload(self.d_last, last), self._upload(self.d_indices, indices)
+
     def set_kv_cache(self, kv_cache: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> None:
         """kv_cache[page, 0, slot] = k ; kv_cache[page, 1, slot] = v (flashinfer_utils.py:144-145, 243-244)."""
         ops.kv_append(kv_cache, k, v, self.plan_rows, n_rows=min(k.shape[0], self.n_rows_padded))
@@ -81,10 +106,7 @@ class FlashInferPrefillWrapper(_PagedWrapper):
     def plan(self, qo_indptr, paged_kv_indptr, paged_kv_indices, paged_kv_last_page_len,
              dtype: torch.dtype = torch.bfloat16, n_rows_padded: Optional[int] = None):
         n_req = len(paged_kv_last_page_len)
-        qo = self._upload(self.d_qo, qo_indptr)
-        ip = self._upload(self.d_indptr, paged_kv_indptr)
-        ix = self._upload(self.d_indices, paged_kv_indices)
-        la = self._upload(self.d_last, paged_kv_last_page_len)
+        qo, ip, la, ix = self._upload_tables(qo_indptr, paged_kv_indptr, paged_kv_last_page_len, paged_kv_indices)
         total = int(qo_indptr[-1])
         self.n_rows = total
         self.n_rows_padded = total if n_rows_padded is None else n_rows_padded
@@ -98,9 +120,7 @@ class FlashInferPrefillWrapper(_PagedWrapper):
 class FlashInferDecodeWrapper(_PagedWrapper):
     def plan(self, paged_kv_indptr, paged_kv_indices, paged_kv_last_page_len, dtype: torch.dtype = torch.bfloat16):
         n_req = len(paged_kv_last_page_len)
-        ip = self._upload(self.d_indptr, paged_kv_indptr)
-        ix = self._upload(self.d_indices, paged_kv_indices)
-        la = self._upload(self.d_last, paged_kv_last_page_len)
+        _, ip, la, ix = self._upload_tables(None, paged_kv_indptr, paged_kv_last_page_len, paged_kv_indices)
         self.batch_size = n_req
         self.n_rows = self.n_rows_padded = n_req
         self.paged_kv_indptr, self.paged_kv_indices = paged_kv_indptr, paged_kv_indices

@@ -665,6 +665,29 @@ def test_sampler_quotients(ops, penalty):
         assert (ops.sample(pair, "greedy", rep_cache=mark, penalty=penalty) == 0).all()
 
 
+@pytest.mark.parametrize("V", [1, 3, 4, 6, 2047, 4098, 40964, 81925, 156940])
+@pytest.mark.parametrize("strategy", ["greedy", "top_p", "top_k_top_p", "min_p"])
+def test_sampler_row_layouts(ops, V, strategy):
+    """Rows on every boundary -- read four tokens, two, or one at a time -- give the same tokens; values that the quotient cannot take from the
+    reciprocal, infinities and NaNs among them; the first unit, a remainder of every size, a last thread without a token."""
+    g = torch.Generator("cuda").manual_seed(V)
+    R = 5
+    x = (torch.randn(R, V, generator=g, device="cuda") * 3).bfloat16()
+    if V > 6:
+        x[0, 1], x[1, 2], x[2, 3], x[3, :5], x[4, V - 1] = 0.0, -float("inf"), float("nan"), 2.0 ** -130, 3.0e38
+        x[4, V - 2] = -3.0e38
+    cache = torch.rand(R, 2, 1, V, generator=g, device="cuda") < 0.1
+    kw = dict(top_p=0.8, top_k=7, min_p=0.05, temperature=0.6, penalty=1.3, seed=11, rep_cache=cache)
+    want = ops.sample(x, strategy, **kw)
+    for pad in (1, 2, 3, 4, 7):
+        wide = torch.full((R, V + pad), float("nan"), device="cuda").bfloat16()
+        wide[:, :V] = x
+        assert torch.equal(ops.sample(wide[:, :V], strategy, **kw), want), pad
+    if strategy == "greedy":
+        y = ops.apply_repetition_penalty(x.view(R, 1, V), cache, 1.3).view(R, V).float().nan_to_num(nan=-float("inf"), posinf=float("inf"), neginf=-float("inf"))
+        assert torch.equal(want.view(-1), y.argmax(-1))
+
+
 @pytest.mark.parametrize("rows,dim,tiled", [(1, 8, False), (3, 2040, False), (33, 2056, True), (1, 3072, True), (2, 8192, False), (2, 8200, False)])
 def test_rmsnorm_rows(ops, rows, dim, tiled):
     """Rows on 16-byte boundaries against the same rows with weights that are not, which take the general kernel."""

@@ -92,8 +92,9 @@ __device__ __forceinline__ double philox_uniform(uint64_t seed, uint64_t offset,
 // from the probability where it is needed.  Every pass is then a short loop over the thread's pairs: with the keys in registers the
 // passes had to be unrolled forty tokens deep, and reading that code once took longer than running it (top-p, cold: 32 rows of 2,051
 // tokens 61 us against 18 here; 32 rows of 156,940 tokens in a row of calls 53 against 39, and 67 with 1024 threads that spilled).
-// Above that row's 2.3 us of traffic it now spends 16 us on launch, load latency and the largest key, 15 on the two exponentials a
-// token, and 10 on the draws.
+// A row's time (28 us in a row of calls, of which 2.3 are traffic) goes to the loads and the first loop (8 us), the two exponentials a token
+// and the conversions to masses (6: those units take 8 cycles a warp), and a microsecond and more for each meeting of the cluster: six where the
+// first draw is accepted.
 constexpr int SMP_THREADS = 1024;        // (cta, thread, pair) order of the tokens
 constexpr int SMP_PAIRS = 20;            // 40 tokens per thread: 40960 tokens per CTA, 327680 per 8-CTA cluster
 constexpr int SMP_MAX_CLUSTER = 8;
@@ -201,26 +202,34 @@ __device__ __forceinline__ unsigned long long block_excl_scan(unsigned long long
   return res;
 }
 
-// a / b to the nearest, for one divisor of many dividends: quotient by the correctly rounded reciprocal and two corrections by the
+// the division, out of line: hardly any token needs it
+__device__ __noinline__ float smp_quotient(float a, float b) { return a / b; }
+// a / b to the nearest with y = 1 / b, for one divisor of many dividends: quotient by the correctly rounded reciprocal and two corrections by the
 // exact remainder (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34, 1990).
-// Dividends or divisors far from 1, zeros (the remainder loses their sign), infinities and NaNs take the division itself.
-struct SmpDiv {
-  float b, y;
-  bool fast;
-  __device__ __forceinline__ explicit SmpDiv(float d) : b(d), y(1.f / d), fast(d > 0x1p-40f && d < 0x1p40f) {}
-  __device__ __forceinline__ float operator()(float a) const {
-    float q = a * y;
-    q = fmaf(fmaf(-q, b, a), y, q);
-    q = fmaf(fmaf(-q, b, a), y, q);
-    const float m = fabsf(a);
-    if (!(fast && m > 0x1p-60f && m < 0x1p60f)) q = a / b;
-    return q;
-  }
-};
+// `far` grows past SMP_FAR where the product leaves [2^-79, 2^81): extreme dividends, zeros (the remainder loses their sign), infinities
+// and NaNs.  Those take the division itself.  (The quotients of bf16 values by one of few bits lie on the middle of two bf16 values so often
+// that asking whether the product's rounding is sure costs more than the corrections.)
+constexpr uint32_t SMP_FAR = 0xa0000000u;
+__device__ __forceinline__ float smp_div(float a, float b, float y, uint32_t& far) {
+  float q = a * y;
+  far = max(far, (__float_as_uint(q) << 1) - 0x30000000u);
+  q = fmaf(fmaf(-q, b, a), y, q);
+  return fmaf(fmaf(-q, b, a), y, q);
+}
+__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
 // the two keys of a pair of bf16 codes, and back (bf16_key / key_value on both halves at once)
 __device__ __forceinline__ uint32_t key_pair(uint32_t bits) {
   const uint32_t neg = (bits >> 15) & 0x00010001u;
   return bits ^ (0x80008000u | neg * 0x7fffu);
+}
+// the value of a token's word whose low half is zero
+__device__ __forceinline__ float word_value(uint32_t t) {
+  const uint32_t m = static_cast<uint32_t>(~static_cast<int32_t>(t) >> 31);          // all ones where the key is a negative value's
+  return __uint_as_float(t ^ (0x80000000u | (m & 0x7fff0000u)));
 }
 // a probability (bf16 in the low half of a token's word) as a mass: floor(p 2^32), saturating at 2^32 - 1
 __device__ __forceinline__ uint32_t smp_mass(uint32_t word) { return __float2uint_rz(bf16_lo(word) * 4294967296.f); }
@@ -238,10 +247,10 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
   pdl_sync();
 
   // ---- one pass over the row: keys (0 = no token / NaN) ----
-  // Load latency first: ten token pairs at a time -- one 32-bit load for the two logits, one 16-bit load for their repetition flags,
-  // all in flight together -- and only then finished (penalty, mask, temperature: same operations and rounding points as
-  // token_value()).  Rows whose layout does not allow the paired loads (odd leading dimension / vocabulary, unaligned base) take the
-  // scalar path.  A thread reads back only what it wrote itself.
+  // Load latency first: a thread takes up to ten units of four neighbouring tokens -- one 64-bit load for the logits, one 32-bit load for
+  // their repetition flags, all of them in flight together -- and only then finishes them (penalty, mask, temperature: same operations and
+  // rounding points as token_value()) in a loop of one unit, whose code is short.  Rows off these boundaries are read by pairs, or token by
+  // token.  32 rows of 156,940 tokens, cold: 14.3 us with pairs in two turns of straight-line code, 8.7 now.
   const __nv_bfloat16* lrow = p.logits + static_cast<size_t>(row) * p.ld;
   const uint8_t* rep0 = nullptr;
   size_t rep_wstride = 0;
@@ -252,76 +261,98 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
     rep_wstride = static_cast<size_t>(p.C_cache) * p.vocab;
     rep0 = p.rep_cache + (static_cast<size_t>(b) * p.W * p.C_cache + cc) * p.vocab;
   }
-  const bool paired = ((p.ld | p.vocab) & 1) == 0 && (reinterpret_cast<uintptr_t>(lrow) & 3) == 0 &&
-                      ((reinterpret_cast<uintptr_t>(rep0) | rep_wstride) & 1) == 0;
+  const uintptr_t odd = (reinterpret_cast<uintptr_t>(lrow) >> 1) | static_cast<uintptr_t>(p.vocab) | reinterpret_cast<uintptr_t>(rep0) | rep_wstride;
+  const bool wide = (odd & 3) == 0, even = (odd & 1) == 0;
   const int n_seen = rep0 ? p.W : 0;
-  const SmpDiv by_penalty(p.penalty), by_temperature(scaled ? p.temperature : 1.f);
-  auto tok_index = [&](int j, int half) { return 2 * ((j * S + rank) * SMP_THREADS + tid) + half; };
-  constexpr int SMP_BATCH = 10;
+  const float inv_temperature = 1.f / p.temperature;
+  const uint32_t far_temperature = p.temperature > 0x1p-40f && p.temperature < 0x1p40f ? 0u : SMP_FAR;
   uint32_t kloc = 0u;
-#pragma unroll 1
-  for (int j0 = 0; j0 < npairs; j0 += SMP_BATCH) {
-    uint32_t lw[SMP_BATCH], sb[SMP_BATCH];
-    if (paired) {
+  auto tok_index = [&](int j, int half) { return 2 * ((j * S + rank) * SMP_THREADS + tid) + half; };
+  {
+    constexpr int UNITS = SMP_PAIRS / 2;
+    const int n_units = npairs * (SMP_THREADS / 2);
+    auto unit_token = [&](int u) {         // first token of unit u: pairs 2 u and 2 u + 1 of the CTA, in (pair, thread) order
+      return 2 * (((2 * u / SMP_THREADS) * S + rank) * SMP_THREADS + 2 * u % SMP_THREADS);
+    };
+    // as they come, into the place of their keys: the loop that finishes them is a short one
+    if (even) {
+      uint2 lw[UNITS];
+      uint32_t sb[UNITS];
 #pragma unroll
-      for (int jj = 0; jj < SMP_BATCH; ++jj) {
-        const int i0 = tok_index(j0 + jj, 0);
-        const bool in = j0 + jj < npairs && i0 < p.vocab;
-        lw[jj] = in ? __ldg(reinterpret_cast<const uint32_t*>(lrow + i0)) : 0u;
-        sb[jj] = in && n_seen ? __ldg(reinterpret_cast<const unsigned short*>(rep0 + i0)) : 0u;
-      }
-#pragma unroll 1
-      for (int w = 1; w < n_seen; ++w) {
-        const uint8_t* rw = rep0 + w * rep_wstride;
-#pragma unroll
-        for (int jj = 0; jj < SMP_BATCH; ++jj) {
-          const int i0 = tok_index(j0 + jj, 0);
-          if (j0 + jj < npairs && i0 < p.vocab) sb[jj] |= __ldg(reinterpret_cast<const unsigned short*>(rw + i0));
+      for (int q = 0; q < UNITS; ++q) {
+        const int u = q * SMP_THREADS + tid, i0 = unit_token(u);
+        const bool in = u < n_units && i0 < p.vocab;
+        if (wide) {
+          lw[q] = in ? __ldg(reinterpret_cast<const uint2*>(lrow + i0)) : make_uint2(0u, 0u);
+          sb[q] = in && n_seen ? __ldg(reinterpret_cast<const uint32_t*>(rep0 + i0)) : 0u;
+        } else {
+          const bool in2 = in && i0 + 2 < p.vocab;
+          lw[q].x = in ? __ldg(reinterpret_cast<const uint32_t*>(lrow + i0)) : 0u;
+          lw[q].y = in2 ? __ldg(reinterpret_cast<const uint32_t*>(lrow + i0 + 2)) : 0u;
+          sb[q] = in && n_seen ? __ldg(reinterpret_cast<const unsigned short*>(rep0 + i0)) : 0u;
+          if (in2 && n_seen) sb[q] |= static_cast<uint32_t>(__ldg(reinterpret_cast<const unsigned short*>(rep0 + i0 + 2))) << 16;
         }
       }
-    } else {
 #pragma unroll
-      for (int jj = 0; jj < SMP_BATCH; ++jj) {
-        const int i0 = tok_index(j0 + jj, 0);
-        lw[jj] = sb[jj] = 0u;
-        if (j0 + jj < npairs && i0 < p.vocab) {
-          const bool two = i0 + 1 < p.vocab;
-          lw[jj] = __ldg(reinterpret_cast<const unsigned short*>(lrow + i0));
-          if (two) lw[jj] |= static_cast<uint32_t>(__ldg(reinterpret_cast<const unsigned short*>(lrow + i0 + 1))) << 16;
-          for (int w = 0; w < n_seen; ++w) {
-            sb[jj] |= __ldg(rep0 + w * rep_wstride + i0);
-            if (two) sb[jj] |= static_cast<uint32_t>(__ldg(rep0 + w * rep_wstride + i0 + 1)) << 8;
-          }
-        }
+      for (int q = 0; q < UNITS; ++q) {
+        const int u = q * SMP_THREADS + tid;
+        if (u < n_units) *reinterpret_cast<uint4*>(&tok_sm[2 * u]) = make_uint4(lw[q].x, lw[q].y, sb[q], 0u);
       }
     }
-#pragma unroll
-    for (int jj = 0; jj < SMP_BATCH; ++jj) {
-      if (j0 + jj < npairs) {
-        const int i0 = tok_index(j0 + jj, 0);
-        float l[2] = {bf16_lo(lw[jj]), bf16_hi(lw[jj])};
-        if (sb[jj]) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-            if (sb[jj] >> (8 * h) & 0xffu) l[h] = round_bf16(l[h] > 0.f ? by_penalty(l[h]) : l[h] * p.penalty);   // sampling.py:143-144
+    uint32_t kmax2 = 0u;                   // of the even tokens and of the odd ones
+    int i0 = unit_token(tid);
+#pragma unroll 1
+    for (int u = tid; u < n_units; u += SMP_THREADS, i0 += 4 * S * SMP_THREADS) {
+      uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+      if (even) {
+        raw = *reinterpret_cast<const uint4*>(&tok_sm[2 * u]);
+        for (int w = 1; w < n_seen; ++w)
+          for (int h = 0; h < 4 && i0 + h < p.vocab; h += 2)
+            raw.z |= static_cast<uint32_t>(__ldg(reinterpret_cast<const unsigned short*>(rep0 + w * rep_wstride + i0 + h))) << (8 * h);
+      } else {
+        for (int h = 0; h < 4 && i0 + h < p.vocab; ++h) {
+          const uint32_t l = __ldg(reinterpret_cast<const unsigned short*>(lrow + i0 + h)) << (16 * (h & 1));
+          (h < 2 ? raw.x : raw.y) |= l;
+          for (int w = 0; w < n_seen; ++w) raw.z |= static_cast<uint32_t>(__ldg(rep0 + w * rep_wstride + i0 + h)) << (8 * h);
         }
-        if ((i0 ^ p.mask_token) >> 1 == 0) {
-          if (p.mask_token & 1) l[1] = -INFINITY; else l[0] = -INFINITY;
-        }
-        if (scaled) {
-          l[0] = by_temperature(l[0]);
-          l[1] = by_temperature(l[1]);
-        }
-        uint32_t keep = 0u;
-        if (i0 < p.vocab) {
-          if (l[0] == l[0]) keep = 0xffffu;
-          if (i0 + 1 < p.vocab && l[1] == l[1]) keep |= 0xffff0000u;
-        }
-        const uint32_t keys = key_pair(pack_bf16(l[0], l[1])) & keep;
-        tok_sm[(j0 + jj) * SMP_THREADS + tid] = make_uint2(keys << 16, keys & 0xffff0000u);
-        kloc = max(kloc, max(keys & 0xffffu, keys >> 16));
       }
+      float l[4] = {bf16_lo(raw.x), bf16_hi(raw.x), bf16_lo(raw.y), bf16_hi(raw.y)};
+      if (raw.z) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          if (raw.z >> (8 * h) & 0xffu) l[h] = round_bf16(l[h] > 0.f ? smp_quotient(l[h], p.penalty) : l[h] * p.penalty);   // sampling.py:143-144
+      }
+      if (static_cast<uint32_t>(p.mask_token - i0) < 4u) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          if (p.mask_token - i0 == h) l[h] = -INFINITY;
+      }
+      if (scaled) {
+        float s[4];
+        uint32_t far = far_temperature;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) s[h] = smp_div(l[h], p.temperature, inv_temperature, far);
+        if (far >= SMP_FAR) {
+#pragma unroll
+          for (int h = 0; h < 4; ++h) s[h] = smp_quotient(l[h], p.temperature);
+        }
+#pragma unroll
+        for (int h = 0; h < 4; ++h) l[h] = s[h];
+      }
+      uint32_t k0 = key_pair(pack_bf16(l[0], l[1])), k1 = key_pair(pack_bf16(l[2], l[3]));
+      const float any_nan = (l[0] + l[1]) + (l[2] + l[3]);
+      if (any_nan != any_nan || i0 + 4 > p.vocab) {          // (a sum of both infinities is looked at as well)
+        uint32_t keep[2] = {0u, 0u};
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          if (i0 + h < p.vocab && l[h] == l[h]) keep[h >> 1] |= h & 1 ? 0xffff0000u : 0xffffu;
+        k0 &= keep[0];
+        k1 &= keep[1];
+      }
+      *reinterpret_cast<uint4*>(&tok_sm[2 * u]) = make_uint4(k0 << 16, k0 & 0xffff0000u, k1 << 16, k1 & 0xffff0000u);
+      kmax2 = max_u16x2(max_u16x2(kmax2, k0), k1);
     }
+    kloc = max(kmax2 & 0xffffu, kmax2 >> 16);
   }
 
   // ---- max key ----
@@ -368,12 +399,13 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
   // ---- softmax denominator (fp32) ----
   const float xmax = key_value(kmax);
   float zpart = 0.f;
+  const uint32_t z_word = max(z_floor, 1u) << 16;          // (key 0: no token)
 #pragma unroll 4
   for (int j = 0; j < npairs; ++j) {
     const uint2 t = tok_sm[j * SMP_THREADS + tid];
-    const uint32_t a = t.x >> 16, b = t.y >> 16;
-    if (a != 0u && a >= z_floor) zpart += smp_ex2((key_value(a) - xmax) * kLog2e);
-    if (b != 0u && b >= z_floor) zpart += smp_ex2((key_value(b) - xmax) * kLog2e);
+    const float ex = smp_ex2((word_value(t.x) - xmax) * kLog2e), ey = smp_ex2((word_value(t.y) - xmax) * kLog2e);
+    if (t.x >= z_word) zpart += ex;
+    if (t.y >= z_word) zpart += ey;
   }
   const float Z = smp_sum_f32(zpart, c);
   const float log2Z = log2f(Z);
@@ -381,22 +413,41 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
   // ---- probabilities: bf16-rounded softmax output; filtered tokens get 0 ----
   const uint32_t keep_floor = (p.strategy == 1 || p.strategy == 3) ? k_floor : 0u;
   const float minp_thr = (p.strategy == 4) ? p.min_p * round_bf16(smp_ex2(-log2Z)) : 0.f;
-  auto probability = [&](uint32_t k) -> uint32_t {
+  const uint32_t keep_word = max(max(z_floor, keep_floor), 1u) << 16;
+  auto probability = [&](uint32_t t) {
     // softmax output e^(x - max) / Z as ONE exponential: 2^((x - max) log2 e - log2 Z)
-    const float pr = round_bf16(smp_ex2((key_value(k) - xmax) * kLog2e - log2Z));
-    return k != 0u && k >= z_floor && k >= keep_floor && pr >= minp_thr ? __float_as_uint(pr) >> 16 : 0u;
+    const float e = smp_ex2((word_value(t) - xmax) * kLog2e - log2Z);
+    return t >= keep_word ? e : 0.f;
   };
   unsigned long long mine = 0ull;           // this thread's share of the candidates' mass
 #pragma unroll 4
   for (int j = 0; j < npairs; ++j) {
     uint2 t = tok_sm[j * SMP_THREADS + tid];
-    t.x |= probability(t.x >> 16);
-    t.y |= probability(t.y >> 16);
+    uint32_t pr = pack_bf16(probability(t.x), probability(t.y));
+    if (p.strategy == 4) pr = (bf16_lo(pr) >= minp_thr ? pr & 0xffffu : 0u) | (bf16_hi(pr) >= minp_thr ? pr & 0xffff0000u : 0u);
+    t.x = __byte_perm(pr, t.x, 0x7610);
+    t.y = __byte_perm(pr, t.y, 0x7632);
     tok_sm[j * SMP_THREADS + tid] = t;
-    mine += smp_mass(t.x);
-    mine += smp_mass(t.y);
+    mine += smp_mass(pr);
+    mine += __float2uint_rz(bf16_hi(pr) * 4294967296.f);
   }
-  unsigned long long Mc = smp_reduce<SMP_SUM>(mine, c);   // mass of the current candidate set
+  // prefixes of the masses over the cluster in (cta, thread, pair) order, and their sum: the candidates' mass
+  unsigned long long Mc, lo;
+  auto prefix = [&](unsigned long long v) {
+    unsigned long long cta_total;
+    const unsigned long long excl = block_excl_scan(v, sh, &cta_total);
+    if (tid < 32) c.publish(cta_total);
+    c.sync();
+    unsigned long long base = 0ull, total = 0ull;
+    for (int r = 0; r < S; ++r) {
+      if (r == rank) base = total;
+      total += c.xch[c.buf][r];
+    }
+    c.buf ^= 1;
+    lo = base + excl;
+    return total;
+  };
+  Mc = prefix(mine);
   const uint64_t seed = p.rng_state ? p.rng_state[0] : p.seed;
   const uint64_t offset = p.rng_state ? p.rng_state[1] : p.offset;
   if (Mc == 0ull || !(Z > 0.f)) {
@@ -412,18 +463,10 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
     unsigned long long result = 0ull;
 #pragma unroll 1
     for (uint32_t round = 0; round < 64u; ++round) {
-      // inverse CDF over the candidates in (cta, thread, pair) order
-      unsigned long long cta_total;
-      const unsigned long long excl = block_excl_scan(mine, sh, &cta_total);
-      if (tid < 32) c.publish(cta_total);
-      c.sync();
-      unsigned long long base = 0ull;
-      for (int r = 0; r < rank; ++r) base += c.xch[c.buf][r];
-      c.buf ^= 1;
+      // inverse CDF over the candidates
       const double u = philox_uniform(seed, offset, static_cast<uint32_t>(row), round);
       unsigned long long target = static_cast<unsigned long long>(u * static_cast<double>(Mc));
       if (target >= Mc) target = Mc - 1;
-      const unsigned long long lo = base + excl;
       if (mine != 0ull && lo <= target && target < lo + mine) {
         unsigned long long run = lo;
         unsigned long long found = 0ull;
@@ -457,7 +500,7 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
         if ((t.x >> 16) > kj) mine += smp_mass(t.x);
         if ((t.y >> 16) > kj) mine += smp_mass(t.y);
       }
-      const unsigned long long above = smp_reduce<SMP_SUM>(mine, c);
+      const unsigned long long above = prefix(mine);
       if (above < P) break;                  // j is inside the nucleus: accept
       pivot = kj;                            // nothing with p <= p_j is: drop it and redraw
       Mc = above;

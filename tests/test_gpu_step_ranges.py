@@ -1,4 +1,6 @@
 """Kernels of a step at the edges of their ranges: first and last sizes of a tile or a dispatch rule, remainders, odd sizes."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -411,6 +413,57 @@ def test_channels_last_depthwise_and_last(B, T, C, dil, lo, hi, big):
     last = _cl.last_conv(xs, w, b[:1], 7, 3, lo, hi, tanh=False)
     ref = torch.nn.functional.conv1d(x.double().transpose(1, 2), w.double()[None], b[:1].double(), padding=3)[..., lo:hi]
     _close(last, ref, 5e-6)
+
+
+@pytest.mark.parametrize("B,T,C,ksize,left,lo,hi", [(1, 1, 64, 3, 2, 0, 1), (2, 129, 96, 3, 2, 0, 129), (3, 40, 4, 3, 0, 5, 38), (1, 300, 256, 7, 3, 1, 300), (2, 17, 68, 5, 4, 0, 17),
+                                                   (1, 130, 128, 16, 15, 0, 130), (2, 16, 32, 1, 0, 0, 16)])
+def test_channels_last_one_output_channel(B, T, C, ksize, left, lo, hi):
+    """Runs of sixteen positions with and without rows before and behind the sequence; a position's sum is the same wherever it lies."""
+    from vox_serve_b200.tokenizer import _cl
+
+    g = torch.Generator(device="cuda").manual_seed(T + C)
+    x, w, b = (torch.randn(*n, generator=g, device="cuda") for n in ((B, T, C), (C, ksize), (1,)))
+    act = _cl.Act(x.reshape(-1).clone(), B, T, C)
+    y = _cl.last_conv(act, w, b, ksize, left, lo, hi, tanh=False)
+    ref = torch.nn.functional.conv1d(torch.nn.functional.pad(x.double().transpose(1, 2), (left, ksize - 1)), w.double()[None], b.double())[..., lo:hi]
+    _close(y, ref, 2e-6)                       # chains of at most 4 * ksize * C / 64 roundings and four additions
+    if hi - lo > 3:
+        assert torch.equal(_cl.last_conv(act, w, b, ksize, left, lo + 3, hi, tanh=False), y[..., 3:])
+
+
+@pytest.mark.parametrize("B,T,H,D,parts", [(1, 1, 1, 4, False), (2, 20, 8, 64, True), (1, 33, 2, 32, True), (2, 64, 3, 128, True), (1, 64, 1, 256, True), (3, 31, 2, 36, False), (1, 9, 2, 68, False)])
+def test_vocoder_chunk_attention_and_norm(B, T, H, D, parts):
+    from vox_serve_b200._lib import call
+    from vox_serve_b200.tokenizer import _cl
+
+    C, period = H * D, 1e4
+    g = torch.Generator(device="cuda").manual_seed(T + D)
+    buf = torch.randn(B * T * 3 * C + 2, generator=g, device="cuda")
+    for at in (0, 2):                          # rows on 16- and on 8-byte boundaries
+        qkv = buf[at:at + B * T * 3 * C].view(B, T, 3, H, D)
+        out = _cl.Act.empty(B, T, C, "cuda", parts)
+        call("vb_cl_chunk_attention_parts", out.ptr, out.codes, qkv.data_ptr(), B, C, H, T, period, 0)
+        torch.cuda.synchronize()
+        got = _cl.conv(out, _cl.pack(torch.eye(C, device="cuda")), C).tensor() if parts else out.tensor()
+        angle = torch.arange(T, device="cuda")[:, None].double() * torch.exp(torch.arange(D // 2, device="cuda").double() * (-math.log(period) * 2 / D))
+        rot = torch.polar(torch.ones_like(angle), angle)
+        turn = lambda t: torch.view_as_real(torch.view_as_complex(t.double().reshape(B, T, H, D // 2, 2).contiguous()) * rot[:, None]).flatten(-2)   # noqa: E731
+        q, k, v = turn(qkv[:, :, 0]), turn(qkv[:, :, 1]), qkv[:, :, 2].double()
+        s = torch.einsum("bqhd,bkhd->bhqk", q, k) * D ** -0.5
+        s = s.masked_fill(torch.ones(T, T, device="cuda").triu(1).bool(), -math.inf).softmax(-1)
+        _close(got, torch.einsum("bhqk,bkhd->bqhd", s, v).reshape(B, T, C), 5e-6)       # scores of a few units: their roundings reach the weights
+    x, w, b = torch.randn(B * T, C, generator=g, device="cuda") + 3, *torch.randn(2, C, generator=g, device="cuda")
+    if C <= 1024:
+        y = _cl.Act.empty(B, T, C, "cuda")
+        call("vb_cl_layernorm_parts", y.ptr, None, x.data_ptr(), w.contiguous().data_ptr(), b.contiguous().data_ptr(), B * T, C, 1e-5, 0)
+        torch.cuda.synchronize()
+        _close(y.tensor().reshape(B * T, C), torch.nn.functional.layer_norm(x.double(), (C,), w.double(), b.double(), 1e-5), 2e-6)
+    if T > 2:                                  # a value that is not a number stays out of the positions before it
+        buf[2 * C * 3 + 2 * C] = math.nan
+        out = _cl.Act.empty(B, T, C, "cuda")
+        call("vb_cl_chunk_attention_parts", out.ptr, None, buf.data_ptr(), B, C, H, T, period, 0)
+        torch.cuda.synchronize()
+        assert torch.isfinite(out.tensor()[0, :2]).all() and torch.isnan(out.tensor()[0, 2:, 0]).all()
 
 
 # prompt rows of window attention on tcgen05: head sizes, heads per key head (rows per tile), page sizes down to one 8-token group, row

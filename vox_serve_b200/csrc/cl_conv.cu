@@ -1224,39 +1224,69 @@ __global__ void __launch_bounds__(256) cl_dwconv7_kernel(float* __restrict__ y, 
 // ------------------------------------------------------------------------------------------
 // last convolution of a decoder: one output channel, ksize taps, `left` positions of context before; optional tanh
 // ------------------------------------------------------------------------------------------
-constexpr int LC_T = 128;
-__global__ void __launch_bounds__(LC_T) cl_last_conv_kernel(float* __restrict__ y, const float* __restrict__ x, long long x_bstride,
+// Bound by reading x once: sixteen lanes hold sixteen positions, four channels a lane, rows straight from global memory in whole lines and all in
+// flight (taps known: 18 rows for 3 taps); sixteen sums a lane then change places in fifteen exchanges, a position a lane.  Against rows staged in
+// shared memory and read again for every tap: 32 x 2,048 positions of 64 channels, 7 taps 16.5 us -> 10.9 in a row of calls; 32 x 19,200 positions,
+// 3 taps 59 us -> 57, where the kernel in front leaves 157 MB that L2 still has to write back.
+constexpr int LC_T = 128, LC_RUN = 16;
+template <int KSIZE>          // 0: any
+__global__ void __launch_bounds__(LC_T, 4) cl_last_conv_kernel(float* __restrict__ y, const float* __restrict__ x, long long x_bstride,
                                                             const float* __restrict__ w, const float* __restrict__ bias, int C,
                                                             int T, int ksize, int left, int t0, int t1, int use_tanh) {
-  extern __shared__ float lsm[];            // [ksize][C] weights, then [LC_T + ksize - 1][C + 4] rows
-  float* ws = lsm;
-  float* xs = lsm + ksize * C;
-  const int b = blockIdx.y, tb = t0 + blockIdx.x * LC_T, ld = C + 4, rows = min(LC_T, t1 - tb) + ksize - 1, c4n = C >> 2;
-  for (int i = threadIdx.x; i < ksize * C; i += LC_T) ws[i] = __ldg(&w[(i % C) * ksize + i / C]);
-  const float bv = __ldg(bias);
-  pdl_sync();
+  // the last rows first: they are what the kernel in front left in L2
+  const int b = gridDim.y - 1 - blockIdx.y, lane = threadIdx.x & 15, tb = t0 + (gridDim.x - 1 - blockIdx.x) * LC_T + (threadIdx.x >> 4) * LC_RUN;
   const float* xb = x + static_cast<size_t>(b) * x_bstride;
-  for (int i = threadIdx.x; i < rows * c4n; i += LC_T) {
-    const int r = i / c4n, c = i - r * c4n, t = tb - left + r;
-    *reinterpret_cast<float4*>(xs + r * ld + c * 4) =
-        (t >= 0 && t < T) ? __ldcg(reinterpret_cast<const float4*>(xb + static_cast<size_t>(t) * C) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  __syncthreads();
-  const int t = tb + threadIdx.x;
-  if (t >= t1) return;
-  float a0 = bv, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-  for (int k = 0; k < ksize; ++k) {
-    const float4* xr = reinterpret_cast<const float4*>(xs + (threadIdx.x + k) * ld);
-    const float4* wr = reinterpret_cast<const float4*>(ws + k * C);
-    for (int c = 0; c < c4n; ++c) {
-      const float4 v = xr[c], q = wr[c];
-      a0 += v.x * q.x;
-      a1 += v.y * q.y;
-      a2 += v.z * q.z;
-      a3 += v.w * q.w;
+  float acc[LC_RUN] = {};
+  auto tap = [&](int c, int k) {
+    return c < C ? make_float4(__ldg(w + (c + 0) * ksize + k), __ldg(w + (c + 1) * ksize + k), __ldg(w + (c + 2) * ksize + k), __ldg(w + (c + 3) * ksize + k))
+                 : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  auto row = [&](int c, int t) {
+    return c < C && t >= 0 && t < T ? __ldcg(reinterpret_cast<const float4*>(xb + static_cast<size_t>(t) * C + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  auto add = [](float& a, const float4& v, const float4& q) { a = fmaf(v.w, q.w, fmaf(v.z, q.z, fmaf(v.y, q.y, fmaf(v.x, q.x, a)))); };
+  const float bv = __ldg(bias);
+  if constexpr (KSIZE > 0) {
+    float4 wk[KSIZE];
+#pragma unroll
+    for (int k = 0; k < KSIZE; ++k) wk[k] = tap(lane * 4, k);
+    pdl_sync();
+    for (int c = lane * 4;;) {
+      if (tb < t1) {
+#pragma unroll
+        for (int r = 0; r < LC_RUN + KSIZE - 1; ++r) {
+          const float4 v = row(c, tb - left + r);
+#pragma unroll
+          for (int k = 0; k < KSIZE; ++k)
+            if (r - k >= 0 && r - k < LC_RUN) add(acc[r - k], v, wk[k]);
+        }
+      }
+      if ((c += 64) - lane * 4 >= C) break;
+#pragma unroll
+      for (int k = 0; k < KSIZE; ++k) wk[k] = tap(c, k);
+    }
+  } else {
+    pdl_sync();
+    for (int c = lane * 4; tb < t1 && c - lane * 4 < C; c += 64) {
+      for (int k = 0; k < ksize; ++k) {
+        const float4 q = tap(c, k);
+#pragma unroll
+        for (int j = 0; j < LC_RUN; ++j) add(acc[j], row(c, tb - left + j + k), q);
+      }
     }
   }
-  const float o = (a0 + a1) + (a2 + a3);
+#pragma unroll
+  for (int o = LC_RUN / 2; o; o >>= 1) {           // (the two halves of a sum are added in the same order for every position)
+    const bool up = lane & o;
+#pragma unroll
+    for (int j = 0; j < o; ++j) {
+      const float give = up ? acc[j] : acc[j + o], keep = up ? acc[j + o] : acc[j];
+      acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  const int t = tb + lane;
+  if (t >= t1) return;
+  const float o = acc[0] + bv;
   y[static_cast<size_t>(b) * (t1 - t0) + (t - t0)] = use_tanh ? tanhf(o) : o;
 }
 
@@ -1272,6 +1302,7 @@ __global__ void __launch_bounds__(256) cl_from_codes_kernel(float* __restrict__ 
   const int32_t* codes[3] = {c0, c1, c2};
   const int strides[3] = {s0, s1, s2};
   __shared__ float e[3][16];
+  const bool wide = cb_dim % 4 == 0 && reinterpret_cast<uintptr_t>(pw) % 16 == 0;
   pdl_sync();
   if (threadIdx.x < 3 * cb_dim) {
     const int i = threadIdx.x / cb_dim, d = threadIdx.x % cb_dim, tl = T / strides[i];
@@ -1281,13 +1312,30 @@ __global__ void __launch_bounds__(256) cl_from_codes_kernel(float* __restrict__ 
   }
   __syncthreads();
   for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    float acc = 0.f;
+    float acc = 0.f, a[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      float a = pb[i * C + c];
-      for (int d = 0; d < cb_dim; ++d) a += pw[(static_cast<size_t>(i) * C + c) * cb_dim + d] * e[i][d];
-      acc += a;
+    for (int i = 0; i < 3; ++i) a[i] = __ldg(&pb[i * C + c]);
+    for (int d = 0; d < cb_dim; d += 4) {          // (four entries of the three rows in flight together)
+      float q[3][4];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const float* r = pw + (static_cast<size_t>(i) * C + c) * cb_dim + d;
+        if (wide) {
+          const float4 v = __ldg(reinterpret_cast<const float4*>(r));
+          q[i][0] = v.x; q[i][1] = v.y; q[i][2] = v.z; q[i][3] = v.w;
+        } else {
+#pragma unroll
+          for (int h = 0; h < 4; ++h) q[i][h] = d + h < cb_dim ? __ldg(r + h) : 0.f;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          if (d + h < cb_dim) a[i] += q[i][h] * e[i][d + h];
     }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) acc += a[i];
     z[(static_cast<size_t>(b) * T + t) * C + c] = acc;
   }
 }
@@ -1337,6 +1385,14 @@ __global__ void __launch_bounds__(256) cl_upsample_kernel(float* __restrict__ y,
 __global__ void __launch_bounds__(128) cl_layernorm_kernel(float* __restrict__ y, uint8_t* __restrict__ code, const float* __restrict__ x, const float* __restrict__ w,
                                                            const float* __restrict__ bias, int rows, int C, float eps) {
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, n4 = C >> 2;
+  float4 ww[8], bb[8];               // (read while the kernel in front still runs)
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (lane + 32 * i < n4) {
+      ww[i] = __ldg(reinterpret_cast<const float4*>(w) + lane + 32 * i);
+      bb[i] = __ldg(reinterpret_cast<const float4*>(bias) + lane + 32 * i);
+    }
+  }
   pdl_sync();
   if (row >= rows) return;
   const float4* xr = reinterpret_cast<const float4*>(x + static_cast<size_t>(row) * C);
@@ -1362,9 +1418,8 @@ __global__ void __launch_bounds__(128) cl_layernorm_kernel(float* __restrict__ y
   for (int i = 0; i < 8; ++i) {
     const int c = lane + 32 * i;
     if (c < n4) {                    // (with codes: C is a multiple of 32, alike for the eight lanes of a block)
-      const float4 ww = __ldg(reinterpret_cast<const float4*>(w) + c), bb = __ldg(reinterpret_cast<const float4*>(bias) + c);
-      const float4 o = make_float4((v[i].x - mean) * rstd * ww.x + bb.x, (v[i].y - mean) * rstd * ww.y + bb.y,
-                                   (v[i].z - mean) * rstd * ww.z + bb.z, (v[i].w - mean) * rstd * ww.w + bb.w);
+      const float4 o = make_float4((v[i].x - mean) * rstd * ww[i].x + bb[i].x, (v[i].y - mean) * rstd * ww[i].y + bb[i].y,
+                                   (v[i].z - mean) * rstd * ww[i].z + bb[i].z, (v[i].w - mean) * rstd * ww[i].w + bb[i].w);
       const size_t at = static_cast<size_t>(row) * C + 4 * c;
       if (code) cl_put4(reinterpret_cast<uint32_t*>(y), code, at, o);
       else *reinterpret_cast<float4*>(y + at) = o;
@@ -1373,81 +1428,123 @@ __global__ void __launch_bounds__(128) cl_layernorm_kernel(float* __restrict__ y
 }
 
 // causal attention inside one chunk of T <= 64 positions, rotary pairs (2j, 2j + 1); qkv [B][T][3 C] -> out [B][T][C].
-// One block per (head, batch entry): a chunk is a few dozen positions, so scores and weights stay in shared memory.
+// One block per (head, batch entry), latency bound: a chunk is a few dozen positions.  The angles do not depend on the input and are found
+// while the kernel in front still runs; a thread's rows are all in flight at once; a warp owns four queries (a key of its own per lane, so one read of
+// a key serves four sums, and the softmax needs the warp alone), and what it reads in each step of p v are the four weights of a key in
+// one load.  32 chunks of 20 positions, 8 heads of 64 dims: 15.8 us of a layer in a row of calls with a block-wide pass per stage; now 9.4.
+constexpr int CA_ROWS = 4;
 __global__ void __launch_bounds__(256) cl_chunk_attention_kernel(float* __restrict__ out, uint8_t* __restrict__ code, const float* __restrict__ qkv, int C, int H,
                                                                  int T, float max_period) {
-  extern __shared__ float asm_[];      // q, k, v [T][D + 4], p [T][T + 1], frequencies
-  const int h = blockIdx.x, b = blockIdx.y, D = C / H, ld = D + 4, half = D >> 1;
-  float* q = asm_;
+  extern __shared__ float4 asm_[];     // p [8 warps][T] of four queries, q, k, v [T][D + 4], frequencies
+  const int h = blockIdx.x, b = blockIdx.y, D = C / H, ld = D + 4, half = D >> 1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float4* p = asm_ + warp * T;
+  float* q = reinterpret_cast<float*>(asm_ + 8 * T);
   float* k = q + T * ld;
   float* v = k + T * ld;
-  float* p = v + T * ld;
-  float* freq = p + T * (T + 1);       // [D / 2]
+  float* freq = v + T * ld;            // [D / 2]
   for (int j = threadIdx.x; j < half; j += blockDim.x)
     freq[j] = expf(static_cast<float>(j) * (-logf(max_period) * 2.f / static_cast<float>(D)));
-  pdl_sync();
   __syncthreads();
   const float* base = qkv + static_cast<size_t>(b) * T * 3 * C + h * D;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < T * half; i += blockDim.x) {
-    const int t = i / half, j = i - t * half;
-    const float* row = base + static_cast<size_t>(t) * 3 * C + 2 * j;
-    const float2 a = __ldcg(reinterpret_cast<const float2*>(row)), e = __ldcg(reinterpret_cast<const float2*>(row + C)),
-                 f = __ldcg(reinterpret_cast<const float2*>(row + 2 * C));
-    float sn, cs;
-    sincosf(static_cast<float>(t) * freq[j], &sn, &cs);
-    const int o = t * ld + 2 * j;
-    q[o] = a.x * cs - a.y * sn;
-    q[o + 1] = a.x * sn + a.y * cs;
-    k[o] = e.x * cs - e.y * sn;
-    k[o + 1] = e.x * sn + e.y * cs;
-    v[o] = f.x;
-    v[o + 1] = f.y;
+  for (int i0 = threadIdx.x; i0 - static_cast<int>(threadIdx.x) < T * half; i0 += 4 * 256) {
+    float sn[4], cs[4];
+    int at[4];
+    float2 a[4], e[4], f[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * 256, t = i / half, j = i - t * half;
+      at[u] = i < T * half ? t * ld + 2 * j : -1;
+      if (at[u] >= 0) sincosf(static_cast<float>(t) * freq[j], &sn[u], &cs[u]);
+    }
+    if (i0 == static_cast<int>(threadIdx.x)) pdl_sync();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * 256, t = i / half, j = i - t * half;
+      if (at[u] < 0) continue;
+      const float* row = base + static_cast<size_t>(t) * 3 * C + 2 * j;
+      a[u] = __ldcg(reinterpret_cast<const float2*>(row));
+      e[u] = __ldcg(reinterpret_cast<const float2*>(row + C));
+      f[u] = __ldcg(reinterpret_cast<const float2*>(row + 2 * C));
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (at[u] < 0) continue;
+      *reinterpret_cast<float2*>(q + at[u]) = make_float2(a[u].x * cs[u] - a[u].y * sn[u], a[u].x * sn[u] + a[u].y * cs[u]);
+      *reinterpret_cast<float2*>(k + at[u]) = make_float2(e[u].x * cs[u] - e[u].y * sn[u], e[u].x * sn[u] + e[u].y * cs[u]);
+      *reinterpret_cast<float2*>(v + at[u]) = f[u];
+    }
   }
   __syncthreads();
   const float scale = rsqrtf(static_cast<float>(D));
   const int d4 = D >> 2;
-  for (int i = threadIdx.x; i < T * T; i += blockDim.x) {
-    const int tq = i / T, tk = i - tq * T;
-    float s = 0.f;
-    if (tk <= tq) {
-      const float4* a = reinterpret_cast<const float4*>(q + tq * ld);
-      const float4* c = reinterpret_cast<const float4*>(k + tk * ld);
-      float s1 = 0.f, s2 = 0.f, s3 = 0.f;
+  for (int t0 = warp; t0 < T; t0 += 8 * CA_ROWS) {           // queries t0, t0 + 8, ...; past the end the last one is repeated and not written
+    int tq[CA_ROWS];
+    float s[2][CA_ROWS], den[CA_ROWS], inv[CA_ROWS];
+#pragma unroll
+    for (int r = 0; r < CA_ROWS; ++r) tq[r] = min(t0 + 8 * r, T - 1);
+    const int last = tq[CA_ROWS - 1];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int tk = lane + 32 * u;
+      if (32 * u > last) break;
+      const float4* c = reinterpret_cast<const float4*>(k + min(tk, T - 1) * ld);
+      float sum[CA_ROWS][4] = {};
 #pragma unroll 4
       for (int d = 0; d < d4; ++d) {
-        const float4 x = a[d], y = c[d];
-        s += x.x * y.x;
-        s1 += x.y * y.y;
-        s2 += x.z * y.z;
-        s3 += x.w * y.w;
+        const float4 y = c[d];
+#pragma unroll
+        for (int r = 0; r < CA_ROWS; ++r) {
+          const float4 x = reinterpret_cast<const float4*>(q + tq[r] * ld)[d];
+          sum[r][0] += x.x * y.x;
+          sum[r][1] += x.y * y.y;
+          sum[r][2] += x.z * y.z;
+          sum[r][3] += x.w * y.w;
+        }
       }
-      s = (s + s1) + (s2 + s3);
+#pragma unroll
+      for (int r = 0; r < CA_ROWS; ++r) s[u][r] = ((sum[r][0] + sum[r][1]) + (sum[r][2] + sum[r][3])) * scale;
     }
-    p[tq * (T + 1) + tk] = s * scale;
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int tq = warp; tq < T; tq += 8) {
-    float mx = -INFINITY;
-    for (int tk = lane; tk <= tq; tk += 32) mx = fmaxf(mx, p[tq * (T + 1) + tk]);
-    mx = warp_max(mx);
-    float den = 0.f;
-    for (int tk = lane; tk <= tq; tk += 32) {
-      const float e = expf(p[tq * (T + 1) + tk] - mx);
-      p[tq * (T + 1) + tk] = e;
-      den += e;
+#pragma unroll
+    for (int r = 0; r < CA_ROWS; ++r) {
+      float mx = lane <= tq[r] ? s[0][r] : -INFINITY;
+      if (lane + 32 <= tq[r]) mx = fmaxf(mx, s[1][r]);
+      mx = warp_max(mx);
+      s[0][r] = lane <= tq[r] ? expf(s[0][r] - mx) : 0.f;
+      s[1][r] = lane + 32 <= tq[r] ? expf(s[1][r] - mx) : 0.f;
+      den[r] = warp_sum(s[0][r] + s[1][r]);
+      inv[r] = 1.f / den[r];
     }
-    const float inv = 1.f / warp_sum(den);
+    __syncwarp();                      // (the weights of the queries before have been read)
+    if (lane <= last) p[lane] = make_float4(s[0][0], s[0][1], s[0][2], s[0][3]);
+    if (lane + 32 <= last) p[lane + 32] = make_float4(s[1][0], s[1][1], s[1][2], s[1][3]);
     __syncwarp();
-    for (int d = lane; d < D; d += 32) {
-      float a = 0.f;
-      for (int tk = 0; tk <= tq; ++tk) a += p[tq * (T + 1) + tk] * v[tk * ld + d];
-      const size_t at = (static_cast<size_t>(b) * T + tq) * C + h * D + d;
-      if (code) cl_put1(reinterpret_cast<uint32_t*>(out), code, at >> 5, a * inv);         // (D is a multiple of 32)
-      else out[at] = a * inv;
+    for (int d0 = 0; d0 < D; d0 += 64) {
+      float o[2][CA_ROWS] = {};
+      const int d = d0 + lane, da = min(d, D - 1), db = min(d + 32, D - 1);
+#pragma unroll 4
+      for (int tk = 0; tk <= last; ++tk) {
+        const float4 w = p[tk];
+        const float x = v[tk * ld + da], y = v[tk * ld + db], ws[CA_ROWS] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int r = 0; r < CA_ROWS; ++r) {
+          if (tk <= tq[r]) {           // (a key that is not a number stays out of the queries before it)
+            o[0][r] += ws[r] * x;
+            o[1][r] += ws[r] * y;
+          }
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < CA_ROWS; ++r) {
+        if (t0 + 8 * r >= T) break;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const size_t at = (static_cast<size_t>(b) * T + tq[r]) * C + h * D + d + 32 * u;
+          if (d0 + 32 * u >= D) break;
+          if (code) cl_put1(reinterpret_cast<uint32_t*>(out), code, at >> 5, o[u][r] * inv[r]);         // (D is a multiple of 32)
+          else if (d + 32 * u < D) out[at] = o[u][r] * inv[r];
+        }
+      }
     }
-    __syncwarp();
   }
 }
 
@@ -1724,10 +1821,13 @@ int vb_cl_last_conv(float* d_y, const float* d_x, long long x_bstride, const flo
   VB_CHECK_ARG(on16(d_x), "vb_cl_last_conv: rows must start on 16-byte boundaries");
   VB_CHECK_ARG(0 <= t0 && t0 < t1 && t1 <= T, "vb_cl_last_conv: bad output range [%d, %d) of %d", t0, t1, T);
   if (B <= 0) return 0;
-  VB_CHECK_CUDA(max_dyn_smem_once(cl_last_conv_kernel));
-  const size_t smem = (static_cast<size_t>(ksize) * C + static_cast<size_t>(LC_T + ksize - 1) * (C + 4)) * sizeof(float);
-  VB_LAUNCH_PDL(cl_last_conv_kernel, dim3((t1 - t0 + LC_T - 1) / LC_T, B), LC_T, smem, stream, d_y, d_x, x_bstride, d_w, d_bias, C, T, ksize,
-                left, t0, t1, use_tanh);
+  const dim3 grid((t1 - t0 + LC_T - 1) / LC_T, B);
+  if (ksize == 3)
+    VB_LAUNCH_PDL(cl_last_conv_kernel<3>, grid, LC_T, 0, stream, d_y, d_x, x_bstride, d_w, d_bias, C, T, ksize, left, t0, t1, use_tanh);
+  else if (ksize == 7)
+    VB_LAUNCH_PDL(cl_last_conv_kernel<7>, grid, LC_T, 0, stream, d_y, d_x, x_bstride, d_w, d_bias, C, T, ksize, left, t0, t1, use_tanh);
+  else
+    VB_LAUNCH_PDL(cl_last_conv_kernel<0>, grid, LC_T, 0, stream, d_y, d_x, x_bstride, d_w, d_bias, C, T, ksize, left, t0, t1, use_tanh);
   return 0;
 }
 
@@ -1782,7 +1882,7 @@ int vb_cl_chunk_attention_parts(float* d_out, void* d_code, const float* d_qkv, 
   VB_CHECK_ARG(H >= 1 && C % H == 0 && (C / H) % 4 == 0 && C / H <= 256 && T >= 1 && T <= 64, "vb_cl_chunk_attention: C %d, H %d, T %d (<= 64)", C, H, T);
   VB_CHECK_ARG(!d_code || (C / H) % 32 == 0, "vb_cl_chunk_attention: parts need heads of a multiple of 32, not %d", C / H);
   if (B <= 0) return 0;
-  const size_t smem = (static_cast<size_t>(3) * T * (C / H + 4) + static_cast<size_t>(T) * (T + 1) + C / H / 2) * sizeof(float);
+  const size_t smem = (static_cast<size_t>(3) * T * (C / H + 4) + static_cast<size_t>(8) * T * 4 + C / H / 2) * sizeof(float);
   VB_CHECK_ARG(smem <= VB_MAX_DYN_SMEM, "vb_cl_chunk_attention: head size %d too large", C / H);
   VB_CHECK_CUDA(max_dyn_smem_once(cl_chunk_attention_kernel));
   VB_LAUNCH_PDL(cl_chunk_attention_kernel, dim3(H, B), 256, smem, stream, d_out, static_cast<uint8_t*>(d_code), d_qkv, C, H, T, max_period);

@@ -24,7 +24,7 @@
 // What bounds it (640 rows of 512 x 2048, split in four: 12.8 us, was 28.4; 5120 x 1536 x 1024: 60 us, was 161): the wide layers the bytes
 // through L2 and shared memory, 0.6 us for 64 channels and one tap of 128 x 128; the layers of many positions the epilogue's instructions,
 // some 30 per value (153600 x 128 with residual 61 us, was 71, 30 of DRAM time).
-// Measured (one pass): SNAC 32 windows 652 -> 543 us, 1 window 262 -> 246, Mimi 32 chunks 1926 -> 1333.
+// Measured (one pass): SNAC 32 windows 652 -> 532 us, 1 window 262 -> 242, Mimi 32 chunks 1926 -> 1257, the small kernels below among them.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 32
 #include "common.cuh"
@@ -948,7 +948,7 @@ __global__ void __launch_bounds__(ClRoles<PARTS>::THREADS, 1) cl_conv_kernel(con
     const int quarter = warp & 3, lane_row = quarter * 32 + lane;
     const ClHot h{p.cols, p.N, p.epi, p.act, p.y && (p.y2 || p.yp), p.epi != CE_PLAIN, p.yp != nullptr};
     ClBoxes bx{smem_u32(boxes) + (warp - FIRST_EPI) * 4096, &res_full[warp - FIRST_EPI], 0u, 0u};
-    int it = 0;
+    int it = 0, skew = 0;
     for (int u = u_first; u < p.units && !bw.dead; u += u_step, ++it) {
       const ClUnit g = cl_unit(p, u);
       const int acc = p.acc_bufs > 1 ? it & 1 : 0;
@@ -957,8 +957,13 @@ __global__ void __launch_bounds__(ClRoles<PARTS>::THREADS, 1) cl_conv_kernel(con
       const int width = min(128, p.N - g.m0), copies = cl_copies(width);        // (N is a multiple of 32)
       const int row = copies == 1 ? lane_row : lane_row & (width - 1);
       const bool mine = row < width;
-      // this warp's chunks of eight columns: every `turns`-th one
-      const int turn = ((warp - FIRST_EPI) >> 2) * copies + (copies == 4 ? quarter : copies == 2 ? quarter >> 1 : 0), turns = EPI_WARPS / 4 * copies;
+      // This warp's chunks of eight columns: every `turns`-th one.  Which warps have one more than the others goes round from unit to unit (there are
+      // two accumulators): 16 chunks for the 6 warps of 64 channels are 8 in three units instead of 3 in each.  Mimi, 32 windows in a row of calls: 614400 x 64
+      // with residual 117 -> 112 us, 614400 x 32 88 -> 84, 153600 x 256 to two outputs 114 -> 110.
+      const int turns = EPI_WARPS / 4 * copies;
+      int turn = ((warp - FIRST_EPI) >> 2) * copies + (copies == 4 ? quarter : copies == 2 ? quarter >> 1 : 0) - skew;
+      if (turn < 0) turn += turns;
+      skew = (skew + h.cols / CL_EC) % turns;
       ClEpiState e;
       e.n = g.m0 + row;
       const int nm = p.cmod == h.N ? e.n : e.n % p.cmod;

@@ -145,27 +145,45 @@ __global__ void __launch_bounds__(SS_THREADS) ssd_step_kernel(SsdParams p) {
 
 constexpr int SD_ROWS = 64;
 
-// the tile's step sizes and running log decays (warp 0; lane l holds rows l and l + 32)
-__device__ __forceinline__ void ssd_tile_decays(const SsdParams& p, int h, int row0, int L, float* dts, double* cum) {
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    const double A = -static_cast<double>(expf(p.A_log[h]));
+// A tile's step sizes and running log decays, by one warp (lane l holds rows l and l + 32).  Its loads are apart from the rest: asked for behind
+// a tile's copies they waited for all of them, and this was a third of the tile's time (4.8 of 16 us).
+struct SdSteps {
+  float dt[2], bias, log_a;
+  __device__ __forceinline__ void load(const SsdParams& p, int h, int row0, int L) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) dt[u] = lane + 32 * u < L ? p.dt[static_cast<size_t>(row0 + lane + 32 * u) * p.ld_dt + h] : 0.f;
+    bias = p.dt_bias[h];
+    log_a = p.A_log[h];
+  }
+  __device__ __forceinline__ void decays(int L, float* dts, double* cum) const {
+    const int lane = threadIdx.x & 31;
+    const double A = -static_cast<double>(expf(log_a));
     double v[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      const int r = lane + 32 * u;
-      const float dt = r < L ? sd_softplus(p.dt[static_cast<size_t>(row0 + r) * p.ld_dt + h] + p.dt_bias[h]) : 0.f;
-      dts[r] = dt;
-      v[u] = A * dt;
+      const float d = lane + 32 * u < L ? sd_softplus(dt[u] + bias) : 0.f;
+      dts[lane + 32 * u] = d;
+      v[u] = A * d;
+    }
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const double w = __shfl_up_sync(0xffffffffu, v[u], o);
-        if (lane >= o) v[u] += w;
+    for (int o = 1; o < 32; o <<= 1) {
+      const double w0 = __shfl_up_sync(0xffffffffu, v[0], o), w1 = __shfl_up_sync(0xffffffffu, v[1], o);
+      if (lane >= o) {
+        v[0] += w0;
+        v[1] += w1;
       }
     }
     const double first = __shfl_sync(0xffffffffu, v[0], 31);
     cum[lane] = v[0];
     cum[lane + 32] = first + v[1];
+  }
+};
+__device__ __forceinline__ void ssd_tile_decays(const SsdParams& p, int h, int row0, int L, float* dts, double* cum) {
+  if (threadIdx.x < 32) {
+    SdSteps st;
+    st.load(p, h, row0, L);
+    st.decays(L, dts, cum);
   }
   __syncthreads();
 }
@@ -258,9 +276,14 @@ __global__ void __launch_bounds__(256) ssd_tile_scan_kernel(SsdParams p) {
     float4 s = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(S + i);
     for (int c0 = 0; c0 < n_tiles; c0 += 8) {
       float4 uv[8];
+      float d8[8];                         // (both asked for before the first store, which the compiler keeps loads behind)
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (c0 + j < n_tiles) uv[j] = *reinterpret_cast<const float4*>(sc + (c0 + j) * step + i);
+      for (int j = 0; j < 8; ++j) {
+        if (c0 + j < n_tiles) {
+          uv[j] = *reinterpret_cast<const float4*>(sc + (c0 + j) * step + i);
+          d8[j] = dec[static_cast<size_t>(c0 + j) * p.H];
+        }
+      }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         if (c0 + j < n_tiles) {
@@ -274,7 +297,7 @@ __global__ void __launch_bounds__(256) ssd_tile_scan_kernel(SsdParams p) {
           } else {
             *reinterpret_cast<float4*>(sc + (c0 + j) * step + i) = s;
           }
-          const float d = dec[static_cast<size_t>(c0 + j) * p.H];
+          const float d = d8[j];
           s.x = fmaf(d, s.x, uv[j].x); s.y = fmaf(d, s.y, uv[j].y); s.z = fmaf(d, s.z, uv[j].z); s.w = fmaf(d, s.w, uv[j].w);
         }
       }
@@ -439,8 +462,8 @@ __device__ __forceinline__ void sd_stage(__nv_bfloat16* __restrict__ dst, int ld
 
 __global__ void __launch_bounds__(128) ssd_tile_state_mma_kernel(SsdParams p, int hb) {
   extern __shared__ __align__(16) uint8_t sd_raw[];
-  __shared__ float dts[SD_ROWS];
-  __shared__ double cum[SD_ROWS];
+  __shared__ float wgt[4][SD_ROWS];       // of the heads' rows (a warp finds a head's decays, all heads at once)
+  __shared__ double cum[4][SD_ROWS];
   pdl_sync();
   const int tile = blockIdx.x, h0 = blockIdx.y * hb, e0 = blockIdx.z * p.dvb, g = h0 / (p.H / p.G);
   const int row0 = p.tile_row0[tile], L = min(SD_ROWS, p.qo_indptr[p.tile_req[tile] + 1] - row0);
@@ -450,26 +473,46 @@ __global__ void __launch_bounds__(128) ssd_tile_state_mma_kernel(SsdParams p, in
   __nv_bfloat16* Xl = Xh + SD_ROWS * ldx;
   const __nv_bfloat16* xbc = static_cast<const __nv_bfloat16*>(p.xbc) + static_cast<size_t>(row0) * p.ld;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, vb = DV / 8;
+  SdSteps st;
+  if (warp < hb) st.load(p, h0 + warp, row0, L);
+  // a head's x, up to four pieces a thread, is asked for while the head before is multiplied
+  uint4 q[4];
+  auto fetch = [&](int h) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = tid + 128 * k, r = i / vb, c = (i - r * vb) * 8;
+      q[k] = make_uint4(0u, 0u, 0u, 0u);
+      if (i < SD_ROWS * vb && r < L) q[k] = *reinterpret_cast<const uint4*>(xbc + static_cast<size_t>(r) * p.ld + h * V + e0 + c);
+    }
+  };
+  fetch(h0);
   sd_stage(Bs, ldb, xbc + p.H * V + g * N, p.ld, N, L);
+  if (warp < hb) {
+    st.decays(L, wgt[warp], cum[warp]);
+    __syncwarp();
+    const double last = cum[warp][L - 1];
+    if (lane == 0 && blockIdx.z == 0) p.tile_decay[static_cast<size_t>(tile) * p.H + h0 + warp] = static_cast<float>(exp(last));
+#pragma unroll
+    for (int u = 0; u < 2; ++u) wgt[warp][lane + 32 * u] *= expf(static_cast<float>(last - cum[warp][lane + 32 * u]));
+  }
   for (int h = h0; h < h0 + hb; ++h) {
     __syncthreads();                      // (the last head's x is consumed)
-    ssd_tile_decays(p, h, row0, L, dts, cum);
-    const double last = cum[L - 1];
-    if (tid == 0 && blockIdx.z == 0) p.tile_decay[static_cast<size_t>(tile) * p.H + h] = static_cast<float>(exp(last));
-    for (int i = tid; i < SD_ROWS * vb; i += 128) {
-      const int r = i / vb, c = (i - r * vb) * 8;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = tid + 128 * k, r = i / vb, c = (i - r * vb) * 8;
+      if (i >= SD_ROWS * vb) continue;
       uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
       if (r < L) {
-        const float w = expf(static_cast<float>(last - cum[r])) * dts[r];
-        const uint4 q = *reinterpret_cast<const uint4*>(xbc + static_cast<size_t>(r) * p.ld + h * V + e0 + c);
-        hi.x = sd_split(w * bf16_lo(q.x), w * bf16_hi(q.x), lo.x);
-        hi.y = sd_split(w * bf16_lo(q.y), w * bf16_hi(q.y), lo.y);
-        hi.z = sd_split(w * bf16_lo(q.z), w * bf16_hi(q.z), lo.z);
-        hi.w = sd_split(w * bf16_lo(q.w), w * bf16_hi(q.w), lo.w);
+        const float w = wgt[h - h0][r];
+        hi.x = sd_split(w * bf16_lo(q[k].x), w * bf16_hi(q[k].x), lo.x);
+        hi.y = sd_split(w * bf16_lo(q[k].y), w * bf16_hi(q[k].y), lo.y);
+        hi.z = sd_split(w * bf16_lo(q[k].z), w * bf16_hi(q[k].z), lo.z);
+        hi.w = sd_split(w * bf16_lo(q[k].w), w * bf16_hi(q[k].w), lo.w);
       }
       *reinterpret_cast<uint4*>(Xh + r * ldx + c) = hi;
       *reinterpret_cast<uint4*>(Xl + r * ldx + c) = lo;
     }
+    if (h + 1 < h0 + hb) fetch(h + 1);
     __syncthreads();
     float* U = p.scratch + (static_cast<size_t>(tile) * p.H + h) * N * V + e0;
     for (int m0 = warp * 16; m0 < N; m0 += 64) {
@@ -508,6 +551,8 @@ __global__ void __launch_bounds__(128) ssd_tile_state_mma_kernel(SsdParams p, in
 }
 
 // 8 warps: warp w owns the 16 rows of w / 2 and one half of the value dims
+// Bound by latency before its traffic: of a tile's 16 us 4.8 were one warp's chain of decays behind the copies and 4.4 the gate's loads behind
+// everything.  Asked for first, and with the state kernel's heads side by side, a prompt of 1001 rows of the whole model takes 810 us, was 826.
 __global__ void __launch_bounds__(256) ssd_tile_out_mma_kernel(SsdParams p) {
   extern __shared__ __align__(16) uint8_t sd_raw[];
   __shared__ float dts[SD_ROWS], cumf[SD_ROWS];
@@ -532,6 +577,23 @@ __global__ void __launch_bounds__(256) ssd_tile_out_mma_kernel(SsdParams p) {
     }
   };
   pdl_sync();
+  // what is read last, or by one warp's chain, is asked for first: a load behind the copies waits for them
+  const int rb = warp >> 1, v0 = (warp & 1) * 32, rA = rb * 16 + (lane >> 2), rB = rA + 8;
+  SdSteps st;
+  if (warp == 0) st.load(p, h, row0, L);
+  float2 zs[2][4];
+#pragma unroll
+  for (int half = 0; half < 2; ++half)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int r = rA + 8 * half, c = v0 + n * 8 + (lane & 3) * 2;
+      zs[half][n] = make_float2(0.f, 0.f);
+      if (r < L && c < DV) {
+        const float* z = p.z + static_cast<size_t>(row0 + r) * p.ld_z + h * V + e0 + c;
+        zs[half][n] = make_float2(z[0], z[1]);
+      }
+    }
+  const float D = p.D[h];
   copy(Bs, ldb, xbc + p.H * V + g * N, p.ld, N, SD_ROWS, L);
   copy(Cs, ldb, xbc + p.H * V + p.G * N + g * N, p.ld, N, SD_ROWS, L);
   asm volatile("cp.async.commit_group;" ::: "memory");
@@ -540,12 +602,15 @@ __global__ void __launch_bounds__(256) ssd_tile_out_mma_kernel(SsdParams p) {
   copy(Sh, ldx, Sb, V, DV, N, N);
   copy(Sl, ldx, Sb + static_cast<size_t>(N) * V, V, DV, N, N);
   asm volatile("cp.async.commit_group;" ::: "memory");
-  ssd_tile_decays(p, h, row0, L, dts, cum);
-  if (tid < SD_ROWS) cumf[tid] = static_cast<float>(cum[tid]);
+  if (warp == 0) {
+    st.decays(L, dts, cum);
+    __syncwarp();
+    cumf[lane] = static_cast<float>(cum[lane]);
+    cumf[lane + 32] = static_cast<float>(cum[lane + 32]);
+  }
   asm volatile("cp.async.wait_group 1;" ::: "memory");
   __syncthreads();
   // scores of the warp's 16 rows with the rows up to its last one
-  const int rb = warp >> 1, v0 = (warp & 1) * 32;
   const __nv_bfloat16* Crow = Cs + (rb * 16 + (lane & 15)) * ldb + (lane >> 4) * 8;
   float sc[8][4];
 #pragma unroll
@@ -566,7 +631,6 @@ __global__ void __launch_bounds__(256) ssd_tile_out_mma_kernel(SsdParams p) {
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   if (v0 >= DV) return;
-  const int rA = rb * 16 + (lane >> 2), rB = rA + 8;
   float o[4][4];
 #pragma unroll
   for (int n = 0; n < 4; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
@@ -622,13 +686,11 @@ __global__ void __launch_bounds__(256) ssd_tile_out_mma_kernel(SsdParams p) {
       }
     }
   }
-  const float D = p.D[h];
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     const int r = half ? rB : rA;
     if (r >= L) continue;
     const size_t t = row0 + r;
-    const float* z = p.z + t * p.ld_z + h * V + e0;
     float* out = p.out + t * p.H * V + h * V + e0;
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
@@ -636,7 +698,7 @@ __global__ void __launch_bounds__(256) ssd_tile_out_mma_kernel(SsdParams p) {
       if (c < DV) {
         const uint32_t x = *reinterpret_cast<const uint32_t*>(Xs + r * ldx + c);
         const float y0 = fmaf(D, bf16_lo(x), o[n][2 * half]), y1 = fmaf(D, bf16_hi(x), o[n][2 * half + 1]);
-        *reinterpret_cast<float2*>(out + c) = make_float2(y0 * sd_silu(z[c]), y1 * sd_silu(z[c + 1]));
+        *reinterpret_cast<float2*>(out + c) = make_float2(y0 * sd_silu(zs[half][n].x), y1 * sd_silu(zs[half][n].y));
       }
     }
   }
@@ -794,7 +856,7 @@ int vb_ssd_tiled(float* d_out, float* d_state, float* d_scratch, const void* d_x
     while (hb < 4 && (H / G) % (2 * hb) == 0 && n_tiles * (H / (2 * hb)) * zb >= 2 * 148) hb *= 2;
     p.before = reinterpret_cast<bf16*>(d_scratch + static_cast<size_t>(n_tiles) * H * N * V);
     const dim3 mgrid(n_tiles, H / hb, zb);
-    VB_CHECK_CUDA(cudaFuncSetAttribute(ssd_tile_state_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VB_MAX_DYN_SMEM - 2048));
+    VB_CHECK_CUDA(cudaFuncSetAttribute(ssd_tile_state_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VB_MAX_DYN_SMEM - 4096));
     VB_CHECK_CUDA(cudaFuncSetAttribute(ssd_tile_out_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VB_MAX_DYN_SMEM - 2048));
     VB_LAUNCH_PDL(ssd_tile_state_mma_kernel, mgrid, 128, ssd_mma_smem1(N, p.dvb), stream, p, hb);
     VB_LAUNCH_PDL(ssd_tile_scan_kernel, scan_grid, 256, 0, stream, p);

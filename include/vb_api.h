@@ -158,12 +158,6 @@ int vb_paged_prefill_attn(void* d_out, const void* d_q, const void* d_kv, int64_
 int vb_prefill_attn_tc_timeouts(void);      /* as vb_gemm_wide_timeouts */
 int vb_window_attn_tc_timeouts(void);
 int vb_prefill_attn_tc_tile_rows(int n_q, int n_kv);
-/* ..._keys: `keys`, the cached keys of all requests (pages counted whole) where the caller knows them, 0 otherwise: portions that continue long
- * contexts share a row tile's keys between two blocks. */
-int vb_paged_prefill_attn_tc_keys(void* d_out, const void* d_q, const void* d_kv, int64_t slab_base,
-                                  const int32_t* d_qo_indptr, const int32_t* d_kv_indptr, const int32_t* d_kv_indices,
-                                  const int32_t* d_row_kvlen, int n_req, int n_rows, int n_q, int n_kv, int head_dim,
-                                  int page_size, float sm_scale, int out_xt_tile, long long keys, void* stream);
 int vb_paged_prefill_attn_tc(void* d_out, const void* d_q, const void* d_kv, int64_t slab_base,
                              const int32_t* d_qo_indptr, const int32_t* d_kv_indptr, const int32_t* d_kv_indices,
                              const int32_t* d_row_kvlen, int n_req, int n_rows, int n_q, int n_kv, int head_dim,

@@ -585,11 +585,11 @@ def test_paged_prompt_attention_pages(ops, page, D, H, G, kv, new):
     assert _lib.load().vb_prefill_attn_tc_timeouts() == 0
 
 
-# row tiles whose keys two blocks share: the fewest key tiles that are shared, a key before and behind; a second half that ends in a key tile of
-# one key, with rows of the tile that see nothing of it; boxes and rows of cp.async; both layouts of the result
+# rows on several key tiles, one key before and behind the end of a key tile; a last key tile of one key, with rows of the tile that see nothing
+# of it; boxes and rows of cp.async; both layouts of the result
 @pytest.mark.parametrize("page,tiled", [(64, True), (16, False), (20, False)])
 @pytest.mark.parametrize("D,H,G,kv,new", [(128, 6, 2, [320, 321, 384, 385], [1, 64, 100, 43]), (64, 4, 4, [449, 1000, 64], [449, 3, 2])])
-def test_paged_prompt_attention_shared_tiles(ops, page, tiled, D, H, G, kv, new):
+def test_paged_prompt_attention_several_tiles(ops, page, tiled, D, H, G, kv, new):
     from vox_serve_b200 import _lib
 
     g = torch.Generator(device="cuda").manual_seed(page + D)
@@ -608,12 +608,82 @@ def test_paged_prompt_attention_shared_tiles(ops, page, tiled, D, H, G, kv, new)
         at += new[b]
     plan = ops.RowPlan(T, "cuda")
     ops.plan_rows(plan, _i32([0] + np.cumsum(new).tolist()), _i32(ip), _i32(list(range(ip[-1]))), _i32([(x - 1) % page + 1 for x in kv]), len(kv), T,
-                  page, page, keys=ip[-1] * page)
+                  page, page)
     out = ops.TiledAct(T, H * D, "cuda") if tiled else None
     out = ops.paged_attn(q, cache, 0, plan, T, G, page, page, None, out=out, prefill_tiles="tc")
     got = out.to_rows().view(T, H, D) if tiled else out
     _close(got, torch.cat(want), 2 ** -8)            # probabilities and the output rounded to bf16
     assert _lib.load().vb_prefill_attn_tc_timeouts() == 0
+
+
+@pytest.mark.parametrize("D,H,G,kv,new,at", [(128, 6, 2, 400, 400, 1), (64, 4, 4, 700, 100, 0), (128, 8, 1, 1500, 37, 2)])
+def test_paged_prompt_attention_alone_and_in_a_step(ops, D, H, G, kv, new, at):
+    """A request's rows are the same bits alone, beside other prompts, and in portions; through the operator shim too."""
+    from vox_serve_b200.flashinfer_utils import FlashInferPrefillWrapper
+
+    page, g = 64, torch.Generator(device="cuda").manual_seed(kv)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()      # noqa: E731
+    pages = lambda n: (n + page - 1) // page                                     # noqa: E731
+    others = [(900, 900), (1030, 700), (64, 64)]                                 # (cached with the new rows, new)
+    reqs = others[:at] + [(kv, new)] + others[at:]
+    first = np.concatenate([[0], np.cumsum([pages(n) for n, _ in reqs])]).tolist()
+    cache, q = rnd(first[-1], 2, page, G, D), [rnd(r, H, D) for _, r in reqs]
+
+    def run(chosen, shim=False):
+        """chosen: (request, its rows from, to) of the step"""
+        lens = [reqs[i][0] - reqs[i][1] + b for i, _, b in chosen]
+        idx = [first[i] + j for (i, _, _), n in zip(chosen, lens) for j in range(pages(n))]
+        qo, ip = ([0] + np.cumsum(v).tolist() for v in ([b - a for _, a, b in chosen], [pages(n) for n in lens]))
+        last, rows = [(n - 1) % page + 1 for n in lens], torch.cat([q[i][a:b] for i, a, b in chosen])
+        if shim:
+            w = FlashInferPrefillWrapper(attn_buffer=None, n_qo_head=H, n_kv_head=G, n_state=H * D, page_size=page, device="cuda", max_seq_len=4096)
+            w.plan(*(torch.tensor(v, dtype=torch.int32) for v in (qo, ip, idx, last)))
+            out = w.run(rows, cache).view(-1, H, D)
+        else:
+            plan = ops.RowPlan(qo[-1], "cuda")
+            ops.plan_rows(plan, _i32(qo), _i32(ip), _i32(idx), _i32(last), len(chosen), qo[-1], page, page)
+            out = ops.paged_attn(rows, cache, 0, plan, qo[-1], G, page, page, None, prefill_tiles="tc")
+        n = [i for i, _, _ in chosen].index(at)
+        return out[qo[n]:qo[n + 1]]
+
+    step = [(i, 0, r) for i, (_, r) in enumerate(reqs)]
+    want = run([(at, 0, new)])
+    assert torch.equal(run(step), want)
+    cut = new // 3
+    assert torch.equal(torch.cat((run([(at, 0, cut)]), run(step[:at] + [(at, cut, new)] + step[at + 1:]))), want)
+    if new >= 100:                                       # (fewer rows alone take the row kernel)
+        assert torch.equal(run([(at, 0, new)], True), run(step, True))
+
+
+@pytest.mark.parametrize("n,old,window,keep", [(500, 0, 0, 0), (640, 100, 300, 4)])
+def test_window_attention_alone_and_in_a_step(ops, n, old, window, keep):
+    """A prompt's rows are the same bits alone and beside other prompts."""
+    D, H, G, page = 128, 16, 4, 64
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()      # noqa: E731
+    reqs = [(1000, 0), (n, old), (900, 0)]
+    pages = [(r + o + page - 1) // page for r, o in reqs]
+    first = np.concatenate([[0], np.cumsum(pages)]).tolist()
+    q, kc, vc = [rnd(r, H * D) for r, _ in reqs], rnd(first[-1], page, G, D), rnd(first[-1], page, G, D)
+
+    def run(chosen):
+        T, qo, treq, trow, pos, idx, ip = 0, [0], [], [], [], [], [0]
+        for k, i in enumerate(chosen):
+            r, o = reqs[i]
+            treq += [k] * ((r + 63) // 64)
+            trow += list(range(T, T + r, 64))
+            pos += list(range(o, o + r))
+            idx += list(range(first[i], first[i + 1]))
+            T += r
+            qo.append(T)
+            ip.append(len(idx))
+        out = torch.empty(T, H * D, device="cuda").bfloat16()
+        ops.window_attn(torch.cat([q[i] for i in chosen]), kc, vc, out, None, None, _i32(pos), _i32(ip), _i32(idx), T, H, G, D, D, window, D ** -0.5,
+                        tiles=(_i32(qo), _i32(treq), _i32(trow), len(treq)), keep_first=keep)
+        k = chosen.index(1)
+        return out[qo[k]:qo[k + 1]]
+
+    assert torch.equal(run([0, 1, 2]), run([1]))
 
 
 @pytest.mark.parametrize("H", [128, 129, 200])

@@ -1,7 +1,7 @@
 // The tcgen05 attention core of prompt rows, shared by prefill_attn_tc.cu (paged cache of the speech LMs) and window_attn_tc.cu
 // (sliding windows of the text LMs): one accumulator row of 128 per softmax thread, scores and probabilities in TMEM, K and V
 // tiles of 64 keys through two-stage rings.  A kernel brings an object `rows` that says what its thread's row sees:
-//   n_tiles, tile(it)        the key tiles that the block walks, in order (tile i holds keys 64 i ..)
+//   n_tiles, tile(it)        the key tiles to walk, in order (tile i holds keys 64 i ..)
 //   scale_log2               what a score is multiplied by, times log2(e)
 //   full(tok0), visible(kj)  whether all 64 keys from tok0 / key kj are visible to this thread's row
 //   group, q_row(t, g)       accumulator row r is row t = r / group of the tile, head g = r % group of the group: its query row, or nullptr
@@ -67,9 +67,6 @@ __device__ __forceinline__ uint32_t ptc_left(float p0, float p1, uint32_t h) {
 constexpr int PTC_THREADS = 224;       // 4 softmax warps, 1 MMA warp, 2 loader warps
 constexpr int PTC_KT = 64;             // tokens per K / V tile
 constexpr int PTC_STAGES = 2;          // K and V tiles in flight, each with barriers of their own
-// Where a launch has clusters of two blocks, row tiles that walk at least this many key tiles share them between the two (PtcHalf).  They meet at
-// the end, some 3 us, 1.3 us being a key tile's: nothing to gain below.
-constexpr int PTC_SPLIT_TILES = 6;
 constexpr float PTC_RESCALE = 8.f;     // growth of a row's maximum (base 2) that moves the exponents' reference
 
 template <int D>
@@ -186,13 +183,12 @@ __device__ __forceinline__ void ptc_put32(uint8_t* smem, int c0, const uint32_t 
     *ptc_staged<D>(smem, threadIdx.x, (c0 >> 3) + c) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
-// columns [c_lo, c_lo + C) of all rows, once the four softmax warps have put theirs
-template <int D, int C, class Rows>
-__device__ __forceinline__ void ptc_send(uint8_t* smem, const Rows& rows, int c_lo) {
-  constexpr int CPR = C / 8;
+// all rows, once the four softmax warps have put theirs
+template <int D, class Rows>
+__device__ __forceinline__ void ptc_send(uint8_t* smem, const Rows& rows) {
+  constexpr int CPR = D / 8, STEP = 128 / CPR;
   asm volatile("bar.sync 1, 128;" ::: "memory");
-  constexpr int STEP = 128 / CPR;
-  const int c = (c_lo >> 3) + threadIdx.x % CPR, r0 = threadIdx.x / CPR;
+  const int c = threadIdx.x % CPR, r0 = threadIdx.x / CPR;
   PtcWalk<STEP> w(r0, rows.group);
 #pragma unroll 4
   for (int i = 0; i < CPR; ++i, w.next()) {
@@ -201,68 +197,9 @@ __device__ __forceinline__ void ptc_send(uint8_t* smem, const Rows& rows, int c_
   }
 }
 
-// The key tiles of a block: all of the row tile's, or its half of them where the cluster's two blocks share a row tile.
-struct PtcHalf {
-  int first, n, rank;
-  bool split;
-  __device__ __forceinline__ PtcHalf(int n_tiles, bool shared, int rank_) : rank(rank_) {
-    split = shared && n_tiles >= PTC_SPLIT_TILES;
-    const int half = (n_tiles + 1) >> 1;
-    first = split && rank ? half : 0;
-    n = split ? (rank ? n_tiles - half : half) : (rank ? 0 : n_tiles);
-  }
-};
-// What a thread of a shared row tile leaves for the other block, in its own block's K and V stages (their last tile has been multiplied): the
-// accumulated row's columns of the other block's half, [column][128 rows], the exponents' reference and the denominator.
-template <int D>
-__device__ __forceinline__ void ptc_give(uint8_t* smem, uint32_t t_lane, int rank, float m, float l) {
-  float* buf = reinterpret_cast<float*>(smem + PtcLayout<D>::K) + threadIdx.x;
-  const int c_other = (1 - rank) * (D / 2);
-#pragma unroll
-  for (int c0 = 0; c0 < D / 2; c0 += 32) {
-    uint32_t o[32];
-    tmem_ld_32x32(t_lane + 128 + c_other + c0, o);
-    tmem_ld_wait();
-#pragma unroll
-    for (int i = 0; i < 32; ++i) buf[(c0 + i) * 128] = __uint_as_float(o[i]);
-  }
-  buf[(D / 2) * 128] = m;
-  buf[(D / 2 + 1) * 128] = l;
-}
-// ... and the merge of this block's half of the columns, once both have met
-template <int D, class Rows>
-__device__ __forceinline__ void ptc_merge(uint8_t* smem, uint32_t tmem, const Rows& rows, int rank, float m, float l) {
-  const uint32_t t_lane = tmem + ((threadIdx.x >> 5) * 32u << 16);
-  uint32_t far;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(smem_u32(smem + PtcLayout<D>::K) + threadIdx.x * 4), "r"(1 - rank));
-  auto get = [&](int c) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(far + c * 512) : "memory");
-    return v;
-  };
-  const float m1 = get(D / 2), l1 = get(D / 2 + 1), M = fmaxf(m, m1);
-  const float a0 = m == -INFINITY ? 0.f : ptc_ex2(m - M), a1 = m1 == -INFINITY ? 0.f : ptc_ex2(m1 - M);
-  const float f = rows.finish(M, l * a0 + l1 * a1);
-#pragma unroll 1
-  for (int c0 = 0; c0 < D / 2; c0 += 32) {
-    uint32_t o[32];
-    float r[32];
-    tmem_ld_32x32(t_lane + 128 + rank * (D / 2) + c0, o);
-#pragma unroll
-    for (int i = 0; i < 32; ++i) r[i] = get(c0 + i);
-    tmem_ld_wait();
-#pragma unroll
-    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * a0 + r[i] * a1);
-    if (rows.STAGED) ptc_put32<D>(smem, rank * (D / 2) + c0, o, f);
-    else rows.store(rank * (D / 2) + c0, o, f);
-  }
-  if (rows.STAGED) ptc_send<D, D / 2>(smem, rows, rank * (D / 2));
-}
-
 // ================= warps 0..3: softmax =================
 template <int D, class Rows>
-__device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const Rows& rows, const PtcHalf& half, float& m_out, float& l_out,
-                                            BoundedWait& bw) {
+__device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const Rows& rows, BoundedWait& bw) {
   using L = PtcLayout<D>;
   constexpr int KBD = D / 64, CPR = D * 2 / 16;
   const int tid = threadIdx.x, warp = tid >> 5, n_tiles = rows.n_tiles;
@@ -369,12 +306,6 @@ __device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const 
   }
   if (bw.dead) return;
   tc_fence_after();
-  if (half.split) {
-    ptc_give<D>(smem, t_lane, half.rank, m_ref, l_run);
-    m_out = m_ref;
-    l_out = l_run;
-    return;
-  }
   const float f = rows.finish(m_ref, l_run);
 #pragma unroll 1
   for (int c0 = 0; c0 < D; c0 += 32) {
@@ -389,7 +320,7 @@ __device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const 
     if (rows.STAGED) ptc_put32<D>(smem, c0, o, f);
     else rows.store(c0, o, f);
   }
-  if (rows.STAGED) ptc_send<D, D>(smem, rows, 0);
+  if (rows.STAGED) ptc_send<D>(smem, rows);
 }
 
 // ================= warp 4: MMA issuer (the whole warp walks the loop, one elected lane issues: operands stay in uniform registers) =================

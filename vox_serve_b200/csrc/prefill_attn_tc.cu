@@ -25,8 +25,9 @@
 // four portions of 997 rows on up to 1063 cached tokens 112 / 40, three prompts of 1024 rows each 187 / 61, four of 600 with 64-wide heads
 // 74 / 32.
 // Query rows come and results leave in whole rows, a few neighbouring threads each (a row per thread took 6 us until the rows were there and 3 us
-// at the end of a launch of cold data, 2 and 2 now); where portions continue long contexts two blocks of a cluster share a row tile's keys
-// and merge through distributed shared memory.  The 997 rows above: 45 us a layer of cold data, 36 with whole rows, 26 shared as well.
+// at the end of a launch of cold data, 2 and 2 now).  The 997 rows above: 45 us a layer of cold data, 36 with whole rows.
+// A row's result depends on its own request alone, whatever else is in the step and whichever portion it comes in: the tiles of its keys are
+// walked in order by one block.  (Sharing them between two blocks where a launch leaves room, 26 us, moved its roundings with its neighbours.)
 // What bounds it: the serial chain of a tile (scores -> maximum -> exponentials -> P V, about 1.3 us), some 5 us around it.
 // Every wait is bounded (BoundedWait): a block whose wait runs out sets its flag, stops issuing and leaves.
 #include "../../include/vb_api.h"
@@ -47,7 +48,6 @@ struct PrefillTcParams {
   int n_req, n_rows, n_q, n_kv, G, TQ, page_size;
   int out_xt_tile;
   int box_tokens;
-  int shared;
   float scale_log2;
   unsigned char* wait_flag;
 };
@@ -57,9 +57,9 @@ struct PagedRows {
   static constexpr bool HOLE = false, STAGED = true;
   static constexpr int hole0 = 0, hole1 = 0;
   const PrefillTcParams& p;
-  int n_tiles, first, kl, row0, nrows, head0, group, D;
+  int n_tiles, kl, row0, nrows, head0, group, D;
   float scale_log2;
-  __device__ __forceinline__ int tile(int it) const { return first + it; }
+  __device__ __forceinline__ int tile(int it) const { return it; }
   __device__ __forceinline__ bool full(int tok0) const { return tok0 + PTC_KT <= kl; }
   __device__ __forceinline__ bool visible(int kj) const { return kj < kl; }
   __device__ __forceinline__ const __nv_bfloat16* q_row(int t, int g) const {
@@ -100,8 +100,7 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
   pdl_sync();
 
   // rows beyond the last request (CUDA-graph padding) produce zeros
-  // key heads fastest; where row tiles may be shared a cluster is two blocks of one of them
-  const int rank = p.shared ? blockIdx.x & 1 : 0, hk = p.shared ? blockIdx.x >> 1 : blockIdx.x;
+  const int hk = blockIdx.x;                        // key heads fastest
   if (blockIdx.x == 0) {
     const int n_valid = p.qo_indptr[p.n_req];
     for (int row = n_valid + blockIdx.y; row < p.n_rows && blockIdx.z == 0; row += gridDim.y)
@@ -150,22 +149,16 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
   }
   __syncthreads();
   const int req = sh->tile[0];
-  bool split = false;                             // alike in both blocks
   if (req >= 0) {
     const int row0 = sh->tile[1], nrows = sh->tile[2];
     // the tile's largest bound (the bounds do not decrease inside a request: the last row's)
     const int kmax = p.row_kvlen[row0 + nrows - 1];
-    const PtcHalf half((kmax + PTC_KT - 1) / PTC_KT, p.shared != 0, rank);
-    const int n_tiles = half.n, first = half.first;
-    split = half.split;
+    const int n_tiles = (kmax + PTC_KT - 1) / PTC_KT;
     const int t = tid / p.G;                      // (softmax) this thread's accumulator row: prompt row t of the tile, head tid % G
     const bool ok = warp < 4 && t < nrows;
-    const PagedRows rows{p, n_tiles, first, ok ? p.row_kvlen[row0 + t] : 0, row0, nrows, hk * p.G, p.G, D, p.scale_log2};
-    float m = 0.f, l = 0.f;
-    if (rank == 1 && !split) {
-      // (the other block's row tile alone)
-    } else if (warp < 4) {
-      ptc_softmax<D>(smem, sh, rows, half, m, l, bw);
+    const PagedRows rows{p, n_tiles, ok ? p.row_kvlen[row0 + t] : 0, row0, nrows, hk * p.G, p.G, D, p.scale_log2};
+    if (warp < 4) {
+      ptc_softmax<D>(smem, sh, rows, bw);
     } else if (warp == 4) {
       ptc_issue<D>(smem, sh, n_tiles, bw);
     } else if (TMA) {
@@ -184,7 +177,7 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
       const int ltok = tid - 160, pbase = p.kv_indptr[req];
       const size_t page_elems = static_cast<size_t>(p.page_size) * p.n_kv * D;
       auto fetch = [&](int j, int is_v) {
-        const int tok = (first + j) * PTC_KT + ltok;
+        const int tok = j * PTC_KT + ltok;
         const uint32_t dst = smem_u32(smem + (is_v ? L::V : L::K) + (j & 1) * L::TILE) + ltok * 128;
         if (tok < kmax) {
           const int page = __ldg(&p.kv_indices[pbase + tok / p.page_size]);
@@ -226,13 +219,6 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
         mbar_arrive(&sh->v_full[(n_tiles - 1) & 1]);
       }
     }
-    if (split) {
-      __syncwarp();
-      cluster_sync_all();
-      if (warp < 4 && !bw.dead) ptc_merge<D>(smem, tmem_base, rows, rank, m, l);
-      __syncwarp();
-      cluster_sync_all();                         // (the other block has read what this one gave)
-    }
   }
   tc_fence_before();
   __syncthreads();
@@ -248,7 +234,7 @@ static int launch_prefill_tc(const PrefillTcParams& p, const CUtensorMap& map, d
   // (a fixed size per instantiation -- safe under CUDA-graph replay)
   constexpr int smem_bytes = PtcLayout<D>::TOTAL;
   VB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-  VB_LAUNCH_PDL_CLUSTER(kern, grid, PTC_THREADS, smem_bytes, stream, p.shared ? 2 : 1, p, map);
+  VB_LAUNCH_PDL(kern, grid, PTC_THREADS, smem_bytes, stream, p, map);
   return 0;
 }
 }  // namespace vb
@@ -270,14 +256,6 @@ int vb_paged_prefill_attn_tc(void* d_out, const void* d_q, const void* d_kv, int
                              const int32_t* d_qo_indptr, const int32_t* d_kv_indptr, const int32_t* d_kv_indices,
                              const int32_t* d_row_kvlen, int n_req, int n_rows, int n_q, int n_kv, int head_dim,
                              int page_size, float sm_scale, int out_xt_tile, void* stream) {
-  return vb_paged_prefill_attn_tc_keys(d_out, d_q, d_kv, slab_base, d_qo_indptr, d_kv_indptr, d_kv_indices, d_row_kvlen, n_req, n_rows, n_q, n_kv,
-                                       head_dim, page_size, sm_scale, out_xt_tile, 0, stream);
-}
-
-int vb_paged_prefill_attn_tc_keys(void* d_out, const void* d_q, const void* d_kv, int64_t slab_base,
-                                  const int32_t* d_qo_indptr, const int32_t* d_kv_indptr, const int32_t* d_kv_indices,
-                                  const int32_t* d_row_kvlen, int n_req, int n_rows, int n_q, int n_kv, int head_dim,
-                                  int page_size, float sm_scale, int out_xt_tile, long long keys, void* stream) {
   VB_CHECK_ARG(d_out && d_q && d_kv && d_qo_indptr && d_kv_indptr && d_kv_indices && d_row_kvlen,
                "vb_paged_prefill_attn_tc: null pointer");
   VB_CHECK_ARG(n_kv > 0 && n_q % n_kv == 0 && n_q / n_kv <= 128, "vb_paged_prefill_attn_tc: %d query heads / %d kv heads",
@@ -300,12 +278,7 @@ int vb_paged_prefill_attn_tc_keys(void* d_out, const void* d_q, const void* d_kv
   p.out_xt_tile = out_xt_tile;
   p.scale_log2 = sm_scale * 1.4426950408889634f;
   const unsigned tiles = static_cast<unsigned>((n_rows + p.TQ - 1) / p.TQ) + static_cast<unsigned>(n_req), slices = (tiles + 65534) / 65535;
-  // Row tiles shared by two blocks: where portions continue long contexts -- the cached keys, pages counted whole, are more than twice the rows
-  // -- and the longest of them would run on alone (four portions of 997 rows on up to 1063 cached tokens: 36 us a layer, 26 shared), and where
-  // even twice the blocks find an SM of their own.  Elsewhere the clusters only start later (1024 rows of three fresh prompts, 20 launches
-  // around: 549 us, 565 shared).
-  p.shared = keys > 2LL * n_rows + static_cast<long long>(n_req) * page_size || static_cast<long long>(tiles) * n_kv * 2 <= 148;
-  const dim3 grid((p.shared ? 2 : 1) * n_kv, (tiles + slices - 1) / slices, slices);
+  const dim3 grid(n_kv, (tiles + slices - 1) / slices, slices);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   p.box_tokens = ptc_box_tokens(page_size);
   CUtensorMap map = {};

@@ -27,7 +27,6 @@ struct WindowTcParams {
   const float* sink;             // [H] or nullptr
   int ld_gate, H, G, R, TQ, subs, page_size, window, chunk, keep, v_share, out_f32, head_gate, box_tokens;
   float scale_log2;
-  int shared;
   unsigned char* wait_flag;
 };
 
@@ -42,13 +41,13 @@ __device__ __forceinline__ void wtc_tma_4d(uint32_t dst, const CUtensorMap* m, u
 struct WindowRows {
   static constexpr bool HOLE = true, STAGED = false;
   const WindowTcParams& p;
-  int n_tiles, first, n0, t1;    // of the row tile's key tiles 0 .. n0 - 1 hold kept tokens, the rest start at t1; the block's start with `first`
+  int n_tiles, n0, t1;           // tiles 0 .. n0 - 1 hold kept tokens, the rest start at t1
   int hole0, hole1;              // between the kept tokens and the first key that the block's first row sees
   int pos, lo, row, head, D;
   int row0, nrows, head0, group;
   bool ok;
   float scale_log2;
-  __device__ __forceinline__ int tile(int it) const { return first + it < n0 ? first + it : t1 + (first + it - n0); }
+  __device__ __forceinline__ int tile(int it) const { return it < n0 ? it : t1 + (it - n0); }
   __device__ __forceinline__ bool full(int tok0) const { return ok && tok0 + PTC_KT - 1 <= pos && tok0 >= lo; }
   __device__ __forceinline__ bool visible(int kj) const { return ok && kj <= pos && (kj >= lo || kj < p.keep); }
   __device__ __forceinline__ const __nv_bfloat16* q_row(int t, int g) const {
@@ -118,9 +117,7 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) window_attn_tc_kernel(const Wi
   pdl_sync();
 
   // later tiles of a prompt see more keys: they are started first so that the short ones fill the tail
-  // where row tiles may be shared a cluster is two blocks of one of them
-  const int rank = p.shared ? blockIdx.x & 1 : 0;
-  const int unit = p.shared ? (gridDim.x >> 1) - 1 - (blockIdx.x >> 1) : gridDim.x - 1 - blockIdx.x, ti = unit / p.subs, b = p.tile_req[ti], g = blockIdx.y;
+  const int unit = gridDim.x - 1 - blockIdx.x, ti = unit / p.subs, b = p.tile_req[ti], g = blockIdx.y;
   const int row0 = p.tile_row0[ti] + (unit - ti * p.subs) * p.TQ;
   const int nrows = min(min(row0 + p.TQ, p.tile_row0[ti] + 64), p.qo_indptr[b + 1]) - row0;
   if (nrows > 0) {
@@ -129,17 +126,12 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) window_attn_tc_kernel(const Wi
       return p.chunk > 0 ? max(lo, ps - ps % p.chunk) : lo;
     };
     const int pos0 = p.pos[row0], kmax = pos0 + nrows, lo0 = first_key(pos0);
-    const int n0 = (min(p.keep, lo0) + PTC_KT - 1) / PTC_KT, t1 = max(lo0 / PTC_KT, n0);
-    const PtcHalf half(n0 + (kmax + PTC_KT - 1) / PTC_KT - t1, p.shared != 0, rank);
-    const int n_tiles = half.n;
+    const int n0 = (min(p.keep, lo0) + PTC_KT - 1) / PTC_KT, t1 = max(lo0 / PTC_KT, n0), n_tiles = n0 + (kmax + PTC_KT - 1) / PTC_KT - t1;
     const int t = tid / p.R;
     const bool ok = warp < 4 && t < nrows;
-    const WindowRows rows{p, n_tiles, half.first, n0, t1, min(p.keep, lo0), lo0, pos0 + t, first_key(pos0 + t), row0 + t, g * p.R + tid - t * p.R, D, row0, nrows, g * p.R, p.R, ok, p.scale_log2};
-    float m = 0.f, l = 0.f;
-    if (rank == 1 && !half.split) {
-      // (the other block's row tile alone)
-    } else if (warp < 4) {
-      ptc_softmax<D>(smem, sh, rows, half, m, l, bw);
+    const WindowRows rows{p, n_tiles, n0, t1, min(p.keep, lo0), lo0, pos0 + t, first_key(pos0 + t), row0 + t, g * p.R + tid - t * p.R, D, row0, nrows, g * p.R, p.R, ok, p.scale_log2};
+    if (warp < 4) {
+      ptc_softmax<D>(smem, sh, rows, bw);
     } else if (warp == 4) {
       ptc_issue<D>(smem, sh, n_tiles, bw);
     } else {
@@ -153,13 +145,6 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) window_attn_tc_kernel(const Wi
         ptc_clear_unseen<D>(smem, sh, rows, kmax, bw);
       }
       __syncwarp();
-    }
-    if (half.split) {
-      __syncwarp();
-      cluster_sync_all();
-      if (warp < 4 && !bw.dead) ptc_merge<D>(smem, tmem_base, rows, rank, m, l);
-      __syncwarp();
-      cluster_sync_all();                         // (the other block has read what this one gave)
     }
   }
   tc_fence_before();
@@ -200,16 +185,13 @@ int window_attn_tc(void* out, const void* q, const void* k_cache, const void* v_
                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     VB_CHECK_ARG(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(window cache) failed: CUresult %d", static_cast<int>(r));
   }
-  // Row tiles shared by two blocks where all of them find a place at once (16 heads on 4 of two prompts of 1001 rows, 128 row tiles: the step
-  // of three layers 839 us, 827 shared)
-  p.shared = static_cast<long long>(n_tiles) * p.subs * G <= 148;
-  const dim3 grid((p.shared ? 2 : 1) * n_tiles * p.subs, G);
+  const dim3 grid(n_tiles * p.subs, G);
   if (dim == 128) {
     VB_CHECK_CUDA(cudaFuncSetAttribute(window_attn_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PtcLayout<128>::TOTAL));
-    VB_LAUNCH_PDL_CLUSTER(window_attn_tc_kernel<128>, grid, PTC_THREADS, PtcLayout<128>::TOTAL, stream, p.shared ? 2 : 1, p, maps[0], maps[1]);
+    VB_LAUNCH_PDL(window_attn_tc_kernel<128>, grid, PTC_THREADS, PtcLayout<128>::TOTAL, stream, p, maps[0], maps[1]);
   } else {
     VB_CHECK_CUDA(cudaFuncSetAttribute(window_attn_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, PtcLayout<64>::TOTAL));
-    VB_LAUNCH_PDL_CLUSTER(window_attn_tc_kernel<64>, grid, PTC_THREADS, PtcLayout<64>::TOTAL, stream, p.shared ? 2 : 1, p, maps[0], maps[1]);
+    VB_LAUNCH_PDL(window_attn_tc_kernel<64>, grid, PTC_THREADS, PtcLayout<64>::TOTAL, stream, p, maps[0], maps[1]);
   }
   return 0;
 }

@@ -113,8 +113,7 @@ class FlashInferPrefillWrapper(_PagedWrapper):
         self.qo_indptr = qo_indptr if isinstance(qo_indptr, torch.Tensor) else torch.tensor(qo_indptr, dtype=torch.int32)
         self.paged_kv_indptr, self.paged_kv_indices = paged_kv_indptr, paged_kv_indices
         self.paged_kv_last_page_len = paged_kv_last_page_len
-        ops.plan_rows(self.plan_rows, qo, ip, ix, la, n_req, self.n_rows_padded, self.page_size, self.chunk,
-                      keys=ix.numel() * self.page_size)
+        ops.plan_rows(self.plan_rows, qo, ip, ix, la, n_req, self.n_rows_padded, self.page_size, self.chunk)
 
 
 class FlashInferDecodeWrapper(_PagedWrapper):

@@ -228,12 +228,11 @@ class RowPlan:
         self.kv_indptr: Optional[torch.Tensor] = None
         self.n_rows = 0
         self.n_req = 0
-        self.keys = 0              # cached keys of all requests, pages counted whole, where the caller knows them
 
 
 def plan_rows(plan: RowPlan, qo_indptr: Optional[torch.Tensor], kv_indptr: torch.Tensor, kv_indices: torch.Tensor,
               last_page_len: Optional[torch.Tensor], n_req: int, n_rows: int, page_size: int, chunk_tokens: int,
-              kv_len: Optional[torch.Tensor] = None, keys: int = 0) -> RowPlan:
+              kv_len: Optional[torch.Tensor] = None) -> RowPlan:
     _need_cuda(kv_indptr, kv_indices, last_page_len, kv_len)
     assert n_rows <= plan.max_rows
     call("vb_plan_rows", _p(qo_indptr), kv_indptr.data_ptr(), kv_indices.data_ptr(), _p(last_page_len), _p(kv_len),
@@ -244,7 +243,6 @@ def plan_rows(plan: RowPlan, qo_indptr: Optional[torch.Tensor], kv_indptr: torch
     plan.n_req = n_req
     plan.kv_indices = kv_indices
     plan.qo_indptr, plan.kv_indptr = qo_indptr, kv_indptr
-    plan.keys = keys
     return plan
 
 
@@ -354,12 +352,9 @@ def paged_attn(q: torch.Tensor, kv_cache, slab_base: int, plan: RowPlan, n_rows:
         assert plan.qo_indptr is not None, "the tiled prefill kernel needs a prefill plan (qo_indptr)"
         fn = "vb_paged_prefill_attn_tc" if prefill_tiles == "tc" else (
             _prefill_entry(n_q // n_kv) if prefill_tiles is None else "vb_paged_prefill_attn")
-        args = (out_ptr, q.data_ptr(), kv_cache.data_ptr(), int(slab_base), plan.qo_indptr.data_ptr(), plan.kv_indptr.data_ptr(),
-                plan.kv_indices.data_ptr(), plan.row_kvlen.data_ptr(), plan.n_req, n_rows, n_q, n_kv, d, page_size, sc, xt)
-        if fn == "vb_paged_prefill_attn_tc":
-            call("vb_paged_prefill_attn_tc_keys", *args, plan.keys, _stream())
-        else:
-            call(fn, *args, _stream())
+        call(fn, out_ptr, q.data_ptr(), kv_cache.data_ptr(), int(slab_base),
+             plan.qo_indptr.data_ptr(), plan.kv_indptr.data_ptr(), plan.kv_indices.data_ptr(),
+             plan.row_kvlen.data_ptr(), plan.n_req, n_rows, n_q, n_kv, d, page_size, sc, xt, _stream())
         return out
     grid = workspace.grid if grid_ctas is None else min(int(grid_ctas), workspace.grid)
     call("vb_paged_attn", out_ptr, q.data_ptr(), kv_cache.data_ptr(), int(slab_base), plan.row_kvlen.data_ptr(),

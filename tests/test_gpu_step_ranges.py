@@ -194,6 +194,28 @@ def test_channels_last_conv_reuses_stages(B, T, C, N, ksize):
         assert torch.equal(_cl.conv(xa, wp, N, ksize=ksize).tensor(), y)
 
 
+# tiles of 128 channels and a last one of 32 or 64, three and more units a CTA, so that a CTA goes from one width to the other; without boxes
+# (parts, 288) and with them
+@pytest.mark.parametrize("T,C,N,ksize", [(32768, 256, 288, 3), (32768, 512, 320, 1), (20000, 512, 544, 1), (9001, 256, 320, 3)])
+@pytest.mark.parametrize("parts", [False, True])
+def test_channels_last_conv_of_two_tile_widths(T, C, N, ksize, parts):
+    from vox_serve_b200 import _lib
+    from vox_serve_b200.tokenizer import _cl
+
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x, w = torch.randn(1, T, C, generator=g, device="cuda"), torch.randn(N, C, ksize, generator=g, device="cuda") * (C * ksize) ** -0.5
+    act = _cl.Act(x.reshape(-1).clone(), 1, T, C)
+    if parts:
+        act = _cl.conv(act, _cl.pack(torch.eye(C, device="cuda")), C, out="parts")
+    ref = torch.nn.functional.conv1d(torch.nn.functional.pad(x.double().transpose(1, 2), (ksize - 1, 0)), w.double()).transpose(1, 2)
+    y, z = _cl.conv(act, _cl.pack_conv(w.reshape(N, -1), C, ksize), N, ksize=ksize, act="elu", both=True, out="parts")
+    single = _cl.conv(act, _cl.pack_conv(w.reshape(N, -1), C, ksize), N, ksize=ksize).tensor()
+    back = _cl.conv(z, _cl.pack(torch.eye(N, device="cuda")), N).tensor()
+    err = lambda got, want: (((got.double() - want).norm(dim=2) / want.norm(dim=2)).max()).item()      # noqa: E731  (of the worst position)
+    assert err(y.tensor(), ref) < 1e-5 and err(single, ref) < 1e-5 and err(back, torch.nn.functional.elu(ref)) < 1e-5
+    assert _lib.load().vb_cl_timeouts() == 0
+
+
 # activations kept as parts: several entries and their halos in a tile, runs with a remainder, taps further apart than a tile's halo holds, K
 # divided over a cluster, boxes of results and none, two results; values of ordinary size, larger than fp16 and all below its normal range
 @pytest.mark.parametrize("B,T,C,N,ksize,dil,lo,hi,epi,act,both,size", [

@@ -960,10 +960,10 @@ __global__ void __launch_bounds__(ClRoles<PARTS>::THREADS, 1) cl_conv_kernel(con
       // This warp's chunks of eight columns: every `turns`-th one.  Which warps have one more than the others goes round from unit to unit (there are
       // two accumulators): 16 chunks for the 6 warps of 64 channels are 8 in three units instead of 3 in each.  Mimi, 32 windows in a row of calls: 614400 x 64
       // with residual 117 -> 112 us, 614400 x 32 88 -> 84, 153600 x 256 to two outputs 114 -> 110.
-      const int turns = EPI_WARPS / 4 * copies;
-      int turn = ((warp - FIRST_EPI) >> 2) * copies + (copies == 4 ? quarter : copies == 2 ? quarter >> 1 : 0) - skew;
+      const int turns = EPI_WARPS / 4 * copies;          // (of a tile's own width: it divides EPI_WARPS, so `skew` is kept modulo that)
+      int turn = ((warp - FIRST_EPI) >> 2) * copies + (copies == 4 ? quarter : copies == 2 ? quarter >> 1 : 0) - skew % turns;
       if (turn < 0) turn += turns;
-      skew = (skew + h.cols / CL_EC) % turns;
+      skew = (skew + h.cols / CL_EC) % EPI_WARPS;
       ClEpiState e;
       e.n = g.m0 + row;
       const int nm = p.cmod == h.N ? e.n : e.n % p.cmod;

@@ -495,7 +495,8 @@ int vb_gemm_bf16_grouped_glu(void* d_y, const void* d_w_tiles, const void* x_map
  * vb_wait_flags: eight bytes of host memory, one flag per kind of kernel whose waits give up after two seconds -- 0 prompt projections, 1
  * vocoder convolutions, 2 prompt attention, 3 window attention of prompts, 4 vb_wait_check.  A kernel whose wait ran out sets its
  * flag and leaves its output incomplete: look at them after synchronising, before results are used, and clear them (NULL: no device).
- * vb_wait_check: one kernel that waits on a barrier at most limit_us from the moment a second warp opens it, pause_us after the start;
+ * vb_wait_check: one kernel that waits on a barrier at most limit_us from the moment a second warp opens it, pause_us after the start (both warps
+ * then agree on whether it ran out: the flag is 3);
  * that warp then completes the barrier, or with complete = 0 does not (flag 4). */
 int vb_gemm_bf16_wide(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
                       int mode, int split_k, int tile_rows, int n_out, int y_tiled, const void* d_bias, int act, int n_tok,

@@ -865,6 +865,21 @@ def test_a_wait_that_runs_out_is_reported(ops):
         _lib.call("vb_wait_check", -1, 0, 1, ops._stream())
 
 
+def test_warps_agree_on_a_wait_that_ran_out(ops):
+    """One warp's wait runs out, the other's does not: both meet, and both know."""
+    import ctypes
+
+    from vox_serve_b200 import _lib
+
+    flags = (ctypes.c_ubyte * 8).from_address(_lib.load().vb_wait_flags())
+    at = _lib.WAIT_KINDS.index("vb_wait_check")
+    for complete in (1, 0, 1):
+        _lib.call("vb_wait_check", 1000, 100, complete, ops._stream())
+        torch.cuda.synchronize()
+        assert flags[at] == (0 if complete else 3)
+        flags[at] = 0
+
+
 def test_snac_decoder_that_ends_wide(monkeypatch):
     """A decoder whose last convolution has more channels than the channels-last one takes decodes channel-first."""
     from vox_serve_b200.tokenizer.snac import SNAC

@@ -70,7 +70,8 @@ int wait_ran_out(WaitKind kind) {
   return *(volatile unsigned char*)(g_wait_host + kind);
 }
 
-// A barrier that one warp waits for and another completes (or not) after a pause: what the flags and the gate are tested with
+// A barrier that one warp waits for and another completes (or not) after a pause: what the flags and the gate are tested with.  Then both meet: where
+// the first warp's wait ran out the second one sets the flag's next bit.
 __global__ void wait_check_kernel(unsigned char* flag, unsigned long long limit, unsigned long long pause, int complete) {
   __shared__ uint64_t bar;
   __shared__ uint32_t gate;
@@ -80,8 +81,8 @@ __global__ void wait_check_kernel(unsigned char* flag, unsigned long long limit,
     gate = 0u;
   }
   __syncthreads();
+  BoundedWait bw{flag, smem_u32(&gate), limit};
   if (threadIdx.x == 0) {
-    BoundedWait bw{flag, smem_u32(&gate), limit};
     bw.wait(&bar, 0);
   } else if (threadIdx.x == 32) {
     const unsigned long long t0 = gtimer();
@@ -89,6 +90,8 @@ __global__ void wait_check_kernel(unsigned char* flag, unsigned long long limit,
     wait_gate_open(smem_u32(&gate));
     if (complete) mbar_arrive(&bar);
   }
+  __syncwarp();
+  if (warps_any<1, 64>(bw.dead) && threadIdx.x == 32) *reinterpret_cast<volatile unsigned char*>(flag) = 3;
 }
 // weak: a library built from a subset of the sources (vox_serve_b200/build.py profiles) lacks some of these
 __attribute__((weak)) cudaError_t trace_set_elementwise(unsigned long long*);

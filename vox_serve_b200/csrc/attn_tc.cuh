@@ -183,17 +183,40 @@ __device__ __forceinline__ void ptc_put32(uint8_t* smem, int c0, const uint32_t 
     *ptc_staged<D>(smem, threadIdx.x, (c0 >> 3) + c) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
-// all rows, once the four softmax warps have put theirs
+// all rows, once the four softmax warps have put theirs; none if one of them has given up
 template <int D, class Rows>
-__device__ __forceinline__ void ptc_send(uint8_t* smem, const Rows& rows) {
+__device__ __forceinline__ void ptc_send(uint8_t* smem, const Rows& rows, BoundedWait& bw) {
   constexpr int CPR = D / 8, STEP = 128 / CPR;
-  asm volatile("bar.sync 1, 128;" ::: "memory");
+  if (warps_any<1, 128>(bw.dead)) {
+    bw.dead = true;
+    return;
+  }
   const int c = threadIdx.x % CPR, r0 = threadIdx.x / CPR;
   PtcWalk<STEP> w(r0, rows.group);
 #pragma unroll 4
   for (int i = 0; i < CPR; ++i, w.next()) {
     uint4* dst = rows.out_at(w.t, w.g, c);
     if (dst) *dst = *ptc_staged<D>(smem, r0 + i * STEP, c);
+  }
+}
+
+// this thread's accumulated row, once the last tile has been multiplied
+template <int D, class Rows>
+__device__ __forceinline__ void ptc_finish_rows(uint8_t* smem, const Rows& rows, uint32_t t_lane, int n_tiles, float m_ref, float l_run) {
+  tc_fence_after();
+  const float f = rows.finish(m_ref, l_run);
+#pragma unroll 1
+  for (int c0 = 0; c0 < D; c0 += 32) {
+    uint32_t o[32];
+    if (n_tiles > 0) {
+      tmem_ld_32x32(t_lane + 128 + c0, o);
+      tmem_ld_wait();
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) o[i] = 0u;
+    }
+    if (rows.STAGED) ptc_put32<D>(smem, c0, o, f);
+    else rows.store(c0, o, f);
   }
 }
 
@@ -304,23 +327,8 @@ __device__ __forceinline__ void ptc_softmax(uint8_t* smem, PtcShared* sh, const 
     bw.wait(&sh->o_last, 0);
     if (!__all_sync(0xffffffffu, !bw.dead)) bw.dead = true;
   }
-  if (bw.dead) return;
-  tc_fence_after();
-  const float f = rows.finish(m_ref, l_run);
-#pragma unroll 1
-  for (int c0 = 0; c0 < D; c0 += 32) {
-    uint32_t o[32];
-    if (n_tiles > 0) {
-      tmem_ld_32x32(t_lane + 128 + c0, o);
-      tmem_ld_wait();
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) o[i] = 0u;
-    }
-    if (rows.STAGED) ptc_put32<D>(smem, c0, o, f);
-    else rows.store(c0, o, f);
-  }
-  if (rows.STAGED) ptc_send<D>(smem, rows);
+  if (!bw.dead) ptc_finish_rows<D>(smem, rows, t_lane, n_tiles, m_ref, l_run);
+  if (rows.STAGED) ptc_send<D>(smem, rows, bw);          // (all four warps come here)
 }
 
 // ================= warp 4: MMA issuer (the whole warp walks the loop, one elected lane issues: operands stay in uniform registers) =================

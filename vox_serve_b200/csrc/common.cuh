@@ -327,6 +327,17 @@ struct BoundedWait {
     }
   }
 };
+// Several warps that meet behind waits of their own: true in all of them if it is in one.  (A warp that gave up has to come here all the same: the
+// others would wait for it without a limit.)
+template <int BARRIER, int THREADS>
+__device__ __forceinline__ bool warps_any(bool dead) {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
+               : "=r"(r)
+               : "r"(dead ? 1u : 0u), "n"(BARRIER), "n"(THREADS)
+               : "memory");
+  return r != 0u;
+}
 __device__ __forceinline__ void wait_gate_open(uint32_t gate) {
   asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(gate), "r"(1u) : "memory");
 }

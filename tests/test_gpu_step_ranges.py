@@ -707,6 +707,35 @@ def test_window_attention_alone_and_in_a_step(ops, n, old, window, keep):
 
     assert torch.equal(run([0, 1, 2]), run([1]))
 
+def test_a_plan_of_pinned_tables_inside_a_graph(ops):
+    """Pinned tables are copied from where they lie: a plan can be captured, and every replay reads them again."""
+    from vox_serve_b200.flashinfer_utils import FlashInferDecodeWrapper, FlashInferPrefillWrapper
+
+    D, H, G, page = 128, 6, 2, 16
+    g = torch.Generator(device="cuda").manual_seed(5)
+    cache = torch.randn(24, 2, page, G, D, generator=g, device="cuda").bfloat16()
+    pin = lambda v: torch.tensor(v, dtype=torch.int32).pin_memory()              # noqa: E731
+    for cls, new in ((FlashInferPrefillWrapper, [40, 23]), (FlashInferDecodeWrapper, [1, 1])):
+        q = torch.randn(sum(new), H, D, generator=g, device="cuda").bfloat16()
+        tables = [pin(v) for v in ([0, new[0], sum(new)], [0, 4, 9], list(range(9)), [9, 3])][0 if len(q) > 2 else 1:]
+        make = lambda: cls(attn_buffer=None, n_qo_head=H, n_kv_head=G, n_state=H * D, page_size=page, device="cuda")     # noqa: E731
+        w = make()
+        w.plan(*tables)
+        w.run(q, cache)
+        torch.cuda.synchronize()
+        graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=s):
+            w.plan(*tables)
+            out = w.run(q, cache)
+        for idx, last in (([3, 20, 5, 11, 0, 7, 23, 2, 9], [16, 5]), ([8, 7, 6, 5, 4, 3, 2, 1, 0], [9, 16])):
+            tables[-2].copy_(torch.tensor(idx))
+            tables[-1].copy_(torch.tensor(last))
+            graph.replay()
+            torch.cuda.synchronize()
+            ref = make()
+            ref.plan(*(t.clone() for t in tables))
+            assert torch.equal(out, ref.run(q, cache))
+
 
 @pytest.mark.parametrize("H", [128, 129, 200])
 def test_paged_prompt_attention_many_heads_per_key_head(ops, H):

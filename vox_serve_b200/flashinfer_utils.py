@@ -66,10 +66,12 @@ class _PagedWrapper:
         return dst[:n]
 
     def _upload_tables(self, qo, indptr, last, indices):
-        """The tables of a plan -> their places on the device (``qo`` None: a decode plan).  int32 tensors on the host go up in one copy
-        from a staging tensor (pageable: it may be written again once the call returns)."""
+        """The tables of a plan -> their places on the device (``qo`` None: a decode plan).  int32 tensors in pageable host memory go up in
+        one copy from a staging tensor (pageable itself: it may be written again once the call returns).  Pinned ones are copied from where
+        they lie: the call does not wait for the copies, and a replay of a graph that holds the plan reads the tables again."""
         tables = (qo, indptr, last, indices)
-        if all(t is None or (isinstance(t, torch.Tensor) and t.device.type == "cpu" and t.dtype == torch.int32 and t.dim() == 1) for t in tables):
+        if all(t is None or (isinstance(t, torch.Tensor) and t.device.type == "cpu" and t.dtype == torch.int32 and t.dim() == 1
+                             and not t.is_pinned()) for t in tables):
             out, host, lo = [], self._host, None
             for t, a, d in zip(tables, self._at, (self.d_qo, self.d_indptr, self.d_last, self.d_indices)):
                 if t is None:

@@ -276,6 +276,77 @@ def test_channels_last_parts_special_values(code, C, ksize):
     else:
         assert torch.equal(~torch.isfinite(y), bad)
 
+def _kept_as_parts(x):
+    """x [B, T, C] as parts, exactly where they can hold it: written by the epilogue from a residual"""
+    from vox_serve_b200.tokenizer import _cl
+
+    B, T, C = x.shape
+    zero = _cl.Act(torch.zeros(B * T * C, device="cuda"), B, T, C)
+    return _cl.conv(zero, _cl.pack(torch.eye(C, device="cuda")), C, epi="resid", resid=_cl.Act(x.reshape(-1).clone(), B, T, C), out="parts")
+
+
+# several entries in a tile, flattened rows, a tile of one entry, K divided over a cluster, taps that have stages of their own
+_MIXED = [(5, 16, 64, 96, 3, 1), (5, 40, 64, 64, 1, 1), (2, 700, 32, 32, 3, 1), (5, 17, 1024, 256, 2, 1), (3, 130, 128, 64, 5, 30), (1, 500, 64, 128, 1, 1)]
+
+
+@pytest.mark.parametrize("B,T,C,N,ksize,dil", _MIXED)
+@pytest.mark.parametrize("parts", [False, True])
+def test_channels_last_conv_of_quiet_passages(B, T, C, N, ksize, dil, parts):
+    """Passages of very different magnitude in one tile: each result is as exact as its own inputs let it be."""
+    from vox_serve_b200.tokenizer import _cl
+
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    x, w = torch.randn(B, T, C, generator=g, device="cuda"), torch.randn(N, C, ksize, generator=g, device="cuda") * (C * ksize) ** -0.5
+    levels = torch.tensor([1.0, 1e-9, 1e-4, 3e4, 1e-7, 1e-5, 0.0], device="cuda")
+    run = torch.arange(B * T, device="cuda").view(B, T) // (13 if T < 100 else 61)           # passages that end anywhere in a chunk of rows
+    level = run % len(levels)
+    x = x * levels[level][..., None]
+    act = _kept_as_parts(x) if parts else _cl.Act(x.reshape(-1).clone(), B, T, C)
+    y = _cl.conv(act, _cl.pack_conv(w.reshape(N, -1), C, ksize), N, ksize=ksize, dil=dil).tensor().double()
+    back = (ksize - 1) * dil
+    ref = torch.nn.functional.conv1d(torch.nn.functional.pad(x.double().transpose(1, 2), (back, 0)), w.double(), dilation=dil).transpose(1, 2)
+    whole = torch.ones(B, T, dtype=torch.bool, device="cuda")                    # the results of one passage alone
+    for s in range(dil, back + 1, dil):
+        whole[:, s:] &= run[:, s:] == run[:, :T - s]
+    for k, m in enumerate(levels.tolist()):
+        sel = whole & (level == k)
+        if m == 0.0:
+            assert not y[sel].any()
+        elif sel.any():
+            _close(y[sel], ref[sel], 5e-6)
+
+
+@pytest.mark.parametrize("B,T,C,N,ksize,dil", [m for m in _MIXED if m[0] == 5] + [(5, 300, 32, 32, 3, 1), (2000, 5, 64, 96, 3, 1)])
+@pytest.mark.parametrize("parts", [False, True])
+def test_channels_last_conv_alone_and_in_a_batch(B, T, C, N, ksize, dil, parts):
+    """An entry's results are the same bits whatever lies beside it: ordinary, quiet, large and silent entries, one that is not a number;
+    as floats and as what the next convolution reads."""
+    from vox_serve_b200.tokenizer import _cl
+
+    g = torch.Generator(device="cuda").manual_seed(T + C)
+    x, w = torch.randn(B, T, C, generator=g, device="cuda"), torch.randn(N, C, ksize, generator=g, device="cuda") * (C * ksize) ** -0.5
+    b = torch.randn(N, generator=g, device="cuda") * 1e-3
+    x[1::5] *= 1e-9
+    x[2::5, T // 2, 5] = math.nan
+    x[3::5, T // 3:] *= 3e3
+    x[4::5, T // 4:] = 0.0
+    wp = _cl.pack_conv(w.reshape(N, -1), C, ksize)
+
+    def run(v):
+        """bits of every entry: [plain, activated], [parts, their codes]"""
+        n, res = v.shape[0], []
+        act = _kept_as_parts(v) if parts else _cl.Act(v.reshape(-1).clone(), n, T, C)
+        for out in ("f32", "parts"):
+            y, z = _cl.conv(act, wp, N, b, ksize=ksize, dil=dil, act="elu", both=True, out=out)
+            res.append([t.buf[:n * T * N].view(torch.int32).view(n, -1) for t in (y, z)])
+            if out == "parts":
+                res.append([z.buf[n * T * N:].view(torch.uint8)[:n * T * N // 32].view(n, -1)])
+        return [torch.cat([t[i].reshape(-1).int() for r in res for t in r]) for i in range(n)]
+
+    together = run(x)
+    for i in [*range(5), *range(B - 5, B)]:
+        assert torch.equal(together[i], run(x[i:i + 1])[0]), i
+
 
 def _activated(values, act, alpha=None):
     """The epilogue's activation of given fp32 values: a convolution of zeros with the values as its residual"""

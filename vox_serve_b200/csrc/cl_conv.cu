@@ -10,9 +10,11 @@
 // Products: both operands as two fp16 parts, v = hi + lo / 2048 (the low part scaled into the normal range: 22 bits and a sign), hi_w hi_x in
 // one accumulator, hi_w lo_x + lo_w hi_x in a second one; what is dropped is below 2^-22 of a product.  Half the MMA time and half the
 // weight bytes of the two tf32 parts that stood here, at the same width; error against 64 bits of a decode 4.7e-6 (Mimi, was 2.8e-5).  Weights are
-// scaled per output channel by a power of two when they are packed.  Activations by 16: their parts hold 22 bits where a tile's largest
-// value lies in [2^-16, 4092) (smaller values in such a tile to 2^-40 absolute).  A tile that is outside -- NaN, infinity, huge values, or a
-// whole tile of nothing but tiny ones -- is multiplied again in fp32 on CUDA cores (cl_exact_chunk), eight positions at a time.
+// scaled per output channel by a power of two when they are packed.  Activations by 16: their parts hold 22 bits of a value in [2^-16, 4092) and smaller
+// ones to 2^-40 absolute.  A row's block of 32 channels with a value from 4092 on, an infinity, a NaN, or nothing but values below 2^-16 is kept as
+// it is in fp32, and the positions into which it goes are multiplied in fp32 on CUDA cores (cl_exact_chunk).  So every value is held to 2^-24
+// of the largest beside it, however quiet the passage; and since a row's code and a position's way follow from what goes into them alone, an
+// entry's bits do not depend on its batch.
 // What only these convolutions read is written as parts by the kernel that produces it, in the bytes its fp32 values would have taken, and
 // fetched by TMA: nothing is converted here, and a tap is the same tile in shared memory read from a later row on.  Activations that come
 // as fp32 are split on the way by eight warps, once per tile and 64 channels for all taps.
@@ -40,9 +42,10 @@ constexpr int CL_ROWS = 256;                // rows of a stage of activations: c
 constexpr int CL_W_BLOCK = 128 * 128;       // 128 output channels x 32 input channels, high and low parts
 constexpr int CL_TAIL = 8192;               // barriers, tables, alignment
 constexpr float CL_X_SCALE = 16.f, CL_LO_SCALE = 2048.f;      // of activations; of low parts against high ones
-// what the two parts of an activation hold to 2^-22: a tile whose largest value is not between these (or zero) is multiplied on CUDA cores
+// what the two parts of an activation hold to 2^-22.  Where the largest value is not between these (or zero) -- of a block kept as parts, of what goes
+// into one result of fp32 activations -- the products are taken on CUDA cores
 constexpr float CL_X_TOP = 65472.f / CL_X_SCALE, CL_X_LOW = 0x1p-12f / CL_X_SCALE;
-enum ClCode { CB_NORMAL = 1, CB_QUIET = 2, CB_RAW = 4 };      // of a block of 32 activations kept as parts (all zero: 0)
+enum ClCode { CB_NORMAL = 1, CB_RAW = 4 };      // of a block of 32 activations kept as parts (all zero: 0)
 
 struct ClConvParams {
   const uint8_t* w;          // [128 channels][32 of K][128][32 hi | 32 lo], rows of 128 bytes swizzled
@@ -97,6 +100,11 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, uint32_t src,
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const float (&v)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
                ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
@@ -114,6 +122,13 @@ __device__ __forceinline__ float2 unpack_f16(uint32_t v) {
 __device__ __forceinline__ float max3_abs(float a, float b, float c) {
   float r;
   asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// the smaller magnitude of three
+__device__ __forceinline__ float min3_abs(float a, float b, float c) {
+  float r;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
 
@@ -167,8 +182,9 @@ __device__ __forceinline__ void cl_exchange(uint32_t hi, uint32_t lo, uint32_t& 
   w1 = __byte_perm(own, got, odd ? 0x3276u : 0x7632u);
 }
 // what a block of 32 activations with the largest magnitude m is kept as
-__device__ __forceinline__ uint32_t cl_code(float m) { return !(m < CL_X_TOP) ? CB_RAW : m == 0.f ? 0u : m < CL_X_LOW ? CB_QUIET : CB_NORMAL; }
-// Activations kept as parts: 128 bytes per 32 channels as in fp32, [32 high | 32 low] fp16 -- or, where one of the 32 is out of range, the fp32
+__device__ __forceinline__ bool cl_fits(float m) { return __float_as_uint(m) - __float_as_uint(CL_X_LOW) < __float_as_uint(CL_X_TOP) - __float_as_uint(CL_X_LOW); }
+__device__ __forceinline__ uint32_t cl_code(float m) { return cl_fits(m) ? CB_NORMAL : m == 0.f ? 0u : CB_RAW; }      // (zeros are the same bits either way)
+// Activations kept as parts: 128 bytes per 32 channels as in fp32, [32 high | 32 low] fp16 -- or, where the largest of the 32 is out of range, the fp32
 // values themselves, with CB_RAW in the block's code byte.  Here for eight neighbouring lanes that hold a block's channels, four each.
 __device__ __forceinline__ void cl_put4(uint32_t* yp, uint8_t* code, size_t at, const float4& v) {
   float m = max3_abs(max3_abs(v.x, v.y, v.z), v.w, v.w);
@@ -180,7 +196,7 @@ __device__ __forceinline__ void cl_put4(uint32_t* yp, uint8_t* code, size_t at, 
   }
   const uint32_t c = cl_code(m), in = static_cast<uint32_t>(at) & 31u;
   uint32_t* blk = yp + (at - in);
-  if (c == CB_RAW) {
+  if (!cl_fits(m)) {
     *reinterpret_cast<float4*>(blk + in) = v;
   } else {
     uint2 hi, lo;
@@ -200,7 +216,7 @@ __device__ __forceinline__ void cl_put1(uint32_t* yp, uint8_t* code, size_t bloc
   uint32_t hi, lo, word, unused;
   cl_parts(f2(v, 0.f), CL_X_SCALE, hi, lo);
   cl_exchange(hi, lo, word, unused);
-  if (c == CB_RAW) yp[block * 32 + lane] = __float_as_uint(v);
+  if (!cl_fits(m)) yp[block * 32 + lane] = __float_as_uint(v);
   else yp[block * 32 + (lane & 1 ? 16 : 0) + (lane >> 1)] = word;
   if (lane == 0) code[block] = static_cast<uint8_t>(c);
 }
@@ -280,20 +296,63 @@ __device__ __forceinline__ ClUnit cl_unit(const ClConvParams& p, int u) {
   return r;
 }
 
-// Eight columns of a tile outside the split's range, in fp32: this warp's 32 channels, blocks [blk_lo, blk_hi) of K.  The weights come from their
-// packed parts.  Writes the accumulators, so that the epilogue goes on as if the products had.
+// Which of eight columns are outside the parts' range: a bit each.  Of activations as fp32 this block's own channels [blk_lo, blk_hi) count -- all
+// tiny, or one too large -- of parts the codes of all of them: in either case what the flag that a unit is looked at for was found from.
+template <bool PARTS>
+__device__ __noinline__ uint32_t cl_exact_columns(const ClConvParams& p, const int4* col_tab, int t0, int b0, int c0, int blk_lo, int blk_hi) {
+  const int lane = threadIdx.x & 31, part = lane >> 3, e = col_tab[c0 + (lane & 7)].x;         // four lanes a column
+  uint32_t code = 0u;
+  float m = 0.f;
+  const int b = b0 + (e >> 16), t = t0 + (e & 0xffff);
+  if (e >= 0 && b < p.B && t < p.n_hi) {
+#pragma unroll 1
+    for (int tap = 0; tap < p.ksize; ++tap) {
+      const int ts = t - (p.ksize - 1 - tap) * p.dil;
+      if (ts < 0 || ts >= p.Tx) continue;
+      const long long row = b * p.x_bstride + static_cast<long long>(ts) * p.Cin;
+      if (PARTS) {
+#pragma unroll 4
+        for (int k = part; k < p.Cin >> 5; k += 4) code |= __ldcg(p.x_code + (row >> 5) + k);
+      } else {
+#pragma unroll 4
+        for (int k = blk_lo * 32 + part * 4; k < blk_hi * 32; k += 16) {
+          const float4 v = __ldcg(reinterpret_cast<const float4*>(p.x + row + k));
+          m = max3_abs(max3_abs(m, v.x, v.y), v.z, v.w);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 8; o < 32; o <<= 1) {
+    const float other = __shfl_xor_sync(0xffffffffu, m, o);
+    m = max3_abs(m, other, other);
+    code |= __shfl_xor_sync(0xffffffffu, code, o);
+  }
+  return __ballot_sync(0xffffffffu, (PARTS ? code : cl_code(m)) & CB_RAW) & 0xffu;
+}
+// Eight columns of a unit that is looked at: the accumulators in the plain scale, and the columns of `mask` multiplied again in fp32 -- this warp's
+// 32 channels, blocks [blk_lo, blk_hi) of K.  The weights come from their packed parts.  The epilogue goes on as if the products had given this,
+// the factor of the channel being 1.
 __device__ __noinline__ void cl_exact_chunk(const ClConvParams& p, const int4* col_tab, int m0, int t0, int b0, int c0, int lane_row,
-                                            int blk_lo, int blk_hi, uint32_t t_hi, uint32_t t_lo) {
+                                            int blk_lo, int blk_hi, uint32_t t_hi, uint32_t t_lo, uint32_t mask, float inv) {
   float out[8];
+  {
+    uint32_t hi[8], lo[8];
+    tmem_ld_32x8(t_hi, hi);
+    tmem_ld_32x8(t_lo, lo);
+    tmem_ld_wait();
+#pragma unroll
+    for (int c = 0; c < 8; ++c) out[c] = fmaf(__uint_as_float(lo[c]), 1.f / CL_LO_SCALE, __uint_as_float(hi[c])) * inv;
+  }
   const int blocks_per_tap = p.Cin >> 5;
   const uint8_t* wt = p.w + static_cast<size_t>(m0 >> 7) * (blocks_per_tap * p.ksize) * CL_W_BLOCK + lane_row * 128;
   const float w_scale = p.w_inv[m0 + lane_row] * CL_X_SCALE;
 #pragma unroll 1
   for (int c = 0; c < 8; ++c) {
-    const int e = col_tab[c0 + c].x;
+    if (!(mask >> c & 1u)) continue;
     float acc = 0.f;
-    if (e >= 0) {
-      const int b = b0 + (e >> 16), t = t0 + (e & 0xffff);
+    {
+      const int e = col_tab[c0 + c].x, b = b0 + (e >> 16), t = t0 + (e & 0xffff);
 #pragma unroll 1
       for (int tap = 0; tap < p.ksize; ++tap) {
         const int ts = t - (p.ksize - 1 - tap) * p.dil;
@@ -318,7 +377,8 @@ __device__ __noinline__ void cl_exact_chunk(const ClConvParams& p, const int4* c
         }
       }
     }
-    out[c] = acc;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) out[k] = k == c ? acc : out[k];
   }
   tmem_st_32x8(t_hi, out);
 #pragma unroll
@@ -347,11 +407,6 @@ struct ClHot {
 // The epilogue works on eight columns at a time, in a loop that is short enough for the instruction caches: sixteen columns in straight-line
 // code took twice as long (Mimi's 1x1 layer of 153600 x 128 85 us).
 constexpr int CL_EC = 8;
-__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(taddr));
-}
 // where column c0 + (lane & 7) lies: its entry in the table, or x = -1 where there is no such position
 __device__ __forceinline__ int4 cl_column(const ClConvParams& p, const ClUnit& g, const int4* col_tab, int c0) {
   int4 tb = col_tab[c0 + (threadIdx.x & (CL_EC - 1))];
@@ -448,28 +503,66 @@ __device__ __forceinline__ void cl_store(const ClConvParams& p, const ClHot& h, 
   }
   cl_store(p, h, g, col_tab, c0, inside, reinterpret_cast<uint32_t*>(y), w);
 }
-// eight rows of a block as parts.  One code for all of them: what is out of range somewhere in a chunk is kept as it is in all of it
+// Whether eight rows of a block are all of ordinary size: no value out of range, and a lane none of whose rows is tiny.  (Nearly always; a chunk that
+// this does not hold for is looked at row by row.)  `rows`: a bit for each that there is.  One code for a chunk, its largest value's, cost 8 of Mimi's
+// 1262 us less, and let a loud row's neighbours lose what they are made of.
+__device__ __forceinline__ bool cl_ordinary(const F2 (&v)[CL_EC / 2], uint32_t rows) {
+  float top = 0.f, low = CL_X_TOP;
+#pragma unroll
+  for (int c = 0; c < CL_EC / 2; ++c) {
+    float2 x = f2_get(v[c]);
+    if (rows != 0xffu) {
+      if (!(rows >> (2 * c) & 1u)) x.x = 1.f;
+      if (!(rows >> (2 * c) & 2u)) x.y = 1.f;
+    }
+    top = max3_abs(top, x.x, x.y);
+    low = min3_abs(low, x.x, x.y);
+  }
+  return __all_sync(0xffffffffu, top < CL_X_TOP) && __any_sync(0xffffffffu, low >= CL_X_LOW);
+}
+// a row of a block on its own: word `at` of the row -> its bits, and the row's code
+__device__ __forceinline__ uint32_t cl_odd_row(float x, int& at, uint32_t& bits) {
+  const int lane = threadIdx.x & 31;
+  float m = x;
+  asm volatile("redux.sync.max.NaN.abs.f32 %0, %0, 0xffffffff;" : "+f"(m));
+  const uint32_t code = cl_code(m);
+  uint32_t hi, lo, unused;
+  cl_parts(f2(x, 0.f), CL_X_SCALE, hi, lo);
+  cl_exchange(hi, lo, bits, unused);
+  at = (lane & 1 ? 16 : 0) + (lane >> 1);
+  if (!cl_fits(m)) {
+    at = lane;
+    bits = __float_as_uint(x);
+  }
+  return code;
+}
+// ... eight of them; the lane's row: whether there is one, and its offset -> the lane's code
+__device__ __noinline__ uint32_t cl_odd_store(uint32_t* yp, int ok, int where, F2 a, F2 b, F2 c, F2 d) {
+  const F2 v[CL_EC / 2] = {a, b, c, d};
+  uint32_t code = 0u;
+#pragma unroll
+  for (int r = 0; r < CL_EC; ++r) {
+    const float2 xy = f2_get(v[r >> 1]);
+    int at;
+    uint32_t bits;
+    const uint32_t row = cl_odd_row(r & 1 ? xy.y : xy.x, at, bits);
+    const bool there = __shfl_sync(0xffffffffu, ok, r);
+    const int o = __shfl_sync(0xffffffffu, where, r);
+    if (there) yp[o + at] = bits;
+    if ((threadIdx.x & 7) == r) code = row;
+  }
+  return code;
+}
+// eight rows of a block as parts; rows out of range as they are
 __device__ __forceinline__ void cl_store_parts(const ClConvParams& p, const ClHot& h, const ClEpiState& e, const ClUnit& g, const int4* col_tab, int c0, int inside,
                                                const F2 (&v)[CL_EC / 2]) {
   const int lane = threadIdx.x & 31;
   const int4 tb = cl_column(p, g, col_tab, c0);
-  float m = 0.f;
-#pragma unroll
-  for (int c = 0; c < CL_EC / 2; ++c) {
-    float2 x = f2_get(v[c]);
-    if (c0 + CL_EC > inside) {
-      x.x = __shfl_sync(0xffffffffu, tb.x, 2 * c) >= 0 ? x.x : 0.f;
-      x.y = __shfl_sync(0xffffffffu, tb.x, 2 * c + 1) >= 0 ? x.y : 0.f;
-    }
-    m = max3_abs(m, x.x, x.y);
-  }
-  asm volatile("redux.sync.max.NaN.abs.f32 %0, %0, 0xffffffff;" : "+f"(m));
-  const uint32_t code = cl_code(m);
+  uint32_t code = CB_NORMAL;
+  const bool ordinary = cl_ordinary(v, __ballot_sync(0xffffffffu, tb.x >= 0) & 0xffu);
+  if (!ordinary) code = cl_odd_store(e.yp, tb.x >= 0, tb.y, v[0], v[1], v[2], v[3]);
   if (lane < CL_EC && tb.x >= 0) e.code[tb.y >> 5] = static_cast<uint8_t>(code);
-  if (code == CB_RAW) {
-    cl_store(p, h, g, col_tab, c0, inside, reinterpret_cast<float*>(e.yp + lane), v);
-    return;
-  }
+  if (!ordinary) return;
   uint32_t w[CL_EC];
 #pragma unroll
   for (int c = 0; c < CL_EC / 2; ++c) {
@@ -505,7 +598,7 @@ __device__ __forceinline__ void cl_boxed_chunks(const ClHot& h, const ClMaps& ma
   const int lane = threadIdx.x & 31, cols = h.cols;
   const bool two = h.two, res = h.res, parts = h.parts;
 #pragma unroll 1
-  for (int c0 = c_first; c0 < cols; c0 += c_step) {
+  for (int c0 = c_first; c0 < inside; c0 += c_step) {          // (chunks behind the last position have nothing to leave)
     const uint32_t in = bx.at + (bx.flip ? 1024u : 0u) + lane * 4;                       // residuals, or plain values
     const uint32_t out = bx.at + (res ? 2048u : two ? (bx.flip ? 3072u : 1024u) : 2048u) + (res || !two ? (bx.flip ? 1024u : 0u) : 0u);
     const uint32_t plain = bx.at + (bx.flip ? 2048u : 0u);
@@ -513,7 +606,7 @@ __device__ __forceinline__ void cl_boxed_chunks(const ClHot& h, const ClMaps& ma
       bw.wait(bx.res_full, bx.res_ph);
       if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; return; }
       bx.res_ph ^= 1u;
-      if (lane == 0 && c0 + c_step < cols) {           // (the other box has been read: every lane has passed the chunk in front)
+      if (lane == 0 && c0 + c_step < inside) {         // (the other box has been read: every lane has passed the chunk in front)
         mbar_arrive_expect_tx(bx.res_full, 1024u);
         tma_load_3d(bx.at + (bx.flip ? 0u : 1024u), &maps.r, smem_u32(bx.res_full), n_box, t0 + c0 + c_step, b0);
       }
@@ -553,26 +646,8 @@ __device__ __forceinline__ void cl_boxed_chunks(const ClHot& h, const ClMaps& ma
     if (two) put(plain + lane * 4);
     cl_act<ACT>(e, v);
     if (parts) {
-      float m = 0.f;
-      if (c0 + CL_EC <= inside) {
-#pragma unroll
-        for (int c = 0; c < CL_EC / 2; ++c) {
-          const float2 x = f2_get(v[c]);
-          m = max3_abs(m, x.x, x.y);
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < CL_EC / 2; ++c) {
-          const float2 x = f2_get(v[c]);
-          m = max3_abs(m, c0 + 2 * c < inside ? x.x : 0.f, c0 + 2 * c + 1 < inside ? x.y : 0.f);
-        }
-      }
-      asm volatile("redux.sync.max.NaN.abs.f32 %0, %0, 0xffffffff;" : "+f"(m));
-      const uint32_t code = cl_code(m);
-      if (lane < CL_EC && c0 + lane < inside) e.code[(c0 + lane) * (h.N >> 5)] = static_cast<uint8_t>(code);
-      if (code == CB_RAW) {
-        put(out + lane * 4);
-      } else {
+      uint32_t code = CB_NORMAL;
+      if (c0 + CL_EC <= inside && cl_ordinary(v, 0xffu)) {          // (the last chunk of a sequence may go row by row)
         const uint32_t a = out + (lane & 1 ? 64u : 0u) + (lane >> 1) * 4;
 #pragma unroll
         for (int c = 0; c < CL_EC / 2; ++c) {
@@ -582,7 +657,20 @@ __device__ __forceinline__ void cl_boxed_chunks(const ClHot& h, const ClMaps& ma
           asm volatile("st.shared.b32 [%0], %1;" ::"r"(a + 2 * c * 128), "r"(w0) : "memory");
           asm volatile("st.shared.b32 [%0], %1;" ::"r"(a + (2 * c + 1) * 128), "r"(w1) : "memory");
         }
+      } else {
+        put(out + lane * 4);
+#pragma unroll 1
+        for (int r = 0; r < CL_EC; ++r) {          // (every lane has read its value when the lanes have exchanged theirs)
+          float x;
+          int at;
+          uint32_t bits;
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(out + r * 128 + lane * 4) : "memory");
+          const uint32_t row = cl_odd_row(x, at, bits);
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(out + r * 128 + at * 4), "r"(bits) : "memory");
+          if ((lane & 7) == r) code = row;
+        }
       }
+      if (lane < CL_EC && c0 + lane < inside) e.code[(c0 + lane) * (h.N >> 5)] = static_cast<uint8_t>(code);
     } else {
       put(out + lane * 4);
     }
@@ -601,7 +689,7 @@ struct ClSplit {
   uint32_t smem0;
   int x_bytes, u_first, u_step, kb_lo, x_steps;
   uint64_t *x_ready, *x_empty, *top_full, *top_empty;
-  float* tops;
+  uint32_t* tops;
   const int2* row_tab;
 };
 // The split's loop.  A thread takes one 16-byte chunk of every 16th row (32nd where a stage is 32 channels wide): NP rows of a stage, in batches
@@ -650,7 +738,7 @@ __device__ __forceinline__ void cl_split(const ClConvParams& p, const ClSplit& s
   }
   int s = 0, it = 0;
   uint32_t ph = 0;
-  float top = 0.f;
+  uint32_t top = 0u, low = 0xffffffffu;        // bits of the largest four-channel magnitude, and of the smallest that is not zero, less one
 #pragma unroll 1
   while (u < p.units) {
     int nu = u, ns = st, nh = half + 1;
@@ -681,7 +769,9 @@ __device__ __forceinline__ void cl_split(const ClConvParams& p, const ClSplit& s
           uint32_t h0, h1, l0, l1;
           cl_parts(f2(v[j].x, v[j].y), CL_X_SCALE, h0, l0);
           cl_parts(f2(v[j].z, v[j].w), CL_X_SCALE, h1, l1);
-          top = max3_abs(max3_abs(top, v[j].x, v[j].y), v[j].z, v[j].w);
+          const uint32_t m = __float_as_uint(max3_abs(max3_abs(v[j].x, v[j].y, v[j].z), v[j].w, v[j].w));         // (a NaN has the largest)
+          top = max(top, m);
+          low = min(low, m - 1u);
           const uint32_t a = dst0 + s * sp.x_bytes + pass * rows_pass * 128;
           asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(h0), "r"(h1) : "memory");
           asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a ^ 64u), "r"(l0), "r"(l1) : "memory");
@@ -697,10 +787,11 @@ __device__ __forceinline__ void cl_split(const ClConvParams& p, const ClSplit& s
       if (on && j % PB == PB - 1 && (HALVES == 1 || half == HALVES - 1)) {        // the warp's rows of the stage are there
         const bool last = st + j / PB + 1 == sp.x_steps;
         if (last) {
-          asm volatile("redux.sync.max.NaN.abs.f32 %0, %0, 0xffffffff;" : "+f"(top));
+          const bool look = __any_sync(0xffffffffu, top >= __float_as_uint(CL_X_TOP) || low < __float_as_uint(CL_X_LOW) - 1u);
           bw.wait(&sp.top_empty[it & 7], ((it >> 3) & 1) ^ 1);
-          if (lane == 0) sp.tops[(it & 7) * CL_SPLIT_WARPS + wsp] = top;
-          top = 0.f;
+          if (lane == 0) sp.tops[(it & 7) * CL_SPLIT_WARPS + wsp] = look;
+          top = 0u;
+          low = 0xffffffffu;
         }
         __syncwarp();
         if (lane == 0) {
@@ -742,7 +833,7 @@ __global__ void __launch_bounds__(ClRoles<PARTS>::THREADS, 1) cl_conv_kernel(con
   uint64_t* res_full = top_empty + CL_TOPS;                     // [EPI_WARPS]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(res_full + 12);
   const uint32_t gate = smem_u32(tmem_slot + 1);                // set once the kernels in front have completed
-  float* tops = reinterpret_cast<float*>(tail + 640);           // [CL_TOPS][CL_SPLIT_WARPS] largest magnitudes; with PARTS one word of codes
+  uint32_t* tops = reinterpret_cast<uint32_t*>(tail + 640);     // [CL_TOPS][CL_SPLIT_WARPS] whether a unit may have columns out of range (PARTS: one word)
   int2* row_tab = reinterpret_cast<int2*>(tail + 1024);         // [CL_ROWS] (entry << 16 | row of the entry) or -1, offset in x
   int4* col_tab = reinterpret_cast<int4*>(tail + 1024 + CL_ROWS * 8);      // [CL_ROWS] the same or -1, offsets in y, resid, noise
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -920,11 +1011,11 @@ __global__ void __launch_bounds__(ClRoles<PARTS>::THREADS, 1) cl_conv_kernel(con
       }
       code = __reduce_or_sync(0xffffffffu, code);
       code |= code >> 16;
-      code = (code | code >> 8) & 0xffu;
+      const bool look = (code | code >> 8) & CB_RAW;
       bw.wait(&top_empty[it & (CL_TOPS - 1)], ((it / CL_TOPS) & 1) ^ 1);
       if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
       if (lane == 0) {
-        tops[(it & (CL_TOPS - 1)) * CL_SPLIT_WARPS] = __uint_as_float(code);
+        tops[(it & (CL_TOPS - 1)) * CL_SPLIT_WARPS] = look;
         mbar_arrive(&top_full[it & (CL_TOPS - 1)]);
       }
       __syncwarp();
@@ -996,29 +1087,22 @@ __global__ void __launch_bounds__(ClRoles<PARTS>::THREADS, 1) cl_conv_kernel(con
         if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; return; }
         tc_fence_after();
         first = false;
-        bool exact;
-        if (PARTS) {
-          const uint32_t code = __float_as_uint(tops[(it & (CL_TOPS - 1)) * CL_SPLIT_WARPS]);
-          exact = (code & CB_RAW) || code == CB_QUIET;
-        } else {                                                        // (a NaN has the largest bits)
-          const float top = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(tops[(it & (CL_TOPS - 1)) * CL_SPLIT_WARPS + (lane & 7)])));
-          exact = !(top < CL_X_TOP) || (top < CL_X_LOW && top > 0.f);
-        }
-        __syncwarp();
+        const bool look = __any_sync(0xffffffffu, tops[(it & (CL_TOPS - 1)) * CL_SPLIT_WARPS + (PARTS ? 0 : lane & 7)] != 0u);
         if (lane == 0) mbar_arrive(&top_empty[it & (CL_TOPS - 1)]);
-        if (exact) {
+        if (look) {
           if (mine) {
+            const int blk_lo = kb_lo * p.group, blk_hi = (kb_lo + kb_n) * p.group;
 #pragma unroll 1
             for (int c0 = turn * CL_EC; c0 < p.cols; c0 += turns * CL_EC)
-              cl_exact_chunk(p, col_tab, g.m0, g.t0, g.b0, c0, lane_row, kb_lo * p.group, (kb_lo + kb_n) * p.group, taddr + c0,
-                             taddr + p.cols + c0);
+              cl_exact_chunk(p, col_tab, g.m0, g.t0, g.b0, c0, lane_row, blk_lo, blk_hi, taddr + c0, taddr + p.cols + c0,
+                             cl_exact_columns<PARTS>(p, col_tab, g.t0, g.b0, c0, blk_lo, blk_hi), inv);
           }
           inv = 1.f;
         }
       };
       if (p.staged) {
         const int c_first = turn * CL_EC, c_step = turns * CL_EC, n_box = g.m0 + (row & ~31);
-        const bool some = mine && c_first < h.cols;
+        const bool some = mine && c_first < inside;
         if (some && h.res && lane == 0) {          // the first residuals, asked for before the accumulator is waited for
           mbar_arrive_expect_tx(bx.res_full, 1024u);
           tma_load_3d(bx.at + (bx.flip ? 1024u : 0u), &maps.r, smem_u32(bx.res_full), n_box, g.t0 - p.n_lo + c_first, g.b0);

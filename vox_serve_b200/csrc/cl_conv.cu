@@ -105,10 +105,11 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&v)[8]) {
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const float (&v)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-               ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-               : "memory");
+__device__ __forceinline__ void tmem_ld_32x4(uint32_t taddr, uint32_t (&v)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st_32x4(uint32_t taddr, const float (&v)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
 }
 __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
   uint32_t r;
@@ -330,60 +331,71 @@ __device__ __noinline__ uint32_t cl_exact_columns(const ClConvParams& p, const i
   }
   return __ballot_sync(0xffffffffu, (PARTS ? code : cl_code(m)) & CB_RAW) & 0xffu;
 }
-// Eight columns of a unit that is looked at: the accumulators in the plain scale, and the columns of `mask` multiplied again in fp32 -- this warp's
+// Four columns of a unit that is looked at: the accumulators in the plain scale, and the columns of `mask` multiplied again in fp32 -- this warp's
 // 32 channels, blocks [blk_lo, blk_hi) of K.  The weights come from their packed parts.  The epilogue goes on as if the products had given this,
-// the factor of the channel being 1.
+// the factor of the channel being 1.  A block of 32 inputs at a time: a lane holds its channel's weights and, of every column, the input of its
+// number, which goes round by shuffles.  5120 rows of 1536 x 1024 take 50 us, with one value of 5000 132, with nothing but such values 4.3 ms (element
+// by element 61 and 141 ms); 640 rows of 2048 x 512 15, 52 and 440 us.  (Four or eight weights more in flight cost the epilogue registers: Mimi 1262 us,
+// 1273 and 1285.)
 __device__ __noinline__ void cl_exact_chunk(const ClConvParams& p, const int4* col_tab, int m0, int t0, int b0, int c0, int lane_row,
                                             int blk_lo, int blk_hi, uint32_t t_hi, uint32_t t_lo, uint32_t mask, float inv) {
-  float out[8];
-  {
-    uint32_t hi[8], lo[8];
-    tmem_ld_32x8(t_hi, hi);
-    tmem_ld_32x8(t_lo, lo);
-    tmem_ld_wait();
-#pragma unroll
-    for (int c = 0; c < 8; ++c) out[c] = fmaf(__uint_as_float(lo[c]), 1.f / CL_LO_SCALE, __uint_as_float(hi[c])) * inv;
-  }
-  const int blocks_per_tap = p.Cin >> 5;
+  const int lane = threadIdx.x & 31, blocks_per_tap = p.Cin >> 5, sw = lane_row & 7;
   const uint8_t* wt = p.w + static_cast<size_t>(m0 >> 7) * (blocks_per_tap * p.ksize) * CL_W_BLOCK + lane_row * 128;
   const float w_scale = p.w_inv[m0 + lane_row] * CL_X_SCALE;
+  const long long base = b0 * p.x_bstride + static_cast<long long>(t0) * p.Cin;
+  float acc[4] = {};
 #pragma unroll 1
-  for (int c = 0; c < 8; ++c) {
-    if (!(mask >> c & 1u)) continue;
-    float acc = 0.f;
-    {
-      const int e = col_tab[c0 + c].x, b = b0 + (e >> 16), t = t0 + (e & 0xffff);
+  for (int tap = 0; tap < p.ksize && mask; ++tap) {
+    const int shift = (p.ksize - 1 - tap) * p.dil;
+    // lane c: where column c's row lies; the columns that have one
+    const int e = col_tab[c0 + (lane & 3)].x, q0 = (e & 0xffff) - shift, at_lane = static_cast<int>((e >> 16) * p.x_bstride) + q0 * p.Cin;
+    const uint32_t in = __ballot_sync(0xffffffffu, t0 + q0 >= 0 && t0 + q0 < p.Tx) & mask;
 #pragma unroll 1
-      for (int tap = 0; tap < p.ksize; ++tap) {
-        const int ts = t - (p.ksize - 1 - tap) * p.dil;
-        const bool in = b < p.B && ts >= 0 && ts < p.Tx;
-        const long long row = in ? b * p.x_bstride + static_cast<long long>(ts) * p.Cin : 0ll;
+    for (int blk = blk_lo; blk < blk_hi; ++blk) {
+      float x[4];
+      const uint32_t parts = __ballot_sync(0xffffffffu, p.x_code && (in >> (lane & 3) & 1u) && !(__ldcg(p.x_code + ((base + at_lane) >> 5) + blk) & CB_RAW));
+#pragma unroll
+      for (int c = 0; c < 4; ++c) x[c] = in >> c & 1u ? __ldcg(p.x + base + __shfl_sync(0xffffffffu, at_lane, c) + blk * 32 + lane) : 0.f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if (parts >> c & 1u) {
+          const uint32_t word = __float_as_uint(x[c]);
+          const float2 fh = unpack_f16(__shfl_sync(0xffffffffu, word, lane >> 1)), fl = unpack_f16(__shfl_sync(0xffffffffu, word, 16 + (lane >> 1)));
+          x[c] = fmaf(lane & 1 ? fl.y : fl.x, 1.f / CL_LO_SCALE, lane & 1 ? fh.y : fh.x) * (1.f / CL_X_SCALE);
+        }
+      }
+      const uint8_t* wb = wt + static_cast<size_t>(tap * blocks_per_tap + blk) * CL_W_BLOCK;
 #pragma unroll 1
-        for (int k = blk_lo * 32; k < blk_hi * 32; ++k) {
-          const uint8_t* blk = wt + static_cast<size_t>(tap * blocks_per_tap + (k >> 5)) * CL_W_BLOCK + (k & 7) * 2;
-          const int chunk = (k >> 3) & 3, sw = lane_row & 7;
-          const float hi = __half2float(*reinterpret_cast<const __half*>(blk + ((chunk ^ sw) << 4))),
-                      lo = __half2float(*reinterpret_cast<const __half*>(blk + (((chunk + 4) ^ sw) << 4)));
-          float xv = 0.f;
-          if (in) {
-            if (!p.x_code || (__ldcg(p.x_code + ((row + k) >> 5)) & CB_RAW)) {
-              xv = __ldcg(p.x + row + k);
-            } else {
-              const __half* xb = reinterpret_cast<const __half*>(p.x + ((row + k) & ~31ll));
-              xv = fmaf(__half2float(__ldcg(xb + 32 + (k & 31))), 1.f / CL_LO_SCALE, __half2float(__ldcg(xb + (k & 31)))) * (1.f / CL_X_SCALE);
-            }
-          }
-          acc = fmaf(xv, fmaf(lo, 1.f / CL_LO_SCALE, hi) * w_scale, acc);
+      for (int q = 0; q < 4; ++q) {
+        const uint4 hi = __ldg(reinterpret_cast<const uint4*>(wb + ((q ^ sw) << 4))), lo = __ldg(reinterpret_cast<const uint4*>(wb + (((q + 4) ^ sw) << 4)));
+        const uint32_t h[4] = {hi.x, hi.y, hi.z, hi.w}, l[4] = {lo.x, lo.y, lo.z, lo.w};
+        float w[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 fh = unpack_f16(h[i]), fl = unpack_f16(l[i]);
+          w[2 * i] = fmaf(fl.x, 1.f / CL_LO_SCALE, fh.x) * w_scale;
+          w[2 * i + 1] = fmaf(fl.y, 1.f / CL_LO_SCALE, fh.y) * w_scale;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (!(mask >> c & 1u)) continue;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) acc[c] = fmaf(__shfl_sync(0xffffffffu, x[c], 8 * q + k), w[k], acc[c]);
         }
       }
     }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) out[k] = k == c ? acc : out[k];
   }
-  tmem_st_32x8(t_hi, out);
+  uint32_t hi[4], lo[4];
+  tmem_ld_32x4(t_hi, hi);
+  tmem_ld_32x4(t_lo, lo);
+  tmem_ld_wait();
 #pragma unroll
-  for (int c = 0; c < 8; ++c) out[c] = 0.f;
-  tmem_st_32x8(t_lo, out);
+  for (int c = 0; c < 4; ++c)
+    if (!(mask >> c & 1u)) acc[c] = fmaf(__uint_as_float(lo[c]), 1.f / CL_LO_SCALE, __uint_as_float(hi[c])) * inv;
+  tmem_st_32x4(t_hi, acc);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) acc[c] = 0.f;
+  tmem_st_32x4(t_lo, acc);
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
@@ -1093,9 +1105,12 @@ __global__ void __launch_bounds__(ClRoles<PARTS>::THREADS, 1) cl_conv_kernel(con
           if (mine) {
             const int blk_lo = kb_lo * p.group, blk_hi = (kb_lo + kb_n) * p.group;
 #pragma unroll 1
-            for (int c0 = turn * CL_EC; c0 < p.cols; c0 += turns * CL_EC)
-              cl_exact_chunk(p, col_tab, g.m0, g.t0, g.b0, c0, lane_row, blk_lo, blk_hi, taddr + c0, taddr + p.cols + c0,
-                             cl_exact_columns<PARTS>(p, col_tab, g.t0, g.b0, c0, blk_lo, blk_hi), inv);
+            for (int c0 = turn * CL_EC; c0 < p.cols; c0 += turns * CL_EC) {
+              const uint32_t mask = cl_exact_columns<PARTS>(p, col_tab, g.t0, g.b0, c0, blk_lo, blk_hi);
+#pragma unroll 1
+              for (int c = c0; c < c0 + CL_EC; c += 4)
+                cl_exact_chunk(p, col_tab, g.m0, g.t0, g.b0, c, lane_row, blk_lo, blk_hi, taddr + c, taddr + p.cols + c, mask >> (c - c0) & 15u, inv);
+            }
           }
           inv = 1.f;
         }

@@ -209,7 +209,9 @@ __device__ __noinline__ float smp_quotient(float a, float b) { return a / b; }
 // `far` grows past SMP_FAR where the product leaves [2^-79, 2^81): extreme dividends, zeros (the remainder loses their sign), infinities
 // and NaNs.  Those take the division itself.  (The quotients of bf16 values by one of few bits lie on the middle of two bf16 values so often
 // that asking whether the product's rounding is sure costs more than the corrections.)
+// The remainder is exact while its last bit, 2^-46 of quotient times divisor, is an fp32 value: divisors from 2^-20 on (2^-79 2^-20 2^-46 = 2^-145).
 constexpr uint32_t SMP_FAR = 0xa0000000u;
+constexpr float SMP_DIVISOR_LOW = 0x1p-20f;
 __device__ __forceinline__ float smp_div(float a, float b, float y, uint32_t& far) {
   float q = a * y;
   far = max(far, (__float_as_uint(q) << 1) - 0x30000000u);
@@ -265,7 +267,7 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SamplePara
   const bool wide = (odd & 3) == 0, even = (odd & 1) == 0;
   const int n_seen = rep0 ? p.W : 0;
   const float inv_temperature = 1.f / p.temperature;
-  const uint32_t far_temperature = p.temperature > 0x1p-40f && p.temperature < 0x1p40f ? 0u : SMP_FAR;
+  const uint32_t far_temperature = p.temperature > SMP_DIVISOR_LOW && p.temperature < 0x1p40f ? 0u : SMP_FAR;
   uint32_t kloc = 0u;
   auto tok_index = [&](int j, int half) { return 2 * ((j * S + rank) * SMP_THREADS + tid) + half; };
   {

@@ -914,11 +914,11 @@ def test_sampler_quotients(ops, penalty):
 @pytest.mark.parametrize("a,b,t", [(2.7506567809241528e-36, 2.7624117244323756e-36, 1.0830623507415704e-12), (5.571843222897643e-36, 5.5953531099140885e-36, 1.3514122546715024e-12),
                                    (4.490388420141138e-36, 4.513898307157584e-36, 1.893335098077098e-12)])
 def test_sampler_quotients_of_tiny_values(ops, a, b, t):
-    x = torch.tensor([[a, b]], device="cuda").bfloat16().repeat(64, 1)
+    x = torch.tensor([[a, b, a, b]], device="cuda").bfloat16().repeat(64, 1)          # (four: a token of a unit past the vocabulary takes the division)
     q = (x.cpu().float() / torch.full_like(x.cpu().float(), t)).bfloat16()      # (divided: a scalar divisor may be taken as a factor)
-    assert (q[:, 0] == q[:, 1]).all()
-    ids = ops.sample(x, "top_k", top_k=1, temperature=t, seed=3)                 # a tie: both are drawn
-    assert set(ids.flatten().tolist()) == {0, 1}
+    assert (q == q[0, 0]).all()
+    ids = ops.sample(x, "top_k", top_k=1, temperature=t, seed=3)                 # a tie: all are drawn
+    assert set(ids.flatten().tolist()) == {0, 1, 2, 3}
 
 
 @pytest.mark.parametrize("V", [1, 3, 4, 6, 2047, 4098, 40964, 81925, 156940])

@@ -22,11 +22,11 @@
 // Warps: 0 copies weights (one bulk copy a stage), 1 issues the MMAs, 2 copies activations, 3 looks at the codes of a tile's rows (with fp32
 // activations 2..9 split), the rest is the epilogue.  Persistent CTAs, two accumulator pairs where they fit, weights that stay in shared
 // memory where a CTA's units share them.  Long sums of narrow layers are divided over a cluster (cl_splits) and added through
-// distributed shared memory in rank order, by the layer alone: an entry's values do not depend on its batch.
+// distributed shared memory in rank order, by the layer alone and not by the number of rows.
 // What bounds it (640 rows of 512 x 2048, split in four: 12.8 us, was 28.4; 5120 x 1536 x 1024: 60 us, was 161): the wide layers the bytes
 // through L2 and shared memory, 0.6 us for 64 channels and one tap of 128 x 128; the layers of many positions the epilogue's instructions,
-// some 30 per value (153600 x 128 with residual 61 us, was 71, 30 of DRAM time).
-// Measured (one pass): SNAC 32 windows 652 -> 532 us, 1 window 262 -> 242, Mimi 32 chunks 1926 -> 1257, the small kernels below among them.
+// some 50 for the 32 values of a warp (153600 x 128 with residual 61 us, was 71, 30 of DRAM time).
+// Measured (one pass): SNAC 32 windows 652 -> 532 us, 1 window 262 -> 242, Mimi 32 chunks 1926 -> 1262, the small kernels below among them.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 32
 #include "common.cuh"
@@ -943,8 +943,9 @@ __global__ void __launch_bounds__(ClRoles<PARTS>::THREADS, 1) cl_conv_kernel(con
       const uint32_t d = tmem_base + acc * p.acc_cols, d2 = d + p.cols;
       for (int i = 0; i < x_steps && !bw.dead; ++i) {
         bw.wait(&x_ready[xs], xph);
-        // parts written by threads, to be read by the tensor core.  (The fence stands here and not with the writers: there it would wait
-        // for the loads that they have on the way.)
+        // Parts written by threads, to be read by the tensor core.  The fence stands here and not with the writers, where it would wait for the
+        // loads that they have on the way.  It orders them all the same: a proxy fence counts anywhere on the path from the writes to the reads,
+        // and the writes come before it by the writers' arrivals (release) and this warp's wait (acquire), the MMAs after it in program order.
         if (!PARTS) fence_proxy_async();
         for (int tap = 0; tap < p.taps; ++tap) {
           if (!p.resident || it == 0) bw.wait(&w_full[ws], wph);
@@ -1698,6 +1699,10 @@ int vb_cl_pack(void* d_dst, const float* d_w, int N, int K, void* stream) {
 namespace vb {
 // Long sums of narrow layers are one chain of products on few CTAs: 640 rows of 512 x 2048 23.3 us in one part, 15.7 in two, 12.9 in four; 1024 x 3584
 // 33.9, 26.0, 23.6.  Shorter sums and wider layers lose (5120 rows of 256 x 1536 20.6 -> 27.9, 640 of 4096 x 2048 38.8 -> 60.6).
+// By the layer alone, since the parts round in another order than one sum: what fills the chip without them pays for that.  512 x 2048 / 1024 x 3584 in one
+// part and in four (us), by rows: 20 21.4 9.1 / 29.4 11.2; 160 21.7 9.9 / 30.2 13.8; 640 23.1 12.3 / 32.8 22.7; 1280 24.2 27.3 / 40.2 44.9; 2560 27.2
+// 41.8 / 55.5 94.4; 10240 71 127 / 213 309.  The line is where 32 streams of ten frames lie, 640 rows: split launches are not persistent, every
+// CTA starts, meets its cluster twice and ends for one unit.
 static int cl_splits(int blocks, int m_tiles, int kb) {
   return blocks >= 64 && m_tiles <= 8 ? min(4, kb) : 1;
 }

@@ -21,9 +21,9 @@
 // 98 KB of shared memory and 256 TMEM columns per CTA: two CTAs share an SM and fill each other's waits.
 // The form before this one had one warp group for everything -- loads, an element-wise transpose of every V tile, softmax, both
 // waits on the tensor cores -- one after the other (2.5 us per 64-token tile), and the kernel for smaller prompts ran on
-// mma.sync.  Measured per launch (mma.sync / this kernel, us, back to back): one 133-row prompt 11.6 / 10.1, eight of them 29 / 14,
-// four portions of 997 rows on up to 1063 cached tokens 112 / 40, three prompts of 1024 rows each 187 / 61, four of 600 with 64-wide heads
-// 74 / 32.
+// mma.sync.  Measured per launch (mma.sync / this kernel, us, back to back): one 133-row prompt 12.0 / 10.3, eight of them 29 / 13,
+// four portions of 997 rows, two of them on some 1000 cached tokens, 88 / 33, three prompts of 1024 rows each 186 / 53, four of 600 with 64-wide
+// heads 74 / 31.
 // Query rows come and results leave in whole rows, a few neighbouring threads each (a row per thread took 6 us until the rows were there and 3 us
 // at the end of a launch of cold data, 2 and 2 now).  The 997 rows above: 45 us a layer of cold data, 36 with whole rows.
 // A row's result depends on its own request alone, whatever else is in the step and whichever portion it comes in: the tiles of its keys are

@@ -93,8 +93,8 @@ __device__ __forceinline__ double philox_uniform(uint64_t seed, uint64_t offset,
 // passes had to be unrolled forty tokens deep, and reading that code once took longer than running it (top-p, cold: 32 rows of 2,051
 // tokens 61 us against 18 here; 32 rows of 156,940 tokens in a row of calls 53 against 39, and 67 with 1024 threads that spilled).
 // A row's time (28 us in a row of calls, of which 2.3 are traffic) goes to the loads and the first loop (8 us), the two exponentials a token
-// and the conversions to masses (6: those units take 8 cycles a warp), and a microsecond and more for each meeting of the cluster: six where the
-// first draw is accepted.
+// and the conversions to masses (6: those units take 8 cycles a warp), and a microsecond and more for each meeting of the cluster: five where the
+// first draw is accepted (largest key, denominator, masses, the draw, the mass above it).
 constexpr int SMP_THREADS = 1024;        // (cta, thread, pair) order of the tokens
 constexpr int SMP_PAIRS = 20;            // 40 tokens per thread: 40960 tokens per CTA, 327680 per 8-CTA cluster
 constexpr int SMP_MAX_CLUSTER = 8;

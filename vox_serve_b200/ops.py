@@ -306,9 +306,9 @@ _PREFILL_TC = os.environ.get("VB_PREFILL_TC", "auto")
 
 def _prefill_entry(group: int) -> str:
     """The kernel of a prefill-shaped plan with ``group`` query heads per key head (more than a row tile of the tcgen05 kernel holds run on
-    mma.sync).  Measured per launch, mma.sync / tcgen05 (us): 4 x 600 rows 74 / 32, 8 x 133 rows 29 / 14,
-    one 133-row prompt 11.6 / 10.1, 31 decode rows beside a 133-row prompt 54 / 26, one of 435 rows 28 / 15, 16 x 50 rows 16.9 / 12.6,
-    16 x 24 rows 8.8 / 9.6 (the one where most of a 128-row tile is padding)."""
+    mma.sync).  Measured per launch, mma.sync / tcgen05 (us): 4 x 600 rows (heads of 64) 74 / 31, 8 x 133 rows 29 / 13,
+    one 133-row prompt 12.0 / 10.3, 31 decode rows on 500 tokens beside a 133-row prompt 42 / 18, one of 435 rows 26 / 15, 16 x 50 rows 17.0 / 9.6,
+    16 x 24 rows 8.8 / 9.1 (the one where most of a 128-row tile is padding)."""
     return "vb_paged_prefill_attn" if _PREFILL_TC == "0" or group > 128 else "vb_paged_prefill_attn_tc"
 
 

@@ -516,17 +516,20 @@ __device__ __forceinline__ void cl_store(const ClConvParams& p, const ClHot& h, 
   cl_store(p, h, g, col_tab, c0, inside, reinterpret_cast<uint32_t*>(y), w);
 }
 // Whether eight rows of a block are all of ordinary size: no value out of range, and a lane none of whose rows is tiny.  (Nearly always; a chunk that
-// this does not hold for is looked at row by row.)  `rows`: a bit for each that there is.  One code for a chunk, its largest value's, cost 8 of Mimi's
-// 1262 us less, and let a loud row's neighbours lose what they are made of.
-__device__ __forceinline__ bool cl_ordinary(const F2 (&v)[CL_EC / 2], uint32_t rows) {
+// this does not hold for is looked at row by row.)  `rows`: a bit for each that there is; the others become 1.  One code for a chunk, its largest
+// value's, cost 8 of Mimi's 1262 us less, and let a loud row's neighbours lose what they are made of.
+__device__ __forceinline__ bool cl_ordinary(F2 (&v)[CL_EC / 2], uint32_t rows) {
+  if (rows != 0xffu) {
+#pragma unroll
+    for (int c = 0; c < CL_EC / 2; ++c) {
+      const float2 x = f2_get(v[c]);
+      v[c] = f2(rows >> (2 * c) & 1u ? x.x : 1.f, rows >> (2 * c) & 2u ? x.y : 1.f);
+    }
+  }
   float top = 0.f, low = CL_X_TOP;
 #pragma unroll
   for (int c = 0; c < CL_EC / 2; ++c) {
-    float2 x = f2_get(v[c]);
-    if (rows != 0xffu) {
-      if (!(rows >> (2 * c) & 1u)) x.x = 1.f;
-      if (!(rows >> (2 * c) & 2u)) x.y = 1.f;
-    }
+    const float2 x = f2_get(v[c]);
     top = max3_abs(top, x.x, x.y);
     low = min3_abs(low, x.x, x.y);
   }
@@ -567,7 +570,7 @@ __device__ __noinline__ uint32_t cl_odd_store(uint32_t* yp, int ok, int where, F
 }
 // eight rows of a block as parts; rows out of range as they are
 __device__ __forceinline__ void cl_store_parts(const ClConvParams& p, const ClHot& h, const ClEpiState& e, const ClUnit& g, const int4* col_tab, int c0, int inside,
-                                               const F2 (&v)[CL_EC / 2]) {
+                                               F2 (&v)[CL_EC / 2]) {
   const int lane = threadIdx.x & 31;
   const int4 tb = cl_column(p, g, col_tab, c0);
   uint32_t code = CB_NORMAL;
@@ -659,7 +662,7 @@ __device__ __forceinline__ void cl_boxed_chunks(const ClHot& h, const ClMaps& ma
     cl_act<ACT>(e, v);
     if (parts) {
       uint32_t code = CB_NORMAL;
-      if (c0 + CL_EC <= inside && cl_ordinary(v, 0xffu)) {          // (the last chunk of a sequence may go row by row)
+      if (cl_ordinary(v, c0 + CL_EC <= inside ? 0xffu : (1u << (inside - c0)) - 1u)) {
         const uint32_t a = out + (lane & 1 ? 64u : 0u) + (lane >> 1) * 4;
 #pragma unroll
         for (int c = 0; c < CL_EC / 2; ++c) {

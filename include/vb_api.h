@@ -524,7 +524,7 @@ int vb_wait_check(int limit_us, int pause_us, int complete, void* stream);
  * vb_cl_from_codes, vb_cl_codes_sum, vb_cl_upsample (w [C][2 s]), vb_cl_layernorm, vb_cl_chunk_attention (qkv [B][T][3 C], T <= 64).
  * Parts: an activation whose only readers are these convolutions can be kept as what they multiply -- in the place of 32 fp32 channels
  *   [32 high | 32 low] fp16, v = (high + low / 2048) / 16, with one code byte per 32 channels (1 ordinary, 0 all zero, 4 the 32 fp32 values
- *   themselves: one of them 4092 or more or not a number, or all of them below 2^-16).  The codes of element e lie at e / 32.  vb_cl_conv_parts takes x as
+ *   themselves: one of them 4092 or more or not a number, or all of them below 2^-14).  The codes of element e lie at e / 32.  vb_cl_conv_parts takes x as
  *   parts (d_x_code) or as fp32 (NULL), and gives the activated values as parts in d_yp / d_yp_code (d_y: the plain ones, or NULL; not with
  *   d_y2); entries of parts lie multiples of 32 floats apart.  vb_cl_{dwconv7, codes_sum, layernorm, chunk_attention}_parts: the result as
  *   parts where the codes are not NULL (D, C and the head size then multiples of 32).

@@ -10,9 +10,9 @@
 // Products: both operands as two fp16 parts, v = hi + lo / 2048 (the low part scaled into the normal range: 22 bits and a sign), hi_w hi_x in
 // one accumulator, hi_w lo_x + lo_w hi_x in a second one; what is dropped is below 2^-22 of a product.  Half the MMA time and half the
 // weight bytes of the two tf32 parts that stood here, at the same width; error against 64 bits of a decode 4.7e-6 (Mimi, was 2.8e-5).  Weights are
-// scaled per output channel by a power of two when they are packed.  Activations by 16: their parts hold 22 bits of a value in [2^-16, 4092) and smaller
-// ones to 2^-40 absolute.  A row's block of 32 channels with a value from 4092 on, an infinity, a NaN, or nothing but values below 2^-16 is kept as
-// it is in fp32, and the positions into which it goes are multiplied in fp32 on CUDA cores (cl_exact_chunk).  So every value is held to 2^-24
+// scaled per output channel by a power of two when they are packed.  Activations by 16: their parts hold 22 bits of a value in [2^-14, 4092) and smaller
+// ones to 2^-40 absolute.  A row's block of 32 channels with a value from 4092 on, an infinity, a NaN, or nothing but values below 2^-14 is kept as
+// it is in fp32, and the positions into which it goes are multiplied in fp32 on CUDA cores (cl_exact_chunk).  So every value is held to 2^-26
 // of the largest beside it, however quiet the passage; and since a row's code and a position's way follow from what goes into them alone, an
 // entry's bits do not depend on its batch.
 // What only these convolutions read is written as parts by the kernel that produces it, in the bytes its fp32 values would have taken, and
@@ -44,7 +44,7 @@ constexpr int CL_TAIL = 8192;               // barriers, tables, alignment
 constexpr float CL_X_SCALE = 16.f, CL_LO_SCALE = 2048.f;      // of activations; of low parts against high ones
 // what the two parts of an activation hold to 2^-22.  Where the largest value is not between these (or zero) -- of a block kept as parts, of what goes
 // into one result of fp32 activations -- the products are taken on CUDA cores
-constexpr float CL_X_TOP = 65472.f / CL_X_SCALE, CL_X_LOW = 0x1p-12f / CL_X_SCALE;
+constexpr float CL_X_TOP = 65472.f / CL_X_SCALE, CL_X_LOW = 0x1p-10f / CL_X_SCALE;
 enum ClCode { CB_NORMAL = 1, CB_RAW = 4 };      // of a block of 32 activations kept as parts (all zero: 0)
 
 struct ClConvParams {

@@ -530,6 +530,13 @@ int vb_wait_check(int limit_us, int pause_us, int complete, void* stream);
  *   parts where the codes are not NULL (D, C and the head size then multiples of 32).
  * vb_cl_timeouts: as vb_gemm_wide_timeouts. */
 int vb_cl_timeouts(void);
+/* A residual unit of SNAC in one launch: y = x + W s_mid(dw7(s_in(x)) + dw_b) + bias for rows [t_lo, t_hi), Snake of the result if d_alpha_out; as fp32 (d_y)
+ * or as parts (d_yp, d_yp_code).  The bits of vb_cl_dwconv7_parts and vb_cl_conv_parts one after the other.  dw_w [7][C], alphas [2][C] as above, W packed by
+ * vb_cl_pack; C a multiple of 64 up to 1024.  vb_cl_dw_unit_pays: 1 where it is the faster way for `rows` positions of B entries. */
+int vb_cl_dw_unit_pays(int B, int C, int rows, int dilation);
+int vb_cl_dw_unit(float* d_y, void* d_yp, void* d_yp_code, const float* d_x, long long x_bstride, const float* d_dw_w, const float* d_dw_b,
+                  const float* d_alpha_in, const float* d_alpha_mid, const void* d_w, const float* d_bias, const float* d_alpha_out, int B, int C, int T,
+                  int dilation, int t_lo, int t_hi, void* stream);
 int vb_cl_conv_parts(float* d_y, float* d_y2, void* d_yp, void* d_yp_code, const void* d_x, const void* d_x_code, long long x_bstride, int Tx,
                      const void* d_w, const float* d_bias, const float* d_resid, long long r_bstride, const float* d_scale, const float* d_noise,
                      int noise_ld, const float* d_alpha, int epilogue, int act, int B, int Cin, int N, int cmod, int ksize, int dil, int n_lo,

@@ -521,6 +521,45 @@ def test_channels_last_depthwise_and_last(B, T, C, dil, lo, hi, big):
     _close(last, ref, 5e-6)
 
 
+@pytest.mark.parametrize("B,T,C,dil,lo,hi", [(1, 1, 64, 1, 0, 1), (2, 127, 64, 3, 0, 127), (3, 253, 128, 9, 7, 251), (1, 300, 256, 1, 0, 300), (40, 130, 128, 9, 0, 130),
+                                             (2, 65, 192, 3, 0, 65), (1, 40, 1024, 1, 0, 40), (2, 1000, 64, 9, 111, 999), (1, 500, 64, 64, 0, 500), (5, 33, 320, 5, 1, 32)])
+@pytest.mark.parametrize("last", [False, True])
+@pytest.mark.parametrize("odd", [False, True])
+def test_channels_last_residual_unit(B, T, C, dil, lo, hi, last, odd):
+    """A unit in one launch is the same bits as its depthwise and its 1x1 convolution, also where parts cannot hold a value; and an entry's do not depend on its batch."""
+    from vox_serve_b200 import _lib
+    from vox_serve_b200.tokenizer import _cl
+
+    g = torch.Generator(device="cuda").manual_seed(B * T + C + dil)
+    rnd = lambda *s, std=1.0: torch.randn(*s, generator=g, device="cuda") * std          # noqa: E731
+    x, dw, db, w, b = rnd(B, T, C), rnd(7, C, std=7 ** -0.5), rnd(C, std=0.05), _cl.pack(rnd(C, C, std=C ** -0.5)), rnd(C, std=0.05)
+    a = [torch.cat((v, 1.0 / (v + 1e-9))) for v in (0.5 + torch.rand(C, generator=g, device="cuda") for _ in range(3))]
+    if odd:
+        db.zero_()
+        x[0, T // 2, 3] = 1e6                      # out of the parts' range, and past what the sine reduces
+        x[-1, T // 3] *= 1e-9
+        x[0, T // 4] = 0.0
+        x[-1, T - 1, C - 1] = float("nan")
+
+    def fused(v):
+        X = _cl.Act(v.contiguous().view(-1), v.shape[0], T, C)
+        return X, _cl.dw_unit(X, dw, db, a[0], a[1], w, b, dil, lo, hi, a[2] if last else None, "parts" if last else "f32")
+
+    def bits(y):
+        n = y.B * T * C
+        codes = y.buf.view(torch.uint8)[4 * n:4 * n + n // 32].view(y.B, T, -1)[:, lo:hi] if y.parts else torch.zeros(1, device="cuda")
+        return y.buf[:n].view(torch.int32).view(y.B, T, C)[:, lo:hi], codes
+
+    X, got = fused(x)
+    h = _cl.depthwise7(X, dw, db, a[0], a[1], dil, lo, hi, parts=True)
+    want = _cl.conv(h, w, C, b, epi="resid", resid=X, act="snake" if last else None, alpha=a[2] if last else None, lo=lo, hi=hi, out="parts" if last else "f32")
+    for p, q in zip(bits(got), bits(want)):
+        assert torch.equal(p, q)
+    for p, q in zip(bits(fused(x[-1:])[1]), bits(got)):
+        assert torch.equal(p, q[-1:] if p.dim() == 3 else q)
+    assert _lib.load().vb_cl_timeouts() == 0
+
+
 @pytest.mark.parametrize("B,T,C,ksize,left,lo,hi", [(1, 1, 64, 3, 2, 0, 1), (2, 129, 96, 3, 2, 0, 129), (3, 40, 4, 3, 0, 5, 38), (1, 300, 256, 7, 3, 1, 300), (2, 17, 68, 5, 4, 0, 17),
                                                    (1, 130, 128, 16, 15, 0, 130), (2, 16, 32, 1, 0, 0, 16)])
 def test_channels_last_one_output_channel(B, T, C, ksize, left, lo, hi):

@@ -69,6 +69,8 @@ SIGNATURES = {
     "vb_cl_conv_parts": (c_int, [P, P, P, P, P, P, C.c_longlong, c_int, P, P, P, C.c_longlong, P, P, c_int, P, c_int, c_int, c_int, c_int, c_int,
                                  c_int, c_int, c_int, c_int, c_int, C.c_longlong, P]),
     "vb_cl_dwconv7_parts": (c_int, [P, P, P, C.c_longlong, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P]),
+    "vb_cl_dw_unit_pays": (c_int, [c_int, c_int, c_int, c_int]),
+    "vb_cl_dw_unit": (c_int, [P, P, P, P, C.c_longlong, P, P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P]),
     "vb_cl_codes_sum_parts": (c_int, [P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P]),
     "vb_cl_layernorm_parts": (c_int, [P, P, P, P, P, c_int, c_int, c_float, P]),
     "vb_cl_chunk_attention_parts": (c_int, [P, P, P, c_int, c_int, c_int, c_int, c_float, P]),
@@ -291,7 +293,7 @@ def check_waits():
 
 # kernels (+ memset nodes) each entry point enqueues; everything not listed launches exactly one
 LAUNCHES = {"vb_set_pdl": 0, "vb_set_trace": 0, "vb_weight_tiles_bytes": 0, "vb_tensor_map_kv": 0,
-            "vb_tensor_map_2d_bf16": 0, "vb_gemm_wide_timeouts": 0, "vb_wait_flags": 0, "vb_cl_timeouts": 0, "vb_prefill_attn_tc_timeouts": 0, "vb_window_attn_tc_timeouts": 0, "vb_cl_pack_bytes": 0, "vb_device_info": 0, "vb_sample": 1, "vb_update_repetition_cache": 1,
+            "vb_tensor_map_2d_bf16": 0, "vb_gemm_wide_timeouts": 0, "vb_wait_flags": 0, "vb_cl_timeouts": 0, "vb_prefill_attn_tc_timeouts": 0, "vb_window_attn_tc_timeouts": 0, "vb_cl_pack_bytes": 0, "vb_cl_dw_unit_pays": 0, "vb_device_info": 0, "vb_sample": 1, "vb_update_repetition_cache": 1,
             "vb_set_gemm_smem_kb": 0, "vb_window_attn_tile_rows": 0, "vb_decay_attn_tile_rows": 0, "vb_decay_attn_tiled": 3, "vb_window_attn": 2, "vb_mingru_tiled": 3, "vb_mingru_scratch_floats": 0,
             "vb_short_conv": 2, "vb_selective_scan_tiled": 3, "vb_selective_scan_piece_rows": 0,
             "vb_selective_scan_scratch_floats": 0, "vb_sigmoid_attn": 1, "vb_ssd_tiled": 3, "vb_ssd_tile_rows": 0,

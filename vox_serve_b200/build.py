@@ -21,7 +21,7 @@ LIB = os.path.join(LIBDIR, "libvoxb200.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 SOURCES = ["api.cu", "elementwise.cu", "attn.cu", "prefill_attn.cu", "prefill_attn_tc.cu", "kvcopy.cu", "encoder.cu", "gemm.cu", "gemm_wide.cu", "sampler.cu", "snac.cu", "snac_mma.cu",
-           "cl_conv.cu", "multicodebook.cu", "mimi.cu", "codec.cu", "norm_linear.cu", "window_attn.cu", "window_attn_tc.cu", "linear_attn.cu", "gated_recurrence.cu", "moe.cu", "short_conv.cu", "sigmoid_attn.cu", "selective_scan.cu",
+           "cl_conv.cu", "cl_unit.cu", "multicodebook.cu", "mimi.cu", "codec.cu", "norm_linear.cu", "window_attn.cu", "window_attn_tc.cu", "linear_attn.cu", "gated_recurrence.cu", "moe.cu", "short_conv.cu", "sigmoid_attn.cu", "selective_scan.cu",
            "hyper.cu", "ssd.cu"]
 # subsets of the sources that serve one family of models: a first run that only needs that family compiles only these
 # (into lib/libvoxb200_<profile>.so; entry points of the other sources are absent from it)

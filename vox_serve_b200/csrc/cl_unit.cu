@@ -1,0 +1,639 @@
+// Residual units of the vocoders over channels-last activations [B][T][C] (fp32), a unit in one launch:
+//   y = x + W s2(dw7(s1(x)) + b1) + b2       (vb_cl_dw_unit: SNAC; s1, s2 Snakes, dw7 a depthwise convolution of 7 taps with dilation)
+// A block owns `nr` positions of one channel tile.  What goes into the product never leaves the block: a warp takes 64 channels, two a lane, and walks a
+// run of positions `dil` apart, so a row of x is loaded and put through its Snake once for the seven sums that it is part of, all in registers; the sums'
+// Snakes are written as the two fp16 parts that the tensor cores multiply (cl_common.cuh) into the operand in shared memory, and the products of 64
+// channels are issued as soon as all their runs are done.  The arithmetic -- order of the sums, parts, what is multiplied in fp32 because parts
+// cannot hold it -- is that of cl_dwconv7 and cl_conv one after the other, bit for bit.
+#include "../../include/vb_api.h"
+#define VB_PDL_FAMILY 32
+#include "cl_common.cuh"
+
+namespace vb {
+constexpr int CU_W_STAGES = 4, CU_MAX_CHUNKS = 16;      // (a block of 32 channels has a bit in a row's word)
+
+struct CuDwParams {
+  const float* x;            // [b * x_bstride + t * C + c]
+  const float* dw_w;         // [7][C]
+  const float* dw_b;         // [C]
+  const float* alpha_in;     // [2][C] alpha, 1 / (alpha + 1e-9)
+  const float* alpha_mid;
+  const uint8_t* w;          // packed (vb_cl_pack)
+  const float* w_inv;
+  const float* bias;         // [C]
+  const float* alpha_out;    // Snake of the result, or null
+  float* y;                  // fp32 result, or
+  uint32_t* yp;              // the result as parts
+  uint8_t* yp_code;
+  long long x_bstride, y_bstride;
+  int C, T, dil, t_lo, t_hi;
+  int nr, cols;              // positions of a block; columns of its products
+  int classes, segs, len;    // runs: position (class + dil (seg len + j)) of a block, j < len
+  int m_tiles, chunks, w_stages, tmem_cols;
+  uint32_t runs_inv, segs_inv, dil_inv, m_tiles_inv;      // for cu_div
+  unsigned char* wait_flag;
+};
+// a / b for 0 <= a < 2^31 with inv = ceil(2^32 / b), 0 for b == 1: the quotient or one more, as a product
+__device__ __forceinline__ int cu_div(int a, int b, uint32_t inv) {
+  if (inv == 0u) return a;
+  const int q = static_cast<int>(__umulhi(static_cast<uint32_t>(a), inv));
+  return q * static_cast<long long>(b) > a ? q - 1 : q;
+}
+
+// What a warp of an epilogue needs of its unit: a lane is a channel
+struct CuOut {
+  float bias, alpha, ialpha;
+  const float* resid;        // this channel at the block's first position
+  float* y;
+  uint32_t* yp;              // the warp's block of 32 channels there
+  uint8_t* code;
+  int N;
+};
+__device__ __forceinline__ void cu_resid(const CuOut& o, int c0, int inside, float (&rs)[CL_EC]) {
+  const float* r = o.resid + static_cast<long long>(c0) * o.N;
+  if (c0 + CL_EC <= inside) {
+#pragma unroll
+    for (int c = 0; c < CL_EC; ++c) rs[c] = __ldcg(r + c * o.N);
+    return;
+  }
+#pragma unroll
+  for (int c = 0; c < CL_EC; ++c) rs[c] = c0 + c < inside ? __ldcg(r + c * o.N) : 0.f;
+}
+// Columns [c_first, inside) in steps of c_step, eight at a time: accumulators + bias + residual, activation, fp32 or parts.  `rs`: the first residuals.
+template <int ACT>
+__device__ __forceinline__ void cu_chunks(const CuOut& o, uint32_t taddr, int cols, int inside, int c_first, int c_step, float inv, float (&rs)[CL_EC]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int c0 = c_first; c0 < inside; c0 += c_step) {
+    const uint32_t rows = c0 + CL_EC <= inside ? 0xffu : (1u << (inside - c0)) - 1u;
+    F2 v[CL_EC / 2];
+    cl_load_acc(taddr + c0, cols, inv, v);
+#pragma unroll
+    for (int c = 0; c < CL_EC / 2; ++c) v[c] = f2_add(f2_add(v[c], f2(o.bias)), f2(rs[2 * c], rs[2 * c + 1]));
+    if (c0 + c_step < inside) cu_resid(o, c0 + c_step, inside, rs);
+    cl_act<ACT>(o.alpha, o.ialpha, v);
+    const long long at = static_cast<long long>(c0) * o.N;
+    if (!o.yp) {
+      float* y = o.y + at;
+      if (rows == 0xffu) {
+#pragma unroll
+        for (int c = 0; c < CL_EC; ++c) {
+          const float2 x = f2_get(v[c >> 1]);
+          y[c * o.N] = c & 1 ? x.y : x.x;
+        }
+        continue;
+      }
+#pragma unroll
+      for (int c = 0; c < CL_EC; ++c) {
+        const float2 x = f2_get(v[c >> 1]);
+        if (rows >> c & 1u) y[c * o.N] = c & 1 ? x.y : x.x;
+      }
+      continue;
+    }
+    uint32_t* yp = o.yp + at;
+    uint32_t code = CB_NORMAL;
+    if (cl_ordinary(v, rows)) {
+      uint32_t* q = yp + (lane & 1 ? 16 : 0) + (lane >> 1);
+#pragma unroll
+      for (int c = 0; c < CL_EC / 2; ++c) {
+        uint32_t hi, lo, w0, w1;
+        cl_parts(v[c], CL_X_SCALE, hi, lo);
+        cl_exchange(hi, lo, w0, w1);
+        if (rows >> (2 * c) & 1u) q[2 * c * o.N] = w0;
+        if (rows >> (2 * c) & 2u) q[(2 * c + 1) * o.N] = w1;
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < CL_EC; ++c) {
+        const float2 x = f2_get(v[c >> 1]);
+        int word;
+        uint32_t bits;
+        const uint32_t row = cl_odd_row(c & 1 ? x.y : x.x, word, bits);
+        if (rows >> c & 1u) yp[c * o.N + word] = bits;
+        if ((lane & 7) == c) code = row;
+      }
+    }
+    if (lane < CL_EC && (rows >> lane & 1u)) o.code[(at + static_cast<long long>(lane) * o.N) >> 5] = static_cast<uint8_t>(code);
+  }
+}
+
+// The inputs of a product as they lie in shared memory: [block of 32 channels][row][128 bytes, swizzled], parts or (a bit in the row's word) fp32
+struct CuOperand {
+  uint32_t at;               // first row of the first block
+  int blk_bytes, blocks, ksize, skip;       // (rows below `skip` lie in front of the entry)
+  const uint32_t* raw;
+};
+// The products of four columns that `mask` names again in fp32, for this warp's 32 channels, into the accumulators (plain scale; the columns that are
+// not named in the plain scale as well): cl_exact_chunk of cl_conv.cu with the inputs in shared memory, in the same order.
+__device__ __noinline__ void cu_exact_chunk(const CuOperand& x, const uint8_t* w, float w_scale, int lane_row, int c0, uint32_t mask, uint32_t t_hi, uint32_t t_lo,
+                                            float inv) {
+  const int lane = threadIdx.x & 31, sw = lane_row & 7;
+  float acc[4] = {};
+#pragma unroll 1
+  for (int tap = 0; tap < x.ksize && mask; ++tap) {
+#pragma unroll 1
+    for (int blk = 0; blk < x.blocks; ++blk) {
+      float v[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int r = c0 + c + tap;
+        v[c] = 0.f;
+        if (!(mask >> c & 1u) || r < x.skip) continue;
+        const uint32_t row = x.at + blk * x.blk_bytes + r * 128;
+        if (x.raw[r] >> blk & 1u) {
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[c]) : "r"(row + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4));
+        } else {
+          const uint32_t a = row + (((lane >> 3) ^ (r & 7)) << 4) + (lane & 7) * 2;
+          uint16_t hi, lo;
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hi) : "r"(a));
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(lo) : "r"(a ^ 64u));
+          v[c] = fmaf(__half2float(__ushort_as_half(lo)), 1.f / CL_LO_SCALE, __half2float(__ushort_as_half(hi))) * (1.f / CL_X_SCALE);
+        }
+      }
+      const uint8_t* wb = w + static_cast<size_t>(tap * x.blocks + blk) * CL_W_BLOCK + lane_row * 128;
+#pragma unroll 1
+      for (int q = 0; q < 4; ++q) {
+        const uint4 hi = __ldg(reinterpret_cast<const uint4*>(wb + ((q ^ sw) << 4))), lo = __ldg(reinterpret_cast<const uint4*>(wb + (((q + 4) ^ sw) << 4)));
+        const uint32_t h[4] = {hi.x, hi.y, hi.z, hi.w}, l[4] = {lo.x, lo.y, lo.z, lo.w};
+        float f[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 fh = unpack_f16(h[i]), fl = unpack_f16(l[i]);
+          f[2 * i] = fmaf(fl.x, 1.f / CL_LO_SCALE, fh.x) * w_scale;
+          f[2 * i + 1] = fmaf(fl.y, 1.f / CL_LO_SCALE, fh.y) * w_scale;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (!(mask >> c & 1u)) continue;
+          if (c0 + c + tap < x.skip) continue;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) acc[c] = fmaf(__shfl_sync(0xffffffffu, v[c], 8 * q + k), f[k], acc[c]);
+        }
+      }
+    }
+  }
+  uint32_t hi[4], lo[4];
+  tmem_ld_32x4(t_hi, hi);
+  tmem_ld_32x4(t_lo, lo);
+  tmem_ld_wait();
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    if (!(mask >> c & 1u)) acc[c] = fmaf(__uint_as_float(lo[c]), 1.f / CL_LO_SCALE, __uint_as_float(hi[c])) * inv;
+  tmem_st_32x4(t_hi, acc);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) acc[c] = 0.f;
+  tmem_st_32x4(t_lo, acc);
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// ... all columns of a warp that are made of a row kept in fp32
+__device__ __noinline__ void cu_exact(const CuOperand& x, const uint8_t* w, const float* w_inv, int lane_row, int inside, int c_first, int c_step, uint32_t taddr,
+                                      int cols, float inv) {
+#pragma unroll 1
+  for (int c0 = c_first; c0 < inside; c0 += c_step) {
+    uint32_t mask = 0u;
+    for (int c = 0; c < CL_EC; ++c) {
+      uint32_t any = 0u;
+      for (int tap = 0; tap < x.ksize; ++tap)
+        if (c0 + c < inside && c0 + c + tap >= x.skip) any |= x.raw[c0 + c + tap];
+      mask |= any ? 1u << c : 0u;
+    }
+#pragma unroll 1
+    for (int c = 0; c < CL_EC; c += 4)
+      cu_exact_chunk(x, w, w_inv[lane_row] * CL_X_SCALE, lane_row, c0 + c, mask >> c & 15u, taddr + c0 + c, taddr + cols + c0 + c, inv);
+  }
+}
+
+// sin(y)^2 of arguments past what cl_sin_sq reduces (each value by itself: its result does not depend on the others)
+__device__ __noinline__ F2 cu_sin_sq_large(F2 y, F2 s) {
+  const float2 p = f2_get(y), q = f2_get(s);
+  const float sx = sinf(p.x), sy = sinf(p.y);
+  return f2(fabsf(p.x) <= CL_SIN_MAX ? q.x : sx * sx, fabsf(p.y) <= CL_SIN_MAX ? q.y : sy * sy);
+}
+// The constants of cl_sin_sq, held in registers: the compiler moves them into a pair wherever one is used otherwise
+struct CuSine {
+  F2 inv_pi, magic, unmagic, pi_hi, pi_lo, c3, c2, c1, c0;
+};
+__device__ __forceinline__ F2 cu_pin(float x) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r.v) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ CuSine cu_sine() {
+  return CuSine{cu_pin(0.318309886f), cu_pin(12582912.f), cu_pin(-12582912.f), cu_pin(-3.14159274101f), cu_pin(8.742278012619e-08f), cu_pin(2.605780761e-06f),
+                cu_pin(-1.980960296e-04f), cu_pin(8.333066247e-03f), cu_pin(-1.666665955e-01f)};
+}
+// v + inv sin(a v)^2 of two channels at N positions
+template <int N>
+__device__ __forceinline__ void cu_snake(F2 (&v)[N], F2 a, F2 inv, const CuSine& K) {
+  F2 y[N], s[N];
+  float m = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    y[i] = f2_mul(a, v[i]);
+    const F2 k = f2_add(f2_fma(y[i], K.inv_pi, K.magic), K.unmagic), r = f2_fma(k, K.pi_lo, f2_fma(k, K.pi_hi, y[i])), u = f2_mul(r, r);
+    F2 q = f2_fma(u, K.c3, K.c2);
+    q = f2_fma(u, q, K.c1);
+    q = f2_fma(u, q, K.c0);
+    q = f2_fma(f2_mul(r, u), q, r);
+    s[i] = f2_mul(q, q);
+    const float2 p = f2_get(y[i]);
+    m = max3_abs(m, p.x, p.y);
+  }
+  if (!(m <= CL_SIN_MAX)) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) s[i] = cu_sin_sq_large(y[i], s[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = f2_fma(inv, s[i], v[i]);
+}
+struct CuTaps {              // of a lane's two channels
+  F2 w[7], b, ai, ii, ao, io;
+};
+__device__ __forceinline__ CuTaps cu_taps(const CuDwParams& p, int c) {
+  auto ld = [&](const float* q) {
+    const float2 v = __ldg(reinterpret_cast<const float2*>(q + c));
+    return f2(v.x, v.y);
+  };
+  CuTaps t;
+#pragma unroll
+  for (int i = 0; i < 7; ++i) t.w[i] = ld(p.dw_w + i * p.C);
+  t.b = ld(p.dw_b);
+  t.ai = ld(p.alpha_in);
+  t.ii = ld(p.alpha_in + p.C);
+  t.ao = ld(p.alpha_mid);
+  t.io = ld(p.alpha_mid + p.C);
+  return t;
+}
+// A run once more, row by row, for the blocks of rows that parts cannot hold: those stay fp32, a bit in the row's word
+__device__ __noinline__ void cu_odd_run(const CuDwParams& p, const float* x, int t_first, int n, int r0, int c, int block, uint32_t dst, uint32_t* raw, uint32_t* any) {
+  const int lane = threadIdx.x & 31, in = (lane & 15) * 2;
+  const CuTaps tp = cu_taps(p, c);
+  const CuSine K = cu_sine();
+#pragma unroll 1
+  for (int j = 0; j < n; ++j) {
+    F2 o = tp.b;
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+      const int t = t_first + (j + k - 3) * p.dil;
+      float2 v = make_float2(0.f, 0.f);
+      if (t >= 0 && t < p.T) v = __ldcg(reinterpret_cast<const float2*>(x + static_cast<long long>(t) * p.C));
+      F2 one[1] = {f2(v.x, v.y)};
+      cu_snake(one, tp.ai, tp.ii, K);
+      o = f2_fma(tp.w[k], one[0], o);
+    }
+    F2 one[1] = {o};
+    cu_snake(one, tp.ao, tp.io, K);
+    const float2 v = f2_get(one[0]);
+    float m = max3_abs(v.x, v.y, v.y);
+#pragma unroll
+    for (int q = 1; q < 16; q <<= 1) {
+      const float other = __shfl_xor_sync(0xffffffffu, m, q);
+      m = max3_abs(m, other, other);
+    }
+    if (cl_code(m) != CB_RAW) continue;          // (the parts are there)
+    const int r = r0 + j * p.dil;
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dst + r * 128 + (((in >> 2) ^ (r & 7)) << 4) + (in & 2) * 4), "f"(v.x), "f"(v.y) : "memory");
+    if (in == 0) {
+      atomicOr(raw + r, 1u << block);
+      *any = 1u;
+    }
+  }
+}
+
+template <int P>             // warps that make the operand; one more copies weights and issues the products
+__global__ void __launch_bounds__(32 * (P + 1), P == 9 ? 2 : 1) cl_dw_unit_kernel(const __grid_constant__ CuDwParams p) {
+  constexpr int EPI_WARPS = P / 4 * 4;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int C = p.C, cols = p.cols, blk_bytes = cols * 128;
+  uint8_t* w_smem = smem + 2 * p.chunks * blk_bytes;
+  uint64_t* op_full = reinterpret_cast<uint64_t*>(w_smem + p.w_stages * 2 * CL_W_BLOCK);          // 64 channels of all positions are there
+  uint64_t* w_full = op_full + CU_MAX_CHUNKS;
+  uint64_t* w_empty = w_full + CU_W_STAGES;
+  uint64_t* acc_full = w_empty + CU_W_STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  uint32_t* any = tmem_slot + 1;
+  const uint32_t gate = smem_u32(tmem_slot + 2);
+  uint32_t* raw = tmem_slot + 4;                                             // [cols] a bit for every block of a row that is kept in fp32
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tt = cu_div(blockIdx.x, p.m_tiles, p.m_tiles_inv), m0 = (blockIdx.x - tt * p.m_tiles) * 128, t0 = p.t_lo + tt * p.nr, b = blockIdx.y;
+  const int inside = min(p.nr, p.t_hi - t0), runs = p.classes * p.segs;
+  const uint8_t* w = p.w + static_cast<size_t>(m0 >> 7) * (2 * p.chunks) * CL_W_BLOCK;
+  BoundedWait bw{p.wait_flag, gate};
+
+  if (warp == P) {
+    if (lane == 0) {
+      tmem_slot[2] = 0u;
+      *any = 0u;
+      for (int i = 0; i < p.chunks; ++i) mbar_init(&op_full[i], runs);
+      for (int i = 0; i < CU_W_STAGES; ++i) {
+        mbar_init(&w_full[i], 1);
+        mbar_init(&w_empty[i], 1);
+      }
+      mbar_init(acc_full, 1);
+      fence_barrier_init();
+    }
+    __syncwarp();
+    tmem_alloc(tmem_slot, p.tmem_cols);
+    tmem_relinquish();
+  } else {
+    for (int i = threadIdx.x; i < cols; i += 32 * P) raw[i] = 0u;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == P) {
+    // ================= weights and products =================
+    if (lane == 0) {
+      for (int i = 0; i < min(p.w_stages, p.chunks); ++i) {          // (weights do not depend on the kernels in front)
+        mbar_arrive_expect_tx(&w_full[i], 2 * CL_W_BLOCK);
+        cl_bulk(smem_u32(w_smem) + i * 2 * CL_W_BLOCK, w + static_cast<size_t>(i) * 2 * CL_W_BLOCK, 2 * CL_W_BLOCK, smem_u32(&w_full[i]));
+      }
+      pdl_wait();
+      wait_gate_open(gate);
+      pdl_trigger();
+    }
+    __syncwarp();
+    const uint64_t w_desc0 = umma_desc_sw128_kmajor(smem_u32(w_smem)), x_desc0 = umma_desc_sw128_kmajor(smem_u32(smem));
+    const uint32_t idesc = umma_idesc(128, cols, 0u);
+    for (int k = 0; k < p.chunks && !bw.dead; ++k) {
+      const int ws = k % p.w_stages;
+      bw.wait(&op_full[k], 0u);
+      bw.wait(&w_full[ws], (k / p.w_stages) & 1);
+      if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+      tc_fence_after();
+      if (elect_one()) {
+        uint64_t w_hi = w_desc0 + static_cast<uint64_t>(ws) * (2 * CL_W_BLOCK >> 4), x_hi = x_desc0 + static_cast<uint64_t>(2 * k) * (blk_bytes >> 4);
+        // (a loop: unrolled, nvcc 12.9 gave the tensor cores descriptors of the weights without their upper halves)
+#pragma unroll 1
+        for (int g = 0; g < 2; ++g) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {            // (the low parts lie 64 bytes behind the high ones)
+            const uint32_t go = (k | g | i) ? 1u : 0u;
+            umma_bf16(tmem_base, w_hi + 2 * i, x_hi + 2 * i, idesc, go);
+            umma_bf16(tmem_base + cols, w_hi + 2 * i, x_hi + 4 + 2 * i, idesc, go);
+            umma_bf16(tmem_base + cols, w_hi + 4 + 2 * i, x_hi + 2 * i, idesc, 1u);
+          }
+          w_hi += CL_W_BLOCK >> 4;
+          x_hi += blk_bytes >> 4;
+        }
+        umma_commit(&w_empty[ws]);
+        if (k + 1 == p.chunks) umma_commit(acc_full);
+      }
+      __syncwarp();
+      if (k >= 1 && k - 1 + p.w_stages < p.chunks) {          // the stage in front is free when its products are done
+        const int was = (k - 1) % p.w_stages, next = k - 1 + p.w_stages;
+        bw.wait(&w_empty[was], ((k - 1) / p.w_stages) & 1);
+        if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&w_full[was], 2 * CL_W_BLOCK);
+          cl_bulk(smem_u32(w_smem) + was * 2 * CL_W_BLOCK, w + static_cast<size_t>(next) * 2 * CL_W_BLOCK, 2 * CL_W_BLOCK, smem_u32(&w_full[was]));
+        }
+        __syncwarp();
+      }
+    }
+    if (bw.dead && lane == 0) {            // let the copies in flight land before the block may leave
+      const unsigned long long from = gtimer();
+      while (gtimer() - from < 2000000ull) __nanosleep(1000);
+    }
+    __syncwarp();
+  } else {
+    // ================= the operand =================
+    const int items = p.chunks * runs;
+    const float* xb = p.x + b * p.x_bstride + lane * 2;
+    const long long step = static_cast<long long>(p.dil) * C;
+    const uint32_t at_step = p.dil * 128;
+    bool first = true;
+    const CuSine K = cu_sine();
+#pragma unroll 1
+    for (int item = warp; item < items; item += P) {
+      const int k = cu_div(item, runs, p.runs_inv), run = item - k * runs, cls = cu_div(run, p.segs, p.segs_inv), seg = run - cls * p.segs;
+      const int c = k * 64 + lane * 2, r0 = cls + seg * p.len * p.dil;                      // first position of the run
+      const int n = r0 < inside ? min(p.len, cu_div(inside - 1 - r0, p.dil, p.dil_inv) + 1) : 0;
+      const CuTaps tp = cu_taps(p, c);
+      if (first) {
+        pdl_wait();
+        first = false;
+      }
+      const uint32_t dst = smem_u32(smem) + (2 * k + (lane >> 4)) * blk_bytes;
+      const int in = (lane & 15) * 2;
+      const uint32_t chunk = (in >> 3 << 4) + (in & 6) * 2;
+      const float* x = xb + k * 64;
+      float top = 0.f, low = CL_X_TOP;
+      F2 h[10], got[4];              // six inputs through their Snake from the step before and four new ones; the next four
+      int t_next = t0 + r0 - 3 * p.dil;
+      const float* from = x + static_cast<long long>(t_next) * C;
+      const bool within = t_next >= 0 && t_next + (n + 9) * p.dil < p.T;          // (of every row that may be asked for)
+      auto load4 = [&]() {
+        if (within) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 v = __ldcg(reinterpret_cast<const float2*>(from));
+            got[i] = f2(v.x, v.y);
+            from += step;
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float2 v = make_float2(0.f, 0.f);
+            if (t_next >= 0 && t_next < p.T) v = __ldcg(reinterpret_cast<const float2*>(from));
+            got[i] = f2(v.x, v.y);
+            from += step;
+            t_next += p.dil;
+          }
+        }
+      };
+#pragma unroll
+      for (int i = 0; i < 6; ++i) h[i] = f2(0.f);
+      if (n > 0) load4();
+      uint32_t at = dst + (r0 - 6 * p.dil) * 128;            // the row of sum j
+#pragma unroll 1
+      for (int j = -6; n > 0 && j < n; j += 4) {           // inputs j + 6 .. j + 9, sums j .. j + 3
+        cu_snake(got, tp.ai, tp.ii, K);           // (the activation of zero is zero)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) h[6 + i] = got[i];
+        if (j + 4 < n) load4();
+        if (j > -4) {
+          F2 o[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) o[i] = tp.b;
+#pragma unroll
+          for (int q = 0; q < 7; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[i] = f2_fma(tp.w[q], h[i + q], o[i]);
+          cu_snake(o, tp.ao, tp.io, K);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (j + i >= 0 && j + i < n) {
+              const float2 v = f2_get(o[i]);
+              top = max3_abs(top, v.x, v.y);
+              low = min3_abs(low, v.x, v.y);
+              uint32_t hi, lo;
+              cl_parts(o[i], CL_X_SCALE, hi, lo);
+              const uint32_t q = at + i * at_step, a = q + (chunk ^ (q >> 3 & 0x70u));          // (the row's number modulo 8, swizzled)
+              asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(hi) : "memory");
+              asm volatile("st.shared.b32 [%0], %1;" ::"r"(a ^ 64u), "r"(lo) : "memory");
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 6; ++i) h[i] = h[i + 4];
+        at += 4 * at_step;
+      }
+      // No value out of range, and in either block a lane none of whose values is tiny: nearly always
+      const uint32_t fine = __ballot_sync(0xffffffffu, top < CL_X_TOP), large = __ballot_sync(0xffffffffu, low >= CL_X_LOW);
+      if (n > 0 && !(fine == 0xffffffffu && (large & 0xffffu) && large >> 16))
+        cu_odd_run(p, x, t0 + r0, n, r0, c, 2 * k + (lane >> 4), dst, raw, any);
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&op_full[k]);
+    }
+    if (first) pdl_wait();
+  }
+  // ================= epilogue =================
+  if (warp < EPI_WARPS) {
+    const int quarter = warp & 3, lane_row = quarter * 32 + lane, width = min(128, C - m0), copies = cl_copies(width);
+    const int row = copies == 1 ? lane_row : lane_row & (width - 1), n = m0 + row;
+    const int turns = EPI_WARPS / 4 * copies, c_step = turns * CL_EC;
+    const int c_first = ((warp >> 2) * copies + (copies == 4 ? quarter : copies == 2 ? quarter >> 1 : 0)) * CL_EC;
+    const bool some = row < width && c_first < inside;
+    const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const long long at = static_cast<long long>(t0) * C;
+    float inv = 0.f, rs[CL_EC];
+    CuOut o{};
+    if (some) {
+      o.N = C;
+      o.resid = p.x + b * p.x_bstride + at + n;
+      cu_resid(o, c_first, inside, rs);          // asked for before the accumulator is waited for
+      inv = __ldg(p.w_inv + m0 + lane_row);
+      o.bias = __ldg(p.bias + n);
+      if (p.alpha_out) o.alpha = __ldg(p.alpha_out + n), o.ialpha = __ldg(p.alpha_out + C + n);
+    }
+    for (int k = 0; k < p.chunks; ++k) bw.wait(&op_full[k], 0u);          // (what `any` and the rows' words say is seen with them)
+    bw.wait(acc_full, 0u);
+    const bool alive = __all_sync(0xffffffffu, !bw.dead);
+    tc_fence_after();
+    if (alive && some) {
+      if (*any) {
+        const CuOperand x{smem_u32(smem), blk_bytes, 2 * p.chunks, 1, 0, raw};
+        cu_exact(x, w, p.w_inv + m0, lane_row, inside, c_first, c_step, taddr, cols, inv);
+        inv = 1.f;
+      }
+      const long long to = b * p.y_bstride + at;
+      if (p.y) o.y = p.y + to + n;
+      if (p.yp) o.yp = p.yp + to + (n & ~31), o.code = p.yp_code + ((to + (n & ~31)) >> 5);
+      if (p.alpha_out) cu_chunks<CA_SNAKE>(o, taddr, cols, inside, c_first, c_step, inv, rs);
+      else cu_chunks<CA_NONE>(o, taddr, cols, inside, c_first, c_step, inv, rs);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == P) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, p.tmem_cols);
+  }
+}
+
+static bool on16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }      // (a null pointer is)
+
+static int cu_sms() {
+  static int sms = 0;
+  if (!sms) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+  }
+  return sms;
+}
+// shared memory of a block
+static int cu_dw_smem(int C, int cols, int w_stages) {
+  return 1024 + C / 32 * cols * 128 + w_stages * 2 * CL_W_BLOCK + (CU_MAX_CHUNKS + 2 * CU_W_STAGES + 1) * 8 + 16 + cols * 4;
+}
+// How a launch is divided: positions of a block, and whether two blocks of nine producing warps share an SM or one of eighteen has it.  Positions are
+// multiples of nine: runs of the dilations 1, 3 and 9 then come out alike, one for each of the nine warps.
+struct CuDwPlan {
+  int nr, cols, classes, segs, len, warps, w_stages, smem;
+};
+static CuDwPlan cu_dw_plan(int C, int dil, long long range, long long B, int sms) {
+  static const int kRows[] = {126, 108, 90, 72, 63, 54, 45, 36, 27, 18, 9};
+  const int chunks = C / 64, m_tiles = (C + 127) / 128;
+  CuDwPlan best{};
+  double least = 0.0;
+  for (int nr : kRows) {
+    const int cols = (nr + 15) / 16 * 16;
+    const long long units = m_tiles * ((range + nr - 1) / nr) * B;
+    for (int warps = 9; warps <= 18; warps += 9) {
+      const int limit = warps == 9 ? 113 * 1024 : VB_MAX_DYN_SMEM;
+      int ws = min(chunks, CU_W_STAGES);
+      while (ws > min(chunks, 2) && cu_dw_smem(C, cols, ws) > limit) --ws;
+      if (cu_dw_smem(C, cols, ws) > limit) continue;
+      const int classes = min(dil, nr), want = chunks == 1 ? warps : 9, segs = max(1, (want + classes / 2) / classes);
+      const int len = ((nr + dil - 1) / dil + segs - 1) / segs, items = chunks * classes * segs, rounds = (items + warps - 1) / warps;
+      // instructions of a run (a row's Snake with its load 24, a sum with its own and its parts 40), of the epilogue; cycles where `warps` or twice
+      // as many share an SM
+      const double run = (len + 6) * 24.0 + len * 40.0 + 60, epi = cols / 8.0 * min(4, C / 32) * 80;
+      const long long slots = static_cast<long long>(sms) * (warps == 9 ? 2 : 1);
+      const double waves = static_cast<double>((units + slots - 1) / slots), on_sm = warps == 9 && units > sms ? 18.0 : warps;
+      const double cost = waves * (3500 + rounds * run * fmax(2.5, on_sm / 2.2) + epi / (warps == 9 ? 1.2 : 2.2) * (on_sm > warps ? 1.0 : 0.6));
+      if (best.nr == 0 || cost < least) {
+        least = cost;
+        best = CuDwPlan{nr, cols, classes, segs, len, warps, ws, cu_dw_smem(C, cols, ws)};
+      }
+    }
+  }
+  return best;
+}
+}  // namespace vb
+
+using namespace vb;
+
+extern "C" {
+
+int vb_cl_dw_unit_pays(int B, int C, int rows, int dilation) {
+  if (B <= 0 || rows <= 0 || C <= 0 || C % 64 || C > 256 || dilation < 1 || dilation > 64) return 0;
+  return C <= 128 || (C + 127) / 128 * ((rows + 125LL) / 126) * B <= cu_sms();
+}
+
+int vb_cl_dw_unit(float* d_y, void* d_yp, void* d_yp_code, const float* d_x, long long x_bstride, const float* d_dw_w, const float* d_dw_b,
+                  const float* d_alpha_in, const float* d_alpha_mid, const void* d_w, const float* d_bias, const float* d_alpha_out, int B, int C, int T,
+                  int dilation, int t_lo, int t_hi, void* stream) {
+  VB_CHECK_ARG(!d_y != !d_yp && !d_yp == !d_yp_code, "vb_cl_dw_unit: one result, as fp32 or as parts with their codes");
+  VB_CHECK_ARG(d_x && d_dw_w && d_dw_b && d_alpha_in && d_alpha_mid && d_w && d_bias, "vb_cl_dw_unit: null pointer");
+  VB_CHECK_ARG(C > 0 && C % 64 == 0 && C <= 64 * CU_MAX_CHUNKS && dilation >= 1 && dilation <= 64, "vb_cl_dw_unit: C = %d (a multiple of 64, <= 1024), dilation %d",
+               C, dilation);
+  VB_CHECK_ARG(x_bstride % 4 == 0 && on16(d_x) && on16(d_y) && on16(d_yp), "vb_cl_dw_unit: rows must start on 16-byte boundaries");
+  VB_CHECK_ARG(on16(d_dw_w) && on16(d_dw_b) && on16(d_alpha_in) && on16(d_alpha_mid) && on16(d_w) && on16(d_bias) && on16(d_alpha_out),
+               "vb_cl_dw_unit: weights, biases and alphas must lie on 16-byte boundaries");
+  VB_CHECK_ARG(0 <= t_lo && t_lo <= t_hi && t_hi <= T, "vb_cl_dw_unit: range [%d, %d) outside [0, %d)", t_lo, t_hi, T);
+  VB_CHECK_ARG(B <= 65535, "vb_cl_dw_unit: %d entries", B);
+  if (B <= 0 || t_lo == t_hi) return 0;
+  const CuDwPlan g = cu_dw_plan(C, dilation, t_hi - t_lo, B, cu_sms());
+  CuDwParams p = {};
+  VB_CHECK_ARG(p.wait_flag = wait_flag(WK_CL_CONV), "vb_cl_dw_unit: no mapped host memory");
+  const long long n_pad = (C + 127LL) / 128 * 128;
+  p.x = d_x; p.dw_w = d_dw_w; p.dw_b = d_dw_b; p.alpha_in = d_alpha_in; p.alpha_mid = d_alpha_mid;
+  p.w = static_cast<const uint8_t*>(d_w);
+  p.w_inv = reinterpret_cast<const float*>(p.w + n_pad * C * 4);
+  p.bias = d_bias; p.alpha_out = d_alpha_out; p.y = d_y; p.yp = static_cast<uint32_t*>(d_yp); p.yp_code = static_cast<uint8_t*>(d_yp_code);
+  p.x_bstride = x_bstride; p.y_bstride = static_cast<long long>(T) * C;
+  p.C = C; p.T = T; p.dil = dilation; p.t_lo = t_lo; p.t_hi = t_hi;
+  p.nr = g.nr; p.cols = g.cols; p.classes = g.classes; p.segs = g.segs; p.len = g.len; p.m_tiles = (C + 127) / 128; p.chunks = C / 64; p.w_stages = g.w_stages;
+  auto inverse = [](int b) { return b > 1 ? static_cast<uint32_t>(((1ULL << 32) + b - 1) / b) : 0u; };
+  p.runs_inv = inverse(g.classes * g.segs); p.segs_inv = inverse(g.segs); p.dil_inv = inverse(dilation); p.m_tiles_inv = inverse(p.m_tiles);
+  p.tmem_cols = 32;
+  while (p.tmem_cols < 2 * g.cols) p.tmem_cols *= 2;
+  const long long tiles = static_cast<long long>(p.m_tiles) * ((static_cast<long long>(t_hi) - t_lo + g.nr - 1) / g.nr);
+  VB_CHECK_ARG(tiles <= 0x7fffffffLL, "vb_cl_dw_unit: too many tiles");
+  const dim3 grid(static_cast<unsigned>(tiles), B);
+  if (g.warps == 9) {
+    VB_CHECK_CUDA(max_dyn_smem_once(cl_dw_unit_kernel<9>));
+    VB_LAUNCH_PDL(cl_dw_unit_kernel<9>, grid, 320, g.smem, stream, p);
+  } else {
+    VB_CHECK_CUDA(max_dyn_smem_once(cl_dw_unit_kernel<18>));
+    VB_LAUNCH_PDL(cl_dw_unit_kernel<18>, grid, 608, g.smem, stream, p);
+  }
+  return 0;
+}
+
+}  // extern "C"

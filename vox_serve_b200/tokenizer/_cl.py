@@ -115,6 +115,20 @@ def depthwise7(x: Act, w: torch.Tensor, bias, alpha_in, alpha_out, dil: int, lo:
     return y
 
 
+def dw_unit_pays(x: Act, dil: int, rows: int) -> bool:
+    """whether ``dw_unit`` is the faster way (the results are the same bits)"""
+    return bool(_lib.load().vb_cl_dw_unit_pays(x.B, x.C, rows, dil))
+
+
+def dw_unit(x: Act, dw_w: torch.Tensor, dw_b, alpha_in, alpha_mid, w: torch.Tensor, bias, dil: int, lo: int, hi: int, alpha_out=None,
+            out: str = "f32") -> Act:
+    """x + 1x1(Snake(depthwise7(Snake(x)))) for rows [lo, hi), then a Snake if ``alpha_out``: ``depthwise7`` and ``conv`` in one launch"""
+    y = Act.empty(x.B, x.T, x.C, x.buf.device, out == "parts")
+    call("vb_cl_dw_unit", None if y.parts else y.ptr, y.ptr if y.parts else None, y.codes, x.ptr, x.bstride, dw_w.data_ptr(), dw_b.data_ptr(),
+         alpha_in.data_ptr(), alpha_mid.data_ptr(), w.data_ptr(), bias.data_ptr(), _ptr(alpha_out), x.B, x.C, x.T, dil, lo, hi, ops._stream())
+    return y
+
+
 def last_conv(x: Act, w: torch.Tensor, bias, ksize: int, left: int, t0: int, t1: int, tanh: bool) -> torch.Tensor:
     """one output channel -> [B, 1, t1 - t0]; w [C, ksize]"""
     y = torch.empty(x.B, 1, t1 - t0, dtype=torch.float32, device=x.buf.device)

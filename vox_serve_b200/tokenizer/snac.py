@@ -280,11 +280,16 @@ class SNAC:
             x = _cl.conv(up, self.tc[f"b{bi}.noise_w"], ch, epi="noise", resid=u, noise=nz.view(B, u.T), lo=c_lo, hi=c_hi)
             for j, dil in enumerate((1, 3, 9)):
                 q, (u_lo, u_hi) = f"b{bi}.r{j}.", units[j]
-                h = _cl.depthwise7(x, self.tc[q + "dw_w"], w[q + "dw_b"], self.tc[q + "alpha1"], self.tc[q + "alpha2"], dil, u_lo, u_hi, parts=True)
                 # the last unit's output only feeds the next stage's Snake: fused into this epilogue
                 nxt = None if j < 2 else self.tc[f"b{bi + 1}.alpha" if bi + 1 < nb else "out.alpha"]
+                out = "parts" if j == 2 and bi + 1 < nb else "f32"
+                dw = (self.tc[q + "dw_w"], w[q + "dw_b"], self.tc[q + "alpha1"], self.tc[q + "alpha2"])
+                if _cl.dw_unit_pays(x, dil, u_hi - u_lo):
+                    x = _cl.dw_unit(x, *dw, self.tc[q + "pw_w"], w[q + "pw_b"], dil, u_lo, u_hi, nxt, out)
+                    continue
+                h = _cl.depthwise7(x, *dw, dil, u_lo, u_hi, parts=True)
                 x = _cl.conv(h, self.tc[q + "pw_w"], ch, w[q + "pw_b"], epi="resid", resid=x, act=None if nxt is None else "snake",
-                             alpha=nxt, lo=u_lo, hi=u_hi, out="parts" if j == 2 and bi + 1 < nb else "f32")
+                             alpha=nxt, lo=u_lo, hi=u_hi, out=out)
         return _cl.last_conv(x, w["out.w"], w["out.b"], 7, 3, *out_range, tanh=True)
 
     @torch.no_grad()

@@ -543,6 +543,10 @@ int vb_cl_conv_parts(float* d_y, float* d_y2, void* d_yp, void* d_yp_code, const
                      int n_hi, long long y_bstride, void* stream);
 int vb_cl_dwconv7_parts(float* d_y, void* d_code, const float* d_x, long long x_bstride, const float* d_w, const float* d_bias,
                         const float* d_alpha_in, const float* d_alpha_out, int B, int C, int T, int dilation, int t_lo, int t_hi, void* stream);
+/* The end of Mimi's decoder in one launch: out[b][t] = bl + sum_j wl[c][j] e(y[t - 2 + j][c]), y = x + W3 e(h) + b3, h[t] = b1 + sum_j W1_j e(x[t - 2 + j]),
+ * e = ELU, zeros in front of an entry; x [B][T][64], W1 (32 channels, 3 taps) and W3 (64 channels) packed by vb_cl_pack, wl [64][3]. */
+int vb_cl_res_tail(float* d_y, const float* d_x, long long x_bstride, const void* d_w1, const float* d_b1, const void* d_w3, const float* d_b3,
+                   const float* d_wl, const float* d_bl, int B, int T, void* stream);
 int vb_cl_codes_sum_parts(float* d_z0, float* d_z1, void* d_code0, void* d_code1, const int64_t* d_codes, const float* d_emb, int B, int K, int bins,
                           int D, int T, void* stream);
 int vb_cl_layernorm_parts(float* d_y, void* d_code, const float* d_x, const float* d_w, const float* d_b, int rows, int C, float eps, void* stream);

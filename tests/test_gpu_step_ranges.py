@@ -560,6 +560,50 @@ def test_channels_last_residual_unit(B, T, C, dil, lo, hi, last, odd):
     assert _lib.load().vb_cl_timeouts() == 0
 
 
+@pytest.mark.parametrize("B,T", [(1, 1), (3, 4), (2, 123), (2, 124), (1, 125), (3, 249), (2, 1000), (300, 130)])
+@pytest.mark.parametrize("kind", ["plain", "one", "quiet", "mixed", "nan", "hidden"])
+def test_channels_last_tail(B, T, kind):
+    """The last unit of Mimi and its convolution to one channel in one launch against 64 bits, also where parts cannot hold a value; and an entry alone."""
+    from vox_serve_b200 import _lib
+    from vox_serve_b200.tokenizer import _cl
+
+    g = torch.Generator(device="cuda").manual_seed(7 * B + T)
+    rnd = lambda *s, std=1.0: torch.randn(*s, generator=g, device="cuda") * std          # noqa: E731
+    w1, b1, w3, b3 = rnd(32, 64, 3, std=192 ** -0.5), rnd(32, std=0.05), rnd(64, 32, std=0.5 * 32 ** -0.5), rnd(64, std=0.05)
+    wl, bl, x = rnd(1, 64, 3, std=0.5 * 192 ** -0.5), rnd(1, std=0.01), rnd(B, T, 64)
+    if kind == "one":
+        x[0, T // 2, 3] = 1e6
+    elif kind == "quiet":
+        x *= 1e-9
+    elif kind == "mixed":
+        x[:, ::3] *= 1e4
+        x[:, 1::3] *= 1e-7
+    elif kind == "nan":
+        x[-1, T // 2, 63] = float("nan")
+    elif kind == "hidden":                         # parts hold the inputs, not what is made of them
+        w1, b1 = w1 * 3e4, b1 * 0
+        w1[::2] *= 1e-9
+    p1, p3, wf = _cl.pack_conv(w1.reshape(32, -1), 64, 3), _cl.pack(w3), wl.reshape(1, -1).contiguous()
+    run = lambda v: _cl.res_tail(_cl.Act(v.contiguous().view(-1), v.shape[0], T, 64), p1, b1, p3, b3, wf, bl)          # noqa: E731
+    got = run(x)
+    elu = lambda v: v.where(v > 0, torch.expm1(v))          # noqa: E731
+
+    def taps(v, w):                                # a product per tap (the library's convolution spreads a NaN further than its taps)
+        k = w.shape[2]
+        v = torch.cat((v.new_zeros(B, k - 1, v.shape[2]), v), 1)
+        return sum(v[:, j:j + T] @ w[:, :, j].T for j in range(k))
+
+    d, e = x.double(), [v.double() for v in (w1, b1, w3[:, :, None], b3, wl, bl)]
+    h = taps(elu(d), e[0]) + e[1]
+    want = (taps(elu(d + taps(elu(h), e[2]) + e[3]), e[4]) + e[5]).transpose(1, 2)
+    assert torch.equal(got.isnan(), want.isnan())
+    ok = want.isfinite()
+    # both factors to 2^-22, sums of 192 in 32 bits: 1.4e-7 measured, as with a launch a convolution
+    assert float((got.double() - want)[ok].norm()) <= 5e-7 * float(want[ok].norm())
+    assert torch.equal(run(x[-1:])[0].view(torch.int32), got[-1].view(torch.int32))
+    assert _lib.load().vb_cl_timeouts() == 0
+
+
 @pytest.mark.parametrize("B,T,C,ksize,left,lo,hi", [(1, 1, 64, 3, 2, 0, 1), (2, 129, 96, 3, 2, 0, 129), (3, 40, 4, 3, 0, 5, 38), (1, 300, 256, 7, 3, 1, 300), (2, 17, 68, 5, 4, 0, 17),
                                                    (1, 130, 128, 16, 15, 0, 130), (2, 16, 32, 1, 0, 0, 16)])
 def test_channels_last_one_output_channel(B, T, C, ksize, left, lo, hi):

@@ -71,6 +71,7 @@ SIGNATURES = {
     "vb_cl_dwconv7_parts": (c_int, [P, P, P, C.c_longlong, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P]),
     "vb_cl_dw_unit_pays": (c_int, [c_int, c_int, c_int, c_int]),
     "vb_cl_dw_unit": (c_int, [P, P, P, P, C.c_longlong, P, P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P]),
+    "vb_cl_res_tail": (c_int, [P, P, C.c_longlong, P, P, P, P, P, P, c_int, c_int, P]),
     "vb_cl_codes_sum_parts": (c_int, [P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P]),
     "vb_cl_layernorm_parts": (c_int, [P, P, P, P, P, c_int, c_int, c_float, P]),
     "vb_cl_chunk_attention_parts": (c_int, [P, P, P, c_int, c_int, c_int, c_int, c_float, P]),

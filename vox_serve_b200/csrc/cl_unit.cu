@@ -1,5 +1,6 @@
 // Residual units of the vocoders over channels-last activations [B][T][C] (fp32), a unit in one launch:
 //   y = x + W s2(dw7(s1(x)) + b1) + b2       (vb_cl_dw_unit: SNAC; s1, s2 Snakes, dw7 a depthwise convolution of 7 taps with dilation)
+// and the end of Mimi's decoder (vb_cl_res_tail, further down).
 // A block owns `nr` positions of one channel tile.  What goes into the product never leaves the block: a warp takes 64 channels, two a lane, and walks a
 // run of positions `dil` apart, so a row of x is loaded and put through its Snake once for the seven sums that it is part of, all in registers; the sums'
 // Snakes are written as the two fp16 parts that the tensor cores multiply (cl_common.cuh) into the operand in shared memory, and the products of 64
@@ -584,6 +585,400 @@ static CuDwPlan cu_dw_plan(int C, int dil, long long range, long long B, int sms
   }
   return best;
 }
+
+// ------------------------------------------------------------------------------------------
+// the end of Mimi's decoder: last residual unit, ELU and the convolution to one channel
+// ------------------------------------------------------------------------------------------
+// out[t] = bl + sum_j wl_j . e(y[t - 2 + j]),  y = x + W3 e(h) + b3,  h[t] = b1 + sum_j W1_j e(x[t - 2 + j]),  e = ELU, 64 channels, 32 hidden ones
+//
+// Here positions are the lanes of the accumulators and channels their columns: a thread has a position's channels side by side, so parts need no exchange
+// between lanes and the last sum over the channels is the thread's own.  A group of eight warps takes 128 positions -- two of them only for the unit's
+// first convolution, two more for the last one -- through five steps: the tile of x by TMA, its ELU as parts in its place (a thread keeps its 32 values for the
+// residual), three taps of products, ELU of the hidden channels as parts, products, ELU and the taps of the last convolution.  The next tile comes
+// while the second half runs.  Nothing but x is read and nothing but the samples is written; two groups run into the gaps of one another.
+// What bounds it: instructions, some 12,000 of a warp's a tile (the ELUs more than half) at 45 % of the issue slots, two groups of one SM waiting for products
+// between their steps.  32 x 19,200 positions: 127 us, before as three launches 88 + 113 + 60, and the convolution in front writes its result once
+// (111 -> 70 us).  With x kept in shared memory and fetched between tiles 143.
+constexpr int CT_C = 64, CT_H = 32, CT_TAPS = 3, CT_ROWS = 128, CT_OUT = CT_ROWS - 2 * (CT_TAPS - 1), CT_PAD = 8;
+constexpr int CT_GROUPS = 2, CT_GROUP_THREADS = 256, CT_THREADS = CT_GROUPS * CT_GROUP_THREADS;
+constexpr int CT_X = CT_ROWS * 256, CT_OP1 = 2 * (CT_PAD + CT_ROWS) * 128, CT_OP2 = CT_ROWS * 128, CT_GROUP_BYTES = CT_OP1 + CT_OP2;
+constexpr int CT_W1 = CT_TAPS * 2 * 2 * CT_H * 128, CT_W3 = 2 * CT_C * 128;          // every row twice, the second time with its low parts in front
+struct CtTables {            // behind the tiles in shared memory
+  float inv1[CT_H], b1[CT_H], inv3[CT_C], b3[CT_C], wl[CT_TAPS][CT_C];
+  float sums[CT_GROUPS][2][CT_TAPS][CT_ROWS];
+  uint8_t raw1[CT_GROUPS][2][CT_PAD + CT_ROWS], raw2[CT_GROUPS][CT_ROWS], odd[CT_GROUPS][2][CT_ROWS];
+  uint64_t x_full[CT_GROUPS], m1[CT_GROUPS], m3[CT_GROUPS];
+  uint32_t tmem, gate;
+};
+constexpr int CT_SMEM = 1024 + CT_GROUPS * CT_GROUP_BYTES + CT_W1 + CT_W3 + static_cast<int>(sizeof(CtTables)) + 16;
+static_assert(CT_SMEM <= VB_MAX_DYN_SMEM, "tail of Mimi: shared memory");
+struct CtParams {
+  const uint8_t *w1, *w3;    // packed (vb_cl_pack)
+  const float *inv1, *b1, *inv3, *b3, *wl, *bl;
+  float* y;                  // [B][T]
+  int T, t_tiles, tiles;
+  uint32_t t_tiles_inv;
+  unsigned char* wait_flag;
+};
+__device__ __forceinline__ float4 ct_lds4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void ct_sts4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+// sixteen channels of a row as parts: 16-byte chunks `at` and `at` + 1 of the high ones, four further on the low ones
+__device__ __forceinline__ void ct_put16(uint32_t row, int sw, int at, const F2 (&v)[8]) {
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cl_parts(v[4 * c + i], CL_X_SCALE, hi[i], lo[i]);
+    ct_sts4(row + (((at + c) ^ sw) << 4), hi[0], hi[1], hi[2], hi[3]);
+    ct_sts4(row + (((at + c + 4) ^ sw) << 4), lo[0], lo[1], lo[2], lo[3]);
+  }
+}
+// what is multiplied for channel c of a row of an operand, and for input c of row n of the weights
+__device__ __forceinline__ float ct_value(uint32_t row, int r, int c, bool raw) {
+  float f;
+  if (raw) {
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(row + (((c >> 2) ^ (r & 7)) << 4) + (c & 3) * 4));
+    return f;
+  }
+  const uint32_t a = row + (((c >> 3) ^ (r & 7)) << 4) + (c & 7) * 2;
+  uint16_t hi, lo;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hi) : "r"(a));
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(lo) : "r"(a ^ 64u));
+  return fmaf(__half2float(__ushort_as_half(lo)), 1.f / CL_LO_SCALE, __half2float(__ushort_as_half(hi)));
+}
+// The hidden channels of a thread's position once more where its inputs or they themselves may not be parts: in fp32 if an input is not, and kept as
+// what the whole block of 32 says.  All lanes load, those that `redo` names store.
+__device__ __noinline__ bool ct_hidden(const CtTables& tb, int group, int row, int first, uint32_t op1, uint32_t w1, uint32_t op2, uint32_t d, bool redo) {
+  float v[CT_H];
+  for (int c = 0; c < CT_H; c += 8) {
+    uint32_t hi[8], lo[8];
+    tmem_ld_32x8(d + c, hi);
+    tmem_ld_32x8(d + CT_H + c, lo);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      v[c + i] = fmaf(fmaf(__uint_as_float(lo[i]), 1.f / CL_LO_SCALE, __uint_as_float(hi[i])), tb.inv1[c + i], tb.b1[c + i]);
+  }
+  if (!redo) return false;
+  bool exact = false;
+  for (int j = 0; j < CT_TAPS; ++j) exact |= tb.raw1[group][0][CT_PAD + row - 2 + j] | tb.raw1[group][1][CT_PAD + row - 2 + j];
+  float m = 0.f;
+#pragma unroll 1
+  for (int n = 0; n < CT_H; ++n) {
+    float a = v[n];
+    if (exact) {
+      a = 0.f;
+#pragma unroll 1
+      for (int j = 0; j < CT_TAPS; ++j) {
+        const int r = CT_PAD + row - 2 + j;
+        if (r < first) continue;           // (in front of the entry)
+#pragma unroll 1
+        for (int b = 0; b < 2; ++b) {
+          const bool raw = tb.raw1[group][b][r];
+          const uint32_t x = op1 + b * (CT_OP1 / 2) + r * 128, w = w1 + (j * 2 + b) * 2 * CT_H * 128 + n * 128;
+#pragma unroll 1
+          for (int k = 0; k < 32; ++k)
+            a = fmaf(ct_value(x, r, k, raw) * (raw ? 1.f : 1.f / CL_X_SCALE), ct_value(w, n, k, false) * (tb.inv1[n] * CL_X_SCALE), a);
+        }
+      }
+      a += tb.b1[n];
+    }
+    a = f2_get(cl_elu(f2(a, a))).x;
+    v[n] = a;
+    m = max3_abs(m, a, a);
+  }
+  const bool raw = cl_code(m) == CB_RAW;
+  const uint32_t o = op2 + row * 128;
+  for (int c = 0; c < 8; ++c) {
+    uint32_t q[4];
+    for (int i = 0; i < 4; ++i) {
+      if (raw) {
+        q[i] = __float_as_uint(v[4 * c + i]);
+      } else {
+        const int at = (c & 3) * 8 + 2 * i;
+        uint32_t hi, lo;
+        cl_parts(f2(v[at], v[at + 1]), CL_X_SCALE, hi, lo);
+        q[i] = c < 4 ? hi : lo;
+      }
+    }
+    ct_sts4(o + ((c ^ (row & 7)) << 4), q[0], q[1], q[2], q[3]);
+  }
+  return raw;
+}
+// the last step for a warp some of whose positions have hidden channels that are not parts
+__device__ __noinline__ void ct_last(const CtTables& tb, int row, int half, const F2 (&x)[16], uint32_t w3, uint32_t op2, uint32_t d, bool raw, float (&s)[CT_TAPS]) {
+  float v[32];
+  for (int c = 0; c < 32; c += 8) {
+    uint32_t hi[8], lo[8];
+    tmem_ld_32x8(d + c, hi);
+    tmem_ld_32x8(d + CT_C + c, lo);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      v[c + i] = fmaf(fmaf(__uint_as_float(lo[i]), 1.f / CL_LO_SCALE, __uint_as_float(hi[i])), tb.inv3[half * 32 + c + i], tb.b3[half * 32 + c + i]);
+  }
+#pragma unroll 1
+  for (int c = 0; c < 32; ++c) {
+    const int n = half * 32 + c;
+    float a = v[c];
+    if (raw) {
+      a = 0.f;
+#pragma unroll 1
+      for (int k = 0; k < CT_H; ++k) a = fmaf(ct_value(op2 + row * 128, row, k, true), ct_value(w3 + n * 128, n, k, false) * (tb.inv3[n] * CL_X_SCALE), a);
+      a += tb.b3[n];
+    }
+    const float2 res = f2_get(x[c >> 1]);
+    a += c & 1 ? res.y : res.x;
+    a = f2_get(cl_elu(f2(a, a))).x;
+#pragma unroll
+    for (int j = 0; j < CT_TAPS; ++j) s[j] = fmaf(tb.wl[j][n], a, s[j]);
+  }
+}
+
+__global__ void __launch_bounds__(CT_THREADS, 1) cl_res_tail_kernel(const __grid_constant__ CtParams p, const __grid_constant__ CUtensorMap xmap) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  CtTables& tb = *reinterpret_cast<CtTables*>(smem + CT_GROUPS * CT_GROUP_BYTES + CT_W1 + CT_W3);
+  const int group = threadIdx.x / CT_GROUP_THREADS, tid = threadIdx.x % CT_GROUP_THREADS, warp = tid >> 5, lane = tid & 31;
+  const int half = warp >> 2, row = (warp & 3) * 32 + lane, sw = row & 7;
+  const uint32_t op1 = smem_u32(smem) + group * CT_GROUP_BYTES, op2 = op1 + CT_OP1;
+  const uint32_t w1 = smem_u32(smem) + CT_GROUPS * CT_GROUP_BYTES, w3 = w1 + CT_W1, gate = smem_u32(&tb.gate);
+  BoundedWait bw{p.wait_flag, gate};
+
+  if (threadIdx.x == 0) {
+    tb.gate = 0u;
+    prefetch_tmap(&xmap);
+    for (int i = 0; i < CT_GROUPS; ++i) {
+      mbar_init(&tb.x_full[i], 1);
+      mbar_init(&tb.m1[i], 1);
+      mbar_init(&tb.m3[i], 1);
+    }
+    fence_barrier_init();
+  }
+  if (threadIdx.x < 32) {
+    tmem_alloc(&tb.tmem, 512);
+    tmem_relinquish();
+  }
+  for (int i = threadIdx.x; i < CT_C; i += CT_THREADS) {
+    if (i < CT_H) tb.inv1[i] = __ldg(p.inv1 + i), tb.b1[i] = __ldg(p.b1 + i);
+    tb.inv3[i] = __ldg(p.inv3 + i);
+    tb.b3[i] = __ldg(p.b3 + i);
+    for (int j = 0; j < CT_TAPS; ++j) tb.wl[j][i] = __ldg(p.wl + i * CT_TAPS + j);
+  }
+  // Weights (they do not depend on the kernels in front): the first 32 or 64 of a packed block's 128 rows as high parts, and again as low ones, so that one
+  // instruction multiplies the activations' high parts by both
+  auto weights = [&](const uint8_t* src, int rows, uint32_t dst) {
+    for (int i = threadIdx.x; i < rows * 8; i += CT_THREADS) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(src) + i);
+      ct_sts4(dst + i * 16, v.x, v.y, v.z, v.w);
+      ct_sts4(dst + rows * 128 + (i ^ 4) * 16, v.x, v.y, v.z, v.w);
+    }
+  };
+  for (int i = 0; i < CT_TAPS * 2; ++i) weights(p.w1 + static_cast<size_t>(i) * CL_W_BLOCK, CT_H, w1 + i * 2 * CT_H * 128);
+  weights(p.w3, CT_C, w3);
+  for (int i = tid; i < 2 * CT_PAD; i += CT_GROUP_THREADS) tb.raw1[group][i / CT_PAD][i % CT_PAD] = 0;
+  for (int i = tid; i < 2 * CT_PAD * 8; i += CT_GROUP_THREADS)          // rows in front of a tile: read for positions that nothing is made of
+    ct_sts4(op1 + (i / (CT_PAD * 8)) * (CT_OP1 / 2) + (i % (CT_PAD * 8)) * 16, 0u, 0u, 0u, 0u);
+  fence_proxy_async();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t d1 = tb.tmem + group * 256, d3 = d1 + 2 * CT_H, lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
+  const float bl = __ldg(p.bl);
+  pdl_wait();
+  if (threadIdx.x == 0) wait_gate_open(gate);
+  pdl_trigger();
+  auto tile_of = [&](int i, int& b, int& t0) {
+    b = cu_div(i, p.t_tiles, p.t_tiles_inv);
+    t0 = (i - b * p.t_tiles) * CT_OUT - 2 * (CT_TAPS - 1);           // position of row 0
+  };
+  auto fetch = [&](int i) {
+    int b, t0;
+    tile_of(i, b, t0);
+    mbar_arrive_expect_tx(&tb.x_full[group], CT_X);
+    for (int k = 0; k < 2; ++k) tma_load_3d(op1 + k * (CT_OP1 / 2) + CT_PAD * 128, &xmap, smem_u32(&tb.x_full[group]), k * 32, t0, b);
+  };
+  auto meet = [&](bool any) { return group == 0 ? warps_any<1, CT_GROUP_THREADS>(any) : warps_any<2, CT_GROUP_THREADS>(any); };
+  const uint64_t a1 = umma_desc_sw128_kmajor(op1 + (CT_PAD - CT_TAPS + 1) * 128), a3 = umma_desc_sw128_kmajor(op2);
+  const uint64_t b1 = umma_desc_sw128_kmajor(w1), b3 = umma_desc_sw128_kmajor(w3);
+  const int step = CT_GROUPS * gridDim.x;
+  int tile = blockIdx.x + group * gridDim.x;
+  if (tid == 0 && tile < p.tiles) fetch(tile);
+  uint32_t ph = 0;
+#pragma unroll 1
+  for (; tile < p.tiles; tile += step, ph ^= 1u) {
+    int b, t0;
+    tile_of(tile, b, t0);
+    bw.wait(&tb.x_full[group], ph);
+    // ---- ELU of the tile as parts, in its place: a thread's position, 32 of its channels, which it keeps for the residual ----
+    const uint32_t o1 = op1 + half * (CT_OP1 / 2) + (CT_PAD + row) * 128;
+    F2 x[16];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float4 v = ct_lds4(o1 + ((c ^ sw) << 4));
+      x[2 * c] = f2(v.x, v.y);
+      x[2 * c + 1] = f2(v.z, v.w);
+    }
+    float m = 0.f;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      F2 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        v[i] = cl_elu(x[8 * q + i]);
+        const float2 e = f2_get(v[i]);
+        m = max3_abs(m, e.x, e.y);
+      }
+      ct_put16(o1, sw, 2 * q, v);
+    }
+    const bool raw = cl_code(m) == CB_RAW;
+    if (raw) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float2 e = f2_get(cl_elu(x[2 * c])), f = f2_get(cl_elu(x[2 * c + 1]));
+        ct_sts4(o1 + ((c ^ sw) << 4), __float_as_uint(e.x), __float_as_uint(e.y), __float_as_uint(f.x), __float_as_uint(f.y));
+      }
+    }
+    tb.raw1[group][half][CT_PAD + row] = raw;
+    fence_proxy_async();
+    const bool odd1 = meet(raw);
+    if (warp == 0) {
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll 1
+        for (int i = 0; i < 2 * CT_TAPS; ++i) {          // tap, then block of 32 channels
+          const uint64_t a = a1 + (i >> 1) * 8 + (i & 1) * (CT_OP1 / 2 >> 4), w = b1 + i * (2 * CT_H * 128 >> 4);
+#pragma unroll 1
+          for (int k = 0; k < 2; ++k) {
+            umma_bf16(d1, a + 2 * k, w + 2 * k, umma_idesc(128, 2 * CT_H, 0u), (i | k) ? 1u : 0u);
+            umma_bf16(d1 + CT_H, a + 4 + 2 * k, w + 2 * k, umma_idesc(128, CT_H, 0u), 1u);
+          }
+        }
+        umma_commit(&tb.m1[group]);
+      }
+      __syncwarp();
+    }
+    bw.wait(&tb.m1[group], ph);
+    __syncwarp();
+    tc_fence_after();
+    if (tid == 0 && !odd1 && tile + step < p.tiles) fetch(tile + step);          // (the operand has been read; where fp32 is in it, once more below)
+    // ---- ELU of the hidden channels as parts: sixteen of them ----
+    {
+      uint32_t hi[16], lo[16];
+      tmem_ld_32x16(d1 + lanes + half * 16, hi);
+      tmem_ld_32x16(d1 + lanes + CT_H + half * 16, lo);
+      tmem_ld_wait();
+      F2 v[8];
+      m = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float2 s = *reinterpret_cast<const float2*>(tb.inv1 + half * 16 + 2 * i), c = *reinterpret_cast<const float2*>(tb.b1 + half * 16 + 2 * i);
+        v[i] = f2_fma(f2(__uint_as_float(lo[2 * i]), __uint_as_float(lo[2 * i + 1])), f2(1.f / CL_LO_SCALE), f2(__uint_as_float(hi[2 * i]), __uint_as_float(hi[2 * i + 1])));
+        v[i] = cl_elu(f2_fma(v[i], f2(s.x, s.y), f2(c.x, c.y)));
+        const float2 e = f2_get(v[i]);
+        m = max3_abs(m, e.x, e.y);
+      }
+      ct_put16(op2 + row * 128, sw, 2 * half, v);
+    }
+    // (both halves in range: the block of 32 is)
+    tb.odd[group][half][row] = !cl_fits(m);
+    fence_proxy_async();
+    tc_fence_before();
+    const bool odd = meet(odd1 || !cl_fits(m));
+    if (odd) {
+      if (half == 0) {
+        tc_fence_after();
+        bool redo = tb.odd[group][0][row] || tb.odd[group][1][row];
+        for (int j = row < 2 ? 2 - row : 0; j < CT_TAPS; ++j) redo |= tb.raw1[group][0][CT_PAD + row - 2 + j] || tb.raw1[group][1][CT_PAD + row - 2 + j];
+        tb.raw2[group][row] = ct_hidden(tb, group, row, CT_PAD - t0, op1, w1, op2, d1 + lanes, redo && row >= 2);
+        fence_proxy_async();
+        tc_fence_before();
+      }
+      meet(false);
+    }
+    if (warp == 0) {
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll 1
+        for (int k = 0; k < 2; ++k) {
+          umma_bf16(d3, a3 + 2 * k, b3 + 2 * k, umma_idesc(128, 2 * CT_C, 0u), k);
+          umma_bf16(d3 + CT_C, a3 + 4 + 2 * k, b3 + 2 * k, umma_idesc(128, CT_C, 0u), 1u);
+        }
+        umma_commit(&tb.m3[group]);
+      }
+      __syncwarp();
+    }
+    bw.wait(&tb.m3[group], ph);
+    __syncwarp();
+    tc_fence_after();
+    // ---- residual, ELU, the taps of the last convolution: 32 channels ----
+    float s[CT_TAPS] = {};
+    if (!odd || !__any_sync(0xffffffffu, tb.raw2[group][row])) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint32_t hi[16], lo[16];
+        tmem_ld_32x16(d3 + lanes + half * 32 + q * 16, hi);
+        tmem_ld_32x16(d3 + lanes + CT_C + half * 32 + q * 16, lo);
+        const int n0 = half * 32 + q * 16;
+        tmem_ld_wait();
+        F2 v[8], sum[CT_TAPS];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float4 g = *reinterpret_cast<const float4*>(tb.inv3 + n0 + 4 * c), a = *reinterpret_cast<const float4*>(tb.b3 + n0 + 4 * c);
+          auto one = [&](int i, F2 g2, F2 a2, F2 x2) {
+            F2 u = f2_fma(f2(__uint_as_float(lo[i]), __uint_as_float(lo[i + 1])), f2(1.f / CL_LO_SCALE), f2(__uint_as_float(hi[i]), __uint_as_float(hi[i + 1])));
+            return f2_add(f2_fma(u, g2, a2), x2);
+          };
+          v[2 * c] = one(4 * c, f2(g.x, g.y), f2(a.x, a.y), x[8 * q + 2 * c]);
+          v[2 * c + 1] = one(4 * c + 2, f2(g.z, g.w), f2(a.z, a.w), x[8 * q + 2 * c + 1]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = cl_elu(v[i]);
+#pragma unroll
+        for (int j = 0; j < CT_TAPS; ++j) {
+          sum[j] = f2(0.f);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const float4 g = *reinterpret_cast<const float4*>(tb.wl[j] + n0 + 4 * c);
+            sum[j] = f2_fma(v[2 * c], f2(g.x, g.y), sum[j]);
+            sum[j] = f2_fma(v[2 * c + 1], f2(g.z, g.w), sum[j]);
+          }
+          const float2 e = f2_get(sum[j]);
+          s[j] += e.x + e.y;
+        }
+      }
+    } else {
+      ct_last(tb, row, half, x, w3, op2, d3 + lanes + half * 32, tb.raw2[group][row], s);
+    }
+#pragma unroll
+    for (int j = 0; j < CT_TAPS; ++j) tb.sums[group][half][j][row] = t0 + row < 0 ? 0.f : s[j];
+    tc_fence_before();
+    if (meet(bw.dead)) break;
+    if (tid == 0 && odd1 && tile + step < p.tiles) fetch(tile + step);
+    if (half == 0 && row >= 2 * (CT_TAPS - 1) && t0 + row < p.T) {
+      float o = bl;
+#pragma unroll
+      for (int j = 0; j < CT_TAPS; ++j) o += tb.sums[group][0][j][row - 2 + j] + tb.sums[group][1][j][row - 2 + j];
+      p.y[static_cast<long long>(b) * p.T + t0 + row] = o;
+    }
+  }
+  if (__syncthreads_or(bw.dead) && threadIdx.x == 0) {            // let the copies in flight land before the block may leave
+    const unsigned long long from = gtimer();
+    while (gtimer() - from < 2000000ull) __nanosleep(1000);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    tc_fence_after();
+    tmem_dealloc(tb.tmem, 512);
+  }
+}
 }  // namespace vb
 
 using namespace vb;
@@ -633,6 +1028,34 @@ int vb_cl_dw_unit(float* d_y, void* d_yp, void* d_yp_code, const float* d_x, lon
     VB_CHECK_CUDA(max_dyn_smem_once(cl_dw_unit_kernel<18>));
     VB_LAUNCH_PDL(cl_dw_unit_kernel<18>, grid, 608, g.smem, stream, p);
   }
+  return 0;
+}
+
+int vb_cl_res_tail(float* d_y, const float* d_x, long long x_bstride, const void* d_w1, const float* d_b1, const void* d_w3, const float* d_b3,
+                   const float* d_wl, const float* d_bl, int B, int T, void* stream) {
+  VB_CHECK_ARG(d_y && d_x && d_w1 && d_b1 && d_w3 && d_b3 && d_wl && d_bl, "vb_cl_res_tail: null pointer");
+  VB_CHECK_ARG(T > 0 && x_bstride % 4 == 0 && on16(d_x) && on16(d_w1) && on16(d_w3), "vb_cl_res_tail: rows and weights must start on 16-byte boundaries");
+  if (B <= 0) return 0;
+  VB_CHECK_ARG(encode_fn(), "cuTensorMapEncodeTiled not available (no CUDA driver?)");
+  CtParams p = {};
+  VB_CHECK_ARG(p.wait_flag = wait_flag(WK_CL_CONV), "vb_cl_res_tail: no mapped host memory");
+  p.w1 = static_cast<const uint8_t*>(d_w1); p.w3 = static_cast<const uint8_t*>(d_w3);
+  p.inv1 = reinterpret_cast<const float*>(p.w1 + static_cast<size_t>(CT_TAPS) * 2 * CL_W_BLOCK); p.inv3 = reinterpret_cast<const float*>(p.w3 + CL_W_BLOCK);
+  p.b1 = d_b1; p.b3 = d_b3; p.wl = d_wl; p.bl = d_bl; p.y = d_y; p.T = T;
+  p.t_tiles = (T + CT_OUT - 1) / CT_OUT;
+  const long long tiles = static_cast<long long>(p.t_tiles) * B;
+  VB_CHECK_ARG(tiles < 0x7fffffffLL - 2 * CT_GROUPS * 1024, "vb_cl_res_tail: too many tiles");
+  p.tiles = static_cast<int>(tiles);
+  p.t_tiles_inv = p.t_tiles > 1 ? static_cast<uint32_t>(((1ULL << 32) + p.t_tiles - 1) / p.t_tiles) : 0u;
+  CUtensorMap map;
+  cuuint64_t dims[3] = {CT_C, static_cast<cuuint64_t>(T), static_cast<cuuint64_t>(B)};
+  cuuint64_t strides[2] = {CT_C * 4, static_cast<cuuint64_t>(B > 1 ? x_bstride : static_cast<long long>(T) * CT_C) * 4};
+  cuuint32_t box[3] = {32, CT_ROWS, 1}, estr[3] = {1, 1, 1};
+  const CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(d_x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  VB_CHECK_ARG(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(tail) failed: CUresult %d", static_cast<int>(r));
+  VB_CHECK_CUDA(max_dyn_smem_once(cl_res_tail_kernel));
+  VB_LAUNCH_PDL(cl_res_tail_kernel, min(p.tiles, cu_sms()), CT_THREADS, CT_SMEM, stream, p, map);
   return 0;
 }
 

@@ -129,6 +129,14 @@ def dw_unit(x: Act, dw_w: torch.Tensor, dw_b, alpha_in, alpha_mid, w: torch.Tens
     return y
 
 
+def res_tail(x: Act, w1: torch.Tensor, b1, w3: torch.Tensor, b3, wl: torch.Tensor, bl) -> torch.Tensor:
+    """The last residual unit of 64 channels (three taps to 32, ELU, 1x1 back), ELU and the convolution of three taps to one channel -> [B, 1, T]"""
+    y = torch.empty(x.B, 1, x.T, dtype=torch.float32, device=x.buf.device)
+    call("vb_cl_res_tail", y.data_ptr(), x.ptr, x.bstride, w1.data_ptr(), b1.data_ptr(), w3.data_ptr(), b3.data_ptr(), wl.data_ptr(), bl.data_ptr(), x.B, x.T,
+         ops._stream())
+    return y
+
+
 def last_conv(x: Act, w: torch.Tensor, bias, ksize: int, left: int, t0: int, t1: int, tanh: bool) -> torch.Tensor:
     """one output channel -> [B, 1, t1 - t0]; w [C, ksize]"""
     y = torch.empty(x.B, 1, t1 - t0, dtype=torch.float32, device=x.buf.device)

@@ -264,7 +264,12 @@ class MimiDecoder:
                 x = _cl.conv(x, tc[d + "w"], ch, w[d + "b"], ksize=cfg.kernel_size, act="elu", out="parts")
             elif kind == "convtr":
                 ch //= 2
-                plain, x = _cl.conv_transposed(x, tc[d + "w"], ch, ratios.pop(0), w[d + "b"], act="elu", both=True, out="parts")
+                tail = len(ratios) == 1 and (ch, ch // cfg.compress, cfg.residual_kernel_size, cfg.last_kernel_size) == (64, 32, 3, 3)
+                args = x, tc[d + "w"], ch, ratios.pop(0), w[d + "b"]
+                if tail:                                   # what is left runs as one launch
+                    (_, r), (_, o) = self.layout[-2:]
+                    return _cl.res_tail(_cl.conv_transposed(*args), tc[f"d{r}.w1"], w[f"d{r}.b1"], tc[f"d{r}.w3"], w[f"d{r}.b3"], w[f"d{o}.w"], w[f"d{o}.b"])
+                plain, x = _cl.conv_transposed(*args, act="elu", both=True, out="parts")
             elif kind == "res":
                 h = _cl.conv(x, tc[d + "w1"], ch // cfg.compress, w[d + "b1"], ksize=cfg.residual_kernel_size, act="elu", out="parts")
                 x = _cl.conv(h, tc[d + "w3"], ch, w[d + "b3"], epi="resid", resid=plain, act="elu", out="parts" if ratios else "f32")

@@ -501,6 +501,11 @@ int vb_gemm_bf16_grouped_glu(void* d_y, const void* d_w_tiles, const void* x_map
 int vb_gemm_bf16_wide(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
                       int mode, int split_k, int tile_rows, int n_out, int y_tiled, const void* d_bias, int act, int n_tok,
                       void* stream);
+/* ... with a table of token tiles: d_tiles int32 [1 + tiles_max][4], the first entry their number, then (group, first row, rows, -), up to 256 rows each (what
+ * vb_moe_group_tiles writes).  It must not come from the kernel right in front: it is read while that one runs.  x_maps: four tensor maps of the rows with
+ * boxes of 64, 80, 96 and 128. */
+int vb_gemm_bf16_wide_tiles(void* d_y, const void* d_w_tiles, const void* const* x_maps, int T, int N, int K, int ldy, int mode, int tile_rows, int n_out, int act,
+                            const int32_t* d_tiles, int tiles_max, long long group_bytes, int w_kb_stride, int group_kb, float glu_limit, float glu_slope, void* stream);
 int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
                               int mode, int split_k, int tile_rows, int n_out, int y_tiled, const void* d_bias, int act, int n_tok,
                               const int32_t* d_tile_group, long long group_bytes, int w_kb_stride, int group_kb, int kb_base,
@@ -783,6 +788,10 @@ int vb_moe_group(int32_t* d_row_off, int32_t* d_sorted_token, int32_t* d_pair_ro
 /* (tile_rows > 0: every expert's rows start at a multiple of tile_rows; padding rows get token -1; d_tile_group[i] =
  * the expert of row tile i, 0 for tiles past the last expert, i < n_tiles >= ceil(T * top / tile_rows) + experts)
  * vb_moe_gather_rows: out[r] = token[r] >= 0 ? x[token[r]] : 0, bf16 rows of `width` (a multiple of 8) */
+/* Pairs by expert for vb_gemm_bf16_wide_tiles: with `shared` rows [0, T) are every token once (group `experts`), then every expert's rows from a multiple of 16 on;
+ * token -1 elsewhere.  (n_a, k_a), (n_b, k_b): the two projections that the height of the tiles is chosen for.  rows_max >= round16(T if shared) + T top + 15 experts. */
+int vb_moe_group_tiles(int32_t* d_sorted_token, int32_t* d_pair_row, int32_t* d_tiles, const int32_t* d_idx, int T, int experts, int top, int shared, int rows_max,
+                       int tiles_max, int n_a, int k_a, int n_b, int k_b, void* stream);
 int vb_moe_gather_rows(void* d_out, const void* d_x, const int32_t* d_token, int rows, int width, void* stream);
 /* dense form (bf16): act [T][ld] holds silu(gate) * up of EVERY expert side by side (expert e at columns e * ff ..), then
  * the shared expert's; columns of expert e are scaled by the token's routing weight for e, or zeroed if e was not chosen */

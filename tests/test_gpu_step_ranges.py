@@ -152,6 +152,57 @@ def test_wide_grouped_projection(ops, groups, tt, N, K):
 
 # channels-last vocoder convolutions: one row and several batch entries in a box, box sizes around 128 rows, a range inside the
 # sequence, column tiles with a remainder, dilated taps reaching in front of the start; every epilogue and activation
+@pytest.mark.parametrize("T,E,top,shared,N,K,skew", [(1, 4, 1, True, 256, 128, False), (17, 3, 2, False, 320, 200, False), (700, 8, 2, True, 512, 256, False),
+                                                     (1001, 8, 2, True, 384, 192, True), (513, 70, 4, False, 128, 64, False), (300, 5, 3, True, 256, 128, True)])
+@pytest.mark.parametrize("mode,tile_rows", [(0, 128), (1, 128), (2, 96), (2, 64)])
+def test_projection_of_tile_tables(ops, T, E, top, shared, N, K, skew, mode, tile_rows):
+    """Every row times its expert's weights, with experts that nobody picked and one that everybody did; the shared expert's rows are the tokens."""
+    N = N // (2 * tile_rows) * 2 * tile_rows if mode == 2 else N
+    N = max(N, 2 * tile_rows) if mode == 2 else N
+    g = torch.Generator(device="cuda").manual_seed(T + E + mode)
+    G = E + int(shared)
+    w, x = torch.randn(G, N, K, generator=g, device="cuda").bfloat16(), torch.randn(T, K, generator=g, device="cuda").bfloat16()
+    pick = torch.argsort(torch.rand(T, E, generator=g, device="cuda"), 1)[:, :top].to(torch.int32)
+    if skew:                                   # expert 0 for all, the others from the upper half
+        pick = torch.cat((torch.zeros(T, 1, device="cuda", dtype=torch.int32), E // 2 + pick[:, :top - 1] % (E - E // 2)), 1)
+    idx = pick.contiguous()
+    rows = ((T + 15) // 16 * 16 if shared else 0) + T * top + 16 * E
+    token, pair = torch.full((rows,), -7, dtype=torch.int32, device="cuda"), torch.zeros(T * top, dtype=torch.int32, device="cuda")
+    tiles = torch.zeros(1 + (T * top + 255) // 256 + (T + 255) // 256 + E + 20, 4, dtype=torch.int32, device="cuda")
+    ops.moe_group_tiles(idx, T, E, top, shared, token, pair, tiles, ((N, K), (K, N)))
+    xs = ops.moe_gather_rows(x, token, torch.zeros(rows, K, dtype=torch.bfloat16, device="cuda"))
+    pack = lambda m: ops.pack_weight(ops.interleave_gate_up(m[:N // 2], m[N // 2:], tile_rows // 2) if mode == 2 else m, tile_rows)          # noqa: E731
+    packed = [pack(m.contiguous()) for m in w]
+    gb = ops.weight_tiles_bytes(N, K, tile_rows)
+    whole = ops.PackedWeight(torch.cat([q.data[:gb] for q in packed]), N, K, tile_rows)
+    out = torch.full((rows, N // 2 if mode == 2 else N), -1.0, dtype=torch.float32 if mode == 1 else torch.bfloat16, device="cuda")
+    ops.gemm_tiles(xs, whole, out, mode, N, K, tiles, group_bytes=gb)
+    tab = tiles.cpu()
+    n, covered = int(tab[0, 0]), []
+    for e, r0, m, _ in tab[1:1 + n].tolist():
+        assert 0 < m <= 256 and r0 % 16 == 0
+        covered += [(r, e) for r in range(r0, r0 + m)]
+    tok = token.cpu()
+    assert len(covered) == len(set(r for r, _ in covered)) == T * top + (T if shared else 0) == int((tok >= 0).sum())
+    if shared:
+        assert tok[:T].tolist() == list(range(T))
+    flat = idx.cpu().view(-1).tolist()
+    of = dict(covered)
+    for i, r in enumerate(pair.tolist()):
+        assert tok[r] == i // top and of[r] == flat[i]
+    group = torch.tensor([of.get(r, 0) for r in range(rows)], device="cuda")
+    for e in range(G):
+        r = ((group == e) & (token >= 0)).nonzero()[:, 0]
+        y = xs[r].float() @ w[e].float().T
+        if mode == 2:
+            a, b = y[:, :N // 2].bfloat16().float(), y[:, N // 2:].bfloat16().float()
+            y = (a / (1 + torch.exp(-a))).bfloat16().float() * b
+        if r.numel():
+            d = (out[r].float() - y).abs()
+            assert float(d.max()) <= (1e-5 * K ** 0.5 * 4 if mode == 1 else 2 ** -7 * float(y.abs().max()))          # sums of K in 32 bits; one rounding to bf16 beside ties
+    assert ops.check_waits() is None
+
+
 @pytest.mark.parametrize("B,T,C,N,ksize,dil,lo,hi,epi,act", [
     (1, 1, 32, 32, 1, 1, 0, 1, "plain", None), (7, 16, 64, 96, 1, 1, 0, 16, "resid", "snake"), (2, 128, 32, 128, 3, 1, 0, 128, "plain", "elu"),
     (3, 129, 96, 160, 1, 1, 5, 129, "noise", None), (1, 300, 64, 64, 7, 9, 130, 299, "scale_resid", "gelu"), (40, 3, 128, 512, 2, 1, 0, 3, "resid", None)])

@@ -56,6 +56,8 @@ SIGNATURES = {
     "vb_pack_weight_tiles": (c_int, [P, P, c_int, c_int, c_int64, c_int, P]),
     "vb_gemm_bf16": (c_int, [P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, c_int, P]),
     "vb_gemm_bf16_wide": (c_int, [P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, c_int, c_int, P]),
+    "vb_gemm_bf16_wide_tiles": (c_int, [P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, c_int, C.c_longlong, c_int, c_int, c_float, c_float, P]),
+    "vb_moe_group_tiles": (c_int, [P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P]),
     "vb_gemm_bf16_wide_grouped": (c_int, [P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, c_int, c_int, P,
                                           C.c_longlong, c_int, c_int, c_int, c_float, c_float, P]),
     "vb_gemm_wide_timeouts": (c_int, []),

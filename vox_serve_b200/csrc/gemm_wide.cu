@@ -24,6 +24,7 @@
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 2
 #include "common.cuh"
+#include <type_traits>
 
 namespace vb {
 
@@ -40,6 +41,8 @@ struct GemmWideParams {
   const uint8_t* x_tiles;      // XT(x_tile) layout, or nullptr: x_map
   const __nv_bfloat16* bias;
   const int32_t* tile_group;   // group of every token tile (nullptr: one group)
+  const int4* tiles;           // or a table of token tiles: [0].x of them, then (group, first row, rows, -) each
+  int tiles_max;
   long long group_bytes;
   int T, N, K, ldy, mode, split_k, tile_rows, sub, n_out, act, y_tiled, x_tile;
   int n_tok;                   // token rows per tile (multiple of 16, <= 256)
@@ -120,11 +123,36 @@ __device__ __forceinline__ void gw_div8(float (&a)[8], const float (&d)[8]) {
   for (int i = 0; i < 8; ++i) a[i] = q[i];
 }
 
+// boxes of half a token tile, by its rows: a table's tiles differ, and what a box has beyond its tile is copied for nothing
+constexpr int GW_BOXES = 4;
+template <bool TABLE>
+struct GwMaps {
+  CUtensorMap m[TABLE ? GW_BOXES : 1];     // 64, 80, 96, 128 rows; without a table half of n_tok
+};
+__host__ __device__ __forceinline__ int gw_box(int half) { return half <= 64 ? 0 : half <= 80 ? 1 : half <= 96 ? 2 : 3; }
+__host__ __device__ __forceinline__ int gw_box_rows(int i) { return i == 0 ? 64 : i == 1 ? 80 : i == 2 ? 96 : 128; }
 struct GwUnit {
   int split, pair, tblk, kb0, kb1, t0, n_cur;    // n_cur: token rows of the tile rounded up to 16
 };
-__device__ __forceinline__ GwUnit gw_unit(const GemmWideParams& p, int u) {
-  GwUnit r;
+struct GwTableUnit : GwUnit {
+  int t_end, group;
+};
+template <bool TABLE>
+__device__ __forceinline__ std::conditional_t<TABLE, GwTableUnit, GwUnit> gw_unit(const GemmWideParams& p, const int4* table, int n_tiles, int u) {
+  std::conditional_t<TABLE, GwTableUnit, GwUnit> r;
+  if constexpr (TABLE) {
+    r.split = 0;
+    r.pair = u / n_tiles;
+    r.tblk = u - r.pair * n_tiles;
+    r.kb0 = 0;
+    r.kb1 = p.num_kb;
+    const int4 t = table[r.tblk];
+    r.group = t.x;
+    r.t0 = t.y;
+    r.t_end = t.y + t.z;
+    r.n_cur = (t.z + 15) & ~15;
+    return r;
+  }
   // token tiles fastest: the pairs that run side by side share weight tiles in L2
   const int per_split = p.n_pairs * p.t_blocks;
   r.split = u / per_split;
@@ -138,9 +166,12 @@ __device__ __forceinline__ GwUnit gw_unit(const GemmWideParams& p, int u) {
   return r;
 }
 
+__device__ __forceinline__ int gw_end(const GemmWideParams& p, const GwUnit&) { return p.T; }
+__device__ __forceinline__ int gw_end(const GemmWideParams&, const GwTableUnit& g) { return g.t_end; }
 // (bounded to 128 registers: what is left of the file holds the first blocks of the kernel behind this one, which start early)
+template <bool TABLE>          // token tiles from a table (p.tiles)
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
-    gemm_wide_kernel(const GemmWideParams p, const __grid_constant__ CUtensorMap x_map) {
+    gemm_wide_kernel(const GemmWideParams p, const __grid_constant__ GwMaps<TABLE> maps) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int b_bytes = p.n_tok * 64;                 // half of the token tile's rows (a multiple of 1024)
@@ -153,6 +184,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
   uint64_t* acc_empty = acc_full + 2;                                             // (leader) [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   const uint32_t gate = smem_u32(tmem_slot + 1);                                  // set once the kernels in front have completed
+  int4* table = reinterpret_cast<int4*>(smem + p.stages * stage_bytes + 512);     // of p.tiles
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -161,7 +193,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
 
   if (warp == 0 && lane == 0) {
     tmem_slot[1] = 0u;
-    if (!p.x_tiles) prefetch_tmap(&x_map);
+    if (!p.x_tiles) prefetch_tmap(&maps.m[0]);
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&peer[s], 1);
@@ -178,6 +210,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
+#define GW_UNITS (TABLE ? n_tiles * p.n_pairs : p.units)
+  // (the table does not come from the kernel in front, but from one before it: it has completed)
+  const int n_tiles = TABLE ? min(__ldcg(reinterpret_cast<const int*>(p.tiles)), p.tiles_max) : 0;
+  if (TABLE)
+    for (int i = threadIdx.x; i < n_tiles; i += GW_THREADS) table[i] = __ldcg(p.tiles + 1 + i);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();
@@ -192,8 +229,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
       const uint32_t a_rows_bytes = static_cast<uint32_t>(p.tile_rows) * 128u;
       bool waited = false;
       const uint32_t smem_a = smem_u32(smem), bar_full = smem_u32(full);
-      for (int u = first; u < p.units; u += step) {
-        const GwUnit g = gw_unit(p, u);
+      for (int u = first; u < GW_UNITS; u += step) {
+        const auto g = gw_unit<TABLE>(p, table, n_tiles, u);
         const int w0 = (g.pair * 2 + static_cast<int>(rank)) * p.sub;
         const int n_sub = max(0, min(p.sub, p.n_tiles - w0));
         const size_t w_kbs = p.w_kb_stride ? p.w_kb_stride : p.num_kb;
@@ -203,7 +240,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
         const int xb = p.x_tiles ? row0 / p.x_tile : 0, in0 = row0 - xb * p.x_tile;
         const uint32_t r0 = static_cast<uint32_t>(p.x_tiles ? min(half, p.x_tile - in0) : 0) * 128u;
         const uint32_t r1 = p.x_tiles ? static_cast<uint32_t>(half) * 128u - r0 : 0u;
-        const uint32_t bytes = static_cast<uint32_t>(n_sub) * a_rows_bytes + (p.x_tiles ? r0 + r1 : static_cast<uint32_t>(b_bytes));
+        const uint32_t bytes = static_cast<uint32_t>(n_sub) * a_rows_bytes + (p.x_tiles ? r0 + r1 : static_cast<uint32_t>(TABLE ? gw_box_rows(gw_box(half)) * 128 : b_bytes));
         const size_t x_step = static_cast<size_t>(p.x_tile) * 128;
         // a single thread feeds the ring: what it does per stage is kept to a handful of additions
         const uint8_t* wsrc = p.w_tiles + static_cast<size_t>(w0) * sub_stride + static_cast<size_t>(p.kb_base + g.kb0) * a_rows_bytes;
@@ -229,7 +266,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
               xsrc += x_step;
               xsrc1 += x_step;
             } else {
-              gw_tma_2d(dst, &x_map, bar, kx, row0);
+              gw_tma_2d(dst, &maps.m[TABLE ? gw_box(half) : 0], bar, kx, row0);
               kx += GW_BLOCK_K;
             }
           }
@@ -245,11 +282,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
               load_a(smem_a + i * stage_bytes, nk, bar_full + 8 * i);
             }
           };
-          if (!p.tile_group) pre_a();
+          if constexpr (TABLE) wsrc += g.group * (p.group_bytes + static_cast<size_t>(p.group_kb) * a_rows_bytes);
+          if (TABLE || !p.tile_group) pre_a();
           pdl_wait();
           wait_gate_open(gate);
           pdl_trigger();
-          if (p.tile_group) {
+          if (!TABLE && p.tile_group) {
             const size_t grp = p.tile_group[g.tblk];
             wsrc += grp * p.group_bytes + grp * p.group_kb * a_rows_bytes;
             pre_a();
@@ -260,6 +298,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
           s = npre == p.stages ? 0 : npre;
           ph = npre == p.stages ? 1u : 0u;
           waited = true;
+        } else if constexpr (TABLE) {
+          wsrc += g.group * (p.group_bytes + static_cast<size_t>(p.group_kb) * a_rows_bytes);
         } else if (p.tile_group) {
           const size_t grp = p.tile_group[g.tblk];
           wsrc += grp * p.group_bytes + grp * p.group_kb * a_rows_bytes;
@@ -292,8 +332,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
       // (the whole warp walks the loop and one elected lane issues: the operands stay in uniform registers; with a loop under
       // `if (lane == 0)` moving them there cost 70 cycles per MMA)
       const uint64_t desc0 = umma_desc_sw128_kmajor(smem_u32(smem));
-      for (int u = first; u < p.units && !bw.dead; u += step, ++it) {
-        const GwUnit g = gw_unit(p, u);
+      for (int u = first; u < GW_UNITS && !bw.dead; u += step, ++it) {
+        const auto g = gw_unit<TABLE>(p, table, n_tiles, u);
         const int acc = it & 1;
         bw.wait(&acc_empty[acc], ((it >> 1) & 1) ^ 1);
         if (!__all_sync(0xffffffffu, !bw.dead)) { bw.dead = true; break; }
@@ -323,8 +363,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
     } else if (lane == 0) {
       // ================= relay: this CTA's half of a stage has landed =================
       const uint32_t peer0 = cluster_addr(peer, 0);
-      for (int u = first; u < p.units && !bw.dead; u += step) {
-        const GwUnit g = gw_unit(p, u);
+      for (int u = first; u < GW_UNITS && !bw.dead; u += step) {
+        const auto g = gw_unit<TABLE>(p, table, n_tiles, u);
         for (int kb = g.kb0; kb < g.kb1; kb += GW_KPS) {
           bw.wait(&full[s], ph);
           if (bw.dead) break;
@@ -341,8 +381,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
     const int sub_i = (quarter * 32) / p.tile_rows;           // which of the CTA's weight tiles this quarter's rows belong to
     const int row_in = row - sub_i * p.tile_rows;
     int it = 0;
-    for (int u = first; u < p.units && !bw.dead; u += step, ++it) {
-      const GwUnit g = gw_unit(p, u);
+    for (int u = first; u < GW_UNITS && !bw.dead; u += step, ++it) {
+      const auto g = gw_unit<TABLE>(p, table, n_tiles, u);
       const int acc = it & 1;
       const int tile = (g.pair * 2 + static_cast<int>(rank)) * p.sub + sub_i;
       const bool row_ok = sub_i < p.sub && row_in < p.tile_rows && tile < p.n_tiles;
@@ -407,7 +447,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
 #pragma unroll
             for (int i = 0; i < 8; ++i) o[i] = round_bf16(gt[i]) * round_bf16(up[i]);
           }
-          const int lim = live ? p.T - tc : 0;
+          const int lim = live ? gw_end(p, g) - tc : 0;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const int j = 2 * i + (hi ? 1 : 0);
@@ -425,7 +465,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
             tmem_ld_32x16(taddr + c0, v);
             tmem_ld_wait();
             if (live) {
-              const int t = g.t0 + c0, m = min(16, p.T - t);
+              const int t = g.t0 + c0, m = min(16, gw_end(p, g) - t);
 #pragma unroll
               for (int j = 0; j < 16; ++j)
                 if (j < m) y[static_cast<size_t>(t + j) * p.ldy] = __uint_as_float(v[j]);
@@ -452,7 +492,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
               for (int j = 0; j < 16; ++j) a[j] = gw_act(a[j], 3);
             }
             if (live) {
-              const int t = g.t0 + c0, m = min(16, p.T - t);
+              const int t = g.t0 + c0, m = min(16, gw_end(p, g) - t);
 #pragma unroll
               for (int j = 0; j < 16; ++j)
                 if (j < m) y[static_cast<size_t>(t + j) * p.ldy] = __float2bfloat16_rn(a[j]);
@@ -475,6 +515,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
   }
 }
 
+#undef GW_UNITS
 static int gw_pairs() {
   static int pairs = 0;
   if (!pairs) {
@@ -495,11 +536,11 @@ int vb_gemm_wide_timeouts(void) {
   return wait_ran_out(WK_GEMM_WIDE);
 }
 
-int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
+static int gw_launch(void* d_y, const void* d_w_tiles, const void* const* x_maps, const void* d_x_tiles, int T, int N, int K, int ldy,
                       int mode, int split_k, int tile_rows, int n_out, int y_tiled, const void* d_bias, int act, int n_tok,
-                      const int32_t* d_tile_group, long long group_bytes, int w_kb_stride, int group_kb, int kb_base,
+                      const int32_t* d_tile_group, const int32_t* d_tiles, int tiles_max, long long group_bytes, int w_kb_stride, int group_kb, int kb_base,
                       float glu_limit, float glu_slope, void* stream) {
-  VB_CHECK_ARG(d_y && d_w_tiles && (x_map || d_x_tiles), "vb_gemm_bf16_wide: null pointer");
+  VB_CHECK_ARG(d_y && d_w_tiles && (x_maps || d_x_tiles), "vb_gemm_bf16_wide: null pointer");
   VB_CHECK_ARG(T > 0 && N > 0 && K > 0 && K % 8 == 0, "vb_gemm_bf16_wide: T=%d N=%d K=%d (K a multiple of 8)", T, N, K);
   VB_CHECK_ARG(mode >= 0 && mode <= 2, "vb_gemm_bf16_wide: mode %d", mode);
   VB_CHECK_ARG(mode == 1 || split_k == 1, "vb_gemm_bf16_wide: split_k > 1 needs mode 1 (fp32 partials)");
@@ -510,16 +551,18 @@ int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_ma
   VB_CHECK_ARG(mode != 2 || N % tile_rows == 0, "vb_gemm_bf16_wide: mode 2 needs N %% tile_rows == 0");
   VB_CHECK_ARG(n_tok >= 16 && n_tok <= 256 && n_tok % 16 == 0, "vb_gemm_bf16_wide: n_tok %d outside [16, 256] or not a multiple of 16", n_tok);
   VB_CHECK_ARG(group_bytes >= 0 && w_kb_stride >= 0 && group_kb >= 0 && kb_base >= 0, "vb_gemm_bf16_wide: offsets");
-  VB_CHECK_ARG(!d_tile_group || x_map, "vb_gemm_bf16_wide: groups need row-major activations");
+  VB_CHECK_ARG(!(d_tile_group || d_tiles) || x_maps, "vb_gemm_bf16_wide: groups need row-major activations");
   VB_CHECK_ARG(glu_limit >= 0.f && (glu_limit == 0.f || (mode == 2 && act == 0)), "vb_gemm_bf16_wide: a positive limit belongs to mode 2 without an activation");
-  static const CUtensorMap dummy_map = {};
+  VB_CHECK_ARG(!d_tiles || (tiles_max > 0 && tiles_max <= 4096 && reinterpret_cast<uintptr_t>(d_tiles) % 16 == 0 && split_k == 1 && !d_x_tiles && !d_tile_group && n_tok == 256),
+               "vb_gemm_bf16_wide: a table of tiles stands alone, on a 16-byte boundary, with up to 4096 of them");
   GemmWideParams p = {};
   VB_CHECK_ARG(p.wait_flag = wait_flag(WK_GEMM_WIDE), "vb_gemm_bf16_wide: no mapped host memory");
   p.num_kb = (K + GW_BLOCK_K - 1) / GW_BLOCK_K;
   VB_CHECK_ARG(split_k >= 1 && split_k <= p.num_kb, "vb_gemm_bf16_wide: split_k %d outside [1, %d]", split_k, p.num_kb);
   p.y = d_y; p.w_tiles = static_cast<const uint8_t*>(d_w_tiles); p.x_tiles = static_cast<const uint8_t*>(d_x_tiles);
   p.bias = static_cast<const __nv_bfloat16*>(d_bias);
-  p.tile_group = d_tile_group; p.group_bytes = group_bytes; p.w_kb_stride = w_kb_stride; p.group_kb = group_kb; p.kb_base = kb_base;
+  p.tile_group = d_tile_group; p.tiles = reinterpret_cast<const int4*>(d_tiles); p.tiles_max = tiles_max;
+  p.group_bytes = group_bytes; p.w_kb_stride = w_kb_stride; p.group_kb = group_kb; p.kb_base = kb_base;
   p.T = T; p.N = N; p.K = K; p.ldy = ldy; p.mode = mode; p.split_k = split_k; p.tile_rows = tile_rows; p.sub = 128 / tile_rows;
   p.n_out = n_out > 0 ? n_out : (mode == 2 ? N / 2 : N);
   p.act = act; p.y_tiled = y_tiled; p.x_tile = vb_gemm_t_tile(T); p.n_tok = n_tok;
@@ -530,14 +573,40 @@ int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_ma
   VB_CHECK_ARG(static_cast<long long>(p.n_pairs) * p.t_blocks * split_k <= 0x3fffffffLL, "vb_gemm_bf16_wide: too many tiles");
   p.units = p.n_pairs * p.t_blocks * split_k;
   const int stage_bytes = GW_KPS * (GW_A_BYTES + n_tok * 64);
-  const int tail = 1024 /*barriers*/ + 1024 /*alignment*/;
+  const int tail = 1024 /*barriers*/ + 1024 /*alignment*/ + tiles_max * 16;
   p.stages = min(GW_MAX_STAGES, (VB_MAX_DYN_SMEM - tail) / stage_bytes);
   const int smem = p.stages * stage_bytes + tail;
-  VB_CHECK_CUDA(max_dyn_smem_once(gemm_wide_kernel));
-  const int pairs = min(p.units, gw_pairs());
-  VB_CHECK_CUDA(launch_kernel(gemm_wide_kernel, dim3(2 * pairs), dim3(GW_THREADS), smem, static_cast<cudaStream_t>(stream), true, p,
-                              x_map ? *static_cast<const CUtensorMap*>(x_map) : dummy_map));
+  if (d_tiles) {
+    const int pairs = static_cast<int>(min(static_cast<long long>(p.n_pairs) * tiles_max, static_cast<long long>(gw_pairs())));
+    GwMaps<true> maps;
+    for (int i = 0; i < GW_BOXES; ++i) {
+      VB_CHECK_ARG(x_maps[i], "vb_gemm_bf16_wide: null pointer");
+      maps.m[i] = *static_cast<const CUtensorMap*>(x_maps[i]);
+    }
+    VB_CHECK_CUDA(max_dyn_smem_once(gemm_wide_kernel<true>));
+    VB_CHECK_CUDA(launch_kernel(gemm_wide_kernel<true>, dim3(2 * pairs), dim3(GW_THREADS), smem, static_cast<cudaStream_t>(stream), true, p, maps));
+    return 0;
+  }
+  static const GwMaps<false> none = {};
+  VB_CHECK_CUDA(max_dyn_smem_once(gemm_wide_kernel<false>));
+  VB_CHECK_CUDA(launch_kernel(gemm_wide_kernel<false>, dim3(2 * min(p.units, gw_pairs())), dim3(GW_THREADS), smem, static_cast<cudaStream_t>(stream), true, p,
+                              x_maps ? *static_cast<const GwMaps<false>*>(x_maps[0]) : none));
   return 0;
+}
+
+int vb_gemm_bf16_wide_grouped(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,
+                      int mode, int split_k, int tile_rows, int n_out, int y_tiled, const void* d_bias, int act, int n_tok,
+                      const int32_t* d_tile_group, long long group_bytes, int w_kb_stride, int group_kb, int kb_base,
+                      float glu_limit, float glu_slope, void* stream) {
+  return gw_launch(d_y, d_w_tiles, x_map ? &x_map : nullptr, d_x_tiles, T, N, K, ldy, mode, split_k, tile_rows, n_out, y_tiled, d_bias, act, n_tok, d_tile_group,
+                   nullptr, 0, group_bytes, w_kb_stride, group_kb, kb_base, glu_limit, glu_slope, stream);
+}
+
+int vb_gemm_bf16_wide_tiles(void* d_y, const void* d_w_tiles, const void* const* x_maps, int T, int N, int K, int ldy, int mode, int tile_rows, int n_out, int act,
+                            const int32_t* d_tiles, int tiles_max, long long group_bytes, int w_kb_stride, int group_kb, float glu_limit, float glu_slope, void* stream) {
+  VB_CHECK_ARG(d_tiles && x_maps, "vb_gemm_bf16_wide_tiles: null pointer");
+  return gw_launch(d_y, d_w_tiles, x_maps, nullptr, T, N, K, ldy, mode, 1, tile_rows, n_out, 0, nullptr, act, 256, nullptr, d_tiles, tiles_max, group_bytes, w_kb_stride,
+                   group_kb, 0, glu_limit, glu_slope, stream);
 }
 
 int vb_gemm_bf16_wide(void* d_y, const void* d_w_tiles, const void* x_map, const void* d_x_tiles, int T, int N, int K, int ldy,

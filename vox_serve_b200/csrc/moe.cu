@@ -11,6 +11,7 @@
 //                   shared expert's per-token gate sigmoid(w_sg . h) when asked
 //   vb_moe_group    counting sort (shared-memory counters, one CTA) of the (token, choice) pairs by expert: row_off[E + 1], the token of every sorted row and
 //                   the sorted row of every (token, choice)
+//   vb_moe_group_tiles  the same with a table of token tiles for vb_gemm_bf16_wide_tiles, the shared expert among them
 //   vb_moe_scale_dense  the dense form for tensor-core projections: every expert runs on every token as ONE stacked
 //                   gate/up projection [E * ff (+ shared ff)] and ONE stacked down projection over that whole axis; in
 //                   between, the activation columns of expert e are multiplied by the token's routing weight for e, or
@@ -294,6 +295,74 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(int32_t* __restrict__ r
   }
 }
 
+// The same for token tiles of any height (vb_gemm_bf16_wide_tiles): the shared expert's rows in front (every token once, group E), then the pairs by expert,
+// every expert's rows from a multiple of 16 on and cut into even tiles.  One height for the launch: pairs of SMs work through (tile, 256 weight rows) in
+// waves, and a tile's time hardly depends on its rows (0.52 us a stage of 128 k up to 128 of them, 0.0008 more for each further one, 2.5 beside), so the
+// height that fills the waves of both projections best.  8 experts, 2002 pairs and 1001 shared rows of 2048 x 2048: 118 units on 74 pairs, where tiles
+// of 128 rows took 192, empty ones among them, and the shared expert 56 in a launch of its own (an up or down projection with it 46 us, now 35; a step of
+// three such layers 815 -> 747).
+struct MoeTilesParams {
+  int32_t *sorted_token, *pair_row;
+  const int32_t* idx;
+  int4* tiles;               // [0].x: how many
+  int T, E, top, shared, rows_max, tiles_max;
+  int units[2], kb[2], pairs;      // of the two projections: pairs of weight tiles, blocks of 64 k
+};
+__global__ void __launch_bounds__(1024) moe_group_tiles_kernel(const MoeTilesParams p) {
+  __shared__ int cnt[1025], base[1026], first[1026], best_height;
+  __shared__ float cost[16];
+  pdl_sync();
+  const int tid = threadIdx.x, lane = tid & 31, n = p.T * p.top, groups = p.E + (p.shared ? 1 : 0);
+  for (int e = tid; e <= p.E; e += 1024) cnt[e] = e == p.E && p.shared ? p.T : 0;
+  __syncthreads();
+  for (int i = tid; i < n; i += 1024) atomicAdd(&cnt[p.idx[i]], 1);
+  for (int r = tid; r < p.rows_max; r += 1024) p.sorted_token[r] = p.shared && r < p.T ? r : -1;
+  __syncthreads();
+  {                          // a warp a height: 256, 240, .. 32
+    const int h = 256 - 16 * (tid >> 5);
+    if (tid < 15 * 32) {
+      int tiles = 0;
+      for (int e = lane; e < groups; e += 32) tiles += (cnt[e] + h - 1) / h;
+      tiles = __reduce_add_sync(0xffffffffu, tiles);
+      const float stage = 0.52f + 0.0008f * max(0, h - 128);
+      float c = 0.f;
+      for (int i = 0; i < 2; ++i)
+        c += static_cast<float>((static_cast<long long>(tiles) * p.units[i] + p.pairs - 1) / p.pairs) * (stage * 0.5f * (p.kb[i] + 1) + 2.5f);
+      if (lane == 0) cost[tid >> 5] = tiles <= p.tiles_max ? c : INFINITY;
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    int at = 0;
+    for (int i = 1; i < 15; ++i)
+      if (cost[i] < cost[at]) at = i;
+    const int h = 256 - 16 * at;
+    int row = 0, tile = 0;
+    for (int g = 0; g < groups; ++g) {           // (the shared expert first)
+      const int e = p.shared ? (g == 0 ? p.E : g - 1) : g;
+      base[e] = row;
+      first[e] = tile;
+      row += (cnt[e] + 15) / 16 * 16;
+      tile += (cnt[e] + h - 1) / h;
+    }
+    best_height = h;
+    p.tiles[0] = make_int4(tile, h, 0, 0);
+  }
+  __syncthreads();
+  for (int e = tid; e < groups; e += 1024) {
+    const int c = cnt[e], k = (c + best_height - 1) / best_height, rows = k ? ((c + k - 1) / k + 15) / 16 * 16 : 0;
+    for (int i = 0; i < k; ++i) p.tiles[1 + first[e] + i] = make_int4(e, base[e] + i * rows, max(0, min(rows, c - i * rows)), 0);
+  }
+  __syncthreads();
+  for (int e = tid; e < p.E; e += 1024) cnt[e] = 0;
+  __syncthreads();
+  for (int i = tid; i < n; i += 1024) {          // (the order of an expert's rows varies from run to run, as above)
+    const int e = p.idx[i], r = base[e] + atomicAdd(&cnt[e], 1);
+    p.sorted_token[r] = i / p.top;
+    p.pair_row[i] = r;
+  }
+}
+
 __global__ void moe_combine_kernel(float* __restrict__ y, const float* __restrict__ expert_out,
                                    const float* __restrict__ shared_out, const float* __restrict__ wts,
                                    const int32_t* __restrict__ pair_row, int W, int top,
@@ -462,6 +531,23 @@ int vb_moe_group(int32_t* d_row_off, int32_t* d_sorted_token, int32_t* d_pair_ro
   if (T <= 0) return 0;
   VB_LAUNCH_PDL(moe_group_kernel, 1, 1024, 0, stream, d_row_off, d_sorted_token, d_pair_row, d_idx, T, experts, top,
                 tile_rows, d_tile_group, n_tiles);
+  return 0;
+}
+
+int vb_moe_group_tiles(int32_t* d_sorted_token, int32_t* d_pair_row, int32_t* d_tiles, const int32_t* d_idx, int T, int experts, int top, int shared, int rows_max,
+                       int tiles_max, int n_a, int k_a, int n_b, int k_b, void* stream) {
+  VB_CHECK_ARG(d_sorted_token && d_pair_row && d_tiles && d_idx, "vb_moe_group_tiles: null pointer");
+  VB_CHECK_ARG(experts >= 1 && experts <= 1024 && top >= 1, "vb_moe_group_tiles: experts %d (<= 1024), top %d", experts, top);
+  VB_CHECK_ARG(n_a > 0 && k_a > 0 && n_b > 0 && k_b > 0 && reinterpret_cast<uintptr_t>(d_tiles) % 16 == 0, "vb_moe_group_tiles: projections, table on a 16-byte boundary");
+  if (T <= 0) return 0;
+  const long long pairs = static_cast<long long>(T) * top, shared_rows = shared ? (T + 15LL) / 16 * 16 : 0;
+  VB_CHECK_ARG(rows_max >= shared_rows + pairs + 15LL * experts && tiles_max >= (pairs + 255) / 256 + experts + (shared ? (T + 255) / 256 : 0),
+               "vb_moe_group_tiles: %d rows and %d tiles do not hold %lld pairs", rows_max, tiles_max, pairs);
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+  const MoeTilesParams p{d_sorted_token, d_pair_row, d_idx, reinterpret_cast<int4*>(d_tiles), T, experts, top, shared ? 1 : 0, rows_max, tiles_max,
+                         {(n_a + 255) / 256, (n_b + 255) / 256}, {(k_a + 63) / 64, (k_b + 63) / 64}, max(1, sms / 2)};
+  VB_LAUNCH_PDL(moe_group_tiles_kernel, 1, 1024, 0, stream, p);
   return 0;
 }
 

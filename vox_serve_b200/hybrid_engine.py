@@ -1199,7 +1199,9 @@ class HybridEngine:
             top, E = max(f.top for f in moe), max(f.experts for f in moe)
             # grouped tensor-core form: row tiles of GROUP_TILE rows, every expert's rows padded to whole tiles
             self.moe_tiles = (R * top + self.GROUP_TILE - 1) // self.GROUP_TILE + E
-            rmax = self.moe_tiles * self.GROUP_TILE
+            # tables of token tiles (vb_moe_group_tiles): the pairs beside every token for the shared expert, experts at multiples of 16 rows
+            rmax = max(self.moe_tiles * self.GROUP_TILE, (R + 15) // 16 * 16 + R * top + 16 * E)
+            self.moe_table = torch.zeros(1 + (R * top + 255) // 256 + (R + 255) // 256 + E + 64, 4, dtype=I32, device=dev)
             self.moe_tile_group = torch.zeros(self.moe_tiles, dtype=I32, device=dev)
             self.moe_xs = torch.zeros(rmax * W if weights.tensor_core else 8, dtype=CT, device=dev)
             self.moe_idx = torch.zeros(R * top, dtype=I32, device=dev)
@@ -1361,6 +1363,8 @@ class HybridEngine:
             ops.moe_route_table(s.ids, w["table"], f.experts, idx, wts, h, sg, sgate)
         else:
             ops.moe_route_sigmoid(h, w["router"], w.get("correction"), f.top, idx, wts, f.groups, f.groups_keep, sg, sgate)
+        if self._by_tiles(w, "up_all", T):
+            return self._moe_by_tiles(f, w, T, idx, wts, h, out, "up_all", sgate)
         if "grouped" in w and T >= self.GROUPED_MIN_ROWS:
             g, tt = w["grouped"], self.GROUP_TILE
             n_tiles = (T * f.top + tt - 1) // tt + f.experts
@@ -1399,6 +1403,37 @@ class HybridEngine:
             shared = self._proj(sa, w["s_down"], self.s_out[:T])
         return ops.moe_combine(eo, shared, wts, self.moe_pair_row, f.top, out, shared_scale=sgate)
 
+    def _by_tiles(self, w: Dict[str, Any], up: str, T: int) -> bool:
+        return ("grouped" in w and T >= self.GROUPED_MIN_ROWS and w[up].tile_rows in ops.WIDE_TILE_ROWS and w["down_all"].tile_rows in ops.WIDE_TILE_ROWS
+                and self.moe_table.shape[0] <= 4097)
+
+    def _moe_by_tiles(self, f: MoEConfig, w: Dict[str, Any], T: int, idx: torch.Tensor, wts: torch.Tensor, h: torch.Tensor, out: torch.Tensor, up: str,
+                      sgate: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """Compute-bound steps: tokens sorted by expert, cut into tiles whose height fills the waves of pairs of SMs, each multiplied by its expert's
+        slice of the packed buffers that the dense form uses; a shared expert as wide as the others is one more of them, with every token."""
+        g, W, gated = w["grouped"], self.cfg.width, up == "gu_all"
+        glu, n_up = ((f.limit, f.slope) if f.act == "clamped_glu" else None), (2 * f.ff if gated else f.ff)
+        merged = bool(f.shared_ff) and f.shared_ff == f.ff
+        rows = ((T + 15) // 16 * 16 if merged else 0) + T * f.top + 16 * f.experts
+        token = self.moe_sorted[:rows]
+        ops.moe_group_tiles(idx, T, f.experts, f.top, merged, token, self.moe_pair_row, self.moe_table, ((n_up, W), (W, f.ff)))
+        xs = ops.moe_gather_rows(h, token, self.moe_xs[:rows * W].view(rows, W))
+        act, eo = self.moe_act[:rows * f.ff].view(rows, f.ff), self.moe_out[:rows * W].view(rows, W)
+        ops.gemm_tiles(xs, w[up], act, 2 if gated else 0, n_up, W, self.moe_table, group_bytes=g["group_bytes"], act=None if gated else f.act, glu=glu)
+        ops.gemm_tiles(act, w["down_all"], eo, 1, W, f.ff, self.moe_table, w_kb_stride=g["kb_total"], group_kb=g["group_kb"])
+        shared = eo[:T] if merged else None
+        if f.shared_ff and not merged:
+            sa = self.s_act[:T * f.shared_ff].view(T, f.shared_ff)
+            if glu:
+                ops.gemm_glu(h, w["s_gu_view"], sa, *glu)
+            elif gated:
+                ops.gemm(h, w["s_gu_view"], mode=2, out=sa, tile_rows=w["s_gu_view"].tile_rows, n_out=f.shared_ff)
+            else:
+                ops.gemm(h, w["s_up_view"], mode=0, out=sa, tile_rows=w["s_up_view"].tile_rows, act=f.act)
+            shared = ops.gemm_grouped(sa, w["down_all"], self.s_out[:T], 1, W, f.shared_ff, ops.gemm_t_tile(T), None, w_kb_stride=g["kb_total"],
+                                      kb_base=f.experts * g["group_kb"])
+        return ops.moe_combine(eo, shared, wts, self.moe_pair_row, f.top, out, shared_scale=sgate)
+
     def _moe(self, f: MoEConfig, w: Dict[str, Any], s: StepInputs, h: Optional[torch.Tensor] = None,
              out: Optional[torch.Tensor] = None) -> torch.Tensor:
         T, W = s.T, self.cfg.width
@@ -1411,10 +1446,11 @@ class HybridEngine:
             ops.moe_route_groups(h, w["router"], f.top, idx, wts, f.groups, f.groups_keep, scores="softmax", group_rank="max")
         else:
             ops.moe_route(h, w["router"], w["router_b"], f.top, idx, wts)
+        if self._by_tiles(w, "gu_all", T):
+            return self._moe_by_tiles(f, w, T, idx, wts, h, out, "gu_all")
         glu = (f.limit, f.slope) if f.act == "clamped_glu" else None
         if "grouped" in w and T >= self.GROUPED_MIN_ROWS:
-            # compute-bound steps: tokens sorted by expert into whole row tiles, each tile multiplied by its expert's slice of
-            # the same packed buffers the dense form uses (tcgen05, gemm.cu), the shared expert as two plain projections
+            # weight tiles that the kernel of many rows does not take: whole row tiles of GROUP_TILE rows an expert, the shared expert as two plain projections
             g, tt = w["grouped"], self.GROUP_TILE
             n_tiles = (T * f.top + tt - 1) // tt + f.experts
             rows = n_tiles * tt

@@ -1568,6 +1568,32 @@ def gemm_grouped(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, mode: in
     return out
 
 
+def moe_group_tiles(idx: torch.Tensor, T: int, experts: int, top: int, shared: bool, sorted_token: torch.Tensor, pair_row: torch.Tensor, tiles: torch.Tensor,
+                    shapes) -> None:
+    """Pairs by expert beside the shared expert's rows (every token, in front), and the table of token tiles that ``gemm_tiles`` works through;
+    ``shapes``: (N, K) of the two projections."""
+    (na, ka), (nb, kb) = shapes
+    call("vb_moe_group_tiles", sorted_token.data_ptr(), pair_row.data_ptr(), tiles.data_ptr(), idx.data_ptr(), T, experts, top, int(shared), sorted_token.numel(),
+         tiles.shape[0] - 1, na, ka, nb, kb, _stream())
+
+
+def gemm_tiles(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, mode: int, N: int, K: int, tiles: torch.Tensor, group_bytes: int = 0, w_kb_stride: int = 0,
+               group_kb: int = 0, act: Optional[str] = None, glu: Optional[Tuple[float, float]] = None) -> torch.Tensor:
+    """``gemm_grouped`` (with ``glu``: ``gemm_grouped_glu``) over the token tiles of a table on the device (``moe_group_tiles``; a kernel must stand between)"""
+    _need_cuda(x, out)
+    assert x.dtype == BF16 and x.dim() == 2 and x.shape[1] == K and out.is_contiguous() and w.tile_rows in WIDE_TILE_ROWS
+    if act is not None and mode != 0:
+        raise VoxB200Error(f"gemm_tiles: activation {act!r} is a mode 0 option")
+    if glu is not None:
+        _positive_limit(glu[0])
+    n_out = N // 2 if mode == 2 else N
+    maps = [tensor_map_2d(x, rows) for rows in (64, 80, 96, 128)]
+    call("vb_gemm_bf16_wide_tiles", out.data_ptr(), w.data.data_ptr(), (ctypes.c_void_p * 4)(*(m.ptr for m in maps)), x.shape[0], N, K, n_out, mode, w.tile_rows, n_out,
+         GEMM_ACTS[act], tiles.data_ptr(), tiles.shape[0] - 1, int(group_bytes), int(w_kb_stride), int(group_kb), *map(float, glu or (0.0, 0.0)),
+         _stream())
+    return out
+
+
 def moe_combine(expert_out: torch.Tensor, shared_out: Optional[torch.Tensor], wts: torch.Tensor, pair_row: torch.Tensor,
                 top: int, out: torch.Tensor, shared_scale: Optional[torch.Tensor] = None) -> torch.Tensor:
     """shared_scale fp32 [T]: the shared expert's output is multiplied by it per token."""

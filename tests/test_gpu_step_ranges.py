@@ -203,6 +203,39 @@ def test_projection_of_tile_tables(ops, T, E, top, shared, N, K, skew, mode, til
     assert ops.check_waits() is None
 
 
+@pytest.mark.parametrize("lens,old", [([64], [0]), ([65], [2]), ([3, 70, 1, 9], [0, 1, 5, 2]), ([8, 8, 8, 100, 2], [0, 0, 3, 7, 0]), ([200], [0])])
+@pytest.mark.parametrize("taps,C,act,residual,shift", [(4, 512, "silu", False, 0), (4, 516, "silu", True, 1), (3, 260, None, True, 0), (2, 4, "silu", False, 0)])
+def test_short_convolution_rows(ops, lens, old, taps, C, act, residual, shift):
+    """Groups of rows inside a request, across its edges, past the end; taps on and off 16-byte boundaries; activations whose quotients leave the short way."""
+    g = torch.Generator(device="cuda").manual_seed(sum(lens) + taps)
+    rnd = lambda *n: torch.randn(*n, generator=g, device="cuda")          # noqa: E731
+    T, B, K = sum(lens), len(lens), taps - 1
+    x, w, b, ib = rnd(T, C), rnd(C * taps + shift)[shift:].view(C, taps), rnd(C), rnd(C)
+    x[T // 2, :4] = torch.tensor([300.0, -300.0, 1e30, -1e-30], device="cuda")
+    state = rnd(B, K, C)
+    was, qo = state.clone(), [0]
+    for n in lens:
+        qo.append(qo[-1] + n)
+    req = [i for i, n in enumerate(lens) for _ in range(n)]
+    pos = [o + r for n, o in zip(lens, old) for r in range(n)]
+    out = torch.empty(T, C, device="cuda")
+    ops.short_conv(x, w, b, state, _i32(qo), _i32(req), _i32(pos), _i32(list(range(B))), B, out_f32=out, act=act, residual=residual, in_bias=ib)
+    u = x.double() + ib.double()
+    for i, n in enumerate(lens):
+        at = slice(qo[i], qo[i + 1])
+        front = was[i].double().clone()
+        front[:max(0, K - old[i])] = 0                      # positions before the first
+        full = torch.cat((front, u[at]))
+        y = sum(full[j:j + n] * w[:, j].double() for j in range(taps)) + b.double()
+        size = sum(full[j:j + n].abs() * w[:, j].double().abs() for j in range(taps)) + b.double().abs()
+        # the sum to 2^-22 of its terms; the activation's slope is below 1.1, its exponential and quotient good to a few units
+        want, slack = (y * torch.sigmoid(y), 1.1) if act else (y, 1.0)
+        if residual:
+            want, size = want + u[at], size + u[at].abs()
+        assert bool(((out[at].double() - want).abs() <= slack * 1e-6 * size + 1e-37).all())
+        assert torch.equal(state[i], torch.cat((front, u[at]))[-K:].float() if n >= K else torch.cat((front.float(), (x + ib)[at]))[-K:])
+
+
 @pytest.mark.parametrize("B,T,C,N,ksize,dil,lo,hi,epi,act", [
     (1, 1, 32, 32, 1, 1, 0, 1, "plain", None), (7, 16, 64, 96, 1, 1, 0, 16, "resid", "snake"), (2, 128, 32, 128, 3, 1, 0, 128, "plain", "elu"),
     (3, 129, 96, 160, 1, 1, 5, 129, "noise", None), (1, 300, 64, 64, 7, 9, 130, 299, "scale_resid", "gelu"), (40, 3, 128, 512, 2, 1, 0, 3, "resid", None)])

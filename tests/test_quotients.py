@@ -1,4 +1,4 @@
-"""The quotient of the gate/up epilogue (csrc/gemm_wide.cu, gw_div8) restated with exactly rounded single-precision steps."""
+"""The quotient of the gate/up epilogue (csrc/quotient.cuh, div8) restated with exactly rounded single-precision steps."""
 from fractions import Fraction
 
 import numpy as np

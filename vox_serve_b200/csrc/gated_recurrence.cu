@@ -25,7 +25,7 @@
 //                    (a, sqrt(1 - a^2) i u) per channel, which a walk in order or the piecewise scan above turns into rows.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 1
-#include "common.cuh"
+#include "quotient.cuh"
 
 namespace vb {
 
@@ -303,10 +303,12 @@ __global__ void __launch_bounds__(256) rglru_gates_kernel(RgLruParams p) {
 // bf16 matrices, blocks of a multiple of 16 channels: CTA = 64 rows x 32 channels of one block (64 gate columns: r, then i), 4
 // warps x 16 rows, mma.sync m16n8k16 with fp32 accumulators over chunks of 64 inputs; u enters as two bf16 terms (its rounding
 // and the remainder's).  The next chunk's loads are in flight while a chunk is multiplied.
+// Bound by instructions, most of them the epilogue's exponentials and roots: four blocks an SM (128 registers) 40 -> 35 us for 1001 rows of 2048; five
+// spill and are slower again.
 constexpr int RM_R = 64, RM_CH = 32, RM_K = 64, RM_LD = RM_K + 8;
 
 template <typename CT>
-__global__ void __launch_bounds__(128) rglru_gates_mma_kernel(RgLruParams p) {
+__global__ void __launch_bounds__(128, 4) rglru_gates_mma_kernel(RgLruParams p) {
   __shared__ __align__(16) __nv_bfloat16 Uh[RM_R * RM_LD], Ul[RM_R * RM_LD], Ws[2 * RM_CH * RM_LD];
   const int per = (p.bs + RM_CH - 1) / RM_CH, blk = blockIdx.x / per, c0 = (blockIdx.x - blk * per) * RM_CH;
   const int t0 = blockIdx.y * RM_R, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -415,15 +417,25 @@ __global__ void __launch_bounds__(128) rglru_gates_mma_kernel(RgLruParams p) {
         y[n][e] = ok && single ? yr[n * 8 + e] + (p.y_bias ? p.y_bias[gc + n * 8 + e] : 0.f) : 0.f;
       }
     }
+    // (the sigmoids of eight channels go through their steps together)
+    float gr[8], gi[8], dr[8], di[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      gr[i] = gi[i] = 1.f;
+      dr[i] = 1.f + expf(-(acc[i >> 1][2 * half + (i & 1)] + br[i >> 1][i & 1]));
+      di[i] = 1.f + expf(-(acc[(i >> 1) + 4][2 * half + (i & 1)] + bi[i >> 1][i & 1]));
+    }
+    div8(gr, dr);
+    div8(gi, di);
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
       if (lc + n * 8 >= p.bs) continue;
       float a[2], v[2];
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const float la = -rate[n][e] * mg_sigmoid(acc[n][2 * half + e] + br[n][e]);
+        const float la = -rate[n][e] * gr[2 * n + e];
         a[e] = expf(la);
-        v[e] = sqrtf(-expm1f(2.f * la)) * mg_sigmoid(acc[n + 4][2 * half + e] + bi[n][e]) * (e ? u[n].y : u[n].x);
+        v[e] = sqrtf(-expm1f(2.f * la)) * gi[2 * n + e] * (e ? u[n].y : u[n].x);
       }
       if (single) {
 #pragma unroll

@@ -23,7 +23,7 @@
 // Every wait is bounded (BoundedWait): a CTA whose wait runs out sets its flag, stops issuing and leaves.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 2
-#include "common.cuh"
+#include "quotient.cuh"
 #include <type_traits>
 
 namespace vb {
@@ -92,35 +92,6 @@ __device__ __forceinline__ float gw_act(float v, int act) {
   if (act == 2) return 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
   if (act == 3) return 0.5f * v * (1.f + tanhf(0.79788456080286536f * (v + 0.044715f * v * v * v)));
   return v;
-}
-
-// a / d to the nearest, eight at a time and d >= 1: reciprocal, one Newton step, quotient, one correction by the exact remainder (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34, 1990).  The corrected quotient is right
-// where the reciprocal is.  From an estimate within two units of the last place one step leaves it wrong for a few dozen of the 2^23
-// mantissas, and of those three of the largest have dividends that it spoils (tests/test_quotients.py walks them).  These mantissas, and
-// dividends, divisors or quotients so large or small that a remainder would leave the normal range, send all eight to the division
-// itself; there is no branch between the eight.  Zeros are right as they are, and a NaN stays one on either way.
-__device__ __forceinline__ void gw_div8(float (&a)[8], const float (&d)[8]) {
-  float q[8], large = 0.f, small = 1.f;
-  uint32_t mantissa = 0u;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d[i]));
-    y = fmaf(fmaf(-d[i], y, 1.f), y, y);
-    const float q0 = a[i] * y;
-    const bool zero = a[i] == 0.f;
-    q[i] = zero ? q0 : fmaf(fmaf(-q0, d[i], a[i]), y, q0);
-    large = fmaxf(large, fmaxf(fabsf(a[i]), d[i]));
-    small = fminf(small, zero ? 1.f : fabsf(q0));
-    mantissa = max(mantissa, __float_as_uint(d[i]) | 0xff800000u);
-  }
-  if (!(large < 0x1p100f && small > 0x1p-100f) || mantissa >= 0xfffffffbu) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = a[i] / d[i];
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) a[i] = q[i];
 }
 
 // boxes of half a token tile, by its rows: a table's tiles differ, and what a box has beyond its tile is copied for nothing
@@ -425,7 +396,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
               up[i] = fminf(fmaxf(up[i], -p.glu_limit), p.glu_limit);
               o[i] = 1.0f + expf(-p.glu_slope * gt[i]);
             }
-            gw_div8(gt, o);
+            div8(gt, o);
 #pragma unroll
             for (int i = 0; i < 8; ++i) o[i] = gt[i] * (up[i] + 1.0f);
           } else if (p.act == 1) {
@@ -443,7 +414,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
               gt[i] = round_bf16(gt[i]);
               o[i] = 1.0f + expf(-gt[i]);
             }
-            gw_div8(gt, o);
+            div8(gt, o);
 #pragma unroll
             for (int i = 0; i < 8; ++i) o[i] = round_bf16(gt[i]) * round_bf16(up[i]);
           }

@@ -15,7 +15,7 @@
 //   vb_group_rmsnorm rows of channels in equal neighbourhoods, each divided by its own root mean square, times a weight.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 1
-#include "common.cuh"
+#include "quotient.cuh"
 
 namespace vb {
 
@@ -451,12 +451,26 @@ __global__ void __launch_bounds__(256) ssd_tile_out_kernel(SsdParams p) {
 // rows [0, L) x n columns of bf16 (16-byte pieces) into smem [64][ld], zeros below
 __device__ __forceinline__ void sd_stage(__nv_bfloat16* __restrict__ dst, int ld, const __nv_bfloat16* __restrict__ src, int ld_src, int n,
                                          int L) {
-  const int v = n / 8;
-  for (int i = threadIdx.x; i < SD_ROWS * v; i += 128) {
-    const int r = i / v, c = (i - r * v) * 8;
-    uint4 q = make_uint4(0u, 0u, 0u, 0u);
-    if (r < L) q = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * ld_src + c);
-    *reinterpret_cast<uint4*>(dst + r * ld + c) = q;
+  const int v = n / 8, whole = 128 / v, r0 = threadIdx.x / v, c = (threadIdx.x - r0 * v) * 8;          // whole rows in step
+  if (whole == 0) {
+    for (int i = threadIdx.x; i < SD_ROWS * v; i += 128) {
+      const int r = i / v, e = (i - r * v) * 8;
+      *reinterpret_cast<uint4*>(dst + r * ld + e) = r < L ? *reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * ld_src + e) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    return;
+  }
+  if (r0 >= whole) return;
+  for (int rb = r0; rb < SD_ROWS; rb += 4 * whole) {          // four pieces a thread in flight
+    uint4 q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = rb + i * whole;
+      q[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (r < min(L, SD_ROWS)) q[i] = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * ld_src + c);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (rb + i * whole < SD_ROWS) *reinterpret_cast<uint4*>(dst + (rb + i * whole) * ld + c) = q[i];
   }
 }
 
@@ -477,12 +491,19 @@ __global__ void __launch_bounds__(128) ssd_tile_state_mma_kernel(SsdParams p, in
   if (warp < hb) st.load(p, h0 + warp, row0, L);
   // a head's x, up to four pieces a thread, is asked for while the head before is multiplied
   uint4 q[4];
+  int qr[4], qc[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = tid + 128 * k;
+    qr[k] = i / vb;
+    qc[k] = (i - qr[k] * vb) * 8;
+  }
   auto fetch = [&](int h) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int i = tid + 128 * k, r = i / vb, c = (i - r * vb) * 8;
+      const int r = qr[k], c = qc[k];
       q[k] = make_uint4(0u, 0u, 0u, 0u);
-      if (i < SD_ROWS * vb && r < L) q[k] = *reinterpret_cast<const uint4*>(xbc + static_cast<size_t>(r) * p.ld + h * V + e0 + c);
+      if (r < min(L, SD_ROWS)) q[k] = *reinterpret_cast<const uint4*>(xbc + static_cast<size_t>(r) * p.ld + h * V + e0 + c);
     }
   };
   fetch(h0);
@@ -499,8 +520,8 @@ __global__ void __launch_bounds__(128) ssd_tile_state_mma_kernel(SsdParams p, in
     __syncthreads();                      // (the last head's x is consumed)
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int i = tid + 128 * k, r = i / vb, c = (i - r * vb) * 8;
-      if (i >= SD_ROWS * vb) continue;
+      const int r = qr[k], c = qc[k];
+      if (r >= SD_ROWS) continue;
       uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
       if (r < L) {
         const float w = wgt[h - h0][r];
@@ -569,12 +590,12 @@ __global__ void __launch_bounds__(256) ssd_tile_out_mma_kernel(SsdParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // every copy is in flight before anything is waited for: B and C first (the scores need them), then x and the state
   auto copy = [&](__nv_bfloat16* dst, int ld, const __nv_bfloat16* src, int ld_src, int n, int rows, int valid) {
-    const int v = n / 8;
-    for (int i = tid; i < rows * v; i += 256) {
-      const int r = i / v, c = (i - r * v) * 8;
+    const int v = n / 8, whole = 256 / v, r0 = tid / v, c = (tid - r0 * v) * 8;          // whole rows in step: a division a call and not one a piece
+    if (r0 >= whole) return;
+    const __nv_bfloat16* at = src + c;
+    for (int r = r0; r < rows; r += whole)
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + r * ld + c)),
-                   "l"(src + static_cast<size_t>(r < valid ? r : 0) * ld_src + c), "r"(r < valid ? 16u : 0u) : "memory");
-    }
+                   "l"(at + static_cast<size_t>(r < valid ? r : 0) * ld_src), "r"(r < valid ? 16u : 0u) : "memory");
   };
   pdl_sync();
   // what is read last, or by one warp's chain, is asked for first: a load behind the copies waits for them
@@ -582,6 +603,7 @@ __global__ void __launch_bounds__(256) ssd_tile_out_mma_kernel(SsdParams p) {
   SdSteps st;
   if (warp == 0) st.load(p, h, row0, L);
   float2 zs[2][4];
+  const bool pairs = ((p.ld_z | V | e0) & 1) == 0 && reinterpret_cast<uintptr_t>(p.z) % 8 == 0;
 #pragma unroll
   for (int half = 0; half < 2; ++half)
 #pragma unroll
@@ -590,7 +612,7 @@ __global__ void __launch_bounds__(256) ssd_tile_out_mma_kernel(SsdParams p) {
       zs[half][n] = make_float2(0.f, 0.f);
       if (r < L && c < DV) {
         const float* z = p.z + static_cast<size_t>(row0 + r) * p.ld_z + h * V + e0 + c;
-        zs[half][n] = make_float2(z[0], z[1]);
+        zs[half][n] = pairs ? *reinterpret_cast<const float2*>(z) : make_float2(z[0], z[1]);
       }
     }
   const float D = p.D[h];
@@ -692,13 +714,20 @@ __global__ void __launch_bounds__(256) ssd_tile_out_mma_kernel(SsdParams p) {
     if (r >= L) continue;
     const size_t t = row0 + r;
     float* out = p.out + t * p.H * V + h * V + e0;
+    float gate[8], d[8];               // z sigmoid(z) of the row's eight channels: their quotients go through the steps together
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      gate[i] = i & 1 ? zs[half][i >> 1].y : zs[half][i >> 1].x;
+      d[i] = 1.f + expf(-gate[i]);
+    }
+    div8(gate, d);
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
       const int c = v0 + n * 8 + (lane & 3) * 2;
       if (c < DV) {
         const uint32_t x = *reinterpret_cast<const uint32_t*>(Xs + r * ldx + c);
         const float y0 = fmaf(D, bf16_lo(x), o[n][2 * half]), y1 = fmaf(D, bf16_hi(x), o[n][2 * half + 1]);
-        *reinterpret_cast<float2*>(out + c) = make_float2(y0 * sd_silu(zs[half][n].x), y1 * sd_silu(zs[half][n].y));
+        *reinterpret_cast<float2*>(out + c) = make_float2(y0 * gate[2 * n], y1 * gate[2 * n + 1]);
       }
     }
   }

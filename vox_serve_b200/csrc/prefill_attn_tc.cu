@@ -15,7 +15,7 @@
 //    after the output's rounding / a plan of two layers: 1.94e-3 / 89 us with one term and the lag, 1.92e-3 / 101 us with one term and
 //    the exact maximum (most tiles rescale), 1.59e-3 / 102 us with two terms and the lag;
 //  * warp 4 issues the MMAs: the scores of tile j + 1 are multiplied while the softmax works on tile j (two score buffers);
-//  * warps 5 and 6 bring K and V tiles as boxes of a tensor map over the paged cache (pages of a multiple of 8 tokens; cp.async
+//  * warp 5 brings K tiles and warp 6 V tiles as boxes of a tensor map over the paged cache (pages of a multiple of 8 tokens; cp.async
 //    per token row otherwise), the 128-byte-swizzled images that the MMAs read.  V is
 //    the B operand of P V as it lies in memory, [token][dim] (MN-major): nothing is transposed.
 // 98 KB of shared memory and 256 TMEM columns per CTA: two CTAs share an SM and fill each other's waits.
@@ -28,7 +28,9 @@
 // at the end of a launch of cold data, 2 and 2 now).  The 997 rows above: 45 us a layer of cold data, 36 with whole rows.
 // A row's result depends on its own request alone, whatever else is in the step and whichever portion it comes in: the tiles of its keys are
 // walked in order by one block.  (Sharing them between two blocks where a launch leaves room, 26 us, moved its roundings with its neighbours.)
-// What bounds it: the serial chain of a tile (scores -> maximum -> exponentials -> P V, about 1.3 us), some 5 us around it.
+// What bounds it: the serial chain of a tile (scores -> maximum -> exponentials -> P V, 0.95 us whatever the pages; 1.02 in pages of 128 keys and 2.1 in pages
+// of 16 when one lane looked up and fetched K and V box by box), some 5 us around it.  Two softmax threads a row, 32 scores each, change nothing: 0.95
+// us alone, 38.8 us instead of 37.3 for the 997 rows above.
 // Every wait is bounded (BoundedWait): a block whose wait runs out sets its flag, stops issuing and leaves.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 1
@@ -162,15 +164,16 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) paged_prefill_attn_tc_kernel(c
     } else if (warp == 4) {
       ptc_issue<D>(smem, sh, n_tiles, bw);
     } else if (TMA) {
-      if (warp == 5 && lane == 0) {
-        const int pbase = p.kv_indptr[req];
-        ptc_load<D>(smem, sh, rows, kmax, p.box_tokens, bw, [&](int tok, int is_v, uint32_t dst, int dim, uint32_t bar) {
-          const int page = __ldg(&p.kv_indices[pbase + tok / p.page_size]);
-          ptc_tma_5d(dst, &kv_map, bar, dim, hk, tok % p.page_size, is_v, p.slab_base + page);
-        });
-      } else if (warp == 6 && n_tiles > 0) {
-        ptc_clear_unseen<D>(smem, sh, rows, kmax, bw);
-      }
+      const int pbase = p.kv_indptr[req];
+      auto place = [&](int tok) {
+        const int i = tok / p.page_size;
+        return make_int2(__ldg(&p.kv_indices[pbase + i]), tok - i * p.page_size);
+      };
+      auto box = [&](int is_v) {
+        return [&, is_v](int page, int slot, uint32_t dst, int dim, uint32_t bar) { ptc_tma_5d(dst, &kv_map, bar, dim, hk, slot, is_v, p.slab_base + page); };
+      };
+      if (warp == 5) ptc_load_k<D>(smem, sh, rows, kmax, p.box_tokens, bw, place, box(0));
+      else ptc_load_v<D>(smem, sh, rows, kmax, p.box_tokens, bw, place, box(1));
       __syncwarp();
     } else {
       // ================= loaders for pages that do not divide into 8-token groups: one token's K / V row per thread =================

@@ -135,15 +135,17 @@ __global__ void __launch_bounds__(PTC_THREADS, 2) window_attn_tc_kernel(const Wi
     } else if (warp == 4) {
       ptc_issue<D>(smem, sh, n_tiles, bw);
     } else {
-      if (warp == 5 && lane == 0) {
-        const int pbase = p.page_indptr[b], gv = g / p.v_share;
-        ptc_load<D>(smem, sh, rows, kmax, p.box_tokens, bw, [&](int tok, int is_v, uint32_t dst, int dim, uint32_t bar) {
-          const int page = __ldg(&p.page_indices[pbase + tok / p.page_size]);
-          wtc_tma_4d(dst, is_v ? &v_map : &k_map, bar, dim, is_v ? gv : g, tok % p.page_size, page);
-        });
-      } else if (warp == 6) {
-        ptc_clear_unseen<D>(smem, sh, rows, kmax, bw);
-      }
+      const int pbase = p.page_indptr[b], gv = g / p.v_share;
+      auto place = [&](int tok) {
+        const int i = tok / p.page_size;
+        return make_int2(__ldg(&p.page_indices[pbase + i]), tok - i * p.page_size);
+      };
+      if (warp == 5)
+        ptc_load_k<D>(smem, sh, rows, kmax, p.box_tokens, bw, place,
+                      [&](int page, int slot, uint32_t dst, int dim, uint32_t bar) { wtc_tma_4d(dst, &k_map, bar, dim, g, slot, page); });
+      else
+        ptc_load_v<D>(smem, sh, rows, kmax, p.box_tokens, bw, place,
+                      [&](int page, int slot, uint32_t dst, int dim, uint32_t bar) { wtc_tma_4d(dst, &v_map, bar, dim, gv, slot, page); });
       __syncwarp();
     }
   }

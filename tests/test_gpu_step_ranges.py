@@ -605,6 +605,38 @@ def test_channels_last_depthwise_and_last(B, T, C, dil, lo, hi, big):
     _close(last, ref, 5e-6)
 
 
+@pytest.mark.parametrize("C,rows,dil", [(64, 1, 1), (512, 15, 9), (512, 17, 1), (256, 33, 3), (256, 97, 64), (320, 129, 9)])
+@pytest.mark.parametrize("parts", [False, True])
+def test_channels_last_depthwise_tiles(C, rows, dil, parts):
+    """A row's result does not depend on the height of the tile it is computed in (by the batch and the range: 16 to 128 rows), a sine past its reduction among them."""
+    from vox_serve_b200.tokenizer import _cl
+
+    T, g = rows + 5, torch.Generator(device="cuda").manual_seed(rows + C)
+    x, w = torch.randn(80, T, C, generator=g, device="cuda"), torch.randn(7, C, generator=g, device="cuda")
+    x[::3, rows // 2, 5] = 3e5
+    b, *a = (torch.rand(C, generator=g, device="cuda") + 0.5 for _ in range(3))
+    a = [torch.cat((v, 1 / (v + 1e-9))) for v in a]
+
+    def result(x, lo, hi):
+        n = x.numel()
+        y = _cl.depthwise7(_cl.Act(x.reshape(-1).clone(), x.shape[0], T, C), w, b, *a, dil, lo, hi, parts=parts).buf
+        bits = y[:n].view(torch.int32).view(-1, T, C)[:, lo:hi].clone()
+        return torch.cat((bits, y[n:].view(torch.uint8)[:n // 32].view(-1, T, C // 32)[:, lo:hi].int()), 2) if parts else bits
+
+    whole = result(x, 3, 3 + rows)
+    for n in (1, 3, 9, 20, 40):
+        assert torch.equal(result(x[:n], 3, 3 + rows), whole[:n]), n
+    for lo in {3, 3 + rows // 2, 2 + rows}:
+        assert torch.equal(result(x[:2], lo, lo + 1), whole[:2, lo - 3: lo - 2]), lo
+    if not parts:
+        v = x[:4].double().transpose(1, 2)
+        snake = lambda v, a: v + torch.sin((v.float() * a[:C, None]).double()) ** 2 / (a[:C].double()[:, None] + 1e-9)  # noqa: E731
+        v = torch.nn.functional.conv1d(snake(v, a[0]), w.t().double()[:, None], b.double(), dilation=dil, padding=3 * dil, groups=C)
+        ref = snake(v, a[1]).transpose(1, 2)[:, 3:3 + rows]
+        bad = ref.abs() > 1e4                                                    # (the second sine's argument has rounded by more than its period there)
+        _close(torch.where(bad, 0, whole[:4].view(torch.float32)), torch.where(bad, 0, ref), 5e-6)
+
+
 @pytest.mark.parametrize("B,T,C,dil,lo,hi", [(1, 1, 64, 1, 0, 1), (2, 127, 64, 3, 0, 127), (3, 253, 128, 9, 7, 251), (1, 300, 256, 1, 0, 300), (40, 130, 128, 9, 0, 130),
                                              (2, 65, 192, 3, 0, 65), (1, 40, 1024, 1, 0, 40), (2, 1000, 64, 9, 111, 999), (1, 500, 64, 64, 0, 500), (5, 33, 320, 5, 1, 32)])
 @pytest.mark.parametrize("last", [False, True])

@@ -995,19 +995,19 @@ __global__ void __launch_bounds__(256) cl_pack_kernel(uint4* __restrict__ dst, c
 // ------------------------------------------------------------------------------------------
 // depthwise convolution, 7 taps, dilation d, "same" padding; Snake on the input and on the output (optional both)
 // ------------------------------------------------------------------------------------------
-// A block owns 64 channels x DW_T positions: the (activated) input rows with their halo are staged once in shared memory, so
-// every element is read and put through its sine once, in 256-byte rows; a thread finishes four channels of DW_T / 16 rows, whose
+// A block owns 64 channels x up to DW_T positions: the (activated) input rows with their halo are staged once in shared memory, so
+// every element is read and put through its sine once, in 256-byte rows; a thread finishes four channels of every 16th row, whose
 // chains interleave (the activation branches once per four values, to the library's sine when an argument is out of range).
 // DW_T 128 and four-wide activations against 64 and one by one: 12 to 30 us a layer -> 4 to 14 (SNAC, 32 windows).
 constexpr int DW_T = 128;
 __global__ void __launch_bounds__(256) cl_dwconv7_kernel(float* __restrict__ y, uint8_t* __restrict__ code, const float* __restrict__ x, long long x_bstride,
                                                          const float* __restrict__ w, const float* __restrict__ bias,
                                                          const float* __restrict__ alpha_in, const float* __restrict__ alpha_out,
-                                                         int C, int T, int dil, int t_lo, int t_hi) {
+                                                         int C, int T, int dil, int t_lo, int t_hi, int tile_rows) {
   extern __shared__ float4 tile[];          // [rows][16]
   const int c4 = threadIdx.x & 15, r0 = threadIdx.x >> 4;
-  const int c = blockIdx.y * 64 + c4 * 4, b = blockIdx.z, t0 = t_lo + blockIdx.x * DW_T;
-  const int halo = 3 * dil, n_out = min(DW_T, t_hi - t0), rows = n_out + 2 * halo;
+  const int c = blockIdx.y * 64 + c4 * 4, b = blockIdx.z, t0 = t_lo + blockIdx.x * tile_rows;
+  const int halo = 3 * dil, n_out = min(tile_rows, t_hi - t0), rows = n_out + 2 * halo;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   auto ld4 = [&](const float* p) { return p ? __ldg(reinterpret_cast<const float4*>(p + c)) : zero; };
   const float4 ai = ld4(alpha_in), ii = ld4(alpha_in ? alpha_in + C : nullptr), ao = ld4(alpha_out),
@@ -1033,8 +1033,7 @@ __global__ void __launch_bounds__(256) cl_dwconv7_kernel(float* __restrict__ y, 
   __syncthreads();
   const size_t y0 = static_cast<size_t>(b) * T * C + c;
 #pragma unroll 2
-  for (int r = r0; r < DW_T; r += 16) {
-    if (r >= n_out) break;           // (alike for the sixteen lanes of a row)
+  for (int r = r0; r < n_out; r += 16) {          // (alike for the sixteen lanes of a row)
     float4 o = bv;
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
@@ -1380,6 +1379,25 @@ __global__ void __launch_bounds__(256) cl_chunk_attention_kernel(float* __restri
 
 static bool on16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }      // (a null pointer is)
 
+// Rows of a block of the depthwise convolution, by what a launch was measured to take (us): a block alone on its SM 2 and 0.034 a row, each further one on
+// it 0.9 and 0.0155 a row, some more for the halo.  Blocks of 128 rows / of the rows chosen here: 80 x 512 of one window 4.7 / 2.5, 330 x 256 of one 6.4 / 2.5, of 4 6.4 /
+// 3.4, of 16 8.3 / 6.7, of 32 13.1 / 11.9; 1024 x 256 of 16 15.3 / 15.3 (in blocks of 16 29.3).
+static int cl_dw_rows(int range, int channel_blocks, int B, int dil, int sms) {
+  static const int kRows[] = {DW_T, 96, 64, 48, 32, 16};
+  int best = DW_T;
+  double least = 0.0;
+  for (int rows : kRows) {
+    const long long blocks = static_cast<long long>((range + rows - 1) / rows) * channel_blocks * B, on_sm = (blocks + sms - 1) / sms;
+    const int n = min(rows, range);
+    const double cost = 2.0 + 0.034 * n + 0.07 * dil + static_cast<double>(on_sm - 1) * (0.9 + 0.0155 * n + 0.03 * dil);
+    if (rows == DW_T || cost < least) {
+      least = cost;
+      best = rows;
+    }
+  }
+  return best;
+}
+
 static int cl_sms() {
   static int sms = 0;
   if (!sms) {
@@ -1639,8 +1657,9 @@ int vb_cl_dwconv7_parts(float* d_y, void* d_code, const float* d_x, long long x_
   VB_CHECK_ARG(0 <= t_lo && t_lo <= t_hi && t_hi <= T, "vb_cl_dwconv7: range [%d, %d) outside [0, %d)", t_lo, t_hi, T);
   if (B <= 0 || t_lo == t_hi) return 0;
   VB_CHECK_CUDA(max_dyn_smem_once(cl_dwconv7_kernel));
-  VB_LAUNCH_PDL(cl_dwconv7_kernel, dim3((t_hi - t_lo + DW_T - 1) / DW_T, C / 64, B), 256, static_cast<size_t>(DW_T + 6 * dilation) * 256, stream,
-                d_y, static_cast<uint8_t*>(d_code), d_x, x_bstride, d_w, d_bias, d_alpha_in, d_alpha_out, C, T, dilation, t_lo, t_hi);
+  const int tile = cl_dw_rows(t_hi - t_lo, C / 64, B, dilation, cl_sms());
+  VB_LAUNCH_PDL(cl_dwconv7_kernel, dim3((t_hi - t_lo + tile - 1) / tile, C / 64, B), 256, static_cast<size_t>(tile + 6 * dilation) * 256, stream,
+                d_y, static_cast<uint8_t*>(d_code), d_x, x_bstride, d_w, d_bias, d_alpha_in, d_alpha_out, C, T, dilation, t_lo, t_hi, tile);
   return 0;
 }
 int vb_cl_dwconv7(float* d_y, const float* d_x, long long x_bstride, const float* d_w, const float* d_bias, const float* d_alpha_in,

@@ -1078,6 +1078,49 @@ def test_reduce_residual_rmsnorm_many_rows(ops, T, N, S, resid, tiled, hidden):
     assert ((y.float() - ref.float()).abs() <= ref.float().abs() * 2.0 ** -7).all()
 
 
+@pytest.mark.parametrize("T,N,S,resid,tiled", [(65, 8, 2, True, False), (66, 1024, 3, True, True), (129, 1032, 1, False, True), (200, 2048, 8, True, False), (70, 2056, 2, True, True),
+                                               (133, 3072, 4, True, True), (193, 3080, 1, False, False), (300, 4096, 5, True, True), (67, 4104, 2, True, False)])
+def test_reduce_residual_rmsnorm_rows(ops, T, N, S, resid, tiled):
+    """A step past 64 rows (128 threads to a row, one to four groups of columns; past 4096 columns the clusters) against the same rows 64 at a time, which clusters of 8 take."""
+    g = torch.Generator("cuda").manual_seed(T)
+    parts = torch.randn(S, T, N, generator=g, device="cuda")
+    res = torch.randn(T, N, generator=g, device="cuda").to(torch.bfloat16) if resid else None
+    w = torch.randn(N, generator=g, device="cuda").to(torch.bfloat16)
+    out = ops.TiledAct(T, N, torch.device("cuda")) if tiled else None
+    h, y = ops.reduce_residual_rmsnorm(parts, res, w, 1e-6, normed_out=out)
+    y = y.to_rows() if tiled else y
+    cut = [slice(a, min(a + 64, T)) for a in range(0, T, 64)]
+    want = [ops.reduce_residual_rmsnorm(parts[:, c].contiguous(), None if res is None else res[c].contiguous(), w, 1e-6) for c in cut]
+    assert torch.equal(h, torch.cat([a for a, _ in want]))           # (the planes are added in their order by both)
+    # against 64 bits: a sum of N squares in fp32 is off by less than 2^-13 of itself (its chains are shorter than 2^10 terms), the scale by half of that; then bf16
+    hd = h.double()
+    ref = hd * torch.rsqrt((hd * hd).mean(1, keepdim=True) + 1e-6) * w.double()
+    assert ((y.double() - ref).abs() <= ref.abs() * (2.0 ** -8 + 2.0 ** -13)).all()
+
+
+@pytest.mark.parametrize("T,n_q,n_kv,D,S", [(193, 14, 2, 64, 2), (256, 24, 8, 128, 3)])
+def test_qkv_rope_append_rows_from_193(ops, T, n_q, n_kv, D, S):
+    """193 to 256 rows against the same rows in steps of 192, which spread a row's heads: the same bits."""
+    g = torch.Generator("cuda").manual_seed(T)
+    page, W = 16, (n_q + 2 * n_kv) * D
+    parts = torch.randn(S, T, W, generator=g, device="cuda")
+    freq = torch.rand(D, generator=g, device="cuda")
+    pos = torch.randint(0, 4000, (T,), generator=g, device="cuda", dtype=torch.int32)
+    row_page, row_slot = torch.arange(T, device="cuda", dtype=torch.int32) // page, torch.arange(T, device="cuda", dtype=torch.int32) % page
+
+    def run(cuts):
+        kv, q = torch.zeros((T + page - 1) // page, 2, page, n_kv, D, device="cuda", dtype=torch.bfloat16), torch.zeros(T, n_q, D, device="cuda", dtype=torch.bfloat16)
+        for c in cuts:
+            p, n = parts[:, c].contiguous(), c.stop - c.start
+            at = [v[c].contiguous() for v in (pos, row_page, row_slot)]
+            ops.call("vb_qkv_rope_append", q[c].data_ptr(), kv.data_ptr(), p.data_ptr(), S, at[0].data_ptr(), freq.data_ptr(), at[1].data_ptr(), at[2].data_ptr(), n, n_q, n_kv, D,
+                     page, D, 0, None, None, 0.0, None, ops._stream())
+        return q, kv
+
+    for a, b in zip(run([slice(0, T)]), run([slice(0, 192), slice(192, T)])):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("T,n_q,n_kv,D,S,bias", [(257, 1, 1, 16, 1, False), (300, 24, 8, 128, 1, False), (258, 5, 1, 80, 3, True), (600, 2, 2, 256, 2, False)])
 def test_qkv_rope_append_many_rows(ops, T, n_q, n_kv, D, S, bias):
     """A step of more than 256 rows against the same rows in steps of at most 256; rows without a page keep the cache as it is."""

@@ -371,84 +371,88 @@ __global__ void __launch_bounds__(RR_THREADS) reduce_residual_rmsnorm_kernel(
   trace_end(tr);
 }
 
-// The same for steps of many rows: one WARP per row, no shared memory and no barrier.  A lane takes 8 columns of every 256, all
-// planes of four such groups in flight together, keeps the new row as packed bf16 and writes 16 bytes at a time.  With a CTA per row
-// a 1024-row step of 3072 columns took 23.5 us for 31 MB (three loads in flight per thread, then two barriers), now 16.7.
-constexpr int RW_GROUPS = 16;       // N <= 256 * RW_GROUPS
-__global__ void __launch_bounds__(128) reduce_residual_rmsnorm_rows_kernel(
+// The same for steps of more than 64 rows: 128 threads to a row, G groups of 8 columns each.  A row is one chain of a load, a sum over it and a store, so
+// every load of a plane is in flight at once, the norm's weights before the kernel in front has ended, behind one barrier (for the sum of squares).
+// us behind the kernel that writes the planes, before (a warp to a row past 512 rows, else a cluster of 4, 2 or 1 CTAs) / now: 1024 rows of 1024 columns 4.1 / 2.6,
+// 2048 6.7 / 3.7, 3072 9.0 / 5.2, 4096 11.0 / 6.5; three planes of 512 rows 4.7 / 2.9, 6.1 / 4.0, 7.8 / 5.0, 9.9 / 6.3; four of 133 3.8 / 2.6, 3.6 / 3.1, 5.1 / 3.6, 4.8 / 4.1; two of
+// 65 2.8 / 1.8, 3.0 / 2.2, 3.2 / 2.6, 3.1 / 3.0.  Three groups held to 80 registers spill: 133 rows of 3072 6.0.
+template <int G>
+__global__ void __launch_bounds__(128, G <= 2 ? 8 : 5) reduce_residual_rmsnorm_rows_kernel(
     __nv_bfloat16* __restrict__ hidden_out, __nv_bfloat16* __restrict__ normed_out, const float* __restrict__ partials, int split_k,
     const __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ norm_w, int T, int N, float eps, int xt_tile) {
-  const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  __shared__ float part[4];
+  const int t = blockIdx.x, c0 = threadIdx.x * 8;
   const size_t plane = static_cast<size_t>(T) * N, row = static_cast<size_t>(t) * N;
+  uint4 w4[G], r[G], h[G];
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    const int n = g * 1024 + c0;
+    w4[g] = normed_out && n < N ? __ldg(reinterpret_cast<const uint4*>(norm_w + n)) : make_uint4(0u, 0u, 0u, 0u);
+  }
   pdl_sync();
-  if (t >= T) return;
-  uint4 h[RW_GROUPS];
-  float ss = 0.f;
+  float4 a[G][2];
 #pragma unroll
-  for (int g0 = 0; g0 < RW_GROUPS; g0 += 4) {
-    if (g0 * 256 < N) {
-      float4 a[4][2];
-      uint4 r[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int n = (g0 + i) * 256 + lane * 8;
-        a[i][0] = a[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-        r[i] = make_uint4(0u, 0u, 0u, 0u);
-        if (n < N) {
-          const float4* src = reinterpret_cast<const float4*>(partials + row + n);
-          a[i][0] = __ldcg(src);
-          a[i][1] = __ldcg(src + 1);
-          if (residual) r[i] = __ldcg(reinterpret_cast<const uint4*>(residual + row + n));
-        }
-      }
-      for (int s = 1; s < split_k; ++s) {
-        float4 b[4][2];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int n = (g0 + i) * 256 + lane * 8;
-          b[i][0] = b[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (n < N) {
-            const float4* src = reinterpret_cast<const float4*>(partials + s * plane + row + n);
-            b[i][0] = __ldcg(src);
-            b[i][1] = __ldcg(src + 1);
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            a[i][k].x += b[i][k].x; a[i][k].y += b[i][k].y; a[i][k].z += b[i][k].z; a[i][k].w += b[i][k].w;
-          }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int n = (g0 + i) * 256 + lane * 8;
-        const float x[8] = {a[i][0].x, a[i][0].y, a[i][0].z, a[i][0].w, a[i][1].x, a[i][1].y, a[i][1].z, a[i][1].w};
-        const uint32_t rr[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
-        uint32_t o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float u = round_bf16(x[2 * j]), v = round_bf16(x[2 * j + 1]);
-          if (residual) {
-            u = round_bf16(bf16_lo(rr[j]) + u);
-            v = round_bf16(bf16_hi(rr[j]) + v);
-          }
-          o[j] = pack_bf16(u, v);
-          ss += u * u + v * v;
-        }
-        h[g0 + i] = make_uint4(o[0], o[1], o[2], o[3]);
-        if (hidden_out && n < N) *reinterpret_cast<uint4*>(hidden_out + row + n) = h[g0 + i];
-      }
+  for (int g = 0; g < G; ++g) {
+    const int n = g * 1024 + c0;
+    a[g][0] = a[g][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    r[g] = make_uint4(0u, 0u, 0u, 0u);
+    if (n < N) {
+      const float4* src = reinterpret_cast<const float4*>(partials + row + n);
+      a[g][0] = __ldcg(src);
+      a[g][1] = __ldcg(src + 1);
+      if (residual) r[g] = __ldcg(reinterpret_cast<const uint4*>(residual + row + n));
     }
   }
-  if (!normed_out) return;
-  const float rcp = rsqrtf(warp_sum(ss) / static_cast<float>(N) + eps);
+#pragma unroll G <= 2 ? 2 : 1
+  for (int s = 1; s < split_k; ++s) {
+    float4 b[G][2];
 #pragma unroll
-  for (int g = 0; g < RW_GROUPS; ++g) {
-    const int n = g * 256 + lane * 8;
+    for (int g = 0; g < G; ++g) {
+      const int n = g * 1024 + c0;
+      b[g][0] = b[g][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (n < N) {
+        const float4* src = reinterpret_cast<const float4*>(partials + s * plane + row + n);
+        b[g][0] = __ldcg(src);
+        b[g][1] = __ldcg(src + 1);
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        a[g][k].x += b[g][k].x; a[g][k].y += b[g][k].y; a[g][k].z += b[g][k].z; a[g][k].w += b[g][k].w;
+      }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    const int n = g * 1024 + c0;
+    const float x[8] = {a[g][0].x, a[g][0].y, a[g][0].z, a[g][0].w, a[g][1].x, a[g][1].y, a[g][1].z, a[g][1].w};
+    const uint32_t rr[4] = {r[g].x, r[g].y, r[g].z, r[g].w};
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float u = round_bf16(x[2 * j]), v = round_bf16(x[2 * j + 1]);
+      if (residual) {
+        u = round_bf16(bf16_lo(rr[j]) + u);
+        v = round_bf16(bf16_hi(rr[j]) + v);
+      }
+      o[j] = pack_bf16(u, v);
+      ss += u * u + v * v;
+    }
+    h[g] = make_uint4(o[0], o[1], o[2], o[3]);
+    if (hidden_out && n < N) *reinterpret_cast<uint4*>(hidden_out + row + n) = h[g];
+  }
+  if (!normed_out) return;
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  const float rcp = rsqrtf((part[0] + part[1] + part[2] + part[3]) / static_cast<float>(N) + eps);
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    const int n = g * 1024 + c0;
     if (n < N) {
-      const uint4 w4 = __ldg(reinterpret_cast<const uint4*>(norm_w + n));
-      const uint32_t hv[4] = {h[g].x, h[g].y, h[g].z, h[g].w}, wv[4] = {w4.x, w4.y, w4.z, w4.w};
+      const uint32_t hv[4] = {h[g].x, h[g].y, h[g].z, h[g].w}, wv[4] = {w4[g].x, w4[g].y, w4[g].z, w4[g].w};
       uint32_t o[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) o[j] = pack_bf16(bf16_lo(hv[j]) * rcp * bf16_lo(wv[j]), bf16_hi(hv[j]) * rcp * bf16_hi(wv[j]));
@@ -743,21 +747,18 @@ int vb_reduce_residual_rmsnorm(void* d_hidden_out, void* d_normed_out, const flo
   VB_CHECK_ARG(!d_normed_out || d_norm_weight, "vb_reduce_residual_rmsnorm: norm output needs a weight");
   if (T <= 0) return 0;
   auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
-  // (512 rows of 3072, operands cold: 14.3 us with a CTA per row, 15.1 with a warp; 1024 rows: 23.5 and 16.7.  Launches back to back,
-  // CTA / warp: 512 rows of 1024 columns 4.9 / 4.1 us, 2048 7.4 / 7.4, 3072 9.9 / 10.2, 4096 11.9 / 13.1; 640 rows 6.5 / 4.5, 10.1 / 7.9,
-  // 13.4 / 10.7, 17.0 / 13.7: the line holds for every width)
-  if (T > 512 && N % 8 == 0 && N <= 256 * RW_GROUPS && aligned(d_partials) && aligned(d_hidden_out) && aligned(d_normed_out) &&
-      aligned(d_residual) && aligned(d_norm_weight)) {
-    VB_LAUNCH_PDL(reduce_residual_rmsnorm_rows_kernel, (T + 3) / 4, 128, 0, stream, static_cast<__nv_bfloat16*>(d_hidden_out),
+  if (T > 64 && N % 8 == 0 && N <= 4096 && aligned(d_partials) && aligned(d_hidden_out) && aligned(d_normed_out) && aligned(d_residual) &&
+      aligned(d_norm_weight)) {
+    const auto rows = N <= 1024 ? reduce_residual_rmsnorm_rows_kernel<1> : N <= 2048 ? reduce_residual_rmsnorm_rows_kernel<2> :
+                      N <= 3072 ? reduce_residual_rmsnorm_rows_kernel<3> : reduce_residual_rmsnorm_rows_kernel<4>;
+    VB_LAUNCH_PDL(rows, T, 128, 0, stream, static_cast<__nv_bfloat16*>(d_hidden_out),
                   static_cast<__nv_bfloat16*>(d_normed_out), d_partials, split_k, static_cast<const __nv_bfloat16*>(d_residual),
                   static_cast<const __nv_bfloat16*>(d_norm_weight), T, N, eps, normed_xt_tile);
     return 0;
   }
-  // widest cluster (<= 8, the portable limit) that divides the row into float4-aligned parts; few rows -> more parts
   int parts = 1;
-  // (past some 512 CTAs a split row costs more than it gives: 256 rows of 3072, operands cold, 15.4 us in four parts, 11 whole.  Launches
-  // back to back, where a neighbour covers a row's latency, want whole rows earlier, in 4 / 2 / 1 parts: 128 rows of 1024 columns
-  // 4.6 / 2.5 / 1.8 us, 3072 5.7 / 4.4 / 4.3, 4096 6.1 / 4.8 / 5.8; 192 rows 6.6 / 4.4 / 2.0, 8.8 / 8.2 / 5.3, 9.2 / 8.5 / 6.4)
+  // widest cluster (<= 8, the portable limit) that divides the row into float4-aligned parts; few rows -> more parts (past some 512 CTAs a
+  // split row costs more than it gives)
   const int want = T <= 64 ? 8 : (T <= 128 ? 4 : (T <= 192 ? 2 : 1));
   for (int c = want; c >= 1; c >>= 1)
     if (N % (4 * c) == 0) { parts = c; break; }
@@ -783,10 +784,9 @@ int vb_qkv_rope_append(void* d_q_out, void* d_layer_kv, const float* d_partials,
   if (T <= 0) return 0;
   const int n_heads = n_q + 2 * n_kv;
   auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
-  // (257 rows of 40 heads of 128, operands cold: 11.3 us by the kernel below, 9.2 here; it spreads a row's heads over CTAs up to 256 rows.
-  // Launches back to back, below / here: 257 rows of 24 + 8 + 8 heads of 128 7.5 / 4.9 us, 32 + 8 + 8 of 64 5.3 / 3.3, 14 + 2 + 2 of 64
-  // 3.2 / 2.3, 16 + 8 + 8 of 128 6.6 / 3.7; down to some 100 rows this kernel is ahead there too, 4.0 / 3.6, 3.1 / 2.2, 2.5 / 2.1, 3.1 / 2.5)
-  if (T > 256 && !interleave && rotary_dim == head_dim && head_dim % 16 == 0 && head_dim <= 256 && !d_q_norm && aligned(d_q_out) &&
+  // (Behind the kernel that writes the planes, the kernel below / this one, us: 200 rows in four planes of 24 + 8 + 8 heads of 128 6.1 / 5.3, 32 + 8 + 8 of 64
+  // 5.8 / 3.8, 14 + 2 + 2 of 64 3.3 / 3.0, 16 + 8 + 8 of 128 4.6 / 4.0, 32 + 2 + 2 of 128 6.2 / 5.4; 133 rows 4.4 / 4.8, 4.0 / 3.3, 3.4 / 3.0, 4.0 / 3.3, 4.3 / 4.7.)
+  if (T > 192 && !interleave && rotary_dim == head_dim && head_dim % 16 == 0 && head_dim <= 256 && !d_q_norm && aligned(d_q_out) &&
       aligned(d_layer_kv) && aligned(d_partials)) {
     VB_LAUNCH_PDL(qkv_rope_rows_kernel, T, 256, 2 * head_dim * sizeof(float), stream, static_cast<__nv_bfloat16*>(d_q_out),
                   static_cast<__nv_bfloat16*>(d_layer_kv), d_partials, split_k, d_pos, d_freq, d_row_page, d_row_slot, T, n_q, n_kv, head_dim,

@@ -208,6 +208,7 @@ class LlamaEngine:
         self.act_t = ops.TiledAct(self.FUSED_MAX_ROWS, I, dev, max_T=self.tiled_max_rows)
         self.hidden_t = ops.TiledAct(self.FUSED_MAX_ROWS, H, dev)
         self.max_out_rows = min(R, 64)     # logits are only ever needed for one row per request
+        self.last_hidden = torch.zeros(self.max_out_rows, H, dtype=BF16, device=dev)
         self.last_normed = torch.zeros(self.max_out_rows, H, dtype=BF16, device=dev)
         self.logits = torch.zeros(self.max_out_rows, d.vocab_size, dtype=BF16, device=dev)
         self.attn_ws = ops.AttnWorkspace(R, hq, hkv, D, dev)
@@ -276,15 +277,17 @@ class LlamaEngine:
             ops.rmsnorm(hidden, w.norm, d.rms_norm_eps, out=x_final)
         else:
             x_final = self._layers_unfused(position_ids, R, plan)
-        hidden_rows = None
-        if last_rows is not None or want_hidden:
-            if isinstance(x_final, ops.TiledAct):      # a gather needs rows: redo the final norm row-major
-                ops.rmsnorm(hidden, w.norm, d.rms_norm_eps, out=normed)
         if last_rows is not None:
             n_out = last_rows.numel() if n_out is None else n_out
-            x = ops.gather_rows(normed, last_rows, out=self.last_normed[:n_out], idx_offset=last_rows_offset)
+            if isinstance(x_final, ops.TiledAct):      # a gather needs rows: those of the stream, then their norm
+                rows = ops.gather_rows(hidden, last_rows, out=self.last_hidden[:n_out], idx_offset=last_rows_offset)
+                x = ops.rmsnorm(rows, w.norm, d.rms_norm_eps, out=self.last_normed[:n_out])
+            else:
+                x = ops.gather_rows(normed, last_rows, out=self.last_normed[:n_out], idx_offset=last_rows_offset)
             hidden_rows = x
         else:
+            if want_hidden and isinstance(x_final, ops.TiledAct):
+                ops.rmsnorm(hidden, w.norm, d.rms_norm_eps, out=normed)
             n_out, x = R, x_final
             hidden_rows = normed
         if n_out > self.max_out_rows:

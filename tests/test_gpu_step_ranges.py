@@ -1078,6 +1078,27 @@ def test_reduce_residual_rmsnorm_many_rows(ops, T, N, S, resid, tiled, hidden):
     assert ((y.float() - ref.float()).abs() <= ref.float().abs() * 2.0 ** -7).all()
 
 
+@pytest.mark.parametrize("hq,hkv,D", [(32, 2, 64), (16, 2, 128), (16, 1, 64), (24, 8, 128)])
+def test_paged_attention_many_short_rows(ops, hq, hkv, D):
+    """Rows of a tile or less behind one another in a CTA: every row with its own Q, however often (the next row's came too early now and then)."""
+    g, page, B = torch.Generator("cuda").manual_seed(hq + hkv), 128, 96
+    lens = [1 + 7 * i % 128 for i in range(B)]
+    kv = torch.randn(B, 2, page, hkv, D, generator=g, device="cuda").to(torch.bfloat16)
+    q = torch.randn(B, hq, D, generator=g, device="cuda").to(torch.bfloat16)
+    k, v = (kv[:, j].double().repeat_interleave(hq // hkv, 2) for j in range(2))
+    s = torch.einsum("bhd,bkhd->bhk", q.double(), k) * D ** -0.5
+    s = s.masked_fill(torch.arange(page, device="cuda") >= torch.tensor(lens, device="cuda")[:, None, None], -float("inf"))
+    want = torch.einsum("bhk,bkhd->bhd", torch.softmax(s, -1), v)
+    chunk = ops.attn_chunk_tokens(page, hkv)
+    plan = ops.plan_rows(ops.RowPlan(B, "cuda"), None, _i32(list(range(B + 1))), _i32(list(range(B))), _i32(lens), B, B, page, chunk)
+    ws = ops.paged_attn_workspace(B, None, hq, hkv, D, "cuda")
+    for grid in (1, 3, 7, 20):
+        for _ in range(20):
+            out = ops.paged_attn(q, kv, 0, plan, B, hkv, page, chunk, ws, grid_ctas=grid)
+            err = (out.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)
+            assert err.max() < 2.0 ** -8, (grid, lens[int(err.argmax())])      # weights rounded to bf16, then the result: 2^-9 each at most
+
+
 @pytest.mark.parametrize("T,N,S,resid,tiled", [(65, 8, 2, True, False), (66, 1024, 3, True, True), (129, 1032, 1, False, True), (200, 2048, 8, True, False), (70, 2056, 2, True, True),
                                                (133, 3072, 4, True, True), (193, 3080, 1, False, False), (300, 4096, 5, True, True), (67, 4104, 2, True, False)])
 def test_reduce_residual_rmsnorm_rows(ops, T, N, S, resid, tiled):

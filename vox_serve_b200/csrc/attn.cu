@@ -320,8 +320,6 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
           qb[nt][ks][1] = ok ? *reinterpret_cast<const uint32_t*>(qsm + hq * (D * 2) + d0 + 16) : 0u;
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&qempty[0]);
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -350,9 +348,13 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
         for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(S[nt], a, qb[nt][ks][0], qb[nt][ks][1]);
       }
     }
-    // this warp is done with the K half-stage
+    // this warp is done with the K half-stage, and has its Q: the products have read all of it.  (An arrival does not wait for loads that nothing has used yet:
+    // right behind them, with the conflicts of all warps' loads in the queue, the next row's Q could land first)
     __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[stage]);
+    if (lane == 0) {
+      mbar_arrive(&empty[stage]);
+      if (m.flags & 1) mbar_arrive(&qempty[0]);
+    }
     if (++stage == STAGES) { stage = 0; ph ^= 1; }
     // ---- mask, running max, P = exp2(S - m) rounded to bf16, sums of the rounded values ----
     const int tok_lo = m.token0 + slab * 16 + g;

@@ -1078,6 +1078,32 @@ def test_reduce_residual_rmsnorm_many_rows(ops, T, N, S, resid, tiled, hidden):
     assert ((y.float() - ref.float()).abs() <= ref.float().abs() * 2.0 ** -7).all()
 
 
+@pytest.mark.parametrize("page,hq,hkv,D", [(128, 24, 8, 128), (16, 16, 8, 64), (64, 12, 4, 128), (128, 16, 1, 64), (16, 32, 2, 128), (16, 16, 1, 128), (48, 18, 6, 64)])
+def test_paged_attention_runs_of_rows(ops, page, hq, hkv, D):
+    """Cache rows copied by twos, fours and singly: lengths around the ends of runs, slabs and tiles, against 64 bits; what lies behind a row's end in its page is never seen."""
+    g = torch.Generator("cuda").manual_seed(page + hq)
+    lens = [*range(1, 20), 31, 32, 33, 47, 48, 49, 63, 64, 65, 127, 128, 129, 400]
+    pages = [(n + page - 1) // page for n in lens]
+    kv = torch.randn(sum(pages), 2, page, hkv, D, generator=g, device="cuda").to(torch.bfloat16)
+    q = torch.randn(len(lens), hq, D, generator=g, device="cuda").to(torch.bfloat16)
+    order = torch.randperm(sum(pages), generator=g, device="cuda").tolist()
+    indptr = [sum(pages[:i]) for i in range(len(lens) + 1)]
+    want = []
+    for i, n in enumerate(lens):
+        own = order[indptr[i]:indptr[i + 1]]
+        kv[own[-1], :, (n - 1) % page + 1:] = 100.0
+        k, v = (kv[own, j].reshape(-1, hkv, D)[:n].double().repeat_interleave(hq // hkv, 1) for j in range(2))
+        w = torch.softmax(torch.einsum("hd,khd->hk", q[i].double(), k) * D ** -0.5, -1)
+        want.append(torch.einsum("hk,khd->hd", w, v))
+    want = torch.stack(want)
+    chunk = ops.attn_chunk_tokens(page, hkv)
+    plan = ops.plan_rows(ops.RowPlan(len(lens), "cuda"), None, _i32(indptr), _i32(order), _i32([(n - 1) % page + 1 for n in lens]), len(lens), len(lens), page, chunk)
+    ws = ops.paged_attn_workspace(len(lens), None, hq, hkv, D, "cuda")
+    for grid in (None, 1, 7):
+        out = ops.paged_attn(q, kv, 0, plan, len(lens), hkv, page, chunk, ws, grid_ctas=grid)
+        _close(out, want, 2.0 ** -8)               # weights rounded to bf16, then the result: 2^-9 each at most
+
+
 @pytest.mark.parametrize("hq,hkv,D", [(32, 2, 64), (16, 2, 128), (16, 1, 64), (24, 8, 128)])
 def test_paged_attention_many_short_rows(ops, hq, hkv, D):
     """Rows of a tile or less behind one another in a CTA: every row with its own Q, however often (the next row's came too early now and then)."""

@@ -11,13 +11,13 @@
 //    shared-memory copies of the plan -- and feeds a ring of HALF-stages (the K rows of a tile, then its V rows:
 //    32 KiB + skew each) behind full/empty mbarriers with the TMA unit's LINEAR bulk copies
 //    (cp.async.bulk.shared.global, L2 evict_first: a layer's KV is not read again before the next step): one
-//    copy per token row (n_kv * D * 2 bytes, all heads), issued by the warp's lanes in parallel.  Three
+//    copy per run of one to four token rows (n_kv * D * 2 bytes each, all heads), issued by the warp's lanes in parallel.  Three
 //    half-stages (~100 KiB) keep a CTA below half an SM's shared memory, so the CTA of a NEIGHBOURING kernel of
 //    the programmatic-dependent-launch chain (the next layer's attention in a back-to-back run; the O projection's
 //    weight prefetch or the QKV tail in a decode step) is resident beside it: its launch latency, plan look-up
-//    and the KV of tokens that were already in the cache stream in while this kernel is still running.  Rows land with a 16-byte
-//    skew (row stride n_kv * D * 2 + 16) so that the consumers' ldmatrix reads of 8 consecutive tokens are
-//    bank-conflict free without a swizzle.  (A tiled tensor-map box must keep a 128-byte inner extent under the
+//    and the KV of tokens that were already in the cache stream in while this kernel is still running.  Runs land with a 16-byte
+//    skew behind each, and the eight rows of an ldmatrix are taken from different runs, so that they lie in different
+//    banks without a swizzle.  (A tiled tensor-map box must keep a 128-byte inner extent under the
 //    128B swizzle; measured, the TMA unit then spends ~19 cycles per 128-byte row and caps the kernel below
 //    2 TB/s -- 2 KiB linear rows are 16x fewer requests.)  The row's Q (all heads) is bulk-copied into a double
 //    buffer at each segment start;
@@ -51,6 +51,7 @@ struct AttnParams {
   float* part_o;                 // [grid * 2][n_q][D]
   int slab_base;
   int n_rows, n_q, n_kv, G, page_size, tok, stages;
+  int run_log2;                  // token rows per copy: 1, 2 or 4
   int out_xt_tile;               // 0: out is [row][n_q][D]; else the tiled XT(out_xt_tile) layout of [row][n_q * D]
   float scale_log2;
 };
@@ -94,8 +95,8 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
 // shared-memory carve-up (host and device agree through this one function)
 struct AttnLayout {
   int stage_bytes, off_q, off_meta, off_bar, off_wml, off_flag, off_ored, off_plan, total;
-  __host__ __device__ AttnLayout(int D, int tok, int n_kv, int n_q, int G, int stages, int n_rows) {
-    stage_bytes = tok * (n_kv * D * 2 + 16);                    // one half-stage: K (or V) rows, each skewed by 16 bytes
+  __host__ __device__ AttnLayout(int D, int tok, int n_kv, int n_q, int G, int stages, int n_rows, int run_log2) {
+    stage_bytes = tok * n_kv * D * 2 + (tok >> run_log2) * 16;        // one half-stage: K (or V) rows, each run of them skewed by 16 bytes
     off_q = stages * stage_bytes;
     off_meta = off_q + ATTN_QBUF * n_q * D * 2;
     off_bar = off_meta + ATTN_MAX_STAGES * 32;                  // full[8], empty[8], qfull, qempty
@@ -120,11 +121,11 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
   const int G = p.G, TOK = p.tok, STAGES = p.stages;
-  const AttnLayout L(D, TOK, p.n_kv, p.n_q, G, STAGES, p.n_rows);
+  const AttnLayout L(D, TOK, p.n_kv, p.n_q, G, STAGES, p.n_rows, p.run_log2);
   const int NW = p.n_kv * (TOK / 16);   // consumer warps
   const int NC = NW * 32;
   const int ROWB = p.n_kv * D * 2;      // bytes of one token row (all heads) in the cache
-  const int RS = ROWB + 16;             // its stride in shared memory (16-byte skew)
+  const int RUN_L = p.run_log2, RUNB = ROWB << RUN_L, RS = RUNB + 16;   // a run of rows, one copy, and its stride in shared memory (16-byte skew)
   TileMeta* meta = reinterpret_cast<TileMeta*>(smem + L.off_meta);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.off_bar);
   uint64_t* empty = full + ATTN_MAX_STAGES;
@@ -256,8 +257,8 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
             }
             __syncwarp();
             uint8_t* dst = smem + stage * L.stage_bytes;
-            for (int t = lane; t < TOK; t += 32)
-              bulk_copy_g2s_hint(dst + t * RS, src0 + kvsel * page_elems + static_cast<size_t>(t) * p.n_kv * D, ROWB,
+            for (int t = lane; t << RUN_L < TOK; t += 32)
+              bulk_copy_g2s_hint(dst + t * RS, src0 + kvsel * page_elems + static_cast<size_t>(t << RUN_L) * p.n_kv * D, RUNB,
                                  &full[stage], pol_kv);
             __syncwarp();
             if (++stage == STAGES) { stage = 0; ph ^= 1; }
@@ -291,6 +292,14 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
   const int slab = warp / p.n_kv;  // 16-token slab of the tile
   const int hoff = head * D * 2;   // byte offset of this warp's head inside a token row
   const int mi = lane >> 3, r8 = lane & 7;
+  // row r of half h of a slab's MMA rows: the runs are dealt over the eight rows, so that rows of one ldmatrix lie in different banks
+  auto tok_of = [&](int h, int r) {
+    const int rest = r >> (4 - RUN_L), step = 8 >> (4 - RUN_L);       // (of 16 >> RUN_L runs)
+    return RUN_L == 0 ? h * 8 + r : ((r & ((16 >> RUN_L) - 1)) << RUN_L) + rest + h * step;
+  };
+  auto row_at = [&](int h, int r) { const int t = slab * 16 + tok_of(h, r); return (t >> RUN_L) * RS + (t & ((1 << RUN_L) - 1)) * ROWB; };
+  const int k_at = row_at(mi & 1, r8) + hoff + (mi >> 1) * 16, v_at = row_at(mi >> 1, r8) + hoff + (mi & 1) * 16;
+  const int t_lo = slab * 16 + tok_of(0, g), t_hi = slab * 16 + tok_of(1, g);
 
   uint32_t qb[NT][KS][2];
   float O[MT][NT][4];
@@ -338,8 +347,7 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) S[nt][0] = S[nt][1] = S[nt][2] = S[nt][3] = 0.f;
     {
-      const int trow = slab * 16 + r8 + (mi & 1) * 8;
-      const uint32_t rbase = kbase + trow * RS + hoff + (mi >> 1) * 16;
+      const uint32_t rbase = kbase + k_at;
 #pragma unroll
       for (int ks = 0; ks < KS; ++ks) {
         uint32_t a[4];
@@ -357,8 +365,7 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
     }
     if (++stage == STAGES) { stage = 0; ph ^= 1; }
     // ---- mask, running max, P = exp2(S - m) rounded to bf16, sums of the rounded values ----
-    const int tok_lo = m.token0 + slab * 16 + g;
-    const bool in_lo = tok_lo < m.kvlen, in_hi = tok_lo + 8 < m.kvlen;
+    const bool in_lo = m.token0 + t_lo < m.kvlen, in_hi = m.token0 + t_hi < m.kvlen;
     uint32_t pb[NT][2];
     float alpha[NT][2];
     bool rescale = false;
@@ -390,9 +397,7 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
     // ---- O^T = O^T * alpha + V^T P^T ----
     mbar_wait(&full[stage], ph);
     {
-      const uint32_t vbase = smem_u32(smem + stage * L.stage_bytes);
-      const int trow = slab * 16 + r8 + (mi >> 1) * 8;
-      const uint32_t rbase = vbase + trow * RS + hoff + (mi & 1) * 16;
+      const uint32_t rbase = smem_u32(smem + stage * L.stage_bytes) + v_at;
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         uint32_t a[4];
@@ -641,7 +646,7 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
 
 template <int D, bool HI, int MINB>
 static int launch_attn(const AttnParams& p, int grid, cudaStream_t stream) {
-  const AttnLayout L(D, p.tok, p.n_kv, p.n_q, p.G, p.stages, p.n_rows);
+  const AttnLayout L(D, p.tok, p.n_kv, p.n_q, p.G, p.stages, p.n_rows, p.run_log2);
   VB_CHECK_ARG(L.total <= VB_MAX_DYN_SMEM, "vb_paged_attn: %d rows / %d-token tiles need %d bytes of shared memory",
                p.n_rows, p.tok, L.total);
   auto kern = paged_attn_kernel<D, HI, MINB>;
@@ -708,6 +713,13 @@ int vb_paged_attn(void* d_out, const void* d_q, const void* d_kv, int64_t slab_b
   p.slab_base = static_cast<int>(slab_base);
   p.n_rows = n_rows; p.n_q = n_q; p.n_kv = n_kv; p.G = n_q / n_kv; p.page_size = page_size;
   p.tok = chunk_tokens;
+  // Rows per copy: a copy of one row costs the copy engine some 15 ns beside its bytes, so a run of rows travels in one, with the skew behind each run.  Up to two rows
+  // in a run leave ldmatrix without bank conflicts, four make them two-way.  us of one launch, rows singly / by 2 / by 4 / by 8, 64 requests, cold: 24 heads on 8 of 128
+  // (rows of 2 KB) 301 to 2304 tokens 69 / 57 / 58 / 59, 2048 tokens 103 / 84 / 85 / 85 (6.4 TB/s); 1024 tokens, 32 on 8 of 64 (1 KB) 53 / 40 / 34 / 35, 32 on 4 of 128 74 / 64 /
+  // 61 / 64, 14 on 2 of 64 (256 B) 46 / 34 / 32 / 33.  Where two warps work off a tile of small rows with two column tiles each, their own chain is the limit and single
+  // rows are no slower: 32 on 2 of 128 in pages of 16 60 / 88 / 89, 24 on 2 86 / 85 / 86.
+  const int row_bytes = n_kv * head_dim * 2;
+  p.run_log2 = p.G > 8 && p.tok * row_bytes < 16384 ? 0 : row_bytes >= 2048 ? 1 : 2;
   p.out_xt_tile = out_xt_tile;
   p.scale_log2 = sm_scale * 1.4426950408889634f;
   // deepest ring of half-stages that fits the budget next to the fixed buffers.  Measured on B200 (28 launches back to
@@ -722,13 +734,13 @@ int vb_paged_attn(void* d_out, const void* d_q, const void* d_kv, int64_t slab_b
     budget = (kb >= 64 && kb <= 227 ? kb : 224) * 1024;
   }
   int stages = ATTN_MAX_STAGES;
-  while (stages > 2 && AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows).total > budget) --stages;
-  VB_CHECK_ARG(AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows).total <= VB_MAX_DYN_SMEM,
+  while (stages > 2 && AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows, p.run_log2).total > budget) --stages;
+  VB_CHECK_ARG(AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows, p.run_log2).total <= VB_MAX_DYN_SMEM,
                "vb_paged_attn: %d rows need more shared memory than an SM has", n_rows);
   p.stages = stages;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool hi = p.G > 8;
-  const bool two = 2 * (AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows).total + 1024) <= 232448;
+  const bool two = 2 * (AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows, p.run_log2).total + 1024) <= 232448;
   if (two) {
     if (head_dim == 128) return hi ? launch_attn<128, true, 2>(p, grid_ctas, st) : launch_attn<128, false, 2>(p, grid_ctas, st);
     return hi ? launch_attn<64, true, 2>(p, grid_ctas, st) : launch_attn<64, false, 2>(p, grid_ctas, st);

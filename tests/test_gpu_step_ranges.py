@@ -1125,10 +1125,11 @@ def test_paged_attention_many_short_rows(ops, hq, hkv, D):
             assert err.max() < 2.0 ** -8, (grid, lens[int(err.argmax())])      # weights rounded to bf16, then the result: 2^-9 each at most
 
 
-@pytest.mark.parametrize("T,N,S,resid,tiled", [(65, 8, 2, True, False), (66, 1024, 3, True, True), (129, 1032, 1, False, True), (200, 2048, 8, True, False), (70, 2056, 2, True, True),
-                                               (133, 3072, 4, True, True), (193, 3080, 1, False, False), (300, 4096, 5, True, True), (67, 4104, 2, True, False)])
+@pytest.mark.parametrize("T,N,S,resid,tiled", [(1, 8, 2, True, False), (3, 264, 9, False, True), (64, 1032, 8, True, True), (65, 1024, 3, True, True), (148, 2048, 16, True, False),
+                                               (130, 4096, 7, True, True), (149, 8, 1, True, False), (300, 1032, 3, False, True), (258, 2056, 2, True, True), (259, 3080, 1, False, False),
+                                               (300, 4096, 5, True, True), (67, 4104, 2, True, False)])
 def test_reduce_residual_rmsnorm_rows(ops, T, N, S, resid, tiled):
-    """A step past 64 rows (128 threads to a row, one to four groups of columns; past 4096 columns the clusters) against the same rows 64 at a time, which clusters of 8 take."""
+    """A thread to 8 columns up to 148 rows, beyond 128 threads to a row with one to four groups of columns; past 4096 columns the clusters."""
     g = torch.Generator("cuda").manual_seed(T)
     parts = torch.randn(S, T, N, generator=g, device="cuda")
     res = torch.randn(T, N, generator=g, device="cuda").to(torch.bfloat16) if resid else None
@@ -1136,9 +1137,11 @@ def test_reduce_residual_rmsnorm_rows(ops, T, N, S, resid, tiled):
     out = ops.TiledAct(T, N, torch.device("cuda")) if tiled else None
     h, y = ops.reduce_residual_rmsnorm(parts, res, w, 1e-6, normed_out=out)
     y = y.to_rows() if tiled else y
-    cut = [slice(a, min(a + 64, T)) for a in range(0, T, 64)]
-    want = [ops.reduce_residual_rmsnorm(parts[:, c].contiguous(), None if res is None else res[c].contiguous(), w, 1e-6) for c in cut]
-    assert torch.equal(h, torch.cat([a for a, _ in want]))           # (the planes are added in their order by both)
+    acc = parts[0].clone()
+    for p in parts[1:]:
+        acc += p
+    want = acc.to(torch.bfloat16) if res is None else res + acc.to(torch.bfloat16)
+    assert torch.equal(h, want)                                      # (the planes are added in their order)
     # against 64 bits: a sum of N squares in fp32 is off by less than 2^-13 of itself (its chains are shorter than 2^10 terms), the scale by half of that; then bf16
     hd = h.double()
     ref = hd * torch.rsqrt((hd * hd).mean(1, keepdim=True) + 1e-6) * w.double()

@@ -371,11 +371,11 @@ __global__ void __launch_bounds__(RR_THREADS) reduce_residual_rmsnorm_kernel(
   trace_end(tr);
 }
 
-// The same for steps of more than 64 rows: 128 threads to a row, G groups of 8 columns each.  A row is one chain of a load, a sum over it and a store, so
+// The same for steps of more rows than there are SMs: 128 threads to a row, G groups of 8 columns each.  A row is one chain of a load, a sum over it and a store, so
 // every load of a plane is in flight at once, the norm's weights before the kernel in front has ended, behind one barrier (for the sum of squares).
-// us behind the kernel that writes the planes, before (a warp to a row past 512 rows, else a cluster of 4, 2 or 1 CTAs) / now: 1024 rows of 1024 columns 4.1 / 2.6,
-// 2048 6.7 / 3.7, 3072 9.0 / 5.2, 4096 11.0 / 6.5; three planes of 512 rows 4.7 / 2.9, 6.1 / 4.0, 7.8 / 5.0, 9.9 / 6.3; four of 133 3.8 / 2.6, 3.6 / 3.1, 5.1 / 3.6, 4.8 / 4.1; two of
-// 65 2.8 / 1.8, 3.0 / 2.2, 3.2 / 2.6, 3.1 / 3.0.  Three groups held to 80 registers spill: 133 rows of 3072 6.0.
+// us behind the kernel that writes the planes, before (a warp to a row past 512 rows, else a CTA or a cluster) / now: 1024 rows of 1024 columns 4.1 / 2.6,
+// 2048 6.7 / 3.7, 3072 9.0 / 5.2, 4096 11.0 / 6.5; three planes of 512 rows 4.7 / 2.9, 6.1 / 4.0, 7.8 / 5.0, 9.9 / 6.3.  Three groups held to 80 registers spill:
+// four planes of 133 rows of 3072 6.0 for 3.6.
 template <int G>
 __global__ void __launch_bounds__(128, G <= 2 ? 8 : 5) reduce_residual_rmsnorm_rows_kernel(
     __nv_bfloat16* __restrict__ hidden_out, __nv_bfloat16* __restrict__ normed_out, const float* __restrict__ partials, int split_k,
@@ -460,6 +460,72 @@ __global__ void __launch_bounds__(128, G <= 2 ? 8 : 5) reduce_residual_rmsnorm_r
       *reinterpret_cast<uint4*>(normed_out + oi) = make_uint4(o[0], o[1], o[2], o[3]);
     }
   }
+}
+
+// The same for steps of few rows: a thread to every 8 columns of a row and eight planes in flight, one barrier.  us behind the kernel that writes the planes, a cluster of
+// 8 CTAs to a row (its launch and its meeting) / now: eight planes of 1, 8, 32 and 64 rows of 3072 columns 4.1 / 3.0, 4.3 / 3.2, 4.5 / 3.2, 8.5 / 3.5; four 3.3 / 2.6, 3.5 / 2.8, 3.7 / 3.0,
+// 6.5 / 2.9; eight of 32 rows of 1024 columns 4.2 / 2.7, of 4096 4.2 / 3.8.
+constexpr int RW_PLANES = 7;        // beside the first
+__global__ void __launch_bounds__(512) reduce_residual_rmsnorm_row_kernel(
+    __nv_bfloat16* __restrict__ hidden_out, __nv_bfloat16* __restrict__ normed_out, const float* __restrict__ partials, int split_k,
+    const __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ norm_w, int T, int N, float eps, int xt_tile) {
+  __shared__ float part[16];
+  const int t = blockIdx.x, n = threadIdx.x * 8;
+  const bool in = n < N;
+  const size_t plane = static_cast<size_t>(T) * N, row = static_cast<size_t>(t) * N;
+  const int tr = (threadIdx.x == 0 && trace_block0()) ? trace_begin(5, split_k) : -1;
+  const uint4 w4 = normed_out && in ? __ldg(reinterpret_cast<const uint4*>(norm_w + n)) : make_uint4(0u, 0u, 0u, 0u);
+  pdl_sync();
+  const float4* src = reinterpret_cast<const float4*>(partials + row + n);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 a[2] = {in ? __ldcg(src) : zero, in ? __ldcg(src + 1) : zero};
+  const uint4 r = residual && in ? __ldcg(reinterpret_cast<const uint4*>(residual + row + n)) : make_uint4(0u, 0u, 0u, 0u);
+  for (int s0 = 1; s0 < split_k; s0 += RW_PLANES) {
+    float4 b[RW_PLANES][2];
+#pragma unroll
+    for (int i = 0; i < RW_PLANES; ++i)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) b[i][k] = in && s0 + i < split_k ? __ldcg(src + (s0 + i) * (plane >> 2) + k) : zero;
+#pragma unroll
+    for (int i = 0; i < RW_PLANES; ++i)
+      if (s0 + i < split_k) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          a[k].x += b[i][k].x; a[k].y += b[i][k].y; a[k].z += b[i][k].z; a[k].w += b[i][k].w;
+        }
+      }
+  }
+  float ss = 0.f;
+  const float x[8] = {a[0].x, a[0].y, a[0].z, a[0].w, a[1].x, a[1].y, a[1].z, a[1].w};
+  const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
+  uint32_t h[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float u = round_bf16(x[2 * j]), v = round_bf16(x[2 * j + 1]);
+    if (residual) {
+      u = round_bf16(bf16_lo(rr[j]) + u);
+      v = round_bf16(bf16_hi(rr[j]) + v);
+    }
+    h[j] = pack_bf16(u, v);
+    ss += u * u + v * v;
+  }
+  if (hidden_out && in) *reinterpret_cast<uint4*>(hidden_out + row + n) = make_uint4(h[0], h[1], h[2], h[3]);
+  if (!normed_out) { trace_end(tr); return; }
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float total = 0.f;
+  for (int i = 0; i < static_cast<int>(blockDim.x >> 5); ++i) total += part[i];
+  const float rcp = rsqrtf(total / static_cast<float>(N) + eps);
+  if (in) {
+    const uint32_t wv[4] = {w4.x, w4.y, w4.z, w4.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = pack_bf16(bf16_lo(h[j]) * rcp * bf16_lo(wv[j]), bf16_hi(h[j]) * rcp * bf16_hi(wv[j]));
+    const size_t oi = xt_tile ? xt_index(t, n, xt_tile, (N + 63) >> 6) : row + n;
+    *reinterpret_cast<uint4*>(normed_out + oi) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  trace_end(tr);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -747,11 +813,15 @@ int vb_reduce_residual_rmsnorm(void* d_hidden_out, void* d_normed_out, const flo
   VB_CHECK_ARG(!d_normed_out || d_norm_weight, "vb_reduce_residual_rmsnorm: norm output needs a weight");
   if (T <= 0) return 0;
   auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
-  if (T > 64 && N % 8 == 0 && N <= 4096 && aligned(d_partials) && aligned(d_hidden_out) && aligned(d_normed_out) && aligned(d_residual) &&
-      aligned(d_norm_weight)) {
-    const auto rows = N <= 1024 ? reduce_residual_rmsnorm_rows_kernel<1> : N <= 2048 ? reduce_residual_rmsnorm_rows_kernel<2> :
-                      N <= 3072 ? reduce_residual_rmsnorm_rows_kernel<3> : reduce_residual_rmsnorm_rows_kernel<4>;
-    VB_LAUNCH_PDL(rows, T, 128, 0, stream, static_cast<__nv_bfloat16*>(d_hidden_out),
+  if (N % 8 == 0 && N <= 4096 && aligned(d_partials) && aligned(d_hidden_out) && aligned(d_normed_out) && aligned(d_residual) && aligned(d_norm_weight)) {
+    // (a thread to 8 columns, of which an SM holds one row / 128 threads to a row, us: four planes of 133 rows of 2048, 3072, 4096 columns 2.7 / 3.2, 3.1 / 3.5, 3.3 / 4.0, of
+    // 256 rows 3.2 / 3.3, 4.9 / 3.9, 5.7 / 4.7; one of 1024 4.4 / 3.7, 6.1 / 5.0, 8.5 / 6.4)
+    const auto rows = T <= 148   ? reduce_residual_rmsnorm_row_kernel
+                      : N <= 1024 ? reduce_residual_rmsnorm_rows_kernel<1>
+                      : N <= 2048 ? reduce_residual_rmsnorm_rows_kernel<2>
+                      : N <= 3072 ? reduce_residual_rmsnorm_rows_kernel<3>
+                                  : reduce_residual_rmsnorm_rows_kernel<4>;
+    VB_LAUNCH_PDL(rows, T, T <= 148 ? (N / 8 + 31) / 32 * 32 : 128, 0, stream, static_cast<__nv_bfloat16*>(d_hidden_out),
                   static_cast<__nv_bfloat16*>(d_normed_out), d_partials, split_k, static_cast<const __nv_bfloat16*>(d_residual),
                   static_cast<const __nv_bfloat16*>(d_norm_weight), T, N, eps, normed_xt_tile);
     return 0;
@@ -759,7 +829,7 @@ int vb_reduce_residual_rmsnorm(void* d_hidden_out, void* d_normed_out, const flo
   int parts = 1;
   // widest cluster (<= 8, the portable limit) that divides the row into float4-aligned parts; few rows -> more parts (past some 512 CTAs a
   // split row costs more than it gives)
-  const int want = T <= 64 ? 8 : (T <= 128 ? 4 : (T <= 192 ? 2 : 1));
+  const int want = T <= 64 ? 8 : (T <= 128 ? 4 : (T <= 192 ? 2 : 1));          // (wide or unaligned rows)
   for (int c = want; c >= 1; c >>= 1)
     if (N % (4 * c) == 0) { parts = c; break; }
   while (N / parts > RR_THREADS * 4 * RR_MAX_ITER) {

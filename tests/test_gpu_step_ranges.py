@@ -1148,27 +1148,27 @@ def test_reduce_residual_rmsnorm_rows(ops, T, N, S, resid, tiled):
     assert ((y.double() - ref).abs() <= ref.abs() * (2.0 ** -8 + 2.0 ** -13)).all()
 
 
-@pytest.mark.parametrize("T,n_q,n_kv,D,S", [(193, 14, 2, 64, 2), (256, 24, 8, 128, 3)])
-def test_qkv_rope_append_rows_from_193(ops, T, n_q, n_kv, D, S):
-    """193 to 256 rows against the same rows in steps of 192, which spread a row's heads: the same bits."""
+@pytest.mark.parametrize("T,n_q,n_kv,D,S,bias", [(1, 1, 1, 16, 1, False), (3, 24, 8, 128, 3, True), (33, 5, 1, 80, 4, False), (64, 14, 2, 64, 5, True), (256, 2, 2, 256, 8, False)])
+def test_qkv_rope_append_few_rows(ops, T, n_q, n_kv, D, S, bias):
+    """Up to 256 rows (a row's items over blocks, four planes at a time) against the same rows in a step of 300: the same bits; a row without a page is not stored."""
     g = torch.Generator("cuda").manual_seed(T)
-    page, W = 16, (n_q + 2 * n_kv) * D
-    parts = torch.randn(S, T, W, generator=g, device="cuda")
+    page, W, R = 16, (n_q + 2 * n_kv) * D, 300
+    parts = torch.randn(S, R, W, generator=g, device="cuda")
     freq = torch.rand(D, generator=g, device="cuda")
-    pos = torch.randint(0, 4000, (T,), generator=g, device="cuda", dtype=torch.int32)
-    row_page, row_slot = torch.arange(T, device="cuda", dtype=torch.int32) // page, torch.arange(T, device="cuda", dtype=torch.int32) % page
+    b = torch.randn(W, generator=g, device="cuda").to(torch.bfloat16) if bias else None
+    pos = torch.randint(0, 4000, (R,), generator=g, device="cuda", dtype=torch.int32)
+    row_page, row_slot = torch.arange(R, device="cuda", dtype=torch.int32) // page, torch.arange(R, device="cuda", dtype=torch.int32) % page
+    row_page[T // 2] = -1
 
-    def run(cuts):
-        kv, q = torch.zeros((T + page - 1) // page, 2, page, n_kv, D, device="cuda", dtype=torch.bfloat16), torch.zeros(T, n_q, D, device="cuda", dtype=torch.bfloat16)
-        for c in cuts:
-            p, n = parts[:, c].contiguous(), c.stop - c.start
-            at = [v[c].contiguous() for v in (pos, row_page, row_slot)]
-            ops.call("vb_qkv_rope_append", q[c].data_ptr(), kv.data_ptr(), p.data_ptr(), S, at[0].data_ptr(), freq.data_ptr(), at[1].data_ptr(), at[2].data_ptr(), n, n_q, n_kv, D,
-                     page, D, 0, None, None, 0.0, None, ops._stream())
-        return q, kv
+    def run(n):
+        kv, q = torch.zeros((R + page - 1) // page, 2, page, n_kv, D, device="cuda", dtype=torch.bfloat16), torch.zeros(R, n_q, D, device="cuda", dtype=torch.bfloat16)
+        p = parts[:, :n].contiguous()
+        ops.call("vb_qkv_rope_append", q.data_ptr(), kv.data_ptr(), p.data_ptr(), S, pos.data_ptr(), freq.data_ptr(), row_page.data_ptr(), row_slot.data_ptr(), n, n_q, n_kv, D,
+                 page, D, 0, None, None, 0.0, None if b is None else b.data_ptr(), ops._stream())
+        return q[:T], kv.transpose(1, 2).reshape(-1, 2, n_kv, D)[:T]
 
-    for a, b in zip(run([slice(0, T)]), run([slice(0, 192), slice(192, T)])):
-        assert torch.equal(a, b)
+    for a, want in zip(run(T), run(R)):
+        assert torch.equal(a, want)
 
 
 @pytest.mark.parametrize("T,n_q,n_kv,D,S,bias", [(257, 1, 1, 16, 1, False), (300, 24, 8, 128, 1, False), (258, 5, 1, 80, 3, True), (600, 2, 2, 256, 2, False)])

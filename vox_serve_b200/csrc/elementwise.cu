@@ -624,6 +624,38 @@ __global__ void __launch_bounds__(256) qkv_rope_append_kernel(
   trace_end(tr);
 }
 
+// 8 columns of a head and the 8 that turn with them, summed: bias, rounding, rotation (not of V), and their place; sm: cos | sin of the row
+__device__ __forceinline__ void qkv_rope_finish(float (&x)[2][8], const float* sm, int t, int h, int e, int D, int n_q, int n_kv, __nv_bfloat16* q_out, __nv_bfloat16* kd,
+                                                size_t slab, const __nv_bfloat16* qkv_bias) {
+  const int half = D >> 1, n = h * D + e;
+      uint32_t o[2][4];
+      float y[2][8];
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (qkv_bias) x[k][j] += __bfloat162float(qkv_bias[n + k * half + j]);
+          x[k][j] = round_bf16(x[k][j]);
+        }
+      const bool rot = h < n_q + n_kv;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        y[0][j] = rot ? x[0][j] * sm[e + j] + -x[1][j] * sm[D + e + j] : x[0][j];
+        y[1][j] = rot ? x[1][j] * sm[e + half + j] + x[0][j] * sm[D + e + half + j] : x[1][j];
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[k][j] = pack_bf16(y[k][2 * j], y[k][2 * j + 1]);
+      __nv_bfloat16* dst = nullptr;
+      if (h < n_q) dst = q_out + (static_cast<size_t>(t) * n_q + h) * D + e;
+      else if (kd) dst = kd + (h < n_q + n_kv ? (h - n_q) * D : slab + (h - n_q - n_kv) * D) + e;
+      if (dst) {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]);
+        *reinterpret_cast<uint4*>(dst + half) = make_uint4(o[1][0], o[1][1], o[1][2], o[1][3]);
+      }
+}
+
 // The tail for whole heads rotated in halves without norms, steps of many rows: a thread finishes 8 columns of a head and the 8 that
 // turn with them, straight from the planes (no shared-memory row, one barrier for the row's cos / sin), in 16-byte pieces.  1024 rows of 40 heads of 128: 21.5 -> 15.4 us.
 __global__ void __launch_bounds__(256) qkv_rope_rows_kernel(__nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ kv,
@@ -662,33 +694,79 @@ __global__ void __launch_bounds__(256) qkv_rope_rows_kernel(__nv_bfloat16* __res
         const float4 a = __ldcg(src), b = __ldcg(src + 1);
         x[k][0] += a.x; x[k][1] += a.y; x[k][2] += a.z; x[k][3] += a.w; x[k][4] += b.x; x[k][5] += b.y; x[k][6] += b.z; x[k][7] += b.w;
       }
-    uint32_t o[2][4];
-    float y[2][8];
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (qkv_bias) x[k][j] += __bfloat162float(qkv_bias[n + k * half + j]);
-        x[k][j] = round_bf16(x[k][j]);
-      }
-    const bool rot = h < n_q + n_kv;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      y[0][j] = rot ? x[0][j] * sm[e + j] + -x[1][j] * sm[D + e + j] : x[0][j];
-      y[1][j] = rot ? x[1][j] * sm[e + half + j] + x[0][j] * sm[D + e + half + j] : x[1][j];
-    }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) o[k][j] = pack_bf16(y[k][2 * j], y[k][2 * j + 1]);
-    __nv_bfloat16* dst = nullptr;
-    if (h < n_q) dst = q_out + (t * n_q + h) * D + e;
-    else if (kd) dst = kd + (h < n_q + n_kv ? (h - n_q) * D : slab + (h - n_q - n_kv) * D) + e;
-    if (dst) {
-      *reinterpret_cast<uint4*>(dst) = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]);
-      *reinterpret_cast<uint4*>(dst + half) = make_uint4(o[1][0], o[1][1], o[1][2], o[1][3]);
-    }
+    qkv_rope_finish(x, sm, static_cast<int>(t), h, e, D, n_q, n_kv, q_out, kd, slab, qkv_bias);
   }
+}
+
+// ... and steps of few rows: a row's items over blocks of 32 (128, of more than 64 rows), four planes in flight, and the row's angles in the shadow of their loads.
+__global__ void __launch_bounds__(128) qkv_rope_row_kernel(__nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ kv, const float* __restrict__ partials, int split_k,
+                                                           const int32_t* __restrict__ pos, const float* __restrict__ freq, const int32_t* __restrict__ row_page,
+                                                           const int32_t* __restrict__ row_slot, int T, int n_q, int n_kv, int D, int page_size,
+                                                           const __nv_bfloat16* __restrict__ qkv_bias) {
+  extern __shared__ float sm[];      // [D] cos, [D] sin
+  constexpr int PLANES = 3;          // beside the first
+  const size_t t = blockIdx.y;
+  const int n_heads = n_q + 2 * n_kv, half = D >> 1, per_head = half >> 3, W = n_heads * D, i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int h = i / per_head, e = (i - h * per_head) * 8;
+  const bool in = h < n_heads;
+  const size_t plane = static_cast<size_t>(T) * W;
+  const int tr = (threadIdx.x == 0 && trace_block0()) ? trace_begin(6, split_k) : -1;
+  pdl_sync();
+  const float* src = partials + t * W + h * D + e;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 a[2][2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) a[k][j] = in ? __ldcg(reinterpret_cast<const float4*>(src + k * half) + j) : zero;
+  const int at = pos[t], page = row_page[t], slot = row_slot[t];
+  for (int s0 = 1; s0 < split_k; s0 += PLANES) {
+    float4 b[PLANES][2][2];
+#pragma unroll
+    for (int s = 0; s < PLANES; ++s)
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          b[s][k][j] = in && s0 + s < split_k ? __ldcg(reinterpret_cast<const float4*>(src + (s0 + s) * plane + k * half) + j) : zero;
+    if (s0 == 1)
+      for (int d = threadIdx.x; d < D; d += blockDim.x) {
+        float sn, cs;
+        sincosf(static_cast<float>(at) * freq[d], &sn, &cs);
+        sm[d] = cs;
+        sm[D + d] = sn;
+      }
+#pragma unroll
+    for (int s = 0; s < PLANES; ++s)
+      if (s0 + s < split_k) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            a[k][j].x += b[s][k][j].x; a[k][j].y += b[s][k][j].y; a[k][j].z += b[s][k][j].z; a[k][j].w += b[s][k][j].w;
+          }
+      }
+  }
+  if (split_k == 1)
+    for (int d = threadIdx.x; d < D; d += blockDim.x) {
+      float sn, cs;
+      sincosf(static_cast<float>(at) * freq[d], &sn, &cs);
+      sm[d] = cs;
+      sm[D + d] = sn;
+    }
+  __syncthreads();
+  if (in) {
+    const size_t row_elems = static_cast<size_t>(n_kv) * D, slab = static_cast<size_t>(page_size) * row_elems;
+    __nv_bfloat16* kd = page >= 0 ? kv + static_cast<size_t>(page) * 2 * slab + static_cast<size_t>(slot) * row_elems : nullptr;
+    float x[2][8];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      x[k][0] = a[k][0].x; x[k][1] = a[k][0].y; x[k][2] = a[k][0].z; x[k][3] = a[k][0].w;
+      x[k][4] = a[k][1].x; x[k][5] = a[k][1].y; x[k][6] = a[k][1].z; x[k][7] = a[k][1].w;
+    }
+    qkv_rope_finish(x, sm, static_cast<int>(t), h, e, D, n_q, n_kv, q_out, kd, slab, qkv_bias);
+  }
+  trace_end(tr);
 }
 
 __global__ void embedding_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ table,
@@ -854,9 +932,18 @@ int vb_qkv_rope_append(void* d_q_out, void* d_layer_kv, const float* d_partials,
   if (T <= 0) return 0;
   const int n_heads = n_q + 2 * n_kv;
   auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
-  // (Behind the kernel that writes the planes, the kernel below / this one, us: 200 rows in four planes of 24 + 8 + 8 heads of 128 6.1 / 5.3, 32 + 8 + 8 of 64
-  // 5.8 / 3.8, 14 + 2 + 2 of 64 3.3 / 3.0, 16 + 8 + 8 of 128 4.6 / 4.0, 32 + 2 + 2 of 128 6.2 / 5.4; 133 rows 4.4 / 4.8, 4.0 / 3.3, 3.4 / 3.0, 4.0 / 3.3, 4.3 / 4.7.)
-  if (T > 192 && !interleave && rotary_dim == head_dim && head_dim % 16 == 0 && head_dim <= 256 && !d_q_norm && aligned(d_q_out) &&
+  // Whole heads in halves without norms: 256 items of 16 columns and more to a row (rows kernel) past 256 rows, before that a row's items over blocks (row kernel); the rest
+  // below.  us behind the kernel that writes the planes, below / row / rows kernel, 24 + 8 + 8 heads of 128: three planes of 1 row 3.1 / 2.4, of 32 3.3 / 2.8, four of 133 4.5 / 3.8 / 4.8,
+  // three of 256 6.6 / 4.8 / 4.9, one of 512 5.5 (row) / 5.2 (rows), of 1024 8.2 / 7.5; 32 + 8 + 8 of 64: 3.2 / 2.7, 3.2 / 2.7, 4.0 / 3.2 / 3.3, 6.0 / 3.3 / 3.4, 4.2 / 3.5, 5.4 / 5.1.
+  if (T <= 256 && !interleave && rotary_dim == head_dim && head_dim % 16 == 0 && head_dim <= 256 && !d_q_norm && aligned(d_q_out) && aligned(d_layer_kv) &&
+      aligned(d_partials)) {
+    const int rb = T <= 64 ? 32 : 128;          // (in a decode step of 32 rows, two layers: blocks of 32 / 64 / 128 193.2 / 193.9 / 194.6 us)
+    VB_LAUNCH_PDL(qkv_rope_row_kernel, dim3((n_heads * (head_dim / 16) + rb - 1) / rb, T), rb, 2 * head_dim * sizeof(float), stream, static_cast<__nv_bfloat16*>(d_q_out),
+                  static_cast<__nv_bfloat16*>(d_layer_kv), d_partials, split_k, d_pos, d_freq, d_row_page, d_row_slot, T, n_q, n_kv, head_dim,
+                  page_size, static_cast<const __nv_bfloat16*>(d_qkv_bias));
+    return 0;
+  }
+  if (T > 256 && !interleave && rotary_dim == head_dim && head_dim % 16 == 0 && head_dim <= 256 && !d_q_norm && aligned(d_q_out) &&
       aligned(d_layer_kv) && aligned(d_partials)) {
     VB_LAUNCH_PDL(qkv_rope_rows_kernel, T, 256, 2 * head_dim * sizeof(float), stream, static_cast<__nv_bfloat16*>(d_q_out),
                   static_cast<__nv_bfloat16*>(d_layer_kv), d_partials, split_k, d_pos, d_freq, d_row_page, d_row_slot, T, n_q, n_kv, head_dim,

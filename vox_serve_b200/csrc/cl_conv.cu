@@ -26,7 +26,8 @@
 // What bounds it (640 rows of 512 x 2048, split in four: 12.8 us, was 28.4; 5120 x 1536 x 1024: 60 us, was 161): the wide layers the bytes
 // through L2 and shared memory, 0.6 us for 64 channels and one tap of 128 x 128; the layers of many positions the epilogue's instructions,
 // some 50 for the 32 values of a warp (153600 x 128 with residual 61 us, was 71, 30 of DRAM time).
-// Measured (one pass): SNAC 32 windows 652 -> 532 us, 1 window 262 -> 242, Mimi 32 chunks 1926 -> 1262, the small kernels below among them.
+// Measured (one pass): SNAC 32 windows 652 -> 532 us, 1 window 262 -> 242, Mimi 32 chunks 1926 -> 1262, the small kernels below among them; with the fused units of
+// cl_unit.cu and the depthwise tiles by their time 487, 183 and 1089.
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 32
 #include "cl_common.cuh"

@@ -7,7 +7,7 @@
 // tokens, then from the tile of the first key that the CTA's first row sees; within a tile the mask is per key.  What lies between the two is
 // nobody's to read (a page table may name other requests' pages there, or unwritten ones): its boxes are skipped, its V rows cleared.
 // Measured (16 query heads on 4 key heads of 128, two prompts of 1001 rows in all): the three-layer prompt step around it 1058 us with
-// mma.sync, 884 here.
+// mma.sync, 884 here (724 with the steps around it since, 720 with a loading warp each for K and V).
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 1
 #include "attn_tc.cuh"

@@ -283,6 +283,9 @@ int vb_latest_window(int32_t* d_first, const int32_t* d_n_out, const int32_t* d_
 int vb_gather_windows(int64_t* d_windows, const int32_t* d_history, const int32_t* d_slot, const int32_t* d_first,
                       const int32_t* d_n_valid, int n, int history_cap, int window, void* stream);
 /* embedding gather: orpheus.py:408 */
+/* the rows and their norm (what vb_rmsnorm makes of them, in rows or XT(normed_xt_tile)) in one launch: dim a multiple of 8 up to 8192, 16-byte boundaries */
+int vb_embedding_rmsnorm(void* d_hidden, void* d_normed, const void* d_table, const int32_t* d_ids, const void* d_weight, int T, int dim, int vocab, float eps,
+                         int normed_xt_tile, void* stream);
 int vb_embedding(void* d_out, const void* d_table, const int32_t* d_ids, int T, int dim, int vocab, void* stream);
 /* Multi-codebook glue of the depth-transformer adapters (vox_serve/model/csm.py:158-168, 637-663, 700-701;
  * cuda_graph_worker.py:1058-1160 does these with torch ops and host indices between graph replays):

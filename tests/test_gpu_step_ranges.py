@@ -1148,6 +1148,18 @@ def test_reduce_residual_rmsnorm_rows(ops, T, N, S, resid, tiled):
     assert ((y.double() - ref).abs() <= ref.abs() * (2.0 ** -8 + 2.0 ** -13)).all()
 
 
+@pytest.mark.parametrize("T,dim,tiled", [(1, 8, False), (3, 2056, False), (65, 3072, True), (130, 8192, True), (2, 8200, False)])
+def test_embedding_rmsnorm(ops, T, dim, tiled):
+    """The same bits as the two launches; ids off the table's ends are taken to them; rows past 8192 columns take the two."""
+    g = torch.Generator("cuda").manual_seed(dim)
+    table, w = (torch.randn(n, dim, generator=g, device="cuda").to(torch.bfloat16) for n in (50, 1))
+    ids = torch.randint(-3, 53, (T,), generator=g, device="cuda", dtype=torch.int32)
+    hidden, normed = torch.empty(T, dim, device="cuda", dtype=torch.bfloat16), ops.TiledAct(T, dim, "cuda") if tiled else torch.empty(T, dim, device="cuda", dtype=torch.bfloat16)
+    ops.embedding_rmsnorm(table, ids, w[0], 1e-6, hidden, normed)
+    assert torch.equal(hidden, table[ids.clamp(0, 49).long()])
+    assert torch.equal(normed.to_rows() if tiled else normed, ops.rmsnorm(hidden, w[0], 1e-6))
+
+
 @pytest.mark.parametrize("T,n_q,n_kv,D,S,bias", [(1, 1, 1, 16, 1, False), (3, 24, 8, 128, 3, True), (33, 5, 1, 80, 4, False), (64, 14, 2, 64, 5, True), (256, 2, 2, 256, 8, False)])
 def test_qkv_rope_append_few_rows(ops, T, n_q, n_kv, D, S, bias):
     """Up to 256 rows (a row's items over blocks, four planes at a time) against the same rows in a step of 300: the same bits; a row without a page is not stored."""

@@ -20,6 +20,7 @@ SIGNATURES = {
     "vb_device_info": (c_int, [P, P]),
     "vb_tensor_map_kv": (c_int, [P, P, c_int64, c_int, c_int, c_int, c_int]),
     "vb_tensor_map_2d_bf16": (c_int, [P, P, c_int64, c_int64, c_int64, c_int]),
+    "vb_embedding_rmsnorm": (c_int, [P, P, P, P, P, c_int, c_int, c_int, c_float, c_int, P]),
     "vb_rmsnorm": (c_int, [P, P, P, c_int, c_int, c_float, c_int, P]),
     "vb_rope_freqs": (c_int, [P, c_int, c_int, c_float, c_float, c_int, c_float, c_float, c_float, P]),
     "vb_rope": (c_int, [P, P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P]),

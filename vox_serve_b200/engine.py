@@ -267,16 +267,18 @@ class LlamaEngine:
         if R > self.max_rows:
             raise VoxB200Error(f"{R} rows exceed the engine's max_rows {self.max_rows}")
         hidden, normed = self.hidden[:R], self.normed[:R]
-        if input_ids is not None:
+        fused = R <= self.FUSED_MAX_ROWS and self.fused_ok and not self.force_unfused
+        first = input_ids if input_ids is not None and not fused and input_ids.numel() == R else None      # (its rows come with their norm)
+        if input_ids is not None and first is None:
             ops.embedding(w.embed, input_ids, out=hidden)
         x_final = normed
-        if R <= self.FUSED_MAX_ROWS and self.fused_ok and not self.force_unfused:
+        if fused:
             self._layers_fused(position_ids, R, plan)
             if last_rows is None and self.tiled_acts:
                 x_final = self.normed_t.view_rows(R)
             ops.rmsnorm(hidden, w.norm, d.rms_norm_eps, out=x_final)
         else:
-            x_final = self._layers_unfused(position_ids, R, plan)
+            x_final = self._layers_unfused(position_ids, R, plan, first)
         if last_rows is not None:
             n_out = last_rows.numel() if n_out is None else n_out
             if isinstance(x_final, ops.TiledAct):      # a gather needs rows: those of the stream, then their norm
@@ -334,10 +336,10 @@ class LlamaEngine:
             ops.proj_residual(act_x, L["down"], hidden, self.fsplit_down, hidden_out=hidden, ssq_out=ssq,
                               hidden_tiles_out=hidden_t)
 
-    def _layers_unfused(self, position_ids: torch.Tensor, R: int, plan: ops.RowPlan):
+    def _layers_unfused(self, position_ids: torch.Tensor, R: int, plan: ops.RowPlan, input_ids: Optional[torch.Tensor] = None):
         """8 launches per layer.  Activations travel between kernels in the tiled layout (the attention output only in
         decode-sized steps and only with VB_ATTN_TILED=1); returns what holds the final normed rows (a TiledAct then,
-        else self.normed[:R])."""
+        else self.normed[:R]).  input_ids: the embedding rows are still to be fetched."""
         d, w = self.dims, self.w
         hq, hkv, D, H, I = d.num_attention_heads, d.num_key_value_heads, d.head_dim, d.hidden_size, d.intermediate_size
         hidden = self.hidden[:R]
@@ -346,7 +348,10 @@ class LlamaEngine:
         attn_tiled = tiled and self.attn_tiled and R <= self.FUSED_MAX_ROWS
         attn_o = self.attn_t.view_rows(R) if attn_tiled else self.attn[:R]
         act = self.act_t.view_rows(R) if tiled else self.act[:R]
-        ops.rmsnorm(hidden, w.layers[0]["ln1"], d.rms_norm_eps, out=normed)
+        if input_ids is None:
+            ops.rmsnorm(hidden, w.layers[0]["ln1"], d.rms_norm_eps, out=normed)
+        else:
+            ops.embedding_rmsnorm(w.embed, input_ids, w.layers[0]["ln1"], d.rms_norm_eps, hidden, normed)
         s_qkv, s_o, s_dn = self._splits(R)
         q = self.q[:R]
         n_layers = len(w.layers)

@@ -767,6 +767,21 @@ def embedding(table: torch.Tensor, ids: torch.Tensor, out: Optional[torch.Tensor
     return out
 
 
+def embedding_rmsnorm(table: torch.Tensor, ids: torch.Tensor, weight: torch.Tensor, eps: float, hidden: torch.Tensor, normed) -> None:
+    """``embedding`` into ``hidden`` [T, dim] and ``rmsnorm`` of it into ``normed`` (rows or a TiledAct), in one launch where the rows allow it (the same bits)."""
+    T, dim = ids.numel(), table.shape[1]
+    tiled = isinstance(normed, TiledAct)
+    out = normed.data if tiled else normed
+    if dim % 8 or dim > 8192 or any(t.data_ptr() % 16 for t in (table, weight, hidden, out)):
+        rmsnorm(embedding(table, ids, out=hidden), weight, eps, out=normed)
+        return
+    _need_cuda(table, ids, weight)
+    assert ids.dtype == torch.int32 and table.dtype == BF16 and weight.dtype == BF16 and hidden.is_contiguous() and hidden.shape == (T, dim)
+    assert (normed.T == T and normed.K == dim) if tiled else (normed.is_contiguous() and normed.shape == (T, dim))
+    call("vb_embedding_rmsnorm", hidden.data_ptr(), out.data_ptr(), table.data_ptr(), ids.data_ptr(), weight.data_ptr(), T, dim, table.shape[0], float(eps),
+         normed.t_tile if tiled else 0, _stream())
+
+
 def multi_embed_sum(out: torch.Tensor, ids: torch.Tensor, table_a: Optional[torch.Tensor], col_offset: int = 0,
                     col0: int = 0, n_cols_a: Optional[int] = None, table_b: Optional[torch.Tensor] = None,
                     mask: Optional[torch.Tensor] = None, round_each: bool = False) -> torch.Tensor:

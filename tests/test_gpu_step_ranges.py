@@ -1148,6 +1148,50 @@ def test_reduce_residual_rmsnorm_rows(ops, T, N, S, resid, tiled):
     assert ((y.double() - ref).abs() <= ref.abs() * (2.0 ** -8 + 2.0 ** -13)).all()
 
 
+def _squares(h, parts):
+    """Sums of the rows' squares in 32 bits, in order: with ``parts`` blocks to a row a thread takes 4 columns of every 1024 of its part, with 0 a lane 8 of every 256."""
+    T, N = h.shape
+    tree = lambda v: v[..., 0] if v.shape[-1] == 1 else tree(v[..., :v.shape[-1] // 2] + v[..., v.shape[-1] // 2:])          # noqa: E731
+    pad = lambda v, n: torch.nn.functional.pad(v, (0, -v.shape[-1] % n))                                                     # noqa: E731
+    if parts == 0:
+        v = pad(h, 256).view(T, -1, 32, 4, 2)
+        v = v[..., 0] * v[..., 0] + v[..., 1] * v[..., 1]              # (squares of bf16 values are exact)
+        ss = torch.zeros(T, 32, device=h.device)
+        for g in range(v.shape[1]):
+            for j in range(4):
+                ss = ss + v[:, g, :, j]
+        return tree(ss)
+    v = pad(h.view(T, parts, N // parts), 1024).view(T, parts, -1, 256, 4)
+    ss = torch.zeros(T, parts, 256, device=h.device)
+    for g in range(v.shape[2]):
+        for j in range(4):
+            ss = ss + v[:, :, g, :, j] * v[:, :, g, :, j]
+    ss, total = tree(tree(ss.view(T, parts, 8, 32))), torch.zeros(T, device=h.device)
+    for p in range(parts):
+        total = total + ss[:, p]
+    return total
+
+
+@pytest.mark.parametrize("T", [1, 33, 64, 65, 128, 129, 148, 149, 192, 193, 512, 513, 1000])
+@pytest.mark.parametrize("N", [8, 264, 1032, 2048, 3072, 4096])
+def test_reduce_residual_rmsnorm_order_of_squares(ops, T, N):
+    """The bits of the norm: a row's squares are added in one order for a number of rows, which rows off the 16-byte boundaries (another kernel) have as well."""
+    g = torch.Generator("cuda").manual_seed(T + N)
+    parts, w = torch.randn(3, T, N, generator=g, device="cuda"), torch.randn(N, generator=g, device="cuda").to(torch.bfloat16)
+    res = torch.randn(T * N + 8, generator=g, device="cuda").to(torch.bfloat16)
+    shifted = res.roll(4)[4:4 + T * N].view(T, N)                      # (8 bytes off)
+    res = res[:T * N].view(T, N)
+    assert torch.equal(res, shifted) and shifted.data_ptr() % 16 == 8
+    h, y = ops.reduce_residual_rmsnorm(parts, res, w, 1e-6)
+    split = next(c for c in (8, 4, 2, 1) if c <= (8 if T <= 64 else 4 if T <= 128 else 2 if T <= 192 else 1) and N % (4 * c) == 0)
+    total = _squares(h.float(), 0 if T > 512 else split)
+    rcp = torch.rsqrt(total / torch.full_like(total, N) + 1e-6)[:, None]
+    assert torch.equal(y, (h.float() * rcp * w.float()).to(torch.bfloat16))
+    if T <= 512:
+        for a, b in zip((h, y), ops.reduce_residual_rmsnorm(parts, shifted, w, 1e-6)):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("T,dim,tiled", [(1, 8, False), (3, 2056, False), (65, 3072, True), (130, 8192, True), (2, 8200, False)])
 def test_embedding_rmsnorm(ops, T, dim, tiled):
     """The same bits as the two launches; ids off the table's ends are taken to them; rows past 8192 columns take the two."""

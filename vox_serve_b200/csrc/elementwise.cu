@@ -381,16 +381,81 @@ __global__ void __launch_bounds__(RR_THREADS) reduce_residual_rmsnorm_kernel(
   trace_end(tr);
 }
 
+// The kernels below add a row's squares in the order in which the one above does with `parts` CTAs to a row -- a thread 4 columns of every 1024 of its part, a warp's
+// threads and a CTA's warps pairwise, the CTAs one after the other -- so a row has the same bits whichever of them it comes to, aligned or not.  Steps of more than 512
+// rows (parts == RR_WARP) add 8 columns of every 256 to a lane, as a warp to a row has done for them.
+// A thread here holds 8 neighbouring columns: two threads there, 16 lanes a warp.  Where parts are whole warps the sums stay in registers (0.3 us of a launch more than in
+// the threads' own order); else they are taken from the row in shared memory (0.9 us more).
+constexpr int RR_WARP = 0;
+__device__ __forceinline__ void rr_squares(float (&ss)[2], const uint4& h) {          // of two threads there
+  const uint32_t w[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float a = bf16_lo(w[j]), b = bf16_hi(w[j]);
+    ss[j >> 1] += a * a;
+    ss[j >> 1] += b * b;
+  }
+}
+__device__ __forceinline__ float rr_half_warp(float (&ss)[2]) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
+    ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+    ss[1] += __shfl_xor_sync(0xffffffffu, ss[1], o);
+  }
+  return ss[0] + ss[1];
+}
+// red[2 * part + ..]: a part's eight warps, of which `used` have something; a lane a part
+__device__ __forceinline__ float rr_total(const float4* red, int parts, int used) {
+  const int lane = threadIdx.x & 7;
+  const float4 a = red[2 * lane], b = red[2 * lane + 1];
+  float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int i = 1; i < 8; ++i)
+    if (i >= used) w[i] = 0.f;
+  const float sum = ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+  float total = 0.f;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const float part = __shfl_sync(0xffffffffu, sum, r);
+    if (r < parts) total += part;
+  }
+  return total;
+}
+// the row in shared memory; what all threads wrote of it before is seen
+__device__ __noinline__ float rr_from_row(const uint4* row, float4* red4, int N, int parts) {
+  float* red = reinterpret_cast<float*>(red4);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  __syncthreads();
+  const int quads = N / (4 * parts), used = min(8, (quads + 31) >> 5);          // of a part: groups of 4 columns, warps that have some
+  const uint2* q = reinterpret_cast<const uint2*>(row);
+  for (int i = warp; i < parts * used; i += warps) {
+    const int part = i / used, w = i - part * used;
+    float ss = 0.f;
+    for (int c = w * 32 + lane; c < quads; c += RR_THREADS) {
+      const uint2 v = q[part * quads + c];
+      const float h[4] = {bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y)};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ss += h[j] * h[j];
+    }
+    ss = warp_sum(ss);
+    if (lane == 0) red[part * 8 + w] = ss;
+  }
+  __syncthreads();
+  return rr_total(red4, parts, used);
+}
+
 // The same for steps of more rows than there are SMs: 128 threads to a row, G groups of 8 columns each.  A row is one chain of a load, a sum over it and a store, so
-// every load of a plane is in flight at once, the norm's weights before the kernel in front has ended, behind one barrier (for the sum of squares).
-// us behind the kernel that writes the planes, before (a warp to a row past 512 rows, else a CTA or a cluster) / now: 1024 rows of 1024 columns 4.1 / 2.6,
-// 2048 6.7 / 3.7, 3072 9.0 / 5.2, 4096 11.0 / 6.5; three planes of 512 rows 4.7 / 2.9, 6.1 / 4.0, 7.8 / 5.0, 9.9 / 6.3.  Three groups held to 80 registers spill:
-// four planes of 133 rows of 3072 6.0 for 3.6.
+// every load of a plane is in flight at once, the norm's weights before the kernel in front has ended, behind a barrier or two (for the sum of squares).
+// us behind the kernel that writes the planes, before (a warp to a row past 512 rows, else a CTA or a cluster) / now: 1024 rows of 1024 columns 4.1 / 2.7,
+// 2048 6.7 / 3.9, 3072 8.9 / 5.6, 4096 10.9 / 6.9; three planes of 512 rows 4.7 / 3.1, 6.1 / 3.9, 8.1 / 5.5, 9.8 / 6.5.  Three groups held to 80 registers spilled
+// when all planes of a row were loaded at once: four planes of 133 rows of 3072 6.0 for 3.6.
 template <int G>
 __global__ void __launch_bounds__(128, G <= 2 ? 8 : 5) reduce_residual_rmsnorm_rows_kernel(
     __nv_bfloat16* __restrict__ hidden_out, __nv_bfloat16* __restrict__ normed_out, const float* __restrict__ partials, int split_k,
-    const __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ norm_w, int T, int N, float eps, int xt_tile) {
-  __shared__ float part[4];
+    const __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ norm_w, int T, int N, float eps, int xt_tile, int parts) {
+  __shared__ uint4 kept[G * 128];
+  __shared__ float4 red4[16];
+  float* red = reinterpret_cast<float*>(red4);
   const int t = blockIdx.x, c0 = threadIdx.x * 8;
   const size_t plane = static_cast<size_t>(T) * N, row = static_cast<size_t>(t) * N;
   uint4 w4[G], r[G], h[G];
@@ -433,13 +498,18 @@ __global__ void __launch_bounds__(128, G <= 2 ? 8 : 5) reduce_residual_rmsnorm_r
         a[g][k].x += b[g][k].x; a[g][k].y += b[g][k].y; a[g][k].z += b[g][k].z; a[g][k].w += b[g][k].w;
       }
   }
-  float ss = 0.f;
+  // (one or two parts: where the second begins, and whether the sums can stay in the threads)
+  const int split = parts == 2 ? N / 2 : N;
+  const bool whole = parts == 1 || (parts == 2 && split % 128 == 0);
+  float ss[2] = {}, first[2] = {};
+  bool second = false;
 #pragma unroll
   for (int g = 0; g < G; ++g) {
     const int n = g * 1024 + c0;
     const float x[8] = {a[g][0].x, a[g][0].y, a[g][0].z, a[g][0].w, a[g][1].x, a[g][1].y, a[g][1].z, a[g][1].w};
     const uint32_t rr[4] = {r[g].x, r[g].y, r[g].z, r[g].w};
     uint32_t o[4];
+    float two[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       float u = round_bf16(x[2 * j]), v = round_bf16(x[2 * j + 1]);
@@ -448,16 +518,58 @@ __global__ void __launch_bounds__(128, G <= 2 ? 8 : 5) reduce_residual_rmsnorm_r
         v = round_bf16(bf16_hi(rr[j]) + v);
       }
       o[j] = pack_bf16(u, v);
-      ss += u * u + v * v;
+      two[j] = u * u + v * v;
     }
     h[g] = make_uint4(o[0], o[1], o[2], o[3]);
+    if (whole) {
+      if (!second && n >= split) {
+        second = true;
+        first[0] = ss[0]; first[1] = ss[1];
+        ss[0] = ss[1] = 0.f;
+      }
+      rr_squares(ss, h[g]);
+    } else {
+      kept[g * 128 + threadIdx.x] = parts != RR_WARP ? h[g]
+                                                     : make_uint4(__float_as_uint(two[0]), __float_as_uint(two[1]), __float_as_uint(two[2]), __float_as_uint(two[3]));
+    }
     if (hidden_out && n < N) *reinterpret_cast<uint4*>(hidden_out + row + n) = h[g];
   }
   if (!normed_out) return;
-  ss = warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  const float rcp = rsqrtf((part[0] + part[1] + part[2] + part[3]) / static_cast<float>(N) + eps);
+  float total;
+  if (parts == RR_WARP) {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4 * G; ++i) {
+        if (i * 256 < N) {          // (columns past the row are zeros)
+          const float4 t = reinterpret_cast<const float4*>(kept)[i * 32 + threadIdx.x];
+          sum = sum + t.x + t.y + t.z + t.w;
+        }
+      }
+      sum = warp_sum(sum);
+      if (threadIdx.x == 0) red[0] = sum;
+    }
+    __syncthreads();
+    total = red[0];
+  } else if (whole) {
+    const int w = threadIdx.x >> 4;
+    if (second) {
+      const float t = ss[0], u = ss[1];
+      ss[0] = first[0]; ss[1] = first[1];
+      first[0] = t; first[1] = u;
+    }
+    const float a0 = rr_half_warp(ss), a1 = parts == 2 ? rr_half_warp(first) : 0.f;
+    if ((threadIdx.x & 15) == 0) {
+      red[w] = a0;
+      if (parts == 2) red[8 + ((w - (split >> 7)) & 7)] = a1;
+    }
+    __syncthreads();
+    total = rr_total(red4, parts, 8);
+  } else {
+    total = rr_from_row(kept, red4, N, parts);
+  }
+  const float rcp = rsqrtf(total / static_cast<float>(N) + eps);
 #pragma unroll
   for (int g = 0; g < G; ++g) {
     const int n = g * 1024 + c0;
@@ -473,17 +585,24 @@ __global__ void __launch_bounds__(128, G <= 2 ? 8 : 5) reduce_residual_rmsnorm_r
 }
 
 // The same for steps of few rows: a thread to every 8 columns of a row and eight planes in flight, one barrier.  us behind the kernel that writes the planes, a cluster of
-// 8 CTAs to a row (its launch and its meeting) / now: eight planes of 1, 8, 32 and 64 rows of 3072 columns 4.1 / 3.0, 4.3 / 3.2, 4.5 / 3.2, 8.5 / 3.5; four 3.3 / 2.6, 3.5 / 2.8, 3.7 / 3.0,
-// 6.5 / 2.9; eight of 32 rows of 1024 columns 4.2 / 2.7, of 4096 4.2 / 3.8.
+// 8 CTAs to a row (its launch and its meeting) / now: eight planes of 1, 32 and 64 rows of 3072 columns 4.4 / 3.5, 4.6 / 3.7, 8.7 / 3.8; four 3.5 / 3.0, 3.6 / 3.1 of 1 and 32;
+// eight of 32 rows of 1024 columns 4.2 / 2.9, of 4096 4.2 / 4.2.
 constexpr int RW_PLANES = 7;        // beside the first
 __global__ void __launch_bounds__(512) reduce_residual_rmsnorm_row_kernel(
     __nv_bfloat16* __restrict__ hidden_out, __nv_bfloat16* __restrict__ normed_out, const float* __restrict__ partials, int split_k,
-    const __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ norm_w, int T, int N, float eps, int xt_tile) {
-  __shared__ float part[16];
+    const __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ norm_w, int T, int N, float eps, int xt_tile, int parts) {
+  __shared__ uint4 kept[512];
+  __shared__ float4 red4[16];
+  float* red = reinterpret_cast<float*>(red4);
+  float2* chain = reinterpret_cast<float2*>(kept);
   const int t = blockIdx.x, n = threadIdx.x * 8;
   const bool in = n < N;
   const size_t plane = static_cast<size_t>(T) * N, row = static_cast<size_t>(t) * N;
   const int tr = (threadIdx.x == 0 && trace_block0()) ? trace_begin(5, split_k) : -1;
+  // where the thread's columns are with `parts` parts: which part, its groups of 4 columns before them, and whether the chain of squares comes from a thread 1024 columns in front
+  // and goes on in one behind
+  const int quads = N / (4 * parts), part = 2 * threadIdx.x / quads, at = 2 * threadIdx.x - part * quads;
+  const bool whole = quads % 32 == 0, from = at >= RR_THREADS, on = at + RR_THREADS < quads;
   const uint4 w4 = normed_out && in ? __ldg(reinterpret_cast<const uint4*>(norm_w + n)) : make_uint4(0u, 0u, 0u, 0u);
   pdl_sync();
   const float4* src = reinterpret_cast<const float4*>(partials + row + n);
@@ -505,7 +624,6 @@ __global__ void __launch_bounds__(512) reduce_residual_rmsnorm_row_kernel(
         }
       }
   }
-  float ss = 0.f;
   const float x[8] = {a[0].x, a[0].y, a[0].z, a[0].w, a[1].x, a[1].y, a[1].z, a[1].w};
   const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
   uint32_t h[4];
@@ -517,15 +635,31 @@ __global__ void __launch_bounds__(512) reduce_residual_rmsnorm_row_kernel(
       v = round_bf16(bf16_hi(rr[j]) + v);
     }
     h[j] = pack_bf16(u, v);
-    ss += u * u + v * v;
   }
   if (hidden_out && in) *reinterpret_cast<uint4*>(hidden_out + row + n) = make_uint4(h[0], h[1], h[2], h[3]);
   if (!normed_out) { trace_end(tr); return; }
-  ss = warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  float total = 0.f;
-  for (int i = 0; i < static_cast<int>(blockDim.x >> 5); ++i) total += part[i];
+  const uint4 h4 = make_uint4(h[0], h[1], h[2], h[3]);
+  float total;
+  if (whole) {
+    float ss[2] = {};
+    if (!from) rr_squares(ss, h4);
+    if (quads > RR_THREADS) {
+      if (!from && on && in) chain[threadIdx.x] = make_float2(ss[0], ss[1]);
+      __syncthreads();
+      if (from && in) {
+        const float2 before = chain[threadIdx.x - RR_THREADS / 2];
+        ss[0] = before.x; ss[1] = before.y;
+        rr_squares(ss, h4);
+      }
+    }
+    const float sum = rr_half_warp(ss);
+    if ((threadIdx.x & 15) == 0 && in && !on) red[part * 8 + ((at & (RR_THREADS - 1)) >> 5)] = sum;
+    __syncthreads();
+    total = rr_total(red4, parts, min(8, quads >> 5));
+  } else {
+    kept[threadIdx.x] = h4;
+    total = rr_from_row(kept, red4, N, parts);
+  }
   const float rcp = rsqrtf(total / static_cast<float>(N) + eps);
   if (in) {
     const uint32_t wv[4] = {w4.x, w4.y, w4.z, w4.w};
@@ -901,9 +1035,15 @@ int vb_reduce_residual_rmsnorm(void* d_hidden_out, void* d_normed_out, const flo
   VB_CHECK_ARG(!d_normed_out || d_norm_weight, "vb_reduce_residual_rmsnorm: norm output needs a weight");
   if (T <= 0) return 0;
   auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
+  // widest cluster (<= 8, the portable limit) that divides the row into float4-aligned parts; few rows -> more parts (past some 512 CTAs a
+  // split row costs more than it gives)
+  int parts = 1;
+  const int want = T <= 64 ? 8 : (T <= 128 ? 4 : (T <= 192 ? 2 : 1));
+  for (int c = want; c >= 1; c >>= 1)
+    if (N % (4 * c) == 0) { parts = c; break; }
   if (N % 8 == 0 && N <= 4096 && aligned(d_partials) && aligned(d_hidden_out) && aligned(d_normed_out) && aligned(d_residual) && aligned(d_norm_weight)) {
-    // (a thread to 8 columns, of which an SM holds one row / 128 threads to a row, us: four planes of 133 rows of 2048, 3072, 4096 columns 2.7 / 3.2, 3.1 / 3.5, 3.3 / 4.0, of
-    // 256 rows 3.2 / 3.3, 4.9 / 3.9, 5.7 / 4.7; one of 1024 4.4 / 3.7, 6.1 / 5.0, 8.5 / 6.4)
+    // (a thread to 8 columns, of which an SM holds one row / 128 threads to a row, us: four planes of 133 rows of 2048, 3072, 4096 columns 2.9 / 3.5, 3.5 / 3.9, 3.7 / 5.0, of
+    // 256 rows 3.5 / 3.7, 5.7 / 4.2, 6.3 / 5.6)
     const auto rows = T <= 148   ? reduce_residual_rmsnorm_row_kernel
                       : N <= 1024 ? reduce_residual_rmsnorm_rows_kernel<1>
                       : N <= 2048 ? reduce_residual_rmsnorm_rows_kernel<2>
@@ -911,15 +1051,9 @@ int vb_reduce_residual_rmsnorm(void* d_hidden_out, void* d_normed_out, const flo
                                   : reduce_residual_rmsnorm_rows_kernel<4>;
     VB_LAUNCH_PDL(rows, T, T <= 148 ? (N / 8 + 31) / 32 * 32 : 128, 0, stream, static_cast<__nv_bfloat16*>(d_hidden_out),
                   static_cast<__nv_bfloat16*>(d_normed_out), d_partials, split_k, static_cast<const __nv_bfloat16*>(d_residual),
-                  static_cast<const __nv_bfloat16*>(d_norm_weight), T, N, eps, normed_xt_tile);
+                  static_cast<const __nv_bfloat16*>(d_norm_weight), T, N, eps, normed_xt_tile, T > 512 ? RR_WARP : parts);
     return 0;
   }
-  int parts = 1;
-  // widest cluster (<= 8, the portable limit) that divides the row into float4-aligned parts; few rows -> more parts (past some 512 CTAs a
-  // split row costs more than it gives)
-  const int want = T <= 64 ? 8 : (T <= 128 ? 4 : (T <= 192 ? 2 : 1));          // (wide or unaligned rows)
-  for (int c = want; c >= 1; c >>= 1)
-    if (N % (4 * c) == 0) { parts = c; break; }
   while (N / parts > RR_THREADS * 4 * RR_MAX_ITER) {
     VB_CHECK_ARG(parts < 8 && N % (8 * parts) == 0, "vb_reduce_residual_rmsnorm: N %d too wide", N);
     parts *= 2;

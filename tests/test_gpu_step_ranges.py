@@ -1104,6 +1104,28 @@ def test_paged_attention_runs_of_rows(ops, page, hq, hkv, D):
         _close(out, want, 2.0 ** -8)               # weights rounded to bf16, then the result: 2^-9 each at most
 
 
+@pytest.mark.parametrize("page,hkv,D", [(16, 2, 64), (16, 2, 128), (16, 4, 64), (32, 1, 128)])
+def test_paged_attention_bits_whatever_the_runs(ops, page, hkv, D):
+    """A head's result does not depend on how the cache rows were copied: with twelve heads to a key head they come singly, with four by fours."""
+    g, B = torch.Generator("cuda").manual_seed(page + D), 600
+    lens = torch.randint(1, 40 * page, (B,), generator=g, device="cuda").tolist()
+    pages = [(n + page - 1) // page for n in lens]
+    kv = torch.randn(sum(pages), 2, page, hkv, D, generator=g, device="cuda").to(torch.bfloat16)
+    q = torch.randn(B, hkv, 12, D, generator=g, device="cuda").to(torch.bfloat16)
+    indptr = [sum(pages[:i]) for i in range(B + 1)]
+    chunk = ops.attn_chunk_tokens(page, hkv)
+    plan = ops.plan_rows(ops.RowPlan(B, "cuda"), None, _i32(indptr), _i32(list(range(sum(pages)))), _i32([(n - 1) % page + 1 for n in lens]), B, B, page, chunk)
+
+    def run(q):
+        hq = q.shape[1] * q.shape[2]
+        ws = ops.paged_attn_workspace(B, None, hq, hkv, D, "cuda")
+        return ops.paged_attn(q.reshape(B, hq, D).contiguous(), kv, 0, plan, B, hkv, page, chunk, ws, grid_ctas=100).view(B, hkv, -1, D)
+
+    whole = run(q)
+    for first in (0, 4, 8):
+        assert torch.equal(run(q[:, :, first:first + 4]), whole[:, :, first:first + 4])
+
+
 @pytest.mark.parametrize("hq,hkv,D", [(32, 2, 64), (16, 2, 128), (16, 1, 64), (24, 8, 128)])
 def test_paged_attention_many_short_rows(ops, hq, hkv, D):
     """Rows of a tile or less behind one another in a CTA: every row with its own Q, however often (the next row's came too early now and then)."""

@@ -51,7 +51,7 @@ struct AttnParams {
   float* part_o;                 // [grid * 2][n_q][D]
   int slab_base;
   int n_rows, n_q, n_kv, G, page_size, tok, stages;
-  int run_log2;                  // token rows per copy: 1, 2 or 4
+  int run_log2;                  // token rows per copy: 1, 2 or 4 (RUN_L of the kernel)
   int out_xt_tile;               // 0: out is [row][n_q][D]; else the tiled XT(out_xt_tile) layout of [row][n_q * D]
   float scale_log2;
 };
@@ -113,7 +113,8 @@ struct AttnLayout {
 
 // MINB = CTAs per SM the register allocation is sized for: 1 -> up to 168 registers, no spills (deep ring, the SM to
 // itself); 2 -> 96 registers (some spills) so that a second CTA -- this kernel's or a neighbouring kernel's -- fits.
-template <int D, bool HI, int MINB>
+// RUN_L: the cache's token rows come 1 << RUN_L a copy (1, 2 or 4).
+template <int D, bool HI, int MINB, int RUN_L>
 __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams p) {
   constexpr int KS = D / 16;            // k-steps of K Q^T
   constexpr int MT = D / 16;            // m-tiles of V^T P^T
@@ -121,11 +122,11 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
   const int G = p.G, TOK = p.tok, STAGES = p.stages;
-  const AttnLayout L(D, TOK, p.n_kv, p.n_q, G, STAGES, p.n_rows, p.run_log2);
+  const AttnLayout L(D, TOK, p.n_kv, p.n_q, G, STAGES, p.n_rows, RUN_L);
   const int NW = p.n_kv * (TOK / 16);   // consumer warps
   const int NC = NW * 32;
   const int ROWB = p.n_kv * D * 2;      // bytes of one token row (all heads) in the cache
-  const int RUN_L = p.run_log2, RUNB = ROWB << RUN_L, RS = RUNB + 16;   // a run of rows, one copy, and its stride in shared memory (16-byte skew)
+  const int RUNB = ROWB << RUN_L, RS = RUNB + 16;   // a run of rows, one copy, and its stride in shared memory (16-byte skew)
   TileMeta* meta = reinterpret_cast<TileMeta*>(smem + L.off_meta);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.off_bar);
   uint64_t* empty = full + ATTN_MAX_STAGES;
@@ -257,8 +258,9 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
             }
             __syncwarp();
             uint8_t* dst = smem + stage * L.stage_bytes;
-            for (int t = lane; t << RUN_L < TOK; t += 32)
-              bulk_copy_g2s_hint(dst + t * RS, src0 + kvsel * page_elems + static_cast<size_t>(t << RUN_L) * p.n_kv * D, RUNB,
+            // (the run as the launch says it: with RUN_L here the loop of 64 requests of 1024 tokens, 32 heads on 2 of 128 in pages of 16, took 82 us for 60)
+            for (int t = lane; t << p.run_log2 < TOK; t += 32)
+              bulk_copy_g2s_hint(dst + t * RS, src0 + kvsel * page_elems + static_cast<size_t>(t << p.run_log2) * p.n_kv * D, RUNB,
                                  &full[stage], pol_kv);
             __syncwarp();
             if (++stage == STAGES) { stage = 0; ph ^= 1; }
@@ -297,6 +299,16 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
     const int rest = r >> (4 - RUN_L), step = 8 >> (4 - RUN_L);       // (of 16 >> RUN_L runs)
     return RUN_L == 0 ? h * 8 + r : ((r & ((16 >> RUN_L) - 1)) << RUN_L) + rest + h * step;
   };
+  // The weights of a slab are added in one order, whatever its runs: a lane adds those of tokens j and j + 8 and keeps the sum over its tiles, and at the end lanes meet by
+  // the bits of j, lowest first.  (The products over 16 tokens give the same bits in any order.)  Dealt in runs, j and j + 8 lie in partners' lanes, of which the upper keeps what
+  // its second half has: by twos token 2 r + h is in row r of half h, by fours 4 (r & 3) + (r >> 2) + 2 h.  Two shuffles a column tile, not seen in the times below.
+  const int partner = RUN_L == 1 ? 16 : 8;
+  const bool upper = lane & partner;
+  auto pair_sum = [&](float lo, float hi) {
+    if (RUN_L == 0) return lo + hi;
+    return (upper ? hi : lo) + __shfl_xor_sync(0xffffffffu, upper ? lo : hi, partner);
+  };
+  const int meet[3] = {RUN_L == 0 ? 4 : 16, RUN_L == 1 ? 4 : 8, RUN_L == 0 ? 16 : RUN_L == 1 ? 8 : 4};
   auto row_at = [&](int h, int r) { const int t = slab * 16 + tok_of(h, r); return (t >> RUN_L) * RS + (t & ((1 << RUN_L) - 1)) * ROWB; };
   const int k_at = row_at(mi & 1, r8) + hoff + (mi >> 1) * 16, v_at = row_at(mi >> 1, r8) + hoff + (mi & 1) * 16;
   const int t_lo = slab * 16 + tok_of(0, g), t_hi = slab * 16 + tok_of(1, g);
@@ -387,8 +399,8 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
       mrun[nt][0] = n0; mrun[nt][1] = n1;
       const float p0 = round_bf16(ex2_approx(s0 - u0)), p1 = round_bf16(ex2_approx(s1 - u1));
       const float p2 = round_bf16(ex2_approx(s2 - u0)), p3 = round_bf16(ex2_approx(s3 - u1));
-      lrun[nt][0] = lrun[nt][0] * alpha[nt][0] + (p0 + p2);
-      lrun[nt][1] = lrun[nt][1] * alpha[nt][1] + (p1 + p3);
+      lrun[nt][0] = lrun[nt][0] * alpha[nt][0] + pair_sum(p0, p2);
+      lrun[nt][1] = lrun[nt][1] * alpha[nt][1] + pair_sum(p1, p3);
       // C layout (token g | g+8, heads 2qd, 2qd+1) -> B layout (tokens 2qd, 2qd+1 | +8, head g)
       pb[nt][0] = movmatrix_trans(pack_bf16(p0, p1));
       pb[nt][1] = movmatrix_trans(pack_bf16(p2, p3));
@@ -426,9 +438,9 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-      for (int o = 4; o < 32; o <<= 1) {
-        lrun[nt][0] += __shfl_xor_sync(0xffffffffu, lrun[nt][0], o);
-        lrun[nt][1] += __shfl_xor_sync(0xffffffffu, lrun[nt][1], o);
+      for (int i = 0; i < 3; ++i) {
+        lrun[nt][0] += __shfl_xor_sync(0xffffffffu, lrun[nt][0], meet[i]);
+        lrun[nt][1] += __shfl_xor_sync(0xffffffffu, lrun[nt][1], meet[i]);
       }
     if (TOK == 16) {
       // ---- one slab per tile: this warp owns its kv head outright, no block-level step at all ----
@@ -644,16 +656,23 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
   trace_end(tr);
 }
 
-template <int D, bool HI, int MINB>
+template <int D, bool HI, int MINB, int RUN_L>
 static int launch_attn(const AttnParams& p, int grid, cudaStream_t stream) {
-  const AttnLayout L(D, p.tok, p.n_kv, p.n_q, p.G, p.stages, p.n_rows, p.run_log2);
+  const AttnLayout L(D, p.tok, p.n_kv, p.n_q, p.G, p.stages, p.n_rows, RUN_L);
   VB_CHECK_ARG(L.total <= VB_MAX_DYN_SMEM, "vb_paged_attn: %d rows / %d-token tiles need %d bytes of shared memory",
                p.n_rows, p.tok, L.total);
-  auto kern = paged_attn_kernel<D, HI, MINB>;
+  auto kern = paged_attn_kernel<D, HI, MINB, RUN_L>;
   VB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, VB_MAX_DYN_SMEM));
   const int threads = (p.n_kv * (p.tok / 16) + 1) * 32;
   VB_LAUNCH_PDL(kern, grid, threads, L.total, stream, p);
   return 0;
+}
+template <int D, int MINB>
+static int launch_attn_runs(const AttnParams& p, int grid, cudaStream_t stream) {
+  const int run_log2 = p.run_log2;
+  if (p.G <= 8) return run_log2 == 1 ? launch_attn<D, false, MINB, 1>(p, grid, stream) : launch_attn<D, false, MINB, 2>(p, grid, stream);
+  if (run_log2 == 0) return launch_attn<D, true, MINB, 0>(p, grid, stream);          // (of more than eight heads to a key head only)
+  return run_log2 == 1 ? launch_attn<D, true, MINB, 1>(p, grid, stream) : launch_attn<D, true, MINB, 2>(p, grid, stream);
 }
 
 }  // namespace vb
@@ -719,7 +738,7 @@ int vb_paged_attn(void* d_out, const void* d_q, const void* d_kv, int64_t slab_b
   // 61 / 64, 14 on 2 of 64 (256 B) 46 / 34 / 32 / 33.  Where two warps work off a tile of small rows with two column tiles each, their own chain is the limit and single
   // rows are no slower: 32 on 2 of 128 in pages of 16 60 / 88 / 89, 24 on 2 86 / 85 / 86.
   const int row_bytes = n_kv * head_dim * 2;
-  p.run_log2 = p.G > 8 && p.tok * row_bytes < 16384 ? 0 : row_bytes >= 2048 ? 1 : 2;
+  const int run_log2 = p.run_log2 = p.G > 8 && p.tok * row_bytes < 16384 ? 0 : row_bytes >= 2048 ? 1 : 2;
   p.out_xt_tile = out_xt_tile;
   p.scale_log2 = sm_scale * 1.4426950408889634f;
   // deepest ring of half-stages that fits the budget next to the fixed buffers.  Measured on B200 (28 launches back to
@@ -734,19 +753,14 @@ int vb_paged_attn(void* d_out, const void* d_q, const void* d_kv, int64_t slab_b
     budget = (kb >= 64 && kb <= 227 ? kb : 224) * 1024;
   }
   int stages = ATTN_MAX_STAGES;
-  while (stages > 2 && AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows, p.run_log2).total > budget) --stages;
-  VB_CHECK_ARG(AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows, p.run_log2).total <= VB_MAX_DYN_SMEM,
+  while (stages > 2 && AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows, run_log2).total > budget) --stages;
+  VB_CHECK_ARG(AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows, run_log2).total <= VB_MAX_DYN_SMEM,
                "vb_paged_attn: %d rows need more shared memory than an SM has", n_rows);
   p.stages = stages;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const bool hi = p.G > 8;
-  const bool two = 2 * (AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows, p.run_log2).total + 1024) <= 232448;
-  if (two) {
-    if (head_dim == 128) return hi ? launch_attn<128, true, 2>(p, grid_ctas, st) : launch_attn<128, false, 2>(p, grid_ctas, st);
-    return hi ? launch_attn<64, true, 2>(p, grid_ctas, st) : launch_attn<64, false, 2>(p, grid_ctas, st);
-  }
-  if (head_dim == 128) return hi ? launch_attn<128, true, 1>(p, grid_ctas, st) : launch_attn<128, false, 1>(p, grid_ctas, st);
-  return hi ? launch_attn<64, true, 1>(p, grid_ctas, st) : launch_attn<64, false, 1>(p, grid_ctas, st);
+  const bool two = 2 * (AttnLayout(head_dim, p.tok, n_kv, n_q, p.G, stages, n_rows, run_log2).total + 1024) <= 232448;
+  if (two) return head_dim == 128 ? launch_attn_runs<128, 2>(p, grid_ctas, st) : launch_attn_runs<64, 2>(p, grid_ctas, st);
+  return head_dim == 128 ? launch_attn_runs<128, 1>(p, grid_ctas, st) : launch_attn_runs<64, 1>(p, grid_ctas, st);
 }
 
 }  // extern "C"

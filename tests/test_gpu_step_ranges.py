@@ -720,6 +720,70 @@ def test_channels_last_tail(B, T, kind):
     assert _lib.load().vb_cl_timeouts() == 0
 
 
+def _tail_weights(g):
+    """weights of the end of Mimi's decoder, as it keeps them"""
+    from vox_serve_b200.tokenizer import _cl
+
+    rnd = lambda *s, std=1.0: torch.randn(*s, generator=g, device="cuda") * std          # noqa: E731
+    w1, b1, w3, b3 = rnd(32, 64, 3, std=192 ** -0.5), rnd(32, std=0.05), rnd(64, 32, std=0.5 * 32 ** -0.5), rnd(64, std=0.05)
+    return _cl.pack_conv(w1.reshape(32, -1), 64, 3), b1, _cl.pack(w3), b3, rnd(1, 192, std=0.5 * 192 ** -0.5), rnd(1, std=0.01)
+
+
+@pytest.mark.parametrize("where", [0, 60, 122, 130, 379])
+def test_channels_last_tail_beside_a_loud_value(where):
+    """Positions that a loud value is not part of keep their bits, in its tile and in its warp."""
+    from vox_serve_b200.tokenizer import _cl
+
+    g, T = torch.Generator(device="cuda").manual_seed(where), 380
+    w, x = _tail_weights(g), torch.randn(2, T, 64, generator=g, device="cuda")
+    run = lambda: _cl.res_tail(_cl.Act(x.clone().view(-1), 2, T, 64), *w).view(2, T)     # noqa: E731
+    plain = run()
+    x[1, where, 7] = 1e6
+    got = run()
+    far = torch.ones(2, T, dtype=torch.bool, device="cuda")
+    far[1, where:where + 5] = False              # (two taps, two taps)
+    assert torch.equal(got[far], plain[far]) and not torch.equal(got[~far], plain[~far])
+
+
+@pytest.mark.parametrize("kind", ["plain", "one", "one a tile", "silence", "quiet", "loud"])
+def test_channels_last_tail_is_no_slower_than_its_convolutions(kind):
+    """One launch against a launch a convolution, whatever its inputs are: what parts cannot hold is a warp's work and not a lane's (0.3 to 0.6 of their time; once 14 times)."""
+    from vox_serve_b200.tokenizer import _cl
+
+    B, T = 8, 9600
+    g = torch.Generator(device="cuda").manual_seed(1)
+    (w1, b1, w3, b3, wl, bl), x = _tail_weights(g), torch.randn(B, T, 64, generator=g, device="cuda")
+    if kind == "one":
+        x[0, T // 2, 3] = 1e6
+    elif kind == "one a tile":
+        x[:, 50::124, 3] = 1e6
+    elif kind == "silence":
+        x[:, T // 2:T // 2 + 240] *= 1e-9
+    elif kind != "plain":
+        x *= 1e-9 if kind == "quiet" else 1e5
+    X = _cl.Act(x.view(-1), B, T, 64)
+    xp = _cl.conv(X, _cl.pack(torch.eye(64, device="cuda")), 64, act="elu", out="parts")
+
+    def launches():
+        h = _cl.conv(xp, w1, 32, b1, ksize=3, act="elu", out="parts")
+        return _cl.last_conv(_cl.conv(h, w3, 64, b3, epi="resid", resid=X, act="elu"), wl, bl, 3, 2, 0, T, tanh=False)
+
+    def us(f):
+        times = []
+        for _ in range(6):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            for _ in range(4):
+                f()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b) * 250)
+        return min(times)
+
+    one, three = us(lambda: _cl.res_tail(X, w1, b1, w3, b3, wl, bl)), us(launches)
+    assert one <= 1.5 * three, (one, three)
+
+
 @pytest.mark.parametrize("B,T,C,ksize,left,lo,hi", [(1, 1, 64, 3, 2, 0, 1), (2, 129, 96, 3, 2, 0, 129), (3, 40, 4, 3, 0, 5, 38), (1, 300, 256, 7, 3, 1, 300), (2, 17, 68, 5, 4, 0, 17),
                                                    (1, 130, 128, 16, 15, 0, 130), (2, 16, 32, 1, 0, 0, 16)])
 def test_channels_last_one_output_channel(B, T, C, ksize, left, lo, hi):

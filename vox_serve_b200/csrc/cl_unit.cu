@@ -597,8 +597,11 @@ static CuDwPlan cu_dw_plan(int C, int dil, long long range, long long B, int sms
 // residual), three taps of products, ELU of the hidden channels as parts, products, ELU and the taps of the last convolution.  The next tile comes
 // while the second half runs.  Nothing but x is read and nothing but the samples is written; two groups run into the gaps of one another.
 // What bounds it: instructions, some 12,000 of a warp's a tile (the ELUs more than half) at 45 % of the issue slots, two groups of one SM waiting for products
-// between their steps.  32 x 19,200 positions: 127 us, before as three launches 88 + 113 + 60, and the convolution in front writes its result once
+// between their steps.  32 x 19,200 positions: 117 us (125 with x in local memory, where a call for it had put it), before as three launches 88 + 113 + 60, and the convolution in front writes its result once
 // (111 -> 70 us).  With x kept in shared memory and fetched between tiles 143.
+// What parts cannot hold is multiplied in fp32 by warps, a lane a channel.  32 x 19,200 positions with one such value in all 128 us, one in every tile 455, one every 16
+// positions 556, 10 ms of silence an entry 248, nothing but silence 1340, nothing but loud values 1820; in three launches 283, 884, 1600, 350, 2340 and 3070.  (With a lane
+// for all 6144 products of its position 814, 12800, 13000, 1220, 8950 and 10100.)
 constexpr int CT_C = 64, CT_H = 32, CT_TAPS = 3, CT_ROWS = 128, CT_OUT = CT_ROWS - 2 * (CT_TAPS - 1), CT_PAD = 8;
 constexpr int CT_GROUPS = 2, CT_GROUP_THREADS = 256, CT_THREADS = CT_GROUPS * CT_GROUP_THREADS;
 constexpr int CT_X = CT_ROWS * 256, CT_OP1 = 2 * (CT_PAD + CT_ROWS) * 128, CT_OP2 = CT_ROWS * 128, CT_GROUP_BYTES = CT_OP1 + CT_OP2;
@@ -652,68 +655,126 @@ __device__ __forceinline__ float ct_value(uint32_t row, int r, int c, bool raw) 
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(lo) : "r"(a ^ 64u));
   return fmaf(__half2float(__ushort_as_half(lo)), 1.f / CL_LO_SCALE, __half2float(__ushort_as_half(hi)));
 }
-// The hidden channels of a thread's position once more where its inputs or they themselves may not be parts: in fp32 if an input is not, and kept as
-// what the whole block of 32 says.  All lanes load, those that `redo` names store.
-__device__ __noinline__ bool ct_hidden(const CtTables& tb, int group, int row, int first, uint32_t op1, uint32_t w1, uint32_t op2, uint32_t d, bool redo) {
-  float v[CT_H];
+// The hidden channels of a thread's position once more where they may not be parts, kept as what the whole block of 32 says (whether that is fp32).  All lanes
+// load, those that `redo` names store.
+__device__ __noinline__ bool ct_hidden(const CtTables& tb, int row, uint32_t op2, uint32_t d, bool redo) {
+  F2 v[CT_H / 2];
+  float m = 0.f;
+#pragma unroll
   for (int c = 0; c < CT_H; c += 8) {
     uint32_t hi[8], lo[8];
     tmem_ld_32x8(d + c, hi);
     tmem_ld_32x8(d + CT_H + c, lo);
     tmem_ld_wait();
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      v[c + i] = fmaf(fmaf(__uint_as_float(lo[i]), 1.f / CL_LO_SCALE, __uint_as_float(hi[i])), tb.inv1[c + i], tb.b1[c + i]);
+    for (int i = 0; i < 8; i += 2) {
+      float a[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) a[k] = fmaf(fmaf(__uint_as_float(lo[i + k]), 1.f / CL_LO_SCALE, __uint_as_float(hi[i + k])), tb.inv1[c + i + k], tb.b1[c + i + k]);
+      v[(c + i) >> 1] = cl_elu(f2(a[0], a[1]));
+      const float2 e = f2_get(v[(c + i) >> 1]);
+      m = max3_abs(m, e.x, e.y);
+    }
   }
   if (!redo) return false;
-  bool exact = false;
-  for (int j = 0; j < CT_TAPS; ++j) exact |= tb.raw1[group][0][CT_PAD + row - 2 + j] | tb.raw1[group][1][CT_PAD + row - 2 + j];
-  float m = 0.f;
+  const uint32_t o = op2 + row * 128;
+  if (cl_code(m) != CB_RAW) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) ct_put16(o, row & 7, 2 * c, reinterpret_cast<const F2(&)[8]>(v[8 * c]));
+    return false;
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const float2 x = f2_get(v[2 * c]), y = f2_get(v[2 * c + 1]);
+    ct_sts4(o + ((c ^ (row & 7)) << 4), __float_as_uint(x.x), __float_as_uint(x.y), __float_as_uint(y.x), __float_as_uint(y.y));
+  }
+  return true;
+}
+// eight inputs, 8 q and on, of row n of weights in shared memory
+__device__ __forceinline__ void ct_weights(uint32_t row, int n, int q, float scale, float (&f)[8]) {
+  const float4 hi = ct_lds4(row + ((q ^ (n & 7)) << 4)), lo = ct_lds4(row + (((q + 4) ^ (n & 7)) << 4));
+  const float h[4] = {hi.x, hi.y, hi.z, hi.w}, l[4] = {lo.x, lo.y, lo.z, lo.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 fh = unpack_f16(__float_as_uint(h[i])), fl = unpack_f16(__float_as_uint(l[i]));
+    f[2 * i] = fmaf(fl.x, 1.f / CL_LO_SCALE, fh.x) * scale;
+    f[2 * i + 1] = fmaf(fl.y, 1.f / CL_LO_SCALE, fh.y) * scale;
+  }
+}
+// The hidden channels in fp32 of the positions row0 + i that `mask` names, those with inputs that are not parts: a lane a channel, four positions at a time, their inputs
+// a lane each going round by shuffles.
+__device__ __noinline__ void ct_hidden_exact(CtTables& tb, int group, int row0, uint32_t mask, int first, uint32_t op1, uint32_t w1, uint32_t op2) {
+  const int lane = threadIdx.x & 31;
+  const float scale = tb.inv1[lane] * CL_X_SCALE;
 #pragma unroll 1
-  for (int n = 0; n < CT_H; ++n) {
-    float a = v[n];
-    if (exact) {
-      a = 0.f;
+  while (mask) {
+    int row[4];
+    float acc[4] = {};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      row[c] = mask ? row0 + __ffs(mask) - 1 : -CT_PAD;
+      mask &= mask - 1u;
+    }
 #pragma unroll 1
-      for (int j = 0; j < CT_TAPS; ++j) {
-        const int r = CT_PAD + row - 2 + j;
-        if (r < first) continue;           // (in front of the entry)
+    for (int j = 0; j < CT_TAPS; ++j) {
 #pragma unroll 1
-        for (int b = 0; b < 2; ++b) {
+      for (int b = 0; b < 2; ++b) {
+        float x[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int r = CT_PAD + row[c] - 2 + j;
+          x[c] = 0.f;
+          if (row[c] < 0 || r < first) continue;           // (none, or in front of the entry)
           const bool raw = tb.raw1[group][b][r];
-          const uint32_t x = op1 + b * (CT_OP1 / 2) + r * 128, w = w1 + (j * 2 + b) * 2 * CT_H * 128 + n * 128;
+          x[c] = ct_value(op1 + b * (CT_OP1 / 2) + r * 128, r, lane, raw) * (raw ? 1.f : 1.f / CL_X_SCALE);
+        }
 #pragma unroll 1
-          for (int k = 0; k < 32; ++k)
-            a = fmaf(ct_value(x, r, k, raw) * (raw ? 1.f : 1.f / CL_X_SCALE), ct_value(w, n, k, false) * (tb.inv1[n] * CL_X_SCALE), a);
+        for (int q = 0; q < 4; ++q) {
+          float f[8];
+          ct_weights(w1 + (j * 2 + b) * 2 * CT_H * 128 + lane * 128, lane, q, scale, f);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (row[c] < 0 || CT_PAD + row[c] - 2 + j < first) continue;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[c] = fmaf(__shfl_sync(0xffffffffu, x[c], 8 * q + k), f[k], acc[c]);
+          }
         }
       }
-      a += tb.b1[n];
     }
-    a = f2_get(cl_elu(f2(a, a))).x;
-    v[n] = a;
-    m = max3_abs(m, a, a);
-  }
-  const bool raw = cl_code(m) == CB_RAW;
-  const uint32_t o = op2 + row * 128;
-  for (int c = 0; c < 8; ++c) {
-    uint32_t q[4];
-    for (int i = 0; i < 4; ++i) {
-      if (raw) {
-        q[i] = __float_as_uint(v[4 * c + i]);
-      } else {
-        const int at = (c & 3) * 8 + 2 * i;
-        uint32_t hi, lo;
-        cl_parts(f2(v[at], v[at + 1]), CL_X_SCALE, hi, lo);
-        q[i] = c < 4 ? hi : lo;
-      }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (row[c] < 0) continue;
+      const float a = acc[c] + tb.b1[lane];
+      int word;
+      uint32_t bits;
+      const uint32_t code = cl_odd_row(f2_get(cl_elu(f2(a, a))).x, word, bits);
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(op2 + row[c] * 128 + (((word >> 2) ^ (row[c] & 7)) << 4) + (word & 3) * 4), "r"(bits) : "memory");
+      if (lane == 0) tb.raw2[group][row[c]] = code == CB_RAW;
     }
-    ct_sts4(o + ((c ^ (row & 7)) << 4), q[0], q[1], q[2], q[3]);
   }
-  return raw;
 }
-// the last step for a warp some of whose positions have hidden channels that are not parts
+// What a tile has of either kind: a thread's position, or sixteen of the warp's
+__device__ __noinline__ void ct_odd(CtTables& tb, int group, int row, int half, int first, uint32_t op1, uint32_t w1, uint32_t op2, uint32_t d) {
+  const int lane = threadIdx.x & 31, row0 = (row & ~31) + half * 16;
+  auto exact = [&](int r) {
+    bool any = false;
+    for (int j = r >= 2 ? 0 : CT_TAPS; j < CT_TAPS; ++j)          // (nothing is made of rows 0 and 1)
+      any |= tb.raw1[group][0][CT_PAD + r - 2 + j] || tb.raw1[group][1][CT_PAD + r - 2 + j];
+    return any;
+  };
+  if (half == 0) {
+    const bool mine = !exact(row), raw = ct_hidden(tb, row, op2, d, mine && row >= 2 && (tb.odd[group][0][row] || tb.odd[group][1][row]));
+    if (mine) tb.raw2[group][row] = raw;
+  }
+  const uint32_t mask = __ballot_sync(0xffffffffu, lane < 16 && exact(row0 + (lane & 15)));
+  if (mask) ct_hidden_exact(tb, group, row0, mask, first, op1, w1, op2);
+}
+// The last step for a warp some of whose positions have hidden channels that are not parts (`raw`): their channels in fp32, a lane a channel, before the sums that the others
+// go through as well
 __device__ __noinline__ void ct_last(const CtTables& tb, int row, int half, const F2 (&x)[16], uint32_t w3, uint32_t op2, uint32_t d, bool raw, float (&s)[CT_TAPS]) {
+  const int lane = threadIdx.x & 31, n = half * 32 + lane;
   float v[32];
+#pragma unroll
   for (int c = 0; c < 32; c += 8) {
     uint32_t hi[8], lo[8];
     tmem_ld_32x8(d + c, hi);
@@ -723,21 +784,45 @@ __device__ __noinline__ void ct_last(const CtTables& tb, int row, int half, cons
     for (int i = 0; i < 8; ++i)
       v[c + i] = fmaf(fmaf(__uint_as_float(lo[i]), 1.f / CL_LO_SCALE, __uint_as_float(hi[i])), tb.inv3[half * 32 + c + i], tb.b3[half * 32 + c + i]);
   }
+  const float scale = tb.inv3[n] * CL_X_SCALE;
 #pragma unroll 1
-  for (int c = 0; c < 32; ++c) {
-    const int n = half * 32 + c;
-    float a = v[c];
-    if (raw) {
-      a = 0.f;
+  for (uint32_t mask = __ballot_sync(0xffffffffu, raw); mask; mask &= mask - 1u) {
+    const int p = __ffs(mask) - 1, at = (row & ~31) + p;
+    float a = 0.f;
 #pragma unroll 1
-      for (int k = 0; k < CT_H; ++k) a = fmaf(ct_value(op2 + row * 128, row, k, true), ct_value(w3 + n * 128, n, k, false) * (tb.inv3[n] * CL_X_SCALE), a);
-      a += tb.b3[n];
-    }
-    const float2 res = f2_get(x[c >> 1]);
-    a += c & 1 ? res.y : res.x;
-    a = f2_get(cl_elu(f2(a, a))).x;
+    for (int q = 0; q < 4; ++q) {
+      float f[8];
+      ct_weights(w3 + n * 128, n, q, scale, f);
+      const float4 h0 = ct_lds4(op2 + at * 128 + (((2 * q) ^ (at & 7)) << 4)), h1 = ct_lds4(op2 + at * 128 + (((2 * q + 1) ^ (at & 7)) << 4));
+      const float h[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
 #pragma unroll
-    for (int j = 0; j < CT_TAPS; ++j) s[j] = fmaf(tb.wl[j][n], a, s[j]);
+      for (int k = 0; k < 8; ++k) a = fmaf(h[k], f[k], a);
+    }
+    a += tb.b3[n];
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+      const float t = __shfl_sync(0xffffffffu, a, c);
+      if (lane == p) v[c] = t;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    F2 sum[CT_TAPS] = {f2(0.f), f2(0.f), f2(0.f)};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int c = q * 16 + 2 * i;
+      const F2 y = cl_elu(f2_add(f2(v[c], v[c + 1]), x[8 * q + i]));
+#pragma unroll
+      for (int j = 0; j < CT_TAPS; ++j) {
+        const float2 g = *reinterpret_cast<const float2*>(tb.wl[j] + half * 32 + c);
+        sum[j] = f2_fma(y, f2(g.x, g.y), sum[j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < CT_TAPS; ++j) {
+      const float2 e = f2_get(sum[j]);
+      s[j] += e.x + e.y;
+    }
   }
 }
 
@@ -892,14 +977,10 @@ __global__ void __launch_bounds__(CT_THREADS, 1) cl_res_tail_kernel(const __grid
     tc_fence_before();
     const bool odd = meet(odd1 || !cl_fits(m));
     if (odd) {
-      if (half == 0) {
-        tc_fence_after();
-        bool redo = tb.odd[group][0][row] || tb.odd[group][1][row];
-        for (int j = row < 2 ? 2 - row : 0; j < CT_TAPS; ++j) redo |= tb.raw1[group][0][CT_PAD + row - 2 + j] || tb.raw1[group][1][CT_PAD + row - 2 + j];
-        tb.raw2[group][row] = ct_hidden(tb, group, row, CT_PAD - t0, op1, w1, op2, d1 + lanes, redo && row >= 2);
-        fence_proxy_async();
-        tc_fence_before();
-      }
+      tc_fence_after();
+      ct_odd(tb, group, row, half, CT_PAD - t0, op1, w1, op2, d1 + lanes);
+      fence_proxy_async();
+      tc_fence_before();
       meet(false);
     }
     if (warp == 0) {
@@ -954,7 +1035,13 @@ __global__ void __launch_bounds__(CT_THREADS, 1) cl_res_tail_kernel(const __grid
         }
       }
     } else {
-      ct_last(tb, row, half, x, w3, op2, d3 + lanes + half * 32, tb.raw2[group][row], s);
+      F2 kept[16];          // (of its own: what a call is given the address of lives in memory, everywhere)
+      float sums[CT_TAPS] = {};
+#pragma unroll
+      for (int i = 0; i < 16; ++i) kept[i] = x[i];
+      ct_last(tb, row, half, kept, w3, op2, d3 + lanes + half * 32, tb.raw2[group][row], sums);
+#pragma unroll
+      for (int j = 0; j < CT_TAPS; ++j) s[j] = sums[j];
     }
 #pragma unroll
     for (int j = 0; j < CT_TAPS; ++j) tb.sums[group][half][j][row] = t0 + row < 0 ? 0.f : s[j];

@@ -121,55 +121,51 @@ __device__ __forceinline__ void cu_chunks(const CuOut& o, uint32_t taddr, int co
 // The inputs of a product as they lie in shared memory: [block of 32 channels][row][128 bytes, swizzled], parts or (a bit in the row's word) fp32
 struct CuOperand {
   uint32_t at;               // first row of the first block
-  int blk_bytes, blocks, ksize, skip;       // (rows below `skip` lie in front of the entry)
+  int blk_bytes, blocks;
   const uint32_t* raw;
 };
 // The products of four columns that `mask` names again in fp32, for this warp's 32 channels, into the accumulators (plain scale; the columns that are
-// not named in the plain scale as well): cl_exact_chunk of cl_conv.cu with the inputs in shared memory, in the same order.
+// not named in the plain scale as well): cl_exact_chunk of cl_conv.cu for one tap with the inputs in shared memory, in the same order.
 __device__ __noinline__ void cu_exact_chunk(const CuOperand& x, const uint8_t* w, float w_scale, int lane_row, int c0, uint32_t mask, uint32_t t_hi, uint32_t t_lo,
                                             float inv) {
   const int lane = threadIdx.x & 31, sw = lane_row & 7;
   float acc[4] = {};
 #pragma unroll 1
-  for (int tap = 0; tap < x.ksize && mask; ++tap) {
+  for (int blk = 0; blk < x.blocks && mask; ++blk) {
+    float v[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int r = c0 + c;
+      v[c] = 0.f;
+      if (!(mask >> c & 1u)) continue;
+      const uint32_t row = x.at + blk * x.blk_bytes + r * 128;
+      if (x.raw[r] >> blk & 1u) {
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[c]) : "r"(row + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4));
+      } else {
+        const uint32_t a = row + (((lane >> 3) ^ (r & 7)) << 4) + (lane & 7) * 2;
+        uint16_t hi, lo;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hi) : "r"(a));
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(lo) : "r"(a ^ 64u));
+        v[c] = fmaf(__half2float(__ushort_as_half(lo)), 1.f / CL_LO_SCALE, __half2float(__ushort_as_half(hi))) * (1.f / CL_X_SCALE);
+      }
+    }
+    const uint8_t* wb = w + static_cast<size_t>(blk) * CL_W_BLOCK + lane_row * 128;
 #pragma unroll 1
-    for (int blk = 0; blk < x.blocks; ++blk) {
-      float v[4];
+    for (int q = 0; q < 4; ++q) {
+      const uint4 hi = __ldg(reinterpret_cast<const uint4*>(wb + ((q ^ sw) << 4))), lo = __ldg(reinterpret_cast<const uint4*>(wb + (((q + 4) ^ sw) << 4)));
+      const uint32_t h[4] = {hi.x, hi.y, hi.z, hi.w}, l[4] = {lo.x, lo.y, lo.z, lo.w};
+      float f[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 fh = unpack_f16(h[i]), fl = unpack_f16(l[i]);
+        f[2 * i] = fmaf(fl.x, 1.f / CL_LO_SCALE, fh.x) * w_scale;
+        f[2 * i + 1] = fmaf(fl.y, 1.f / CL_LO_SCALE, fh.y) * w_scale;
+      }
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        const int r = c0 + c + tap;
-        v[c] = 0.f;
-        if (!(mask >> c & 1u) || r < x.skip) continue;
-        const uint32_t row = x.at + blk * x.blk_bytes + r * 128;
-        if (x.raw[r] >> blk & 1u) {
-          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[c]) : "r"(row + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4));
-        } else {
-          const uint32_t a = row + (((lane >> 3) ^ (r & 7)) << 4) + (lane & 7) * 2;
-          uint16_t hi, lo;
-          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hi) : "r"(a));
-          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(lo) : "r"(a ^ 64u));
-          v[c] = fmaf(__half2float(__ushort_as_half(lo)), 1.f / CL_LO_SCALE, __half2float(__ushort_as_half(hi))) * (1.f / CL_X_SCALE);
-        }
-      }
-      const uint8_t* wb = w + static_cast<size_t>(tap * x.blocks + blk) * CL_W_BLOCK + lane_row * 128;
-#pragma unroll 1
-      for (int q = 0; q < 4; ++q) {
-        const uint4 hi = __ldg(reinterpret_cast<const uint4*>(wb + ((q ^ sw) << 4))), lo = __ldg(reinterpret_cast<const uint4*>(wb + (((q + 4) ^ sw) << 4)));
-        const uint32_t h[4] = {hi.x, hi.y, hi.z, hi.w}, l[4] = {lo.x, lo.y, lo.z, lo.w};
-        float f[8];
+        if (!(mask >> c & 1u)) continue;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 fh = unpack_f16(h[i]), fl = unpack_f16(l[i]);
-          f[2 * i] = fmaf(fl.x, 1.f / CL_LO_SCALE, fh.x) * w_scale;
-          f[2 * i + 1] = fmaf(fl.y, 1.f / CL_LO_SCALE, fh.y) * w_scale;
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if (!(mask >> c & 1u)) continue;
-          if (c0 + c + tap < x.skip) continue;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) acc[c] = fmaf(__shfl_sync(0xffffffffu, v[c], 8 * q + k), f[k], acc[c]);
-        }
+        for (int k = 0; k < 8; ++k) acc[c] = fmaf(__shfl_sync(0xffffffffu, v[c], 8 * q + k), f[k], acc[c]);
       }
     }
   }
@@ -189,15 +185,10 @@ __device__ __noinline__ void cu_exact_chunk(const CuOperand& x, const uint8_t* w
 // ... all columns of a warp that are made of a row kept in fp32
 __device__ __noinline__ void cu_exact(const CuOperand& x, const uint8_t* w, const float* w_inv, int lane_row, int inside, int c_first, int c_step, uint32_t taddr,
                                       int cols, float inv) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll 1
   for (int c0 = c_first; c0 < inside; c0 += c_step) {
-    uint32_t mask = 0u;
-    for (int c = 0; c < CL_EC; ++c) {
-      uint32_t any = 0u;
-      for (int tap = 0; tap < x.ksize; ++tap)
-        if (c0 + c < inside && c0 + c + tap >= x.skip) any |= x.raw[c0 + c + tap];
-      mask |= any ? 1u << c : 0u;
-    }
+    const uint32_t mask = __ballot_sync(0xffffffffu, lane < CL_EC && c0 + lane < inside && x.raw[c0 + lane]);
 #pragma unroll 1
     for (int c = 0; c < CL_EC; c += 4)
       cu_exact_chunk(x, w, w_inv[lane_row] * CL_X_SCALE, lane_row, c0 + c, mask >> c & 15u, taddr + c0 + c, taddr + cols + c0 + c, inv);
@@ -518,7 +509,7 @@ __global__ void __launch_bounds__(32 * (P + 1), P == 9 ? 2 : 1) cl_dw_unit_kerne
     tc_fence_after();
     if (alive && some) {
       if (*any) {
-        const CuOperand x{smem_u32(smem), blk_bytes, 2 * p.chunks, 1, 0, raw};
+        const CuOperand x{smem_u32(smem), blk_bytes, 2 * p.chunks, raw};
         cu_exact(x, w, p.w_inv + m0, lane_row, inside, c_first, c_step, taddr, cols, inv);
         inv = 1.f;
       }

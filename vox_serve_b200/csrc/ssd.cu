@@ -448,17 +448,10 @@ __global__ void __launch_bounds__(256) ssd_tile_out_kernel(SsdParams p) {
 // decayed weights, the weighted x, the state) enters as two bf16 terms, its rounding and the remainder's, so that a product keeps
 // 16 bits of its mantissa.
 // ------------------------------------------------------------------------------------------------------------------
-// rows [0, L) x n columns of bf16 (16-byte pieces) into smem [64][ld], zeros below
+// rows [0, L) x n columns of bf16 (16-byte pieces) into smem [64][ld], zeros below; n up to 1024 (the launch's shared memory ends near 650)
 __device__ __forceinline__ void sd_stage(__nv_bfloat16* __restrict__ dst, int ld, const __nv_bfloat16* __restrict__ src, int ld_src, int n,
                                          int L) {
   const int v = n / 8, whole = 128 / v, r0 = threadIdx.x / v, c = (threadIdx.x - r0 * v) * 8;          // whole rows in step
-  if (whole == 0) {
-    for (int i = threadIdx.x; i < SD_ROWS * v; i += 128) {
-      const int r = i / v, e = (i - r * v) * 8;
-      *reinterpret_cast<uint4*>(dst + r * ld + e) = r < L ? *reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * ld_src + e) : make_uint4(0u, 0u, 0u, 0u);
-    }
-    return;
-  }
   if (r0 >= whole) return;
   for (int rb = r0; rb < SD_ROWS; rb += 4 * whole) {          // four pieces a thread in flight
     uint4 q[4];

@@ -720,6 +720,45 @@ def test_channels_last_tail(B, T, kind):
     assert _lib.load().vb_cl_timeouts() == 0
 
 
+def _us(f):
+    times = []
+    for _ in range(6):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        for _ in range(4):
+            f()
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b) * 250)
+    return min(times)
+
+
+@pytest.mark.parametrize("kind", ["plain", "zero", "one a tile", "silence", "quiet", "loud"])
+def test_channels_last_residual_unit_is_no_slower_than_its_convolutions(kind):
+    """One launch against the depthwise and the 1x1 convolution, whatever its inputs are (0.7 to 1.05 of their time; once 1.9 with loud values, 3 with zeros)."""
+    from vox_serve_b200.tokenizer import _cl
+
+    B, T, C, dil = 32, 6000, 64, 9
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rnd = lambda *s, std=1.0: torch.randn(*s, generator=g, device="cuda") * std          # noqa: E731
+    x, dw, w, b = rnd(B, T, C), rnd(7, C, std=7 ** -0.5), _cl.pack(rnd(C, C, std=C ** -0.5)), rnd(C, std=0.05)
+    db = torch.zeros(C, device="cuda") if kind in ("zero", "quiet", "silence") else rnd(C, std=0.05)
+    a = [torch.cat((v, 1.0 / (v + 1e-9))) for v in (0.5 + torch.rand(C, generator=g, device="cuda") for _ in range(2))]
+    if kind == "one a tile":
+        x[:, 50::124, 3] = 1e6
+    elif kind == "silence":
+        x[:, T // 2:T // 2 + 240] *= 1e-9
+    elif kind != "plain":
+        x *= {"zero": 0.0, "quiet": 1e-9, "loud": 1e6}[kind]
+    X = _cl.Act(x.view(-1), B, T, C)
+
+    def launches():
+        return _cl.conv(_cl.depthwise7(X, dw, db, *a, dil, 0, T, parts=True), w, C, b, epi="resid", resid=X)
+
+    one, two = _us(lambda: _cl.dw_unit(X, dw, db, *a, w, b, dil, 0, T)), _us(launches)
+    assert one <= 1.5 * two, (one, two)
+
+
 def _tail_weights(g):
     """weights of the end of Mimi's decoder, as it keeps them"""
     from vox_serve_b200.tokenizer import _cl
@@ -768,19 +807,7 @@ def test_channels_last_tail_is_no_slower_than_its_convolutions(kind):
         h = _cl.conv(xp, w1, 32, b1, ksize=3, act="elu", out="parts")
         return _cl.last_conv(_cl.conv(h, w3, 64, b3, epi="resid", resid=X, act="elu"), wl, bl, 3, 2, 0, T, tanh=False)
 
-    def us(f):
-        times = []
-        for _ in range(6):
-            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
-            a.record()
-            for _ in range(4):
-                f()
-            b.record()
-            b.synchronize()
-            times.append(a.elapsed_time(b) * 250)
-        return min(times)
-
-    one, three = us(lambda: _cl.res_tail(X, w1, b1, w3, b3, wl, bl)), us(launches)
+    one, three = _us(lambda: _cl.res_tail(X, w1, b1, w3, b3, wl, bl)), _us(launches)
     assert one <= 1.5 * three, (one, three)
 
 

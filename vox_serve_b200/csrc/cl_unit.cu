@@ -256,39 +256,69 @@ __device__ __forceinline__ CuTaps cu_taps(const CuDwParams& p, int c) {
   t.io = ld(p.alpha_mid + p.C);
   return t;
 }
-// A run once more, row by row, for the blocks of rows that parts cannot hold: those stay fp32, a bit in the row's word
+// A run once more for the blocks of rows that parts cannot hold: those stay fp32, a bit in the row's word.  (Two rows at a time: with the kernel's four, or its constants in
+// registers, the kernel spilled around the call and SNAC took 0.5 % longer.)  32 x 6000 positions of 64 channels, dilation 9, with one such value in every tile / nothing but
+// such values / zeros: 192 / 848 / 62 us, in two launches 211 / 840 / 87; with the seven inputs of every row anew, and zeros taken for such values, 394 / 1554 / 261.
 __device__ __noinline__ void cu_odd_run(const CuDwParams& p, const float* x, int t_first, int n, int r0, int c, int block, uint32_t dst, uint32_t* raw, uint32_t* any) {
   const int lane = threadIdx.x & 31, in = (lane & 15) * 2;
   const CuTaps tp = cu_taps(p, c);
-  const CuSine K = cu_sine();
-#pragma unroll 1
-  for (int j = 0; j < n; ++j) {
-    F2 o = tp.b;
+  auto snake = [&](F2 (&v)[2], F2 a, F2 inv) { cl_snake4(v[0], v[1], a, a, inv, inv); };          // (the bits of cu_snake, without its constants in registers)
+  F2 h[8], got[2];              // (the walk of the kernel below)
+  __syncwarp();                 // (every lane's parts of these rows are written)
+  int t = t_first - 3 * p.dil;
+  auto load2 = [&]() {
 #pragma unroll
-    for (int k = 0; k < 7; ++k) {
-      const int t = t_first + (j + k - 3) * p.dil;
+    for (int i = 0; i < 2; ++i, t += p.dil) {
       float2 v = make_float2(0.f, 0.f);
       if (t >= 0 && t < p.T) v = __ldcg(reinterpret_cast<const float2*>(x + static_cast<long long>(t) * p.C));
-      F2 one[1] = {f2(v.x, v.y)};
-      cu_snake(one, tp.ai, tp.ii, K);
-      o = f2_fma(tp.w[k], one[0], o);
+      got[i] = f2(v.x, v.y);
     }
-    F2 one[1] = {o};
-    cu_snake(one, tp.ao, tp.io, K);
-    const float2 v = f2_get(one[0]);
-    float m = max3_abs(v.x, v.y, v.y);
+  };
 #pragma unroll
-    for (int q = 1; q < 16; q <<= 1) {
-      const float other = __shfl_xor_sync(0xffffffffu, m, q);
-      m = max3_abs(m, other, other);
+  for (int i = 0; i < 6; ++i) h[i] = f2(0.f);
+  load2();
+#pragma unroll 1
+  for (int j = -6; j < n; j += 2) {
+    snake(got, tp.ai, tp.ii);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) h[6 + i] = got[i];
+    if (j + 2 < n) load2();
+    if (j >= 0) {
+      F2 o[2];
+      float m[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) o[i] = tp.b;
+#pragma unroll
+      for (int q = 0; q < 7; ++q)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) o[i] = f2_fma(tp.w[q], h[i + q], o[i]);
+      snake(o, tp.ao, tp.io);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float2 v = f2_get(o[i]);
+        m[i] = max3_abs(v.x, v.y, v.y);
+      }
+#pragma unroll
+      for (int q = 1; q < 16; q <<= 1)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float other = __shfl_xor_sync(0xffffffffu, m[i], q);
+          m[i] = max3_abs(m[i], other, other);
+        }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (j + i >= n || cl_code(m[i]) != CB_RAW) continue;          // (the parts are there)
+        const float2 v = f2_get(o[i]);
+        const int r = r0 + (j + i) * p.dil;
+        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dst + r * 128 + (((in >> 2) ^ (r & 7)) << 4) + (in & 2) * 4), "f"(v.x), "f"(v.y) : "memory");
+        if (in == 0) {
+          atomicOr(raw + r, 1u << block);
+          *any = 1u;
+        }
+      }
     }
-    if (cl_code(m) != CB_RAW) continue;          // (the parts are there)
-    const int r = r0 + j * p.dil;
-    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dst + r * 128 + (((in >> 2) ^ (r & 7)) << 4) + (in & 2) * 4), "f"(v.x), "f"(v.y) : "memory");
-    if (in == 0) {
-      atomicOr(raw + r, 1u << block);
-      *any = 1u;
-    }
+#pragma unroll
+    for (int i = 0; i < 6; ++i) h[i] = h[i + 2];
   }
 }
 
@@ -476,8 +506,11 @@ __global__ void __launch_bounds__(32 * (P + 1), P == 9 ? 2 : 1) cl_dw_unit_kerne
       }
       // No value out of range, and in either block a lane none of whose values is tiny: nearly always
       const uint32_t fine = __ballot_sync(0xffffffffu, top < CL_X_TOP), large = __ballot_sync(0xffffffffu, low >= CL_X_LOW);
-      if (n > 0 && !(fine == 0xffffffffu && (large & 0xffffu) && large >> 16))
-        cu_odd_run(p, x, t0 + r0, n, r0, c, 2 * k + (lane >> 4), dst, raw, any);
+      if (n > 0 && !(fine == 0xffffffffu && (large & 0xffffu) && large >> 16)) {
+        const uint32_t some = __ballot_sync(0xffffffffu, top != 0.f);          // (a block of zeros is its parts)
+        if (!(fine == 0xffffffffu && ((large & 0xffffu) || !(some & 0xffffu)) && (large >> 16 || !(some >> 16))))
+          cu_odd_run(p, x, t0 + r0, n, r0, c, 2 * k + (lane >> 4), dst, raw, any);
+      }
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&op_full[k]);

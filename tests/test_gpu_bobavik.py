@@ -260,6 +260,31 @@ def test_grouped_experts_on_long_prompts():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shared_ff", [64, 96])
+def test_grouped_experts_make_no_tensor_maps_for_a_new_number_of_rows(monkeypatch, shared_ff):
+    """The maps of the experts' rows are of whole buffers: a step of a number of rows not seen before encodes none, and gives what a worker gives that has seen no other."""
+    from vox_serve_b200 import ops
+
+    cfg = O.make_config(width=64, layers=("attention", "lightning"), ff=64, shared_ff=shared_ff, experts=4, top=2, dim=16, vdim=16, window=40)
+    sd = O.random_weights(cfg, 23)
+    toks = _tokens(700, cfg["vocab"], 9)
+    w = _worker(cfg, sd, BF16, pages=100, page_size=8, max_rows=768)
+    _replay(w, {"a": toks}, [[("a", 700)]])
+    e, made, call = w.engine, [], ops.call
+    spans = [(b.data_ptr(), b.data_ptr() + b.numel() * b.element_size()) for b in (e.moe_xs, e.moe_act)]
+
+    def spy(fn, *args):
+        if fn == "vb_tensor_map_2d_bf16" and any(lo <= args[1] < hi for lo, hi in spans):
+            made.append(args[2])
+        return call(fn, *args)
+
+    monkeypatch.setattr(ops, "call", spy)
+    got = _replay(w, {"a": toks[:613]}, [[("a", 613)]])["a"]
+    assert not made
+    assert torch.equal(got, _replay(_worker(cfg, sd, BF16, pages=100, page_size=8, max_rows=768), {"a": toks[:613]}, [[("a", 613)]])["a"])
+
+
+@pytest.mark.gpu
 def test_long_decoding_past_window_and_pages():
     cfg = O.make_config(layers=("lightning", "attention"), window=20, decay=(0.99, 0.7))
     sd = O.random_weights(cfg, 9)

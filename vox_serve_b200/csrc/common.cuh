@@ -34,6 +34,15 @@ void set_error(const char* fmt, ...);
 // of the launch at hand): a per-launch value would be baked into nothing -- CUDA-graph kernel nodes replay
 // against whatever the function attribute was set to last, so a later, smaller launch would break them.
 constexpr int VB_MAX_DYN_SMEM = 227 * 1024;
+// SMs of the device in use, asked for once (the devices of a machine are alike); 148 where there is none to ask
+inline int sm_count() {
+  static std::atomic<int> known{0};
+  int sms = known.load(std::memory_order_relaxed), dev = 0;
+  if (sms) return sms;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  known.store(sms, std::memory_order_relaxed);
+  return sms;
+}
 // ... once per kernel and device (one flag per instantiation: call it with the kernel itself, not with a pointer that may
 // name several; two threads that arrive together both set the same value)
 template <typename Kernel>

@@ -543,10 +543,8 @@ int vb_moe_group_tiles(int32_t* d_sorted_token, int32_t* d_pair_row, int32_t* d_
   const long long pairs = static_cast<long long>(T) * top, shared_rows = shared ? (T + 15LL) / 16 * 16 : 0;
   VB_CHECK_ARG(rows_max >= shared_rows + pairs + 15LL * experts && tiles_max >= (pairs + 255) / 256 + experts + (shared ? (T + 255) / 256 : 0),
                "vb_moe_group_tiles: %d rows and %d tiles do not hold %lld pairs", rows_max, tiles_max, pairs);
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
   const MoeTilesParams p{d_sorted_token, d_pair_row, d_idx, reinterpret_cast<int4*>(d_tiles), T, experts, top, shared ? 1 : 0, rows_max, tiles_max,
-                         {(n_a + 255) / 256, (n_b + 255) / 256}, {(k_a + 63) / 64, (k_b + 63) / 64}, max(1, sms / 2)};
+                         {(n_a + 255) / 256, (n_b + 255) / 256}, {(k_a + 63) / 64, (k_b + 63) / 64}, max(1, sm_count() / 2)};
   VB_LAUNCH_PDL(moe_group_tiles_kernel, 1, 1024, 0, stream, p);
   return 0;
 }

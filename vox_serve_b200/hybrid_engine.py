@@ -1417,8 +1417,9 @@ class HybridEngine:
         rows = ((T + 15) // 16 * 16 if merged else 0) + T * f.top + 16 * f.experts
         token = self.moe_sorted[:rows]
         ops.moe_group_tiles(idx, T, f.experts, f.top, merged, token, self.moe_pair_row, self.moe_table, ((n_up, W), (W, f.ff)))
-        xs = ops.moe_gather_rows(h, token, self.moe_xs[:rows * W].view(rows, W))
-        act, eo = self.moe_act[:rows * f.ff].view(rows, f.ff), self.moe_out[:rows * W].view(rows, W)
+        whole = lambda buf, n: buf[:buf.numel() // n * n].view(-1, n)                # noqa: E731
+        xs, act, eo = whole(self.moe_xs, W), whole(self.moe_act, f.ff), self.moe_out[:rows * W].view(rows, W)
+        ops.moe_gather_rows(h, token, xs[:rows])
         ops.gemm_tiles(xs, w[up], act, 2 if gated else 0, n_up, W, self.moe_table, group_bytes=g["group_bytes"], act=None if gated else f.act, glu=glu)
         ops.gemm_tiles(act, w["down_all"], eo, 1, W, f.ff, self.moe_table, w_kb_stride=g["kb_total"], group_kb=g["group_kb"])
         shared = eo[:T] if merged else None

@@ -1594,7 +1594,8 @@ def moe_group_tiles(idx: torch.Tensor, T: int, experts: int, top: int, shared: b
 
 def gemm_tiles(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, mode: int, N: int, K: int, tiles: torch.Tensor, group_bytes: int = 0, w_kb_stride: int = 0,
                group_kb: int = 0, act: Optional[str] = None, glu: Optional[Tuple[float, float]] = None) -> torch.Tensor:
-    """``gemm_grouped`` (with ``glu``: ``gemm_grouped_glu``) over the token tiles of a table on the device (``moe_group_tiles``; a kernel must stand between)"""
+    """``gemm_grouped`` (with ``glu``: ``gemm_grouped_glu``) over the token tiles of a table on the device (``moe_group_tiles``; a kernel must stand between).
+    ``x`` may be longer than its tiles reach: a buffer's whole length has the same tensor maps whatever a step's rows are."""
     _need_cuda(x, out)
     assert x.dtype == BF16 and x.dim() == 2 and x.shape[1] == K and out.is_contiguous() and w.tile_rows in WIDE_TILE_ROWS
     if act is not None and mode != 0:

@@ -150,8 +150,6 @@ def test_wide_grouped_projection(ops, groups, tt, N, K):
     _close(out, ref, 2e-6)
 
 
-# channels-last vocoder convolutions: one row and several batch entries in a box, box sizes around 128 rows, a range inside the
-# sequence, column tiles with a remainder, dilated taps reaching in front of the start; every epilogue and activation
 @pytest.mark.parametrize("T,E,top,shared,N,K,skew", [(1, 4, 1, True, 256, 128, False), (17, 3, 2, False, 320, 200, False), (700, 8, 2, True, 512, 256, False),
                                                      (1001, 8, 2, True, 384, 192, True), (513, 70, 4, False, 128, 64, False), (300, 5, 3, True, 256, 128, True)])
 @pytest.mark.parametrize("mode,tile_rows", [(0, 128), (1, 128), (2, 96), (2, 64)])
@@ -236,6 +234,8 @@ def test_short_convolution_rows(ops, lens, old, taps, C, act, residual, shift):
         assert torch.equal(state[i], torch.cat((front, u[at]))[-K:].float() if n >= K else torch.cat((front.float(), (x + ib)[at]))[-K:])
 
 
+# channels-last vocoder convolutions: one row and several batch entries in a box, box sizes around 128 rows, a range inside the
+# sequence, column tiles with a remainder, dilated taps reaching in front of the start; every epilogue and activation
 @pytest.mark.parametrize("B,T,C,N,ksize,dil,lo,hi,epi,act", [
     (1, 1, 32, 32, 1, 1, 0, 1, "plain", None), (7, 16, 64, 96, 1, 1, 0, 16, "resid", "snake"), (2, 128, 32, 128, 3, 1, 0, 128, "plain", "elu"),
     (3, 129, 96, 160, 1, 1, 5, 129, "noise", None), (1, 300, 64, 64, 7, 9, 130, 299, "scale_resid", "gelu"), (40, 3, 128, 512, 2, 1, 0, 3, "resid", None)])
@@ -1152,7 +1152,7 @@ def test_prompt_attention_probabilities(ops, D, width):
     (516, 1032, 9, True, False, True), (1024, 264, 1, True, False, False),
 ])
 def test_reduce_residual_rmsnorm_many_rows(ops, T, N, S, resid, tiled, hidden):
-    """A step of more than 512 rows against the same rows in steps of 200, which take the other kernel."""
+    """A step of more than 512 rows against the same rows in steps of at most 148, which take the kernel of few rows."""
     g = torch.Generator("cuda").manual_seed(T)
     parts = torch.randn(S, T, N, generator=g, device="cuda")
     res = torch.randn(T, N, generator=g, device="cuda").to(torch.bfloat16) if resid else None
@@ -1160,7 +1160,7 @@ def test_reduce_residual_rmsnorm_many_rows(ops, T, N, S, resid, tiled, hidden):
     out = ops.TiledAct(T, N, torch.device("cuda")) if tiled else None
     h, y = ops.reduce_residual_rmsnorm(parts, res, w, 1e-6, normed_out=out, want_hidden=hidden)
     y = y.to_rows() if tiled else y
-    cut = [slice(a, min(a + 200, T)) for a in range(0, T, 200)]
+    cut = [slice(a, min(a + 148, T)) for a in range(0, T, 148)]
     want = [ops.reduce_residual_rmsnorm(parts[:, c].contiguous(), None if res is None else res[c].contiguous(), w, 1e-6) for c in cut]
     if hidden:
         assert torch.equal(h, torch.cat([a for a, _ in want]))
@@ -1317,9 +1317,26 @@ def test_embedding_rmsnorm(ops, T, dim, tiled):
     assert torch.equal(normed.to_rows() if tiled else normed, ops.rmsnorm(hidden, w[0], 1e-6))
 
 
-@pytest.mark.parametrize("T,n_q,n_kv,D,S,bias", [(1, 1, 1, 16, 1, False), (3, 24, 8, 128, 3, True), (33, 5, 1, 80, 4, False), (64, 14, 2, 64, 5, True), (256, 2, 2, 256, 8, False)])
+def _rotated(parts, bias, pos, freq, n_rot, D):
+    """q | k | v rows of planes [S, T, (n_rot + n_v) D]: summed in order, biased and rounded, and with their first n_rot heads turned in 64 bits; and how far fp32 may be
+    off them: angles, cosines and sines a few 2^-23 of one, the products and their sum as much of the larger, the result half a step of bf16 (8 bits: 2^-8 of itself at most)."""
+    x = parts[0].clone()
+    for p in parts[1:]:
+        x += p
+    x = (x if bias is None else x + bias.float()).to(torch.bfloat16).double().view(x.shape[0], -1, 2, D // 2)
+    turn = (pos.float()[:, None] * freq).double().view(-1, 1, 2, D // 2)          # (the angle in 32 bits, as its rounding is large for late positions)
+    c, s = turn.cos(), turn.sin()
+    y = torch.stack((x[:, :, 0] * c[:, :, 0] - x[:, :, 1] * s[:, :, 0], x[:, :, 1] * c[:, :, 1] + x[:, :, 0] * s[:, :, 1]), 2)
+    off = y.abs() * 2.0 ** -8 + x.abs().sum(2, keepdim=True) * 2.0 ** -20
+    y[:, n_rot:], off[:, n_rot:] = x[:, n_rot:], 0.0
+    return y.flatten(2), off.flatten(2)
+
+
+@pytest.mark.parametrize("T,n_q,n_kv,D,S,bias", [(1, 1, 1, 16, 1, False), (3, 24, 8, 128, 3, True), (33, 5, 1, 80, 4, False), (64, 14, 2, 64, 5, True), (256, 2, 2, 256, 8, False),
+                                                 (17, 3, 2, 16, 2, True), (129, 2, 1, 80, 3, True), (65, 1, 2, 256, 4, True)])
 def test_qkv_rope_append_few_rows(ops, T, n_q, n_kv, D, S, bias):
-    """Up to 256 rows (a row's items over blocks, four planes at a time) against the same rows in a step of 300: the same bits; a row without a page is not stored."""
+    """Up to 256 rows (a row's items over blocks, four planes at a time) against 64 bits, and against the same rows in a step of 300: the same bits; a row without a page is not
+    stored."""
     g = torch.Generator("cuda").manual_seed(T)
     page, W, R = 16, (n_q + 2 * n_kv) * D, 300
     parts = torch.randn(S, R, W, generator=g, device="cuda")
@@ -1336,13 +1353,21 @@ def test_qkv_rope_append_few_rows(ops, T, n_q, n_kv, D, S, bias):
                  page, D, 0, None, None, 0.0, None if b is None else b.data_ptr(), ops._stream())
         return q[:T], kv.transpose(1, 2).reshape(-1, 2, n_kv, D)[:T]
 
-    for a, want in zip(run(T), run(R)):
+    got = run(T)
+    for a, want in zip(got, run(R)):
         assert torch.equal(a, want)
+    want, off = _rotated(parts[:, :T], b, pos[:T], freq, n_q + n_kv, D)
+    kv = got[1].double()
+    assert not kv[T // 2].any()
+    stored = torch.arange(T, device="cuda") != T // 2
+    have = torch.cat((got[0].double(), kv[:, 0], kv[:, 1]), 1)
+    assert ((have - want).abs() <= off)[stored].all() and ((have - want).abs() <= off)[:, :n_q].all()
 
 
 @pytest.mark.parametrize("T,n_q,n_kv,D,S,bias", [(257, 1, 1, 16, 1, False), (300, 24, 8, 128, 1, False), (258, 5, 1, 80, 3, True), (600, 2, 2, 256, 2, False)])
 def test_qkv_rope_append_many_rows(ops, T, n_q, n_kv, D, S, bias):
-    """A step of more than 256 rows against the same rows in steps of at most 256; rows without a page keep the cache as it is."""
+    """A step of more than 256 rows against 64 bits, and against the same rows in steps of at most 200, which take the kernel of few rows; rows without a page keep the cache as
+    it is."""
     g = torch.Generator("cuda").manual_seed(T)
     W, page = (n_q + 2 * n_kv) * D, 16
     parts = torch.randn(S, T, W, generator=g, device="cuda")
@@ -1367,6 +1392,12 @@ def test_qkv_rope_append_many_rows(ops, T, n_q, n_kv, D, S, bias):
     # the same products and one sum, which the compiler may fuse on either side: one bf16 step of the larger term at most
     for got, ref in ((q, torch.cat(want)), (kv[0], kv[1])):
         assert ((got.float() - ref.float()).abs() <= ref.float().abs() * 2.0 ** -7 + 2.0 ** -20 * 8).all()
+    want, off = _rotated(parts, b, pos, freq, n_q + n_kv, D)
+    rows = kv[0].transpose(1, 2).reshape(-1, 2, n_kv, D).double()
+    assert (rows == 7.0).flatten(1).all(1).sum() == n_pages * page - (T - 1)
+    stored = torch.arange(T, device="cuda") != T // 2
+    have = torch.cat((q.double(), rows[at.long(), 0], rows[at.long(), 1]), 1)
+    assert ((have - want).abs() <= off)[stored].all() and ((have - want).abs() <= off)[:, :n_q].all()
 
 
 @pytest.mark.parametrize("penalty", [1.3, 0.7, 3.0, 1.0 + 2.0 ** -23, 2.0 - 2.0 ** -23, 1e-3, 2.0 ** 39, 2.0 ** 41])

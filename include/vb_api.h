@@ -283,10 +283,10 @@ int vb_latest_window(int32_t* d_first, const int32_t* d_n_out, const int32_t* d_
 int vb_gather_windows(int64_t* d_windows, const int32_t* d_history, const int32_t* d_slot, const int32_t* d_first,
                       const int32_t* d_n_valid, int n, int history_cap, int window, void* stream);
 /* embedding gather: orpheus.py:408 */
+int vb_embedding(void* d_out, const void* d_table, const int32_t* d_ids, int T, int dim, int vocab, void* stream);
 /* the rows and their norm (what vb_rmsnorm makes of them, in rows or XT(normed_xt_tile)) in one launch: dim a multiple of 8 up to 8192, 16-byte boundaries */
 int vb_embedding_rmsnorm(void* d_hidden, void* d_normed, const void* d_table, const int32_t* d_ids, const void* d_weight, int T, int dim, int vocab, float eps,
                          int normed_xt_tile, void* stream);
-int vb_embedding(void* d_out, const void* d_table, const int32_t* d_ids, int T, int dim, int vocab, void* stream);
 /* Multi-codebook glue of the depth-transformer adapters (vox_serve/model/csm.py:158-168, 637-663, 700-701;
  * cuda_graph_worker.py:1058-1160 does these with torch ops and host indices between graph replays):
  *   vb_multi_embed_sum: out[t] = bf16(sum over columns c < C with mask[t][c] != 0 (NULL = all) of
@@ -791,11 +791,11 @@ int vb_moe_group(int32_t* d_row_off, int32_t* d_sorted_token, int32_t* d_pair_ro
 /* (tile_rows > 0: every expert's rows start at a multiple of tile_rows; padding rows get token -1; d_tile_group[i] =
  * the expert of row tile i, 0 for tiles past the last expert, i < n_tiles >= ceil(T * top / tile_rows) + experts)
  * vb_moe_gather_rows: out[r] = token[r] >= 0 ? x[token[r]] : 0, bf16 rows of `width` (a multiple of 8) */
+int vb_moe_gather_rows(void* d_out, const void* d_x, const int32_t* d_token, int rows, int width, void* stream);
 /* Pairs by expert for vb_gemm_bf16_wide_tiles: with `shared` rows [0, T) are every token once (group `experts`), then every expert's rows from a multiple of 16 on;
  * token -1 elsewhere.  (n_a, k_a), (n_b, k_b): the two projections that the height of the tiles is chosen for.  rows_max >= round16(T if shared) + T top + 15 experts. */
 int vb_moe_group_tiles(int32_t* d_sorted_token, int32_t* d_pair_row, int32_t* d_tiles, const int32_t* d_idx, int T, int experts, int top, int shared, int rows_max,
                        int tiles_max, int n_a, int k_a, int n_b, int k_b, void* stream);
-int vb_moe_gather_rows(void* d_out, const void* d_x, const int32_t* d_token, int rows, int width, void* stream);
 /* dense form (bf16): act [T][ld] holds silu(gate) * up of EVERY expert side by side (expert e at columns e * ff ..), then
  * the shared expert's; columns of expert e are scaled by the token's routing weight for e, or zeroed if e was not chosen */
 int vb_moe_scale_dense(void* d_act, const int32_t* d_idx, const float* d_wts, int T, int ld, int experts, int ff, int top,

@@ -11,11 +11,10 @@
 //    shared-memory copies of the plan -- and feeds a ring of HALF-stages (the K rows of a tile, then its V rows:
 //    32 KiB + skew each) behind full/empty mbarriers with the TMA unit's LINEAR bulk copies
 //    (cp.async.bulk.shared.global, L2 evict_first: a layer's KV is not read again before the next step): one
-//    copy per run of one to four token rows (n_kv * D * 2 bytes each, all heads), issued by the warp's lanes in parallel.  Three
-//    half-stages (~100 KiB) keep a CTA below half an SM's shared memory, so the CTA of a NEIGHBOURING kernel of
-//    the programmatic-dependent-launch chain (the next layer's attention in a back-to-back run; the O projection's
-//    weight prefetch or the QKV tail in a decode step) is resident beside it: its launch latency, plan look-up
-//    and the KV of tokens that were already in the cache stream in while this kernel is still running.  Runs land with a 16-byte
+//    copy per run of one to four token rows (n_kv * D * 2 bytes each, all heads), issued by the warp's lanes in parallel.  Six
+//    half-stages take the whole SM: a stream needs that much in flight (vb_paged_attn, with both sides measured), more than a CTA
+//    of a neighbouring kernel beside it gives back.  Plan look-up and the KV of tokens that were already in the cache
+//    do not wait for the kernel in front (programmatic dependent launch).  Runs land with a 16-byte
 //    skew behind each, and the eight rows of an ldmatrix are taken from different runs, so that they lie in different
 //    banks without a swizzle.  (A tiled tensor-map box must keep a 128-byte inner extent under the
 //    128B swizzle; measured, the TMA unit then spends ~19 cycles per 128-byte row and caps the kernel below

@@ -1399,15 +1399,6 @@ static int cl_dw_rows(int range, int channel_blocks, int B, int dil, int sms) {
   return best;
 }
 
-static int cl_sms() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-  }
-  return sms;
-}
-
 }  // namespace vb
 
 using namespace vb;
@@ -1530,7 +1521,7 @@ static bool cl_box_map(CUtensorMap* map, const void* base, int N, int rows, int 
 
 template <bool PARTS>
 static int cl_launch(ClConvParams p, cudaStream_t stream) {
-  cl_plan<PARTS>(p, cl_sms());
+  cl_plan<PARTS>(p, sm_count());
   VB_CHECK_ARG(p.units > 0, "vb_cl_conv: too many tiles");
   ClMaps maps = {};
   VB_CHECK_ARG((!PARTS && !p.staged) || encode_fn(), "cuTensorMapEncodeTiled not available (no CUDA driver?)");
@@ -1658,7 +1649,7 @@ int vb_cl_dwconv7_parts(float* d_y, void* d_code, const float* d_x, long long x_
   VB_CHECK_ARG(0 <= t_lo && t_lo <= t_hi && t_hi <= T, "vb_cl_dwconv7: range [%d, %d) outside [0, %d)", t_lo, t_hi, T);
   if (B <= 0 || t_lo == t_hi) return 0;
   VB_CHECK_CUDA(max_dyn_smem_once(cl_dwconv7_kernel));
-  const int tile = cl_dw_rows(t_hi - t_lo, C / 64, B, dilation, cl_sms());
+  const int tile = cl_dw_rows(t_hi - t_lo, C / 64, B, dilation, sm_count());
   VB_LAUNCH_PDL(cl_dwconv7_kernel, dim3((t_hi - t_lo + tile - 1) / tile, C / 64, B), 256, static_cast<size_t>(tile + 6 * dilation) * 256, stream,
                 d_y, static_cast<uint8_t*>(d_code), d_x, x_bstride, d_w, d_bias, d_alpha_in, d_alpha_out, C, T, dilation, t_lo, t_hi, tile);
   return 0;

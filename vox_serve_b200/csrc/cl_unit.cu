@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(32 * (P + 1), P == 9 ? 2 : 1) cl_dw_unit_kerne
       tc_fence_after();
       if (elect_one()) {
         uint64_t w_hi = w_desc0 + static_cast<uint64_t>(ws) * (2 * CL_W_BLOCK >> 4), x_hi = x_desc0 + static_cast<uint64_t>(2 * k) * (blk_bytes >> 4);
-        // (a loop: unrolled, nvcc 12.9 gave the tensor cores descriptors of the weights without their upper halves)
+        // (a loop: unrolled by nvcc 12.9, rows of the result came out of the wrong tile of the weights)
 #pragma unroll 1
         for (int g = 0; g < 2; ++g) {
 #pragma unroll
@@ -563,14 +563,6 @@ __global__ void __launch_bounds__(32 * (P + 1), P == 9 ? 2 : 1) cl_dw_unit_kerne
 
 static bool on16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }      // (a null pointer is)
 
-static int cu_sms() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-  }
-  return sms;
-}
 // shared memory of a block
 static int cu_dw_smem(int C, int cols, int w_stages) {
   return 1024 + C / 32 * cols * 128 + w_stages * 2 * CL_W_BLOCK + (CU_MAX_CHUNKS + 2 * CU_W_STAGES + 1) * 8 + 16 + cols * 4;
@@ -1098,7 +1090,7 @@ extern "C" {
 
 int vb_cl_dw_unit_pays(int B, int C, int rows, int dilation) {
   if (B <= 0 || rows <= 0 || C <= 0 || C % 64 || C > 256 || dilation < 1 || dilation > 64) return 0;
-  return C <= 128 || (C + 127) / 128 * ((rows + 125LL) / 126) * B <= cu_sms();
+  return C <= 128 || (C + 127) / 128 * ((rows + 125LL) / 126) * B <= sm_count();
 }
 
 int vb_cl_dw_unit(float* d_y, void* d_yp, void* d_yp_code, const float* d_x, long long x_bstride, const float* d_dw_w, const float* d_dw_b,
@@ -1114,7 +1106,7 @@ int vb_cl_dw_unit(float* d_y, void* d_yp, void* d_yp_code, const float* d_x, lon
   VB_CHECK_ARG(0 <= t_lo && t_lo <= t_hi && t_hi <= T, "vb_cl_dw_unit: range [%d, %d) outside [0, %d)", t_lo, t_hi, T);
   VB_CHECK_ARG(B <= 65535, "vb_cl_dw_unit: %d entries", B);
   if (B <= 0 || t_lo == t_hi) return 0;
-  const CuDwPlan g = cu_dw_plan(C, dilation, t_hi - t_lo, B, cu_sms());
+  const CuDwPlan g = cu_dw_plan(C, dilation, t_hi - t_lo, B, sm_count());
   CuDwParams p = {};
   VB_CHECK_ARG(p.wait_flag = wait_flag(WK_CL_CONV), "vb_cl_dw_unit: no mapped host memory");
   const long long n_pad = (C + 127LL) / 128 * 128;
@@ -1166,7 +1158,7 @@ int vb_cl_res_tail(float* d_y, const float* d_x, long long x_bstride, const void
                                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   VB_CHECK_ARG(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(tail) failed: CUresult %d", static_cast<int>(r));
   VB_CHECK_CUDA(max_dyn_smem_once(cl_res_tail_kernel));
-  VB_LAUNCH_PDL(cl_res_tail_kernel, min(p.tiles, cu_sms()), CT_THREADS, CT_SMEM, stream, p, map);
+  VB_LAUNCH_PDL(cl_res_tail_kernel, min(p.tiles, sm_count()), CT_THREADS, CT_SMEM, stream, p, map);
   return 0;
 }
 

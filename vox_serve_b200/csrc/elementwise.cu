@@ -447,8 +447,8 @@ __device__ __noinline__ float rr_from_row(const uint4* row, float4* red4, int N,
 // The same for steps of more rows than there are SMs: 128 threads to a row, G groups of 8 columns each.  A row is one chain of a load, a sum over it and a store, so
 // every load of a plane is in flight at once, the norm's weights before the kernel in front has ended, behind a barrier or two (for the sum of squares).
 // us behind the kernel that writes the planes, before (a warp to a row past 512 rows, else a CTA or a cluster) / now: 1024 rows of 1024 columns 4.1 / 2.7,
-// 2048 6.7 / 3.9, 3072 8.9 / 5.6, 4096 10.9 / 6.9; three planes of 512 rows 4.7 / 3.1, 6.1 / 3.9, 8.1 / 5.5, 9.8 / 6.5.  Three groups held to 80 registers spilled
-// when all planes of a row were loaded at once: four planes of 133 rows of 3072 6.0 for 3.6.
+// 2048 6.7 / 3.9, 3072 8.9 / 5.6, 4096 10.9 / 6.9; three planes of 512 rows 4.7 / 3.1, 6.1 / 3.9, 8.1 / 5.5, 9.8 / 6.5.  (Three groups held to 80 registers spilled
+// then: four planes of 133 rows of 3072 6.0 for 3.6.)
 template <int G>
 __global__ void __launch_bounds__(128, G <= 2 ? 8 : 5) reduce_residual_rmsnorm_rows_kernel(
     __nv_bfloat16* __restrict__ hidden_out, __nv_bfloat16* __restrict__ normed_out, const float* __restrict__ partials, int split_k,
@@ -772,32 +772,32 @@ __global__ void __launch_bounds__(256) qkv_rope_append_kernel(
 __device__ __forceinline__ void qkv_rope_finish(float (&x)[2][8], const float* sm, int t, int h, int e, int D, int n_q, int n_kv, __nv_bfloat16* q_out, __nv_bfloat16* kd,
                                                 size_t slab, const __nv_bfloat16* qkv_bias) {
   const int half = D >> 1, n = h * D + e;
-      uint32_t o[2][4];
-      float y[2][8];
+  uint32_t o[2][4];
+  float y[2][8];
 #pragma unroll
-      for (int k = 0; k < 2; ++k)
+  for (int k = 0; k < 2; ++k)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (qkv_bias) x[k][j] += __bfloat162float(qkv_bias[n + k * half + j]);
-          x[k][j] = round_bf16(x[k][j]);
-        }
-      const bool rot = h < n_q + n_kv;
+    for (int j = 0; j < 8; ++j) {
+      if (qkv_bias) x[k][j] += __bfloat162float(qkv_bias[n + k * half + j]);
+      x[k][j] = round_bf16(x[k][j]);
+    }
+  const bool rot = h < n_q + n_kv;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        y[0][j] = rot ? x[0][j] * sm[e + j] + -x[1][j] * sm[D + e + j] : x[0][j];
-        y[1][j] = rot ? x[1][j] * sm[e + half + j] + x[0][j] * sm[D + e + half + j] : x[1][j];
-      }
+  for (int j = 0; j < 8; ++j) {
+    y[0][j] = rot ? x[0][j] * sm[e + j] + -x[1][j] * sm[D + e + j] : x[0][j];
+    y[1][j] = rot ? x[1][j] * sm[e + half + j] + x[0][j] * sm[D + e + half + j] : x[1][j];
+  }
 #pragma unroll
-      for (int k = 0; k < 2; ++k)
+  for (int k = 0; k < 2; ++k)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o[k][j] = pack_bf16(y[k][2 * j], y[k][2 * j + 1]);
-      __nv_bfloat16* dst = nullptr;
-      if (h < n_q) dst = q_out + (static_cast<size_t>(t) * n_q + h) * D + e;
-      else if (kd) dst = kd + (h < n_q + n_kv ? (h - n_q) * D : slab + (h - n_q - n_kv) * D) + e;
-      if (dst) {
-        *reinterpret_cast<uint4*>(dst) = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]);
-        *reinterpret_cast<uint4*>(dst + half) = make_uint4(o[1][0], o[1][1], o[1][2], o[1][3]);
-      }
+    for (int j = 0; j < 4; ++j) o[k][j] = pack_bf16(y[k][2 * j], y[k][2 * j + 1]);
+  __nv_bfloat16* dst = nullptr;
+  if (h < n_q) dst = q_out + (static_cast<size_t>(t) * n_q + h) * D + e;
+  else if (kd) dst = kd + (h < n_q + n_kv ? (h - n_q) * D : slab + (h - n_q - n_kv) * D) + e;
+  if (dst) {
+    *reinterpret_cast<uint4*>(dst) = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]);
+    *reinterpret_cast<uint4*>(dst + half) = make_uint4(o[1][0], o[1][1], o[1][2], o[1][3]);
+  }
 }
 
 // The tail for whole heads rotated in halves without norms, steps of many rows: a thread finishes 8 columns of a head and the 8 that
@@ -1044,12 +1044,13 @@ int vb_reduce_residual_rmsnorm(void* d_hidden_out, void* d_normed_out, const flo
   if (N % 8 == 0 && N <= 4096 && aligned(d_partials) && aligned(d_hidden_out) && aligned(d_normed_out) && aligned(d_residual) && aligned(d_norm_weight)) {
     // (a thread to 8 columns, of which an SM holds one row / 128 threads to a row, us: four planes of 133 rows of 2048, 3072, 4096 columns 2.9 / 3.5, 3.5 / 3.9, 3.7 / 5.0, of
     // 256 rows 3.5 / 3.7, 5.7 / 4.2, 6.3 / 5.6)
-    const auto rows = T <= 148   ? reduce_residual_rmsnorm_row_kernel
+    const bool few = T <= min(sm_count(), 192);          // (192: from there on a row is one part, which the row kernel does not hold)
+    const auto rows = few         ? reduce_residual_rmsnorm_row_kernel
                       : N <= 1024 ? reduce_residual_rmsnorm_rows_kernel<1>
                       : N <= 2048 ? reduce_residual_rmsnorm_rows_kernel<2>
                       : N <= 3072 ? reduce_residual_rmsnorm_rows_kernel<3>
                                   : reduce_residual_rmsnorm_rows_kernel<4>;
-    VB_LAUNCH_PDL(rows, T, T <= 148 ? (N / 8 + 31) / 32 * 32 : 128, 0, stream, static_cast<__nv_bfloat16*>(d_hidden_out),
+    VB_LAUNCH_PDL(rows, T, few ? (N / 8 + 31) / 32 * 32 : 128, 0, stream, static_cast<__nv_bfloat16*>(d_hidden_out),
                   static_cast<__nv_bfloat16*>(d_normed_out), d_partials, split_k, static_cast<const __nv_bfloat16*>(d_residual),
                   static_cast<const __nv_bfloat16*>(d_norm_weight), T, N, eps, normed_xt_tile, T > 512 ? RR_WARP : parts);
     return 0;

@@ -487,15 +487,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(480, 1)
 }
 
 #undef GW_UNITS
-static int gw_pairs() {
-  static int pairs = 0;
-  if (!pairs) {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-    pairs = sms / 2;
-  }
-  return pairs;
-}
+
+static int gw_pairs() { return sm_count() / 2; }
 
 }  // namespace vb
 

@@ -1366,6 +1366,7 @@ class HybridEngine:
         if self._by_tiles(w, "up_all", T):
             return self._moe_by_tiles(f, w, T, idx, wts, h, out, "up_all", sgate)
         if "grouped" in w and T >= self.GROUPED_MIN_ROWS:
+            # weight tiles of 16 rows, which the kernel of many rows does not take, or more token tiles than a table holds: whole row tiles of GROUP_TILE rows an expert
             g, tt = w["grouped"], self.GROUP_TILE
             n_tiles = (T * f.top + tt - 1) // tt + f.experts
             rows = n_tiles * tt
@@ -1451,7 +1452,7 @@ class HybridEngine:
             return self._moe_by_tiles(f, w, T, idx, wts, h, out, "gu_all")
         glu = (f.limit, f.slope) if f.act == "clamped_glu" else None
         if "grouped" in w and T >= self.GROUPED_MIN_ROWS:
-            # weight tiles that the kernel of many rows does not take: whole row tiles of GROUP_TILE rows an expert, the shared expert as two plain projections
+            # more token tiles than a table holds (some million pairs): whole row tiles of GROUP_TILE rows an expert, the shared expert as two plain projections
             g, tt = w["grouped"], self.GROUP_TILE
             n_tiles = (T * f.top + tt - 1) // tt + f.experts
             rows = n_tiles * tt

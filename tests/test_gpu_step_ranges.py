@@ -234,6 +234,26 @@ def test_short_convolution_rows(ops, lens, old, taps, C, act, residual, shift):
         assert torch.equal(state[i], torch.cat((front, u[at]))[-K:].float() if n >= K else torch.cat((front.float(), (x + ib)[at]))[-K:])
 
 
+@pytest.mark.parametrize("taps,act,shift", [(4, "silu", 0), (4, "silu", 1), (3, None, 0), (2, "silu", 0)])
+def test_short_convolution_rows_by_twos_and_fours(ops, taps, act, shift):
+    """A thread takes two rows or four by the size of the launch: the same bits for a quarter of the channels alone, with requests that begin anywhere in a group."""
+    g = torch.Generator(device="cuda").manual_seed(taps)
+    lens, old, C = [3, 70, 1, 9, 2, 5, 611], [0, 1, 5, 2, 0, 0, 7], 2048
+    T, B = sum(lens), len(lens)
+    x, w, bias, state = (torch.randn(*n, generator=g, device="cuda") for n in ((T, C), (C * taps + 1,), (C,), (B, taps - 1, C)))
+    w = w[shift:shift + C * taps].view(C, taps)          # (shifted: taps off the 16-byte boundaries)
+    plan = (_i32([sum(lens[:i]) for i in range(B + 1)]), _i32([i for i, n in enumerate(lens) for _ in range(n)]),
+            _i32([o + k for o, n in zip(old, lens) for k in range(n)]), _i32(list(range(B))), B)
+
+    def run(c):
+        st, out, f32 = state[:, :, :c].clone(memory_format=torch.contiguous_format), torch.zeros(T, c, device="cuda", dtype=torch.bfloat16), torch.zeros(T, c, device="cuda")
+        ops.short_conv(x[:, :c].contiguous(), w[:c], bias[:c].contiguous(), st, *plan, out=out, out_f32=f32, act=act, residual=True)
+        return st, out, f32
+
+    for a, b in zip(run(C), run(C // 4)):
+        assert torch.equal(a[..., :C // 4], b)
+
+
 # channels-last vocoder convolutions: one row and several batch entries in a box, box sizes around 128 rows, a range inside the
 # sequence, column tiles with a remainder, dilated taps reaching in front of the start; every epilogue and activation
 @pytest.mark.parametrize("B,T,C,N,ksize,dil,lo,hi,epi,act", [

@@ -21,6 +21,7 @@
 #include "../../include/vb_api.h"
 #define VB_PDL_FAMILY 4
 #include "quotient.cuh"
+#include <type_traits>
 
 namespace vb {
 
@@ -130,11 +131,11 @@ __global__ void __launch_bounds__(256) short_conv_rows_kernel(ShortConvParams p)
   }
 }
 
-// The same for rows that move in 16-byte pieces: a thread computes SC_VRPT consecutive rows of four neighbouring channels.  Row
+// The same for rows that move in 16-byte pieces: a thread computes R consecutive rows of four neighbouring channels.  Row
 // groups that lie inside one request, past the reach of its slot -- nearly all of a long prompt -- take every input from the
-// rows and check nothing per row; the FMA chain of an output is that of the kernels above.  Eight rows a thread, a channel's taps in one load and the
-// quotients of two rows together (four rows, tap by tap and one after the other: 1001 x 6144 27 us, 20 now; 1001 x 2048 14.5, 10).
-constexpr int SC_VRPT = 8, SC_VTHREADS = 128;
+// rows and check nothing per row; the FMA chain of an output is that of the kernels above.  A channel's taps are one load and the quotients of two rows go
+// through their steps together.
+constexpr int SC_VTHREADS = 128;
 
 template <typename CT> __device__ __forceinline__ void sc_store4(CT* __restrict__ p, float a, float b, float c, float d);
 template <> __device__ __forceinline__ void sc_store4<float>(float* __restrict__ p, float a, float b, float c, float d) {
@@ -144,10 +145,10 @@ template <> __device__ __forceinline__ void sc_store4<__nv_bfloat16>(__nv_bfloat
   *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(a, b), pack_bf16(c, d));
 }
 
-template <typename CT, int TAPS>
+template <typename CT, int TAPS, int R>
 __global__ void __launch_bounds__(SC_VTHREADS) short_conv_rows4_kernel(ShortConvParams p) {
   constexpr int K = TAPS - 1;
-  const int c = (blockIdx.x * SC_VTHREADS + threadIdx.x) * 4, t0 = blockIdx.y * SC_VRPT;
+  const int c = (blockIdx.x * SC_VTHREADS + threadIdx.x) * 4, t0 = blockIdx.y * R;
   if (c >= p.C) { pdl_sync(); return; }
   float w[4][TAPS], bias[4], ib[4];
   if (TAPS == 4 && reinterpret_cast<uintptr_t>(p.w) % 16 == 0) {          // (a channel's taps are one load)
@@ -170,18 +171,18 @@ __global__ void __launch_bounds__(SC_VTHREADS) short_conv_rows4_kernel(ShortConv
     ib[e] = p.in_bias ? p.in_bias[c + e] : 0.f;
   }
   pdl_sync();
-  float u[SC_VRPT + K][4];
+  float u[R + K][4];
 #pragma unroll
-  for (int i = 0; i < SC_VRPT + K; ++i) {
+  for (int i = 0; i < R + K; ++i) {
     const int t = t0 - K + i;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (t >= 0 && t < p.T) v = *reinterpret_cast<const float4*>(p.in + static_cast<size_t>(t) * p.ld_in + c);
     u[i][0] = v.x + ib[0]; u[i][1] = v.y + ib[1]; u[i][2] = v.z + ib[2]; u[i][3] = v.w + ib[3];
   }
   const int b0 = p.row_req[t0];
-  const bool inside = t0 - p.qo_indptr[b0] >= K && p.row_req[min(t0 + SC_VRPT, p.T) - 1] == b0;
+  const bool inside = t0 - p.qo_indptr[b0] >= K && p.row_req[min(t0 + R, p.T) - 1] == b0;
 #pragma unroll
-  for (int r2 = 0; r2 < SC_VRPT; r2 += 2) {          // two rows: eight quotients go through their steps together
+  for (int r2 = 0; r2 < R; r2 += 2) {          // two rows: eight quotients go through their steps together
     if (t0 + r2 >= p.T) break;
     float acc[8];
 #pragma unroll
@@ -335,16 +336,27 @@ int vb_short_conv(void* d_out, int ld_out, float* d_out_f32, int ld_f32, const f
     return q == nullptr || (ld % 4 == 0 && reinterpret_cast<uintptr_t>(q) % bytes == 0);
   };
   const bool vec = rows_form && channels % 4 == 0 && fits(d_in, ld_in, 16) && fits(d_out, ld_out, f32 ? 16 : 8) && fits(d_out_f32, ld_f32, 16);
-  const dim3 vec_grid((channels / 4 + SC_VTHREADS - 1) / SC_VTHREADS, (T + SC_VRPT - 1) / SC_VRPT);
-  if (vec && taps == 2) {
-    if (f32) VB_LAUNCH_PDL((short_conv_rows4_kernel<float, 2>), vec_grid, SC_VTHREADS, 0, stream, p);
-    else VB_LAUNCH_PDL((short_conv_rows4_kernel<bf16, 2>), vec_grid, SC_VTHREADS, 0, stream, p);
-  } else if (vec && taps == 3) {
-    if (f32) VB_LAUNCH_PDL((short_conv_rows4_kernel<float, 3>), vec_grid, SC_VTHREADS, 0, stream, p);
-    else VB_LAUNCH_PDL((short_conv_rows4_kernel<bf16, 3>), vec_grid, SC_VTHREADS, 0, stream, p);
-  } else if (vec && taps == 4) {
-    if (f32) VB_LAUNCH_PDL((short_conv_rows4_kernel<float, 4>), vec_grid, SC_VTHREADS, 0, stream, p);
-    else VB_LAUNCH_PDL((short_conv_rows4_kernel<bf16, 4>), vec_grid, SC_VTHREADS, 0, stream, p);
+  // Rows a thread: two up to three blocks of four rows an SM.  us with 2 / 4 / 8 rows a thread (and with the kernel before, four rows tap by tap): 512 channels, 64 and 1001 rows 4.0 /
+  // 4.7 / 6.3 (5.4), 4.5 / 5.0 / 6.5 (5.7); 2048, 160, 300, 600 and 1001 rows 4.4 / 5.1 / 6.8 (5.8), 5.0 / 5.2 / 6.9 (6.4), 7.1 / 6.2 / 7.5 (8.0), 9.3 / 8.3 / 8.3 (12.0); 6144, 64, 160, 300 and
+  // 1001 rows 4.5 / 5.1 / 7.2 (5.8), 5.8 / 5.8 / 7.3 (7.2), 8.8 / 7.6 / 8.3 (11.0), 19.5 / 15.2 / 16.5 (24.8).
+  const int per_row = (channels / 4 + SC_VTHREADS - 1) / SC_VTHREADS;
+  const bool two = static_cast<long long>(per_row) * ((T + 3) / 4) <= 3LL * sm_count();
+  const dim3 vec_grid(per_row, two ? (T + 1) / 2 : (T + 3) / 4);
+  auto rows4 = [&](auto c, auto t) -> int {
+    using CT = decltype(c);
+    constexpr int TAPS = decltype(t)::value;
+    if (two) VB_LAUNCH_PDL((short_conv_rows4_kernel<CT, TAPS, 2>), vec_grid, SC_VTHREADS, 0, stream, p);
+    else VB_LAUNCH_PDL((short_conv_rows4_kernel<CT, TAPS, 4>), vec_grid, SC_VTHREADS, 0, stream, p);
+    return 0;
+  };
+  auto taps_of = [&](auto c) -> int {
+    if (taps == 2) return rows4(c, std::integral_constant<int, 2>());
+    if (taps == 3) return rows4(c, std::integral_constant<int, 3>());
+    return rows4(c, std::integral_constant<int, 4>());
+  };
+  if (vec) {
+    const int r = f32 ? taps_of(0.f) : taps_of(bf16());
+    if (r) return r;
   } else if (T >= 64 && taps == 2) {
     if (f32) VB_LAUNCH_PDL((short_conv_rows_kernel<float, 2>), rows_grid, 256, 0, stream, p);
     else VB_LAUNCH_PDL((short_conv_rows_kernel<bf16, 2>), rows_grid, 256, 0, stream, p);

@@ -114,6 +114,23 @@ def tensor_map_2d(t: torch.Tensor, box_rows: int, cache: bool = True) -> TensorM
     return tm
 
 
+_TILE_BOXES = (64, 80, 96, 128)          # rows of the boxes of vb_gemm_bf16_wide_tiles
+
+
+def _tile_maps(x: torch.Tensor):
+    """the four maps of ``x`` that token tiles from a table need, as the array that the entry point takes; one place in the cache"""
+    key = (x.data_ptr(), x.shape[0], x.shape[1], x.stride(0), _TILE_BOXES)
+    got = None if _map2d_cache is None else _map2d_cache.get(key)
+    if got is None:
+        maps = [tensor_map_2d(x, rows, cache=False) for rows in _TILE_BOXES]
+        got = _map2d_cache[key] = ((ctypes.c_void_p * len(maps))(*(m.ptr for m in maps)), maps)
+        while len(_map2d_cache) > _MAP2D_CACHE_MAX:
+            _map2d_cache.popitem(last=False)
+    else:
+        _map2d_cache.move_to_end(key)
+    return got[0]
+
+
 # ----------------------------------------------------------------------------------------------
 # norm / rope / paging
 # ----------------------------------------------------------------------------------------------
@@ -1603,8 +1620,7 @@ def gemm_tiles(x: torch.Tensor, w: "PackedWeight", out: torch.Tensor, mode: int,
     if glu is not None:
         _positive_limit(glu[0])
     n_out = N // 2 if mode == 2 else N
-    maps = [tensor_map_2d(x, rows) for rows in (64, 80, 96, 128)]
-    call("vb_gemm_bf16_wide_tiles", out.data_ptr(), w.data.data_ptr(), (ctypes.c_void_p * 4)(*(m.ptr for m in maps)), x.shape[0], N, K, n_out, mode, w.tile_rows, n_out,
+    call("vb_gemm_bf16_wide_tiles", out.data_ptr(), w.data.data_ptr(), _tile_maps(x), x.shape[0], N, K, n_out, mode, w.tile_rows, n_out,
          GEMM_ACTS[act], tiles.data_ptr(), tiles.shape[0] - 1, int(group_bytes), int(w_kb_stride), int(group_kb), *map(float, glu or (0.0, 0.0)),
          _stream())
     return out

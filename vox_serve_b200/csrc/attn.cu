@@ -520,8 +520,10 @@ __global__ void __launch_bounds__(288, MINB) paged_attn_kernel(const AttnParams 
 #pragma unroll
               for (int j = 0; j < D / 32; ++j) acc[hh][j] = 0.f;
             }
-            // (two parts per round keeps the kernel under the 112 registers that let two CTAs share an SM)
-            constexpr int MP = 2;
+            // Parts of a round, whose loads are in flight together: a round is a trip to L2.  Two keep the kernel under the registers that let two CTAs share an SM; with the SM to itself
+            // and 64 columns four fit (with 128 four spill, and 32 rows of 20 to 100 tokens take 10.6 us for 8.9).  32 heads on 8 of 64, us of a launch by two / by four, for 1 row of 257, 800
+            // and 2000 tokens 10.8 / 8.6, 26.3 / 16.1, 58.9 / 31.9; 2 of 188 and 749 23.3 / 14.9; 8 of 100 to 700 26.4 / 17.9; 16 of 193 to 781 15.5 / 13.4.
+            constexpr int MP = MINB == 1 && D == 64 ? 4 : 2;
             for (int cb = 0; cb < n; cb += MP) {
               float mm[MP][4], ll[MP][4], v[MP][4][D / 32];
 #pragma unroll

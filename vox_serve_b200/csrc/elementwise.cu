@@ -1078,8 +1078,8 @@ int vb_qkv_rope_append(void* d_q_out, void* d_layer_kv, const float* d_partials,
   const int n_heads = n_q + 2 * n_kv;
   auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
   // Whole heads in halves without norms: 256 items of 16 columns and more to a row (rows kernel) past 256 rows, before that a row's items over blocks (row kernel); the rest
-  // below.  us behind the kernel that writes the planes, below / row / rows kernel, 24 + 8 + 8 heads of 128: three planes of 1 row 3.1 / 2.4, of 32 3.3 / 2.8, four of 133 4.5 / 3.8 / 4.8,
-  // three of 256 6.6 / 4.8 / 4.9, one of 512 5.5 (row) / 5.2 (rows), of 1024 8.2 / 7.5; 32 + 8 + 8 of 64: 3.2 / 2.7, 3.2 / 2.7, 4.0 / 3.2 / 3.3, 6.0 / 3.3 / 3.4, 4.2 / 3.5, 5.4 / 5.1.
+  // below.  us behind the kernel that writes the planes, below / row / rows kernel, 24 + 8 + 8 heads of 128: three planes of 1 row 2.7 / 2.8, of 32 3.4 / 3.3, four of 133 4.5 / 3.8 / 4.8,
+  // three of 256 6.6 / 4.8 / 4.9, one of 512 5.5 (row) / 5.2 (rows), of 1024 8.2 / 7.5; 32 + 8 + 8 of 64: 3.1 / 2.5, 3.2 / 2.8, 3.9 / 3.1 / 3.3, 6.0 / 3.4 / 3.4, 4.2 / 3.5, 5.4 / 5.1.
   if (T <= 256 && !interleave && rotary_dim == head_dim && head_dim % 16 == 0 && head_dim <= 256 && !d_q_norm && aligned(d_q_out) && aligned(d_layer_kv) &&
       aligned(d_partials)) {
     const int rb = T <= 64 ? 32 : 128;          // (in a decode step of 32 rows, two layers: blocks of 32 / 64 / 128 193.2 / 193.9 / 194.6 us)
